@@ -186,6 +186,7 @@ extern "C" int32_t evb_trim_cache(int32_t device) {
     int prev = 0;
     EVB_CUDA(cudaGetDevice(&prev));
     EVB_CUDA(cudaSetDevice(device));
+    evb_predict_trim(device); // its device blocks go into the cache first
     {
         DevCache &c = g_cache[device];
         std::lock_guard<std::mutex> lock(c.mu);

@@ -229,6 +229,8 @@ int32_t evb_launch_tree_reset(evb_handle *h);
 int32_t evb_launch_scan(evb_handle *h, int level);
 int32_t evb_launch_partition(evb_handle *h, int level); // plan + flags + prefix (+allreduce) + level plan + scatter
 int32_t evb_launch_lonely_barrier(evb_handle *h, int *flags, int *seq, unsigned max_polls);
+int32_t evb_check_device(int device); // evb_rows.cu: makes `device` current
+void evb_predict_trim(int device);       // evb_predict.cu: kept work buffers back to the block cache
 // evb_nccl.cpp
 int32_t evb_nccl_unique_id(uint8_t id[128]);
 int32_t evb_nccl_init(evb_handle *h, const uint8_t id[128], int rank, int world);
@@ -248,6 +250,10 @@ void evb_stream_put(cudaStream_t st);
 cudaError_t evb_event_get(cudaEvent_t *ev);
 void evb_event_put(cudaEvent_t ev);
 
+// fn(ctx, begin, end) over [0, n) in slices by all staging threads and the caller
+void evb_parallel(void (*fn)(void *, size_t, size_t), void *ctx, size_t n, size_t slice);
+// host copies between a packed buffer and nseg strided segments by all staging threads (`up`: strided -> packed)
+void evb_copy_packed(void *packed, const void *strided, size_t seg, size_t stride, size_t off, size_t len, bool up);
 int32_t evb_h2d_staged(void *dst_dev, const void *src_host, size_t bytes, cudaStream_t st, bool drain = true);
 int32_t evb_h2d_staged_strided(void *dst_dev, const void *src_host, size_t seg_bytes, size_t nseg, size_t stride, cudaStream_t st, bool drain = true);
 

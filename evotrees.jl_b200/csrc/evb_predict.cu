@@ -1,0 +1,730 @@
+// Inference over all trees: `_predict` and `_predict_leaf_indices` (src/predict.jl:118-136, 173-185; GPU counterpart
+// ext/EvoTreesKernelAbstractionsExt/predict.jl:115-158), `binarize` of the rows (src/fit-utils.jl:66-72) included.
+//
+// A model is packed once (evb_model_create) and its trees stay on the device; a call then moves only rows and predictions.
+// The kernels take raw features, turn them into bins in shared memory and walk the trees from there: the bins never reach
+// global memory.  Predictions (and leaf ids) are stored straight into pinned host memory.
+#include "evb_device.cuh"
+#include <algorithm>
+#include <atomic>
+#include <mutex>
+#include <new>
+#include <string.h>
+#include <stdlib.h>
+
+namespace {
+
+constexpr unsigned FULL = 0xffffffffu;
+
+// Trees in device memory: tree t at word t * tw, [nnp] packed nodes, then [nnp * K] leaf values (zero padded); nnp = nodes
+// rounded up to a multiple of four, so that every tree starts on a 16-byte boundary.
+struct PredArgs {
+    const void *x;          // raw features (T = float / double) or bins (T = uint8_t)
+    long long ld;           // row-major: elements between rows; column-major: between features
+    int row_major;
+    int vec;                // row-major float rows whose features can be read as float4 (16-byte aligned rows)
+    const void *edges;      // [nfeats][nedges] ascending, same type as x
+    int nedges, nfeats, FW; // FW: words of four bins per row
+    const uint32_t *trees;
+    int nnp, tw, levels;    // levels: tests on the longest path of a tree
+    float *out;             // column k of row i at k * out_ld + i
+    long long out_ld;
+    uint32_t *leaf_idx;     // null, or tree t of row i at t * out_ld + i
+    int n, K, loss, ntrees, apply_link;
+};
+
+// bins 4 w .. 4 w + 3 of row i as one word: searchsortedfirst(edges[j], x) = 1 + number of edges below x.  Four searches
+// side by side; lanes are adjacent rows.
+template <typename T>
+__device__ __forceinline__ uint32_t bin_word(const PredArgs &a, long long i, int w) {
+    const T *x = static_cast<const T *>(a.x);
+    const int j0 = 4 * w, nj = min(4, a.nfeats - j0);
+    T v[4];
+    if (sizeof(T) == 4 && a.vec && nj == 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(a.x) + i * a.ld + j0);
+        v[0] = (T)q.x; v[1] = (T)q.y; v[2] = (T)q.z; v[3] = (T)q.w;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            v[q] = (T)0;
+            if (q < nj) v[q] = a.row_major ? x[i * a.ld + j0 + q] : x[(long long)(j0 + q) * a.ld + i];
+        }
+    }
+    uint32_t word = 0;
+    if constexpr (sizeof(T) == 1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) word |= (uint32_t)v[q] << (8 * q);
+        return word;
+    } else {
+        const T *e = static_cast<const T *>(a.edges) + (size_t)j0 * a.nedges;
+        int lo[4] = {0, 0, 0, 0};
+        int len = a.nedges; // the answer lies in [lo, lo + len]: the four searches halve the same length
+        while (len > 0) {
+            const int half = (len + 1) >> 1;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (q < nj && __ldg(e + (size_t)q * a.nedges + lo[q] + half - 1) < v[q]) lo[q] += half;
+            len -= half;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (q < nj) word |= (uint32_t)(lo[q] + 1) << (8 * q);
+        return word;
+    }
+}
+
+__device__ __forceinline__ void link_row(int loss, int K, float *p) { // apply_prediction_link! (src/predict.jl:105-116)
+    if (loss == EVB_LOGLOSS) { for (int k = 0; k < K; ++k) p[k] = sigmoidf_(p[k]); }
+    else if (loss == EVB_GAUSSIAN_MLE || loss == EVB_LOGISTIC_MLE) { for (int k = 1; k < K; k += 2) p[k] = softplusf_(p[k]); }
+    else if (loss == EVB_POISSON || loss == EVB_GAMMA || loss == EVB_TWEEDIE) { for (int k = 0; k < K; ++k) p[k] = expf(p[k]); }
+    else if (loss == EVB_MLOGLOSS) {
+        float s = 0.0f;
+        for (int k = 0; k < K; ++k) { p[k] = expf(p[k]); s += p[k]; }
+        for (int k = 0; k < K; ++k) p[k] /= s;
+    }
+}
+
+// one test of a node: the child of node `nid` for a row whose word of bins `word` holds the node's feature
+__device__ __forceinline__ int child(uint32_t pk, uint32_t word, int nid) {
+    const uint32_t x = (word >> (8u * (pk & 3u))) & 0xffu, bin = (pk >> 16) & 0xffu;
+    const bool cond = ((pk >> 25) & 1u) ? (x <= bin) : (x == bin);
+    return (nid << 1) + (cond ? 0 : 1); // nid = nid << 1 + !cond (src/predict.jl:7)
+}
+
+// ---------------------------------------------------------------------------------- few rows
+// One CTA per row, one thread per tree: what bounds a call with a handful of rows is latency, so the levels of all trees
+// are walked at the same time and only the sum over the trees is serial (the clamps of `predict!` do not commute, so the
+// trees are added in order).  Bins: one warp per feature counts the edges below the value, 32 edges per load.
+// Measured (call of 1 row x 10 features, 101 trees of depth 6): 365 us with one thread walking all trees, every tree uploaded
+// by the call and a stream and eight events made for it, 31 us like this.
+constexpr int ONE_THREADS = 256;
+template <int KMAX, typename T>
+__global__ void __launch_bounds__(ONE_THREADS) k_predict_one(PredArgs a) {
+    extern __shared__ uint32_t s_one[]; // [FW] bins of the row, then [ONE_THREADS][K] leaf values
+    const int K = a.K, tid = threadIdx.x, lane = tid & 31;
+    const long long i = blockIdx.x;
+    uint8_t *s_bins = reinterpret_cast<uint8_t *>(s_one);
+    float *s_leaf = reinterpret_cast<float *>(s_one + a.FW);
+    for (int j = tid >> 5; j < a.nfeats; j += ONE_THREADS / 32) {
+        const T v = a.row_major ? static_cast<const T *>(a.x)[i * a.ld + j] : static_cast<const T *>(a.x)[(long long)j * a.ld + i];
+        int c = 0;
+        if constexpr (sizeof(T) == 1) c = (int)v;
+        else {
+            const T *e = static_cast<const T *>(a.edges) + (size_t)j * a.nedges;
+            for (int b = 0; b < a.nedges; b += 32) c += __popc(__ballot_sync(FULL, b + lane < a.nedges && __ldg(e + min(b + lane, a.nedges - 1)) < v));
+            ++c;
+        }
+        if (lane == 0) s_bins[j] = (uint8_t)c;
+    }
+    float p[KMAX];
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) p[k] = 0.0f;
+    for (int t0 = 0; t0 < a.ntrees; t0 += ONE_THREADS) {
+        __syncthreads();
+        const int t = t0 + tid;
+        if (t < a.ntrees) {
+            const uint32_t *tr = a.trees + (size_t)t * a.tw;
+            int nid = 1;
+            uint32_t pk = __ldg(tr);
+            while ((pk >> 24) & 1u) {
+                nid = child(pk, s_one[(pk & 0xffffu) >> 2], nid);
+                pk = __ldg(tr + nid - 1);
+            }
+            if (a.leaf_idx) a.leaf_idx[(size_t)t * a.out_ld + i] = (uint32_t)nid;
+            for (int k = 0; k < K; ++k) s_leaf[tid * K + k] = __uint_as_float(__ldg(tr + a.nnp + (nid - 1) * K + k));
+        }
+        __syncthreads();
+        if (tid == 0) {
+            const int nt = min(ONE_THREADS, a.ntrees - t0);
+#pragma unroll 4
+            for (int q = 0; q < nt; ++q) pred_add(a.loss, K, p, s_leaf + q * K);
+        }
+    }
+    if (tid == 0) {
+        if (a.apply_link) link_row(a.loss, K, p);
+        for (int k = 0; k < K; ++k) a.out[(size_t)k * a.out_ld + i] = p[k];
+    }
+}
+
+// ---------------------------------------------------------------------------------- some thousand rows
+// One CTA per 32 rows (lane = row).  Seven warps share the trees of a block of TB and leave the leaf values in shared
+// memory, four trees at a time per lane so that four chains of loads overlap; the eighth warp adds the previous block's
+// values in order meanwhile.  Nodes come through L1: 32 rows do not pay for copying a tree into shared memory.  Bins are
+// word-major ([word of the row][row]): a lane only ever reads its own bank.
+// Measured (call of 20 011 rows x 28, 201 trees of depth 8, five classes): 1.26 ms with 20 CTAs of 1024 rows (378 us of it
+// their kernel), 0.235 ms like this.
+constexpr int MID_WARPS = 8, MID_ILP = 4;
+template <int KMAX, typename T>
+__global__ void __launch_bounds__(MID_WARPS * 32) k_predict_mid(PredArgs a, int TB) {
+    extern __shared__ uint32_t s_mid[]; // [FW][32] bins, then [2][TB][K][32] leaf values
+    const int K = a.K, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long row0 = (long long)blockIdx.x * 32, i = row0 + lane;
+    const bool act = i < a.n;
+    for (int w = wid; w < a.FW; w += MID_WARPS) s_mid[w * 32 + lane] = act ? bin_word<T>(a, i, w) : 0u;
+    float *s_leaf = reinterpret_cast<float *>(s_mid + a.FW * 32);
+    __syncthreads();
+    float p[KMAX];
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) p[k] = 0.0f;
+    int buf = 0;
+    for (int t0 = 0;; t0 += TB, buf ^= 1) {
+        const int nt = min(TB, a.ntrees - t0); // <= 0: only the last block's sum is left
+        if (wid > 0) {
+            for (int tb = wid - 1; tb < nt; tb += (MID_WARPS - 1) * MID_ILP) {
+                const uint32_t *tr[MID_ILP];
+                int nid[MID_ILP];
+                uint32_t pk[MID_ILP];
+#pragma unroll
+                for (int u = 0; u < MID_ILP; ++u) {
+                    const int t = tb + u * (MID_WARPS - 1);
+                    tr[u] = a.trees + (size_t)(t0 + (t < nt ? t : tb)) * a.tw;
+                    nid[u] = 1;
+                    pk[u] = __ldg(tr[u]);
+                }
+                for (int l = 0; l < a.levels; ++l) {
+#pragma unroll
+                    for (int u = 0; u < MID_ILP; ++u) {
+                        if ((pk[u] >> 24) & 1u) {
+                            nid[u] = child(pk[u], s_mid[((pk[u] & 0xffffu) >> 2) * 32 + lane], nid[u]);
+                            pk[u] = __ldg(tr[u] + nid[u] - 1);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < MID_ILP; ++u) {
+                    const int t = tb + u * (MID_WARPS - 1);
+                    if (t < nt) {
+                        const uint32_t *lf = tr[u] + a.nnp + (nid[u] - 1) * K;
+                        float *d = s_leaf + ((size_t)(buf * TB + t) * K) * 32 + lane;
+                        for (int k = 0; k < K; ++k) d[k * 32] = __uint_as_float(__ldg(lf + k));
+                        if (a.leaf_idx && act) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = (uint32_t)nid[u];
+                    }
+                }
+            }
+        } else if (t0 > 0) {
+            const int np = min(TB, a.ntrees - (t0 - TB));
+            const float *s = s_leaf + ((size_t)(buf ^ 1) * TB * K) * 32 + lane;
+            for (int t = 0; t < np; ++t) {
+                float lf[KMAX];
+#pragma unroll
+                for (int k = 0; k < KMAX; ++k) if (k < K) lf[k] = s[(t * K + k) * 32];
+                pred_add(a.loss, K, p, lf);
+            }
+        }
+        if (nt <= 0) break;
+        __syncthreads();
+    }
+    if (wid == 0 && act) {
+        if (a.apply_link) link_row(a.loss, K, p);
+        for (int k = 0; k < K; ++k) a.out[(size_t)k * a.out_ld + i] = p[k];
+    }
+}
+
+// ---------------------------------------------------------------------------------- many rows
+// One thread = one row.  The CTA's bins sit in shared memory word-major, and the trees (nodes + leaf tables) stream through
+// two shared-memory buffers of TB trees each: while the threads walk the trees of one buffer, `cp.async` fills the other,
+// so a traversal step costs two shared-memory loads and the trip to L2 is off the critical path.
+template <int KMAX, typename T>
+__global__ void __launch_bounds__(1024) k_predict_staged(PredArgs a, int TB) {
+    extern __shared__ __align__(16) uint32_t s_pr[]; // [FW][blockDim.x] bins, then 2 x TB x tw tree words
+    const int K = a.K, rows = blockDim.x, tw = a.tw;
+    uint32_t *s_rows = s_pr;
+    uint32_t *s_trees = s_pr + (size_t)rows * a.FW; // rows is a multiple of 4: 16-byte aligned
+    const long long row0 = (long long)blockIdx.x * rows;
+    auto load_block = [&](int t0, int buf) { // trees t0 .. t0 + TB - 1 -> buffer `buf`, 16 bytes per copy
+        const int nt = min(TB, a.ntrees - t0);
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.trees + (size_t)t0 * tw);
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_trees + (size_t)buf * TB * tw);
+        for (int c = threadIdx.x; c < nt * (tw >> 2); c += rows)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)c * 16u), "l"(src + c) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_block(0, 0);
+    const long long i = row0 + threadIdx.x;
+    const bool act = i < a.n;
+    uint32_t *xcol = s_rows + threadIdx.x;
+    if (act)
+        for (int w = 0; w < a.FW; ++w) xcol[w * rows] = bin_word<T>(a, i, w);
+    float p[KMAX];
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) p[k] = 0.0f;
+    int buf = 0;
+    for (int t0 = 0; t0 < a.ntrees; t0 += TB, buf ^= 1) {
+        const int nt = min(TB, a.ntrees - t0);
+        if (t0 + TB < a.ntrees) load_block(t0 + TB, buf ^ 1); // the other buffer was consumed before the last barrier
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads(); // this block's trees are in place for everybody
+        if (act) {
+            for (int t = 0; t < nt; ++t) {
+                const uint32_t *tr = s_trees + ((size_t)buf * TB + t) * tw;
+                int nid = 1;
+                uint32_t pk = tr[0];
+                while ((pk >> 24) & 1u) {
+                    nid = child(pk, xcol[((pk & 0xffffu) >> 2) * rows], nid);
+                    pk = tr[nid - 1];
+                }
+                if (a.leaf_idx) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = (uint32_t)nid;
+                pred_add(a.loss, K, p, reinterpret_cast<const float *>(tr + a.nnp) + (size_t)(nid - 1) * K);
+            }
+        }
+        __syncthreads(); // everybody is done with this buffer: the next iteration refills it
+    }
+    if (!act) return;
+    if (a.apply_link) link_row(a.loss, K, p);
+    for (int k = 0; k < K; ++k) a.out[(size_t)k * a.out_ld + i] = p[k];
+}
+
+// rows of more bins than shared memory holds: bins in global memory ([row][FW] words), one thread per row
+template <typename T>
+__global__ void __launch_bounds__(256) k_bin_rows(PredArgs a, uint32_t *xw) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= a.n) return;
+    for (int w = blockIdx.y; w < a.FW; w += gridDim.y) xw[(size_t)i * a.FW + w] = bin_word<T>(a, i, w);
+}
+template <int KMAX>
+__global__ void __launch_bounds__(256) k_predict_wide(PredArgs a, const uint32_t *xw) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= a.n) return;
+    const uint32_t *xr = xw + (size_t)i * a.FW;
+    float p[KMAX];
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) p[k] = 0.0f;
+    const int K = a.K;
+    for (int t = 0; t < a.ntrees; ++t) {
+        const uint32_t *tr = a.trees + (size_t)t * a.tw;
+        int nid = 1;
+        uint32_t pk = __ldg(tr);
+        while ((pk >> 24) & 1u) {
+            nid = child(pk, xr[(pk & 0xffffu) >> 2], nid);
+            pk = __ldg(tr + nid - 1);
+        }
+        if (a.leaf_idx) a.leaf_idx[(size_t)t * a.out_ld + i] = (uint32_t)nid;
+        pred_add(a.loss, K, p, reinterpret_cast<const float *>(tr + a.nnp) + (size_t)(nid - 1) * K);
+    }
+    if (a.apply_link) link_row(a.loss, K, p);
+    for (int k = 0; k < K; ++k) a.out[(size_t)k * a.out_ld + i] = p[k];
+}
+
+} // namespace
+
+// ================================================================================================= models
+struct evb_model {
+    int device = 0, loss = 0, K = 1, ntrees = 0, nnp = 4, tw = 8, levels = 0, nfeats = 0, nedges = 0;
+    void *block = nullptr;            // trees, then the edges as double and as float
+    const uint32_t *d_trees = nullptr;
+    const double *d_e64 = nullptr;
+    const float *d_e32 = nullptr;
+    // Where the trees and the edges came from and what they held when they were packed: a call compares them while the GPU
+    // works, so a tree that was changed in place since is noticed.
+    std::vector<const void *> src;    // [ntrees][4]: feat, cond_bin, split, leaf_pred
+    std::vector<int32_t> nodes;       // nodes of every tree
+    std::vector<size_t> at;           // offset of every tree's copy in `snap`
+    std::vector<unsigned char> snap;
+    const void *src_edges = nullptr, *src_ft = nullptr;
+    std::vector<unsigned char> snap_edges, snap_ft;
+};
+
+namespace {
+
+size_t tree_bytes(int nn, int K, int part) { return part == 0 ? (size_t)nn * 8 : part == 3 ? (size_t)nn * K * 4 : (size_t)nn; }
+
+struct VerifyJob { const evb_model *m; std::atomic<int> bad; };
+void verify_range(void *c, size_t b, size_t e) {
+    VerifyJob &j = *static_cast<VerifyJob *>(c);
+    for (size_t t = b; t < e && j.bad.load(std::memory_order_relaxed) == 0; ++t) {
+        size_t o = j.m->at[t];
+        for (int q = 0; q < 4; ++q) {
+            const size_t n = tree_bytes(j.m->nodes[t], j.m->K, q);
+            if (memcmp(j.m->src[t * 4 + q], j.m->snap.data() + o, n) != 0) { j.bad.store(1); return; }
+            o += n;
+        }
+    }
+}
+// the sources still hold what was packed
+bool model_current(const evb_model *m) {
+    VerifyJob j{m, {0}};
+    const size_t per = m->ntrees > 0 ? m->snap.size() / m->ntrees : 0;
+    const size_t slice = per ? std::max<size_t>(1, ((size_t)256 << 10) / per) : 1;
+    evb_parallel(verify_range, &j, (size_t)m->ntrees, slice);
+    return j.bad.load() == 0 && (m->snap_edges.empty() || memcmp(m->src_edges, m->snap_edges.data(), m->snap_edges.size()) == 0) &&
+           (m->snap_ft.empty() || memcmp(m->src_ft, m->snap_ft.data(), m->snap_ft.size()) == 0);
+}
+
+// src: [ntrees][4] pointers; packs, uploads and keeps the snapshot.  edges may be null (binned input only).
+int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32_t *nodes, const void *edges, int e_dtype, int nedges,
+                   int nfeats, const uint8_t *feattypes, bool snapshot) {
+    const int K = m->K;
+    int nn = 1;
+    for (int t = 0; t < ntrees; ++t) nn = std::max(nn, (int)nodes[t]);
+    m->ntrees = ntrees; m->nfeats = nfeats; m->nedges = edges ? nedges : 0;
+    m->nnp = (nn + 3) & ~3;
+    m->tw = m->nnp * (1 + K);
+    m->levels = 0;
+    while ((2 << m->levels) - 1 < nn) ++m->levels;
+    const size_t tbytes = (size_t)ntrees * m->tw * 4, ne = (size_t)m->nedges * nfeats;
+    const size_t o64 = (tbytes + 15) & ~(size_t)15, o32 = o64 + ne * 8;
+    std::vector<unsigned char> host(o32 + ne * 4 + 16, 0);
+    uint32_t *tr = reinterpret_cast<uint32_t *>(host.data());
+    for (int t = 0; t < ntrees; ++t, tr += m->tw) {
+        const int64_t *feat = static_cast<const int64_t *>(src[t * 4]);
+        const uint8_t *bin = static_cast<const uint8_t *>(src[t * 4 + 1]), *split = static_cast<const uint8_t *>(src[t * 4 + 2]);
+        for (int i = 0; i < nodes[t]; ++i) {
+            if (!split[i]) continue;
+            const int64_t f = feat[i] - 1;
+            if (f < 0 || f >= nfeats || 2 * i + 2 >= nodes[t]) {
+                evb_set_error("evb_model: node %d of tree %d tests feature %lld of %d or has no children", i + 1, t + 1, (long long)(f + 1), nfeats);
+                return EVB_ERR_ARG;
+            }
+            tr[i] = (uint32_t)f | ((uint32_t)bin[i] << 16) | (1u << 24) | ((feattypes ? (feattypes[f] ? 1u : 0u) : 1u) << 25);
+        }
+        memcpy(tr + m->nnp, src[t * 4 + 3], (size_t)nodes[t] * K * 4);
+    }
+    if (edges) {
+        double *e64 = reinterpret_cast<double *>(host.data() + o64);
+        float *e32 = reinterpret_cast<float *>(host.data() + o32);
+        for (size_t i = 0; i < ne; ++i) {
+            if (e_dtype == EVB_F64) { e64[i] = static_cast<const double *>(edges)[i]; e32[i] = (float)e64[i]; }
+            else { e32[i] = static_cast<const float *>(edges)[i]; e64[i] = e32[i]; }
+        }
+    }
+    EVB_CUDA(evb_dev_alloc(&m->block, host.size()));
+    EVB_CUDA(cudaMemcpy(m->block, host.data(), host.size(), cudaMemcpyHostToDevice));
+    m->d_trees = static_cast<const uint32_t *>(m->block);
+    m->d_e64 = reinterpret_cast<const double *>(static_cast<char *>(m->block) + o64);
+    m->d_e32 = reinterpret_cast<const float *>(static_cast<char *>(m->block) + o32);
+    if (!snapshot) return EVB_OK;
+    m->src.assign(src, src + (size_t)ntrees * 4);
+    m->nodes.assign(nodes, nodes + ntrees);
+    m->at.resize(ntrees);
+    size_t total = 0;
+    for (int t = 0; t < ntrees; ++t) { m->at[t] = total; for (int q = 0; q < 4; ++q) total += tree_bytes(nodes[t], K, q); }
+    m->snap.resize(total);
+    for (int t = 0; t < ntrees; ++t) {
+        size_t o = m->at[t];
+        for (int q = 0; q < 4; ++q) { const size_t n = tree_bytes(nodes[t], K, q); memcpy(m->snap.data() + o, src[t * 4 + q], n); o += n; }
+    }
+    if (edges) { m->src_edges = edges; m->snap_edges.assign((const unsigned char *)edges, (const unsigned char *)edges + ne * (e_dtype == EVB_F64 ? 8 : 4)); }
+    if (feattypes) { m->src_ft = feattypes; m->snap_ft.assign(feattypes, feattypes + nfeats); }
+    return EVB_OK;
+}
+
+} // namespace
+
+extern "C" void evb_model_destroy(evb_model *m) {
+    if (!m) return;
+    int prev = 0;
+    cudaGetDevice(&prev);
+    if (cudaSetDevice(m->device) == cudaSuccess) evb_dev_free(m->block);
+    cudaSetDevice(prev);
+    delete m;
+}
+
+static int32_t model_args(int32_t loss, int32_t K, int32_t ntrees, int32_t nfeats) {
+    if (nfeats < 1 || nfeats > 65535 || ntrees < 0 || K < 1 || K > 64 || loss < 0 || loss > EVB_LOSS_LAST) {
+        evb_set_error("evb_predict: invalid argument");
+        return EVB_ERR_ARG;
+    }
+    return EVB_OK;
+}
+
+extern "C" int32_t evb_model_create(evb_model **out, int32_t device, int32_t loss, int32_t K, int32_t ntrees, const void *const *src,
+                                    const int32_t *nodes, const void *edges, int32_t edges_dtype, int32_t nedges, int32_t nfeats,
+                                    const uint8_t *feattypes) {
+    if (!out) { evb_set_error("evb_model_create: out is null"); return EVB_ERR_ARG; }
+    *out = nullptr;
+    EVB_CHECK(model_args(loss, K, ntrees, nfeats));
+    if ((ntrees > 0 && (!src || !nodes)) || !edges || nedges < 1 || nedges > 254 || (edges_dtype != EVB_F32 && edges_dtype != EVB_F64)) {
+        evb_set_error("evb_model_create: invalid argument");
+        return EVB_ERR_ARG;
+    }
+    EVB_CHECK(evb_check_device(device));
+    evb_model *m = new (std::nothrow) evb_model();
+    if (!m) { evb_set_error("out of host memory"); return EVB_ERR_ARG; }
+    m->device = device; m->loss = loss; m->K = K;
+    const int32_t rc = model_fill(m, ntrees, src, nodes, edges, edges_dtype, nedges, nfeats, feattypes, true);
+    if (rc != EVB_OK) { evb_model_destroy(m); return rc; }
+    *out = m;
+    return EVB_OK;
+}
+
+// ================================================================================================= calls
+namespace {
+
+// Work buffers of one call at a time: three sets of {stream, pinned input, device input, pinned output}.  A call takes one
+// from the device's pool and puts it back; the pool keeps at most KEEP of them (evb_trim_cache gives them back).
+constexpr int PRED_SLOTS = 3;
+struct PredWs {
+    struct Slot {
+        cudaStream_t st = nullptr;
+        cudaEvent_t done = nullptr, t0 = nullptr, t1 = nullptr;
+        char *pin_in = nullptr, *pin_out = nullptr;
+        void *d_in = nullptr, *d_aux = nullptr;
+        size_t cap_pin_in = 0, cap_pin_out = 0, cap_in = 0, cap_aux = 0;
+    } s[PRED_SLOTS];
+    int dev = 0;
+};
+constexpr size_t KEEP = 4;
+struct PredPool { std::mutex mu; std::vector<PredWs *> free_ws; };
+PredPool g_pred_pool[64];
+
+void ws_delete(PredWs *w) {
+    for (auto &s : w->s) {
+        if (s.st) { cudaStreamSynchronize(s.st); cudaStreamDestroy(s.st); }
+        if (s.done) cudaEventDestroy(s.done);
+        if (s.t0) cudaEventDestroy(s.t0);
+        if (s.t1) cudaEventDestroy(s.t1);
+        if (s.pin_in) cudaFreeHost(s.pin_in);
+        if (s.pin_out) cudaFreeHost(s.pin_out);
+        evb_dev_free(s.d_in);
+        evb_dev_free(s.d_aux);
+    }
+    delete w;
+}
+struct WsGuard { // the device is current
+    PredWs *w = nullptr;
+    explicit WsGuard(int dev) {
+        if (dev < 64) {
+            std::lock_guard<std::mutex> g(g_pred_pool[dev].mu);
+            if (!g_pred_pool[dev].free_ws.empty()) { w = g_pred_pool[dev].free_ws.back(); g_pred_pool[dev].free_ws.pop_back(); return; }
+        }
+        w = new PredWs();
+        w->dev = dev;
+    }
+    ~WsGuard() {
+        for (auto &s : w->s) if (s.st) cudaStreamSynchronize(s.st); // an error may have left work behind
+        if (w->dev < 64) {
+            std::lock_guard<std::mutex> g(g_pred_pool[w->dev].mu);
+            if (g_pred_pool[w->dev].free_ws.size() < KEEP) { g_pred_pool[w->dev].free_ws.push_back(w); return; }
+        }
+        ws_delete(w);
+    }
+};
+int32_t slot_streams(PredWs::Slot &s, bool timed) {
+    if (!s.st) EVB_CUDA(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
+    if (!s.done) EVB_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
+    if (timed && !s.t0) { EVB_CUDA(cudaEventCreate(&s.t0)); EVB_CUDA(cudaEventCreate(&s.t1)); }
+    return EVB_OK;
+}
+int32_t pinned_reserve(char *&p, size_t &cap, size_t bytes) {
+    if (cap >= bytes) return EVB_OK;
+    if (p) { cudaFreeHost(p); p = nullptr; cap = 0; }
+    const size_t want = (std::max<size_t>(bytes, 65536) + 65535) & ~(size_t)65535;
+    EVB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&p), want, cudaHostAllocDefault));
+    cap = want;
+    return EVB_OK;
+}
+int32_t device_reserve(void *&p, size_t &cap, size_t bytes) {
+    if (cap >= bytes) return EVB_OK;
+    evb_dev_free(p);
+    p = nullptr; cap = 0;
+    EVB_CUDA(evb_dev_alloc(&p, bytes));
+    cap = bytes;
+    return EVB_OK;
+}
+
+constexpr int MAX_SMEM = 227 * 1024;
+template <typename K>
+int32_t allow_smem(K kern, size_t bytes) { // more than the default 48 KB of dynamic shared memory
+    if (bytes > 48 * 1024) EVB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
+    return EVB_OK;
+}
+
+// which kernel takes a chunk of n rows
+enum { PK_ONE, PK_MID, PK_STAGED, PK_WIDE };
+struct PredPlan { int kind, rows, TB; size_t smem; };
+PredPlan plan_kernel(const evb_model &m, int n, int num_sms) {
+    PredPlan p{PK_WIDE, 256, 0, 0};
+    const int FW = (m.nfeats + 3) / 4;
+    const size_t tree = (size_t)m.tw * 4;
+    // a CTA per row while the rows alone do not give every SM several of the 32-row CTAs of the next kernel
+    const size_t one = (size_t)FW * 4 + (size_t)ONE_THREADS * m.K * 4;
+    if (n <= 4 * num_sms && one <= 96 * 1024) return {PK_ONE, 1, 0, one};
+    // Staged: the largest CTA that still gives every SM one, as long as two blocks of trees fit beside its rows.  Copying
+    // all trees once per CTA has to be worth it: below `mid_rows` rows the trees are read through L1 instead.
+    const int mid_rows = 64 * 1024;
+    if (n > mid_rows) {
+        for (int rows = 1024; rows >= 128; rows >>= 1) {
+            if (rows > 256 && (n + rows - 1) / rows < num_sms) continue;
+            const size_t rb = (size_t)rows * FW * 4, room = (size_t)200 * 1024;
+            if (rb + 2 * tree > room) continue;
+            const int TB = (int)std::min<size_t>(8, (room - rb) / (2 * tree));
+            return {PK_STAGED, rows, TB, rb + 2 * (size_t)TB * tree};
+        }
+    }
+    const size_t rb = (size_t)FW * 128;
+    int TB = std::max(1, 96 / m.K); // 2 x TB x K x 128 bytes <= 24 KB
+    if (TB > (MID_WARPS - 1) * MID_ILP) TB = TB / ((MID_WARPS - 1) * MID_ILP) * ((MID_WARPS - 1) * MID_ILP);
+    const size_t mid = rb + (size_t)2 * TB * m.K * 128;
+    if (mid <= MAX_SMEM - 1024) return {PK_MID, 32, TB, mid};
+    return p;
+}
+
+template <int KMAX, typename T>
+int32_t launch_t(const PredPlan &p, PredArgs &a, uint32_t *xw, cudaStream_t st) {
+    if (p.kind == PK_ONE) {
+        EVB_CHECK(allow_smem(k_predict_one<KMAX, T>, p.smem));
+        k_predict_one<KMAX, T><<<a.n, ONE_THREADS, p.smem, st>>>(a);
+    } else if (p.kind == PK_MID) {
+        EVB_CHECK(allow_smem(k_predict_mid<KMAX, T>, p.smem));
+        k_predict_mid<KMAX, T><<<(a.n + 31) / 32, MID_WARPS * 32, p.smem, st>>>(a, p.TB);
+    } else if (p.kind == PK_STAGED) {
+        EVB_CHECK(allow_smem(k_predict_staged<KMAX, T>, p.smem));
+        k_predict_staged<KMAX, T><<<(a.n + p.rows - 1) / p.rows, p.rows, p.smem, st>>>(a, p.TB);
+    } else {
+        k_bin_rows<T><<<dim3((a.n + 255) / 256, std::min(a.FW, 64)), 256, 0, st>>>(a, xw);
+        k_predict_wide<KMAX><<<(a.n + 255) / 256, 256, 0, st>>>(a, xw);
+    }
+    EVB_CUDA(cudaGetLastError());
+    return EVB_OK;
+}
+template <typename T>
+int32_t launch_k(const PredPlan &p, PredArgs &a, uint32_t *xw, cudaStream_t st) {
+    if (a.K <= 1) return launch_t<1, T>(p, a, xw, st);
+    if (a.K <= 2) return launch_t<2, T>(p, a, xw, st);
+    if (a.K <= 8) return launch_t<8, T>(p, a, xw, st);
+    return launch_t<64, T>(p, a, xw, st);
+}
+
+// x: host rows (x_type 0 float, 2 double, -1 bins); out / leaf_idx: host.  `check`: compare the model's sources while the
+// GPU works and return EVB_ERR_STALE when they changed.
+int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, int row_major, int64_t nobs, int apply_link, float *out,
+                     uint32_t *leaf_idx, double *ms_out, bool check) {
+    if (ms_out) *ms_out = 0.0;
+    if (nobs == 0) return EVB_OK;
+    WsGuard g(m.device);
+    PredWs &w = *g.w;
+    static int num_sms[64] = {};
+    int sms = m.device < 64 ? num_sms[m.device] : 0;
+    if (sms == 0) {
+        EVB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device));
+        if (m.device < 64) num_sms[m.device] = sms;
+    }
+    const size_t es = x_type < 0 ? 1 : x_type == EVB_F64 ? 8 : 4;
+    const size_t in_row = es * m.nfeats, out_row = 4 * ((size_t)m.K + (leaf_idx ? ntrees : 0));
+    // Chunks: big enough that a chunk's fixed costs (about 15 us of launches) vanish in its transfer, small enough that the
+    // first transfer and the last kernel, which nothing overlaps with, do not show.
+    const size_t total = (size_t)nobs * (in_row + out_row);
+    size_t cbytes = total / 6;
+    cbytes = std::min<size_t>(std::max<size_t>(cbytes, (size_t)1 << 20), (size_t)8 << 20);
+    int64_t chunk = (int64_t)std::max<size_t>(1024, cbytes / (in_row + out_row)) / 1024 * 1024;
+    chunk = std::min<int64_t>(chunk, nobs);
+    // one row or a few: the kernel reads them from pinned memory itself
+    const bool zero_copy = (size_t)nobs * in_row <= (size_t)16 * 1024;
+    PredArgs a;
+    a.row_major = row_major; a.nedges = m.nedges; a.nfeats = m.nfeats; a.FW = (m.nfeats + 3) / 4;
+    a.edges = x_type == EVB_F64 ? (const void *)m.d_e64 : (const void *)m.d_e32;
+    a.trees = m.d_trees; a.nnp = m.nnp; a.tw = m.tw; a.levels = m.levels; a.K = m.K; a.loss = m.loss; a.ntrees = ntrees; a.apply_link = apply_link;
+    int64_t first[PRED_SLOTS] = {-1, -1, -1};
+    int rows_in[PRED_SLOTS] = {};
+    double ms = 0.0;
+    auto collect = [&](int q) -> int32_t { // results of the chunk in slot q -> the caller's arrays
+        PredWs::Slot &s = w.s[q];
+        if (first[q] < 0) return EVB_OK;
+        EVB_CUDA(cudaStreamSynchronize(s.st));
+        const int64_t r0 = first[q], nr = rows_in[q];
+        evb_copy_packed(s.pin_out, out + r0, (size_t)nr * 4, (size_t)nobs * 4, 0, (size_t)nr * 4 * m.K, false);
+        if (leaf_idx) evb_copy_packed(s.pin_out + (size_t)nr * 4 * m.K, leaf_idx + r0, (size_t)nr * 4, (size_t)nobs * 4, 0, (size_t)nr * 4 * ntrees, false);
+        if (ms_out) { float v = 0.f; if (cudaEventElapsedTime(&v, s.t0, s.t1) == cudaSuccess) ms += v; }
+        first[q] = -1;
+        return EVB_OK;
+    };
+    int q = 0;
+    for (int64_t r0 = 0; r0 < nobs; r0 += chunk, q = (q + 1) % PRED_SLOTS) {
+        PredWs::Slot &s = w.s[q];
+        const int64_t nr = std::min<int64_t>(chunk, nobs - r0);
+        EVB_CHECK(collect(q));
+        EVB_CHECK(slot_streams(s, ms_out != nullptr));
+        EVB_CHECK(pinned_reserve(s.pin_in, s.cap_pin_in, (size_t)chunk * in_row));
+        EVB_CHECK(pinned_reserve(s.pin_out, s.cap_pin_out, (size_t)chunk * out_row));
+        // rows r0 .. r0 + nr: one piece of a row-major matrix, one segment per feature of a column-major one
+        const char *xs = static_cast<const char *>(x);
+        if (row_major) evb_copy_packed(s.pin_in, xs + (size_t)r0 * in_row, (size_t)nr * in_row, 0, 0, (size_t)nr * in_row, true);
+        else evb_copy_packed(s.pin_in, xs + (size_t)r0 * es, (size_t)nr * es, (size_t)nobs * es, 0, (size_t)nr * in_row, true);
+        a.n = (int)nr; a.ld = row_major ? m.nfeats : nr;
+        a.vec = row_major && es == 4 && (m.nfeats & 3) == 0;
+        a.x = s.pin_in;
+        if (!zero_copy) {
+            EVB_CHECK(device_reserve(s.d_in, s.cap_in, (size_t)chunk * in_row));
+            EVB_CUDA(cudaMemcpyAsync(s.d_in, s.pin_in, (size_t)nr * in_row, cudaMemcpyHostToDevice, s.st));
+            a.x = s.d_in;
+        }
+        a.out = reinterpret_cast<float *>(s.pin_out); a.out_ld = nr;
+        a.leaf_idx = leaf_idx ? reinterpret_cast<uint32_t *>(s.pin_out + (size_t)nr * 4 * m.K) : nullptr;
+        const PredPlan p = plan_kernel(m, (int)nr, sms);
+        if (p.kind == PK_WIDE) EVB_CHECK(device_reserve(s.d_aux, s.cap_aux, (size_t)chunk * a.FW * 4));
+        if (ms_out) EVB_CUDA(cudaEventRecord(s.t0, s.st));
+        uint32_t *xw = static_cast<uint32_t *>(s.d_aux);
+        EVB_CHECK(x_type < 0 ? launch_k<uint8_t>(p, a, xw, s.st) : x_type == EVB_F64 ? launch_k<double>(p, a, xw, s.st) : launch_k<float>(p, a, xw, s.st));
+        if (ms_out) EVB_CUDA(cudaEventRecord(s.t1, s.st));
+        first[q] = r0; rows_in[q] = (int)nr;
+    }
+    if (check && !model_current(&m)) { evb_set_error("evb_model_predict: the model's trees changed since they were packed"); return EVB_ERR_STALE; }
+    for (int k = 0; k < PRED_SLOTS; ++k, q = (q + 1) % PRED_SLOTS) EVB_CHECK(collect(q)); // oldest first
+    if (ms_out) *ms_out = ms;
+    return EVB_OK;
+}
+
+} // namespace
+
+// gives the kept work buffers of a device back (the device is current)
+void evb_predict_trim(int device) {
+    std::vector<PredWs *> ws;
+    { std::lock_guard<std::mutex> g(g_pred_pool[device].mu); ws.swap(g_pred_pool[device].free_ws); }
+    for (PredWs *w : ws) ws_delete(w);
+}
+
+extern "C" int32_t evb_model_predict(const evb_model *m, int32_t ntrees, const void *x, int32_t x_dtype, int32_t x_row_major, int64_t nobs,
+                                     int32_t apply_link, float *out, uint32_t *leaf_idx, double *kernel_ms) {
+    if (!m || !x || !out || nobs < 0 || ntrees < 0 || ntrees > m->ntrees || (x_dtype != EVB_F32 && x_dtype != EVB_F64)) {
+        evb_set_error("evb_model_predict: invalid argument");
+        return EVB_ERR_ARG;
+    }
+    EVB_CUDA(cudaSetDevice(m->device));
+    return predict_rows(*m, ntrees, x, x_dtype, x_row_major, nobs, apply_link, out, leaf_idx, kernel_ms, true);
+}
+
+// one call with trees that are packed for it: evb_predict (bins) and evb_predict_x (raw features)
+static int32_t predict_once(int32_t device, int32_t loss, int32_t K, int32_t ntrees, int32_t nn, const int64_t *feat, const uint8_t *cond_bin,
+                            const uint8_t *split, const float *leaf_pred, const void *x, int x_type, int32_t x_row_major, const void *edges,
+                            int32_t nedges, int64_t nobs, int32_t nfeats, const uint8_t *feattypes, int32_t apply_link, float *out,
+                            uint32_t *leaf_idx, double *ms_out) {
+    if (!feat || !cond_bin || !split || !leaf_pred || !x || !out || nobs < 0 || nn < 1) { evb_set_error("evb_predict: invalid argument"); return EVB_ERR_ARG; }
+    EVB_CHECK(model_args(loss, K, ntrees, nfeats));
+    EVB_CHECK(evb_check_device(device));
+    if (nobs == 0) return EVB_OK;
+    std::vector<const void *> src((size_t)ntrees * 4);
+    std::vector<int32_t> nodes(ntrees, nn);
+    for (int t = 0; t < ntrees; ++t) {
+        const size_t o = (size_t)t * nn;
+        src[4 * t] = feat + o; src[4 * t + 1] = cond_bin + o; src[4 * t + 2] = split + o; src[4 * t + 3] = leaf_pred + o * K;
+    }
+    evb_model m;
+    m.device = device; m.loss = loss; m.K = K;
+    int32_t rc = model_fill(&m, ntrees, src.data(), nodes.data(), edges, x_type < 0 ? EVB_F32 : x_type, nedges, nfeats, feattypes, false);
+    if (rc == EVB_OK) rc = predict_rows(m, ntrees, x, x_type, x_row_major, nobs, apply_link, out, leaf_idx, ms_out, false);
+    evb_dev_free(m.block);
+    return rc;
+}
+
+extern "C" int32_t evb_predict(int32_t device, int32_t loss, int32_t K, int32_t ntrees, int32_t nn, const int64_t *feat,
+                               const uint8_t *cond_bin, const uint8_t *split, const float *leaf_pred, const uint8_t *x_bin,
+                               int64_t nobs, int32_t nfeats, const uint8_t *feattypes, int32_t apply_link, float *out,
+                               uint32_t *leaf_idx) {
+    if (!x_bin) { evb_set_error("evb_predict: x_bin is null"); return EVB_ERR_ARG; }
+    return predict_once(device, loss, K, ntrees, nn, feat, cond_bin, split, leaf_pred, x_bin, -1, 0, nullptr, 0, nobs, nfeats, feattypes, apply_link,
+                        out, leaf_idx, nullptr);
+}
+
+extern "C" int32_t evb_predict_x(int32_t device, int32_t loss, int32_t K, int32_t ntrees, int32_t nn, const int64_t *feat,
+                                 const uint8_t *cond_bin, const uint8_t *split, const float *leaf_pred, const void *x, int32_t x_dtype,
+                                 int32_t x_row_major, const void *edges, int32_t nedges, int64_t nobs, int32_t nfeats,
+                                 const uint8_t *feattypes, int32_t apply_link, float *out, uint32_t *leaf_idx, double *kernel_ms) {
+    if (!x) { evb_set_error("evb_predict_x: x is null"); return EVB_ERR_ARG; }
+    if (!edges || nedges < 1 || nedges > 254 || (x_dtype != EVB_F32 && x_dtype != EVB_F64)) {
+        evb_set_error("evb_predict_x: edges / dtype invalid");
+        return EVB_ERR_ARG;
+    }
+    return predict_once(device, loss, K, ntrees, nn, feat, cond_bin, split, leaf_pred, x, x_dtype, x_row_major, edges, nedges, nobs, nfeats, feattypes,
+                        apply_link, out, leaf_idx, kernel_ms);
+}

@@ -1,19 +1,14 @@
 // Row-parallel kernels: layout conversion of the binned matrix, loss gradients (`update_grads!`,
 // src/loss.jl:100-128, 219-236; GPU counterparts ext/EvoTreesKernelAbstractionsExt/loss.jl:106-191), row
 // subsampling (`subsample`, src/subsample.jl:6-38), the training `predict!` (src/predict.jl:1-62) fused with
-// the gradients of the next round, inference over all trees (`_predict`, src/predict.jl:118-136) and
-// `binarize` (src/fit-utils.jl:66-72).
-#include "evb_internal.cuh"
+// the gradients of the next round and `binarize` (src/fit-utils.jl:66-72).
+#include "evb_device.cuh"
 #include <float.h>
 #include <algorithm>
 
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-
-// ---------------------------------------------------------------------------------- scalar loss math
-__device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }             // loss.jl:249-251
-__device__ __forceinline__ float softplusf_(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); } // loss.jl:257-260
 
 // Gradient record of one row.  Channel c (reference order g_1..g_K, h_1..h_K, w) lives at float
 // (c / NCH) * 4 + c % NCH: the channels of one histogram unit start on a 16-byte boundary.
@@ -110,36 +105,6 @@ __device__ __forceinline__ void grad_row(int loss, int K, int NCH, bool elided, 
             REC(2 * Y + 2 * t + 1) = 2.0f * (ds / scale) * (ds / scale) * w;
         }
     }
-}
-
-// pred[:, i] += leaf with the loss-specific clamps of predict! (src/predict.jl:1-62)
-__device__ __forceinline__ void pred_add(int loss, int K, float *p, const float *leaf) {
-    if (loss == EVB_LOGLOSS) {
-        for (int k = 0; k < K; ++k) p[k] = fminf(fmaxf(p[k] + leaf[k], -15.0f), 15.0f);
-    } else if (loss == EVB_GAUSSIAN_MLE || loss == EVB_LOGISTIC_MLE) {
-        for (int t = 0; t < K / 2; ++t) {
-            p[2 * t] += leaf[2 * t];
-            p[2 * t + 1] = fmaxf(-15.0f, p[2 * t + 1] + leaf[2 * t + 1]);
-        }
-    } else if (loss == EVB_MLOGLOSS) {
-        float m = -INFINITY;
-        for (int k = 0; k < K; ++k) { p[k] += leaf[k]; m = fmaxf(m, p[k]); }
-        for (int k = 0; k < K; ++k) p[k] = fmaxf(-15.0f, p[k] - m);
-    } else {
-        for (int k = 0; k < K; ++k) p[k] += leaf[k];
-    }
-}
-
-__device__ __forceinline__ int traverse(const uint32_t *packed, const uint8_t *xrow) {
-    int nid = 1;
-    uint32_t pk = packed[0];
-    while ((pk >> 24) & 1u) {
-        const uint32_t x = xrow[pk & 0xffffu], bin = (pk >> 16) & 0xffu;
-        const bool cond = ((pk >> 25) & 1u) ? (x <= bin) : (x == bin);
-        nid = (nid << 1) + (cond ? 0 : 1); // nid = nid << 1 + !cond (src/predict.jl:7)
-        pk = packed[nid - 1];
-    }
-    return nid;
 }
 
 // ---------------------------------------------------------------------------------- layout
@@ -586,154 +551,6 @@ __global__ void k_nidx_from_partition(const uint32_t *rows0, const uint32_t *row
     }
 }
 
-// ---------------------------------------------------------------------------------- inference
-struct PredArgs {
-    const uint8_t *xT;
-    const uint32_t *packed; // [ntrees][nn]
-    const float *leaf;      // [ntrees][nn][K]
-    float *out;             // [nobs_total x K] column-major, this chunk starts at row0
-    uint32_t *leaf_idx;     // [nobs_total x ntrees] column-major or NULL
-    long long n, row0, nobs_total;
-    int RS, K, loss, ntrees, nn, apply_link;
-};
-template <int KMAX>
-__global__ void __launch_bounds__(256) k_predict(PredArgs a) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const uint8_t *xrow = a.xT + (size_t)i * a.RS;
-    float p[KMAX];
-#pragma unroll
-    for (int k = 0; k < KMAX; ++k) p[k] = 0.0f;
-    const int K = a.K;
-    for (int t = 0; t < a.ntrees; ++t) {
-        const int nid = traverse(a.packed + (size_t)t * a.nn, xrow);
-        if (a.leaf_idx) a.leaf_idx[(size_t)t * a.nobs_total + a.row0 + i] = (uint32_t)nid;
-        pred_add(a.loss, K, p, a.leaf + ((size_t)t * a.nn + nid - 1) * K);
-    }
-    if (a.apply_link) { // apply_prediction_link! (src/predict.jl:105-116)
-        if (a.loss == EVB_LOGLOSS) { for (int k = 0; k < K; ++k) p[k] = sigmoidf_(p[k]); }
-        else if (a.loss == EVB_GAUSSIAN_MLE || a.loss == EVB_LOGISTIC_MLE) { for (int k = 1; k < K; k += 2) p[k] = softplusf_(p[k]); }
-        else if (a.loss == EVB_POISSON || a.loss == EVB_GAMMA || a.loss == EVB_TWEEDIE) { for (int k = 0; k < K; ++k) p[k] = expf(p[k]); }
-        else if (a.loss == EVB_MLOGLOSS) {
-            float s = 0.0f;
-            for (int k = 0; k < K; ++k) { p[k] = expf(p[k]); s += p[k]; }
-            for (int k = 0; k < K; ++k) p[k] /= s;
-        }
-    }
-    for (int k = 0; k < K; ++k) a.out[(size_t)k * a.nobs_total + a.row0 + i] = p[k];
-}
-
-
-// The same with everything a thread touches in shared memory: the CTA's rows of bins are staged once, word-major
-// ([word of the row][row]: thread t only ever reads column t, so its loads never conflict with its neighbours'
-// whatever features the trees test), and the packed trees + their leaf tables stream through two shared-memory buffers
-// of TB trees each: while the threads walk the trees of one buffer, `cp.async` fills the other, so a traversal step
-// costs two shared-memory loads and the trip to L2 is off the critical path.  One thread = one row; trees are applied
-// in order (the clamps of `predict!` do not commute).  `tw` = words per tree in `trees` ([nnp] packed nodes, then
-// [nnp * K] leaf values; nnp = nn rounded up to a multiple of four so that every tree starts on a 16-byte boundary).
-// Used when 2 * TB trees fit beside the rows.
-__device__ __forceinline__ int traverse_wm(const uint32_t *packed, const uint32_t *xcol, int rows) {
-    int nid = 1;
-    uint32_t pk = packed[0];
-    while ((pk >> 24) & 1u) {
-        const uint32_t f = pk & 0xffffu, bin = (pk >> 16) & 0xffu;
-        const uint32_t x = (xcol[(f >> 2) * rows] >> (8u * (f & 3u))) & 0xffu;
-        const bool cond = ((pk >> 25) & 1u) ? (x <= bin) : (x == bin);
-        nid = (nid << 1) + (cond ? 0 : 1);
-        pk = packed[nid - 1];
-    }
-    return nid;
-}
-template <int KMAX>
-__global__ void __launch_bounds__(1024) k_predict_staged(PredArgs a, const uint32_t *trees, int nnp, int rows_per_cta, int TB) {
-    extern __shared__ __align__(16) uint32_t s_pr[]; // [RS / 4][rows_per_cta] bins, then 2 x TB x tw tree words
-    const int rw = a.RS >> 2;
-    uint32_t *s_rows = s_pr;
-    const int K = a.K, tw = nnp * (1 + K);
-    uint32_t *s_trees = s_pr + (size_t)rows_per_cta * rw;
-    const long long row0 = (long long)blockIdx.x * rows_per_cta;
-    const int nr = (int)min((long long)rows_per_cta, a.n - row0);
-    auto load_block = [&](int t0, int buf) { // trees t0 .. t0 + TB - 1 -> buffer `buf`, 16 bytes per copy
-        const int nt = min(TB, a.ntrees - t0);
-        const uint4 *src = reinterpret_cast<const uint4 *>(trees + (size_t)t0 * tw);
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_trees + (size_t)buf * TB * tw);
-        for (int c = threadIdx.x; c < nt * (tw >> 2); c += blockDim.x)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)c * 16u), "l"(src + c) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    load_block(0, 0);
-    {
-        const uint4 *src = reinterpret_cast<const uint4 *>(a.xT + (size_t)row0 * a.RS);
-        const int cpr = a.RS >> 4, nchunk = nr * cpr;
-        for (int c = threadIdx.x; c < nchunk; c += blockDim.x) {
-            const uint4 v = src[c];
-            const int r = c / cpr, part = c - r * cpr;
-            uint32_t *d = s_rows + (size_t)(part * 4) * rows_per_cta + r;
-            d[0] = v.x; d[rows_per_cta] = v.y; d[2 * rows_per_cta] = v.z; d[3 * rows_per_cta] = v.w;
-        }
-    }
-    const bool act = (int)threadIdx.x < nr;
-    const long long i = row0 + threadIdx.x;
-    const uint32_t *xcol = s_rows + threadIdx.x;
-    float p[KMAX];
-#pragma unroll
-    for (int k = 0; k < KMAX; ++k) p[k] = 0.0f;
-    int buf = 0;
-    for (int t0 = 0; t0 < a.ntrees; t0 += TB, buf ^= 1) {
-        const int nt = min(TB, a.ntrees - t0);
-        if (t0 + TB < a.ntrees) load_block(t0 + TB, buf ^ 1); // the other buffer was consumed before the last barrier
-        else asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads(); // this block's trees (and, the first time, the rows) are in place for everybody
-        if (act) {
-            for (int t = 0; t < nt; ++t) {
-                const uint32_t *pk = s_trees + ((size_t)buf * TB + t) * tw;
-                const int nid = traverse_wm(pk, xcol, rows_per_cta);
-                if (a.leaf_idx) a.leaf_idx[(size_t)(t0 + t) * a.nobs_total + a.row0 + i] = (uint32_t)nid;
-                pred_add(a.loss, K, p, reinterpret_cast<const float *>(pk + nnp) + (size_t)(nid - 1) * K);
-            }
-        }
-        __syncthreads(); // everybody is done with this buffer: the next iteration refills it
-    }
-    if (!act) return;
-    if (a.apply_link) { // apply_prediction_link! (src/predict.jl:105-116)
-        if (a.loss == EVB_LOGLOSS) { for (int k = 0; k < K; ++k) p[k] = sigmoidf_(p[k]); }
-        else if (a.loss == EVB_GAUSSIAN_MLE || a.loss == EVB_LOGISTIC_MLE) { for (int k = 1; k < K; k += 2) p[k] = softplusf_(p[k]); }
-        else if (a.loss == EVB_POISSON || a.loss == EVB_GAMMA || a.loss == EVB_TWEEDIE) { for (int k = 0; k < K; ++k) p[k] = expf(p[k]); }
-        else if (a.loss == EVB_MLOGLOSS) {
-            float sm = 0.0f;
-            for (int k = 0; k < K; ++k) { p[k] = expf(p[k]); sm += p[k]; }
-            for (int k = 0; k < K; ++k) p[k] /= sm;
-        }
-    }
-    for (int k = 0; k < K; ++k) a.out[(size_t)k * a.nobs_total + a.row0 + i] = p[k];
-}
-
-// trees in the layout k_predict_staged streams: tree t = [nnp] packed nodes, then [nnp][K] leaf values (zero padded)
-__global__ void k_pack_staged(const uint32_t *packed, const float *leaf, int ntrees, int nn, int nnp, int K, uint32_t *out) {
-    const int tw = nnp * (1 + K);
-    const long long total = (long long)ntrees * tw;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-        const int t = (int)(e / tw), o = (int)(e - (long long)t * tw);
-        uint32_t v = 0u;
-        if (o < nnp) { if (o < nn) v = packed[(size_t)t * nn + o]; }
-        else { const int q = o - nnp; if (q < nn * K) v = __float_as_uint(leaf[(size_t)t * nn * K + q]); }
-        out[e] = v;
-    }
-}
-
-__global__ void k_pack_trees(const long long *feat, const uint8_t *bin, const uint8_t *split, const uint8_t *feattypes,
-                             long long total, uint32_t *packed) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    uint32_t pk = 0;
-    if (split[i]) {
-        const uint32_t f = (uint32_t)(feat[i] - 1);
-        pk = f | ((uint32_t)bin[i] << 16) | (1u << 24) | ((feattypes ? (feattypes[f] ? 1u : 0u) : 1u) << 25);
-    }
-    packed[i] = pk;
-}
-
 // ---------------------------------------------------------------------------------- binarize
 // searchsortedfirst(edges[j], x): 1 + number of edges strictly below x
 template <typename T>
@@ -750,38 +567,6 @@ __global__ void __launch_bounds__(256) k_binarize(const T *x, long long ld, long
         int lo = 0, hi = nedges;
         while (lo < hi) { const int mid = (lo + hi) >> 1; if (e[mid] < v) lo = mid + 1; else hi = mid; }
         out[(size_t)j * ldo + i] = (uint8_t)(lo + 1);
-    }
-}
-
-// binarize a block of rows of the raw matrix straight into observation-major bins xT[row][RS] (what the traversal
-// reads): 256 rows per CTA, staged through shared memory so that both the reads of x and the writes of xT coalesce
-template <typename T>
-__global__ void __launch_bounds__(256) k_binarize_rows(const T *x, long long ld, int row_major, long long n, int nfeats, const T *edges,
-                                                       int nedges, uint8_t *xT, int RS) {
-    extern __shared__ unsigned char s_tile[]; // [256][RS + 4]: one word of padding, so that the same feature of adjacent rows sits in different banks
-    const int RSP = RS + 4;
-    const long long row0 = (long long)blockIdx.x * 256;
-    const int nr = (int)min((long long)256, n - row0);
-    for (int e = threadIdx.x; e < 64 * RSP; e += 256) reinterpret_cast<uint32_t *>(s_tile)[e] = 0u;
-    __syncthreads();
-    const int total = nr * nfeats;
-    for (int e = threadIdx.x; e < total; e += 256) {
-        int r, j;
-        T v;
-        if (row_major) { r = e / nfeats; j = e - r * nfeats; v = x[(size_t)(row0 + r) * ld + j]; }
-        else { j = e / nr; r = e - j * nr; v = x[(size_t)j * ld + row0 + r]; }
-        const T *ed = edges + (size_t)j * nedges;
-        int lo = 0, hi = nedges;
-        while (lo < hi) { const int mid = (lo + hi) >> 1; if (__ldg(ed + mid) < v) lo = mid + 1; else hi = mid; }
-        s_tile[r * RSP + j] = (uint8_t)(lo + 1);
-    }
-    __syncthreads();
-    uint4 *dst = reinterpret_cast<uint4 *>(xT + (size_t)row0 * RS);
-    const int cpr = RS / 16;
-    for (int e = threadIdx.x; e < nr * cpr; e += 256) {
-        const int r = e / cpr, part = e - r * cpr;
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(s_tile + (size_t)r * RSP) + part * 4;
-        dst[e] = make_uint4(src[0], src[1], src[2], src[3]);
     }
 }
 
@@ -1098,7 +883,7 @@ int32_t evb_upload_binarize(evb_handle *h, const void *x, int32_t dtype, const v
 }
 
 // ---- stateless entry points -----------------------------------------------------------------------
-static int32_t check_device(int device) {
+int32_t evb_check_device(int device) {
     int ndev = 0;
     cudaError_t e = cudaGetDeviceCount(&ndev);
     if (e != cudaSuccess || ndev == 0) {
@@ -1117,180 +902,13 @@ struct DevBuf {
     template <typename T> T *as() { return reinterpret_cast<T *>(p); }
 };
 
-// Common body of evb_predict (binned input) and evb_predict_x (raw input + edges, binarized on the device).
-static int32_t predict_impl(int32_t device, int32_t loss, int32_t K, int32_t ntrees, int32_t nn, const int64_t *feat,
-                            const uint8_t *cond_bin, const uint8_t *split, const float *leaf_pred, const uint8_t *x_bin, const void *x,
-                            int32_t x_dtype, int32_t x_row_major, const void *edges, int32_t nedges, int64_t nobs, int32_t nfeats,
-                            const uint8_t *feattypes, int32_t apply_link, float *out, uint32_t *leaf_idx, double *ms_out) {
-    if (!feat || !cond_bin || !split || !leaf_pred || (!x_bin && !x) || !out || nobs < 0 || nfeats < 1 || nfeats > 65535 ||
-        ntrees < 0 || nn < 1 || K < 1 || K > 64 || loss < 0 || loss > EVB_LOSS_LAST) {
-        evb_set_error("evb_predict: invalid argument");
-        return EVB_ERR_ARG;
-    }
-    if (x && (!edges || nedges < 1 || nedges > 254 || (x_dtype != EVB_F32 && x_dtype != EVB_F64))) {
-        evb_set_error("evb_predict_x: edges / dtype invalid");
-        return EVB_ERR_ARG;
-    }
-    EVB_CHECK(check_device(device));
-    if (nobs == 0) return EVB_OK;
-    cudaStream_t st;
-    EVB_CUDA(cudaStreamCreate(&st));
-    const int RS = (nfeats + 31) / 32 * 32;
-    const size_t es = x_dtype == EVB_F64 ? 8 : 4;
-    const long long total = (long long)ntrees * nn;
-    const int64_t chunk = nobs < (int64_t)1 << 20 ? nobs : (int64_t)1 << 20;
-    // Blocks of `chunk` rows, two of everything: while the kernels of block k run, the host stages block k + 1 through
-    // the pinned ring (several threads) and the copy engine brings it over.
-    DevBuf d_feat, d_bin, d_split, d_ft, d_packed, d_leaf, d_in[2], d_xT[2], d_out, d_lidx, d_edges;
-    cudaEvent_t ev_free[2] = {nullptr, nullptr}, ev_k0[2] = {nullptr, nullptr}, ev_k1[2] = {nullptr, nullptr}, ev_in[2] = {nullptr, nullptr};
-    cudaStream_t cs = nullptr;
-    float kernel_ms = 0.f;
-    // traversal out of shared memory when a tree (packed nodes + leaf table) fits a block of it
-    const int nnp = (nn + 3) & ~3;
-    const size_t treebytes = (size_t)nnp * (1 + K) * 4;
-    int rows_cta = 1024;
-    while (rows_cta > 128 && (size_t)rows_cta * RS > (size_t)132 * 1024) rows_cta >>= 1;
-    const size_t rows_smem = (size_t)rows_cta * RS;
-    int TB = rows_smem < (size_t)200 * 1024 ? (int)(((size_t)200 * 1024 - rows_smem) / (2 * treebytes)) : 0;
-    if (TB > 8) TB = 8;
-    const bool staged = TB >= 1 && RS % 16 == 0 && !getenv("EVB_PREDICT_DIRECT");
-    const size_t pred_smem = rows_smem + (size_t)2 * TB * treebytes;
-    DevBuf d_staged;
-    auto body = [&]() -> int32_t {
-        EVB_CUDA(evb_stream_get(&cs));
-        for (int q = 0; q < 2; ++q) {
-            EVB_CUDA(cudaEventCreateWithFlags(&ev_free[q], cudaEventDisableTiming));
-            EVB_CUDA(cudaEventCreateWithFlags(&ev_in[q], cudaEventDisableTiming));
-            EVB_CUDA(cudaEventCreate(&ev_k0[q])); EVB_CUDA(cudaEventCreate(&ev_k1[q]));
-            EVB_CUDA(d_in[q].alloc((size_t)chunk * nfeats * (x ? es : 1))); EVB_CUDA(d_xT[q].alloc((size_t)chunk * RS));
-            EVB_CUDA(cudaMemsetAsync(d_xT[q].p, 0, (size_t)chunk * RS, st));
-        }
-        EVB_CUDA(d_feat.alloc(total * 8)); EVB_CUDA(d_bin.alloc(total)); EVB_CUDA(d_split.alloc(total));
-        EVB_CUDA(d_packed.alloc(total * 4)); EVB_CUDA(d_leaf.alloc((size_t)total * K * 4));
-        EVB_CUDA(d_out.alloc((size_t)nobs * K * 4));
-        if (leaf_idx) EVB_CUDA(d_lidx.alloc((size_t)nobs * ntrees * 4));
-        if (feattypes) { EVB_CUDA(d_ft.alloc(nfeats)); EVB_CUDA(cudaMemcpyAsync(d_ft.p, feattypes, nfeats, cudaMemcpyHostToDevice, st)); }
-        if (x) { EVB_CUDA(d_edges.alloc((size_t)nedges * nfeats * es)); EVB_CUDA(cudaMemcpyAsync(d_edges.p, edges, (size_t)nedges * nfeats * es, cudaMemcpyHostToDevice, st)); }
-        EVB_CUDA(cudaMemcpyAsync(d_feat.p, feat, total * 8, cudaMemcpyHostToDevice, st));
-        EVB_CUDA(cudaMemcpyAsync(d_bin.p, cond_bin, total, cudaMemcpyHostToDevice, st));
-        EVB_CUDA(cudaMemcpyAsync(d_split.p, split, total, cudaMemcpyHostToDevice, st));
-        EVB_CUDA(cudaMemcpyAsync(d_leaf.p, leaf_pred, (size_t)total * K * 4, cudaMemcpyHostToDevice, st));
-        if (total > 0) {
-            k_pack_trees<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d_feat.as<long long>(), d_bin.as<uint8_t>(), d_split.as<uint8_t>(),
-                                                                           feattypes ? d_ft.as<uint8_t>() : nullptr, total, d_packed.as<uint32_t>());
-            EVB_CUDA(cudaGetLastError());
-        }
-        if (staged && total > 0) {
-            EVB_CUDA(d_staged.alloc((size_t)ntrees * treebytes));
-            k_pack_staged<<<512, 256, 0, st>>>(d_packed.as<uint32_t>(), d_leaf.as<float>(), ntrees, nn, nnp, K, d_staged.as<uint32_t>());
-            EVB_CUDA(cudaGetLastError());
-        }
-        EVB_CUDA(cudaStreamSynchronize(st)); // trees, edges and the cleared row buffers are in place before the copy stream starts
-        int k = 0;
-        for (int64_t r0 = 0; r0 < nobs; r0 += chunk, ++k) {
-            const int q = k & 1;
-            const int64_t nr = nobs - r0 < chunk ? nobs - r0 : chunk;
-            if (k >= 2) { // the kernels of block k - 2 are done with these buffers
-                EVB_CUDA(cudaEventSynchronize(ev_free[q]));
-                float ms = 0.f;
-                if (cudaEventElapsedTime(&ms, ev_k0[q], ev_k1[q]) == cudaSuccess) kernel_ms += ms;
-            }
-            // rows r0 .. r0 + nr of every column (column-major input: one segment per feature), packed as [nfeats][nr]
-            // the host does not wait for the copies: the kernels do (event), and the host goes on gathering the next block
-            if (x && x_row_major) EVB_CHECK(evb_h2d_staged(d_in[q].p, (const char *)x + (size_t)r0 * nfeats * es, (size_t)nr * nfeats * es, cs, false));
-            else if (x) EVB_CHECK(evb_h2d_staged_strided(d_in[q].p, (const char *)x + (size_t)r0 * es, (size_t)nr * es, (size_t)nfeats, (size_t)nobs * es, cs, false));
-            else EVB_CHECK(evb_h2d_staged_strided(d_in[q].p, x_bin + r0, (size_t)nr, (size_t)nfeats, (size_t)nobs, cs, false));
-            EVB_CUDA(cudaEventRecord(ev_in[q], cs));
-            EVB_CUDA(cudaStreamWaitEvent(st, ev_in[q], 0));
-            EVB_CUDA(cudaEventRecord(ev_k0[q], st));
-            if (x) {
-                const unsigned blocks = (unsigned)((nr + 255) / 256);
-                const long long ld = x_row_major ? nfeats : nr;
-                if (256 * (RS + 4) > 48 * 1024) { // rows of more than 188 bins: the tile needs the opt-in shared memory
-                    EVB_CUDA(cudaFuncSetAttribute(k_binarize_rows<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * (RS + 4)));
-                    EVB_CUDA(cudaFuncSetAttribute(k_binarize_rows<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * (RS + 4)));
-                }
-                if (x_dtype == EVB_F32)
-                    k_binarize_rows<float><<<blocks, 256, 256 * (RS + 4), st>>>(d_in[q].as<float>(), ld, x_row_major, nr, nfeats, d_edges.as<float>(), nedges, d_xT[q].as<uint8_t>(), RS);
-                else
-                    k_binarize_rows<double><<<blocks, 256, 256 * (RS + 4), st>>>(d_in[q].as<double>(), ld, x_row_major, nr, nfeats, d_edges.as<double>(), nedges, d_xT[q].as<uint8_t>(), RS);
-                EVB_CUDA(cudaGetLastError());
-            } else {
-                EVB_CHECK(evb_launch_transpose(nullptr, d_in[q].as<uint8_t>(), nr, nr, 0, nfeats, d_xT[q].as<uint8_t>(), RS, st));
-            }
-            PredArgs a;
-            a.xT = d_xT[q].as<uint8_t>(); a.packed = d_packed.as<uint32_t>(); a.leaf = d_leaf.as<float>(); a.out = d_out.as<float>();
-            a.leaf_idx = leaf_idx ? d_lidx.as<uint32_t>() : nullptr; a.n = nr; a.row0 = r0; a.nobs_total = nobs; a.RS = RS; a.K = K;
-            a.loss = loss; a.ntrees = ntrees; a.nn = nn; a.apply_link = apply_link;
-            if (staged) {
-                const unsigned blocks = (unsigned)((nr + rows_cta - 1) / rows_cta);
-#define EVB_PRED_STAGED(KM) do { \
-                    EVB_CUDA(cudaFuncSetAttribute(k_predict_staged<KM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pred_smem)); \
-                    k_predict_staged<KM><<<blocks, rows_cta, pred_smem, st>>>(a, d_staged.as<uint32_t>(), nnp, rows_cta, TB); } while (0)
-                if (K <= 1) EVB_PRED_STAGED(1);
-                else if (K <= 2) EVB_PRED_STAGED(2);
-                else if (K <= 8) EVB_PRED_STAGED(8);
-                else EVB_PRED_STAGED(64);
-#undef EVB_PRED_STAGED
-            } else {
-                const unsigned blocks = (unsigned)((nr + 255) / 256);
-                if (K <= 1) k_predict<1><<<blocks, 256, 0, st>>>(a);
-                else if (K <= 2) k_predict<2><<<blocks, 256, 0, st>>>(a);
-                else if (K <= 8) k_predict<8><<<blocks, 256, 0, st>>>(a);
-                else k_predict<64><<<blocks, 256, 0, st>>>(a);
-            }
-            EVB_CUDA(cudaGetLastError());
-            EVB_CUDA(cudaEventRecord(ev_k1[q], st));
-            EVB_CUDA(cudaEventRecord(ev_free[q], st));
-        }
-        EVB_CUDA(cudaMemcpyAsync(out, d_out.p, (size_t)nobs * K * 4, cudaMemcpyDeviceToHost, st));
-        if (leaf_idx) EVB_CUDA(cudaMemcpyAsync(leaf_idx, d_lidx.p, (size_t)nobs * ntrees * 4, cudaMemcpyDeviceToHost, st));
-        EVB_CUDA(cudaStreamSynchronize(st));
-        for (int q = 0; q < 2 && q < k; ++q) { // the last (up to) two blocks have not been read yet
-            float ms = 0.f;
-            if (cudaEventElapsedTime(&ms, ev_k0[q], ev_k1[q]) == cudaSuccess) kernel_ms += ms;
-        }
-        return EVB_OK;
-    };
-    int32_t rc = body();
-    cudaStreamSynchronize(st);
-    if (cs) { cudaStreamSynchronize(cs); evb_stream_put(cs); }
-    if (ms_out) *ms_out = kernel_ms;
-    for (int q = 0; q < 2; ++q) {
-        if (ev_free[q]) cudaEventDestroy(ev_free[q]);
-        if (ev_in[q]) cudaEventDestroy(ev_in[q]);
-        if (ev_k0[q]) cudaEventDestroy(ev_k0[q]);
-        if (ev_k1[q]) cudaEventDestroy(ev_k1[q]);
-    }
-    cudaStreamDestroy(st);
-    return rc;
-}
-
-extern "C" int32_t evb_predict(int32_t device, int32_t loss, int32_t K, int32_t ntrees, int32_t nn, const int64_t *feat,
-                               const uint8_t *cond_bin, const uint8_t *split, const float *leaf_pred, const uint8_t *x_bin,
-                               int64_t nobs, int32_t nfeats, const uint8_t *feattypes, int32_t apply_link, float *out,
-                               uint32_t *leaf_idx) {
-    if (!x_bin) { evb_set_error("evb_predict: x_bin is null"); return EVB_ERR_ARG; }
-    return predict_impl(device, loss, K, ntrees, nn, feat, cond_bin, split, leaf_pred, x_bin, nullptr, 0, 0, nullptr, 0, nobs, nfeats,
-                        feattypes, apply_link, out, leaf_idx, nullptr);
-}
-
-extern "C" int32_t evb_predict_x(int32_t device, int32_t loss, int32_t K, int32_t ntrees, int32_t nn, const int64_t *feat,
-                                 const uint8_t *cond_bin, const uint8_t *split, const float *leaf_pred, const void *x, int32_t x_dtype,
-                                 int32_t x_row_major, const void *edges, int32_t nedges, int64_t nobs, int32_t nfeats,
-                                 const uint8_t *feattypes, int32_t apply_link, float *out, uint32_t *leaf_idx, double *kernel_ms) {
-    if (!x) { evb_set_error("evb_predict_x: x is null"); return EVB_ERR_ARG; }
-    return predict_impl(device, loss, K, ntrees, nn, feat, cond_bin, split, leaf_pred, nullptr, x, x_dtype, x_row_major, edges, nedges,
-                        nobs, nfeats, feattypes, apply_link, out, leaf_idx, kernel_ms);
-}
-
 extern "C" int32_t evb_binarize(int32_t device, const void *x, int32_t dtype, int64_t nobs, int32_t nfeats, const void *edges,
                                 int32_t nedges, uint8_t *x_bin) {
     if (!x || !edges || !x_bin || nobs < 0 || nfeats < 1 || nedges < 1 || nedges > 254 || (dtype != EVB_F32 && dtype != EVB_F64)) {
         evb_set_error("evb_binarize: invalid argument");
         return EVB_ERR_ARG;
     }
-    EVB_CHECK(check_device(device));
+    EVB_CHECK(evb_check_device(device));
     if (nobs == 0) return EVB_OK;
     const size_t es = dtype == EVB_F32 ? 4 : 8;
     cudaStream_t st;

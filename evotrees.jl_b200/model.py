@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass, field
+from operator import is_
 
 import numpy as np
 
@@ -21,11 +22,17 @@ class Tree:
     pred: np.ndarray      # float32 [nn, K]; row n is the reference's pred[:, n]
     split: np.ndarray     # bool [nn]
 
+    def __setattr__(self, name, value):
+        _Packed.rebinds += 1      # a tree may have been given other arrays: packed models look again
+        object.__setattr__(self, name, value)
+
     @staticmethod
     def empty(depth: int, K: int) -> "Tree":
         nn = 2 ** depth - 1
-        return Tree(np.zeros(nn, np.int64), np.zeros(nn, np.uint8), np.zeros(nn, np.float32), np.zeros(nn, np.float32),
-                    np.zeros((nn, K), np.float32), np.zeros(nn, np.uint8))
+        t = object.__new__(Tree)  # a new tree is in no packed model yet
+        t.__dict__.update(feat=np.zeros(nn, np.int64), cond_bin=np.zeros(nn, np.uint8), w=np.zeros(nn, np.float32),
+                          gain=np.zeros(nn, np.float32), pred=np.zeros((nn, K), np.float32), split=np.zeros(nn, np.uint8))
+        return t
 
     @staticmethod
     def bias(mu: np.ndarray) -> "Tree":
@@ -40,6 +47,9 @@ class EvoTree:
     K: int
     trees: list = field(default_factory=list)
     info: dict = field(default_factory=dict)
+
+    def __getstate__(self):      # copies and pickles of a model pack its trees anew
+        return {k: v for k, v in self.__dict__.items() if k != "_dev"}
 
     def __call__(self, x, ntree_limit: int | None = None, device: int = 0):
         return predict(self, x, ntree_limit=ntree_limit, device=device)
@@ -58,8 +68,72 @@ def _pack(m: EvoTree, ntree_limit: int):
     return nn, feat, cb, sp, lp
 
 
+def _tree_arrays(t: Tree):
+    return t.feat, t.cond_bin, t.split, t.pred
+
+
+class _Packed:
+    """A model's trees, packed on one device (`evb_model_create`), and the arrays they were packed from.  `current` says
+    whether the model still consists of those arrays; whether their contents are still the same is checked by
+    `evb_model_predict` itself, while the GPU works."""
+    rebinds = 0     # attribute assignments on any `Tree` so far
+
+    def __init__(self, m: EvoTree, device: int):
+        self.rebinds = _Packed.rebinds
+        self.device, self.loss, self.K = device, m.loss, m.K
+        self.trees = list(m.trees)
+        self.edges, self.feattypes = m.info["edges"], m.info["feattypes"]
+        arrays, self.shared = [], True      # shared: the library reads the model's own arrays, not copies
+        for t in self.trees:
+            for a, dt in zip(_tree_arrays(t), (np.int64, np.uint8, np.uint8, np.float32)):
+                if a.dtype != dt and not (dt is np.uint8 and a.dtype == bool) or not a.flags.c_contiguous:
+                    a, self.shared = np.ascontiguousarray(a, dt), False
+                arrays.append(a)
+        e, ft = np.asarray(self.edges), np.asarray(self.feattypes)
+        if e.dtype not in (np.float32, np.float64) or not e.flags.c_contiguous:
+            e, self.shared = np.ascontiguousarray(e, np.float64), False
+        if ft.dtype not in (bool, np.uint8) or not ft.flags.c_contiguous:
+            ft, self.shared = np.ascontiguousarray(ft, np.uint8), False
+        self.arrays = arrays
+        self.keep = (e, ft)
+        n = len(self.trees)
+        src = np.array([a.__array_interface__["data"][0] for a in arrays], np.uint64)
+        nodes = np.array([a.size for a in arrays[::4]], np.int32)
+        self.handle = C.c_void_p()
+        _lib.check(_lib.lib().evb_model_create(
+            C.byref(self.handle), C.c_int32(device), C.c_int32(_lib.LOSS_CODES[m.loss]), C.c_int32(m.K), C.c_int32(n), _lib.ptr(src), _lib.ptr(nodes),
+            _lib.ptr(e), C.c_int32(_lib.EVB_F32 if e.dtype == np.float32 else _lib.EVB_F64), C.c_int32(e.shape[1]), C.c_int32(e.shape[0]), _lib.ptr(ft)))
+        self.ptr = self.handle.value
+        self.nfeats = e.shape[0]
+
+    def current(self, m: EvoTree, device: int) -> bool:
+        if not (self.shared and self.device == device and self.loss == m.loss and self.K == m.K and self.edges is m.info["edges"] and
+                self.feattypes is m.info["feattypes"] and len(self.trees) == len(m.trees) and all(map(is_, self.trees, m.trees))):
+            return False
+        if self.rebinds != _Packed.rebinds:
+            now = _Packed.rebinds
+            if not all(map(is_, self.arrays, [a for t in m.trees for a in _tree_arrays(t)])):
+                return False
+            self.rebinds = now
+        return True
+
+    def __del__(self):
+        try:
+            _lib.lib().evb_model_destroy(self.handle)
+        except Exception:
+            pass
+
+
+def _packed(m: EvoTree, device: int, fresh: bool = False) -> _Packed:
+    c = None if fresh else m.__dict__.get("_dev")
+    if c is None or not c.current(m, device):
+        m.__dict__.pop("_dev", None)
+        c = m.__dict__["_dev"] = _Packed(m, device)
+    return c
+
+
 def _run(m: EvoTree, x, ntree_limit, device, apply_link: bool, want_leaf: bool, stats: dict | None = None):
-    """Binarize on the device and apply the trees in one call (`evb_predict_x`).  `x` may be C- or Fortran-ordered:
+    """Binarize on the device and apply the trees in one call (`evb_model_predict`).  `x` may be C- or Fortran-ordered:
     no host-side transpose is made."""
     ntrees = len(m.trees)
     ntree_limit = ntrees if ntree_limit is None else ntree_limit
@@ -68,22 +142,24 @@ def _run(m: EvoTree, x, ntree_limit, device, apply_link: bool, want_leaf: bool, 
     x = np.asarray(x)
     if x.dtype not in (np.float32, np.float64):
         x = x.astype(np.float64)
-    row_major = 1 if (x.flags.c_contiguous and not x.flags.f_contiguous) else 0
-    if not (x.flags.c_contiguous or x.flags.f_contiguous):
+    row_major = x.flags.c_contiguous      # one row, one column: either order describes it
+    if not (row_major or x.flags.f_contiguous):
         x = np.asfortranarray(x)
     nobs, nfeats = x.shape
-    edges = np.ascontiguousarray(m.info["edges"], dtype=x.dtype)   # [nfeats, nedges] C order == [nedges x nfeats] column-major
-    nn, feat, cb, sp, lp = _pack(m, ntree_limit)
-    out = np.empty((nobs, m.K), np.float32, order="F")
+    lib = _lib.lib()
+    p = _packed(m, device)
+    if nfeats != p.nfeats:
+        raise ValueError(f"x has {nfeats} columns, the model was trained on {p.nfeats}")
+    out = np.empty(nobs, np.float32) if m.K == 1 else np.empty((nobs, m.K), np.float32, order="F")
     leaf = np.empty((nobs, ntree_limit), np.uint32, order="F") if want_leaf else None
-    ft = np.ascontiguousarray(m.info["feattypes"], np.uint8)
-    kms = C.c_double(0.0)
-    _lib.check(_lib.lib().evb_predict_x(C.c_int32(device), C.c_int32(_lib.LOSS_CODES[m.loss]), C.c_int32(m.K),
-                                        C.c_int32(ntree_limit), C.c_int32(nn), _lib.ptr(feat), _lib.ptr(cb), _lib.ptr(sp),
-                                        _lib.ptr(lp), _lib.ptr(x), C.c_int32(_lib.EVB_F32 if x.dtype == np.float32 else _lib.EVB_F64),
-                                        C.c_int32(row_major), _lib.ptr(edges), C.c_int32(edges.shape[1]), C.c_int64(nobs),
-                                        C.c_int32(nfeats), _lib.ptr(ft), C.c_int32(1 if apply_link else 0), _lib.ptr(out),
-                                        _lib.ptr(leaf), C.byref(kms)))
+    kms = None if stats is None else C.c_double(0.0)
+    while True:
+        rc = lib.evb_model_predict(p.ptr, ntree_limit, x.ctypes.data, 0 if x.dtype == np.float32 else 2, row_major, nobs, apply_link,
+                                   out.ctypes.data, None if leaf is None else leaf.ctypes.data, None if kms is None else C.addressof(kms))
+        if rc != _lib.ERR_STALE:
+            break
+        p = _packed(m, device, fresh=True)
+    _lib.check(rc)
     if stats is not None:
         stats["kernel_ms"] = kms.value
     return out, leaf
@@ -107,7 +183,7 @@ def predict(m: EvoTree, x, ntree_limit: int | None = None, device: int = 0, stat
     """`predict(m, data; ntree_limit, device=:gpu)` (src/predict.jl:93-96): sums the trees and applies the
     loss's inverse link.  Returns [nobs] when K == 1, else [nobs, K]."""
     out, _ = _run(m, x, ntree_limit, device, True, False, stats)
-    return out[:, 0].copy() if m.K == 1 else out
+    return out
 
 
 def predict_leaf_idx(m: EvoTree, x, ntree_limit: int | None = None, device: int = 0) -> np.ndarray:

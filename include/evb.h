@@ -41,7 +41,8 @@ enum evb_status {
     EVB_ERR_EMPTY = -4,    /* row subsample selected no row (src/subsample.jl:36) */
     EVB_ERR_DEVICE = -5,   /* a kernel reported a failed self-check / bounded wait */
     EVB_ERR_BUSY = -6,     /* handle used concurrently                           */
-    EVB_ERR_LIMIT = -7     /* size beyond a documented limit                     */
+    EVB_ERR_LIMIT = -7,    /* size beyond a documented limit                     */
+    EVB_ERR_STALE = -8     /* evb_model_predict: the trees changed since evb_model_create */
 };
 
 /* 0..3: the losses of the reference's GPU benchmark configurations; 4..7: the other gradient-regression and two-parameter
@@ -265,6 +266,25 @@ EVB_API int32_t evb_predict_x(int32_t device, int32_t loss, int32_t K, int32_t n
                               const uint8_t *cond_bin, const uint8_t *split, const float *leaf_pred, const void *x, int32_t x_dtype,
                               int32_t x_row_major, const void *edges, int32_t nedges, int64_t nobs, int32_t nfeats,
                               const uint8_t *feattypes, int32_t apply_link, float *out, uint32_t *leaf_idx, double *kernel_ms);
+
+/*
+ * A fitted model whose packed trees stay on the device, for programs that predict more than once with it (the reference
+ * uploads every tree in every call, ext/EvoTreesKernelAbstractionsExt/predict.jl:119-131).  evb_model_create packs the
+ * trees; evb_model_predict is evb_predict_x with them.  The host arrays the model was made from must stay allocated: every
+ * call compares them with what was packed (while the GPU works) and returns EVB_ERR_STALE, outputs undefined, when one has
+ * changed -- create the model again then.  A model may be used by several threads at once.
+ *   src     [ntrees][4] host pointers per tree: feat int64, cond_bin uint8, split uint8, leaf_pred float [K x nodes]
+ *   nodes   [ntrees] nodes of every tree
+ *   edges   host [nedges x nfeats] column-major, EVB_F32 / EVB_F64; converted when x has the other type
+ *   ntrees  of evb_model_predict: the first ntrees trees are applied
+ */
+typedef struct evb_model evb_model;
+EVB_API int32_t evb_model_create(evb_model **out, int32_t device, int32_t loss, int32_t K, int32_t ntrees, const void *const *src,
+                                 const int32_t *nodes, const void *edges, int32_t edges_dtype, int32_t nedges, int32_t nfeats,
+                                 const uint8_t *feattypes);
+EVB_API int32_t evb_model_predict(const evb_model *m, int32_t ntrees, const void *x, int32_t x_dtype, int32_t x_row_major, int64_t nobs,
+                                  int32_t apply_link, float *out, uint32_t *leaf_idx, double *kernel_ms);
+EVB_API void evb_model_destroy(evb_model *m);
 
 /*
  * evb_binarize -- `binarize(X; edges)` (src/fit-utils.jl:66-72) on the device: x_bin[i,j] =

@@ -1,0 +1,82 @@
+"""`m(x)` at the sizes where the choice of the inference kernel changes (one CTA per row, 32 rows per CTA, staged trees, rows
+wider than shared memory) and where chunks of rows end, against a walk over the trees in numpy; and a packed model after its
+trees have changed."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(pkg, nfeats, depth, ntrees, K, nbins, loss, seed):
+    rng = np.random.default_rng(seed)
+    edges = np.sort(rng.normal(size=(nfeats, nbins - 1)), axis=1)
+    trees = [pkg.Tree.bias(rng.normal(size=K).astype(np.float32))]
+    for _ in range(ntrees - 1):
+        t = pkg.Tree.empty(depth, K)
+        nn = t.feat.size
+        t.split[: nn // 2] = rng.random(nn // 2) < 0.9
+        t.feat[:] = np.where(t.split, rng.integers(1, nfeats + 1, nn), 0)
+        t.cond_bin[:] = np.where(t.split, rng.integers(1, nbins, nn), 0)
+        t.pred[:] = 0.1 * rng.normal(size=(nn, K))
+        trees.append(t)
+    return pkg.EvoTree(loss, K, trees, {"edges": edges, "feattypes": np.ones(nfeats, bool)})
+
+
+def _walk(m, x):
+    edges = m.info["edges"].astype(x.dtype)
+    xb = np.stack([1 + np.searchsorted(edges[j], x[:, j], side="left") for j in range(x.shape[1])], axis=1)
+    p = np.zeros((x.shape[0], m.K), np.float32)
+    leaves = np.empty((x.shape[0], len(m.trees)), np.uint32)
+    r = np.arange(x.shape[0])
+    for i, t in enumerate(m.trees):
+        n = np.ones(x.shape[0], np.int64)
+        while True:
+            s = t.split[n - 1] != 0
+            if not s.any():
+                break
+            go = xb[r, np.maximum(t.feat[n - 1] - 1, 0)] <= t.cond_bin[n - 1]
+            n = np.where(s, 2 * n + (~go), n)
+        leaves[:, i] = n
+        p += t.pred[n - 1]
+        if m.loss == "mlogloss":
+            p = np.maximum(np.float32(-15), p - p.max(axis=1, keepdims=True))
+    if m.loss == "mlogloss":
+        p = np.exp(p)
+        p /= p.sum(axis=1, keepdims=True)
+    return p, leaves
+
+
+@pytest.mark.parametrize("rows,nfeats,depth,ntrees,K,nbins", [
+    (1, 1, 1, 1, 1, 2), (1, 10, 6, 300, 1, 32), (592, 7, 5, 20, 3, 255), (593, 7, 5, 20, 3, 255), (5_001, 130, 8, 61, 1, 64), (4_097, 30, 4, 90, 64, 33),
+    (33, 1_601, 3, 9, 2, 16), (65_537, 5, 9, 12, 1, 64), (70_001, 12, 11, 5, 2, 64), (300, 60_000, 3, 3, 1, 8)])
+@pytest.mark.parametrize("order,dtype", [("C", np.float32), ("F", np.float64)])
+def test_predict_at_the_edges_of_the_kernel_choice(pkg, rows, nfeats, depth, ntrees, K, nbins, order, dtype):
+    m = _model(pkg, nfeats, depth, ntrees, K, nbins, "mlogloss" if K > 2 else "mse", rows)
+    x = np.asarray(np.random.default_rng(rows).normal(size=(rows, nfeats)), dtype=dtype, order=order)
+    want, leaves = _walk(m, x)
+    np.testing.assert_allclose(pkg.predict(m, x).reshape(want.shape), want, rtol=1e-5, atol=1e-6)
+    assert np.array_equal(pkg.predict_leaf_idx(m, x), leaves)
+
+
+def test_packed_model_notices_changes(pkg):
+    """A tree changed in place, replaced, appended, or given another array: the next call uses the new one."""
+    import copy
+    m = _model(pkg, 6, 5, 8, 1, 16, "mse", 3)
+    x = np.random.default_rng(0).normal(size=(100, 6))
+
+    def check():
+        for _ in range(2):
+            np.testing.assert_allclose(pkg.predict(m, x), _walk(m, x)[0][:, 0], rtol=1e-5, atol=1e-6)
+    check()
+    m.trees[3].pred[5:, 0] += 1.0
+    check()
+    m.trees[2].pred = m.trees[2].pred * 2
+    check()
+    m.trees.append(m.trees[1])
+    check()
+    m.trees[4] = m.trees[5]
+    check()
+    m.info["edges"][2] += 0.25
+    check()
+    m2 = copy.deepcopy(m)
+    np.testing.assert_array_equal(pkg.predict(m2, x), pkg.predict(m, x))
