@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libevotrees_b200.so")
 
 EVB_F32, EVB_U32, EVB_F64 = 0, 1, 2
-ERR_STALE = -8
+ERR_LIMIT, ERR_STALE = -7, -8
 LOSS_CODES = {"mse": 0, "logloss": 1, "mlogloss": 2, "gaussian_mle": 3, "poisson": 4, "gamma": 5, "tweedie": 6, "logistic_mle": 7,
               "mae": 8, "cred_var": 9, "cred_std": 10, "quantile": 11, "multiquantile": 12}
 METRIC_CODES = {"mse": 0, "rmse": 0, "mae": 1, "logloss": 2, "mlogloss": 3, "gaussian_mle": 4, "poisson": 5, "gamma": 6, "tweedie": 7,
@@ -24,7 +24,8 @@ NTIMERS = 12
 TIMER_NAMES = ["grads", "rows_init", "hist", "hist_reduce", "allreduce", "scan", "partition", "plan", "finalize",
                "d2h", "h2d", "tree_total"]
 
-EXPORTS = ["evb_last_error", "evb_version", "evb_create", "evb_create_x", "evb_destroy", "evb_comm_unique_id", "evb_comm_init", "evb_comm_ipc_export", "evb_comm_ipc_import",
+EXPORTS = ["evb_last_error", "evb_version", "evb_create", "evb_create_x", "evb_create_m", "evb_matrix_create", "evb_matrix_edges", "evb_matrix_destroy",
+           "evb_eval_attach_m", "evb_host_range", "evb_host_count", "evb_host_codes", "evb_host_std", "evb_destroy", "evb_comm_unique_id", "evb_comm_init", "evb_comm_ipc_export", "evb_comm_ipc_import",
            "evb_grow_tree", "evb_grow_tree_begin", "evb_grow_tree_end", "evb_eval_attach", "evb_eval_sums", "evb_eval_get_pred", "evb_eval_detach", "evb_test_peer_timeout", "evb_set_timing", "evb_get_pred", "evb_get_grads", "evb_get_nidx", "evb_get_hist", "evb_get_node_sums",
            "evb_get_stream", "evb_get_timings", "evb_reset_timings", "evb_predict", "evb_predict_x", "evb_model_create", "evb_model_predict", "evb_model_destroy", "evb_binarize", "evb_hist_rows", "evb_hist_rows_noalloc", "evb_trim_cache"]
 
@@ -60,10 +61,10 @@ def lib() -> C.CDLL:
         _lib = C.CDLL(LIB_PATH)
         _lib.evb_last_error.restype = C.c_char_p
         for name in EXPORTS:
-            if name not in ("evb_last_error", "evb_destroy", "evb_model_destroy"):
+            if name not in ("evb_last_error", "evb_destroy", "evb_model_destroy", "evb_matrix_destroy"):
                 getattr(_lib, name).restype = C.c_int32
-        _lib.evb_destroy.restype = _lib.evb_model_destroy.restype = None
-        _lib.evb_model_destroy.argtypes = [C.c_void_p]
+        _lib.evb_destroy.restype = _lib.evb_model_destroy.restype = _lib.evb_matrix_destroy.restype = None
+        _lib.evb_model_destroy.argtypes = _lib.evb_matrix_destroy.argtypes = [C.c_void_p]
         # declared: plain integers are then passed without a wrapper object per argument (a call with one row takes ~20 us)
         _lib.evb_model_predict.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int32, C.c_int64, C.c_int32, C.c_void_p,
                                            C.c_void_p, C.c_void_p]

@@ -23,6 +23,14 @@ def _edge_threads() -> int:
     return max(1, min(16, n))
 
 
+def _quantile_ranks(nbins: int, ns: int):
+    """1-based rank of the lower order statistic and weight of the upper one of the quantiles (1:nbins-1)/nbins."""
+    p = np.arange(1, nbins, dtype=np.float64) / nbins
+    aleph = ns * p + (1.0 - p)
+    j = np.clip(np.trunc(aleph).astype(np.int64), 1, max(ns - 1, 1))
+    return j, np.clip(aleph - j, 0.0, 1.0)
+
+
 def get_edges(x: np.ndarray, nbins: int, rng: np.random.Generator):
     """Returns (edges [nfeats, nbins-1] of x.dtype, featbins uint8 [nfeats], feattypes bool [nfeats]).
 
@@ -31,10 +39,7 @@ def get_edges(x: np.ndarray, nbins: int, rng: np.random.Generator):
     nobs, nfeats = x.shape
     ns = min(nobs, 1000 * nbins)
     idx = np.sort(rng.choice(nobs, size=ns, replace=False)) if ns < nobs else slice(None)
-    p = np.arange(1, nbins, dtype=np.float64) / nbins
-    aleph = ns * p + (1.0 - p)
-    j = np.clip(np.trunc(aleph).astype(np.int64), 1, max(ns - 1, 1))
-    g = np.clip(aleph - j, 0.0, 1.0)
+    j, g = _quantile_ranks(nbins, ns)
     rtol = np.sqrt(np.finfo(x.dtype).eps)
     edges = np.empty((nfeats, nbins - 1), dtype=x.dtype)
 
@@ -61,6 +66,49 @@ def get_edges(x: np.ndarray, nbins: int, rng: np.random.Generator):
     featbins = np.full(nfeats, nbins, dtype=np.uint8)
     feattypes = np.ones(nfeats, dtype=bool)
     return edges, featbins, feattypes
+
+
+def sample_rows(nobs: int, nbins: int, rng: np.random.Generator):
+    """The rows `get_edges` takes from `rng`, in no particular order (quantiles do not ask for one); None = all."""
+    ns = min(nobs, 1000 * nbins)
+    return rng.choice(nobs, size=ns, replace=False, shuffle=False).astype(np.uint32) if ns < nobs else None
+
+
+class RawMatrix:
+    """A raw feature matrix on the device (`evb_matrix_create`): edges and bins of a fit are computed from it there.
+    C- and Fortran-ordered arrays are uploaded as they are."""
+
+    def __init__(self, x: np.ndarray, device: int = 0):
+        self.handle = C.c_void_p()
+        self.shape, self.dtype = x.shape, x.dtype
+        row_major = x.flags.c_contiguous
+        if not (row_major or x.flags.f_contiguous):
+            x = np.asfortranarray(x)
+        _lib.check(_lib.lib().evb_matrix_create(C.byref(self.handle), C.c_int32(device), C.c_int64(x.shape[0]), C.c_int32(x.shape[1]), _lib.ptr(x),
+                                                C.c_int32(_lib.EVB_F32 if x.dtype == np.float32 else _lib.EVB_F64), C.c_int32(int(row_major))))
+
+    def edges(self, nbins: int, rows) -> np.ndarray:
+        """What `get_edges` returns for the sampled rows: [nfeats, nbins - 1] of the matrix's type."""
+        ns = self.shape[0] if rows is None else rows.size
+        j, g = _quantile_ranks(nbins, ns)
+        lo, hi = (j - 1).astype(np.int32), np.minimum(j, ns - 1).astype(np.int32)
+        if nbins == 2:          # a single edge is the sample minimum (src/fit-utils.jl:17-19)
+            lo[:] = hi[:] = 0
+        out = np.empty((self.shape[1], nbins - 1), self.dtype)
+        _lib.check(_lib.lib().evb_matrix_edges(self.handle, _lib.ptr(rows), C.c_int32(ns), C.c_int32(nbins - 1), _lib.ptr(lo), _lib.ptr(hi), _lib.ptr(g),
+                                               C.c_double(np.sqrt(np.finfo(self.dtype).eps)), _lib.ptr(out)))
+        return out
+
+    def close(self):
+        if self.handle:
+            _lib.lib().evb_matrix_destroy(self.handle)
+            self.handle = C.c_void_p()
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *_):
+        self.close()
 
 
 def binarize(x: np.ndarray, edges: np.ndarray, device: int = 0) -> np.ndarray:

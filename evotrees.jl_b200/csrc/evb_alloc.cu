@@ -80,6 +80,12 @@ cudaError_t evb_dev_alloc(void **p, size_t bytes) {
     return cudaSuccess;
 }
 
+size_t evb_cached_bytes(int dev) {
+    if (dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lock(g_cache[dev].mu);
+    return g_cache[dev].cached_bytes;
+}
+
 // `really`: hand the block back to the driver (blocks that other processes may have mapped through CUDA IPC)
 void evb_dev_free(void *p, bool really) {
     if (!p) return;

@@ -153,7 +153,7 @@ static void free_handle(evb_handle *h) {
     void *ptrs[] = {h->xH, h->xE, h->hsum_q, h->hcnt_q, h->qs_cnt, h->qs_prefix, h->qs_rank, h->qs_gamma, h->gradq, h->d_gmax, h->d_qinv, h->xT, h->xC, h->grad, h->pred, h->y, h->nidx, h->rows[0], h->rows[1], h->mask_d, h->feattypes_d, h->mono_d,
                     h->js_d, h->seg_start, h->seg_cnt, h->gcnt, h->nleft, (h->gnleft != h->nleft) ? h->gnleft : nullptr, h->kind,
                     h->bslot, h->nsum, h->plan /* base of the tree block */, h->cum, h->slot_node, h->item_node, h->item_left,
-                    h->item_lprefix, h->item_bits, h->scan_tmp, h->hist, h->hcomp, h->scratch, h->fbest_gain, h->fbest_bin, h->obl_gain, h->obl_best};
+                    h->item_lprefix, h->item_bits, h->scan_tmp, h->hist, h->hcomp, h->scratch, h->fbest_gain, h->fbest_bin, h->obl_gain, h->obl_best, h->edges_d};
     phase("exchange buffers");
     for (void *p : ptrs) evb_dev_free(p);
     phase("device buffers");
@@ -173,9 +173,9 @@ static void free_handle(evb_handle *h) {
 
 extern "C" void evb_destroy(evb_handle *h) { free_handle(h); }
 
-// x_bin != NULL: the binned matrix; else the raw matrix x (x_dtype) with its edges, binarized on the device
-static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int32_t nfeats, const uint8_t *x_bin, const void *x,
-                           int32_t x_dtype, const void *edges, int32_t nedges, const void *y,
+// x_bin: the binned matrix; mx: the raw matrix on the device; else the raw matrix x on the host (x_dtype), with its edges
+static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int32_t nfeats, const uint8_t *x_bin, const evb_matrix *mx,
+                           const void *x, int32_t x_dtype, const void *edges, int32_t nedges, const void *y,
                            int32_t y_dtype, int32_t ycols, const float *w, const float *pred0, const float *mu,
                            const uint8_t *feattypes, const int32_t *monotone) {
     // EVB_INIT_TRACE=1: host-side milliseconds of the phases of evb_create / evb_create_x on stderr
@@ -298,14 +298,7 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     // ---- uploads: x_bin is kept feature-major (as given) for the row partition and transposed on the device to
     // observation-major rows for the histogram gathers and the tree traversal
     phase("allocations");
-    EVB_CUDA(cudaMemsetAsync(h->xT, 0, (size_t)n * h->RS, h->st));
     EVB_CUDA(dalloc(&h->xC, (size_t)n * nfeats));
-    phase("xC alloc + xT memset");
-    if (x_bin) EVB_CHECK(evb_h2d_staged(h->xC, x_bin, (size_t)n * nfeats, h->st));
-    else EVB_CHECK(evb_upload_binarize(h, x, x_dtype, edges, nedges));
-    phase("upload (+ binarize)");
-    EVB_CHECK(evb_launch_transpose(h, h->xC, n, n, 0, nfeats, h->xT, h->RS, h->st));
-    phase("transpose to xT");
     if (h->use_q2) {
         const size_t acc = (size_t)h->maxslots * h->B * h->q2.SC;
         EVB_CUDA(dalloc(&h->xH, (size_t)(n + 1) * h->q2.RSH));
@@ -314,16 +307,35 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
         EVB_CUDA(dalloc(&h->hcnt_q, acc));
         EVB_CUDA(cudaMemsetAsync(h->hsum_q, 0, acc * sizeof(unsigned long long), h->st));
         EVB_CUDA(cudaMemsetAsync(h->hcnt_q, 0, acc * sizeof(uint32_t), h->st));
-        EVB_CHECK(evb_q2_build_layout(h));
+    }
+    phase("layouts");
+    if (mx) {
+        const size_t eb = (size_t)nedges * nfeats * (x_dtype == EVB_F64 ? 8 : 4);
+        unsigned char *e = nullptr;
+        EVB_CUDA(dalloc(&e, eb));
+        h->edges_d = e; h->edges_dtype = x_dtype; h->nedges = nedges;
+        EVB_CUDA(cudaMemcpyAsync(e, edges, eb, cudaMemcpyHostToDevice, h->st));
+        if (h->use_q2) EVB_CHECK(evb_q2_clear_layout(h));
+        EVB_CUDA(evb_matrix_join(mx, h->st));
+        EVB_CHECK(evb_matrix_binarize(mx, e, nedges, h->xC, h->xT, h->RS, h->xH, h->use_q2 ? h->q2.RSH : 0, h->xE, h->use_q2 ? h->q2.nmain : nfeats, h->d_err, h->st));
+        phase("binarize");
+    } else {
+        EVB_CUDA(cudaMemsetAsync(h->xT, 0, (size_t)n * h->RS, h->st));
+        if (x_bin) EVB_CHECK(evb_h2d_staged(h->xC, x_bin, (size_t)n * nfeats, h->st));
+        else EVB_CHECK(evb_upload_binarize(h, x, x_dtype, edges, nedges));
+        phase("upload (+ binarize)");
+        EVB_CHECK(evb_launch_transpose(h, h->xC, n, n, 0, nfeats, h->xT, h->RS, h->st));
+        phase("transpose to xT");
+        if (h->use_q2) EVB_CHECK(evb_q2_build_layout(h));
         phase("chunk rows (xH, xE)");
     }
     {
         const size_t ybytes = (size_t)n * (y_dtype == EVB_U32 ? 4 : 4 * (size_t)ycols);
         EVB_CUDA(evb_dev_alloc(&h->y, ybytes ? ybytes : 1));
-        EVB_CUDA(cudaMemcpyAsync(h->y, y, ybytes, cudaMemcpyHostToDevice, h->st));
+        EVB_CHECK(evb_h2d_staged(h->y, y, ybytes, h->st, false));
         float *w_d = nullptr, *p0_d = nullptr, *mu_d = nullptr;
-        if (w) { EVB_CUDA(dalloc(&w_d, (size_t)n)); EVB_CUDA(cudaMemcpyAsync(w_d, w, sizeof(float) * n, cudaMemcpyHostToDevice, h->st)); }
-        if (pred0) { EVB_CUDA(dalloc(&p0_d, (size_t)n * K)); EVB_CUDA(cudaMemcpyAsync(p0_d, pred0, sizeof(float) * n * K, cudaMemcpyHostToDevice, h->st)); }
+        if (w) { EVB_CUDA(dalloc(&w_d, (size_t)n)); EVB_CHECK(evb_h2d_staged(w_d, w, sizeof(float) * n, h->st, false)); }
+        if (pred0) { EVB_CUDA(dalloc(&p0_d, (size_t)n * K)); EVB_CHECK(evb_h2d_staged(p0_d, pred0, sizeof(float) * n * K, h->st, false)); }
         else { EVB_CUDA(dalloc(&mu_d, (size_t)K)); EVB_CUDA(cudaMemcpyAsync(mu_d, mu, sizeof(float) * K, cudaMemcpyHostToDevice, h->st)); }
         int32_t rc = evb_launch_init_state(h, w_d, p0_d, mu_d);
         cudaStreamSynchronize(h->st);
@@ -358,13 +370,13 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     return EVB_OK;
 }
 
-static int32_t create_common(evb_handle **out, const evb_params *p, int64_t nobs, int32_t nfeats, const uint8_t *x_bin, const void *x,
-                             int32_t x_dtype, const void *edges, int32_t nedges, const void *y, int32_t y_dtype, int32_t ycols,
+static int32_t create_common(evb_handle **out, const evb_params *p, int64_t nobs, int32_t nfeats, const uint8_t *x_bin, const evb_matrix *mx,
+                             const void *x, int32_t x_dtype, const void *edges, int32_t nedges, const void *y, int32_t y_dtype, int32_t ycols,
                              const float *w, const float *pred0, const float *mu, const uint8_t *feattypes, const int32_t *monotone) {
     if (!out) { evb_set_error("evb_create: out is null"); return EVB_ERR_ARG; }
     *out = nullptr;
-    if (!p || (!x_bin && !x) || !y || (!pred0 && !mu)) { evb_set_error("evb_create: null argument"); return EVB_ERR_ARG; }
-    if (x && (!edges || (x_dtype != EVB_F32 && x_dtype != EVB_F64) || nedges != p->nbins - 1)) {
+    if (!p || (!x_bin && !mx && !x) || !y || (!pred0 && !mu)) { evb_set_error("evb_create: null argument"); return EVB_ERR_ARG; }
+    if (!x_bin && (!edges || (x_dtype != EVB_F32 && x_dtype != EVB_F64) || nedges != p->nbins - 1)) {
         evb_set_error("evb_create_x: x needs EVB_F32 / EVB_F64 and nbins - 1 edges per feature");
         return EVB_ERR_ARG;
     }
@@ -406,7 +418,7 @@ static int32_t create_common(evb_handle **out, const evb_params *p, int64_t nobs
     if (!h) { evb_set_error("out of host memory"); return EVB_ERR_ARG; }
     memset(&h->tm, 0, sizeof(h->tm));
     { const char *e = getenv("EVB_TEST_FAIL_ALLOC"); g_alloc_countdown = e ? atoi(e) : 0; }
-    int32_t rc = create_impl(h, p, nobs, nfeats, x_bin, x, x_dtype, edges, nedges, y, y_dtype, ycols, w, pred0, mu, feattypes, monotone);
+    int32_t rc = create_impl(h, p, nobs, nfeats, x_bin, mx, x, x_dtype, edges, nedges, y, y_dtype, ycols, w, pred0, mu, feattypes, monotone);
     g_alloc_countdown = 0;
     if (rc != EVB_OK) { free_handle(h); return rc; }
     *out = h;
@@ -417,14 +429,22 @@ extern "C" int32_t evb_create(evb_handle **out, const evb_params *p, int64_t nob
                               const void *y, int32_t y_dtype, int32_t ycols, const float *w, const float *pred0, const float *mu,
                               const uint8_t *feattypes, const int32_t *monotone) {
     if (!x_bin) { evb_set_error("evb_create: x_bin is null"); return EVB_ERR_ARG; }
-    return create_common(out, p, nobs, nfeats, x_bin, nullptr, 0, nullptr, 0, y, y_dtype, ycols, w, pred0, mu, feattypes, monotone);
+    return create_common(out, p, nobs, nfeats, x_bin, nullptr, nullptr, 0, nullptr, 0, y, y_dtype, ycols, w, pred0, mu, feattypes, monotone);
 }
 
 extern "C" int32_t evb_create_x(evb_handle **out, const evb_params *p, int64_t nobs, int32_t nfeats, const void *x, int32_t x_dtype,
                                 const void *edges, int32_t nedges, const void *y, int32_t y_dtype, int32_t ycols, const float *w,
                                 const float *pred0, const float *mu, const uint8_t *feattypes, const int32_t *monotone) {
     if (!x) { evb_set_error("evb_create_x: x is null"); return EVB_ERR_ARG; }
-    return create_common(out, p, nobs, nfeats, nullptr, x, x_dtype, edges, nedges, y, y_dtype, ycols, w, pred0, mu, feattypes, monotone);
+    return create_common(out, p, nobs, nfeats, nullptr, nullptr, x, x_dtype, edges, nedges, y, y_dtype, ycols, w, pred0, mu, feattypes, monotone);
+}
+
+extern "C" int32_t evb_create_m(evb_handle **out, const evb_params *p, const evb_matrix *m, const void *edges, int32_t nedges, const void *y,
+                                int32_t y_dtype, int32_t ycols, const float *w, const float *pred0, const float *mu, const uint8_t *feattypes,
+                                const int32_t *monotone) {
+    if (!m) { evb_set_error("evb_create_m: matrix is null"); return EVB_ERR_ARG; }
+    return create_common(out, p, evb_matrix_rows(m), evb_matrix_feats(m), nullptr, m, nullptr, evb_matrix_dtype(m), edges, nedges, y, y_dtype, ycols, w, pred0, mu,
+                         feattypes, monotone);
 }
 
 extern "C" int32_t evb_comm_unique_id(uint8_t id[128]) {
@@ -640,7 +660,7 @@ extern "C" int32_t evb_grow_tree(evb_handle *h, const uint8_t *row_mask, uint8_t
 }
 
 // ---- evaluation data on the device ---------------------------------------------------------------------------
-static int32_t eval_attach_impl(evb_handle *h, int64_t nobs, const uint8_t *x_bin, const void *y, const float *w, const float *pred0,
+static int32_t eval_attach_impl(evb_handle *h, int64_t nobs, const uint8_t *x_bin, const evb_matrix *mx, const void *y, const float *w, const float *pred0,
                                 const float *bias, int32_t metric, double sums[2]) {
     const int K = h->K;
     h->ev_metric = metric;
@@ -650,24 +670,29 @@ static int32_t eval_attach_impl(evb_handle *h, int64_t nobs, const uint8_t *x_bi
     EVB_CUDA(dalloc(&h->ev_part, (size_t)h->ev_blocks * 2));
     const size_t ybytes = (size_t)nobs * (h->y_dtype == EVB_U32 ? 4 : 4 * (size_t)h->ycols);
     EVB_CUDA(evb_dev_alloc(&h->ev_y, ybytes));
-    EVB_CUDA(cudaMemcpyAsync(h->ev_y, y, ybytes, cudaMemcpyHostToDevice, h->st));
+    EVB_CHECK(evb_h2d_staged(h->ev_y, y, ybytes, h->st, false));
     if (w) {
         EVB_CUDA(dalloc(&h->ev_w, (size_t)nobs));
         EVB_CUDA(cudaMemcpyAsync(h->ev_w, w, sizeof(float) * nobs, cudaMemcpyHostToDevice, h->st));
     }
     if (pred0) EVB_CUDA(cudaMemcpyAsync(h->ev_pred, pred0, sizeof(float) * nobs * K, cudaMemcpyHostToDevice, h->st));
     else EVB_CUDA(cudaMemsetAsync(h->ev_pred, 0, sizeof(float) * nobs * K, h->st));
-    // feature-major upload -> observation-major rows, column block by column block through a bounded staging buffer
-    EVB_CUDA(cudaMemsetAsync(h->ev_xT, 0, (size_t)nobs * h->RS, h->st));
     uint8_t *stage = nullptr;
     float *leaf_d = nullptr;
-    const int jb = (int)std::max<int64_t>(1, std::min<int64_t>(h->nfeats, ((int64_t)256 << 20) / nobs));
-    EVB_CUDA(dalloc(&stage, (size_t)jb * nobs));
     int32_t rc = EVB_OK;
-    for (int j0 = 0; j0 < h->nfeats && rc == EVB_OK; j0 += jb) {
-        const int nj = std::min(jb, h->nfeats - j0);
-        if (cudaMemcpyAsync(stage, x_bin + (size_t)j0 * nobs, (size_t)nj * nobs, cudaMemcpyHostToDevice, h->st) != cudaSuccess) rc = EVB_ERR_CUDA;
-        if (rc == EVB_OK) rc = evb_launch_transpose(h, stage, nobs, nobs, j0, nj, h->ev_xT, h->RS, h->st);
+    if (mx) {
+        EVB_CUDA(evb_matrix_join(mx, h->st));
+        rc = evb_matrix_binarize(mx, h->edges_d, h->nedges, nullptr, h->ev_xT, h->RS, nullptr, 0, nullptr, h->nfeats, nullptr, h->st);
+    } else {
+        // feature-major upload -> observation-major rows, column block by column block through a bounded staging buffer
+        EVB_CUDA(cudaMemsetAsync(h->ev_xT, 0, (size_t)nobs * h->RS, h->st));
+        const int jb = (int)std::max<int64_t>(1, std::min<int64_t>(h->nfeats, ((int64_t)256 << 20) / nobs));
+        EVB_CUDA(dalloc(&stage, (size_t)jb * nobs));
+        for (int j0 = 0; j0 < h->nfeats && rc == EVB_OK; j0 += jb) {
+            const int nj = std::min(jb, h->nfeats - j0);
+            if (cudaMemcpyAsync(stage, x_bin + (size_t)j0 * nobs, (size_t)nj * nobs, cudaMemcpyHostToDevice, h->st) != cudaSuccess) rc = EVB_ERR_CUDA;
+            if (rc == EVB_OK) rc = evb_launch_transpose(h, stage, nobs, nobs, j0, nj, h->ev_xT, h->RS, h->st);
+        }
     }
     h->ev_n = nobs;
     if (rc == EVB_OK) {
@@ -690,10 +715,10 @@ static int32_t eval_attach_impl(evb_handle *h, int64_t nobs, const uint8_t *x_bi
     return EVB_OK;
 }
 
-extern "C" int32_t evb_eval_attach(evb_handle *h, int64_t nobs, const uint8_t *x_bin, const void *y, const float *w, const float *pred0,
-                                   const float *bias, int32_t metric, double sums[2]) {
+static int32_t eval_attach(evb_handle *h, int64_t nobs, const uint8_t *x_bin, const evb_matrix *mx, const void *y, const float *w, const float *pred0,
+                           const float *bias, int32_t metric, double sums[2]) {
     EVB_ENTER(h);
-    if (!x_bin || !y || !sums || nobs < 1 || nobs > 2000000000ll) { evb_set_error("evb_eval_attach: invalid argument"); return EVB_ERR_ARG; }
+    if ((!x_bin && !mx) || !y || !sums || nobs < 1 || nobs > 2000000000ll) { evb_set_error("evb_eval_attach: invalid argument"); return EVB_ERR_ARG; }
     if (h->pending > 0) { evb_set_error("evb_eval_attach: a tree is still in flight"); return EVB_ERR_BUSY; }
     if (h->ev_n > 0) { evb_set_error("evb_eval_attach: evaluation data already attached (evb_eval_detach first)"); return EVB_ERR_ARG; }
     const int loss = h->p.loss;
@@ -704,9 +729,23 @@ extern "C" int32_t evb_eval_attach(evb_handle *h, int64_t nobs, const uint8_t *x
                        metric == EVB_METRIC_QUANTILE || (metric == EVB_METRIC_MULTIQUANTILE && loss == EVB_MULTIQUANTILE));
     if (!ok) { evb_set_error("evb_eval_attach: metric %d is not defined for loss %d", metric, loss); return EVB_ERR_ARG; }
     drop_graphs(h); // the launch sequence of a tree changes
-    int32_t rc = eval_attach_impl(h, nobs, x_bin, y, w, pred0, bias, metric, sums);
+    int32_t rc = eval_attach_impl(h, nobs, x_bin, mx, y, w, pred0, bias, metric, sums);
     if (rc != EVB_OK) free_eval(h);
     return rc;
+}
+
+extern "C" int32_t evb_eval_attach(evb_handle *h, int64_t nobs, const uint8_t *x_bin, const void *y, const float *w, const float *pred0,
+                                   const float *bias, int32_t metric, double sums[2]) {
+    return eval_attach(h, nobs, x_bin, nullptr, y, w, pred0, bias, metric, sums);
+}
+
+extern "C" int32_t evb_eval_attach_m(evb_handle *h, const evb_matrix *m, const void *y, const float *w, const float *pred0, const float *bias,
+                                     int32_t metric, double sums[2]) {
+    if (!h || !m || evb_matrix_feats(m) != h->nfeats || !h->edges_d || evb_matrix_dtype(m) != h->edges_dtype) {
+        evb_set_error("evb_eval_attach_m: the handle keeps no edges (evb_create_m) or the matrix has other columns or another type");
+        return EVB_ERR_ARG;
+    }
+    return eval_attach(h, evb_matrix_rows(m), nullptr, m, y, w, pred0, bias, metric, sums);
 }
 
 extern "C" int32_t evb_eval_sums(evb_handle *h, double sums[2]) {
@@ -720,9 +759,7 @@ extern "C" int32_t evb_eval_sums(evb_handle *h, double sums[2]) {
 extern "C" int32_t evb_eval_get_pred(evb_handle *h, float *pred) {
     EVB_ENTER(h);
     if (!pred || h->ev_n == 0) { evb_set_error("evb_eval_get_pred: no evaluation data attached or null output"); return EVB_ERR_ARG; }
-    EVB_CUDA(cudaMemcpyAsync(pred, h->ev_pred, sizeof(float) * h->ev_n * h->K, cudaMemcpyDeviceToHost, h->st));
-    EVB_CUDA(cudaStreamSynchronize(h->st));
-    return EVB_OK;
+    return evb_d2h_staged(pred, h->ev_pred, sizeof(float) * h->ev_n * h->K, h->st);
 }
 
 extern "C" int32_t evb_eval_detach(evb_handle *h) {
@@ -828,9 +865,7 @@ extern "C" int32_t evb_set_timing(evb_handle *h, int32_t on) {
 extern "C" int32_t evb_get_pred(evb_handle *h, float *pred) {
     EVB_ENTER(h);
     if (!pred) { evb_set_error("null output"); return EVB_ERR_ARG; }
-    EVB_CUDA(cudaMemcpyAsync(pred, h->pred, sizeof(float) * h->n * h->K, cudaMemcpyDeviceToHost, h->st));
-    EVB_CUDA(cudaStreamSynchronize(h->st));
-    return EVB_OK;
+    return evb_d2h_staged(pred, h->pred, sizeof(float) * h->n * h->K, h->st);
 }
 
 extern "C" int32_t evb_get_grads(evb_handle *h, float *grad) {

@@ -554,6 +554,14 @@ int32_t evb_q2_build_layout(evb_handle *h) {
     return EVB_OK;
 }
 
+// what the binarize kernel does not write: the all-zero row n, and the xE words when no feature lives there
+int32_t evb_q2_clear_layout(evb_handle *h) {
+    const Q2Geom &g = h->q2;
+    EVB_CUDA(cudaMemsetAsync(h->xH + (size_t)h->n * g.RSH, 0, g.RSH, h->st));
+    EVB_CUDA(cudaMemsetAsync(h->xE + (g.ntail > 0 ? h->n : 0), 0, sizeof(uint2) * (g.ntail > 0 ? 1 : (size_t)h->n + 1), h->st));
+    return EVB_OK;
+}
+
 int32_t evb_launch_q2_quantize(evb_handle *h) {
     evb_tic(h, EVB_T_GRADS);
     k_q2_quantize<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->grad, h->GS, h->xE, h->n, h->d_gmax, h->d_qinv, h->q2.QB);

@@ -90,6 +90,8 @@ struct evb_handle {
     int busy;
 
     // row data
+    void *edges_d;     // edges of the raw matrix the handle was made from (evb_create_m), dtype edges_dtype
+    int edges_dtype, nedges;
     uint8_t *xT;       // [n][RS]  observation-major bins (1..B), zero padded
     uint8_t *xC;       // [nfeats][n] feature-major copy (the layout of the caller's x_bin) read by the row partition
     float *grad;       // [n][GS]  g_1..g_K,h_1..h_K,w,(pad)
@@ -219,6 +221,7 @@ int32_t evb_launch_hist_reduce(evb_handle *h, int level);
 // evb_histq2.cu
 int32_t evb_q2_configure(evb_handle *h);
 int32_t evb_q2_build_layout(evb_handle *h);
+int32_t evb_q2_clear_layout(evb_handle *h);
 int32_t evb_launch_q2_quantize(evb_handle *h);
 int32_t evb_launch_histq2(evb_handle *h, int level);
 int32_t evb_launch_q2_reduce(evb_handle *h, int level);
@@ -231,6 +234,13 @@ int32_t evb_launch_partition(evb_handle *h, int level); // plan + flags + prefix
 int32_t evb_launch_lonely_barrier(evb_handle *h, int *flags, int *seq, unsigned max_polls);
 int32_t evb_check_device(int device); // evb_rows.cu: makes `device` current
 void evb_predict_trim(int device);       // evb_predict.cu: kept work buffers back to the block cache
+// evb_matrix.cu
+int64_t evb_matrix_rows(const evb_matrix *m);
+int evb_matrix_feats(const evb_matrix *m);
+int evb_matrix_dtype(const evb_matrix *m);
+cudaError_t evb_matrix_join(const evb_matrix *m, cudaStream_t st);
+int32_t evb_matrix_binarize(const evb_matrix *m, const void *edges_dev, int nedges, uint8_t *xC, uint8_t *xT, int RS, uint8_t *xH, int RSH, uint2 *xE, int nmain,
+                            int *err, cudaStream_t st);
 // evb_nccl.cpp
 int32_t evb_nccl_unique_id(uint8_t id[128]);
 int32_t evb_nccl_init(evb_handle *h, const uint8_t id[128], int rank, int world);
@@ -243,6 +253,7 @@ void evb_nccl_destroy(evb_handle *h);
 cudaError_t evb_dev_alloc(void **p, size_t bytes);
 void evb_dev_free(void *p, bool really = false);
 template <typename T> inline cudaError_t evb_dev_alloc(T **p, size_t bytes) { return evb_dev_alloc(reinterpret_cast<void **>(p), bytes); }
+size_t evb_cached_bytes(int dev); // bytes the cache holds for reuse
 cudaError_t evb_host_alloc(void **p, size_t bytes);
 void evb_host_free(void *p);
 cudaError_t evb_stream_get(cudaStream_t *st);
@@ -254,6 +265,7 @@ void evb_event_put(cudaEvent_t ev);
 void evb_parallel(void (*fn)(void *, size_t, size_t), void *ctx, size_t n, size_t slice);
 // host copies between a packed buffer and nseg strided segments by all staging threads (`up`: strided -> packed)
 void evb_copy_packed(void *packed, const void *strided, size_t seg, size_t stride, size_t off, size_t len, bool up);
+int32_t evb_d2h_staged(void *dst_host, const void *src_dev, size_t bytes, cudaStream_t st);
 int32_t evb_h2d_staged(void *dst_dev, const void *src_host, size_t bytes, cudaStream_t st, bool drain = true);
 int32_t evb_h2d_staged_strided(void *dst_dev, const void *src_host, size_t seg_bytes, size_t nseg, size_t stride, cudaStream_t st, bool drain = true);
 

@@ -8,11 +8,12 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 
 import numpy as np
 
 from . import _lib
-from .binning import binarize, get_edges
+from .binning import RawMatrix, binarize, get_edges, sample_rows
 from .learners import EvoTypes
 from .model import EvoTree, Tree
 
@@ -23,6 +24,32 @@ def _logit(x):
 
 def _invsoftplus(x):
     return x + math.log(-math.expm1(-x))  # src/loss.jl:266-268
+
+
+def _class_codes(yt: np.ndarray):
+    """Sorted levels of a class target, codes 1..K (uint32) and the rows of every level."""
+    size, unsigned = yt.dtype.itemsize, yt.dtype.kind in "ub"
+    if yt.dtype.kind in "iub" and yt.dtype.isnative and not (unsigned and size == 8) and yt.size >= 4096:
+        lib, y = _lib.lib(), np.ascontiguousarray(yt)
+        kind, n, rng = C.c_int32(size + (16 if unsigned else 0)), C.c_int64(y.size), (C.c_int64 * 2)()
+        _lib.check(lib.evb_host_range(_lib.ptr(y), kind, n, rng))
+        if rng[1] - rng[0] < 4096:       # counted instead of sorted
+            counts = np.empty(rng[1] - rng[0] + 1, np.int64)
+            _lib.check(lib.evb_host_count(_lib.ptr(y), kind, n, C.c_int64(rng[0]), C.c_int32(counts.size), _lib.ptr(counts)))
+            present = counts > 0
+            codes, code_of = np.empty(y.size, np.uint32), np.cumsum(present).astype(np.uint32)
+            _lib.check(lib.evb_host_codes(_lib.ptr(y), kind, n, C.c_int64(rng[0]), _lib.ptr(code_of), _lib.ptr(codes)))
+            return (np.flatnonzero(present) + rng[0]).astype(yt.dtype), codes, counts[present]
+    levels, codes = np.unique(yt, return_inverse=True)
+    return levels, (codes + 1).astype(np.uint32), np.bincount(codes, minlength=levels.size)
+
+
+def _std(y: np.ndarray) -> float:
+    if y.size >= 1 << 16 and y.flags.c_contiguous:
+        out = C.c_double()
+        _lib.check(_lib.lib().evb_host_std(_lib.ptr(y), C.c_int64(y.size), C.byref(out)))
+        return out.value
+    return float(np.std(y.astype(np.float64), ddof=1))
 
 
 def init_target(loss: str, y_train: np.ndarray, offset, alphas=(0.1, 0.5, 0.9)):
@@ -56,13 +83,12 @@ def init_target(loss: str, y_train: np.ndarray, offset, alphas=(0.1, 0.5, 0.9)):
         yt = np.asarray(y_train)
         if yt.ndim != 1 or not (np.issubdtype(yt.dtype, np.integer) or yt.dtype == bool or yt.dtype.kind in "US"):
             raise ValueError(f"Invalid target eltype: {yt.dtype}")
-        levels, codes = np.unique(yt, return_inverse=True)
+        levels, y, counts = _class_codes(yt)
         K = int(levels.size)
         if K < 2:
             raise ValueError(f"Classification requires a target with at least 2 levels, got {K}")
-        y = (codes + 1).astype(np.uint32)
         ycols = 1
-        prop = np.bincount(codes, minlength=K) / codes.size
+        prop = counts / y.size
         mu = np.log(prop).astype(np.float32)
         mu -= mu.max()
         if offset is not None:
@@ -76,7 +102,7 @@ def init_target(loss: str, y_train: np.ndarray, offset, alphas=(0.1, 0.5, 0.9)):
         sd_factor = math.sqrt(3.0) / math.pi if loss == "logistic_mle" else 1.0   # src/init.jl:86, 95
         for t in range(ycols):
             mu[2 * t] = y2[:, t].mean(dtype=np.float32)
-            mu[2 * t + 1] = _invsoftplus(float(np.std(y2[:, t].astype(np.float64), ddof=1)) * sd_factor)
+            mu[2 * t + 1] = _invsoftplus(_std(y2[:, t]) * sd_factor)
         if offset is not None:
             offset = np.array(offset, np.float32, copy=True)
             offset[:, 1::2] = [[_invsoftplus(float(v)) for v in row] for row in offset[:, 1::2]]
@@ -100,6 +126,7 @@ class Cache:
         self.K = 1
         self.nn = 0
         self.feature_names = None
+        self.edges = None           # edges the handle keeps (made from a RawMatrix), else None
 
     def close(self):
         if self.handle:
@@ -172,11 +199,13 @@ def make_params(params: EvoTypes, K: int, device: int, flags: int = 0) -> _lib.E
 
 
 def init_core_binned(params: EvoTypes, x_bin: np.ndarray, y, ycols: int, K: int, mu: np.ndarray, w=None, pred0=None,
-                     feattypes=None, device: int = 0, flags: int = 0, comm=None, x_raw=None, edges=None) -> Cache:
+                     feattypes=None, device: int = 0, flags: int = 0, comm=None, x_raw=None, edges=None, matrix=None) -> Cache:
     """Creates the device handle from an already binned matrix (uint8, Fortran order, values 1..nbins), or -- with
-    `x_raw` (float32 / float64, Fortran order) and `edges` [nfeats, nbins - 1] -- from the raw features, which are then
-    binarized on the device (`evb_create_x`)."""
-    if x_raw is None:
+    `x_raw` (float32 / float64, Fortran order) or `matrix` (a `RawMatrix`) and `edges` [nfeats, nbins - 1] -- from the raw
+    features, which are then binarized on the device (`evb_create_x`, `evb_create_m`)."""
+    if matrix is not None:
+        nobs, nfeats = matrix.shape
+    elif x_raw is None:
         assert x_bin.dtype == np.uint8 and x_bin.flags.f_contiguous
         nobs, nfeats = x_bin.shape
     else:
@@ -199,17 +228,22 @@ def init_core_binned(params: EvoTypes, x_bin: np.ndarray, y, ycols: int, K: int,
     cp = make_params(params, K, device, flags)
     ydt = _lib.EVB_U32 if params.loss == "mlogloss" else _lib.EVB_F32
     mu32 = np.ascontiguousarray(mu, np.float32)
-    if x_raw is None:
+    if x_raw is None and matrix is None:
         _lib.check(_lib.lib().evb_create(C.byref(cache.handle), C.byref(cp), C.c_int64(nobs), C.c_int32(nfeats), _lib.ptr(x_bin),
                                          _lib.ptr(y), C.c_int32(ydt), C.c_int32(ycols), _lib.ptr(w32), _lib.ptr(p0), _lib.ptr(mu32),
                                          _lib.ptr(ft), _lib.ptr(mono)))
     else:
-        e = np.ascontiguousarray(edges, dtype=x_raw.dtype)  # [nfeats, nedges] C order == [nedges x nfeats] column-major
-        xdt = _lib.EVB_F32 if x_raw.dtype == np.float32 else _lib.EVB_F64
+        e = np.ascontiguousarray(edges, dtype=(x_raw if matrix is None else matrix).dtype)  # [nfeats, nedges] C order == [nedges x nfeats] column-major
+        xdt = _lib.EVB_F32 if e.dtype == np.float32 else _lib.EVB_F64
         try:
-            _lib.check(_lib.lib().evb_create_x(C.byref(cache.handle), C.byref(cp), C.c_int64(nobs), C.c_int32(nfeats), _lib.ptr(x_raw),
-                                               C.c_int32(xdt), _lib.ptr(e), C.c_int32(e.shape[1]), _lib.ptr(y), C.c_int32(ydt),
-                                               C.c_int32(ycols), _lib.ptr(w32), _lib.ptr(p0), _lib.ptr(mu32), _lib.ptr(ft), _lib.ptr(mono)))
+            if matrix is not None:
+                _lib.check(_lib.lib().evb_create_m(C.byref(cache.handle), C.byref(cp), matrix.handle, _lib.ptr(e), C.c_int32(e.shape[1]), _lib.ptr(y),
+                                                   C.c_int32(ydt), C.c_int32(ycols), _lib.ptr(w32), _lib.ptr(p0), _lib.ptr(mu32), _lib.ptr(ft), _lib.ptr(mono)))
+                cache.edges = e
+            else:
+                _lib.check(_lib.lib().evb_create_x(C.byref(cache.handle), C.byref(cp), C.c_int64(nobs), C.c_int32(nfeats), _lib.ptr(x_raw),
+                                                   C.c_int32(xdt), _lib.ptr(e), C.c_int32(e.shape[1]), _lib.ptr(y), C.c_int32(ydt),
+                                                   C.c_int32(ycols), _lib.ptr(w32), _lib.ptr(p0), _lib.ptr(mu32), _lib.ptr(ft), _lib.ptr(mono)))
         except _lib.EvbError as err:
             if "NaN" in str(err):
                 raise ValueError("missing / NaN feature values are not supported") from err   # test/missings.jl
@@ -227,22 +261,57 @@ def init_core(params: EvoTypes, x_train: np.ndarray, y_train, w_train=None, offs
     x_train = np.asarray(x_train)
     if x_train.dtype not in (np.float32, np.float64):
         x_train = x_train.astype(np.float64)
-    x_train = np.asfortranarray(x_train)      # a Julia Matrix is column-major; no copy when it already is
     nobs, nfeats = x_train.shape
     rng = np.random.default_rng(params.seed)
-    edges, featbins, feattypes = get_edges(x_train, params.nbins, rng)
-    if np.isnan(edges).any():                 # the device check below covers the rows the sample did not see
-        raise ValueError("missing / NaN feature values are not supported")   # test/missings.jl
-    offset = None if offset_train is None else np.array(offset_train, np.float32, copy=True).reshape(nobs, -1)
-    K, y, ycols, mu, levels, offset = init_target(params.loss, y_train, offset, params.alphas)
-    if comm is not None:
-        edges, mu = comm.broadcast_host(edges), comm.allreduce_bias(params.loss, y, mu, K, params.alphas)
-    pred0 = None
-    if offset is not None:
-        mu = np.zeros_like(mu)                                               # src/init.jl:164
-        pred0 = np.ascontiguousarray(np.broadcast_to(mu, (nobs, K)) + offset, np.float32)
-    # `binarize(x_train; edges)` runs on the device inside evb_create_x: raw features up, bins never down
-    cache = init_core_binned(params, None, y, ycols, K, mu, w_train, pred0, feattypes, device, flags, comm, x_raw=x_train, edges=edges)
+    host = {}
+
+    def host_work():       # what needs no device: the sample of the edges, target and bias
+        try:
+            host["rows"] = sample_rows(nobs, params.nbins, rng)
+            offset = None if offset_train is None else np.array(offset_train, np.float32, copy=True).reshape(nobs, -1)
+            host["target"] = init_target(params.loss, y_train, offset, params.alphas)
+        except Exception as e:
+            host["error"] = e
+
+    # a thread costs about as much as uploading 4 MB: below that the two follow one another
+    side = threading.Thread(target=host_work) if x_train.nbytes >= 4 << 20 else None
+    if side is not None:
+        side.start()
+    try:
+        matrix = RawMatrix(x_train, device)
+    except _lib.EvbError as e:
+        if e.code != _lib.ERR_LIMIT:
+            raise
+        matrix = None      # larger than the device holds beside the training state: streamed in blocks of features
+    finally:
+        if side is not None:
+            side.join()
+    if side is None:
+        host_work()
+    try:
+        if matrix is None:
+            x_train = np.asfortranarray(x_train)
+            edges = get_edges(x_train, params.nbins, np.random.default_rng(params.seed))[0]
+        else:
+            edges = matrix.edges(params.nbins, host.get("rows"))
+        if np.isnan(edges).any():                 # the device check below covers the rows the sample did not see
+            raise ValueError("missing / NaN feature values are not supported")   # test/missings.jl
+        if "error" in host:
+            raise host["error"]
+        K, y, ycols, mu, levels, offset = host["target"]
+        featbins, feattypes = np.full(nfeats, params.nbins, dtype=np.uint8), np.ones(nfeats, dtype=bool)
+        if comm is not None:
+            edges, mu = comm.broadcast_host(edges), comm.allreduce_bias(params.loss, y, mu, K, params.alphas)
+        pred0 = None
+        if offset is not None:
+            mu = np.zeros_like(mu)                                               # src/init.jl:164
+            pred0 = np.ascontiguousarray(np.broadcast_to(mu, (nobs, K)) + offset, np.float32)
+        # `binarize(x_train; edges)` runs on the device: raw features up, bins never down
+        cache = init_core_binned(params, None, y, ycols, K, mu, w_train, pred0, feattypes, device, flags, comm,
+                                 x_raw=x_train if matrix is None else None, edges=edges, matrix=matrix)
+    finally:
+        if matrix is not None:
+            matrix.close()
     names = [f"feat_{i + 1}" for i in range(nfeats)] if feature_names is None else [str(s) for s in feature_names]
     if len(names) != nfeats:
         raise ValueError("feature_names must have one entry per column of x_train")
@@ -399,7 +468,7 @@ class CallBack:
         if x_eval.ndim != 2 or x_eval.shape[1] != cache.nfeats:
             raise ValueError("x_eval must have the columns of x_train")
         edges = m.info["edges"]
-        x_bin = binarize(x_eval.astype(edges.dtype, copy=False), edges, device)
+        x_eval = x_eval.astype(edges.dtype, copy=False)
         loss, K = params.loss, m.K
         if loss == "mlogloss":
             y = eval_levelcode(y_eval, m.info["target_levels"])
@@ -422,8 +491,21 @@ class CallBack:
         self.cache, self.comm = cache, comm
         bias = np.ascontiguousarray(m.trees[-1].pred[0], np.float32)  # cb(logger, 0, m.trees[end]), src/fit.jl:416
         sums = (C.c_double * 2)()
-        _lib.check(_lib.lib().evb_eval_attach(cache.handle, C.c_int64(nobs), _lib.ptr(x_bin), _lib.ptr(y), _lib.ptr(w),
-                                              _lib.ptr(pred0), _lib.ptr(bias), C.c_int32(_lib.METRIC_CODES[self.metric]), sums))
+        matrix = None
+        if cache.edges is not None and cache.edges.dtype == edges.dtype and np.array_equal(cache.edges, edges):   # the handle can binarize
+            try:
+                matrix = RawMatrix(x_eval, device)
+            except _lib.EvbError as e:
+                if e.code != _lib.ERR_LIMIT:
+                    raise
+        if matrix is not None:
+            with matrix:
+                _lib.check(_lib.lib().evb_eval_attach_m(cache.handle, matrix.handle, _lib.ptr(y), _lib.ptr(w), _lib.ptr(pred0), _lib.ptr(bias),
+                                                        C.c_int32(_lib.METRIC_CODES[self.metric]), sums))
+        else:
+            x_bin = binarize(x_eval, edges, device)
+            _lib.check(_lib.lib().evb_eval_attach(cache.handle, C.c_int64(nobs), _lib.ptr(x_bin), _lib.ptr(y), _lib.ptr(w),
+                                                  _lib.ptr(pred0), _lib.ptr(bias), C.c_int32(_lib.METRIC_CODES[self.metric]), sums))
         self.nobs = nobs
         self.initial = self._metric(sums)
 

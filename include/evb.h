@@ -125,7 +125,38 @@ EVB_API int32_t evb_create(evb_handle **out, const evb_params *p, int64_t nobs, 
 EVB_API int32_t evb_create_x(evb_handle **out, const evb_params *p, int64_t nobs, int32_t nfeats, const void *x, int32_t x_dtype,
                              const void *edges, int32_t nedges, const void *y, int32_t y_dtype, int32_t ycols, const float *w,
                              const float *pred0, const float *mu, const uint8_t *feattypes, const int32_t *monotone);
+/*
+ * evb_matrix -- a raw feature matrix on the device, for `init_core` without host passes over the features: upload it once
+ * (column-major or row-major), take the quantile edges of a sample of its rows from it (`get_edges`, src/fit-utils.jl:7-24:
+ * the caller draws the sample), and make handles from it.  evb_matrix_create returns as soon as the host array has been
+ * read; EVB_ERR_LIMIT when it would not fit beside the training state (use evb_create_x then).
+ * evb_matrix_edges: rows = sampled row ids (0-based, any order), NULL = all rows; edge e of a feature is
+ * a + g[e] (b - a) if |a - b| <= rtol max(|a|, |b|), else (1 - g[e]) a + g[e] b, in double, where a / b are the order
+ * statistics lo[e] / hi[e] (0-based) of the sample; edges: host [nedges x nfeats] column-major, type of x.
+ * evb_create_m: evb_create_x with the matrix in the place of x.  evb_eval_attach_m: evb_eval_attach with raw rows of the
+ * same element type, binarized with the handle's edges.
+ */
+typedef struct evb_matrix evb_matrix;
+EVB_API int32_t evb_matrix_create(evb_matrix **out, int32_t device, int64_t nobs, int32_t nfeats, const void *x, int32_t x_dtype,
+                                  int32_t x_row_major);
+EVB_API int32_t evb_matrix_edges(evb_matrix *m, const uint32_t *rows, int32_t nrows, int32_t nedges, const int32_t *lo, const int32_t *hi,
+                                 const double *g, double rtol, void *edges);
+EVB_API void evb_matrix_destroy(evb_matrix *m);
+EVB_API int32_t evb_create_m(evb_handle **out, const evb_params *p, const evb_matrix *m, const void *edges, int32_t nedges, const void *y,
+                             int32_t y_dtype, int32_t ycols, const float *w, const float *pred0, const float *mu, const uint8_t *feattypes,
+                             const int32_t *monotone);
+EVB_API int32_t evb_eval_attach_m(evb_handle *h, const evb_matrix *m, const void *y, const float *w, const float *pred0, const float *bias,
+                                  int32_t metric, double sums[2]);
 EVB_API void evb_destroy(evb_handle *h);
+/*
+ * Passes over a host target with several threads, for `_init_target` (src/init.jl:10-146): smallest and largest value and
+ * the counts of every value of an integer target, its class codes code_of[y - lo], and the sample standard deviation.
+ *   kind  bytes per value (1, 2, 4, 8), + 16 when unsigned (1, 2, 4)
+ */
+EVB_API int32_t evb_host_range(const void *y, int32_t kind, int64_t n, int64_t range[2]);
+EVB_API int32_t evb_host_count(const void *y, int32_t kind, int64_t n, int64_t lo, int32_t nvalues, int64_t *counts);
+EVB_API int32_t evb_host_codes(const void *y, int32_t kind, int64_t n, int64_t lo, const uint32_t *code_of, uint32_t *codes);
+EVB_API int32_t evb_host_std(const float *y, int64_t n, double *out);
 /*
  * Device memory released by evb_destroy and by the inference calls is kept by the library and reused by the next
  * evb_create* / evb_predict* of about the same size (cudaMalloc and cudaFree take driver-wide locks: a second `fit` of

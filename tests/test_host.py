@@ -182,3 +182,18 @@ def test_julia_glue_loss_codes_match_the_header_and_the_python_binding(pkg):
     assert codes == julia
     assert "LOSS_TYPE_CODE = Dict(T => LOSS_CODE[s] for (s, T) in _loss2type_dict)" in src
     assert "lowercase(" not in src and "LOSS_TYPE_CODE[L]" in src
+
+
+@pytest.mark.parametrize("n", [5, 5_000, 200_000])
+def test_class_codes_equal_unique(pkg, n):
+    """Counting the values of an integer target gives the levels, codes and counts that sorting gives."""
+    from evotrees_b200.fit import _class_codes, _std
+    rng = np.random.default_rng(n)
+    for y in (rng.integers(-3, 4, n), rng.integers(0, 2, n).astype(bool), rng.integers(250, 256, n).astype(np.uint8), 10 ** 12 + rng.integers(0, 3000, n) * 2,
+              rng.integers(0, 10 ** 9, n).astype(np.int32), np.array(["b", "a", "c"])[rng.integers(0, 3, n)]):
+        levels, codes, counts = _class_codes(y)
+        want, inv = np.unique(y, return_inverse=True)
+        assert levels.dtype == y.dtype and np.array_equal(levels, want)
+        assert codes.dtype == np.uint32 and np.array_equal(codes, inv + 1) and np.array_equal(counts, np.bincount(inv))
+    v = rng.normal(5.0, 2.0, n).astype(np.float32)
+    assert abs(_std(v) - np.std(v.astype(np.float64), ddof=1)) < 1e-12
