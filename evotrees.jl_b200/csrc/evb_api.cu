@@ -151,7 +151,7 @@ static void free_handle(evb_handle *h) {
     if (exported) { evb_dev_free(h->hcomp, true); h->hcomp = nullptr; }
     free_eval(h);
     void *ptrs[] = {h->xH, h->xE, h->hsum_q, h->hcnt_q, h->qs_cnt, h->qs_prefix, h->qs_rank, h->qs_gamma, h->gradq, h->d_gmax, h->d_qinv, h->xT, h->xC, h->grad, h->pred, h->y, h->nidx, h->rows[0], h->rows[1], h->mask_d, h->feattypes_d, h->mono_d,
-                    h->js_d, h->seg_start, h->seg_cnt, h->gcnt, h->nleft, (h->gnleft != h->nleft) ? h->gnleft : nullptr, h->kind,
+                    h->gen_d, h->seg_start, h->seg_cnt, h->gcnt, h->nleft, (h->gnleft != h->nleft) ? h->gnleft : nullptr, h->kind,
                     h->bslot, h->nsum, h->plan /* base of the tree block */, h->cum, h->slot_node, h->item_node, h->item_left,
                     h->item_lprefix, h->item_bits, h->scan_tmp, h->hist, h->hcomp, h->scratch, h->fbest_gain, h->fbest_bin, h->obl_gain, h->obl_best, h->edges_d};
     phase("exchange buffers");
@@ -247,7 +247,8 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     EVB_CUDA(dalloc(&h->mask_d, (size_t)n));
     EVB_CUDA(dalloc(&h->feattypes_d, (size_t)nfeats));
     EVB_CUDA(dalloc(&h->mono_d, (size_t)nfeats));
-    EVB_CUDA(dalloc(&h->js_d, (size_t)nfeats));
+    EVB_CUDA(dalloc(&h->gen_d, (size_t)EVB_GEN_WORDS / 2 + (nfeats + 1) / 2));
+    h->js_d = reinterpret_cast<uint32_t *>(h->gen_d) + EVB_GEN_WORDS;
     EVB_CUDA(dalloc(&h->seg_start, (size_t)nids)); EVB_CUDA(dalloc(&h->seg_cnt, (size_t)nids));
     EVB_CUDA(dalloc(&h->gcnt, (size_t)nids)); EVB_CUDA(dalloc(&h->nleft, (size_t)nids));
     h->gnleft = h->nleft;
@@ -265,7 +266,8 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     h->h_tree_bytes = L.total;
     for (int q = 0; q < 2; ++q) {
         EVB_CUDA(evb_host_alloc(&h->h_tree[q], L.total));
-        EVB_CUDA(evb_host_alloc((void **)&h->h_js[q], sizeof(uint32_t) * nfeats));
+        EVB_CUDA(evb_host_alloc((void **)&h->h_js[q], sizeof(uint32_t) * (EVB_GEN_WORDS + nfeats)));
+        memset(h->h_js[q], 0, sizeof(uint32_t) * EVB_GEN_WORDS);
         EVB_CUDA(evb_event_get(&h->ev_done[q]));
     }
     { const char *e = getenv("EVB_GRAPH"); h->use_graphs = e ? atoi(e) != 0 : true; }
@@ -463,9 +465,9 @@ extern "C" int32_t evb_comm_init(evb_handle *h, const uint8_t id[128], int32_t r
 
 // Everything one tree launches, in stream order.  Runs either directly or under stream capture (then it is
 // replayed as one CUDA graph per tree): it must not synchronise and must not touch pageable host memory.
-static int32_t enqueue_tree(evb_handle *h, bool use_mask, uint8_t mask_cond, bool run_grads, bool quantize, bool fuse, int slot) {
+static int32_t enqueue_tree(evb_handle *h, int use_mask, uint8_t mask_cond, bool run_grads, bool quantize, bool fuse, int slot) {
     const int D = h->D;
-    EVB_CUDA(cudaMemcpyAsync(h->js_d, h->h_js[slot], sizeof(uint32_t) * h->F, cudaMemcpyHostToDevice, h->st));
+    EVB_CUDA(cudaMemcpyAsync(h->gen_d, h->h_js[slot], sizeof(uint32_t) * (EVB_GEN_WORDS + h->F), cudaMemcpyHostToDevice, h->st));
     if (run_grads) EVB_CHECK(evb_launch_grads(h));
     if (quantize) EVB_CHECK(h->use_q2 ? evb_launch_q2_quantize(h) : evb_launch_quantize(h)); // fixed-point histogram kernel: the gradients changed since the last tree
     EVB_CHECK(evb_launch_tree_reset(h));
@@ -494,7 +496,7 @@ static int32_t enqueue_tree(evb_handle *h, bool use_mask, uint8_t mask_cond, boo
     if (h->p.loss == EVB_QUANTILE || h->p.loss == EVB_MULTIQUANTILE) {
         // the leaf values need the leaf of every row first: leaf ids, per-leaf quantiles, then the usual update
         EVB_CHECK(evb_launch_finalize(h, false, 1));
-        EVB_CHECK(evb_launch_quantile_leaves(h, use_mask, mask_cond));
+        EVB_CHECK(evb_launch_quantile_leaves(h, use_mask != EVB_MASK_NONE, mask_cond));
         EVB_CHECK(evb_launch_finalize(h, fuse, 2));
     } else {
         EVB_CHECK(evb_launch_finalize(h, fuse, 0));
@@ -509,8 +511,8 @@ static void drop_graphs(evb_handle *h) {
     for (auto &c : h->graph_calls) c = 0;
 }
 
-extern "C" int32_t evb_grow_tree_begin(evb_handle *h, const uint8_t *row_mask, uint8_t mask_cond, const uint32_t *js, int32_t njs,
-                                       int32_t update_grads) {
+static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen, uint8_t mask_cond, const uint32_t *js, int32_t njs,
+                          int32_t update_grads) {
     EVB_ENTER(h);
     if (!js || njs < 1 || njs > h->nfeats) { evb_set_error("evb_grow_tree: invalid argument"); return EVB_ERR_ARG; }
     if (h->pending >= 2 || (h->pending >= 1 && h->timing)) {
@@ -523,7 +525,7 @@ extern "C" int32_t evb_grow_tree_begin(evb_handle *h, const uint8_t *row_mask, u
             evb_set_error("evb_grow_tree: js must be strictly ascending within 1..nfeats");
             return EVB_ERR_ARG;
         }
-        h->h_js[slot][i] = js[i] - 1;
+        h->h_js[slot][EVB_GEN_WORDS + i] = js[i] - 1;
     }
     if (h->world > 1) EVB_CHECK(evb_nccl_check(h));
     if (njs != h->F && h->use_q2) { // this kernel always accumulates all features; the scan reads the sampled ones
@@ -550,12 +552,16 @@ extern "C" int32_t evb_grow_tree_begin(evb_handle *h, const uint8_t *row_mask, u
     if (update_grads) h->bag_idx = 0;
     const bool run_grads = update_grads && !h->grads_fresh;
     const bool fuse = h->bag_idx == h->p.bagging_size - 1;
-    const bool use_mask = row_mask != nullptr;
+    const int use_mask = gen ? EVB_MASK_PCG : row_mask ? EVB_MASK_HOST : EVB_MASK_NONE;
+    if (gen) {
+        EVB_CHECK(evb_pcg_tables(h->dev));
+        memcpy(h->h_js[slot], gen, sizeof(uint32_t) * EVB_GEN_WORDS);
+    }
     if (h->timing) {
         if (!h->ev_tot[0]) { EVB_CUDA(cudaEventCreate(&h->ev_tot[0])); EVB_CUDA(cudaEventCreate(&h->ev_tot[1])); }
         cudaEventRecord(h->ev_tot[0], h->st);
     }
-    if (use_mask) {
+    if (use_mask == EVB_MASK_HOST) {
         evb_tic(h, EVB_T_H2D);
         EVB_CUDA(cudaMemcpyAsync(h->mask_d, row_mask, (size_t)h->n, cudaMemcpyHostToDevice, h->st));
         evb_toc(h, EVB_T_H2D);
@@ -566,7 +572,7 @@ extern "C" int32_t evb_grow_tree_begin(evb_handle *h, const uint8_t *row_mask, u
     if (update_grads) h->gradq_valid = false;
     const bool quantize = (h->q_active || h->use_q2) && !h->gradq_valid;
     if (quantize) h->gradq_valid = true;
-    const int key = (use_mask ? 1 : 0) | (run_grads ? 2 : 0) | (fuse ? 4 : 0) | (slot ? 8 : 0) | (quantize ? 16 : 0);
+    const int key = (use_mask ? 1 : 0) | (use_mask == EVB_MASK_PCG ? 32 : 0) | (run_grads ? 2 : 0) | (fuse ? 4 : 0) | (slot ? 8 : 0) | (quantize ? 16 : 0);
     if (h->graph_mask_cond != (int)mask_cond) { drop_graphs(h); h->graph_mask_cond = mask_cond; }
     bool launched = false;
     // Sharded runs over NCCL stay on direct launches: a run that captured the NCCL collectives into the graph did not
@@ -606,7 +612,18 @@ extern "C" int32_t evb_grow_tree_begin(evb_handle *h, const uint8_t *row_mask, u
     h->bag_idx += 1;
     h->tree_seq += 1;
     h->pending += 1;
+    if (gen) evb_pcg_advance(gen, h->n);
     return EVB_OK;
+}
+
+extern "C" int32_t evb_grow_tree_begin(evb_handle *h, const uint8_t *row_mask, uint8_t mask_cond, const uint32_t *js, int32_t njs,
+                                       int32_t update_grads) {
+    return tree_begin(h, row_mask, nullptr, mask_cond, js, njs, update_grads);
+}
+
+extern "C" int32_t evb_grow_tree_begin_pcg(evb_handle *h, uint64_t gen[6], uint8_t mask_cond, const uint32_t *js, int32_t njs, int32_t update_grads) {
+    if (!gen || gen[4] > 1) { evb_set_error("evb_grow_tree_begin_pcg: invalid generator state"); return EVB_ERR_ARG; }
+    return tree_begin(h, nullptr, gen, mask_cond, js, njs, update_grads);
 }
 
 extern "C" int32_t evb_grow_tree_end(evb_handle *h, int64_t *feat, uint8_t *cond_bin, float *w_node, float *gain, float *leaf_pred,

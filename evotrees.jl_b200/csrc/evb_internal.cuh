@@ -34,7 +34,9 @@ constexpr int EVB_PART_CHUNK = 2048; // rows per partition work item
 constexpr int EVB_PART_THREADS = 256;
 constexpr int EVB_MAX_UNITS_PER_BLOCK = 4;
 constexpr int EVB_MAX_DEPTH = 15;
+constexpr int EVB_GEN_WORDS = 12;    // 32-bit words of a generator state
 
+enum { EVB_MASK_NONE = 0, EVB_MASK_HOST = 1, EVB_MASK_PCG = 2 }; // rows: all, a mask from the host, a mask made on the device
 enum { EVB_KIND_NONE = 0, EVB_KIND_BUILD = 1, EVB_KIND_SUB = 2 };
 
 // Per-level plan, device resident.  Written by the plan kernels, read by hist / reduce / scan.
@@ -103,6 +105,7 @@ struct evb_handle {
     uint8_t *mask_d;   // [n]
     uint8_t *feattypes_d; // [nfeats]
     int32_t *mono_d;      // [nfeats]
+    uint64_t *gen_d;      // [6] generator of the row mask (see k_sel_pcg), followed by js_d in the same block: one copy per tree
     uint32_t *js_d;       // [nfeats] 0-based feature id per slot
     int F;                // njs of the current tree
     bool grads_fresh;     // gradients already computed for the next round (fused into finalize)
@@ -174,14 +177,14 @@ struct evb_handle {
 
     // pinned host staging, double buffered so that tree t+1 can be enqueued before tree t is collected
     void *h_tree[2]; size_t h_tree_bytes;
-    uint32_t *h_js[2];
+    uint32_t *h_js[2];              // EVB_GEN_WORDS words of generator state, then the column sample
     cudaEvent_t ev_done[2];
     int tree_seq, pending;          // trees started / started but not yet collected
     // one CUDA graph per variant of the per-tree launch sequence (mask, gradients first, gradients fused, slot)
     bool use_graphs;
-    cudaGraphExec_t graph[32];
-    int graph_calls[32];
-    int64_t graph_launches[32][EVB_NTIMERS];
+    cudaGraphExec_t graph[64];
+    int graph_calls[64];
+    int64_t graph_launches[64][EVB_NTIMERS];
     int graph_mask_cond;
 
     // multi-GPU
@@ -208,7 +211,9 @@ struct evb_handle {
 int32_t evb_launch_transpose(evb_handle *h, const uint8_t *xcol_dev, int64_t ld, int64_t nrows, int j0, int nj, uint8_t *xT, int RS, cudaStream_t st);
 int32_t evb_launch_grads(evb_handle *h);
 int32_t evb_launch_quantize(evb_handle *h);
-int32_t evb_launch_rows_init(evb_handle *h, bool use_mask, uint8_t mask_cond);
+int32_t evb_launch_rows_init(evb_handle *h, int use_mask, uint8_t mask_cond);
+int32_t evb_pcg_tables(int dev);
+void evb_pcg_advance(uint64_t gen[6], int64_t n);
 int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode); // mode: see FinArgs in evb_rows.cu
 int32_t evb_launch_quantile_leaves(evb_handle *h, bool use_mask, uint8_t mask_cond);
 int32_t evb_launch_nidx_from_partition(evb_handle *h, uint32_t *out_dev);

@@ -5,6 +5,7 @@
 #include "evb_device.cuh"
 #include <float.h>
 #include <algorithm>
+#include <mutex>
 
 namespace {
 
@@ -216,6 +217,55 @@ __global__ void __launch_bounds__(SEL_THREADS) k_sel_count(const uint8_t *mask, 
         int t = 0;
         for (int w = 0; w < SEL_THREADS / 32; ++w) t += s[w];
         bcnt[blockIdx.x] = t;
+    }
+}
+// Row mask bytes from the caller's generator: PCG64 (O'Neill, "PCG: A Family of Simple Fast Space-Efficient Statistically
+// Good Algorithms for Random Number Generation", 2014: 128-bit LCG, XSL-RR output), whose 64-bit outputs are used as two
+// 32-bit words, low one first, of four bytes each.  An LCG can be advanced by any distance in logarithmic time, so every
+// thread makes the eight bytes of its own rows: the bytes of a generator on the host (0.75 ms per million rows, plus the
+// copy over PCIe: 0.85 of the 1.0 ms per tree at 1M rows) without the host.
+// state' after 2^k steps = state * M[k] + inc * G[k]; filled by the host once per device
+typedef unsigned __int128 u128;
+__constant__ u128 c_pcg_m[32], c_pcg_g[32];
+constexpr uint64_t PCG_MULT_HI = 2549297995355413924ull, PCG_MULT_LO = 4865540595714422341ull;
+__device__ __forceinline__ uint64_t pcg_out(u128 s) {
+    const uint64_t hi = (uint64_t)(s >> 64), x = hi ^ (uint64_t)s;
+    const unsigned r = (unsigned)(hi >> 58);
+    return (x >> r) | (x << ((64u - r) & 63u));
+}
+// gen: {state lo, hi, increment lo, hi, left, left word}: left = 1 when the high half of the last output is still to be used
+__global__ void __launch_bounds__(SEL_THREADS) k_sel_pcg(const uint64_t *gen, uint8_t cond, long long n, uint8_t *mask, int32_t *bcnt) {
+    static_assert(SEL_CHUNK == 8 * SEL_THREADS, "eight rows per thread");
+    __shared__ int s[SEL_THREADS / 32];
+    const u128 inc = ((u128)gen[3] << 64) | gen[2];
+    u128 st = ((u128)gen[1] << 64) | gen[0];
+    const unsigned left = (unsigned)gen[4];
+    const long long t = (long long)blockIdx.x * SEL_THREADS + threadIdx.x;
+    // outputs t - left and, when a word is left over, t; output d is made from the state after d + 1 steps
+    uint32_t skip = (uint32_t)(t + 1 - left);
+    for (int k = 0; skip; ++k, skip >>= 1)
+        if (skip & 1u) st = st * c_pcg_m[k] + inc * c_pcg_g[k];
+    uint64_t w = pcg_out(st);
+    if (left) {
+        const uint32_t lo = t == 0 ? (uint32_t)gen[5] : (uint32_t)(w >> 32);
+        st = st * c_pcg_m[0] + inc;
+        w = (uint64_t)lo | ((uint64_t)(uint32_t)pcg_out(st) << 32);
+    }
+    int c = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const uint8_t b = (uint8_t)(w >> (8 * q));
+        if (8 * t + q < n) c += b <= cond;
+    }
+    if (8 * t + 8 <= n) *reinterpret_cast<uint64_t *>(mask + 8 * t) = w;
+    else for (int q = 0; 8 * t + q < n && q < 8; ++q) mask[8 * t + q] = (uint8_t)(w >> (8 * q));
+    c = __reduce_add_sync(FULL, c);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int tot = 0;
+        for (int q = 0; q < SEL_THREADS / 32; ++q) tot += s[q];
+        bcnt[blockIdx.x] = tot;
     }
 }
 __global__ void __launch_bounds__(1024) k_sel_scan(int32_t *bcnt, int nblocks, int32_t *nleft0) {
@@ -720,13 +770,51 @@ int32_t evb_launch_quantize(evb_handle *h) {
     return EVB_OK;
 }
 
-int32_t evb_launch_rows_init(evb_handle *h, bool use_mask, uint8_t mask_cond) {
+int32_t evb_pcg_tables(int dev) { // once per device, outside any capture
+    static std::mutex mu;
+    static bool done[64] = {};
+    std::lock_guard<std::mutex> g(mu);
+    if (dev < 64 && done[dev]) return EVB_OK;
+    u128 m[32], a[32];
+    m[0] = ((u128)PCG_MULT_HI << 64) | PCG_MULT_LO;
+    a[0] = 1;
+    for (int k = 1; k < 32; ++k) { m[k] = m[k - 1] * m[k - 1]; a[k] = (m[k - 1] + 1) * a[k - 1]; }
+    EVB_CUDA(cudaMemcpyToSymbol(c_pcg_m, m, sizeof(m)));
+    EVB_CUDA(cudaMemcpyToSymbol(c_pcg_g, a, sizeof(a)));
+    if (dev < 64) done[dev] = true;
+    return EVB_OK;
+}
+// the generator after the words of n bytes have been taken from it (same six words as k_sel_pcg reads)
+void evb_pcg_advance(uint64_t gen[6], int64_t n) {
+    const u128 inc = ((u128)gen[3] << 64) | gen[2], mult = ((u128)PCG_MULT_HI << 64) | PCG_MULT_LO;
+    u128 st = ((u128)gen[1] << 64) | gen[0];
+    const uint64_t words = (uint64_t)(n + 3) / 4;
+    if (words == 0) return;
+    const uint64_t fresh = words - gen[4], outputs = (fresh + 1) / 2;
+    u128 m = mult, g = 1, am = 1, ag = 0; // am, ag: the steps taken so far
+    for (uint64_t k = outputs; k; k >>= 1) {
+        if (k & 1) { am = am * m; ag = ag * m + g; }
+        g = (m + 1) * g;
+        m = m * m;
+    }
+    st = st * am + inc * ag;
+    gen[0] = (uint64_t)st; gen[1] = (uint64_t)(st >> 64);
+    gen[4] = fresh & 1;
+    if (outputs) {
+        const uint64_t hi = (uint64_t)(st >> 64), x = hi ^ (uint64_t)st;
+        const unsigned r = (unsigned)(hi >> 58);
+        gen[5] = ((x >> r) | (x << ((64u - r) & 63u))) >> 32;
+    }
+}
+
+int32_t evb_launch_rows_init(evb_handle *h, int use_mask, uint8_t mask_cond) {
     evb_tic(h, EVB_T_ROWS_INIT);
     if (!use_mask) {
         k_rows_identity<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->rows[0], h->n, h->nleft);
     } else {
         const int nblocks = (int)((h->n + SEL_CHUNK - 1) / SEL_CHUNK);
-        k_sel_count<<<nblocks, SEL_THREADS, 0, h->st>>>(h->mask_d, mask_cond, h->n, h->scan_tmp);
+        if (use_mask == EVB_MASK_PCG) k_sel_pcg<<<nblocks, SEL_THREADS, 0, h->st>>>(h->gen_d, mask_cond, h->n, h->mask_d, h->scan_tmp);
+        else k_sel_count<<<nblocks, SEL_THREADS, 0, h->st>>>(h->mask_d, mask_cond, h->n, h->scan_tmp);
         k_sel_scan<<<1, 1024, 0, h->st>>>(h->scan_tmp, nblocks, h->nleft);
         k_sel_scatter<<<nblocks, SEL_THREADS, 0, h->st>>>(h->mask_d, mask_cond, h->n, h->scan_tmp, h->rows[0]);
     }

@@ -213,7 +213,7 @@ int32_t evb_h2d_staged(void *dst_dev, const void *src_host, size_t bytes, cudaSt
 int32_t evb_d2h_staged(void *dst_host, const void *src_dev, size_t bytes, cudaStream_t st) {
     int dev = 0;
     EVB_CUDA(cudaGetDevice(&dev));
-    if (bytes < ((size_t)1 << 20) || dev < 0 || dev >= 64) {
+    if (bytes < ((size_t)64 << 10) || dev < 0 || dev >= 64) {
         EVB_CUDA(cudaMemcpyAsync(dst_host, src_dev, bytes, cudaMemcpyDeviceToHost, st));
         EVB_CUDA(cudaStreamSynchronize(st));
         return EVB_OK;

@@ -325,12 +325,46 @@ def init_core(params: EvoTypes, x_train: np.ndarray, y_train, w_train=None, offs
 def sample_round(cache: Cache, params: EvoTypes):
     """Row mask bytes and the ascending column sample of one bag (src/subsample.jl:7, src/fit.jl:16).
     The mask is only drawn when rowsample < 1: with rowsample == 1 every byte passes `mask <= 255`."""
-    mask = cache.rng.integers(0, 256, size=cache.nobs, dtype=np.uint8) if cache.use_mask else None
+    return cache.rng.integers(0, 256, size=cache.nobs, dtype=np.uint8) if cache.use_mask else None, sample_columns(cache)
+
+
+def sample_columns(cache: Cache):
     if cache.njs >= cache.nfeats:
         js = np.arange(1, cache.nfeats + 1, dtype=np.uint32)
     else:
         js = (np.sort(cache.rng_js.choice(cache.nfeats, size=cache.njs, replace=False)) + 1).astype(np.uint32)
-    return mask, js
+    return js
+
+
+class _MaskStream:
+    """`cache.rng` while trees take their row masks from it on the device (`evb_grow_tree_begin_pcg`): the bytes are those
+    `sample_round` would draw, and the generator is left where it would leave it."""
+
+    def __init__(self, cache: Cache):
+        self.bitgen = cache.rng.bit_generator
+        s = self.bitgen.state
+        m = (1 << 64) - 1
+        self.gen = (C.c_uint64 * 6)(s["state"]["state"] & m, s["state"]["state"] >> 64, s["state"]["inc"] & m, s["state"]["inc"] >> 64,
+                                    s["has_uint32"], s["uinteger"])
+
+    @staticmethod
+    def of(cache: Cache):
+        return _MaskStream(cache) if cache.use_mask and isinstance(getattr(cache.rng, "bit_generator", None), np.random.PCG64) else None
+
+    def close(self):
+        g = self.gen
+        self.bitgen.state = {"bit_generator": "PCG64", "state": {"state": g[0] | g[1] << 64, "inc": g[2] | g[3] << 64}, "has_uint32": int(g[4]),
+                             "uinteger": int(g[5])}
+
+
+def _begin_sampled(cache: Cache, params: EvoTypes, stream, update_grads: bool) -> None:
+    """Draws the samples of one tree and enqueues it."""
+    if stream is None:
+        grow_tree_begin(cache, params, *sample_round(cache, params), update_grads)
+        return
+    js = sample_columns(cache)
+    _lib.check(_lib.lib().evb_grow_tree_begin_pcg(cache.handle, stream.gen, C.c_uint8(cache.mask_cond), _lib.ptr(js), C.c_int32(js.size),
+                                                  C.c_int32(1 if update_grads else 0)))
 
 
 def grow_tree(cache: Cache, params: EvoTypes, mask, js, update_grads: bool) -> Tree:
@@ -371,25 +405,32 @@ def grow_rounds(m: EvoTree, cache: Cache, params: EvoTypes, nrounds: int, on_tre
         if on_tree is not None:
             on_tree(collected)
 
+    stream = _MaskStream.of(cache)
     try:
         for _ in range(nrounds):
             for b in range(params.bagging_size):
-                mask, js = sample_round(cache, params)
-                grow_tree_begin(cache, params, mask, js, update_grads=(b == 0))
+                _begin_sampled(cache, params, stream, b == 0)
                 in_flight += 1
                 if in_flight == 2:
                     collect()
             m.info["nrounds"] += 1
     finally:
+        if stream is not None:
+            stream.close()
         while in_flight > 0:
             collect()
 
 
 def grow_evotree(m: EvoTree, cache: Cache, params: EvoTypes) -> None:
     """`grow_evotree!(m, cache, params)`: one boosting round = bagging_size trees."""
-    for b in range(params.bagging_size):
-        mask, js = sample_round(cache, params)
-        m.trees.append(grow_tree(cache, params, mask, js, update_grads=(b == 0)))
+    stream = _MaskStream.of(cache)
+    try:
+        for b in range(params.bagging_size):
+            _begin_sampled(cache, params, stream, b == 0)
+            m.trees.append(grow_tree_end(cache, params))
+    finally:
+        if stream is not None:
+            stream.close()
     m.info["nrounds"] += 1
 
 

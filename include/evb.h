@@ -209,6 +209,14 @@ EVB_API int32_t evb_grow_tree(evb_handle *h, const uint8_t *row_mask, uint8_t ma
  */
 EVB_API int32_t evb_grow_tree_begin(evb_handle *h, const uint8_t *row_mask, uint8_t mask_cond, const uint32_t *js, int32_t njs,
                                     int32_t update_grads);
+/*
+ * evb_grow_tree_begin with the row mask made on the device: byte i of the mask is byte i of the stream of a PCG64 generator
+ * (128-bit LCG, XSL-RR output; the low half of an output is used before the high half, bytes lowest first) -- the bytes
+ * that `rng.integers(0, 256, nobs, uint8)` of a numpy PCG64 generator gives.
+ *   gen   in / out: state (low, high 64 bits), increment (low, high), 1 if a 32-bit word is left over, that word;
+ *         advanced by the words that nobs bytes take
+ */
+EVB_API int32_t evb_grow_tree_begin_pcg(evb_handle *h, uint64_t gen[6], uint8_t mask_cond, const uint32_t *js, int32_t njs, int32_t update_grads);
 EVB_API int32_t evb_grow_tree_end(evb_handle *h, int64_t *feat, uint8_t *cond_bin, float *w_node, float *gain, float *leaf_pred,
                                   uint8_t *split);
 /*

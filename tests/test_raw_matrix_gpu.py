@@ -49,3 +49,26 @@ def test_handle_from_matrix_equals_handle_from_bins(pkg, n, f, order):
         assert np.array_equal(a.pred(), b.pred())
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize("n", [5, 2_047, 2_052, 40_003])
+def test_masks_made_on_the_device_are_the_generators(pkg, n):
+    """Trees whose row masks come from the device equal trees that are given the masks, and the generator ends in the same
+    place; row counts that leave half an output over included."""
+    rng = np.random.default_rng(n)
+    x = rng.random((n, 6)).astype(np.float32)
+    y = x.sum(axis=1).astype(np.float32)
+    params = pkg.EvoTreeRegressor(nrounds=5, max_depth=3, nbins=16, rowsample=0.6, min_weight=0.0)
+    ma, a = pkg.init_core(params, x, y)
+    mb, b = pkg.init_core(params, x, y)
+    pkg.grow_rounds(ma, a, params, 3)
+    pkg.grow_evotree(ma, a, params)
+    for _ in range(4):
+        mask, js = pkg.sample_round(b, params)
+        mb.trees.append(pkg.grow_tree(b, params, mask, js, True))
+    for ta, tb in zip(ma.trees, mb.trees):
+        assert all(np.array_equal(getattr(ta, k), getattr(tb, k)) for k in ("feat", "cond_bin", "w", "pred"))
+    assert np.array_equal(a.pred(), b.pred())
+    assert np.array_equal(a.rng.integers(0, 256, 9, dtype=np.uint8), b.rng.integers(0, 256, 9, dtype=np.uint8))
+    a.close()
+    b.close()
