@@ -13,8 +13,6 @@ static const char *const g_timer_names[EVB_NTIMERS] = {"evb:grads", "evb:rows_in
 
 int32_t evb_launch_check_bins(evb_handle *h);
 int32_t evb_launch_init_state(evb_handle *h, const float *w_dev, const float *pred0_dev, const float *mu_dev);
-int32_t evb_launch_root_plan(evb_handle *h);
-int32_t evb_hist_geometry(const evb_handle *h, int F, HistGeom *g);
 int32_t evb_nccl_check(evb_handle *h);
 
 static thread_local char g_err[512] = "";
@@ -150,10 +148,9 @@ static void free_handle(evb_handle *h) {
     evb_dev_free(h->hsum);
     if (exported) { evb_dev_free(h->hcomp, true); h->hcomp = nullptr; }
     free_eval(h);
-    void *ptrs[] = {h->xH, h->xE, h->hsum_q, h->hcnt_q, h->qs_cnt, h->qs_prefix, h->qs_rank, h->qs_gamma, h->gradq, h->d_gmax, h->d_qinv, h->xT, h->xC, h->grad, h->pred, h->y, h->nidx, h->rows[0], h->rows[1], h->mask_d, h->feattypes_d, h->mono_d,
-                    h->gen_d, h->seg_start, h->seg_cnt, h->gcnt, h->nleft, (h->gnleft != h->nleft) ? h->gnleft : nullptr, h->kind,
-                    h->bslot, h->nsum, h->plan /* base of the tree block */, h->cum, h->slot_node, h->item_node, h->item_left,
-                    h->item_lprefix, h->item_bits, h->scan_tmp, h->hist, h->hcomp, h->scratch, h->fbest_gain, h->fbest_bin, h->obl_gain, h->obl_best, h->edges_d};
+    void *ptrs[] = {h->xH, h->xE, h->hsum_q, h->hcnt_q, h->qs_cnt, h->qs_prefix, h->qs_rank, h->qs_gamma, h->gradq, h->d_gmax, h->d_qinv, h->cur_l, h->cur_r, h->ticket, h->pl, h->xT, h->xC, h->grad, h->pred, h->y, h->nidx, h->rows[0], h->rows[1], h->mask_d, h->feattypes_d, h->mono_d,
+                    h->gen_d, h->seg_start, h->seg_cnt, h->kind,
+                    h->bslot, h->nsum, h->plan /* base of the tree block */, h->cum, h->slot_node, h->scan_tmp, h->hist, h->hcomp, h->fbest_gain, h->fbest_bin, h->fbest_left, h->obl_gain, h->obl_best, h->edges_d};
     phase("exchange buffers");
     for (void *p : ptrs) evb_dev_free(p);
     phase("device buffers");
@@ -191,26 +188,15 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     h->p = *p;
     h->K = p->K; h->C = 2 * p->K + 1; h->B = p->nbins; h->D = p->max_depth; h->nn = (1 << p->max_depth) - 1;
     h->Ce = (p->loss == EVB_MSE && !getenv("EVB_NO_ELISION")) ? p->K + 1 : h->C;
-    h->nfeats = nfeats; h->RS = (nfeats + 31) / 32 * 32; h->GS = (h->Ce + 3) / 4 * 4; h->n = nobs;
+    h->nfeats = nfeats; h->RS = nfeats <= 16 ? 16 : (nfeats + 31) / 32 * 32; h->GS = (h->Ce + 3) / 4 * 4; h->n = nobs;
     { const int nct = (h->Ce + 3) / 4; h->rec_nch = (h->Ce + nct - 1) / nct; }
-    // mse with one target runs the fixed-point histogram kernel (EVB_HIST_Q=0: the float kernel)
-    { const char *e = getenv("EVB_HIST_Q"); h->use_q = p->loss == EVB_MSE && p->K == 1 && h->Ce == 2 && !(e && atoi(e) == 0); }
     h->unit_w = w == nullptr;
-    h->wscale = 1.0f; h->winv = 1.0;
-    if (h->use_q && w) {
-        float wmax = 0.0f;
-        for (int64_t i = 0; i < nobs; ++i) wmax = w[i] > wmax ? w[i] : wmax;
-        if (wmax > 0.0f && wmax < INFINITY) {
-            int e;
-            frexpf(wmax, &e);
-            h->wscale = ldexpf(1.0f, 29 - e);
-            h->winv = ldexp(1.0, e - 29);
-        }
-    }
+    h->ng = h->Ce - 1;                       // gradients (and hessians where they are not 2w)
+    h->nq = h->ng + (h->unit_w ? 0 : 1);     // weights are a channel of their own, row counts are not
+    h->SC = (nfeats + 3) / 4 * 4;
     h->dev = p->device; h->y_dtype = y_dtype; h->ycols = ycols;
     h->timing = (p->flags & EVB_FLAG_TIMING) != 0;
     h->world = 1; h->rank = 0; h->F = nfeats;
-    h->hist_mode = evb_hist_mode_env();
     int cc_major = 0, cc_minor = 0; // single attributes: cudaGetDeviceProperties queries everything and takes milliseconds
     EVB_CUDA(cudaDeviceGetAttribute(&cc_major, cudaDevAttrComputeCapabilityMajor, h->dev));
     EVB_CUDA(cudaDeviceGetAttribute(&cc_minor, cudaDevAttrComputeCapabilityMinor, h->dev));
@@ -224,7 +210,6 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     const int64_t n = nobs;
     const int nids = h->nn + 2, C = h->C, K = h->K, D = h->D;
 
-    EVB_CUDA(dalloc(&h->xT, (size_t)n * h->RS));
     EVB_CUDA(dalloc(&h->grad, (size_t)n * h->GS));
     if (p->loss == EVB_QUANTILE || p->loss == EVB_MULTIQUANTILE) {
         const size_t e = (size_t)2 * (h->nn + 1);
@@ -232,14 +217,14 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
         EVB_CUDA(dalloc(&h->qs_gamma, (size_t)h->nn + 1));
         EVB_CUDA(cudaMemset(h->qs_cnt, 0, e * 256 * sizeof(uint32_t)));
     }
-    // unit weights: the register-direct kernel (EVB_HIST_Q2=0: the staged fixed-point kernel)
-    { const char *e = getenv("EVB_HIST_Q2"); h->use_q2 = h->use_q && h->unit_w && !(e && atoi(e) == 0) && evb_q2_configure(h) == EVB_OK; }
-    if (h->use_q) {
-        if (!h->use_q2) EVB_CUDA(dalloc(&h->gradq, (size_t)n * (h->unit_w ? 1 : 2)));
-        EVB_CUDA(dalloc(&h->d_gmax, (size_t)1));
-        EVB_CUDA(dalloc(&h->d_qinv, (size_t)2));
-        EVB_CUDA(cudaMemset(h->d_gmax, 0, sizeof(unsigned)));
+    EVB_CHECK(evb_hg_configure(h));
+    h->use_q2 = evb_q2_wanted(h) && evb_q2_configure(h) == EVB_OK;
+    if (!h->use_q2) {
+        EVB_CUDA(dalloc(&h->xT, (size_t)n * h->RS));
+        EVB_CUDA(dalloc(&h->gradq, evb_hg_q_words(h)));
     }
+    EVB_CUDA(dalloc(&h->d_gmax, (size_t)h->nq));
+    EVB_CUDA(dalloc(&h->d_qinv, (size_t)h->nq));
     EVB_CUDA(dalloc(&h->pred, (size_t)n * K));
     EVB_CUDA(dalloc(&h->nidx, (size_t)n));
     EVB_CUDA(dalloc(&h->rows[0], (size_t)n));
@@ -250,11 +235,10 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     EVB_CUDA(dalloc(&h->gen_d, (size_t)EVB_GEN_WORDS / 2 + (nfeats + 1) / 2));
     h->js_d = reinterpret_cast<uint32_t *>(h->gen_d) + EVB_GEN_WORDS;
     EVB_CUDA(dalloc(&h->seg_start, (size_t)nids)); EVB_CUDA(dalloc(&h->seg_cnt, (size_t)nids));
-    EVB_CUDA(dalloc(&h->gcnt, (size_t)nids)); EVB_CUDA(dalloc(&h->nleft, (size_t)nids));
-    h->gnleft = h->nleft;
+    EVB_CUDA(dalloc(&h->cur_l, (size_t)nids)); EVB_CUDA(dalloc(&h->cur_r, (size_t)nids));
+    EVB_CUDA(dalloc(&h->ticket, (size_t)nids));
     EVB_CUDA(dalloc(&h->kind, (size_t)nids)); EVB_CUDA(dalloc(&h->bslot, (size_t)nids));
     EVB_CUDA(dalloc(&h->nsum, (size_t)nids * C));
-    EVB_CUDA(cudaMemset(h->nleft, 0, sizeof(int32_t) * nids));
 
     const TreeBlockLayout L = tree_block_layout(D, h->nn, K);
     unsigned char *blk = nullptr;
@@ -275,14 +259,12 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
 
     h->maxslots = evb_level_slots(D > 1 ? D - 1 : 1);
     EVB_CUDA(dalloc(&h->cum, (size_t)h->maxslots + 1)); EVB_CUDA(dalloc(&h->slot_node, (size_t)h->maxslots));
-    h->max_items = (int)(n / EVB_PART_CHUNK) + (1 << (D > 1 ? D - 1 : 0)) + 2;
-    EVB_CUDA(dalloc(&h->item_node, (size_t)(1 << D) + 2));
-    EVB_CUDA(dalloc(&h->item_left, (size_t)h->max_items)); EVB_CUDA(dalloc(&h->item_lprefix, (size_t)h->max_items));
-    EVB_CUDA(dalloc(&h->item_bits, (size_t)h->max_items * (EVB_PART_CHUNK / 32)));
+    EVB_CUDA(dalloc(&h->pl, ((size_t)h->maxslots + 1) * 4));
     EVB_CUDA(dalloc(&h->scan_tmp, (size_t)(n / 2048 + 2)));
     {
         const size_t lv = (size_t)evb_level_nodes(D > 1 ? D - 1 : 1) * nfeats;
         EVB_CUDA(dalloc(&h->fbest_gain, lv)); EVB_CUDA(dalloc(&h->fbest_bin, lv));
+        if (C == 3) EVB_CUDA(dalloc(&h->fbest_left, lv * 3));
         if (p->tree_type == 1) {
             EVB_CUDA(dalloc(&h->obl_gain, ((size_t)evb_level_nodes(D > 1 ? D - 1 : 1) + 1) * nfeats * h->B));
             EVB_CUDA(dalloc(&h->obl_best, (size_t)2));
@@ -293,22 +275,21 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     h->hist_nodes = keep_all ? (1 << (D > 1 ? D - 1 : 0)) : (D >= 2 ? 1 << (D - 2) : 1);
     const size_t FCB = (size_t)nfeats * C * h->B;
     EVB_CUDA(dalloc(&h->hist, (size_t)h->hist_nodes * FCB));
-    EVB_CUDA(dalloc(&h->hcomp, (size_t)h->maxslots * FCB));
-    EVB_CHECK(evb_hist_configure(h));
-    EVB_CUDA(dalloc(&h->scratch, h->scratch_floats));
+    {
+        const size_t acc = (size_t)h->maxslots * h->B * h->SC;
+        EVB_CUDA(dalloc(&h->hsum_q, acc * h->nq));
+        EVB_CUDA(dalloc(&h->hcnt_q, acc));
+        EVB_CUDA(cudaMemsetAsync(h->hsum_q, 0, acc * h->nq * sizeof(unsigned long long), h->st));
+        EVB_CUDA(cudaMemsetAsync(h->hcnt_q, 0, acc * sizeof(uint32_t), h->st));
+    }
 
     // ---- uploads: x_bin is kept feature-major (as given) for the row partition and transposed on the device to
     // observation-major rows for the histogram gathers and the tree traversal
     phase("allocations");
     EVB_CUDA(dalloc(&h->xC, (size_t)n * nfeats));
     if (h->use_q2) {
-        const size_t acc = (size_t)h->maxslots * h->B * h->q2.SC;
         EVB_CUDA(dalloc(&h->xH, (size_t)(n + 1) * h->q2.RSH));
         EVB_CUDA(dalloc(&h->xE, (size_t)n + 1));
-        EVB_CUDA(dalloc(&h->hsum_q, acc));
-        EVB_CUDA(dalloc(&h->hcnt_q, acc));
-        EVB_CUDA(cudaMemsetAsync(h->hsum_q, 0, acc * sizeof(unsigned long long), h->st));
-        EVB_CUDA(cudaMemsetAsync(h->hcnt_q, 0, acc * sizeof(uint32_t), h->st));
     }
     phase("layouts");
     if (mx) {
@@ -322,14 +303,15 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
         EVB_CHECK(evb_matrix_binarize(mx, e, nedges, h->xC, h->xT, h->RS, h->xH, h->use_q2 ? h->q2.RSH : 0, h->xE, h->use_q2 ? h->q2.nmain : nfeats, h->d_err, h->st));
         phase("binarize");
     } else {
-        EVB_CUDA(cudaMemsetAsync(h->xT, 0, (size_t)n * h->RS, h->st));
         if (x_bin) EVB_CHECK(evb_h2d_staged(h->xC, x_bin, (size_t)n * nfeats, h->st));
         else EVB_CHECK(evb_upload_binarize(h, x, x_dtype, edges, nedges));
         phase("upload (+ binarize)");
-        EVB_CHECK(evb_launch_transpose(h, h->xC, n, n, 0, nfeats, h->xT, h->RS, h->st));
-        phase("transpose to xT");
         if (h->use_q2) EVB_CHECK(evb_q2_build_layout(h));
-        phase("chunk rows (xH, xE)");
+        else {
+            EVB_CUDA(cudaMemsetAsync(h->xT, 0, (size_t)n * h->RS, h->st));
+            EVB_CHECK(evb_launch_transpose(h, h->xC, n, n, 0, nfeats, h->xT, h->RS, h->st));
+        }
+        phase("rows of bins");
     }
     {
         const size_t ybytes = (size_t)n * (y_dtype == EVB_U32 ? 4 : 4 * (size_t)ycols);
@@ -459,6 +441,8 @@ extern "C" int32_t evb_comm_init(evb_handle *h, const uint8_t id[128], int32_t r
     if (!id || world < 1 || rank < 0 || rank >= world) { evb_set_error("evb_comm_init: bad rank/world"); return EVB_ERR_ARG; }
     if (h->nccl_comm || h->nccl_pending) { evb_set_error("evb_comm_init: communicator already initialised"); return EVB_ERR_ARG; }
     if (world == 1) return EVB_OK;
+    if (!h->hcomp) EVB_CUDA(dalloc(&h->hcomp, (size_t)h->maxslots * h->nfeats * h->C * h->B));
+    drop_graphs(h);
     EVB_CHECK(evb_nccl_init(h, id, rank, world));
     return EVB_OK;
 }
@@ -467,22 +451,14 @@ extern "C" int32_t evb_comm_init(evb_handle *h, const uint8_t id[128], int32_t r
 // replayed as one CUDA graph per tree): it must not synchronise and must not touch pageable host memory.
 static int32_t enqueue_tree(evb_handle *h, int use_mask, uint8_t mask_cond, bool run_grads, bool quantize, bool fuse, int slot) {
     const int D = h->D;
-    EVB_CUDA(cudaMemcpyAsync(h->gen_d, h->h_js[slot], sizeof(uint32_t) * (EVB_GEN_WORDS + h->F), cudaMemcpyHostToDevice, h->st));
     if (run_grads) EVB_CHECK(evb_launch_grads(h));
-    if (quantize) EVB_CHECK(h->use_q2 ? evb_launch_q2_quantize(h) : evb_launch_quantize(h)); // fixed-point histogram kernel: the gradients changed since the last tree
-    EVB_CHECK(evb_launch_tree_reset(h));
+    EVB_CHECK(evb_launch_tree_begin(h, quantize, use_mask == EVB_MASK_NONE, h->h_js[slot]));
     EVB_CHECK(evb_launch_rows_init(h, use_mask, mask_cond));
-    EVB_CHECK(evb_launch_root_plan(h));
     const int last = D > 1 ? D - 1 : 1;
     const bool full_part = (h->p.flags & EVB_FLAG_FULL_PARTITION) != 0;
     for (int level = 1; level <= last; ++level) {
-        if (h->use_q2) {
-            EVB_CHECK(evb_launch_histq2(h, level));
-            if (!evb_q2_direct(h)) EVB_CHECK(evb_launch_q2_reduce(h, level));
-        } else {
-            EVB_CHECK(evb_launch_hist(h, level));
-            EVB_CHECK(evb_launch_hist_reduce(h, level));
-        }
+        EVB_CHECK(h->use_q2 ? evb_launch_histq2(h, level) : evb_launch_histg(h, level));
+        if (!evb_acc_direct(h)) EVB_CHECK(evb_launch_acc_to_hcomp(h, level));
         if (h->world > 1 && !h->p2p) { // with peer access the ranks' histograms are summed inside the split scan instead
             evb_tic(h, EVB_T_ALLREDUCE);
             int32_t s = evb_nccl_allreduce_f64(h, h->hcomp, (size_t)evb_level_slots(level) * h->F * h->C * h->B);
@@ -490,19 +466,20 @@ static int32_t enqueue_tree(evb_handle *h, int use_mask, uint8_t mask_cond, bool
             EVB_CHECK(s);
         }
         EVB_CHECK(evb_launch_scan(h, level));
-        if (evb_q2_direct(h)) EVB_CHECK(evb_launch_q2_clear(h, level));
-        if (level < D - 1 || (full_part && level == D - 1)) EVB_CHECK(evb_launch_partition(h, level));
+        if (level < D - 1 || (full_part && level == D - 1)) EVB_CHECK(evb_launch_partition(h, level)); // clears the accumulators too
+        else if (evb_acc_direct(h)) EVB_CHECK(evb_launch_acc_clear(h, level));
     }
+    // the last kernel of the tree writes it to pinned memory
+    void *pub = h->ev_n > 0 ? nullptr : h->h_tree[slot];
     if (h->p.loss == EVB_QUANTILE || h->p.loss == EVB_MULTIQUANTILE) {
         // the leaf values need the leaf of every row first: leaf ids, per-leaf quantiles, then the usual update
-        EVB_CHECK(evb_launch_finalize(h, false, 1));
+        EVB_CHECK(evb_launch_finalize(h, false, 1, nullptr));
         EVB_CHECK(evb_launch_quantile_leaves(h, use_mask != EVB_MASK_NONE, mask_cond));
-        EVB_CHECK(evb_launch_finalize(h, fuse, 2));
+        EVB_CHECK(evb_launch_finalize(h, fuse, 2, pub));
     } else {
-        EVB_CHECK(evb_launch_finalize(h, fuse, 0));
+        EVB_CHECK(evb_launch_finalize(h, fuse, 0, pub));
     }
-    if (h->ev_n > 0) EVB_CHECK(evb_launch_eval(h, nullptr));
-    EVB_CUDA(cudaMemcpyAsync(h->h_tree[slot], h->plan, h->h_tree_bytes, cudaMemcpyDeviceToHost, h->st));
+    if (h->ev_n > 0) EVB_CHECK(evb_launch_eval(h, nullptr, h->h_tree[slot]));
     return EVB_OK;
 }
 
@@ -528,25 +505,9 @@ static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen,
         h->h_js[slot][EVB_GEN_WORDS + i] = js[i] - 1;
     }
     if (h->world > 1) EVB_CHECK(evb_nccl_check(h));
-    if (njs != h->F && h->use_q2) { // this kernel always accumulates all features; the scan reads the sampled ones
+    if (njs != h->F) { // the histogram kernels always accumulate all features; the scan reads the sampled ones
         EVB_CUDA(cudaStreamSynchronize(h->st));
         h->F = njs;
-        drop_graphs(h);
-    }
-    if (njs != h->F) {
-        HistGeom g;
-        EVB_CUDA(cudaStreamSynchronize(h->st));
-        h->F = njs;
-        EVB_CHECK(evb_hist_geometry(h, njs, &g));
-        const size_t need = (size_t)g.NUG * g.PG * g.UB * g.img_floats;
-        if (need > h->scratch_floats) {
-            evb_dev_free(h->scratch);
-            h->scratch = nullptr;
-            EVB_CUDA(dalloc(&h->scratch, need));
-            h->scratch_floats = need;
-        }
-        h->hg = g;
-        h->q_active = g.q;
         drop_graphs(h);
     }
     if (update_grads) h->bag_idx = 0;
@@ -570,7 +531,7 @@ static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen,
     // One CUDA graph per variant of the launch sequence, captured on the second call of a variant (the first
     // one runs directly: it also sets function attributes).  Per-kernel timing needs the direct path.
     if (update_grads) h->gradq_valid = false;
-    const bool quantize = (h->q_active || h->use_q2) && !h->gradq_valid;
+    const bool quantize = !h->gradq_valid;
     if (quantize) h->gradq_valid = true;
     const int key = (use_mask ? 1 : 0) | (use_mask == EVB_MASK_PCG ? 32 : 0) | (run_grads ? 2 : 0) | (fuse ? 4 : 0) | (slot ? 8 : 0) | (quantize ? 16 : 0);
     if (h->graph_mask_cond != (int)mask_cond) { drop_graphs(h); h->graph_mask_cond = mask_cond; }
@@ -717,7 +678,7 @@ static int32_t eval_attach_impl(evb_handle *h, int64_t nobs, const uint8_t *x_bi
         std::vector<float> leaf(K, 0.0f);
         if (bias) memcpy(leaf.data(), bias, sizeof(float) * K);
         if (dalloc(&leaf_d, (size_t)K) != cudaSuccess || cudaMemcpyAsync(leaf_d, leaf.data(), sizeof(float) * K, cudaMemcpyHostToDevice, h->st) != cudaSuccess) rc = EVB_ERR_CUDA;
-        if (rc == EVB_OK) rc = evb_launch_eval(h, leaf_d);
+        if (rc == EVB_OK) rc = evb_launch_eval(h, leaf_d, nullptr);
         if (rc == EVB_OK && cudaMemcpyAsync(h->last_eval, h->d_evsum, sizeof(h->last_eval), cudaMemcpyDeviceToHost, h->st) != cudaSuccess) rc = EVB_ERR_CUDA;
     }
     cudaError_t e = cudaStreamSynchronize(h->st);

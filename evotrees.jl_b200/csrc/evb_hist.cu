@@ -21,6 +21,25 @@
 #include <mutex>
 #include <stdlib.h>
 
+constexpr int EVB_MAX_UNITS_PER_BLOCK = 4;
+
+struct HistGeom {
+    int BP;        // padded bins per image: 32/64/128/256
+    int NCH;       // channels per unit image (<= 4)
+    int FPL;       // feature slots per lane (1, 2 or 4): a unit covers 32 * FPL feature slots
+    int NFG;       // feature groups of 32 * FPL slots
+    int NCT;       // channel groups of 4
+    int U;         // units = NFG*NCT
+    int UB;        // units (consumer warps) per block
+    int NUG;       // unit groups = ceil(U/UB)
+    int stages;    // staged tiles in flight
+    int G;         // row-range blocks (grid.x)
+    int PG;        // piece slots per unit group = G + max build slots
+    size_t smem;   // dynamic shared memory per block
+    size_t img_floats;   // floats per unit image in scratch: FPL*NCH*nbins*32
+};
+
+
 namespace {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -418,440 +437,6 @@ __global__ void __launch_bounds__((EVB_MAX_UNITS_PER_BLOCK + 1) * 32) k_hist(His
     }
 }
 
-// ---------------------------------------------------------------------------------------------------------
-// Fixed-point variant for mse with one target.  The quantisation kernel turns the gradient of every row into a
-// fixed-point number q = rint(g * 2^s), |q| < 2^29 (and the weight likewise, unless no weights were given: the w
-// channel is then a row count).  The kernel splits q into hi = q >> 15 (signed) and lo = q & 0x7fff and adds the
-// NW words (hi, lo, 1) or (hi, lo, w_hi, w_lo) into the image [word][bin][lane] of the unit with
-// `red.shared.add.u32`: one shared-memory pass per word and row, no read-modify-write chain.  Integer sums do not
-// depend on the order of the rows, so
-//   * several warps share one image: a CTA (one per SM) keeps a single image per unit of 32 feature slots;
-//   * the shared memory that the float variant spends on one image per warp holds row data in flight instead.
-//     The warps form QT teams with one warp per unit.  The teams take the 32-row tiles of the CTA's row range in
-//     turn; a team stages its tile together with cp.async -- eight adjacent lanes copy the 128 bytes of one row,
-//     so a copy instruction touches 4 lines instead of 32 -- into a ring QDR tiles deep (+1 slot so that one
-//     named barrier per tile is enough), waits with cp.async.wait_group and the team barrier, and then every warp
-//     adds the tile into the image of its unit.  There is no producer warp and no mbarrier.
-//     Row r of a tile is stored rotated by 32 * (r & 3) bytes inside its 128 bytes, so that the four rows which
-//     the consumers read with one load fall into different banks.
-// A piece covers at most 2^17 rows, so neither the sum of the lo words (< 2^32) nor of the hi words (|.| < 2^31)
-// can overflow.  The reduce kernel recombines hi * 2^15 + lo in 64-bit integers and scales by 2^-s: every
-// histogram entry is the exact sum of the quantised gradients, whatever the order and the number of pieces.
-// Needs feature slot s == feature s (no column sample): the unit's bins are then 32 adjacent bytes of a row.
-constexpr int QT = 6;                   // teams per CTA
-constexpr int QDR = 5;                  // tiles in flight per team
-constexpr int QSPLIT = 15;              // scratch words: sum = hi * 2^15 + lo, a piece may hold 2^17 rows (|q| < 2^29)
-// Unit weights (NW == 3): the image has two planes only.  q (|q| < 2^26) is split at bit 8 and the row count rides in
-// the upper 12 bits of the lo word: plane 0 += q >> 8, plane 1 += (q & 0xff) | 1 << 20.  That holds QSUB * QT tiles
-// (at most 4095 rows: lo sum < 2^20, count < 2^12, |hi sum| < 2^30); then the image is flushed into the piece's scratch
-// words (hi, lo, count as above), which are private to the CTA (first flush: stores, later ones: red.global.add).
-constexpr int QSUB = 4095 / (QT * EVB_TILE_ROWS); // tiles per team between two flushes
-__host__ __device__ constexpr int q_planes(int NW) { return NW == 3 ? 2 : 4; }
-__host__ __device__ constexpr int q_tile_bytes(int NW) { return EVB_TILE_ROWS * (128 + (NW == 3 ? 4 : 8)); } // bins + q (+ q of w)
-
-template <uint32_t OFF>
-__device__ __forceinline__ void red_off(uint32_t addr, uint32_t v) {
-    asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(addr), "r"(v), "n"(OFF) : "memory");
-}
-// the words that one row adds to the image: (q >> 8, (q & 0xff) | 1 << 20) without weights, else hi / lo of g and w
-template <int NW>
-__device__ __forceinline__ void row_words(uint32_t qg, uint32_t qw, uint32_t (&w)[4]) {
-    if constexpr (NW == 3) {
-        w[0] = (uint32_t)((int32_t)qg >> 8); w[1] = (qg & 0xffu) | (1u << 20); w[2] = 0u; w[3] = 0u;
-    } else {
-        w[0] = (uint32_t)((int32_t)qg >> QSPLIT); w[1] = qg & ((1u << QSPLIT) - 1);
-        w[2] = qw >> QSPLIT; w[3] = qw & ((1u << QSPLIT) - 1);
-    }
-}
-// adds them into the word planes of the image (plane k starts k * WSZ bytes further)
-template <int NW, uint32_t WSZ>
-__device__ __forceinline__ void red_row(uint32_t addr, const uint32_t (&w)[4]) {
-    red_off<0>(addr, w[0]);
-    red_off<WSZ>(addr, w[1]);
-    if constexpr (NW == 4) { red_off<2 * WSZ>(addr, w[2]); red_off<3 * WSZ>(addr, w[3]); }
-}
-// All rows of one staged tile.  4 * REP rows at a time.  With REP = 1 lane (k = lane & 7, rr = lane >> 3) loads the
-// 32-bit word with the bins of features 4k .. 4k+3 of row r + rr -- one conflict-free load brings the 128 bins of
-// four rows -- and the fixed-point words of that row.  In step j = 0..3 the lane adds its row into feature
-// 4k + ((j + rr) & 3): the four lanes that share k work on four different features, so the 32 lanes of every
-// reduction hit 32 different banks.  A unit with few features (the last one: 8 / REP groups of four features or
-// fewer) keeps REP replicas of its columns instead, k = lane % (8 / REP), rr = lane / (8 / REP), replica rr >> 2,
-// and takes 4 * REP rows per step; the replicas are added when the image is flushed.
-//   tb: shared-space address of the lane's word of row rr of the tile, tw: of the tile's words + rr * (4 or 8),
-//   col[j]: image column of the lane's feature of step j, sel[j]: PRMT selector of that feature's byte.
-template <uint32_t OFF>
-__device__ __forceinline__ uint32_t lds_u32_at(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFF));
-    return v;
-}
-// batch BT of a tile (see q_tile): loads of batch BT + 1 first, then the reductions of batch BT
-template <int NW, uint32_t WSZ, int REP, bool FULL, int BT>
-__device__ __forceinline__ void q_batch(uint32_t tb, uint32_t tw, int nrows, int rr, const uint32_t (&col)[4], const uint32_t (&sel)[4],
-                                        uint32_t bins, uint32_t qg, uint32_t qw) {
-    constexpr int RW = NW == 3 ? 1 : 2;
-    constexpr int RB = 4 * REP, NB = EVB_TILE_ROWS / RB;
-    uint32_t nbins = 0, nqg = 0, nqw = 0;
-    if constexpr (BT + 1 < NB) {
-        nbins = lds_u32_at<(BT + 1) * RB * 128>(tb);
-        nqg = lds_u32_at<(BT + 1) * RB * 4 * RW>(tw);
-        if constexpr (RW == 2) nqw = lds_u32_at<(BT + 1) * RB * 8 + 4>(tw);
-    }
-    if (FULL || BT * RB + rr < nrows) { // FULL: a whole tile of 32 rows, nothing to test
-        uint32_t w[4];
-        row_words<NW>(qg, qw, w);
-        if constexpr (NW == 3) {
-            // the four steps of the lane's row as one block: byte select, image address, two reductions each
-            asm volatile(
-                "{\n .reg .u32 b0, b1, b2, b3, a0, a1, a2, a3;\n"
-                " prmt.b32 b0, %0, 0, %1;\n prmt.b32 b1, %0, 0, %2;\n prmt.b32 b2, %0, 0, %3;\n prmt.b32 b3, %0, 0, %4;\n"
-                " mad.lo.u32 a0, b0, 128, %5;\n mad.lo.u32 a1, b1, 128, %6;\n mad.lo.u32 a2, b2, 128, %7;\n mad.lo.u32 a3, b3, 128, %8;\n"
-                " red.shared.add.u32 [a0], %9;\n red.shared.add.u32 [a0+%11], %10;\n"
-                " red.shared.add.u32 [a1], %9;\n red.shared.add.u32 [a1+%11], %10;\n"
-                " red.shared.add.u32 [a2], %9;\n red.shared.add.u32 [a2+%11], %10;\n"
-                " red.shared.add.u32 [a3], %9;\n red.shared.add.u32 [a3+%11], %10;\n}\n"
-                ::"r"(bins), "r"(sel[0]), "r"(sel[1]), "r"(sel[2]), "r"(sel[3]), "r"(col[0]), "r"(col[1]), "r"(col[2]), "r"(col[3]),
-                  "r"(w[0]), "r"(w[1]), "n"(WSZ)
-                : "memory");
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) red_row<NW, WSZ>(col[j] + __byte_perm(bins, 0u, sel[j]) * 128u, w);
-        }
-    }
-    if constexpr (BT + 1 < NB) q_batch<NW, WSZ, REP, FULL, BT + 1>(tb, tw, nrows, rr, col, sel, nbins, nqg, nqw);
-}
-template <int NW, uint32_t WSZ, int REP, bool FULL>
-__device__ __forceinline__ void q_tile(uint32_t tb, uint32_t tw, int nrows, int rr, const uint32_t (&col)[4], const uint32_t (&sel)[4]) {
-    constexpr int RW = NW == 3 ? 1 : 2;
-    const uint32_t bins = lds_u32(tb), qg = lds_u32(tw), qw = RW == 2 ? lds_u32(tw + 4) : 0u;
-    q_batch<NW, WSZ, REP, FULL, 0>(tb, tw, nrows, rr, col, sel, bins, qg, qw);
-}
-
-template <int BP, int NW>
-__global__ void __launch_bounds__(EVB_MAX_UNITS_PER_BLOCK * QT * 32) k_histq(HistArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    constexpr uint32_t WSZ = (BP + 1) * 128;    // bytes of one word plane [bin 0..BP][lane]
-    constexpr uint32_t IMG = q_planes(NW) * WSZ;
-    constexpr int QTILE = q_tile_bytes(NW), RW = NW == 3 ? 1 : 2, NSLOT = QDR + 1;
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    const int G = gridDim.x, b = blockIdx.x, ug = blockIdx.y;
-    const int nact = min(a.UB, a.U - ug * a.UB);
-    const long long R = a.plan->R;
-    const long long lo = R * b / G, hi = R * (b + 1) / G;
-    if (lo >= hi) return;
-    uint32_t *imgs = reinterpret_cast<uint32_t *>(smem);
-    for (int i = tid; i < a.UB * (int)(IMG / 4); i += blockDim.x) imgs[i] = 0u;
-    __syncthreads();
-    const int team = wid / a.UB, uw = wid % a.UB;
-    if (uw >= nact) return;
-
-    const int nbuild = a.plan->nbuild;
-    int s;
-    {
-        int l = 0, r = nbuild - 1;
-        while (l < r) { int m = (l + r + 1) >> 1; if ((long long)a.cum[m] <= lo) l = m; else r = m - 1; }
-        s = l;
-    }
-    const int fg = ug * a.UB + uw;          // the unit: feature slots fg*32 .. fg*32+31
-    const uint32_t u0 = smem_u32(smem) + (uint32_t)uw * IMG + lane * 4; // column of feature slot `lane` (flush)
-    // groups of four features in this unit -> replicas of its columns (see q_tile)
-    const int nq = min(8, (a.F - fg * 32 + 3) / 4);
-    const int rep = nq <= 1 ? 8 : nq <= 2 ? 4 : nq <= 4 ? 2 : 1, nqp = 8 / rep;
-    const int k = lane % nqp, rr = lane / nqp;
-    uint32_t col[4], sel[4];
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-        const int sh = (jj + rr) & 3;
-        col[jj] = smem_u32(smem) + (uint32_t)uw * IMG + (uint32_t)((rr >> 2) * nqp * 4 + 4 * k + sh) * 4;
-        sel[jj] = 0x4440u | (uint32_t)sh;
-    }
-    unsigned char *ring = smem + (size_t)a.UB * IMG + (size_t)team * (NSLOT * QTILE);
-    const uint32_t ring_s = smem_u32(ring);
-    // the lane's word of row rr inside a tile (rows are rotated by 32 * (row & 3) bytes)
-    const uint32_t rd_off = (uint32_t)rr * 128u + ((uint32_t)(uw * 32 + k * 4 + 32 * (rr & 3)) & 127u);
-    // staging: the team copies 32 rows x nact * 32 bytes of bins as 16-byte chunks, two per lane
-    const int cpr = 2 * nact;               // chunks per row
-    int st_row[2], st_src[2], st_dst[2];
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int c = t * nact * 32 + uw * 32 + lane;
-        st_row[t] = c / cpr;
-        const int pch = c % cpr;
-        st_src[t] = pch * 16;
-        st_dst[t] = st_row[t] * 128 + ((pch + 2 * (st_row[t] & 3)) & 7) * 16;
-    }
-    const uint8_t *xsl = a.xT + (size_t)ug * a.UB * 32;  // the CTA's slice of every row of bins
-    const int32_t *gq = reinterpret_cast<const int32_t *>(a.grad);
-    const size_t RS = a.RS;
-    const uint32_t team_bar = 1 + team, unit_bar = 1 + QT + uw;
-#ifdef EVB_DIAG
-    const bool skip_acc = (a.mode & 16) != 0; // profiling builds only: stage the rows, skip the accumulation
-#else
-    constexpr bool skip_acc = false;
-#endif
-    const int team_threads = nact * 32;
-
-    long long pos = lo;
-    while (pos < hi) {
-        const long long send = min(hi, (long long)a.cum[s + 1]);
-        if (send > pos) {
-            const uint32_t *rows = a.rows + ((long long)a.seg_start[a.slot_node[s]] - a.cum[s]);
-            const long long ntiles = (send - pos + EVB_TILE_ROWS - 1) / EVB_TILE_ROWS;
-            const int nmine = ntiles > team ? (int)((ntiles - team + QT - 1) / QT) : 0; // tiles team, team + QT, ...
-            // All warps of the unit are done with the rows so far: move the image into the scratch words of the piece
-            // (CTA b, slot s) and clear it.  `first`: the piece has no contents yet (store instead of add).
-            bool started = false;
-            auto flush = [&](bool first) {
-                asm volatile("bar.sync %0, %1;" ::"r"(unit_bar), "r"(QT * 32) : "memory");
-                uint32_t *dst = reinterpret_cast<uint32_t *>(a.scratch) + ((size_t)(ug * a.PG + b + s) * a.UB + uw) * a.img_floats + lane;
-                const int pl = a.nbins * 32; // words per scratch plane
-                if constexpr (NW == 3) {
-                    if (team == 0) { // guard rows
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(u0), "r"(0u) : "memory");
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(u0 + WSZ), "r"(0u) : "memory");
-                    }
-                    for (int bin = team; bin < a.nbins; bin += QT) {
-                        const uint32_t ai = u0 + (uint32_t)(bin + 1) * 128u;
-                        uint32_t vh = lds_u32(ai), vp = lds_u32(ai + WSZ);
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(ai), "r"(0u) : "memory");
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(ai + WSZ), "r"(0u) : "memory");
-                        for (int o = 32 / rep; o < 32; o <<= 1) { vh += __shfl_xor_sync(0xffffffffu, vh, o); vp += __shfl_xor_sync(0xffffffffu, vp, o); }
-                        const long long sum = (long long)(int32_t)vh * 256 + (long long)(vp & 0xfffffu);
-                        uint32_t h = (uint32_t)(int32_t)(sum >> QSPLIT), l = (uint32_t)(sum & ((1 << QSPLIT) - 1)), c = vp >> 20;
-                        uint32_t *d = dst + bin * 32;
-                        if (first) { d[0] = h; d[pl] = l; d[2 * pl] = c; }
-                        else { // nothing waits for the result: reductions into words that only this thread touches
-                            asm volatile("red.global.add.u32 [%0], %1;" ::"l"(d), "r"(h) : "memory");
-                            asm volatile("red.global.add.u32 [%0], %1;" ::"l"(d + pl), "r"(l) : "memory");
-                            asm volatile("red.global.add.u32 [%0], %1;" ::"l"(d + 2 * pl), "r"(c) : "memory");
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int q = 0; q < NW; ++q) {
-                        if (team == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(u0 + q * WSZ), "r"(0u) : "memory"); // guard row
-                        for (int bin = team; bin < a.nbins; bin += QT) {
-                            const uint32_t ai = u0 + q * WSZ + (uint32_t)(bin + 1) * 128u;
-                            uint32_t v = lds_u32(ai);
-                            asm volatile("st.shared.u32 [%0], %1;" ::"r"(ai), "r"(0u) : "memory");
-                            for (int o = 32 / rep; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o); // add the replicas
-                            dst[(q * a.nbins + bin) * 32] = v;
-                        }
-                    }
-                }
-                asm volatile("bar.sync %0, %1;" ::"r"(unit_bar), "r"(QT * 32) : "memory");
-            };
-            // Everything below counts in 32-bit offsets from the start of the segment (a row range of a CTA is short).
-            const int seglen = (int)(send - pos), ntl = (int)ntiles;
-            const uint32_t *rows_seg = rows + pos;
-            // row id of row `lane` of the tile at offset o (0 beyond the end of the segment: never copied)
-            auto rid_at = [&](int o) -> uint32_t { return o + lane < seglen ? rows_seg[o + lane] : 0u; };
-            const int step = QT * EVB_TILE_ROWS;
-            int so = team * EVB_TILE_ROWS;       // offset of the tile staged next
-            int co = so;                          // offset of the tile consumed next
-            uint32_t r0 = rid_at(so), r1 = rid_at(so + step);
-            int sslot = 0, cslot = 0, c = 0, until_flush = QSUB;
-            for (int i = 0; i < nmine + QDR - 1; ++i) {
-                const uint32_t r2 = rid_at(so + 2 * step);
-                if (i < nmine) { // stage the team's tile i
-                    const int nrows = min(EVB_TILE_ROWS, seglen - so);
-                    unsigned char *dst = ring + sslot * QTILE;
-#pragma unroll
-                    for (int t = 0; t < 2; ++t) {
-                        const uint32_t rid = __shfl_sync(0xffffffffu, r0, st_row[t]);
-                        if (st_row[t] < nrows) cp_async16(dst + st_dst[t], xsl + (size_t)rid * RS + st_src[t]);
-                    }
-                    if (uw == 0 && lane < nrows) {
-                        if constexpr (RW == 1) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + EVB_TILE_ROWS * 128 + lane * 4)), "l"(gq + r0) : "memory");
-                        else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst + EVB_TILE_ROWS * 128 + lane * 8)), "l"(gq + (size_t)r0 * 2) : "memory");
-                    }
-                    sslot = sslot + 1 == NSLOT ? 0 : sslot + 1;
-                }
-                so += step;
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                r0 = r1; r1 = r2;
-                if (i >= QDR - 1) { // consume the team's tile c
-                    asm volatile("cp.async.wait_group %0;" ::"n"(QDR - 1) : "memory");
-                    // the copies of all warps of the team have landed, and everybody is done with tile c - 1
-                    asm volatile("bar.sync %0, %1;" ::"r"(team_bar), "r"(team_threads) : "memory");
-                    const int nrows = min(EVB_TILE_ROWS, seglen - co);
-                    const uint32_t ts = ring_s + cslot * QTILE;
-                    if (!skip_acc) {
-                        const uint32_t tb = ts + rd_off, tw = ts + EVB_TILE_ROWS * 128 + rr * 4 * RW;
-                        if (rep == 1) { if (nrows == EVB_TILE_ROWS) q_tile<NW, WSZ, 1, true>(tb, tw, nrows, rr, col, sel); else q_tile<NW, WSZ, 1, false>(tb, tw, nrows, rr, col, sel); }
-                        else if (rep == 2) q_tile<NW, WSZ, 2, false>(tb, tw, nrows, rr, col, sel);
-                        else if (rep == 4) q_tile<NW, WSZ, 4, false>(tb, tw, nrows, rr, col, sel);
-                        else q_tile<NW, WSZ, 8, false>(tb, tw, nrows, rr, col, sel);
-                    }
-                    cslot = cslot + 1 == NSLOT ? 0 : cslot + 1;
-                    co += step;
-                    ++c;
-                    if constexpr (NW == 3) { // the packed counters are full after QSUB tiles of every team
-                        if (--until_flush == 0) {
-                            until_flush = QSUB;
-                            if (ntl > c * QT) { flush(!started); started = true; }
-                        }
-                    }
-                }
-            }
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            asm volatile("bar.sync %0, %1;" ::"r"(team_bar), "r"(team_threads) : "memory"); // ring free for the next segment
-            flush(!started);
-        }
-        pos = send;
-        ++s;
-    }
-}
-
-struct ReduceQArgs {
-    const uint32_t *scratch;
-    double *hcomp;
-    const LevelPlan *plan;
-    const int32_t *cum;
-    const double *qinv; // [2]: 2^-s of the g words, and of the w words (1 when w is a row count)
-    int G, PG, UB, NFG, F, nbins, NW;
-    uint32_t img_words;
-};
-
-// pieces of build slot s: CTAs bfirst..blast (the CTAs whose row range intersects the slot's rows)
-__device__ __forceinline__ void slot_pieces(const LevelPlan *plan, const int32_t *cum, int s, int G, int &bfirst, int &blast, long long &R) {
-    const int nbuild = plan->nbuild;
-    R = plan->R;
-    bfirst = 0; blast = -1;
-    if (s < nbuild && R > 0) {
-        const long long c0 = cum[s], c1 = cum[s + 1];
-        if (c1 > c0) {
-            bfirst = (int)(((c0 + 1) * G - 1) / R);
-            blast = (int)((c1 * G - 1) / R);
-        }
-    }
-}
-// hcomp[slot][feature][g, h = 2w, w][bin] from the exact integer sums (K = 1; h: src/loss.jl:52)
-__device__ __forceinline__ void store_q(double *hcomp, int s, int F, int nbins, int slotf, int bin, int ch, double v) {
-    double *dst = hcomp + ((size_t)s * F + slotf) * 3 * nbins + bin;
-    if (ch == 0) dst[0] = v;
-    else { dst[(size_t)2 * nbins] = v; dst[nbins] = 2.0 * v; }
-}
-
-// Sums the pieces of every build slot of the fixed-point variant: grid (build slots of the level, NFG * 2 channels,
-// ceil(nbins / BPB)), 512 threads = NPG piece groups x (BPB bins x 32 feature lanes).
-template <int BPB>
-__global__ void __launch_bounds__(512) k_histq_reduce(ReduceQArgs a) {
-    constexpr int NE = BPB * 32, NPG = 512 / NE;
-    __shared__ long long part_hi[NPG][NE], part_lo[NPG][NE];
-    __shared__ double tile[BPB][33];
-    const int s = blockIdx.x, fg = blockIdx.y >> 1, ch = blockIdx.y & 1, bin0 = blockIdx.z * BPB;
-    const int ug = fg / a.UB, uw = fg % a.UB;
-    const int e = threadIdx.x % NE, pg = threadIdx.x / NE, binl = e >> 5, lane = e & 31;
-    int bfirst, blast;
-    long long R;
-    slot_pieces(a.plan, a.cum, s, a.G, bfirst, blast, R);
-    const bool two = ch == 0 || a.NW == 4;   // hi + lo words, or a single count word
-    const int w0 = ch == 0 ? 0 : 2;
-    long long hi = 0, lo = 0;
-    const int bin = bin0 + binl;
-    if (bin < a.nbins) {
-        const uint32_t *src = a.scratch + ((size_t)(ug * a.PG + s) * a.UB + uw) * a.img_words + (w0 * a.nbins + bin) * 32 + lane;
-        const size_t bstride = (size_t)a.UB * a.img_words, wstride = (size_t)a.nbins * 32;
-        const bool all = R >= a.G;
-        for (int b = bfirst + pg; b <= blast; b += NPG) {
-            if (all || R * b / a.G < R * (b + 1) / a.G) {
-                if (two) { hi += (long long)(int32_t)src[(size_t)b * bstride]; lo += (long long)src[(size_t)b * bstride + wstride]; }
-                else lo += (long long)src[(size_t)b * bstride];
-            }
-        }
-    }
-    part_hi[pg][e] = hi; part_lo[pg][e] = lo;
-    __syncthreads();
-    if (pg == 0) {
-        long long th = 0, tl = 0;
-#pragma unroll
-        for (int q = 0; q < NPG; ++q) { th += part_hi[q][e]; tl += part_lo[q][e]; }
-        tile[binl][lane] = (double)(th * (1ll << QSPLIT) + tl) * a.qinv[ch];
-    }
-    __syncthreads();
-    if (threadIdx.x < NE) {
-        const int fl = threadIdx.x / BPB, bl = threadIdx.x % BPB;
-        const int slotf = fg * 32 + fl, binw = bin0 + bl;
-        if (slotf < a.F && binw < a.nbins) store_q(a.hcomp, s, a.F, a.nbins, slotf, binw, ch, tile[bl][fl]);
-    }
-}
-
-// deep levels (many build slots, few pieces each): one CTA per (build slot, unit)
-__global__ void __launch_bounds__(256) k_histq_reduce_unit(ReduceQArgs a) {
-    __shared__ double tile[64][33];
-    const int s = blockIdx.x, fg = blockIdx.y;
-    const int ug = fg / a.UB, uw = fg % a.UB;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int bfirst, blast;
-    long long R;
-    slot_pieces(a.plan, a.cum, s, a.G, bfirst, blast, R);
-    const bool all = R >= a.G;
-    const size_t bstride = (size_t)a.UB * a.img_words, wstride = (size_t)a.nbins * 32;
-    const uint32_t *src0 = a.scratch + ((size_t)(ug * a.PG + s) * a.UB + uw) * a.img_words + lane;
-    for (int ch = 0; ch < 2; ++ch) {
-        const bool two = ch == 0 || a.NW == 4;
-        const int w0 = ch == 0 ? 0 : 2;
-        for (int bin0 = 0; bin0 < a.nbins; bin0 += 64) {
-            for (int bl = w; bl < 64; bl += 8) {
-                const int bin = bin0 + bl;
-                long long hi = 0, lo = 0;
-                if (bin < a.nbins) {
-                    const uint32_t *src = src0 + (w0 * a.nbins + bin) * 32;
-                    for (int b = bfirst; b <= blast; ++b) {
-                        if (all || R * b / a.G < R * (b + 1) / a.G) {
-                            if (two) { hi += (long long)(int32_t)src[(size_t)b * bstride]; lo += (long long)src[(size_t)b * bstride + wstride]; }
-                            else lo += (long long)src[(size_t)b * bstride];
-                        }
-                    }
-                }
-                tile[bl][lane] = (double)(hi * (1ll << QSPLIT) + lo) * a.qinv[ch];
-            }
-            __syncthreads();
-            for (int e = threadIdx.x; e < 64 * 32; e += 256) {
-                const int fl = e >> 6, bl = e & 63;
-                const int slotf = fg * 32 + fl, binw = bin0 + bl;
-                if (slotf < a.F && binw < a.nbins) store_q(a.hcomp, s, a.F, a.nbins, slotf, binw, ch, tile[bl][fl]);
-            }
-            __syncthreads();
-        }
-    }
-}
-
-template <int BP, int NW>
-cudaError_t launch_histq_t(const HistArgs &a, dim3 grid, int threads, size_t smem, cudaStream_t st) {
-    static bool attr_set[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 64 && !attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_histq<BP, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return e;
-        attr_set[dev] = true;
-    }
-    k_histq<BP, NW><<<grid, threads, smem, st>>>(a);
-    return cudaGetLastError();
-}
-template <int BP, int NW>
-int occupancy_q_t(int threads, size_t smem) {
-    cudaFuncSetAttribute(k_histq<BP, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_histq<BP, NW>, threads, smem) != cudaSuccess) nb = 0;
-    return nb;
-}
-template <int BP>
-int dispatch_q_nw(int NW, bool launch, const HistArgs *a, dim3 grid, int threads, size_t smem, cudaStream_t st) {
-    if (NW == 3) return launch ? (int)launch_histq_t<BP, 3>(*a, grid, threads, smem, st) : occupancy_q_t<BP, 3>(threads, smem);
-    return launch ? (int)launch_histq_t<BP, 4>(*a, grid, threads, smem, st) : occupancy_q_t<BP, 4>(threads, smem);
-}
-int dispatch_q(int BP, int NW, bool launch, const HistArgs *a, dim3 grid, int threads, size_t smem, cudaStream_t st) {
-    switch (BP) {
-    case 32: return dispatch_q_nw<32>(NW, launch, a, grid, threads, smem, st);
-    case 64: return dispatch_q_nw<64>(NW, launch, a, grid, threads, smem, st);
-    case 128: return dispatch_q_nw<128>(NW, launch, a, grid, threads, smem, st);
-    default: return dispatch_q_nw<256>(NW, launch, a, grid, threads, smem, st);
-    }
-}
-
 struct ReduceArgs {
     const float *scratch;
     double *hcomp;
@@ -925,61 +510,6 @@ __global__ void __launch_bounds__(512) k_hist_reduce(ReduceArgs a) {
     }
 }
 
-// Variant for levels with many build slots (each with few pieces): one CTA per (build slot, unit, feature slot
-// of the lane) sums all channels and bins of that sub-image, so that deep levels launch a thousand CTAs with real
-// work each instead of many thousands of tiny ones.  Same fixed summation order as k_hist_reduce.
-__global__ void __launch_bounds__(256) k_hist_reduce_unit(ReduceArgs a) {
-    __shared__ double tile[64][33];
-    const int s = blockIdx.x, u = blockIdx.y / a.FPL, j = blockIdx.y % a.FPL;
-    const int ug = u / a.UB, uw = u % a.UB, ct = u / a.NFG, fg = u % a.NFG;
-    const int nch = min(a.NCH, a.Ce - ct * a.NCH);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nbuild = a.plan->nbuild;
-    const long long R = a.plan->R;
-    int bfirst = 0, blast = -1;
-    if (s < nbuild && R > 0) {
-        const long long c0 = a.cum[s], c1 = a.cum[s + 1];
-        if (c1 > c0) {
-            bfirst = (int)(((c0 + 1) * a.G - 1) / R);
-            blast = (int)((c1 * a.G - 1) / R);
-        }
-    }
-    const bool all_exist = R >= a.G;
-    const size_t bstride = (size_t)a.UB * a.img_floats;
-    const float *src0 = a.scratch + ((size_t)(ug * a.PG + s) * a.UB + uw) * a.img_floats + lane;
-    for (int c = 0; c < nch; ++c) {
-        for (int bin0 = 0; bin0 < a.nbins; bin0 += 64) {
-            for (int bl = w; bl < 64; bl += 8) {
-                const int bin = bin0 + bl;
-                double acc = 0.0;
-                if (bin < a.nbins) {
-                    const float *src = src0 + ((j * a.NCH + c) * a.nbins + bin) * 32;
-                    for (int b = bfirst; b <= blast; ++b)
-                        if (all_exist || R * b / a.G < R * (b + 1) / a.G) acc += (double)src[(size_t)b * bstride];
-                }
-                tile[bl][lane] = acc;
-            }
-            __syncthreads();
-            for (int e = threadIdx.x; e < 64 * 32; e += 256) {
-                const int fl = e >> 6, bl = e & 63;
-                const int slotf = (fg * 32 + fl) * a.FPL + j, binw = bin0 + bl;
-                if (slotf < a.F && binw < a.nbins) {
-                    double *dst = a.hcomp + ((size_t)s * a.F + slotf) * a.C * a.nbins + binw;
-                    const int ce = ct * a.NCH + c;
-                    const double v = tile[bl][fl];
-                    if (a.Ce == a.C || ce < a.K) {
-                        dst[(size_t)ce * a.nbins] = v;
-                    } else { // mse with elided hessians: w, and h_k = 2w
-                        dst[(size_t)(2 * a.K) * a.nbins] = v;
-                        for (int k = 0; k < a.K; ++k) dst[(size_t)(a.K + k) * a.nbins] = 2.0 * v;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
-
 template <int BP, int NCH, int FPL>
 cudaError_t launch_hist_t(const HistArgs &a, dim3 grid, int threads, size_t smem, cudaStream_t st) {
     static bool attr_set[64] = {};
@@ -1039,39 +569,9 @@ size_t unit_image_bytes(int BP, int NCH, int FPL) {
 
 } // namespace
 
-// Geometry for F feature slots.  Called once at create time with F = nfeats (sizes the scratch buffer)
-// and again per tree when the column sample is smaller.
-// fixed-point variant: one unit per 32 feature slots, NCH = words per row, one CTA per SM
-static int32_t histq_geometry(const evb_handle *h, int F, HistGeom *g) {
-    const int B = h->B;
-    g->BP = B <= 32 ? 32 : B <= 64 ? 64 : B <= 128 ? 128 : 256;
-    g->q = true;
-    g->NCT = 1; g->NCH = h->unit_w ? 3 : 4; g->FPL = 1;
-    g->NFG = (F + 31) / 32;
-    g->U = g->NFG;
-    const size_t img = (size_t)q_planes(g->NCH) * (g->BP + 1) * 128, rings = (size_t)QT * (QDR + 1) * q_tile_bytes(g->NCH); // rings: per CTA
-    int UB = g->U < EVB_MAX_UNITS_PER_BLOCK ? g->U : EVB_MAX_UNITS_PER_BLOCK;
-    while (UB > 1 && UB * img + rings > 227 * 1024) --UB;
-    if (UB * img + rings > 227 * 1024) return EVB_ERR_LIMIT; // 256 bins with weights: the caller falls back to the float kernel
-    g->UB = UB; g->NUG = (g->U + UB - 1) / UB; g->stages = QDR;
-    g->smem = UB * img + rings;
-    const int occ = dispatch_q(g->BP, g->NCH, false, nullptr, dim3(), UB * QT * 32, g->smem, 0);
-    if (occ < 1) { evb_set_error("histogram kernel cannot be resident (smem=%zu)", g->smem); return EVB_ERR_CUDA; }
-    g->G = occ * h->num_sms;
-    // the 32-bit partial sums of a piece hold at most 2^17 rows: more (equal) row ranges than resident CTAs if needed
-    if ((long long)g->G * 130000 < h->n) g->G = (int)((h->n + 129999) / 130000 + g->G - 1) / g->G * g->G;
-    g->PG = g->G + h->maxslots;
-    g->img_floats = (size_t)g->NCH * B * 32;
-    return EVB_OK;
-}
-
-int32_t evb_hist_geometry(const evb_handle *h, int F, HistGeom *g) {
-    if (h->use_q && F == h->nfeats) {
-        const int32_t rc = histq_geometry(h, F, g);
-        if (rc != EVB_ERR_LIMIT) return rc;
-    }
+// Geometry for F feature slots.
+static int32_t evb_hist_geometry(const evb_handle *h, int F, HistGeom *g) {
     const int B = h->B, C = h->Ce;
-    g->q = false;
     g->BP = B <= 32 ? 32 : B <= 64 ? 64 : B <= 128 ? 128 : 256;
     g->NCT = (C + 3) / 4;              // channel groups; channels are spread evenly over them
     g->NCH = (C + g->NCT - 1) / g->NCT;
@@ -1128,73 +628,6 @@ int32_t evb_hist_geometry(const evb_handle *h, int F, HistGeom *g) {
     return EVB_OK;
 }
 
-int32_t evb_hist_configure(evb_handle *h) {
-    EVB_CHECK(evb_hist_geometry(h, h->nfeats, &h->hg));
-    h->q_active = h->hg.q;
-    h->scratch_floats = (size_t)h->hg.NUG * h->hg.PG * h->hg.UB * h->hg.img_floats;
-    return EVB_OK;
-}
-
-int32_t evb_launch_hist(evb_handle *h, int level) {
-    const HistGeom &g = h->hg;
-    HistArgs a;
-    a.xT = h->xT; a.grad = h->q_active ? reinterpret_cast<const float *>(h->gradq) : h->grad; a.rows = h->rows[(level - 1) & 1]; a.js0 = h->js_d;
-    a.plan = h->plan + level; a.cum = h->cum; a.slot_node = h->slot_node; a.seg_start = h->seg_start;
-    a.scratch = h->scratch; a.err = h->d_err;
-    a.RS = h->RS; a.GS = h->GS; a.F = h->F; a.nbins = h->B; a.C = h->Ce; a.NFG = g.NFG; a.U = g.U; a.UB = g.UB;
-    a.stages = g.stages; a.PG = g.PG; a.img_floats = (uint32_t)g.img_floats;
-    a.mode = h->hist_mode;
-    a.contig = h->F == h->nfeats ? 1 : 0;
-    dim3 grid(g.G, g.NUG);
-    const int threads = h->q_active ? g.UB * QT * 32 : (g.UB + 1) * 32;
-    evb_tic(h, EVB_T_HIST);
-    cudaError_t e = h->q_active ? (cudaError_t)dispatch_q(g.BP, g.NCH, true, &a, grid, threads, g.smem, h->st) : launch_hist(g, a, grid, threads, h->st);
-    evb_toc(h, EVB_T_HIST);
-    EVB_CUDA(e);
-    return EVB_OK;
-}
-
-int32_t evb_launch_hist_reduce(evb_handle *h, int level) {
-    const HistGeom &g = h->hg;
-    if (h->q_active) {
-        ReduceQArgs a;
-        a.scratch = reinterpret_cast<const uint32_t *>(h->scratch); a.hcomp = h->hcomp; a.plan = h->plan + level; a.cum = h->cum;
-        a.qinv = h->d_qinv; a.G = g.G; a.PG = g.PG; a.UB = g.UB; a.NFG = g.NFG; a.F = h->F; a.nbins = h->B; a.NW = g.NCH;
-        a.img_words = (uint32_t)g.img_floats;
-        const int slots = evb_level_slots(level);
-        evb_tic(h, EVB_T_HIST_REDUCE);
-        if (slots <= 2) k_histq_reduce<1><<<dim3(slots, g.NFG * 2, h->B), 512, 0, h->st>>>(a);
-        else if (slots <= 8) k_histq_reduce<4><<<dim3(slots, g.NFG * 2, (h->B + 3) / 4), 512, 0, h->st>>>(a);
-        else if (slots <= 32) k_histq_reduce<16><<<dim3(slots, g.NFG * 2, (h->B + 15) / 16), 512, 0, h->st>>>(a);
-        else k_histq_reduce_unit<<<dim3(slots, g.NFG), 256, 0, h->st>>>(a);
-        evb_toc(h, EVB_T_HIST_REDUCE);
-        EVB_CUDA(cudaGetLastError());
-        return EVB_OK;
-    }
-    ReduceArgs a;
-    a.scratch = h->scratch; a.hcomp = h->hcomp; a.plan = h->plan + level; a.cum = h->cum;
-    a.G = g.G; a.PG = g.PG; a.UB = g.UB; a.NFG = g.NFG; a.U = g.U; a.F = h->F; a.C = h->C; a.Ce = h->Ce; a.K = h->K; a.nbins = h->B; a.NCH = g.NCH; a.FPL = g.FPL;
-    a.img_floats = (uint32_t)g.img_floats;
-    const int slots = evb_level_slots(level);
-    evb_tic(h, EVB_T_HIST_REDUCE);
-    if (slots <= 2) {           // top of the tree: hundreds of pieces per slot -> 16 piece groups per CTA
-        dim3 grid(slots, g.U * g.FPL * g.NCH, h->B);
-        k_hist_reduce<1><<<grid, 512, 0, h->st>>>(a);
-    } else if (slots <= 8) {
-        dim3 grid(slots, g.U * g.FPL * g.NCH, (h->B + 3) / 4);
-        k_hist_reduce<4><<<grid, 512, 0, h->st>>>(a);
-    } else if (slots <= 32) {
-        dim3 grid(slots, g.U * g.FPL * g.NCH, (h->B + 15) / 16);
-        k_hist_reduce<16><<<grid, 512, 0, h->st>>>(a);
-    } else {                    // deep levels: few pieces per slot -> one CTA per sub-image
-        dim3 grid(slots, g.U * g.FPL);
-        k_hist_reduce_unit<<<grid, 256, 0, h->st>>>(a);
-    }
-    evb_toc(h, EVB_T_HIST_REDUCE);
-    EVB_CUDA(cudaGetLastError());
-    return EVB_OK;
-}
-
 // =====================================================================================================
 // Stand-alone histogram of one list of rows, for callers that hold their own device buffers.
 // evb_hist_rows allocates its work buffers per call; evb_hist_rows_noalloc allocates nothing.
@@ -1223,7 +656,7 @@ __global__ void k_rows_plan_fill(RowsPlan *p, uint32_t *js, int nfeats, long lon
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < nfeats) js[t] = (uint32_t)t;
     if (t == 0) {
-        p->plan.nbuild = 1; p->plan.nitems = 0; p->plan.R = nrows; p->plan.n_sel = (int32_t)nrows; p->plan.pad = 0;
+        p->plan.nbuild = 1; p->plan.npl = 1; p->plan.R = nrows; p->plan.n_sel = (int32_t)nrows; p->plan.pad = 0;
         p->cum[0] = 0; p->cum[1] = (int32_t)nrows;
         p->slot_node[0] = 1; p->slot_node[1] = 0;
         p->seg_start[0] = 0; p->seg_start[1] = 0;

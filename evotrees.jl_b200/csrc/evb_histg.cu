@@ -1,0 +1,173 @@
+// Integer histograms of any loss (device code and its reasons: evb_histg.cuh): geometry, quantisation, launches.
+#include "evb_histg.cuh"
+#include <stdlib.h>
+#include <algorithm>
+
+namespace {
+
+using namespace evb_hg;
+
+struct KArgs {
+    Args a;
+    HGeom g;
+};
+
+template <int NQ, bool CNT, bool PACK>
+__device__ __forceinline__ void run(const Args &a, uint32_t *smem) { accumulate<NQ, CNT, PACK>(a, smem, blockIdx.x, gridDim.x); }
+
+// grid (row ranges, feature groups, channel groups)
+__global__ void __launch_bounds__(1024, 1) k_histg(KArgs k) {
+    extern __shared__ __align__(128) uint32_t s_img[];
+    Args &a = k.a;
+    evb_hg_select(k.g, a, blockIdx.y, blockIdx.z);
+    if ((long long)blockIdx.x * a.min_rows >= max(1ll, (long long)a.plan->R)) return;
+    const int P = evb_hg_planes(k.g, blockIdx.z), words = nparts(a.nfull, a.tails) * (a.B + 1) * P * 32;
+    for (int i = threadIdx.x; i < words; i += blockDim.x) s_img[i] = 0u;
+    __syncthreads();
+    EVB_HG_DISPATCH(k.g, blockIdx.z, run, a, s_img)
+}
+
+// clears the accumulators of the level's build slots (all feature columns, sampled or not)
+__global__ void __launch_bounds__(256) k_hg_clear(unsigned long long *hsum, uint32_t *hcnt, const LevelPlan *plan, size_t per_slot, int nq) {
+    const size_t n = (size_t)plan->nbuild * per_slot, ns = n * nq;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += (size_t)gridDim.x * blockDim.x) {
+        hsum[i] = 0ull;
+        if (i < n) hcnt[i] = 0u;
+    }
+}
+
+// hcomp[slot][f][channel][bin] (doubles, what ranks exchange) from the integer accumulators.  One CTA per (build slot,
+// 32 feature slots).
+struct ConvArgs {
+    const unsigned long long *hsum;
+    const uint32_t *hcnt;
+    double *hcomp;
+    const LevelPlan *plan;
+    const uint32_t *js0;
+    const double *qinv;
+    int B, SC, F, C, K, nq, elide, unit_w;
+};
+__global__ void __launch_bounds__(256) k_hg_to_hcomp(ConvArgs a) {
+    __shared__ double t[64][33];
+    const int s = blockIdx.x, f0 = blockIdx.y * 32;
+    if (s >= a.plan->nbuild) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, f = f0 + lane;
+    const int col = f < a.F ? (int)a.js0[f] : -1;
+    for (int c = 0; c < a.C; ++c) {
+        const bool is_h = a.elide && c >= a.K && c < 2 * a.K; // h = 2w (src/loss.jl:52)
+        const bool is_w = c == a.C - 1 || is_h;
+        const int ch = is_w ? a.nq - 1 : c;
+        const double mul = is_h ? 2.0 : 1.0;
+        for (int bin0 = 0; bin0 < a.B; bin0 += 64) {
+            for (int bl = w; bl < 64; bl += 8) {
+                const int bin = bin0 + bl;
+                double v = 0.0;
+                if (bin < a.B && col >= 0) {
+                    const size_t cell = (size_t)s * a.B + bin;
+                    v = is_w && a.unit_w ? (double)a.hcnt[cell * a.SC + col]
+                                         : (double)(long long)a.hsum[(cell * a.nq + ch) * a.SC + col] * a.qinv[ch];
+                }
+                t[bl][lane] = mul * v;
+            }
+            __syncthreads();
+            for (int e = threadIdx.x; e < 64 * 32; e += 256) {
+                const int fl = e >> 6, bl = e & 63, ff = f0 + fl, bin = bin0 + bl;
+                if (ff < a.F && bin < a.B) a.hcomp[(((size_t)s * a.F + ff) * a.C + c) * a.B + bin] = t[bl][fl];
+            }
+            __syncthreads();
+        }
+    }
+}
+
+constexpr size_t SMEM_TWO = 113 * 1024;  // two CTAs per SM: 228 KB less 1 KB per CTA
+constexpr size_t SMEM_ONE = 226 * 1024;
+
+} // namespace
+
+// Cuts the channels and the words of a row over CTAs so that an image fits shared memory: as many channels per CTA as
+// possible (at most MAX_NQ) with at least one part of eight words, then as many parts as fit.  Two CTAs of 512 threads share an
+// SM when their images do, so that one accumulates while the other empties its image; else one CTA of 1024 threads.
+int32_t evb_hg_configure(evb_handle *h) {
+    HGeom &g = h->hgeo;
+    g.nq = h->nq;
+    g.pack = h->p.loss == EVB_MSE && h->K == 1 && h->unit_w;
+    g.cnt = h->unit_w && !g.pack;
+    g.qbits = g.pack ? 24 : h->p.loss == EVB_MSE ? 29 : 31;
+    g.TE = g.pack ? 255 : 2047;
+    if (g.pack) { g.per = 1; g.ngc = 1; }
+    else {
+        int per = std::min(g.nq, MAX_NQ);
+        while (per > 1 && part_bytes(h->B, planes(per, g.cnt, false)) > SMEM_ONE) --per;
+        g.ngc = (g.nq + per - 1) / per;
+        g.per = (g.nq + g.ngc - 1) / g.ngc;
+    }
+    const size_t part = part_bytes(h->B, planes(g.per, g.cnt, g.pack));
+    if (part > SMEM_ONE) { evb_set_error("histogram image does not fit shared memory (nbins=%d)", h->B); return EVB_ERR_LIMIT; }
+    const int W = (h->nfeats + 3) / 4;
+    int nf, tl;
+    split_words(W, nf, tl);
+    const int parts = nparts(nf, tl), fit = (int)(SMEM_ONE / part);
+    g.ngf = (parts + fit - 1) / fit;
+    const int per_group = (parts + g.ngf - 1) / g.ngf;
+    g.wper = g.ngf == 1 ? W : per_group * 8;
+    g.ngf = (W + g.wper - 1) / g.wper;
+    g.W = W;
+    int most = 0;
+    for (int y = 0; y < g.ngf; ++y) { split_words(std::min(g.wper, W - y * g.wper), nf, tl); most = std::max(most, nparts(nf, tl)); }
+    g.smem = most * part;
+    g.threads = g.smem <= SMEM_TWO ? 512 : 1024;
+    g.min_rows = 512;
+    EVB_CUDA(cudaFuncSetAttribute(k_histg, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    int occ = 0;
+    EVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_histg, g.threads, g.smem));
+    if (occ < 1) { evb_set_error("histogram kernel cannot be resident (smem=%zu)", g.smem); return EVB_ERR_CUDA; }
+    g.G = std::max(1, occ * h->num_sms / (g.ngf * g.ngc));
+    return EVB_OK;
+}
+
+size_t evb_hg_q_words(const evb_handle *h) { return evb_hg_qoff(h->hgeo, h->n, h->hgeo.ngc) + 8; }
+
+void evb_hg_args(const evb_handle *h, int level, evb_hg::Args *a) {
+    a->xT = h->xT; a->q = h->gradq; a->rows = h->rows[(level - 1) & 1]; a->plan = h->plan + level; a->cum = h->cum; a->slot_node = h->slot_node;
+    a->seg_start = h->seg_start; a->hsum = h->hsum_q; a->hcnt = h->hcnt_q; a->RS = h->RS; a->B = h->B; a->SC = h->SC; a->nq = h->nq; a->F = h->nfeats;
+    a->TE = h->hgeo.TE; a->min_rows = h->hgeo.min_rows; a->n = h->n;
+}
+
+void evb_hg_quant_args(const evb_handle *h, evb_hg::QuantArgs *a) {
+    a->grad = h->grad; a->q = h->use_q2 ? reinterpret_cast<int32_t *>(h->xE) : h->gradq; a->gmax = h->d_gmax; a->qinv = h->d_qinv; a->n = h->n;
+    a->GS = h->GS; a->NCH = h->rec_nch; a->q2 = h->use_q2 ? 1 : 0; a->g = h->hgeo;
+}
+
+int32_t evb_launch_histg(evb_handle *h, int level) {
+    const HGeom &g = h->hgeo;
+    KArgs k;
+    k.g = g;
+    evb_hg_args(h, level, &k.a);
+    evb_tic(h, EVB_T_HIST);
+    k_histg<<<dim3(g.G, g.ngf, g.ngc), g.threads, g.smem, h->st>>>(k);
+    evb_toc(h, EVB_T_HIST);
+    EVB_CUDA(cudaGetLastError());
+    return EVB_OK;
+}
+
+int32_t evb_launch_acc_clear(evb_handle *h, int level) {
+    const size_t per_slot = (size_t)h->B * h->SC;
+    const size_t blocks = std::min<size_t>(((size_t)evb_level_slots(level) * per_slot * h->nq + 255) / 256, (size_t)h->num_sms * 8);
+    evb_tic(h, EVB_T_HIST_REDUCE);
+    k_hg_clear<<<(unsigned)blocks, 256, 0, h->st>>>(h->hsum_q, h->hcnt_q, h->plan + level, per_slot, h->nq);
+    evb_toc(h, EVB_T_HIST_REDUCE);
+    EVB_CUDA(cudaGetLastError());
+    return EVB_OK;
+}
+
+// integer accumulators -> hcomp (doubles), for runs that exchange histograms between ranks
+int32_t evb_launch_acc_to_hcomp(evb_handle *h, int level) {
+    ConvArgs a;
+    a.hsum = h->hsum_q; a.hcnt = h->hcnt_q; a.hcomp = h->hcomp; a.plan = h->plan + level; a.js0 = h->js_d; a.qinv = h->d_qinv;
+    a.B = h->B; a.SC = h->SC; a.F = h->F; a.C = h->C; a.K = h->K; a.nq = h->nq; a.elide = h->Ce != h->C; a.unit_w = h->unit_w;
+    evb_tic(h, EVB_T_HIST_REDUCE);
+    k_hg_to_hcomp<<<dim3(evb_level_slots(level), (h->F + 31) / 32), 256, 0, h->st>>>(a);
+    evb_toc(h, EVB_T_HIST_REDUCE);
+    EVB_CUDA(cudaGetLastError());
+    return evb_launch_acc_clear(h, level);
+}

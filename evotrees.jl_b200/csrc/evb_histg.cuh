@@ -1,0 +1,337 @@
+// Histogram accumulation in integers for any loss: `update_hist!` / `_hist!` (src/fit-utils.jl:345-394; GPU counterpart
+// `hist_kernel!`, ext/EvoTreesKernelAbstractionsExt/fit-utils.jl:57-95).  Device code shared by k_histg and by the kernel that
+// grows a whole tree.
+//
+// Numbers.  Every gradient channel of a row is a fixed-point number q = rint(g 2^s), 2^s the power of two that puts the
+// channel's max |g| just below 2^31 (2^29 for weighted least squares).  An image cell holds two 32-bit words per channel, the
+// sums of q >> 16 and of q & 0xffff: 65 504 rows fit, and one `red.shared.add.u32` per word is the whole update -- no
+// read-modify-write chain, all warps of a CTA share one image.  One more word counts the rows.  Least squares with unit
+// weights packs (q >> 6, (q & 63) | 1 << 19 with the row count in the top 13 bits, |q| < 2^24) into two words in all.
+// The sums are exact, whatever the order of the rows and however they are cut into pieces.  The step of 2^-31 of the largest
+// gradient is finer than what 32-bit float sums keep as soon as a sum exceeds 1/128 of that gradient.
+//
+// Lanes.  Lane = row of a tile of 32 rows, so a lane has its row's gradients and bins in registers and nothing is shuffled.  A
+// row of bins is a sequence of 32-bit words (four features each), cut into parts of 8, then 4, 2 or 1 words.  A part owns 32
+// image columns, 8 / W replicas of its W words side by side.  In step s of a part lane l adds the four features of word
+// (l + s) % W into replica (l / W) % (8 / W), starting with feature l / 8.  So the 32 lanes of every reduction hit 32
+// different banks (8 column groups of four lanes, each with another feature), and few features cost few reductions: ten
+// features are 3 words instead of the 16 features of a 16-byte chunk.
+// What bounds it is the shared-memory pipe: 4 features x planes reductions per step against two dozen other instructions.
+// Measured (1.5M x 50 rows at the root, four channels + count): 138 us with the rows spread over the lanes by shuffles.
+#pragma once
+#include "evb_internal.cuh"
+
+namespace evb_hg {
+
+constexpr unsigned FULL = 0xffffffffu;
+constexpr int MAX_NQ = 5;     // channels of a CTA
+
+struct Args {
+    const uint8_t *xT;
+    const int32_t *q;         // [n][NQP] words of this CTA's channels
+    const uint32_t *rows;
+    const LevelPlan *plan;
+    const int32_t *cum, *slot_node, *seg_start;
+    unsigned long long *hsum; // [slot][bin][nq][SC]
+    uint32_t *hcnt;           // [slot][bin][SC]
+    int RS, B, SC, nq, ch0;   // ch0: first channel of this CTA
+    int F, word0, words;      // this CTA's words of a row
+    int nfull, tails;         // parts of 8 words; bit mask of the tail parts (4, 2, 1)
+    int TE;                   // tiles of 32 rows between two flushes
+    int min_rows;             // rows per CTA below which fewer CTAs take part
+    long long n;              // rows of q
+};
+
+__host__ __device__ constexpr int planes(int NQ, bool CNT, bool PACK) { return PACK ? 2 : 2 * NQ + (CNT ? 1 : 0); }
+__host__ __device__ constexpr int nqp(int NQ) { return NQ <= 2 ? NQ : NQ <= 4 ? 4 : 8; }
+__host__ __device__ inline size_t part_bytes(int B, int P) { return (size_t)(B + 1) * P * 128; }
+// words of a row -> parts of 8 and tail parts
+__host__ __device__ inline void split_words(int words, int &nfull, int &tails) {
+    nfull = words >> 3;
+    tails = words & 7;
+    if (tails == 7) { ++nfull; tails = 0; }
+    if (tails == 3) tails = 4;
+}
+__host__ __device__ inline int nparts(int nfull, int tails) { return nfull + ((tails >> 2) & 1) + ((tails >> 1) & 1) + (tails & 1); }
+
+template <int OFF>
+__device__ __forceinline__ void red_at(uint32_t addr, uint32_t v) {
+    asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(addr), "r"(v), "n"(OFF) : "memory");
+}
+template <int NQ, bool CNT, bool PACK, int C = 0>
+__device__ __forceinline__ void red_cell(uint32_t addr, const uint32_t (&hi)[NQ], const uint32_t (&lo)[NQ]) {
+    if constexpr (C < NQ) {
+        red_at<256 * C>(addr, hi[C]);
+        red_at<256 * C + 128>(addr, lo[C]);
+        red_cell<NQ, CNT, PACK, C + 1>(addr, hi, lo);
+    } else if constexpr (CNT && !PACK) {
+        red_at<256 * NQ>(addr, 1u);
+    }
+}
+
+template <int NQ>
+__device__ __forceinline__ void load_q(const int32_t *p, int32_t (&q)[NQ]) {
+    if constexpr (NQ == 1) q[0] = __ldg(p);
+    else if constexpr (NQ == 2) { const int2 v = __ldg(reinterpret_cast<const int2 *>(p)); q[0] = v.x; q[1] = v.y; }
+    else {
+        const int4 v = __ldg(reinterpret_cast<const int4 *>(p));
+        q[0] = v.x; q[1] = v.y; q[2] = v.z;
+        if constexpr (NQ >= 4) q[3] = v.w;
+        if constexpr (NQ == 5) q[4] = __ldg(p + 4);
+    }
+}
+
+// per-lane constants
+struct Lane {
+    uint32_t col[4];   // shared address of the image + the four features, in the lane's order
+    uint32_t sel[4];   // PRMT selectors of their bins
+    __device__ __forceinline__ void init(const void *smem, int lane) {
+        const uint32_t img = (uint32_t)__cvta_generic_to_shared(smem);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int f = (k + (lane >> 3)) & 3;
+            col[k] = img + 4u * (uint32_t)f;
+            sel[k] = 0x4440u | (uint32_t)f;
+        }
+    }
+};
+
+// one part of W = 1 << LW words of the lane's row
+template <int NQ, bool CNT, bool PACK, int LW>
+__device__ __forceinline__ void part_steps(const uint8_t *xw, bool act, const uint32_t (&hi)[NQ], const uint32_t (&lo)[NQ], const Lane &ln, uint32_t poff, int lane) {
+    constexpr int W = 1 << LW;
+    constexpr uint32_t STRIDE = planes(NQ, CNT, PACK) * 128;
+    uint32_t v[W];
+    if (!act) { // past the end of the tile: all bins 0, what the lane adds lands in the guard row
+#pragma unroll
+        for (int s = 0; s < W; ++s) v[s] = 0u;
+    } else if constexpr (W == 1) v[0] = __ldg(reinterpret_cast<const uint32_t *>(xw));
+    else if constexpr (W == 2) { const uint2 t = __ldg(reinterpret_cast<const uint2 *>(xw)); v[0] = t.x; v[1] = t.y; }
+    else {
+#pragma unroll
+        for (int h = 0; h < W / 4; ++h) {
+            const uint4 t = __ldg(reinterpret_cast<const uint4 *>(xw) + h);
+            v[4 * h] = t.x; v[4 * h + 1] = t.y; v[4 * h + 2] = t.z; v[4 * h + 3] = t.w;
+        }
+    }
+    // v[s] <- word (lane + s) % W
+#pragma unroll
+    for (int r = 1; r < W; r <<= 1) {
+        const bool on = (lane & r) != 0;
+        uint32_t t[W];
+#pragma unroll
+        for (int s = 0; s < W; ++s) t[s] = on ? v[(s + r) & (W - 1)] : v[s];
+#pragma unroll
+        for (int s = 0; s < W; ++s) v[s] = t[s];
+    }
+    const uint32_t rep = 16u * (uint32_t)(lane & 7 & ~(W - 1)) + poff;
+#pragma unroll
+    for (int s = 0; s < W; ++s) {
+        const uint32_t base = rep + 16u * (uint32_t)((lane + s) & (W - 1));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) red_cell<NQ, CNT, PACK>(__byte_perm(v[s], 0u, ln.sel[k]) * STRIDE + (ln.col[k] + base), hi, lo);
+    }
+}
+
+// The image -> the accumulators of a build slot; clears the image.  All warps of the CTA: one bin row of one part at a time,
+// lane = image column, replicas added by shuffles.
+template <int NQ, bool CNT, bool PACK, int LW>
+__device__ __forceinline__ void flush_part(const Args &a, uint32_t *part, int f0, int slot) {
+    constexpr int P = planes(NQ, CNT, PACK), W = 1 << LW;
+    const int lane = threadIdx.x & 31, NW = blockDim.x >> 5, f = f0 + lane;
+    const bool out = lane < 4 * W && f < a.F;
+    auto replicas = [](auto v) {
+#pragma unroll
+        for (int o = 4 * W; o < 32; o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+        return v;
+    };
+    for (int bin = threadIdx.x >> 5; bin < a.B; bin += NW) {
+        uint32_t *p = part + (size_t)(bin + 1) * (P * 32) + lane;
+        const size_t cell = (size_t)slot * a.B + bin;
+        if constexpr (PACK) {
+            const uint32_t vh = p[0], vp = p[32];
+            if (__ballot_sync(FULL, vp != 0u) == 0u) continue;
+            p[0] = 0u; p[32] = 0u;
+            const long long sum = replicas(((long long)(int32_t)vh << 6) + (long long)(vp & 0x7ffffu));
+            const uint32_t cnt = replicas(vp >> 19);
+            if (!out || cnt == 0u) continue;
+            asm volatile("red.global.add.u64 [%0], %1;" ::"l"(a.hsum + cell * a.SC + f), "l"(sum) : "memory");
+            asm volatile("red.global.add.u32 [%0], %1;" ::"l"(a.hcnt + cell * a.SC + f), "r"(cnt) : "memory");
+        } else {
+            if constexpr (CNT) {
+                const uint32_t c = p[64 * NQ];
+                if (__ballot_sync(FULL, c != 0u) == 0u) continue; // no row of these cells: all their words are zero
+                p[64 * NQ] = 0u;
+                const uint32_t cnt = replicas(c);
+                if (out && cnt != 0u) asm volatile("red.global.add.u32 [%0], %1;" ::"l"(a.hcnt + cell * a.SC + f), "r"(cnt) : "memory");
+            }
+            uint32_t hi[NQ], lo[NQ];
+#pragma unroll
+            for (int c = 0; c < NQ; ++c) { hi[c] = p[64 * c]; lo[c] = p[64 * c + 32]; }
+#pragma unroll
+            for (int c = 0; c < NQ; ++c) {
+                p[64 * c] = 0u; p[64 * c + 32] = 0u;
+                const long long sum = replicas(((long long)(int32_t)hi[c] << 16) + (long long)lo[c]);
+                if (out && sum != 0) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(a.hsum + (cell * a.nq + a.ch0 + c) * a.SC + f), "l"(sum) : "memory");
+            }
+        }
+    }
+}
+template <int NQ, bool CNT, bool PACK>
+__device__ __forceinline__ void flush(const Args &a, uint32_t *smem, int slot) {
+    const size_t pw = (size_t)(a.B + 1) * planes(NQ, CNT, PACK) * 32; // words of a part
+    int f0 = 4 * a.word0;
+    for (int p = 0; p < a.nfull; ++p, smem += pw, f0 += 32) flush_part<NQ, CNT, PACK, 3>(a, smem, f0, slot);
+    if (a.tails & 4) { flush_part<NQ, CNT, PACK, 2>(a, smem, f0, slot); smem += pw; f0 += 16; }
+    if (a.tails & 2) { flush_part<NQ, CNT, PACK, 1>(a, smem, f0, slot); smem += pw; f0 += 8; }
+    if (a.tails & 1) flush_part<NQ, CNT, PACK, 0>(a, smem, f0, slot);
+}
+
+// Rows of the level's build nodes, cut into equal ranges; this CTA is `b` of `G`.  smem: image of all parts, zero on entry and
+// on exit (guard rows excepted: nothing reads them).
+template <int NQ, bool CNT, bool PACK>
+__device__ __forceinline__ void accumulate(const Args &a, uint32_t *smem, int b, int G) {
+    constexpr int P = planes(NQ, CNT, PACK), NQP = nqp(NQ);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, NW = blockDim.x >> 5;
+    const long long R = a.plan->R;
+    {
+        const long long want = (R + a.min_rows - 1) / a.min_rows;
+        if (want < G) G = want < 1 ? 1 : (int)want;
+    }
+    if (b >= G) return;
+    const int lo = (int)(R * b / G), hi = (int)(R * (b + 1) / G);
+    if (lo >= hi) return;
+    const int nbuild = a.plan->nbuild;
+    int s;
+    {
+        int l = 0, r = nbuild - 1; // largest s with cum[s] <= lo
+        while (l < r) { const int m = (l + r + 1) >> 1; if (a.cum[m] <= lo) l = m; else r = m - 1; }
+        s = l;
+    }
+    Lane ln;
+    ln.init(smem, lane);
+    const uint32_t pb = (uint32_t)(a.B + 1) * P * 128;
+    for (int pos = lo; pos < hi; ++s) {
+        const int c0 = a.cum[s], pe = min(hi, a.cum[s + 1]);
+        if (pe <= pos) continue;
+        const uint32_t *rows = a.rows + ((long long)a.seg_start[a.slot_node[s]] - c0);
+        // a piece; every TE tiles the image is emptied
+        for (int p0 = pos; p0 < pe; p0 += a.TE * 32) {
+            const int p1 = min(pe, p0 + a.TE * 32);
+            int t = p0 + wid * 32;
+            // row ids two tiles ahead; the row after the next is asked into L2 meanwhile (below the root rows are gathered)
+            uint32_t ridN = t + lane < p1 ? __ldg(rows + t + lane) : 0u, ridNN = t + NW * 32 + lane < p1 ? __ldg(rows + t + NW * 32 + lane) : 0u;
+            for (; t < p1; t += NW * 32) {
+                const uint32_t rid = ridN;
+                ridN = ridNN;
+                const bool act = t + lane < p1;
+                int32_t q[NQ];
+#pragma unroll
+                for (int c = 0; c < NQ; ++c) q[c] = 0;
+                if (act) load_q<NQ>(a.q + (size_t)rid * NQP, q);
+                const int tn = t + 2 * NW * 32 + lane;
+                ridNN = tn < p1 ? __ldg(rows + tn) : 0u;
+                if (t + NW * 32 + lane < p1) {
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.xT + (size_t)ridN * a.RS + 4 * a.word0));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.q + (size_t)ridN * NQP));
+                }
+                uint32_t qh[NQ], ql[NQ];
+#pragma unroll
+                for (int c = 0; c < NQ; ++c) {
+                    if constexpr (PACK) { qh[c] = (uint32_t)(q[c] >> 6); ql[c] = ((uint32_t)q[c] & 63u) | (1u << 19); }
+                    else { qh[c] = (uint32_t)(q[c] >> 16); ql[c] = (uint32_t)q[c] & 0xffffu; }
+                }
+                const uint8_t *xw = a.xT + (size_t)rid * a.RS + 4 * a.word0;
+                uint32_t poff = 0;
+                for (int p = 0; p < a.nfull; ++p, poff += pb, xw += 32) part_steps<NQ, CNT, PACK, 3>(xw, act, qh, ql, ln, poff, lane);
+                if (a.tails & 4) { part_steps<NQ, CNT, PACK, 2>(xw, act, qh, ql, ln, poff, lane); poff += pb; xw += 16; }
+                if (a.tails & 2) { part_steps<NQ, CNT, PACK, 1>(xw, act, qh, ql, ln, poff, lane); poff += pb; xw += 8; }
+                if (a.tails & 1) part_steps<NQ, CNT, PACK, 0>(xw, act, qh, ql, ln, poff, lane);
+            }
+            __syncthreads();
+            flush<NQ, CNT, PACK>(a, smem, s);
+            __syncthreads();
+        }
+        pos = pe;
+    }
+}
+
+} // namespace evb_hg
+
+// start of channel group z in the q words of n rows (16-byte aligned)
+__host__ __device__ inline size_t evb_hg_qoff(const HGeom &g, long long n, int z) {
+    size_t o = 0;
+    for (int k = 0; k < z; ++k) o += ((size_t)n * evb_hg::nqp(min(g.per, g.nq - k * g.per)) + 3) & ~(size_t)3;
+    return o;
+}
+__host__ __device__ inline int evb_hg_planes(const HGeom &g, int z) {
+    return evb_hg::planes(min(g.per, g.nq - z * g.per), g.cnt && z == 0, g.pack);
+}
+// words and channels of feature group y, channel group z
+__device__ __forceinline__ void evb_hg_select(const HGeom &g, evb_hg::Args &a, int y, int z) {
+    a.word0 = y * g.wper;
+    a.words = min(g.wper, g.W - a.word0);
+    evb_hg::split_words(a.words, a.nfull, a.tails);
+    a.ch0 = z * g.per;
+    a.q += evb_hg_qoff(g, a.n, z);
+}
+namespace evb_hg {
+// q of every channel of a row, and 2^-s of every channel
+struct QuantArgs {
+    const float *grad;
+    int32_t *q;             // channel groups one after the other, or (q2) the x words of xE
+    const unsigned *gmax;   // [nq] bits of max |g|
+    double *qinv;           // [nq]
+    long long n;
+    int GS, NCH, q2;
+    HGeom g;
+};
+// row i of the grid's rows; every thread of the block calls it
+__device__ __forceinline__ void quantize(const QuantArgs &a, long long i) {
+    __shared__ float s_sc[EVB_MAX_Q];
+    for (int c = threadIdx.x; c < a.g.nq; c += blockDim.x) {
+        const float m = __uint_as_float(a.gmax[c]);
+        float sc = 1.0f;
+        double inv = 1.0;
+        if (m > 0.0f && m < INFINITY) {
+            int e;
+            frexpf(m, &e); // m = f 2^e, f in [0.5, 1)
+            const int s = min(a.g.qbits - e, 127); // a channel of denormals keeps its scale inside the range of a float
+            sc = ldexpf(1.0f, s);
+            inv = ldexp(1.0, -s);
+        }
+        s_sc[c] = sc;
+        if (blockIdx.x == 0) a.qinv[c] = inv;
+    }
+    __syncthreads();
+    if (i >= a.n) return;
+    const float *rec = a.grad + (size_t)i * a.GS;
+    if (a.q2) { a.q[2 * i] = __float2int_rn(rec[0] * s_sc[0]); return; }
+    for (int z = 0; z < a.g.ngc; ++z) {
+        const int c0 = z * a.g.per, nc = min(a.g.per, a.g.nq - c0), np = nqp(nc);
+        int32_t *d = a.q + evb_hg_qoff(a.g, a.n, z) + (size_t)i * np;
+        for (int c = 0; c < np; ++c) d[c] = c < nc ? __float2int_rn(rec[((c0 + c) / a.NCH) * 4 + (c0 + c) % a.NCH] * s_sc[c0 + c]) : 0;
+    }
+}
+} // namespace evb_hg
+void evb_hg_quant_args(const evb_handle *h, evb_hg::QuantArgs *a);
+// FN<channels, count plane, packed>(args...) for channel group z
+#define EVB_HG_DISPATCH(g, z, FN, ...)                                          \
+    if ((g).pack) FN<1, true, true>(__VA_ARGS__);                               \
+    else {                                                                      \
+        const int nc_ = min((g).per, (g).nq - (int)(z) * (g).per);              \
+        if ((g).cnt && (z) == 0) switch (nc_) {                                 \
+            case 1: FN<1, true, false>(__VA_ARGS__); break;                     \
+            case 2: FN<2, true, false>(__VA_ARGS__); break;                     \
+            case 3: FN<3, true, false>(__VA_ARGS__); break;                     \
+            case 4: FN<4, true, false>(__VA_ARGS__); break;                     \
+            default: FN<5, true, false>(__VA_ARGS__); break;                    \
+        } else switch (nc_) {                                                   \
+            case 1: FN<1, false, false>(__VA_ARGS__); break;                    \
+            case 2: FN<2, false, false>(__VA_ARGS__); break;                    \
+            case 3: FN<3, false, false>(__VA_ARGS__); break;                    \
+            case 4: FN<4, false, false>(__VA_ARGS__); break;                    \
+            default: FN<5, false, false>(__VA_ARGS__); break;                   \
+        }                                                                       \
+    }
+void evb_hg_args(const evb_handle *h, int level, evb_hg::Args *a);

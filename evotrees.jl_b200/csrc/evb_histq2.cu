@@ -19,9 +19,7 @@
 // ((l >> 3) & 3).
 // The packed counters hold 8191 rows: after at most 255 tiles, and at the end of a node's rows, the CTA adds the packed
 // image to the node's accumulators in global memory (`red.global.add.u64 / .u32`, cell by cell: consecutive lanes,
-// consecutive addresses) and clears it.  Two CTAs share an SM, so one accumulates while the other flushes.  (Optional:
-// one CTA per SM that keeps a wide image -- 64-bit sums, 32-bit counts -- in shared memory between the flushes to global
-// memory.)  Every histogram entry is therefore the exact integer sum of the quantised gradients, whatever the order of
+// consecutive addresses) and clears it.  Two CTAs share an SM, so one accumulates while the other flushes.   Every histogram entry is therefore the exact integer sum of the quantised gradients, whatever the order of
 // the rows and however the rows are cut into pieces.
 #include "evb_internal.cuh"
 #include <stdlib.h>
@@ -29,15 +27,13 @@
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-// Measured on B200 (10M x 100, depth 11, ms of this kernel per tree).  One CTA per SM with a wide image (64-bit sums in shared
-// memory between the flushes to global memory): 768 threads 1.91, 1024: 2.29, 512: 2.33 (the last two before later
-// changes).  Two CTAs of 384 threads per SM without the wide image, every flush going to global memory: 1.83; three
-// CTAs of 256: 2.28.
-constexpr int Q2_THREADS = 384;
-// Word format.  q has QB bits (|q| < 2^QB); plane 0 takes q >> LB, plane 1 takes (q & (2^LB - 1)) | 1 << CS, and an image
-// cell must hold 2^CB - 1 rows: QB - LB + CB <= 31 (signed plane 0), LB + CB <= CS and CS + CB <= 32 (plane 1).
-// QB = 26: LB 8, CS 20, CB 12 (4095 rows, 127 tiles between flushes); QB = 24: LB 6, CS 19, CB 13 (8191 rows, 255 tiles).
-constexpr int Q2_MAX_EPOCH_26 = 127, Q2_MAX_EPOCH_24 = 255;
+// Two CTAs of 384 threads per SM: while one of them flushes, the other accumulates.  Measured on B200 (10M x 100, depth 11,
+// ms of this kernel per tree): 1.83; one CTA of 768 threads with 64-bit sums in shared memory between the flushes to
+// global memory 1.91; three CTAs of 256: 2.28.
+constexpr int Q2_THREADS = 384, Q2_WARPS = Q2_THREADS / 32;
+// |q| < 2^24; plane 0 takes q >> LB, plane 1 takes (q & (2^LB - 1)) | 1 << CS, and an image cell holds 8191 rows: the signed
+// plane 0 needs 24 - 6 + 13 bits, the low sums of plane 1 6 + 13 <= CS, the row count 13 bits above them.
+constexpr int Q2_LB = 6, Q2_CS = 19, Q2_EPOCH = 255 / Q2_WARPS * Q2_WARPS; // tiles of 32 rows between two flushes
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -52,9 +48,6 @@ struct Q2Args {
     int RSH, B, SC;
     int nmain;                // features held in xH
     int ntail;                // features held in xE (0..4)
-    int TE;                   // tiles between two flushes
-    int LB, CS;               // word format: low bits in plane 1, position of the row count
-    int wide;                 // 1: epochs end in the CTA's wide image in shared memory; 0: no wide image, every flush goes to global memory
     int min_rows;             // rows per CTA below which fewer CTAs take part
     uint32_t zrow;            // index of an all-zero row of xH / xE (bins 0, q 0)
 };
@@ -133,14 +126,14 @@ __device__ __forceinline__ void piece_next(const Q2Args &a, PieceIt &it, int lo,
 // register sets of chunk loads in flight per lane: step s of a tile uses set s % NSET and refills it for step s + NSET
 __host__ __device__ constexpr int q2_nset(int NC) { return NC == 6 ? 3 : NC == 8 ? 4 : NC; }
 
-template <int NC, bool TAIL, int NT>
-__global__ void __launch_bounds__(NT, NT <= 384 ? 2 : 1) k_histq2(Q2Args a) {
+template <int NC, bool TAIL>
+__global__ void __launch_bounds__(Q2_THREADS, 2) k_histq2(Q2Args a) {
     using Cf = Q2Cfg<NC, TAIL>;
     constexpr int NCOL = Cf::NCOL, NSET = q2_nset(NC);
     constexpr uint32_t ROWB = Cf::ROWB, X = Cf::X;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, wid = tid >> 5, l = tid & 31;
-    constexpr int NW = NT / 32;
+    constexpr int NW = Q2_WARPS, NT = Q2_THREADS;
     const int b = blockIdx.x, chunk0 = blockIdx.y * NC;
     const long long R = a.plan->R;
     // few rows: fewer CTAs take part (every CTA costs one pass over its image)
@@ -153,7 +146,7 @@ __global__ void __launch_bounds__(NT, NT <= 384 ? 2 : 1) k_histq2(Q2Args a) {
     const int lo = (int)(R * b / G), hi = (int)(R * (b + 1) / G);
     if (lo >= hi) return;
     uint32_t *img_w = reinterpret_cast<uint32_t *>(smem);
-    for (int i = tid; i < ((a.B + 1) * 2 * NCOL * 4 + (a.wide ? a.B * (16 * NC + (TAIL ? 4 : 0)) * 12 : 0)) / 4; i += NT) img_w[i] = 0u; // packed (+ wide) image
+    for (int i = tid; i < (a.B + 1) * 2 * NCOL; i += NT) img_w[i] = 0u;
     __syncthreads();
 
     const int nbuild = a.plan->nbuild;
@@ -189,19 +182,14 @@ __global__ void __launch_bounds__(NT, NT <= 384 ? 2 : 1) k_histq2(Q2Args a) {
     const uint32_t RSH = (uint32_t)a.RSH;
     const uint32_t zrow = a.zrow; // an all-zero row: its bins land in the image's guard row
 
-    // The packed image is emptied at every boundary.  Inside a node's rows it goes into the CTA's wide image in shared
-    // memory (64-bit sums, 32-bit counts; every cell belongs to one thread, so plain adds); at the end of the node's
-    // rows (`final`) packed + wide go to the accumulators of build slot `slot` in global memory.  All threads of the CTA.
-    constexpr int WC = 16 * NC + (TAIL ? 4 : 0); // columns of the wide image
-    long long *wsum = reinterpret_cast<long long *>(smem + (size_t)(a.B + 1) * 2 * NCOL * 4);
-    uint32_t *wcnt = reinterpret_cast<uint32_t *>(wsum + (size_t)a.B * WC);
-    const int LB = a.LB, CS = a.CS;
-    const uint32_t cmask = (1u << CS) - 1u, lmask = (1u << LB) - 1u, one = 1u << CS;
-    auto flush = [&](int slot, bool final) {
+    // The packed image goes to the accumulators of build slot `slot` in global memory, at the end of a node's rows and when
+    // its row counts may be full.  All threads of the CTA.
+    constexpr int LB = Q2_LB, CS = Q2_CS;
+    constexpr uint32_t cmask = (1u << CS) - 1u, lmask = (1u << LB) - 1u, one = 1u << CS;
+    auto flush = [&](int slot) {
         __syncthreads();
-        if (!a.wide) {
-            // no wide image: the packed image goes to the slot's accumulators cell by cell (consecutive lanes, consecutive
-            // addresses), whether the node's rows end here or only the count field is full
+        {
+            // cell by cell: consecutive lanes, consecutive addresses
             const size_t base = (size_t)slot * a.B;
             constexpr int MC = 16 * NC;
             for (int c = tid; c < a.B * MC; c += NT) {
@@ -235,77 +223,19 @@ __global__ void __launch_bounds__(NT, NT <= 384 ? 2 : 1) k_histq2(Q2Args a) {
                     }
                 }
             }
-            __syncthreads();
-            return;
-        }
-        constexpr int QPR = 4 * NC; // quads of main columns per bin row
-        for (int e = tid; e < a.B * QPR; e += NT) {
-            const int bin = e / QPR, col = (e % QPR) * 4;
-            uint32_t *p = img_w + (size_t)(bin + 1) * 2 * NCOL + col;
-            const uint4 vh = *reinterpret_cast<const uint4 *>(p), vp = *reinterpret_cast<const uint4 *>(p + NCOL);
-            if ((vh.x | vh.y | vh.z | vh.w | vp.x | vp.y | vp.z | vp.w) == 0u) continue;
-            *reinterpret_cast<uint4 *>(p) = make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4 *>(p + NCOL) = make_uint4(0u, 0u, 0u, 0u);
-            const uint32_t h4[4] = {vh.x, vh.y, vh.z, vh.w}, p4[4] = {vp.x, vp.y, vp.z, vp.w};
-            long long sm4[4];
-            uint32_t c4[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) { sm4[k] = ((long long)(int32_t)h4[k] << LB) + (long long)(p4[k] & cmask); c4[k] = p4[k] >> CS; }
-            longlong2 *ws = reinterpret_cast<longlong2 *>(wsum + (size_t)bin * WC + col);
-            uint4 *wc = reinterpret_cast<uint4 *>(wcnt + (size_t)bin * WC + col);
-            longlong2 s0 = ws[0], s1 = ws[1];
-            uint4 cw = *wc;
-            s0.x += sm4[0]; s0.y += sm4[1]; s1.x += sm4[2]; s1.y += sm4[3];
-            cw.x += c4[0]; cw.y += c4[1]; cw.z += c4[2]; cw.w += c4[3];
-            ws[0] = s0; ws[1] = s1; *wc = cw;
-        }
-        if (TAIL) { // 8 replicas of the 4 tail features: one warp per bin row, lane = column of the packed image
-            for (int bin = wid; bin < a.B; bin += NW) {
-                uint32_t *p = img_w + (size_t)(bin + 1) * 2 * NCOL + Cf::TAILCOL + l;
-                const uint32_t vh = p[0], vp = p[NCOL];
-                if (__ballot_sync(FULL, (vh | vp) != 0u) == 0u) continue;
-                p[0] = 0u; p[NCOL] = 0u;
-                long long sum = ((long long)(int32_t)vh << LB) + (long long)(vp & cmask);
-                uint32_t cnt = vp >> CS;
-#pragma unroll
-                for (int o = 4; o < 32; o <<= 1) { sum += __shfl_xor_sync(FULL, sum, o); cnt += __shfl_xor_sync(FULL, cnt, o); }
-                if (l < 4) {
-                    wsum[(size_t)bin * WC + 16 * NC + l] += sum;
-                    wcnt[(size_t)bin * WC + 16 * NC + l] += cnt;
-                }
-            }
-        }
-        if (final) {
-            // the wide image goes to the slot's accumulators cell by cell: consecutive lanes, consecutive addresses
-            __syncthreads();
-            const size_t base = (size_t)slot * a.B;
-            for (int c = tid; c < a.B * WC; c += NT) {
-                const uint32_t cnt = wcnt[c];
-                if (cnt == 0u) continue;
-                const long long sum = wsum[c];
-                wsum[c] = 0; wcnt[c] = 0u;
-                const int bin = c / WC, col = c - bin * WC;
-                const bool main_col = col < 16 * NC;
-                const int f = main_col ? chunk0 * 16 + col : a.nmain + col - 16 * NC;
-                if (main_col ? f < a.nmain : col - 16 * NC < a.ntail) {
-                    const size_t o = (base + bin) * a.SC + f;
-                    asm volatile("red.global.add.u64 [%0], %1;" ::"l"(a.hsum + o), "l"(sum) : "memory");
-                    asm volatile("red.global.add.u32 [%0], %1;" ::"l"(a.hcnt + o), "r"(cnt) : "memory");
-                }
-            }
         }
         __syncthreads();
     };
 
     // the two piece iterators of a warp (accumulate stage, row-id fetch stage) are warp-uniform and touched once per
     // tile: they live in shared memory so that the registers stay with the loads in flight
-    __shared__ PieceIt s_it[NT / 32][2];
+    __shared__ PieceIt s_it[Q2_WARPS][2];
     PieceIt &pc = s_it[wid][0], &pa = s_it[wid][1];
     pc.s = s0; pc.g0 = 0; pc.end = false;
     piece_load(a, pc, lo, hi, nbuild);
     pa = pc;
     __syncwarp();
-    int ep_end = pc.end ? 0 : min(pc.nt, a.TE);
+    int ep_end = pc.end ? 0 : min(pc.nt, Q2_EPOCH);
 
     // row ids of tile g of this CTA (lane = row of the tile); rows past the end of the tile read the zero row
     auto fetch = [&](int g) -> uint32_t {
@@ -334,9 +264,9 @@ __global__ void __launch_bounds__(NT, NT <= 384 ? 2 : 1) k_histq2(Q2Args a) {
         for (;;) {
             if (pc.end) { done = true; break; }
             if (g < pc.g0 + ep_end) break;
-            flush(pc.s, ep_end == pc.nt);
-            if (ep_end == pc.nt) { piece_next(a, pc, lo, hi, nbuild); if (!pc.end) ep_end = min(pc.nt, a.TE); }
-            else ep_end = min(pc.nt, ep_end + a.TE);
+            flush(pc.s);
+            if (ep_end == pc.nt) { piece_next(a, pc, lo, hi, nbuild); if (!pc.end) ep_end = min(pc.nt, Q2_EPOCH); }
+            else ep_end = min(pc.nt, ep_end + Q2_EPOCH);
         }
         if (done) break;
         const uint2 extN = ldg_ext(a.xE + ridB);
@@ -368,55 +298,6 @@ __global__ void __launch_bounds__(NT, NT <= 384 ? 2 : 1) k_histq2(Q2Args a) {
     }
 }
 
-// hcomp[slot][f][g, h = 2w, w][bin] (doubles) from the integer accumulators, which are cleared for the next level.
-// One CTA per (build slot, 32 feature slots).
-struct Q2ConvArgs {
-    unsigned long long *hsum;
-    uint32_t *hcnt;
-    double *hcomp;
-    const LevelPlan *plan;
-    const uint32_t *js0;
-    const double *qinv;
-    int B, SC, F;
-};
-__global__ void __launch_bounds__(256) k_q2_to_hcomp(Q2ConvArgs a) {
-    __shared__ double tg[64][33], tw[64][33];
-    const int s = blockIdx.x, f0 = blockIdx.y * 32;
-    if (s >= a.plan->nbuild) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const double qi = a.qinv[0];
-    const int f = f0 + lane;
-    const int col = f < a.F ? (int)a.js0[f] : -1;
-    for (int bin0 = 0; bin0 < a.B; bin0 += 64) {
-        for (int bl = w; bl < 64; bl += 8) {
-            const int bin = bin0 + bl;
-            double g = 0.0, c = 0.0;
-            if (bin < a.B && col >= 0) {
-                const size_t o = ((size_t)s * a.B + bin) * a.SC + col;
-                g = (double)(long long)a.hsum[o] * qi;
-                c = (double)a.hcnt[o];
-            }
-            tg[bl][lane] = g; tw[bl][lane] = c;
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < 64 * 32; e += 256) {
-            const int fl = e >> 6, bl = e & 63;
-            const int ff = f0 + fl, bin = bin0 + bl;
-            if (ff < a.F && bin < a.B) {
-                double *dst = a.hcomp + ((size_t)s * a.F + ff) * 3 * a.B + bin;
-                const double wv = tw[bl][fl];
-                dst[0] = tg[bl][fl]; dst[a.B] = 2.0 * wv; dst[(size_t)2 * a.B] = wv; // h = 2w (src/loss.jl:52)
-            }
-        }
-        __syncthreads();
-    }
-}
-// clears the accumulators of the level's build slots (all feature columns, sampled or not)
-__global__ void __launch_bounds__(256) k_q2_clear(unsigned long long *hsum, uint32_t *hcnt, const LevelPlan *plan, size_t per_slot) {
-    const size_t n = (size_t)plan->nbuild * per_slot;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) { hsum[i] = 0ull; hcnt[i] = 0u; }
-}
-
 // tail features of every row: xE[i].y = bins of features nmain .. nmain + ntail - 1 (one byte each, zero padded)
 __global__ void __launch_bounds__(256) k_q2_tail(const uint8_t *xC, long long n, int nmain, int ntail, uint2 *xE) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -426,48 +307,23 @@ __global__ void __launch_bounds__(256) k_q2_tail(const uint8_t *xC, long long n,
     xE[i] = make_uint2(0u, t);
 }
 
-// q = rint(g * 2^s), 2^s the largest power of two with max |g| * 2^s < 2^QB, into xE[i].x; 2^-s into qinv[0]
-__global__ void __launch_bounds__(256) k_q2_quantize(const float *grad, int GS, uint2 *xE, long long n, const unsigned *gmax, double *qinv, int QB) {
-    const float m = __uint_as_float(*gmax);
-    float sc = 1.0f;
-    double inv = 1.0;
-    if (m > 0.0f && m < INFINITY) {
-        int e;
-        frexpf(m, &e);
-        sc = ldexpf(1.0f, QB - e);
-        inv = ldexp(1.0, e - QB);
-    }
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) { qinv[0] = inv; qinv[1] = 1.0; }
-    if (i >= n) return;
-    reinterpret_cast<int32_t *>(xE)[2 * i] = __float2int_rn(grad[(size_t)i * GS] * sc);
-}
-
-template <int NC, bool TAIL, int NT>
-int q2_instance_t(bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st) {
+template <int NC, bool TAIL>
+int q2_instance(bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st) {
     static size_t attr_set[64] = {}; // dynamic shared memory the kernel has been allowed on each device
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && attr_set[dev] < smem) {
-        cudaError_t e = cudaFuncSetAttribute(k_histq2<NC, TAIL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(k_histq2<NC, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return launch ? (int)e : 0;
         attr_set[dev] = smem;
     }
     if (!launch) {
         int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_histq2<NC, TAIL, NT>, NT, smem) != cudaSuccess) nb = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_histq2<NC, TAIL>, Q2_THREADS, smem) != cudaSuccess) nb = 0;
         return nb;
     }
-    k_histq2<NC, TAIL, NT><<<grid, NT, smem, st>>>(*a);
+    k_histq2<NC, TAIL><<<grid, Q2_THREADS, smem, st>>>(*a);
     return (int)cudaGetLastError();
-}
-int g_q2_threads = Q2_THREADS;
-template <int NC, bool TAIL>
-int q2_instance(bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st) {
-    if (g_q2_threads == 384) return q2_instance_t<NC, TAIL, 384>(launch, a, grid, smem, st);
-    if (g_q2_threads == 512) return q2_instance_t<NC, TAIL, 512>(launch, a, grid, smem, st);
-    if (g_q2_threads == 768) return q2_instance_t<NC, TAIL, 768>(launch, a, grid, smem, st);
-    return q2_instance_t<NC, TAIL, 1024>(launch, a, grid, smem, st);
 }
 template <bool TAIL>
 int q2_dispatch_nc(int NC, bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st) {
@@ -489,11 +345,20 @@ int q2_dispatch(int NC, bool tail, bool launch, const Q2Args *a, dim3 grid, size
     }
 }
 int q2_ncol(int NC, bool tail) { const int need = 16 * NC + (tail ? 32 : 0); return need <= 32 ? 32 : need <= 64 ? 64 : 128; }
-// shared memory of a CTA: packed image [B + 1][2][NCOL] words + wide image [B][16 NC (+ 4)] x (64-bit sum, 32-bit count)
-bool g_q2_wide = false;
-size_t q2_smem(int B, int NC, bool tail) { return (size_t)(B + 1) * 2 * q2_ncol(NC, tail) * 4 + (g_q2_wide ? (size_t)B * (16 * NC + (tail ? 4 : 0)) * 12 : 0); }
+size_t q2_smem(int B, int NC, bool tail) { return (size_t)(B + 1) * 2 * q2_ncol(NC, tail) * 4; } // packed image [B + 1][2][NCOL] words
 
 } // namespace
+
+// Least squares with one target and unit weights on many rows.  Below Q2_MIN_ROWS the general integer kernel is as fast (it
+// does less for features that do not fill a 16-byte chunk and has the smaller image to flush), and the training predict has
+// to be able to read the chunk rows: tree, leaf values and two tiles of rows within 100 KB.
+bool evb_q2_wanted(const evb_handle *h) {
+    if (h->p.loss != EVB_MSE || h->K != 1 || !h->unit_w) return false;
+    if (const char *e = getenv("EVB_HIST_Q2")) { if (atoi(e) == 0) return false; }
+    else if (h->n < 300000) return false;
+    const int words = (h->nfeats + 15) / 16 * 4 + 8;
+    return (size_t)(h->nn + 4) * 8 + (size_t)2 * 256 * words * 4 <= (size_t)100 * 1024 && words <= 64;
+}
 
 // Chooses the layout: chunks per CTA group, number of groups, tail features.  Returns EVB_ERR_LIMIT when the shape
 // does not fit (the caller then uses the other histogram kernels).
@@ -501,10 +366,6 @@ int32_t evb_q2_configure(evb_handle *h) {
     const int nf = h->nfeats, B = h->B;
     Q2Geom &g = h->q2;
     const size_t smem_max = 224 * 1024; // the kernel also holds a few KB of static shared memory
-    // Default: no wide image -- the packed image alone lets two CTAs of 384 threads share an SM, and while one of them
-    // flushes the other one accumulates.  EVB_Q2_WIDE=1: one CTA of 768 threads with the wide image.
-    if (const char *e = getenv("EVB_Q2_WIDE")) g_q2_wide = atoi(e) != 0;
-    g_q2_threads = g_q2_wide ? 768 : 384;
     const int t = nf % 16;
     const int nc_all = (nf + 15) / 16;
     // one group with the tail in xE if it fits
@@ -523,23 +384,14 @@ int32_t evb_q2_configure(evb_handle *h) {
         g.NC = (nc_all + g.ngroups - 1) / g.ngroups;
     }
     if (g.ngroups > 64) return EVB_ERR_LIMIT;
-    if (const char *e = getenv("EVB_Q2_THREADS")) { const int want = atoi(e); if (want == 384 || want == 512 || want == 768 || want == 1024) g_q2_threads = want; }
     g.nmain = nf - g.ntail;
     g.RSH = g.ngroups * g.NC * 16;
     if ((unsigned long long)(h->n + 1) * g.RSH >= (1ull << 32)) return EVB_ERR_LIMIT; // 32-bit byte offsets into xH
-    g.SC = (nf + 3) / 4 * 4;
     g.smem = q2_smem(B, g.NC, g.ntail > 0);
     const int occ = q2_dispatch(g.NC, g.ntail > 0, false, nullptr, dim3(), g.smem, 0);
     if (occ < 1) { evb_set_error("fixed-point histogram kernel cannot be resident (smem=%zu)", g.smem); return EVB_ERR_CUDA; }
     g.G = occ * h->num_sms;
-    const int NW = g_q2_threads / 32;
-    g.QB = 24;
-    if (const char *e = getenv("EVB_Q2_QBITS")) { const int want = atoi(e); if (want == 24 || want == 26) g.QB = want; }
-    const int max_epoch = g.QB == 26 ? Q2_MAX_EPOCH_26 : Q2_MAX_EPOCH_24;
-    g.TE = max_epoch / NW * NW;
-    if (const char *e = getenv("EVB_Q2_EPOCH")) { const int want = atoi(e); if (want >= 1 && want <= max_epoch) g.TE = want; }
     g.min_rows = 512; // measured: 100k x 10 rows 0.054 ms per tree at 512, 0.059 at 1024, 0.088 at 4096; no difference at 10M rows
-    if (const char *e = getenv("EVB_Q2_MIN_ROWS")) { const int want = atoi(e); if (want >= 32) g.min_rows = want; }
     return EVB_OK;
 }
 
@@ -562,66 +414,16 @@ int32_t evb_q2_clear_layout(evb_handle *h) {
     return EVB_OK;
 }
 
-int32_t evb_launch_q2_quantize(evb_handle *h) {
-    evb_tic(h, EVB_T_GRADS);
-    k_q2_quantize<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->grad, h->GS, h->xE, h->n, h->d_gmax, h->d_qinv, h->q2.QB);
-    evb_toc(h, EVB_T_GRADS);
-    EVB_CUDA(cudaGetLastError());
-    return EVB_OK;
-}
-
 int32_t evb_launch_histq2(evb_handle *h, int level) {
     const Q2Geom &g = h->q2;
     Q2Args a;
     a.xH = h->xH; a.xE = h->xE; a.rows = h->rows[(level - 1) & 1];
     a.plan = h->plan + level; a.cum = h->cum; a.slot_node = h->slot_node; a.seg_start = h->seg_start;
     a.hsum = h->hsum_q; a.hcnt = h->hcnt_q;
-    a.RSH = g.RSH; a.B = h->B; a.SC = g.SC; a.nmain = g.nmain; a.ntail = g.ntail; a.TE = g.TE; a.min_rows = g.min_rows; a.zrow = (uint32_t)h->n;
-    a.LB = g.QB == 26 ? 8 : 6; a.CS = g.QB == 26 ? 20 : 19;
-    a.wide = g_q2_wide ? 1 : 0;
+    a.RSH = g.RSH; a.B = h->B; a.SC = h->SC; a.nmain = g.nmain; a.ntail = g.ntail; a.min_rows = g.min_rows; a.zrow = (uint32_t)h->n;
     evb_tic(h, EVB_T_HIST);
     const cudaError_t e = (cudaError_t)q2_dispatch(g.NC, g.ntail > 0, true, &a, dim3(g.G, g.ngroups), g.smem, h->st);
     evb_toc(h, EVB_T_HIST);
     EVB_CUDA(e);
-    return EVB_OK;
-}
-
-// The split scan reads the integer accumulators itself when nothing else needs the doubles: one GPU (no exchange of
-// hcomp between ranks).  EVB_Q2_DIRECT=0 keeps the conversion kernel.
-bool evb_q2_direct(const evb_handle *h) {
-    static const bool off = getenv("EVB_Q2_DIRECT") != nullptr && atoi(getenv("EVB_Q2_DIRECT")) == 0;
-    return h->use_q2 && h->world == 1 && !off;
-}
-
-// clears the accumulators of the level's build slots (after the scan has read them)
-int32_t evb_launch_q2_clear(evb_handle *h, int level) {
-    const Q2Geom &g = h->q2;
-    const int slots = evb_level_slots(level);
-    const size_t per_slot = (size_t)h->B * g.SC;
-    size_t blocks = ((size_t)slots * per_slot + 255) / 256;
-    if (blocks > (size_t)h->num_sms * 8) blocks = (size_t)h->num_sms * 8;
-    evb_tic(h, EVB_T_HIST_REDUCE);
-    k_q2_clear<<<(unsigned)blocks, 256, 0, h->st>>>(h->hsum_q, h->hcnt_q, h->plan + level, per_slot);
-    evb_toc(h, EVB_T_HIST_REDUCE);
-    EVB_CUDA(cudaGetLastError());
-    return EVB_OK;
-}
-
-// integer accumulators -> hcomp (doubles, the layout of the other histogram kernels), accumulators cleared
-int32_t evb_launch_q2_reduce(evb_handle *h, int level) {
-    const Q2Geom &g = h->q2;
-    Q2ConvArgs a;
-    a.hsum = h->hsum_q; a.hcnt = h->hcnt_q; a.hcomp = h->hcomp; a.plan = h->plan + level; a.js0 = h->js_d; a.qinv = h->d_qinv;
-    a.B = h->B; a.SC = g.SC; a.F = h->F;
-    const int slots = evb_level_slots(level);
-    evb_tic(h, EVB_T_HIST_REDUCE);
-    k_q2_to_hcomp<<<dim3(slots, (h->F + 31) / 32), 256, 0, h->st>>>(a);
-    const size_t per_slot = (size_t)h->B * g.SC;
-    size_t blocks = ((size_t)slots * per_slot + 255) / 256;
-    if (blocks > (size_t)h->num_sms * 8) blocks = (size_t)h->num_sms * 8;
-    k_q2_clear<<<(unsigned)blocks, 256, 0, h->st>>>(h->hsum_q, h->hcnt_q, h->plan + level, per_slot);
-    evb_toc(h, EVB_T_HIST_REDUCE);
-    h->tm.launches[EVB_T_HIST_REDUCE] += 1;
-    EVB_CUDA(cudaGetLastError());
     return EVB_OK;
 }

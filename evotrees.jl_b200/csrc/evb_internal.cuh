@@ -32,37 +32,19 @@ enum { EVB_DERR_NONE = 0, EVB_DERR_WAIT_FULL = 1, EVB_DERR_WAIT_EMPTY = 2, EVB_D
 constexpr int EVB_TILE_ROWS = 32;    // rows per staged tile (one per producer lane)
 constexpr int EVB_PART_CHUNK = 2048; // rows per partition work item
 constexpr int EVB_PART_THREADS = 256;
-constexpr int EVB_MAX_UNITS_PER_BLOCK = 4;
 constexpr int EVB_MAX_DEPTH = 15;
 constexpr int EVB_GEN_WORDS = 12;    // 32-bit words of a generator state
 
 enum { EVB_MASK_NONE = 0, EVB_MASK_HOST = 1, EVB_MASK_PCG = 2 }; // rows: all, a mask from the host, a mask made on the device
 enum { EVB_KIND_NONE = 0, EVB_KIND_BUILD = 1, EVB_KIND_SUB = 2 };
 
-// Per-level plan, device resident.  Written by the plan kernels, read by hist / reduce / scan.
+// Per-level plan, device resident.  Written by k_tree_begin / k_sel_scan (root) and the last CTA of k_partition.
 struct LevelPlan {
     int32_t nbuild;   // build slots used at this level
-    int32_t nitems;   // partition work items at this level
+    int32_t npl;      // sibling pairs at this level (1 at the root)
     int64_t R;        // rows (local) inside build nodes
     int32_t n_sel;    // rows selected by the row mask (root only)
     int32_t pad;
-};
-
-struct HistGeom {
-    int BP;        // padded bins per image: 32/64/128/256
-    int NCH;       // channels per unit image (<= 4)
-    int FPL;       // feature slots per lane (1, 2 or 4): a unit covers 32 * FPL feature slots
-    int NFG;       // feature groups of 32 * FPL slots
-    int NCT;       // channel groups of 4
-    int U;         // units = NFG*NCT
-    int UB;        // units (consumer warps) per block
-    int NUG;       // unit groups = ceil(U/UB)
-    int stages;    // staged tiles in flight
-    int G;         // row-range blocks (grid.x)
-    bool q;        // geometry of the fixed-point kernel
-    int PG;        // piece slots per unit group = G + max build slots
-    size_t smem;   // dynamic shared memory per block
-    size_t img_floats;   // floats per unit image in scratch: FPL*NCH*nbins*32
 };
 
 // geometry of the register-direct fixed-point histogram kernel (evb_histq2.cu)
@@ -72,11 +54,18 @@ struct Q2Geom {
     int ntail;     // features kept beside the gradient word in xE (nfeats % 16 when that is 1..4, else 0)
     int nmain;     // features kept in xH
     int RSH;       // bytes per row of xH
-    int SC;        // feature columns per bin of the accumulators
     int G;         // grid.x
-    int TE;        // tiles of 32 rows between two flushes of a CTA's image
     int min_rows;  // rows per CTA below which fewer CTAs take part
-    int QB;        // bits of the fixed-point gradient: |q| < 2^QB (26 or 24)
+    size_t smem;
+};
+
+// geometry of the integer histogram kernel for any loss (evb_histg.cuh)
+constexpr int EVB_MAX_Q = 72; // quantised channels: 2 K + 1, K <= 32
+struct HGeom {
+    int nq, per, ngc;   // channels; channels per CTA; channel groups (grid.z)
+    int W, wper, ngf;   // words of a row; words per CTA; feature groups (grid.y)
+    int pack, cnt;      // packed words of unit-weight least squares; a plane of row counts in channel group 0
+    int qbits, TE, min_rows, threads, G;
     size_t smem;
 };
 
@@ -94,7 +83,7 @@ struct evb_handle {
     // row data
     void *edges_d;     // edges of the raw matrix the handle was made from (evb_create_m), dtype edges_dtype
     int edges_dtype, nedges;
-    uint8_t *xT;       // [n][RS]  observation-major bins (1..B), zero padded
+    uint8_t *xT;       // [n][RS]  observation-major bins (1..B), zero padded; null when xH / xE hold them
     uint8_t *xC;       // [nfeats][n] feature-major copy (the layout of the caller's x_bin) read by the row partition
     float *grad;       // [n][GS]  g_1..g_K,h_1..h_K,w,(pad)
     float *pred;       // [n][K]
@@ -113,8 +102,9 @@ struct evb_handle {
 
     // node state, indexed by heap id 0..nn (0 unused); children of level D-1 nodes need ids < 2^D
     int32_t *seg_start, *seg_cnt; // local row segment of each node
-    int32_t *gcnt;                // global (all ranks) row count
-    int32_t *nleft, *gnleft;      // left-child row count of split nodes, local / global (gnleft == nleft when world == 1)
+    int32_t *cur_l, *cur_r;       // partition cursors of split nodes
+    uint32_t *ticket;             // [nn+2] features of a node whose scan is done; entry 0: CTAs of k_partition that are done
+    int32_t *pl;                  // 2 x {pl_node, pl_cum}[maxslots+1]: sibling pairs of a level and the running sum of their rows
     uint8_t *kind;
     int32_t *bslot;
     double *nsum;                 // [nn+1][C]
@@ -126,12 +116,11 @@ struct evb_handle {
     LevelPlan *plan;       // [D+1]
     int32_t *cum;          // [maxslots+1] exclusive prefix of build-node row counts (current level)
     int32_t *slot_node;    // [maxslots]
-    int32_t *item_node, *item_chunk, *item_left, *item_lprefix; // partition items
-    uint32_t *item_bits;   // [max_items][EVB_PART_CHUNK/32]
-    int max_items, maxslots;
+    int maxslots;
     int32_t *scan_tmp;     // block counts for the mask compaction
     double *fbest_gain;    // [nodes of a level][nfeats] per-feature best split of the scan
     int32_t *fbest_bin;
+    double *fbest_left;    // [nodes of a level][nfeats][3] left sums of that split (one output)
     double *obl_gain;      // oblivious trees: [nodes of a level + 1][nfeats * B] gain of every candidate, last row = level totals
     double *obl_best;      // [2] gain and candidate index (-1: none) of the level's shared split
     int *d_err;            // device error word
@@ -146,34 +135,31 @@ struct evb_handle {
     int ev_metric, ev_blocks;
     double last_eval[2]; // sums of the tree collected last
 
-    // fixed-point histogram variant (mse, one target): gradq holds the integer words of every row
-    bool use_q, unit_w;   // unit_w: no weights were given, the w channel is a row count
-    bool q_active;        // the current geometry is the fixed-point one (no column sample)
-    bool gradq_valid;     // gradq holds the words of the current gradients
-    int32_t *gradq;       // [n] fixed-point g, or [n][2] fixed-point g and w when weights were given
-    unsigned *d_gmax;     // bits of max |g| over the rows, filled by the gradient kernels
-    double *d_qinv;       // [2] 2^-s of the g words / of the w words
-    float wscale; double winv;
+    // fixed-point gradients (evb_histg.cuh)
+    bool unit_w;          // no weights were given: the w channel is a row count
+    bool gradq_valid;     // the fixed-point words are those of the current gradients
+    int nq, ng;           // quantised channels; those of them that change from round to round (all but the weight)
+    HGeom hgeo;
+    int32_t *gradq;       // words of all rows, channel group by channel group
+    unsigned *d_gmax;     // [nq] bits of max |g| over the rows, filled by the gradient kernels
+    double *d_qinv;       // [nq] 2^-s of every channel
+    int SC;               // feature columns per bin of the accumulators
+    unsigned long long *hsum_q;   // [maxslots][B][nq][SC] sums of q per build slot
+    uint32_t *hcnt_q;             // [maxslots][B][SC] row counts
 
-    // register-direct variant (unit weights): rows as 16-byte chunks + {q, tail bins} per row, integer accumulators
+    // register-direct variant (mse, one target, unit weights, many rows): rows as 16-byte chunks + {q, tail bins} per row
     bool use_q2;
     Q2Geom q2;
     uint8_t *xH;                  // [n][q2.RSH]
     uint2 *xE;                    // [n] {fixed-point gradient, bins of the tail features}
-    unsigned long long *hsum_q;   // [maxslots][B][q2.SC] sums of q per build slot
-    uint32_t *hcnt_q;             // [maxslots][B][q2.SC] row counts
 
     // quantile loss: work memory of the per-leaf order-statistic selection
     uint32_t *qs_cnt, *qs_prefix, *qs_rank; float *qs_gamma;
 
     // histograms
-    HistGeom hg;
-    int hist_mode;    // EVB_HIST_MODE environment override (kernel variants / diagnostics)
     double *hist;     // [2^(D-2) nodes][F][C][B] retained for the subtraction trick
     int hist_nodes;   // nodes with id < hist_nodes are retained
-    double *hcomp;    // [maxslots][F][C][B] freshly built histograms of the level (allreduce buffer)
-    float *scratch;   // [NUG][PG][UB][NCH][B][32] per-piece partial images
-    size_t scratch_floats;
+    double *hcomp;    // [maxslots][F][C][B] freshly built histograms of the level (exchanged between ranks; null on one GPU)
 
     // pinned host staging, double buffered so that tree t+1 can be enqueued before tree t is collected
     void *h_tree[2]; size_t h_tree_bytes;
@@ -210,32 +196,34 @@ struct evb_handle {
 // evb_rows.cu
 int32_t evb_launch_transpose(evb_handle *h, const uint8_t *xcol_dev, int64_t ld, int64_t nrows, int j0, int nj, uint8_t *xT, int RS, cudaStream_t st);
 int32_t evb_launch_grads(evb_handle *h);
-int32_t evb_launch_quantize(evb_handle *h);
 int32_t evb_launch_rows_init(evb_handle *h, int use_mask, uint8_t mask_cond);
 int32_t evb_pcg_tables(int dev);
 void evb_pcg_advance(uint64_t gen[6], int64_t n);
-int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode); // mode: see FinArgs in evb_rows.cu
+int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode, void *publish_to); // pinned host memory for the finished tree or null; mode: see FinArgs in evb_rows.cu
 int32_t evb_launch_quantile_leaves(evb_handle *h, bool use_mask, uint8_t mask_cond);
 int32_t evb_launch_nidx_from_partition(evb_handle *h, uint32_t *out_dev);
-int32_t evb_launch_eval(evb_handle *h, const float *fixed_leaf_dev);
+int32_t evb_launch_eval(evb_handle *h, const float *fixed_leaf_dev, void *publish_to);
 int32_t evb_upload_binarize(evb_handle *h, const void *x, int32_t dtype, const void *edges, int32_t nedges); // raw host matrix -> h->xC
 // evb_hist.cu
-int32_t evb_hist_configure(evb_handle *h);   // fills h->hg from p / nfeats (uses max F = nfeats)
-int32_t evb_launch_hist(evb_handle *h, int level);
-int32_t evb_launch_hist_reduce(evb_handle *h, int level);
+int evb_hist_mode_env();
+// evb_histg.cu
+int32_t evb_hg_configure(evb_handle *h);
+size_t evb_hg_q_words(const evb_handle *h);
+int32_t evb_launch_histg(evb_handle *h, int level);
+int32_t evb_launch_acc_clear(evb_handle *h, int level);
+int32_t evb_launch_acc_to_hcomp(evb_handle *h, int level);
+// The split scan reads the integer accumulators itself unless ranks exchange histograms as doubles.
+static inline bool evb_acc_direct(const evb_handle *h) { return h->world == 1; }
 // evb_histq2.cu
+bool evb_q2_wanted(const evb_handle *h);
 int32_t evb_q2_configure(evb_handle *h);
 int32_t evb_q2_build_layout(evb_handle *h);
 int32_t evb_q2_clear_layout(evb_handle *h);
-int32_t evb_launch_q2_quantize(evb_handle *h);
 int32_t evb_launch_histq2(evb_handle *h, int level);
-int32_t evb_launch_q2_reduce(evb_handle *h, int level);
-int32_t evb_launch_q2_clear(evb_handle *h, int level);
-bool evb_q2_direct(const evb_handle *h);
 // evb_tree.cu
-int32_t evb_launch_tree_reset(evb_handle *h);
+int32_t evb_launch_tree_begin(evb_handle *h, bool quantize, bool all_rows, const uint32_t *gen_js_host);
 int32_t evb_launch_scan(evb_handle *h, int level);
-int32_t evb_launch_partition(evb_handle *h, int level); // plan + flags + prefix (+allreduce) + level plan + scatter
+int32_t evb_launch_partition(evb_handle *h, int level); // rows of the level's split nodes, plan of the next level
 int32_t evb_launch_lonely_barrier(evb_handle *h, int *flags, int *seq, unsigned max_polls);
 int32_t evb_check_device(int device); // evb_rows.cu: makes `device` current
 void evb_predict_trim(int device);       // evb_predict.cu: kept work buffers back to the block cache
@@ -274,8 +262,6 @@ int32_t evb_d2h_staged(void *dst_host, const void *src_dev, size_t bytes, cudaSt
 int32_t evb_h2d_staged(void *dst_dev, const void *src_host, size_t bytes, cudaStream_t st, bool drain = true);
 int32_t evb_h2d_staged_strided(void *dst_dev, const void *src_host, size_t seg_bytes, size_t nseg, size_t stride, cudaStream_t st, bool drain = true);
 
-// EVB_HIST_MODE of the environment, reduced to the documented values (0: TMA bulk staging, 1: cp.async staging)
-int evb_hist_mode_env();
 // timing helpers (evb_api.cu)
 void evb_tic(evb_handle *h, int cls);
 void evb_toc(evb_handle *h, int cls);

@@ -126,21 +126,21 @@ __global__ void k_transpose(const uint8_t *xcol, long long ld, long long nrows, 
     }
 }
 
-// range check of the binned matrix: counts values outside 1..nbins
-__global__ void k_check_bins(const uint8_t *xT, long long n, int RS, int nfeats, int nbins, int *err) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// range check of the binned matrix
+__global__ void k_check_bins(const uint8_t *xC, size_t total, int nbins, int *err) {
     bool bad = false;
-    for (int j = 0; j < nfeats; ++j) {
-        const int v = xT[(size_t)i * RS + j];
-        bad |= (v < 1 || v > nbins);
-    }
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) { const int v = xC[i]; bad |= v < 1 || v > nbins; }
     if (bad) atomicCAS(err, 0, EVB_DERR_BIN_RANGE);
 }
 
 #undef REC
-__global__ void k_init_state(float *grad, float *pred, const float *w, const float *pred0, const float *mu, long long n, int K, int GS, int NCH, int wch) {
+// wmax: null, or the maximum of the weights goes there (they are a channel of the histograms then)
+__global__ void __launch_bounds__(256) k_init_state(float *grad, float *pred, const float *w, const float *pred0, const float *mu, long long n, int K, int GS, int NCH, int wch, unsigned *wmax) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (wmax) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, i < n ? __float_as_uint(w[i]) : 0u);
+        if ((threadIdx.x & 31) == 0 && m > *(volatile unsigned *)wmax) atomicMax(wmax, m);
+    }
     if (i >= n) return;
     float *rec = grad + (size_t)i * GS;
     for (int c = 0; c < GS; ++c) rec[c] = 0.0f;
@@ -149,58 +149,28 @@ __global__ void k_init_state(float *grad, float *pred, const float *w, const flo
 }
 
 // ---------------------------------------------------------------------------------- gradients
-// max |g| over the rows of a 256-thread block -> global maximum (bit pattern of a non-negative float, which orders
-// like an unsigned integer).  Every thread of the block must call it.
-__device__ __forceinline__ void block_absmax(float v, unsigned *gmax) {
-    __shared__ unsigned s_max[8];
-    unsigned m = __reduce_max_sync(FULL, __float_as_uint(fabsf(v)));
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
+// max |g| of every changing channel over the rows of a 256-thread block -> global maxima (bit patterns of non-negative
+// floats, which order like unsigned integers).  rec: the thread's gradient record, or null.  Every thread calls it.
+__device__ __forceinline__ void block_absmax(const float *rec, int NCH, int ng, unsigned *gmax) {
+    __shared__ unsigned s_max[EVB_MAX_Q];
+    if (threadIdx.x < ng) s_max[threadIdx.x] = 0u;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int q = 1; q < 8; ++q) m = max(m, s_max[q]);
-        if (m > *(volatile unsigned *)gmax) atomicMax(gmax, m);
+    for (int c = 0; c < ng; ++c) {
+        const unsigned m = __reduce_max_sync(FULL, rec ? __float_as_uint(fabsf(rec[gpos(c, NCH)])) : 0u);
+        if ((threadIdx.x & 31) == 0 && m > *(volatile unsigned *)(s_max + c)) atomicMax(s_max + c, m);
     }
+    __syncthreads();
+    if (threadIdx.x < ng && s_max[threadIdx.x] > *(volatile unsigned *)(gmax + threadIdx.x)) atomicMax(gmax + threadIdx.x, s_max[threadIdx.x]);
 }
-__global__ void __launch_bounds__(256) k_grads(int loss, int K, int GS, int NCH, int elided, int ycols, long long n, const float *pred, const void *y, float *grad, unsigned *gmax,
+__global__ void __launch_bounds__(256) k_grads(int loss, int K, int GS, int NCH, int elided, int ycols, long long n, const float *pred, const void *y, float *grad, unsigned *gmax, int ng,
                                                AlphaSet alpha) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float g0 = 0.0f;
-    if (i < n) {
-        grad_row(loss, K, NCH, elided != 0, pred + (size_t)i * K, y, ycols, i, grad + (size_t)i * GS, alpha);
-        g0 = grad[(size_t)i * GS];
-    }
-    if (gmax) block_absmax(g0, gmax);
-}
-// Fixed-point gradient of every row for the integer histogram kernel: q = rint(g * 2^s) with 2^s the largest power
-// of two that keeps max |g| * 2^s below 2^qbits (26 when no weights were given and the kernel counts rows inside the
-// low word, else 29); the weight likewise with its own scale.  2^-s goes to qinv for the reduce kernel.
-__global__ void __launch_bounds__(256) k_quantize(const float *grad, int32_t *gradq, long long n, const unsigned *gmax, double *qinv,
-                                                   float wscale, double winv, int unit_w) {
-    const int qbits = unit_w ? 26 : 29;
-    const float m = __uint_as_float(*gmax);
-    float sc = 1.0f;
-    double inv = 1.0;
-    if (m > 0.0f && m < INFINITY) {
-        int e;
-        frexpf(m, &e); // m = f * 2^e, f in [0.5, 1)
-        sc = ldexpf(1.0f, qbits - e);
-        inv = ldexp(1.0, e - qbits);
-    }
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) { qinv[0] = inv; qinv[1] = unit_w ? 1.0 : winv; }
-    if (i >= n) return;
-    const float2 gw = reinterpret_cast<const float2 *>(grad)[i * 2]; // record = g, w, pad, pad
-    const int q = __float2int_rn(gw.x * sc);
-    if (unit_w) gradq[i] = q;
-    else reinterpret_cast<int2 *>(gradq)[i] = make_int2(q, __float2int_rn(gw.y * wscale));
+    float *rec = i < n ? grad + (size_t)i * GS : nullptr;
+    if (rec) grad_row(loss, K, NCH, elided != 0, pred + (size_t)i * K, y, ycols, i, rec, alpha);
+    block_absmax(rec, NCH, ng, gmax);
 }
 
 // ---------------------------------------------------------------------------------- row sampling
-__global__ void k_rows_identity(uint32_t *rows, long long n, int32_t *nleft0) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) rows[i] = (uint32_t)i;
-    if (i == 0) nleft0[0] = (int32_t)n;
-}
 constexpr int SEL_CHUNK = 2048, SEL_THREADS = 256;
 __global__ void __launch_bounds__(SEL_THREADS) k_sel_count(const uint8_t *mask, uint8_t cond, long long n, int32_t *bcnt) {
     __shared__ int s[SEL_THREADS / 32];
@@ -268,7 +238,8 @@ __global__ void __launch_bounds__(SEL_THREADS) k_sel_pcg(const uint64_t *gen, ui
         bcnt[blockIdx.x] = tot;
     }
 }
-__global__ void __launch_bounds__(1024) k_sel_scan(int32_t *bcnt, int nblocks, int32_t *nleft0) {
+struct RootPlan { int32_t *seg_cnt, *cum, *slot_node, *pl_node, *pl_cum; uint8_t *kind; LevelPlan *plan; };
+__global__ void __launch_bounds__(1024) k_sel_scan(int32_t *bcnt, int nblocks, RootPlan r) {
     __shared__ int sm[33];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int carry = 0;
@@ -291,7 +262,12 @@ __global__ void __launch_bounds__(1024) k_sel_scan(int32_t *bcnt, int nblocks, i
         carry += sm[32];
         __syncthreads();
     }
-    if (threadIdx.x == 0) nleft0[0] = carry;
+    if (threadIdx.x == 0) { // the root: its rows are the sampled ones
+        r.seg_cnt[1] = carry; r.kind[1] = EVB_KIND_BUILD;
+        r.cum[0] = 0; r.cum[1] = carry; r.slot_node[0] = 1;
+        r.pl_node[0] = 1; r.pl_cum[0] = 0; r.pl_cum[1] = carry;
+        r.plan[1].nbuild = 1; r.plan[1].npl = 1; r.plan[1].R = carry; r.plan[1].n_sel = carry;
+    }
 }
 __global__ void __launch_bounds__(SEL_THREADS) k_sel_scatter(const uint8_t *mask, uint8_t cond, long long n, const int32_t *boff, uint32_t *rows) {
     constexpr int NW = SEL_CHUNK / 32;
@@ -331,14 +307,23 @@ struct FinArgs {
     float *pred, *grad;
     const void *y;
     uint32_t *nidx;
-    unsigned *gmax; // non-null: track max |g| of the gradients computed here (fixed-point histogram variant)
+    unsigned *gmax; // [ng] max |g| of the gradients computed here
+    int ng;
     long long n;
     int RS, K, GS, NCH, elided, loss, nn, ycols, compute_grads, packed_in_smem;
     AlphaSet alpha;
     int mode; // 0: traverse, add the leaf, next gradients; 1: traverse only (leaf ids); 2: leaf ids are in nidx, add + gradients
+    const uint4 *pub_src; // the finished tree goes to pinned host memory from here (pub_n 16-byte words; 0: a later kernel does it)
+    uint4 *pub_dst;
+    int pub_n;
 };
+// A copy node of the graph would cost 5 to 10 us between the kernels of two trees; these stores cost nothing.
+__device__ __forceinline__ void publish(const uint4 *src, uint4 *dst, int n) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
+}
 __global__ void __launch_bounds__(256) k_finalize(FinArgs a) {
     extern __shared__ uint32_t s_packed[];
+    if (blockIdx.x == 0) publish(a.pub_src, a.pub_dst, a.pub_n);
     const uint32_t *packed = a.t_packed;
     if (a.packed_in_smem) {
         for (int i = threadIdx.x; i < a.nn; i += blockDim.x) s_packed[i] = a.t_packed[i];
@@ -346,18 +331,18 @@ __global__ void __launch_bounds__(256) k_finalize(FinArgs a) {
         packed = s_packed;
     }
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float g0 = 0.0f;
+    float *rec = nullptr;
     if (i < a.n) {
         const int nid = a.mode == 2 ? (int)a.nidx[i] : traverse(packed, a.xT + (size_t)i * a.RS);
         a.nidx[i] = (uint32_t)nid;
         float *p = a.pred + (size_t)i * a.K;
         if (a.mode != 1) pred_add(a.loss, a.K, p, a.t_pred + (size_t)(nid - 1) * a.K);
         if (a.compute_grads && a.mode != 1) {
-            grad_row(a.loss, a.K, a.NCH, a.elided != 0, p, a.y, a.ycols, i, a.grad + (size_t)i * a.GS, a.alpha);
-            g0 = a.grad[(size_t)i * a.GS];
+            rec = a.grad + (size_t)i * a.GS;
+            grad_row(a.loss, a.K, a.NCH, a.elided != 0, p, a.y, a.ycols, i, rec, a.alpha);
         }
     }
-    if (a.gmax && a.compute_grads) block_absmax(g0, a.gmax);
+    if (a.compute_grads && a.mode != 1) block_absmax(rec, a.NCH, a.ng, a.gmax);
 }
 
 // The same update with the rows of bins staged through shared memory: the CTA copies its 256 rows with fully
@@ -366,6 +351,7 @@ __global__ void __launch_bounds__(256) k_finalize(FinArgs a) {
 // rows fall into different banks.  Used when a row is at most 256 bytes.
 __global__ void __launch_bounds__(256) k_finalize_staged(FinArgs a) {
     extern __shared__ uint32_t s_fin[]; // [nn] packed tree, then [256][RS / 4 + 1] words of bins
+    if (blockIdx.x == 0) publish(a.pub_src, a.pub_dst, a.pub_n);
     uint32_t *s_tree = s_fin;
     uint32_t *s_rows = s_fin + a.nn;
     const int rw = a.RS >> 2, rwp = rw + 1; // words per row, padded
@@ -382,18 +368,18 @@ __global__ void __launch_bounds__(256) k_finalize_staged(FinArgs a) {
     }
     __syncthreads();
     const long long i = row0 + threadIdx.x;
-    float g0 = 0.0f;
+    float *rec = nullptr;
     if (i < a.n) {
         const int nid = traverse(s_tree, reinterpret_cast<const uint8_t *>(s_rows + threadIdx.x * rwp));
         a.nidx[i] = (uint32_t)nid;
         float *p = a.pred + (size_t)i * a.K;
         pred_add(a.loss, a.K, p, a.t_pred + (size_t)(nid - 1) * a.K);
         if (a.compute_grads) {
-            grad_row(a.loss, a.K, a.NCH, a.elided != 0, p, a.y, a.ycols, i, a.grad + (size_t)i * a.GS, a.alpha);
-            g0 = a.grad[(size_t)i * a.GS];
+            rec = a.grad + (size_t)i * a.GS;
+            grad_row(a.loss, a.K, a.NCH, a.elided != 0, p, a.y, a.ycols, i, rec, a.alpha);
         }
     }
-    if (a.gmax && a.compute_grads) block_absmax(g0, a.gmax);
+    if (a.compute_grads && a.mode != 1) block_absmax(rec, a.NCH, a.ng, a.gmax);
 }
 
 // The same update as a pipeline: a few CTAs per SM stay resident and walk over tiles of 256 rows.  The tree (and, for
@@ -420,6 +406,7 @@ __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
     // words, so that the row buffers start on a 16-byte boundary (the copies into them are 16 bytes wide)
     extern __shared__ __align__(16) uint32_t s_fp[];
     const FinArgs &f = a.f;
+    if (blockIdx.x == 0) publish(f.pub_src, f.pub_dst, f.pub_n);
     const int nnp = (f.nn + 3) & ~3;
     uint32_t *s_tree = s_fp;
     float *s_leaf = reinterpret_cast<float *>(s_fp + nnp);
@@ -449,7 +436,7 @@ __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float gm = 0.0f;
+    float gm = 0.0f, hm = 0.0f; // largest |g|, |h| of this thread's rows
     int buf = 0;
     stage(blockIdx.x, 0);
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, buf ^= 1) {
@@ -478,12 +465,17 @@ __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
             }
             if (f.compute_grads) {
                 grad_row(loss, MSE1 ? 1 : f.K, NCH, MSE1 ? true : f.elided != 0, p, f.y, MSE1 ? 1 : f.ycols, i, f.grad + (size_t)i * f.GS, f.alpha);
-                gm = fmaxf(gm, fabsf(f.grad[(size_t)i * f.GS]));
+                const float *rec = f.grad + (size_t)i * f.GS;
+                gm = fmaxf(gm, fabsf(rec[0]));
+                if (!MSE1 && f.ng > 1) hm = fmaxf(hm, fabsf(rec[gpos(1, NCH)]));
             }
         }
         __syncthreads(); // everybody is done with this buffer: the next iteration refills it
     }
-    if (f.gmax && f.compute_grads) block_absmax(gm, f.gmax);
+    if (f.compute_grads) {
+        const float m2[2] = {gm, hm};
+        block_absmax(m2, 2, f.ng, f.gmax); // K == 1: one or two channels
+    }
 }
 
 // ---------------------------------------------------------------------------------- quantile leaves
@@ -709,7 +701,7 @@ __global__ void __launch_bounds__(256) k_eval_tree(EvalArgs a) {
         a.part[2 * blockIdx.x + 1] = tw;
     }
 }
-__global__ void __launch_bounds__(256) k_eval_sum(const double *part, int nblocks, double *out) {
+__global__ void __launch_bounds__(256) k_eval_sum(const double *part, int nblocks, double *out, const uint4 *pub_src, uint4 *pub_dst, int pub_n) {
     __shared__ double s_red[2][256];
     double tv = 0.0, tw = 0.0;
     for (int b = threadIdx.x; b < nblocks; b += 256) { tv += part[2 * b]; tw += part[2 * b + 1]; }
@@ -720,6 +712,8 @@ __global__ void __launch_bounds__(256) k_eval_sum(const double *part, int nblock
         __syncthreads();
     }
     if (threadIdx.x == 0) { out[0] = s_red[0][0]; out[1] = s_red[1][0]; }
+    __syncthreads(); // the sums are part of the block
+    publish(pub_src, pub_dst, pub_n);
 }
 
 } // namespace
@@ -741,30 +735,24 @@ int32_t evb_launch_transpose(evb_handle *, const uint8_t *xcol_dev, int64_t ld, 
 }
 
 int32_t evb_launch_check_bins(evb_handle *h) {
-    k_check_bins<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->xT, h->n, h->RS, h->nfeats, h->B, h->d_err);
+    const size_t total = (size_t)h->n * h->nfeats;
+    k_check_bins<<<(unsigned)std::min<size_t>((total + 255) / 256, (size_t)h->num_sms * 16), 256, 0, h->st>>>(h->xC, total, h->B, h->d_err);
     EVB_CUDA(cudaGetLastError());
     return EVB_OK;
 }
 
 int32_t evb_launch_init_state(evb_handle *h, const float *w_dev, const float *pred0_dev, const float *mu_dev) {
-    k_init_state<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->grad, h->pred, w_dev, pred0_dev, mu_dev, h->n, h->K, h->GS, h->rec_nch, h->Ce - 1);
+    k_init_state<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->grad, h->pred, w_dev, pred0_dev, mu_dev, h->n, h->K, h->GS, h->rec_nch, h->Ce - 1,
+                                                                      h->unit_w ? nullptr : h->d_gmax + h->nq - 1);
     EVB_CUDA(cudaGetLastError());
     return EVB_OK;
 }
 
 int32_t evb_launch_grads(evb_handle *h) {
-    if (h->use_q) EVB_CUDA(cudaMemsetAsync(h->d_gmax, 0, sizeof(unsigned), h->st));
+    EVB_CUDA(cudaMemsetAsync(h->d_gmax, 0, sizeof(unsigned) * h->ng, h->st));
     evb_tic(h, EVB_T_GRADS);
     k_grads<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->p.loss, h->K, h->GS, h->rec_nch, h->Ce != h->C, h->ycols, h->n, h->pred, h->y, h->grad,
-                                                                h->use_q ? h->d_gmax : nullptr, evb_alpha_set(h));
-    evb_toc(h, EVB_T_GRADS);
-    EVB_CUDA(cudaGetLastError());
-    return EVB_OK;
-}
-
-int32_t evb_launch_quantize(evb_handle *h) {
-    evb_tic(h, EVB_T_GRADS);
-    k_quantize<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->grad, h->gradq, h->n, h->d_gmax, h->d_qinv, h->wscale, h->winv, h->unit_w ? 1 : 0);
+                                                                h->d_gmax, h->ng, evb_alpha_set(h));
     evb_toc(h, EVB_T_GRADS);
     EVB_CUDA(cudaGetLastError());
     return EVB_OK;
@@ -807,29 +795,29 @@ void evb_pcg_advance(uint64_t gen[6], int64_t n) {
     }
 }
 
+// the sampled rows of a tree, after k_tree_begin
 int32_t evb_launch_rows_init(evb_handle *h, int use_mask, uint8_t mask_cond) {
+    if (!use_mask) return EVB_OK;
+    const int nblocks = (int)((h->n + SEL_CHUNK - 1) / SEL_CHUNK);
+    const RootPlan r{h->seg_cnt, h->cum, h->slot_node, h->pl, h->pl + h->maxslots + 1, h->kind, h->plan};
     evb_tic(h, EVB_T_ROWS_INIT);
-    if (!use_mask) {
-        k_rows_identity<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->rows[0], h->n, h->nleft);
-    } else {
-        const int nblocks = (int)((h->n + SEL_CHUNK - 1) / SEL_CHUNK);
-        if (use_mask == EVB_MASK_PCG) k_sel_pcg<<<nblocks, SEL_THREADS, 0, h->st>>>(h->gen_d, mask_cond, h->n, h->mask_d, h->scan_tmp);
-        else k_sel_count<<<nblocks, SEL_THREADS, 0, h->st>>>(h->mask_d, mask_cond, h->n, h->scan_tmp);
-        k_sel_scan<<<1, 1024, 0, h->st>>>(h->scan_tmp, nblocks, h->nleft);
-        k_sel_scatter<<<nblocks, SEL_THREADS, 0, h->st>>>(h->mask_d, mask_cond, h->n, h->scan_tmp, h->rows[0]);
-    }
+    if (use_mask == EVB_MASK_PCG) k_sel_pcg<<<nblocks, SEL_THREADS, 0, h->st>>>(h->gen_d, mask_cond, h->n, h->mask_d, h->scan_tmp);
+    else k_sel_count<<<nblocks, SEL_THREADS, 0, h->st>>>(h->mask_d, mask_cond, h->n, h->scan_tmp);
+    k_sel_scan<<<1, 1024, 0, h->st>>>(h->scan_tmp, nblocks, r);
+    k_sel_scatter<<<nblocks, SEL_THREADS, 0, h->st>>>(h->mask_d, mask_cond, h->n, h->scan_tmp, h->rows[0]);
     evb_toc(h, EVB_T_ROWS_INIT);
+    h->tm.launches[EVB_T_ROWS_INIT] += 2;
     EVB_CUDA(cudaGetLastError());
     return EVB_OK;
 }
 
-int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode) {
+int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode, void *publish_to) {
     FinArgs a;
     a.xT = h->xT; a.t_packed = h->t_packed; a.t_pred = h->t_pred; a.pred = h->pred; a.grad = h->grad; a.y = h->y;
     a.nidx = h->nidx; a.n = h->n; a.RS = h->RS; a.K = h->K; a.GS = h->GS; a.NCH = h->rec_nch; a.elided = h->Ce != h->C; a.loss = h->p.loss; a.nn = h->nn;
-    a.gmax = h->use_q ? h->d_gmax : nullptr;
-    if (h->use_q && compute_grads) EVB_CUDA(cudaMemsetAsync(h->d_gmax, 0, sizeof(unsigned), h->st));
+    a.gmax = h->d_gmax; a.ng = h->ng; // cleared by the root's scan
     a.ycols = h->ycols; a.compute_grads = compute_grads ? 1 : 0; a.alpha = evb_alpha_set(h); a.mode = mode;
+    a.pub_src = reinterpret_cast<const uint4 *>(h->plan); a.pub_dst = static_cast<uint4 *>(publish_to); a.pub_n = publish_to ? (int)(h->h_tree_bytes / 16) : 0;
     const size_t smem = (size_t)h->nn * 4;
     a.packed_in_smem = smem <= 40 * 1024 ? 1 : 0;
     const size_t staged = smem + (size_t)256 * (h->RS + 4);
@@ -839,7 +827,7 @@ int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode) {
     // pipelined kernel: rows from the chunk layout of the fixed-point histogram kernel when it exists, else from xT
     FinPipeArgs pa;
     pa.f = a;
-    const bool from_q2 = h->use_q2; // xH holds feature f at byte f of the row, the tail features follow in xE
+    const bool from_q2 = h->use_q2; // evb_create sees to it that this kernel can run then; xH holds feature f at byte f of the row, the tail features follow in xE
     pa.rowsA = from_q2 ? h->xH : h->xT;
     pa.xE = from_q2 && h->q2.ntail > 0 ? h->xE : nullptr;
     pa.strideA = from_q2 ? h->q2.RSH : h->RS;
@@ -878,7 +866,7 @@ int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode) {
 
 // applies the current tree (or, with `fixed_leaf_dev`, one leaf for every row) to the evaluation predictions and
 // leaves the metric sums in h->d_evsum
-int32_t evb_launch_eval(evb_handle *h, const float *fixed_leaf_dev) {
+int32_t evb_launch_eval(evb_handle *h, const float *fixed_leaf_dev, void *publish_to) {
     EvalArgs a;
     a.xT = h->ev_xT; a.t_packed = h->t_packed; a.t_pred = h->t_pred; a.fixed_leaf = fixed_leaf_dev; a.pred = h->ev_pred;
     a.y = h->ev_y; a.w = h->ev_w; a.part = h->ev_part; a.n = h->ev_n; a.RS = h->RS; a.K = h->K; a.loss = h->p.loss;
@@ -887,7 +875,8 @@ int32_t evb_launch_eval(evb_handle *h, const float *fixed_leaf_dev) {
     a.packed_in_smem = smem <= 40 * 1024 ? 1 : 0;
     evb_tic(h, EVB_T_FINALIZE);
     k_eval_tree<<<h->ev_blocks, 256, (a.packed_in_smem && !fixed_leaf_dev) ? smem : 0, h->st>>>(a);
-    k_eval_sum<<<1, 256, 0, h->st>>>(h->ev_part, h->ev_blocks, h->d_evsum);
+    k_eval_sum<<<1, 256, 0, h->st>>>(h->ev_part, h->ev_blocks, h->d_evsum, reinterpret_cast<const uint4 *>(h->plan), static_cast<uint4 *>(publish_to),
+                                     publish_to ? (int)(h->h_tree_bytes / 16) : 0);
     evb_toc(h, EVB_T_FINALIZE);
     h->tm.launches[EVB_T_FINALIZE] += 1; // two kernels inside one timed bracket
     EVB_CUDA(cudaGetLastError());

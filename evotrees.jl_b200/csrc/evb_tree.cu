@@ -5,8 +5,9 @@
 // ext/EvoTreesKernelAbstractionsExt/fit-utils.jl:9-31).  Everything a level needs (active nodes, segment
 // bounds, build/subtract choice, work lists) lives in device memory, so the host enqueues a fixed sequence of
 // launches per level and never reads anything back until the tree is complete.
-#include "evb_internal.cuh"
+#include "evb_histg.cuh"
 #include <float.h>
+#include <algorithm>
 
 namespace {
 
@@ -52,44 +53,43 @@ __device__ __forceinline__ int block_excl_scan(int v, int *sm, int *total) {
     return incl - v + sm[wid];
 }
 
-// ------------------------------------------------------------------------------------------ reset / root
-struct ResetArgs {
-    int32_t *seg_start, *seg_cnt, *gcnt, *nleft, *gnleft, *bslot, *t_feat;
+// ------------------------------------------------------------------------------------------ begin of a tree
+struct BeginArgs {
+    int32_t *seg_start, *seg_cnt, *bslot, *t_feat, *cum, *slot_node, *pl_node, *pl_cum;
     uint8_t *kind, *t_bin, *t_split;
     float *t_gain, *t_w, *t_pred;
     uint32_t *t_packed;
     double *nsum;
     LevelPlan *plan;
-    int nids, nn, K, C, D;
+    uint32_t *ticket, *rows;
+    const uint32_t *gen_js_host; // pinned: generator state and column sample of this tree
+    uint32_t *gen_js;
+    int ngen_js;
+    int nids, nn, K, C, D, all_rows;
+    evb_hg::QuantArgs q; // q.grad null: the fixed-point gradients are those of the last tree
 };
-__global__ void k_tree_reset(ResetArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per row and per node: clears the tree, lists all rows and plans the root (without a row sample), and turns the
+// gradients into fixed-point numbers.
+__global__ void __launch_bounds__(256) k_tree_begin(BeginArgs a) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i < a.ngen_js) a.gen_js[i] = __ldcv(a.gen_js_host + i);
+    if (a.q.grad) evb_hg::quantize(a.q, i);
+    if (a.all_rows && i < a.q.n) a.rows[i] = (uint32_t)i;
     if (i < a.nids) {
-        a.seg_start[i] = 0; a.seg_cnt[i] = 0; a.gcnt[i] = 0; a.kind[i] = 0; a.bslot[i] = 0;
-        if (i > 0) { a.nleft[i] = 0; if (a.gnleft != a.nleft) a.gnleft[i] = 0; } // entry 0 carries the root count
+        const bool root = i == 1 && a.all_rows;
+        a.seg_start[i] = 0; a.seg_cnt[i] = root ? (int32_t)a.q.n : 0; a.kind[i] = root ? EVB_KIND_BUILD : EVB_KIND_NONE; a.bslot[i] = 0; a.ticket[i] = 0u;
         for (int c = 0; c < a.C; ++c) a.nsum[(size_t)i * a.C + c] = 0.0;
+        if (root) {
+            a.cum[0] = 0; a.cum[1] = (int32_t)a.q.n; a.slot_node[0] = 1;
+            a.pl_node[0] = 1; a.pl_cum[0] = 0; a.pl_cum[1] = (int32_t)a.q.n;
+            a.plan[1].nbuild = 1; a.plan[1].npl = 1; a.plan[1].R = a.q.n; a.plan[1].n_sel = (int32_t)a.q.n;
+        }
     }
     if (i < a.nn) {
         a.t_feat[i] = 0; a.t_bin[i] = 0; a.t_split[i] = 0; a.t_gain[i] = 0.f; a.t_w[i] = 0.f; a.t_packed[i] = 0u;
         for (int k = 0; k < a.K; ++k) a.t_pred[(size_t)i * a.K + k] = 0.f;
     }
-    if (i >= 2 && i <= a.D) { a.plan[i].nbuild = 0; a.plan[i].nitems = 0; a.plan[i].R = 0; }
-}
-
-struct RootArgs {
-    int32_t *seg_start, *seg_cnt, *gcnt, *bslot, *cum, *slot_node;
-    const int32_t *nleft, *gnleft;
-    uint8_t *kind;
-    LevelPlan *plan;
-};
-__global__ void k_root_plan(RootArgs a) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const int nsel = a.nleft[0];
-        a.seg_start[1] = 0; a.seg_cnt[1] = nsel; a.gcnt[1] = a.gnleft[0];
-        a.kind[1] = EVB_KIND_BUILD; a.bslot[1] = 0;
-        a.cum[0] = 0; a.cum[1] = nsel; a.slot_node[0] = 1;
-        a.plan[1].nbuild = 1; a.plan[1].R = nsel; a.plan[1].n_sel = nsel; a.plan[1].nitems = 0;
-    }
+    if (i >= 2 && i <= a.D) { a.plan[i].nbuild = 0; a.plan[i].npl = 0; a.plan[i].R = 0; }
 }
 
 // ------------------------------------------------------------------------------------------ split scan
@@ -109,6 +109,7 @@ struct ScanArgs {
     uint32_t *t_packed;
     double *fbest_gain; // [nodes of the level][F] best gain of each feature
     int32_t *fbest_bin; // [nodes of the level][F] its bin (0-based) or -1
+    double *fbest_left; // [nodes of the level][F][3] its left sums (one output)
     // oblivious trees (null otherwise): [nodes of the level + 1][F * B] gain of every candidate (0: not eligible),
     // the last row receives the level totals; obl_best = {gain, candidate index or -1} of the shared split
     double *obl_gain, *obl_best;
@@ -122,11 +123,17 @@ struct ScanArgs {
     int F, C, K, B, level, D, hist_nodes, loss;
     int elide_h;        // mse: the h channels equal twice the w channel and are rebuilt instead of read
     // non-null: the built histograms are read straight from the integer accumulators of the fixed-point kernel
-    // ([slot][bin][SC] sums of q and row counts; g = sum * qinv[0], w = count, h = 2w) instead of from hcomp
+    // ([slot][bin][channel][SC] sums of q, [slot][bin][SC] row counts) instead of from hcomp
     const unsigned long long *qsum;
     const uint32_t *qcnt;
     const double *qinv;
-    int SC;
+    int SC, nq, unit_w;
+    // non-null: the last feature of a node to be scanned decides the node (one GPU, binary trees)
+    uint32_t *ticket;
+    unsigned *gmax;           // [ng] cleared by the root's scan: the gradient kernels of this tree start from zero
+    int ng;
+    int32_t *cur_l, *cur_r;   // where the partition puts the next left / right rows of a split node
+    const int32_t *seg_start, *seg_cnt;
     double neb; // -eta / bagging_size
     double lambda, L2, gamma, min_weight;
 };
@@ -175,6 +182,19 @@ __device__ __forceinline__ float leaf_value(const ScanArgs &a, const double *s, 
     return (float)(a.neb * g / fmax(DBL_EPSILON, h + a.lambda * s[C - 1] + a.L2));
 }
 
+// entry (channel c, bin b) of the histogram built for `slot`, feature slot f (feature id `feat`)
+__device__ __forceinline__ double built_entry(const ScanArgs &a, int slot, int f, uint32_t feat, int c, int b, int K, int C) {
+    if (a.qsum) {
+        const size_t cell = (size_t)slot * a.B + b;
+        const bool is_h2w = a.elide_h && c >= K && c < 2 * K; // h = 2w (src/loss.jl:52)
+        if (c < C - 1 && !is_h2w) return (double)(long long)__ldg(a.qsum + (cell * a.nq + c) * a.SC + feat) * __ldg(a.qinv + c);
+        const double w = a.unit_w ? (double)__ldg(a.qcnt + cell * a.SC + feat)
+                                  : (double)(long long)__ldg(a.qsum + (cell * a.nq + a.nq - 1) * a.SC + feat) * __ldg(a.qinv + a.nq - 1);
+        return is_h2w ? 2.0 * w : w;
+    }
+    return a.hcomp[(((size_t)slot * a.F + f) * C + c) * a.B + b];
+}
+
 // Sharded with peer access: sums the ranks' freshly built histograms for the feature slots this rank owns, by
 // loads from the peers' memory past the caches, in rank order (so the result does not depend on timing).  One CTA
 // per (build slot, owned feature); at the root level feature slot 0 is summed on every rank (it gives the root sums).
@@ -216,18 +236,7 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     // outputs and the channel tests fold away
     const int C = K1 ? 3 : a.C, K = K1 ? 1 : a.K, B = a.B, F = a.F;
     const uint32_t feat = a.js0[f];
-    const double *__restrict__ sm = a.hcomp + ((size_t)slot * F + f) * C * B;
-    const double qi = a.qsum ? a.qinv[0] : 0.0;
-    // entry (channel c, bin b) of the histogram built for `slot` and feature slot f
-    auto built = [&](int c, int b) -> double {
-        if (a.qsum) {
-            const size_t o = ((size_t)slot * B + b) * a.SC + feat;
-            if (c < K) return (double)(long long)__ldg(a.qsum + o) * qi;
-            const double w = (double)__ldg(a.qcnt + o);
-            return c == C - 1 ? w : 2.0 * w;
-        }
-        return sm[c * B + b];
-    };
+    auto built = [&](int c, int b) -> double { return built_entry(a, slot, f, feat, c, b, K, C); };
     const int m = 1 << (a.level - 1);
     const size_t FCB = (size_t)F * C * B;
     const double *__restrict__ hp = a.hist + (size_t)(n >> 1) * FCB;
@@ -263,12 +272,24 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     const int b_max = numeric ? B - 1 : B;
     const size_t fo = (size_t)f * C * B;
     const bool elide = a.elide_h != 0; // mse: every h entry is exactly twice the w entry (src/loss.jl:52), it is not read
-    auto val = [&](int c, int b) -> double {
-        const int o = c * B + b;
-        double v = built(c, b);
-        if (sub) v = __ldg(hp + fo + o) - v;
-        if (keep) hn[fo + o] = v;
-        return v;
+    // entries of channel c in the lane's bins: the loads (`fetch`) run ahead of their use (`take`), which subtracts from the
+    // parent's histogram and keeps the result for the children
+    struct Raw { double bv[CH], pv[CH]; };
+    auto fetch = [&](int c, Raw &r) {
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+            const int b = bin0 + j;
+            r.bv[j] = b < B ? built(c, b) : 0.0;
+            r.pv[j] = sub && b < B ? __ldg(hp + fo + (size_t)c * B + b) : 0.0;
+        }
+    };
+    auto take = [&](int c, const Raw &r, double (&v)[CH]) {
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+            const int b = bin0 + j;
+            v[j] = sub ? r.pv[j] - r.bv[j] : r.bv[j];
+            if (keep && b < B) hn[fo + (size_t)c * B + b] = v[j];
+        }
     };
     auto running = [&](double (&v)[CH]) { // inclusive running sum over the bins (numeric features only)
         if (!numeric) return;
@@ -280,16 +301,21 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
 #pragma unroll
         for (int j = 0; j < CH; ++j) v[j] += before;
     };
+    double best_g = 0.0, best_h = 0.0, best_w = 0.0; // left sums of the lane's candidate (K1)
     double lg = a.gamma; // get_best_split starts at gamma and takes strict improvements (fit-utils.jl:444-450)
     int lb = 0x7fffffff;
     if (a.level < a.D) {
-        double wl[CH], gacc[CH];
+        double wl[CH], gacc[CH], g1[CH], h1[CH];
         unsigned okmask = 0xffu;
+        Raw rw, rg, rh;
+        fetch(C - 1, rw);
+        fetch(0, rg);
+        if (!elide) fetch(K, rh);
+        take(C - 1, rw, wl);
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
             gacc[j] = 0.0;
             const int b = bin0 + j;
-            wl[j] = b < B ? val(C - 1, b) : 0.0;
             if (elide && keep && b < B)
                 for (int k = 0; k < K; ++k) hn[fo + (size_t)(K + k) * B + b] = 2.0 * wl[j];
         }
@@ -297,17 +323,18 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
         for (int k = 0; k < K; ++k) {
             const double sg = s_sum[k], sh = s_sum[K + k];
             double gl[CH], hl[CH];
-#pragma unroll
-            for (int j = 0; j < CH; ++j) {
-                const int b = bin0 + j;
-                gl[j] = b < B ? val(k, b) : 0.0;
-                if (!elide) hl[j] = b < B ? val(K + k, b) : 0.0;
+            take(k, rg, gl);
+            if (!elide) take(K + k, rh, hl);
+            if (!K1 && k + 1 < K) { // the next output's entries are on their way while this one is scanned
+                fetch(k + 1, rg);
+                if (!elide) fetch(K + k + 1, rh);
             }
             running(gl);
             if (!elide) running(hl);
 #pragma unroll
             for (int j = 0; j < CH; ++j) {
                 if (elide) hl[j] = 2.0 * wl[j];
+                if (K1) { g1[j] = gl[j]; h1[j] = hl[j]; }
                 const double w_l = wl[j], w_r = w_p - w_l;
                 if (!OWN) gacc[j] += term_gh(gl[j], hl[j], w_l, a.lambda, a.L2) + term_gh(sg - gl[j], sh - hl[j], w_r, a.lambda, a.L2);
                 else gacc[j] += side_gain(a, gl[j], hl[j], w_l, sg, sh, w_p);
@@ -330,44 +357,29 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
             const bool elig = b < b_max && w_l > a.min_weight && w_r > a.min_weight && ((okmask >> j) & 1u);
             if (elig) {
                 g = gacc[j] - gain_p;
-                if (g > lg) { lg = g; lb = b; }
+                if (g > lg) { lg = g; lb = b; if (K1) { best_g = g1[j]; best_h = h1[j]; best_w = wl[j]; } }
             }
             if (OBL && b < B) a.obl_gain[((size_t)(n - m) * F + f) * B + b] = g; // update_gains!, fit-utils.jl:457-463
         }
+        const int mine = lb;
 #pragma unroll
         for (int d = 16; d >= 1; d >>= 1) {
             const double og = __shfl_xor_sync(FULL, lg, d);
             const int ob = __shfl_xor_sync(FULL, lb, d);
             if (og > lg || (og == lg && ob < lb)) { lg = og; lb = ob; }
         }
+        if (K1 && mine == lb && lb != 0x7fffffff) { // a bin is one lane's
+            double *l = a.fbest_left + ((size_t)(n - m) * F + f) * 3;
+            l[0] = best_g; l[1] = best_h; l[2] = best_w;
+            if (a.ticket) __threadfence();
+        }
     }
+    __syncwarp();
     if (lane == 0) {
         a.fbest_gain[(size_t)(n - m) * F + f] = lg;
         a.fbest_bin[(size_t)(n - m) * F + f] = lb == 0x7fffffff ? -1 : lb;
     }
     __syncwarp();
-}
-
-// Stage 1: one warp per (node, owned feature slot), lanes over bins.  The nodes of a level come in pairs sharing a
-// build slot: the build node reads the slot's histogram, its sibling subtracts it from the parent's.  Warps are
-// independent, so even the root level (one node) spreads over many SMs.
-// OWN: the loss brings its own split gain (mae, credibility); OBL: oblivious trees, the gain of every candidate is
-// stored as well.  The default instance carries neither code.
-template <int MAXCHK, bool OWN, bool OBL, bool K1>
-__global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_feat(ScanArgs a) {
-    __shared__ double s_sum_all[8][72];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    const int F = a.F;
-    const int Fown = (F - a.rank + a.world - 1) / a.world;
-    if (Fown <= 0) return;
-    long long gw = (long long)blockIdx.x * wpb + wid;
-    const int which = a.level > 1 ? (int)(gw & 1) : 0;
-    if (a.level > 1) gw >>= 1;
-    const int s = (int)(gw / Fown), fi = (int)(gw % Fown);
-    if (s >= a.plan->nbuild) return;
-    const int f = fi * a.world + a.rank;
-    const int nb = a.slot_node[s];
-    scan_one<MAXCHK, OWN, OBL, K1>(a, which ? nb ^ 1 : nb, which != 0, f, s, s_sum_all[wid], lane, fi == 0);
 }
 
 // Oblivious trees, stage 1b: one thread per candidate (feature slot, bin) adds the gains of the level's nodes in
@@ -464,37 +476,27 @@ __device__ __forceinline__ void apply_split(const ScanArgs &a, int n, bool has, 
 // Stage 2: one warp per node: first strict maximum over the (owned) features in ascending feature order and the
 // left-child sums of the winner (`_child_sums!`, fit-utils.jl:472-486).  Single GPU: the split is applied at once.
 // Sharded with peer access: the rank's candidate is written into every rank's candidate table instead.
-template <bool K1>
-__global__ void __launch_bounds__(256) k_scan_node(ScanArgs a) {
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int C = K1 ? 3 : a.C, B = a.B, F = a.F; // K1: one output, channels g, h, w known at compile time
-    const int m = 1 << (a.level - 1);
-    const int i = blockIdx.x * (blockDim.x >> 5) + wid;
-    __shared__ double s_sum_all[8][72], s_left_all[8][72], s_right_all[8][72];
-    double *s_sum = s_sum_all[wid], *s_left = s_left_all[wid], *s_right = s_right_all[wid];
-    if (i >= m) return;
-    const int n = m + i;
-    // this kernel is a chain of dependent loads: everything that does not depend on the winner is requested up front
-    const int kd = a.kind[n];
-    const int slot_n = a.bslot[n];
+template <int MAXCHK, bool K1>
+__device__ __forceinline__ void node_select(const ScanArgs &a, int n, double *s_sum, double *s_left, double *s_right, int lane) {
+    const int C = K1 ? 3 : a.C, K = K1 ? 1 : a.K, B = a.B, F = a.F; // K1: one output, channels g, h, w known at compile time
+    const int m = 1 << (a.level - 1), i = n - m;
     const int Fown = (F - a.rank + a.world - 1) / a.world;
+    const int slot_n = a.bslot[n];
+    const bool sub = a.kind[n] == EVB_KIND_SUB;
     double fg[4];
     int fb[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
         const int fi = lane + 32 * u;
         fb[u] = -1; fg[u] = 0.0;
-        if (fi < Fown && !a.obl_gain) {
+        if (fi < Fown && !a.obl_gain) { // written by other warps of this launch when the scan is fused: past L1
             const int f = fi * a.world + a.rank;
-            fg[u] = a.fbest_gain[(size_t)i * F + f];
-            fb[u] = a.fbest_bin[(size_t)i * F + f];
+            fg[u] = __ldcg(a.fbest_gain + (size_t)i * F + f);
+            fb[u] = __ldcg(a.fbest_bin + (size_t)i * F + f);
         }
     }
-    for (int c = lane; c < C; c += 32) s_sum[c] = a.nsum[(size_t)n * C + c];
-    if (kd == EVB_KIND_NONE) return;
+    for (int c = lane; c < C; c += 32) s_sum[c] = __ldcg(a.nsum + (size_t)n * C + c);
     const size_t FCB = (size_t)F * C * B;
-    const double *hc = a.hcomp + (size_t)slot_n * FCB;
-    const bool sub = kd == EVB_KIND_SUB;
     const double *hp = a.hist + (size_t)(n >> 1) * FCB;
     const double *hn = a.hist + (size_t)n * FCB;
     __syncwarp();
@@ -506,74 +508,63 @@ __global__ void __launch_bounds__(256) k_scan_node(ScanArgs a) {
         if (e >= 0.0) { bg = a.obl_best[0]; bs = (int)e / B; bb = (int)e % B; }
     } else {
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-        if (fb[u] >= 0 && fg[u] > bg) { bg = fg[u]; bs = (lane + 32 * u) * a.world + a.rank; bb = fb[u]; }
-    for (int fi = lane + 128; fi < Fown; fi += 32) {
-        const int f = fi * a.world + a.rank;
-        const double g = a.fbest_gain[(size_t)i * F + f];
-        const int b = a.fbest_bin[(size_t)i * F + f];
-        if (b >= 0 && g > bg) { bg = g; bs = f; bb = b; }
-    }
+        for (int u = 0; u < 4; ++u)
+            if (fb[u] >= 0 && fg[u] > bg) { bg = fg[u]; bs = (lane + 32 * u) * a.world + a.rank; bb = fb[u]; }
+        for (int fi = lane + 128; fi < Fown; fi += 32) {
+            const int f = fi * a.world + a.rank;
+            const double g = __ldcg(a.fbest_gain + (size_t)i * F + f);
+            const int b = __ldcg(a.fbest_bin + (size_t)i * F + f);
+            if (b >= 0 && g > bg) { bg = g; bs = f; bb = b; }
+        }
 #pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        const double og = __shfl_xor_sync(FULL, bg, d);
-        const int os = __shfl_xor_sync(FULL, bs, d), ob = __shfl_xor_sync(FULL, bb, d);
-        if (os != 0x7fffffff && (og > bg || (og == bg && os < bs))) { bg = og; bs = os; bb = ob; }
-    }
+        for (int d = 16; d >= 1; d >>= 1) {
+            const double og = __shfl_xor_sync(FULL, bg, d);
+            const int os = __shfl_xor_sync(FULL, bs, d), ob = __shfl_xor_sync(FULL, bb, d);
+            if (os != 0x7fffffff && (og > bg || (og == bg && os < bs))) { bg = og; bs = os; bb = ob; }
+        }
     }
     const bool has = bs != 0x7fffffff;
-    if (has) {
-        const bool numeric = a.feattypes[a.js0[bs]] != 0;
+    if (has && K1 && !a.obl_gain) { // kept by the feature's scan
+        if (lane < 3) s_left[lane] = __ldcg(a.fbest_left + ((size_t)i * F + bs) * 3 + lane);
+        __syncwarp();
+    } else if (has) {
+        const uint32_t feat = a.js0[bs];
+        const bool numeric = a.feattypes[feat] != 0;
         const size_t fo = (size_t)bs * C * B;
-        const size_t qo = a.qsum ? (size_t)slot_n * B * a.SC + a.js0[bs] : 0;
-        const double qi = a.qsum ? a.qinv[0] : 0.0;
         // entry (channel c, bin b) of the winner's histogram in this node
         auto entry = [&](int c, int b) -> double {
             const size_t o = fo + (size_t)c * B + b;
             if (a.world > 1) return hn[o]; // sharded: the summed histogram of every scanned node is retained locally for the owned features
-            double built;
-            if (a.qsum) {
-                const size_t q = qo + (size_t)b * a.SC;
-                built = c < a.K ? (double)(long long)a.qsum[q] * qi : (c == C - 1 ? 1.0 : 2.0) * (double)a.qcnt[q];
-            } else {
-                built = hc[o];
-            }
+            const double built = built_entry(a, slot_n, bs, feat, c, b, K, C);
             return sub ? hp[o] - built : built;
         };
-        const int b0 = numeric ? lane : bb, b1 = bb;
-        if (K1) { // the three channels side by side; the mse hessian is twice the weight, entry by entry
-            double vg = 0.0, vh = 0.0, vw = 0.0;
-            for (int b = b0; b <= b1; b += 32) {
-                vg += entry(0, b);
-                if (!a.elide_h) vh += entry(1, b);
-                vw += entry(2, b);
-                if (!numeric) break;
-            }
-            if (numeric) {
+        // eight channels side by side: their loads and their sums over the lanes overlap
+        for (int c0 = 0; c0 < C; c0 += 8) {
+            double v[8];
 #pragma unroll
-                for (int d = 16; d >= 1; d >>= 1) {
-                    vg += __shfl_xor_sync(FULL, vg, d);
-                    vh += __shfl_xor_sync(FULL, vh, d);
-                    vw += __shfl_xor_sync(FULL, vw, d);
+            for (int u = 0; u < 8; ++u) {
+                v[u] = 0.0;
+#pragma unroll
+                for (int j = 0; j < MAXCHK; ++j) {
+                    const int b = lane + 32 * j;
+                    if (c0 + u < C && b < B && (numeric ? b <= bb : b == bb)) v[u] += entry(c0 + u, b);
                 }
             }
-            if (a.elide_h) vh = 2.0 * vw;
-            if (lane == 0) { s_left[0] = vg; s_left[1] = vh; s_left[2] = vw; }
-        } else {
-            for (int c = 0; c < C; ++c) {
-                double v = 0.0;
-                for (int b = b0; b <= b1; b += 32) {
-                    v += entry(c, b);
-                    if (!numeric) break;
-                }
-                if (numeric) v = warp_sum(v);
-                if (lane == 0) s_left[c] = v;
+#pragma unroll
+            for (int d = 16; d >= 1; d >>= 1) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] += __shfl_xor_sync(FULL, v[u], d);
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) if (c0 + u < C) s_left[c0 + u] = v[u];
             }
         }
         __syncwarp();
     }
     if (a.world == 1) {
         apply_split(a, n, has, bg, bs, bb, s_sum, s_left, s_right, lane);
+        if (has && lane == 0) { const int s0 = a.seg_start[n]; a.cur_l[n] = s0; a.cur_r[n] = s0 + a.seg_cnt[n]; }
         return;
     }
     const int RC = 3 + C;
@@ -581,6 +572,45 @@ __global__ void __launch_bounds__(256) k_scan_node(ScanArgs a) {
         double *rec = a.peer_cand[q] + ((size_t)i * a.world + a.rank) * RC;
         if (lane == 0) { rec[0] = bg; rec[1] = has ? (double)bs : -1.0; rec[2] = (double)bb; }
         if (has) for (int c = lane; c < C; c += 32) rec[3 + c] = s_left[c];
+    }
+}
+template <bool K1>
+__global__ void __launch_bounds__(256) k_scan_node(ScanArgs a) {
+    __shared__ double s_sum[8][72], s_left[8][72], s_right[8][72];
+    const int wid = threadIdx.x >> 5, m = 1 << (a.level - 1), i = blockIdx.x * 8 + wid;
+    if (i >= m || a.kind[m + i] == EVB_KIND_NONE) return;
+    node_select<8, K1>(a, m + i, s_sum[wid], s_left[wid], s_right[wid], threadIdx.x & 31);
+}
+
+// Stage 1: one warp per (node, owned feature slot), lanes over bins.  The nodes of a level come in pairs sharing a
+// build slot: the build node reads the slot's histogram, its sibling subtracts it from the parent's.  Warps are
+// independent, so even the root level (one node) spreads over many SMs.
+// OWN: the loss brings its own split gain (mae, credibility); OBL: oblivious trees, the gain of every candidate is
+// stored as well.  The default instance carries neither code.
+template <int MAXCHK, bool OWN, bool OBL, bool K1>
+__global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_feat(ScanArgs a) {
+    __shared__ double s_sum_all[8][72], s_left_all[8][72], s_right_all[8][72];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    const int F = a.F;
+    const int Fown = (F - a.rank + a.world - 1) / a.world;
+    if (blockIdx.x == 0 && a.level == 1 && threadIdx.x < a.ng) a.gmax[threadIdx.x] = 0u;
+    if (Fown <= 0) return;
+    long long gw = (long long)blockIdx.x * wpb + wid;
+    const int which = a.level > 1 ? (int)(gw & 1) : 0;
+    if (a.level > 1) gw >>= 1;
+    const int s = (int)(gw / Fown), fi = (int)(gw % Fown);
+    if (s >= a.plan->nbuild) return;
+    const int f = fi * a.world + a.rank;
+    const int nb = a.slot_node[s];
+    const int n = which ? nb ^ 1 : nb;
+    scan_one<MAXCHK, OWN, OBL, K1>(a, n, which != 0, f, s, s_sum_all[wid], lane, fi == 0);
+    if (!OBL && a.ticket) {
+        // the warp that scans the node's last feature decides the node: no launch of its own for that
+        unsigned last = 0;
+        if (lane == 0) { __threadfence(); last = atomicAdd(a.ticket + n, 1u) == (unsigned)(F - 1); }
+        if (!__shfl_sync(FULL, last, 0)) return;
+        __threadfence();
+        node_select<MAXCHK, K1>(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
     }
 }
 
@@ -618,6 +648,7 @@ __global__ void __launch_bounds__(256) k_scan_final(ScanArgs a) {
     }
     __syncwarp();
     apply_split(a, n, has, bg, bs, bb, s_sum, s_left, s_right, lane);
+    if (has && lane == 0) { const int s0 = a.seg_start[n]; a.cur_l[n] = s0; a.cur_r[n] = s0 + a.seg_cnt[n]; }
 }
 
 // Cross-GPU barrier for the peer-access path: every rank writes the sequence number into its slot of every
@@ -657,256 +688,247 @@ struct PartArgs {
     uint32_t *rows_out;
     const uint8_t *t_split;
     const uint32_t *t_packed;
-    int32_t *seg_start, *seg_cnt, *gcnt, *nleft, *bslot, *cum, *slot_node;
-    const int32_t *gnleft;
+    int32_t *seg_start, *seg_cnt, *bslot, *cum, *slot_node;
+    int32_t *cur_l, *cur_r;     // next free place for left rows (upwards) / past the last free one for right rows (downwards)
+    int32_t *pl_node, *pl_cum;  // sibling pairs of the level (first child's id, the root alone at level 1), running sum of their rows
+    int32_t *pl_node_next, *pl_cum_next;
     uint8_t *kind;
-    int32_t *ibase;       // [level nodes + 1] exclusive prefix of items per node
-    int32_t *item_left, *item_lprefix; // left rows of every item; their running sum over all items of the level
-    int32_t *nbase;       // [level nodes] value of the running sum at the node's first item
-    uint32_t *item_bits;
     LevelPlan *plan;
+    uint32_t *done;             // CTAs that have finished; the last one plans the next level
     const double *nsum; // node sums [id][C]; channel C-1 is the sum of weights
+    unsigned long long *hsum;   // accumulators of the level's build slots, cleared here (the scan has read them)
+    uint32_t *hcnt;
+    size_t acc_sums, acc_cnts;  // words per build slot
     int C, by_weight;   // by_weight: sharded run, pick the build child by weight sum instead of row count
-    int RS, level, D, max_items;
-    int *err;
+    int level, D;
 };
 
-__global__ void __launch_bounds__(1024) k_part_plan(PartArgs a) {
-    __shared__ int sm[33];
-    const int lo = 1 << (a.level - 1), m = lo;
-    int carry = 0;
-    for (int base = 0; base < m; base += blockDim.x) {
-        const int i = base + threadIdx.x;
-        int cnt = 0;
-        if (i < m && a.t_split[lo + i - 1]) cnt = (a.seg_cnt[lo + i] + EVB_PART_CHUNK - 1) / EVB_PART_CHUNK;
-        int total;
-        const int ex = block_excl_scan(cnt, sm, &total);
-        if (i < m) a.ibase[i] = carry + ex;
-        carry += total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        if (carry > a.max_items) { atomicCAS(a.err, 0, EVB_DERR_PLAN); carry = 0; }
-        a.ibase[m] = carry;
-        a.plan[a.level].nitems = carry;
-    }
-}
-
-__device__ __forceinline__ void item_lookup(const PartArgs &a, int item, int &n, int &chunk) {
-    const int m = 1 << (a.level - 1);
-    int l = 0, r = m - 1; // largest i with ibase[i] <= item
-    while (l < r) { const int mid = (l + r + 1) >> 1; if (a.ibase[mid] <= item) l = mid; else r = mid - 1; }
-    n = m + l;
-    chunk = item - a.ibase[l];
-}
-
-__global__ void __launch_bounds__(EVB_PART_THREADS) k_part_flags(PartArgs a) {
-    __shared__ int s_cnt[EVB_PART_THREADS / 32];
-    const int nitems = a.plan[a.level].nitems;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-        int n, chunk;
-        item_lookup(a, item, n, chunk);
-        const int start = a.seg_start[n] + chunk * EVB_PART_CHUNK;
-        const int cnt = min(EVB_PART_CHUNK, a.seg_cnt[n] - chunk * EVB_PART_CHUNK);
-        const uint32_t pk = a.t_packed[n - 1];
-        const uint32_t feat = pk & 0xffffu, bin = (pk >> 16) & 0xffu;
-        const bool numeric = (pk >> 25) & 1u;
-        int local = 0;
-        constexpr int NI = EVB_PART_CHUNK / EVB_PART_THREADS;
-        // all row ids first, then all gathers: eight independent loads in flight per thread in each phase
-        uint32_t row[NI], x[NI];
-#pragma unroll
-        for (int i8 = 0; i8 < NI; ++i8) {
-            const int pos = i8 * EVB_PART_THREADS + threadIdx.x;
-            row[i8] = pos < cnt ? __ldg(a.rows_in + start + pos) : 0xffffffffu;
-        }
-        const uint8_t *xf = a.xC + (size_t)feat * a.n;
-#pragma unroll
-        for (int i8 = 0; i8 < NI; ++i8) x[i8] = row[i8] != 0xffffffffu ? (uint32_t)__ldg(xf + row[i8]) : 0xffffu;
-#pragma unroll
-        for (int i8 = 0; i8 < NI; ++i8) {
-            const bool left = x[i8] != 0xffffu && (numeric ? (x[i8] <= bin) : (x[i8] == bin)); // split_set! predicate (fit-utils.jl:173, 291)
-            const unsigned bal = __ballot_sync(FULL, left);
-            if (lane == 0) {
-                a.item_bits[(size_t)item * (EVB_PART_CHUNK / 32) + i8 * (EVB_PART_THREADS / 32) + wid] = bal;
-                local += __popc(bal);
-            }
-        }
-        if (lane == 0) s_cnt[wid] = local;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int t = 0;
-            for (int w = 0; w < EVB_PART_THREADS / 32; ++w) t += s_cnt[w];
-            a.item_left[item] = t;
-        }
-        __syncthreads();
-    }
-}
-
-// Exclusive prefix of the left counts of every split node's work items and the node's left total.  Runs inside the
-// single-CTA plan kernel.
-__device__ void part_prefix(const PartArgs &a, int *sm) {
-    const int lo = 1 << (a.level - 1), m = lo;
-    const int nitems = a.ibase[m];
-    // one running sum over the items of all nodes (they are ordered by node) ...
-    int running = 0;
-    for (int base = 0; base < nitems; base += blockDim.x) {
-        const int idx = base + threadIdx.x;
-        const int v = idx < nitems ? a.item_left[idx] : 0;
-        int total;
-        const int ex = block_excl_scan(v, sm, &total);
-        if (idx < nitems) a.item_lprefix[idx] = running + ex;
-        running += total;
-        __syncthreads();
-    }
-    __threadfence_block();
-    __syncthreads();
-    // ... and per node the value it had at the node's first item: k_part_scatter subtracts it
-    for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const int j0 = a.ibase[i], j1 = a.ibase[i + 1];
-        const int p0 = j0 < nitems ? a.item_lprefix[j0] : running;
-        const int p1 = j1 < nitems ? a.item_lprefix[j1] : running;
-        a.nbase[i] = p0;
-        a.nleft[lo + i] = p1 - p0; // a node that is not split has no items: 0
-    }
-    __threadfence_block();
-    __syncthreads();
-}
-
-// children segments / counts, build-or-subtract choice (src/fit.jl:123-129: the child with fewer rows is
-// built, ties build the left child), build slots and the histogram plan of the next level
-__global__ void __launch_bounds__(1024) k_level_plan(PartArgs a) {
-    __shared__ int sm[33];
-    part_prefix(a, sm);
+// Children segments / counts, build-or-subtract choice (src/fit.jl:123-129: the child with fewer rows is built, ties build
+// the left child), build slots and the histogram plan of the next level.  One CTA of 256 threads; a level of at most 32
+// nodes is one warp's work (no barriers: 2.1 -> 1 us).
+template <bool WARP>
+__device__ __forceinline__ void plan_level(const PartArgs &a, int *sm) {
     const int lo = 1 << (a.level - 1), m = lo;
     const bool scan_children = a.level + 1 < a.D;
-    int carry_slot = 0, carry_rows = 0;
-    for (int base = 0; base < m; base += blockDim.x) {
+    const int step = WARP ? 32 : (int)blockDim.x;
+    auto excl = [&](int v, int &total) -> int {
+        if constexpr (WARP) {
+            const int incl = warp_incl_scan_i(v, threadIdx.x);
+            total = __shfl_sync(FULL, incl, 31);
+            return incl - v;
+        } else {
+            return block_excl_scan(v, sm, &total);
+        }
+    };
+    int carry_slot = 0, carry_rows = 0, carry_all = 0;
+    for (int base = 0; base < m; base += step) {
         const int i = base + threadIdx.x;
         const int n = lo + i;
-        int sp = 0, cnt_build = 0, build_child = 0;
+        int sp = 0, cnt_build = 0, cnt_all = 0, build_child = 0;
         if (i < m && a.t_split[n - 1]) {
             sp = 1;
             const int L = n << 1, Rn = L + 1;
-            const int nl = a.nleft[n], gl = a.gnleft[n];
-            const int s0 = a.seg_start[n], c0 = a.seg_cnt[n], g0 = a.gcnt[n];
-            a.seg_start[L] = s0; a.seg_cnt[L] = nl; a.gcnt[L] = gl;
-            a.seg_start[Rn] = s0 + nl; a.seg_cnt[Rn] = c0 - nl; a.gcnt[Rn] = g0 - gl;
+            const int s0 = a.seg_start[n], c0 = a.seg_cnt[n], nl = __ldcg(a.cur_l + n) - s0;
+            a.seg_start[L] = s0; a.seg_cnt[L] = nl;
+            a.seg_start[Rn] = s0 + nl; a.seg_cnt[Rn] = c0 - nl;
+            cnt_all = c0;
             if (scan_children) {
-                // The reference builds the child with fewer rows, ties build the left one (src/fit.jl:123-129).
-                // With rows sharded over GPUs the global row counts would cost one more collective per level, so
-                // there the child with the smaller weight sum is built: every rank knows the sums from the split
-                // scan, and with unit weights it is the same rule.
-                const bool build_left = a.by_weight
-                    ? a.nsum[(size_t)Rn * a.C + a.C - 1] >= a.nsum[(size_t)L * a.C + a.C - 1]
-                    : (g0 - gl) >= gl;
+                // With rows sharded over GPUs the global row counts would cost one more collective per level, so there the
+                // child with the smaller weight sum is built: every rank knows the sums from the split scan, and with unit
+                // weights it is the same rule.
+                const bool build_left = a.by_weight ? a.nsum[(size_t)Rn * a.C + a.C - 1] >= a.nsum[(size_t)L * a.C + a.C - 1] : c0 - nl >= nl;
                 a.kind[L] = build_left ? EVB_KIND_BUILD : EVB_KIND_SUB;
                 a.kind[Rn] = build_left ? EVB_KIND_SUB : EVB_KIND_BUILD;
                 build_child = build_left ? L : Rn;
                 cnt_build = build_left ? nl : c0 - nl;
             }
         }
-        int tot_s, tot_r;
-        const int slot = carry_slot + block_excl_scan(scan_children ? sp : 0, sm, &tot_s);
-        __syncthreads();
-        const int cpre = carry_rows + block_excl_scan(cnt_build, sm, &tot_r);
+        int tot_s, tot_r, tot_a;
+        const int slot = carry_slot + excl(sp, tot_s), cpre = carry_rows + excl(cnt_build, tot_r), apre = carry_all + excl(cnt_all, tot_a);
         if (sp && scan_children) {
             a.bslot[n << 1] = slot; a.bslot[(n << 1) + 1] = slot;
             a.slot_node[slot] = build_child;
             a.cum[slot] = cpre;
+            a.pl_node_next[slot] = n << 1;
+            a.pl_cum_next[slot] = apre;
         }
-        carry_slot += tot_s; carry_rows += tot_r;
-        __syncthreads();
+        carry_slot += tot_s; carry_rows += tot_r; carry_all += tot_a;
     }
-    if (threadIdx.x == 0 && a.level + 1 <= a.D) {
+    if (threadIdx.x == 0 && scan_children) {
         a.cum[carry_slot] = carry_rows;
+        a.pl_cum_next[carry_slot] = carry_all;
         a.plan[a.level + 1].nbuild = carry_slot;
+        a.plan[a.level + 1].npl = carry_slot;
         a.plan[a.level + 1].R = carry_rows;
     }
 }
 
-__global__ void __launch_bounds__(EVB_PART_THREADS) k_part_scatter(PartArgs a) {
-    constexpr int NW = EVB_PART_CHUNK / 32;
-    __shared__ uint32_t s_bits[NW];
-    __shared__ int s_pref[NW];
-    const int nitems = a.plan[a.level].nitems;
-    const int lane = threadIdx.x & 31;
-    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-        int n, chunk;
-        item_lookup(a, item, n, chunk);
-        const int start = a.seg_start[n] + chunk * EVB_PART_CHUNK;
-        const int cnt = min(EVB_PART_CHUNK, a.seg_cnt[n] - chunk * EVB_PART_CHUNK);
-        const int nL = a.nleft[n], lp = a.item_lprefix[item] - a.nbase[n - (1 << (a.level - 1))];
-        if (threadIdx.x < NW) s_bits[threadIdx.x] = a.item_bits[(size_t)item * NW + threadIdx.x];
-        __syncthreads();
-        if (threadIdx.x < 32) { // NW == 64: two words per lane
-            const int c0 = __popc(s_bits[2 * lane]), c1 = __popc(s_bits[2 * lane + 1]);
-            const int incl = warp_incl_scan_i(c0 + c1, lane);
-            s_pref[2 * lane] = incl - c0 - c1;
-            s_pref[2 * lane + 1] = incl - c1;
-        }
-        __syncthreads();
-        const int dstL = a.seg_start[n] + lp;
-        const int dstR = a.seg_start[n] + nL + (chunk * EVB_PART_CHUNK - lp);
-        constexpr int NI = EVB_PART_CHUNK / EVB_PART_THREADS;
-        uint32_t row[NI];
+// Stable within a chunk, chunks in any order: left rows fill a node's segment from its start, right rows from its end, and a
+// chunk reserves its places with one atomic per side.  Histogram sums are integers, so the order of the rows of a node means
+// nothing to them; what it is good for is the density of the reads, which a chunk of adjacent rows keeps.  One pass over the
+// row list instead of two, no list of work items, no bit vectors, and the CTA that finishes last plans the next level: three
+// launches and the prefix sums between them less per level.
+// A chunk is NI rows per thread.  A chunk inside one node (nearly all of them while nodes are large) takes the block-wide
+// path, else every warp looks its rows' nodes up and the lanes of the same node and side share an atomic.
+__device__ __forceinline__ bool goes_left(uint32_t pk, uint32_t x) { // split_set! predicate (fit-utils.jl:173, 291)
+    const uint32_t bin = (pk >> 16) & 0xffu;
+    return ((pk >> 25) & 1u) ? (x <= bin) : (x == bin);
+}
+constexpr int PART_WARPS = EVB_PART_THREADS / 32;
+template <int NI>
+__device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G, int npl, int total, uint32_t *s_bits, int *s_pref, int *s_misc) {
+    constexpr int CHUNK = NI * EVB_PART_THREADS;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int nchunks = (total + CHUNK - 1) / CHUNK;
+    // node of position p of the level's row order, its bounds [n0, n1)
+    auto locate = [&](int p, int &node, int &n0, int &n1, int &off) {
+        int l = 0, r = npl - 1; // largest pair with pl_cum <= p
+        while (l < r) { const int mid = (l + r + 1) >> 1; if (a.pl_cum[mid] <= p) l = mid; else r = mid - 1; }
+        const int c0 = a.pl_cum[l], first = a.pl_node[l], cl = a.seg_cnt[first];
+        off = a.seg_start[first] - c0; // position -> place in the row list (the pair's segments are adjacent)
+        if (p < c0 + cl) { node = first; n0 = c0; n1 = c0 + cl; }
+        else { node = first + 1; n0 = c0 + cl; n1 = a.pl_cum[l + 1]; }
+    };
+    for (int chunk = b; chunk < nchunks; chunk += G) {
+        const int p0 = chunk * CHUNK, p1 = min(total, p0 + CHUNK);
+        int node, n0, n1, off;
+        locate(p0, node, n0, n1, off);
+        uint32_t row[NI], x[NI];
+        if (p1 <= n1) { // one node
+            if (!a.t_split[node - 1]) continue; // uniform
+            const uint32_t pk = a.t_packed[node - 1];
+            const uint8_t *xf = a.xC + (size_t)(pk & 0xffffu) * a.n;
+            const uint32_t *in = a.rows_in + (p0 + off);
+            const int cnt = p1 - p0;
+            // all row ids first, then all gathers: NI independent loads in flight per thread in each phase
 #pragma unroll
-        for (int i8 = 0; i8 < NI; ++i8) {
-            const int pos = i8 * EVB_PART_THREADS + threadIdx.x;
-            row[i8] = pos < cnt ? __ldg(a.rows_in + start + pos) : 0u;
-        }
+            for (int i = 0; i < NI; ++i) { const int q = i * EVB_PART_THREADS + threadIdx.x; row[i] = q < cnt ? __ldg(in + q) : 0xffffffffu; }
 #pragma unroll
-        for (int i8 = 0; i8 < NI; ++i8) {
-            const int pos = i8 * EVB_PART_THREADS + threadIdx.x;
-            if (pos < cnt) {
-                const uint32_t word = s_bits[pos >> 5];
-                const int before = s_pref[pos >> 5] + __popc(word & ((1u << lane) - 1u));
-                if ((word >> lane) & 1u) a.rows_out[dstL + before] = row[i8];
-                else a.rows_out[dstR + (pos - before)] = row[i8];
+            for (int i = 0; i < NI; ++i) x[i] = row[i] != 0xffffffffu ? (uint32_t)__ldg(xf + row[i]) : 0xffffu;
+            unsigned left = 0;
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                const unsigned bal = __ballot_sync(FULL, x[i] != 0xffffu && goes_left(pk, x[i]));
+                left |= ((bal >> lane) & 1u) << i;
+                if (lane == 0) s_bits[i * PART_WARPS + wid] = bal;
+            }
+            __syncthreads();
+            if (wid == 0) { // NI * 8 <= 64 words: two per lane
+                const int c0 = 2 * lane < NI * PART_WARPS ? __popc(s_bits[2 * lane]) : 0, c1 = 2 * lane < NI * PART_WARPS ? __popc(s_bits[2 * lane + 1]) : 0;
+                const int incl = warp_incl_scan_i(c0 + c1, lane);
+                s_pref[2 * lane] = incl - c0 - c1;
+                s_pref[2 * lane + 1] = incl - c1;
+                if (lane == 31) {
+                    s_misc[0] = atomicAdd(a.cur_l + node, incl);
+                    s_misc[1] = atomicSub(a.cur_r + node, cnt - incl) - (cnt - incl);
+                }
+            }
+            __syncthreads();
+            const int dl = s_misc[0], dr = s_misc[1];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                const int q = i * EVB_PART_THREADS + threadIdx.x;
+                if (q < cnt) {
+                    const int before = s_pref[q >> 5] + __popc(s_bits[q >> 5] & ((1u << lane) - 1u));
+                    a.rows_out[(left >> i) & 1u ? dl + before : dr + (q - before)] = row[i];
+                }
+            }
+            __syncthreads();
+        } else {
+            // 2 * node + side of every row, 0: not a row of a split node
+            uint32_t key[NI];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                const int q = p0 + i * EVB_PART_THREADS + threadIdx.x;
+                key[i] = 0u;
+                if (q < p1) {
+                    if (q >= n1 || q < n0) locate(q, node, n0, n1, off);
+                    if (a.t_split[node - 1]) { key[i] = (uint32_t)node << 1; row[i] = __ldg(a.rows_in + (q + off)); x[i] = a.t_packed[node - 1]; }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < NI; ++i)
+                if (key[i] && goes_left(x[i], (uint32_t)__ldg(a.xC + (size_t)(x[i] & 0xffffu) * a.n + row[i]))) key[i] |= 1u;
+            int base[NI];
+            unsigned peers[NI];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                peers[i] = __match_any_sync(FULL, key[i]);
+                const int c = __popc(peers[i]);
+                base[i] = 0;
+                if (key[i] && (peers[i] & ((1u << lane) - 1u)) == 0u)
+                    base[i] = (key[i] & 1u) ? atomicAdd(a.cur_l + (key[i] >> 1), c) : atomicSub(a.cur_r + (key[i] >> 1), c) - c;
+            }
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                const int at = __shfl_sync(FULL, base[i], __ffs(peers[i]) - 1);
+                if (key[i]) a.rows_out[at + __popc(peers[i] & ((1u << lane) - 1u))] = row[i];
             }
         }
-        __syncthreads();
     }
+}
+__global__ void __launch_bounds__(EVB_PART_THREADS) k_partition(PartArgs a) {
+    __shared__ uint32_t s_bits[EVB_PART_CHUNK / 32];
+    __shared__ int s_pref[EVB_PART_CHUNK / 32], s_misc[34];
+    const int npl = a.plan[a.level].npl, total = npl > 0 ? a.pl_cum[npl] : 0;
+    {
+        const size_t nb = (size_t)a.plan[a.level].nbuild, ns = nb * a.acc_sums, nc = nb * a.acc_cnts;
+        const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
+        for (size_t i = i0; i < ns; i += st) a.hsum[i] = 0ull;
+        for (size_t i = i0; i < nc; i += st) a.hcnt[i] = 0u;
+    }
+    // few rows: small chunks, so that they spread over the GPU (their chain of dependent loads is what takes the time)
+    if (total > 4 * EVB_PART_THREADS * (int)gridDim.x) partition_chunks<8>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
+    else if (total > EVB_PART_THREADS * (int)gridDim.x) partition_chunks<4>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
+    else partition_chunks<1>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_misc[33] = atomicAdd(a.done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_misc[33]) return;
+    __threadfence();
+    if (threadIdx.x == 0) *a.done = 0u;
+    if (a.level > 6) plan_level<false>(a, s_misc);
+    else if (threadIdx.x < 32) plan_level<true>(a, s_misc);
 }
 
 PartArgs make_part_args(evb_handle *h, int level) {
     PartArgs a;
     a.xC = h->xC; a.n = h->n; a.rows_in = h->rows[(level - 1) & 1]; a.rows_out = h->rows[level & 1];
     a.t_split = h->t_split; a.t_packed = h->t_packed;
-    a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt; a.gcnt = h->gcnt; a.nleft = h->nleft; a.gnleft = h->gnleft;
-    a.bslot = h->bslot; a.cum = h->cum; a.slot_node = h->slot_node; a.kind = h->kind;
-    a.ibase = h->item_node; a.nbase = h->item_node + (1 << (h->D > 1 ? h->D - 1 : 0)) + 1; a.item_left = h->item_left; a.item_lprefix = h->item_lprefix; a.item_bits = h->item_bits;
-    a.plan = h->plan; a.RS = h->RS; a.level = level; a.D = h->D; a.max_items = h->max_items; a.err = h->d_err;
+    a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt;
+    a.bslot = h->bslot; a.cum = h->cum; a.slot_node = h->slot_node; a.kind = h->kind; a.cur_l = h->cur_l; a.cur_r = h->cur_r;
+    const size_t np = (size_t)h->maxslots + 1;
+    int32_t *p0 = h->pl + ((level - 1) & 1 ? 2 * np : 0), *p1 = h->pl + (level & 1 ? 2 * np : 0);
+    a.pl_node = p0; a.pl_cum = p0 + np; a.pl_node_next = p1; a.pl_cum_next = p1 + np;
+    a.plan = h->plan; a.done = h->ticket; a.level = level; a.D = h->D; // entry 0 of the tickets belongs to no node
     a.nsum = h->nsum; a.C = h->C; a.by_weight = h->world > 1 ? 1 : 0;
+    const bool clear = evb_acc_direct(h); // else the conversion to doubles has cleared them
+    a.hsum = h->hsum_q; a.hcnt = h->hcnt_q;
+    a.acc_sums = clear ? (size_t)h->B * h->SC * h->nq : 0; a.acc_cnts = clear ? (size_t)h->B * h->SC : 0;
     return a;
 }
 
 } // namespace
 
-static_assert(EVB_PART_CHUNK == 2048 && EVB_PART_THREADS == 256, "k_part_scatter assumes 64 ballot words per item");
+static_assert(EVB_PART_CHUNK == 2048 && EVB_PART_THREADS == 256, "k_partition assumes 64 ballot words per chunk");
 
-int32_t evb_launch_tree_reset(evb_handle *h) {
-    ResetArgs a;
-    a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt; a.gcnt = h->gcnt; a.nleft = h->nleft; a.gnleft = h->gnleft;
-    a.bslot = h->bslot; a.t_feat = h->t_feat; a.kind = h->kind; a.t_bin = h->t_bin; a.t_split = h->t_split;
-    a.t_gain = h->t_gain; a.t_w = h->t_w; a.t_pred = h->t_pred; a.t_packed = h->t_packed; a.nsum = h->nsum;
-    a.plan = h->plan; a.nids = h->nn + 2; a.nn = h->nn; a.K = h->K; a.C = h->C; a.D = h->D;
-    const int threads = 256, blocks = (a.nids + threads - 1) / threads;
-    evb_tic(h, EVB_T_PLAN);
-    k_tree_reset<<<blocks, threads, 0, h->st>>>(a);
-    evb_toc(h, EVB_T_PLAN);
-    EVB_CUDA(cudaGetLastError());
-    return EVB_OK;
-}
-
-int32_t evb_launch_root_plan(evb_handle *h) {
-    RootArgs a;
-    a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt; a.gcnt = h->gcnt; a.bslot = h->bslot; a.cum = h->cum;
-    a.slot_node = h->slot_node; a.nleft = h->nleft; a.gnleft = h->gnleft; a.kind = h->kind; a.plan = h->plan;
-    evb_tic(h, EVB_T_PLAN);
-    k_root_plan<<<1, 32, 0, h->st>>>(a);
-    evb_toc(h, EVB_T_PLAN);
+int32_t evb_launch_tree_begin(evb_handle *h, bool quantize, bool all_rows, const uint32_t *gen_js_host) {
+    BeginArgs a;
+    a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt; a.bslot = h->bslot; a.t_feat = h->t_feat; a.kind = h->kind; a.t_bin = h->t_bin;
+    a.t_split = h->t_split; a.t_gain = h->t_gain; a.t_w = h->t_w; a.t_pred = h->t_pred; a.t_packed = h->t_packed; a.nsum = h->nsum;
+    a.plan = h->plan; a.ticket = h->ticket; a.rows = h->rows[0]; a.cum = h->cum; a.slot_node = h->slot_node;
+    a.pl_node = h->pl; a.pl_cum = h->pl + h->maxslots + 1;
+    a.nids = h->nn + 2; a.nn = h->nn; a.K = h->K; a.C = h->C; a.D = h->D; a.all_rows = all_rows ? 1 : 0;
+    a.gen_js_host = gen_js_host; a.gen_js = reinterpret_cast<uint32_t *>(h->gen_d); a.ngen_js = EVB_GEN_WORDS + h->F;
+    evb_hg_quant_args(h, &a.q);
+    if (!quantize) a.q.grad = nullptr;
+    const int64_t threads = std::max<int64_t>(quantize || all_rows ? h->n : 0, std::max(a.nids, a.ngen_js));
+    evb_tic(h, EVB_T_ROWS_INIT);
+    k_tree_begin<<<(unsigned)((threads + 255) / 256), 256, 0, h->st>>>(a);
+    evb_toc(h, EVB_T_ROWS_INIT);
     EVB_CUDA(cudaGetLastError());
     return EVB_OK;
 }
@@ -941,10 +963,13 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
     a.F = h->F; a.C = h->C; a.K = h->K; a.B = h->B; a.level = level; a.D = h->D; a.hist_nodes = h->hist_nodes;
     a.loss = h->p.loss; a.neb = -h->p.eta / (double)h->p.bagging_size;
     a.elide_h = h->Ce != h->C ? 1 : 0;
-    const bool direct = evb_q2_direct(h);
-    a.qsum = direct ? h->hsum_q : nullptr; a.qcnt = direct ? h->hcnt_q : nullptr; a.qinv = h->d_qinv; a.SC = h->q2.SC;
+    const bool direct = evb_acc_direct(h);
+    a.qsum = direct ? h->hsum_q : nullptr; a.qcnt = direct ? h->hcnt_q : nullptr; a.qinv = h->d_qinv; a.SC = h->SC; a.nq = h->nq; a.unit_w = h->unit_w ? 1 : 0;
+    const bool fused = h->world == 1 && !h->obl_gain;
+    a.gmax = h->d_gmax; a.ng = h->ng;
+    a.ticket = fused ? h->ticket : nullptr; a.cur_l = h->cur_l; a.cur_r = h->cur_r; a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt;
     a.lambda = h->p.lambda; a.L2 = h->p.L2; a.gamma = h->p.gamma; a.min_weight = h->p.min_weight;
-    a.fbest_gain = h->fbest_gain; a.fbest_bin = h->fbest_bin;
+    a.fbest_gain = h->fbest_gain; a.fbest_bin = h->fbest_bin; a.fbest_left = h->fbest_left;
     a.obl_gain = h->obl_gain; a.obl_best = h->obl_best;
     a.plan = h->plan + level; a.slot_node = h->slot_node;
     const bool p2p = h->p2p && h->world > 1;
@@ -983,14 +1008,16 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
 #undef EVB_SCAN
     }
     evb_toc(h, EVB_T_SCAN);
+    EVB_CUDA(cudaGetLastError());
     if (h->obl_gain && level < h->D) {
         evb_tic(h, EVB_T_SCAN);
         k_obl_sum<<<(h->F * h->B + 127) / 128, 128, 0, h->st>>>(a);
         k_obl_pick<<<1, 1024, 0, h->st>>>(a);
         evb_toc(h, EVB_T_SCAN);
     }
+    if (fused) return EVB_OK;
     evb_tic(h, EVB_T_SCAN);
-    if (h->K == 1 && h->C == 3) k_scan_node<true><<<(m + 7) / 8, 256, 0, h->st>>>(a);
+    if (h->K == 1 && h->C == 3 && h->p.loss < EVB_MAE) k_scan_node<true><<<(m + 7) / 8, 256, 0, h->st>>>(a);
     else k_scan_node<false><<<(m + 7) / 8, 256, 0, h->st>>>(a);
     evb_toc(h, EVB_T_SCAN);
     if (p2p) {
@@ -1005,21 +1032,10 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
 
 int32_t evb_launch_partition(evb_handle *h, int level) {
     PartArgs a = make_part_args(h, level);
-    const int m = evb_level_nodes(level);
-    int pgrid = h->num_sms * 8;
-    if (pgrid > h->max_items) pgrid = h->max_items;
-    if (pgrid < 1) pgrid = 1;
-    evb_tic(h, EVB_T_PLAN);
-    k_part_plan<<<1, 1024, 0, h->st>>>(a);
-    evb_toc(h, EVB_T_PLAN);
+    const int64_t chunks = (h->n + EVB_PART_THREADS - 1) / EVB_PART_THREADS; // the smallest ones
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(h->num_sms * 8, chunks));
     evb_tic(h, EVB_T_PARTITION);
-    k_part_flags<<<pgrid, EVB_PART_THREADS, 0, h->st>>>(a);
-    evb_toc(h, EVB_T_PARTITION);
-    evb_tic(h, EVB_T_PLAN);
-    k_level_plan<<<1, 1024, 0, h->st>>>(a);
-    evb_toc(h, EVB_T_PLAN);
-    evb_tic(h, EVB_T_PARTITION);
-    k_part_scatter<<<pgrid, EVB_PART_THREADS, 0, h->st>>>(a);
+    k_partition<<<grid, EVB_PART_THREADS, 0, h->st>>>(a);
     evb_toc(h, EVB_T_PARTITION);
     EVB_CUDA(cudaGetLastError());
     return EVB_OK;
