@@ -656,7 +656,7 @@ __global__ void k_rows_plan_fill(RowsPlan *p, uint32_t *js, int nfeats, long lon
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < nfeats) js[t] = (uint32_t)t;
     if (t == 0) {
-        p->plan.nbuild = 1; p->plan.npl = 1; p->plan.R = nrows; p->plan.n_sel = (int32_t)nrows; p->plan.pad = 0;
+        p->plan.nbuild = 1; p->plan.npl = 1; p->plan.R = nrows; p->plan.n_sel = (int32_t)nrows; p->plan.total = 0;
         p->cum[0] = 0; p->cum[1] = (int32_t)nrows;
         p->slot_node[0] = 1; p->slot_node[1] = 0;
         p->seg_start[0] = 0; p->seg_start[1] = 0;

@@ -72,6 +72,8 @@ struct BeginArgs {
 // gradients into fixed-point numbers.
 __global__ void __launch_bounds__(256) k_tree_begin(BeginArgs a) {
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    evb_pdl_next();
+    evb_pdl_wait();
     if (i < a.ngen_js) a.gen_js[i] = __ldcv(a.gen_js_host + i);
     if (a.q.grad) evb_hg::quantize(a.q, i);
     if (a.all_rows && i < a.q.n) a.rows[i] = (uint32_t)i;
@@ -82,14 +84,14 @@ __global__ void __launch_bounds__(256) k_tree_begin(BeginArgs a) {
         if (root) {
             a.cum[0] = 0; a.cum[1] = (int32_t)a.q.n; a.slot_node[0] = 1;
             a.pl_node[0] = 1; a.pl_cum[0] = 0; a.pl_cum[1] = (int32_t)a.q.n;
-            a.plan[1].nbuild = 1; a.plan[1].npl = 1; a.plan[1].R = a.q.n; a.plan[1].n_sel = (int32_t)a.q.n;
+            a.plan[1].nbuild = 1; a.plan[1].npl = 1; a.plan[1].R = a.q.n; a.plan[1].n_sel = (int32_t)a.q.n; a.plan[1].total = (int32_t)a.q.n;
         }
     }
     if (i < a.nn) {
         a.t_feat[i] = 0; a.t_bin[i] = 0; a.t_split[i] = 0; a.t_gain[i] = 0.f; a.t_w[i] = 0.f; a.t_packed[i] = 0u;
         for (int k = 0; k < a.K; ++k) a.t_pred[(size_t)i * a.K + k] = 0.f;
     }
-    if (i >= 2 && i <= a.D) { a.plan[i].nbuild = 0; a.plan[i].npl = 0; a.plan[i].R = 0; }
+    if (i >= 2 && i <= a.D) { a.plan[i].nbuild = 0; a.plan[i].npl = 0; a.plan[i].R = 0; a.plan[i].total = 0; }
 }
 
 // ------------------------------------------------------------------------------------------ split scan
@@ -574,6 +576,40 @@ __device__ __forceinline__ void node_select(const ScanArgs &a, int n, double *s_
         if (has) for (int c = lane; c < C; c += 32) rec[3 + c] = s_left[c];
     }
 }
+// The same for one output on one GPU, by the warp that scanned the node's last feature: the node sums are in s_sum already,
+// everything else is requested at once (gains, bins, left sums of up to 32 features) -- one trip to L2 and one reduction.
+__device__ __forceinline__ void node_decide_k1(const ScanArgs &a, int n, const double *s_sum, double *s_left, double *s_right, int lane) {
+    const int F = a.F, i = n - (1 << (a.level - 1));
+    const double *gains = a.fbest_gain + (size_t)i * F;
+    const int32_t *bins = a.fbest_bin + (size_t)i * F;
+    const double *lefts = a.fbest_left + (size_t)i * F * 3;
+    const int s0 = a.seg_start[n], c0 = a.seg_cnt[n];
+    double l0 = 0.0, l1 = 0.0, l2 = 0.0;
+    if (lane < F) { l0 = __ldcg(lefts + lane * 3); l1 = __ldcg(lefts + lane * 3 + 1); l2 = __ldcg(lefts + lane * 3 + 2); }
+    double bg = a.gamma;
+    int bs = 0x7fffffff, bb = -1;
+#pragma unroll 4
+    for (int f = lane; f < F; f += 32) {
+        const double g = __ldcg(gains + f);
+        const int b = __ldcg(bins + f);
+        if (b >= 0 && g > bg) { bg = g; bs = f; bb = b; }
+    }
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) {
+        const double og = __shfl_xor_sync(FULL, bg, d);
+        const int os = __shfl_xor_sync(FULL, bs, d), ob = __shfl_xor_sync(FULL, bb, d);
+        if (os != 0x7fffffff && (og > bg || (og == bg && os < bs))) { bg = og; bs = os; bb = ob; }
+    }
+    const bool has = bs != 0x7fffffff;
+    if (has) {
+        if (bs >= 32) { if (lane < 3) s_left[lane] = __ldcg(lefts + (size_t)bs * 3 + lane); }
+        else if (lane == bs) { s_left[0] = l0; s_left[1] = l1; s_left[2] = l2; }
+        if (lane == 0) { a.cur_l[n] = s0; a.cur_r[n] = s0 + c0; }
+        __syncwarp();
+    }
+    apply_split(a, n, has, bg, bs, bb, s_sum, s_left, s_right, lane);
+}
+
 template <bool K1>
 __global__ void __launch_bounds__(256) k_scan_node(ScanArgs a) {
     __shared__ double s_sum[8][72], s_left[8][72], s_right[8][72];
@@ -593,6 +629,8 @@ __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_fe
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     const int F = a.F;
     const int Fown = (F - a.rank + a.world - 1) / a.world;
+    evb_pdl_next();
+    evb_pdl_wait();
     if (blockIdx.x == 0 && a.level == 1 && threadIdx.x < a.ng) a.gmax[threadIdx.x] = 0u;
     if (Fown <= 0) return;
     long long gw = (long long)blockIdx.x * wpb + wid;
@@ -610,7 +648,8 @@ __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_fe
         if (lane == 0) { __threadfence(); last = atomicAdd(a.ticket + n, 1u) == (unsigned)(F - 1); }
         if (!__shfl_sync(FULL, last, 0)) return;
         __threadfence();
-        node_select<MAXCHK, K1>(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
+        if constexpr (K1) node_decide_k1(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
+        else node_select<MAXCHK, false>(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
     }
 }
 
@@ -759,6 +798,7 @@ __device__ __forceinline__ void plan_level(const PartArgs &a, int *sm) {
         a.pl_cum_next[carry_slot] = carry_all;
         a.plan[a.level + 1].nbuild = carry_slot;
         a.plan[a.level + 1].npl = carry_slot;
+        a.plan[a.level + 1].total = carry_all;
         a.plan[a.level + 1].R = carry_rows;
     }
 }
@@ -795,8 +835,8 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
         locate(p0, node, n0, n1, off);
         uint32_t row[NI], x[NI];
         if (p1 <= n1) { // one node
-            if (!a.t_split[node - 1]) continue; // uniform
             const uint32_t pk = a.t_packed[node - 1];
+            if (!((pk >> 24) & 1u)) continue; // not split; uniform
             const uint8_t *xf = a.xC + (size_t)(pk & 0xffffu) * a.n;
             const uint32_t *in = a.rows_in + (p0 + off);
             const int cnt = p1 - p0;
@@ -843,7 +883,9 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
                 key[i] = 0u;
                 if (q < p1) {
                     if (q >= n1 || q < n0) locate(q, node, n0, n1, off);
-                    if (a.t_split[node - 1]) { key[i] = (uint32_t)node << 1; row[i] = __ldg(a.rows_in + (q + off)); x[i] = a.t_packed[node - 1]; }
+                    x[i] = a.t_packed[node - 1];
+                    row[i] = __ldg(a.rows_in + (q + off));
+                    if ((x[i] >> 24) & 1u) key[i] = (uint32_t)node << 1;
                 }
             }
 #pragma unroll
@@ -870,7 +912,9 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
 __global__ void __launch_bounds__(EVB_PART_THREADS) k_partition(PartArgs a) {
     __shared__ uint32_t s_bits[EVB_PART_CHUNK / 32];
     __shared__ int s_pref[EVB_PART_CHUNK / 32], s_misc[34];
-    const int npl = a.plan[a.level].npl, total = npl > 0 ? a.pl_cum[npl] : 0;
+    evb_pdl_next();
+    evb_pdl_wait();
+    const int npl = a.plan[a.level].npl, total = a.plan[a.level].total;
     {
         const size_t nb = (size_t)a.plan[a.level].nbuild, ns = nb * a.acc_sums, nc = nb * a.acc_cnts;
         const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
@@ -927,9 +971,9 @@ int32_t evb_launch_tree_begin(evb_handle *h, bool quantize, bool all_rows, const
     if (!quantize) a.q.grad = nullptr;
     const int64_t threads = std::max<int64_t>(quantize || all_rows ? h->n : 0, std::max(a.nids, a.ngen_js));
     evb_tic(h, EVB_T_ROWS_INIT);
-    k_tree_begin<<<(unsigned)((threads + 255) / 256), 256, 0, h->st>>>(a);
+    const cudaError_t e = evb_launch_pdl(h->early, k_tree_begin, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, h->st, a);
     evb_toc(h, EVB_T_ROWS_INIT);
-    EVB_CUDA(cudaGetLastError());
+    EVB_CUDA(e);
     return EVB_OK;
 }
 
@@ -999,11 +1043,11 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
         const bool own = h->p.loss >= EVB_MAE;
         const bool obl = h->obl_gain != nullptr;
 #define EVB_SCAN(M) do { \
-            if (own && obl) k_scan_feat<M, true, true, false><<<grid, 256, 0, h->st>>>(a); \
-            else if (own) k_scan_feat<M, true, false, false><<<grid, 256, 0, h->st>>>(a); \
-            else if (obl) k_scan_feat<M, false, true, false><<<grid, 256, 0, h->st>>>(a); \
-            else if (h->K == 1 && h->C == 3) k_scan_feat<M, false, false, true><<<grid, 256, 0, h->st>>>(a); \
-            else k_scan_feat<M, false, false, false><<<grid, 256, 0, h->st>>>(a); } while (0)
+            if (own && obl) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, true, true, false>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (own) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, true, false, false>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (obl) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, true, false>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (h->K == 1 && h->C == 3) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, false>, dim3(grid), dim3(256), 0, h->st, a)); } while (0)
         if (h->B <= 32) EVB_SCAN(1); else if (h->B <= 64) EVB_SCAN(2); else if (h->B <= 128) EVB_SCAN(4); else EVB_SCAN(8);
 #undef EVB_SCAN
     }
@@ -1035,8 +1079,8 @@ int32_t evb_launch_partition(evb_handle *h, int level) {
     const int64_t chunks = (h->n + EVB_PART_THREADS - 1) / EVB_PART_THREADS; // the smallest ones
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(h->num_sms * 8, chunks));
     evb_tic(h, EVB_T_PARTITION);
-    k_partition<<<grid, EVB_PART_THREADS, 0, h->st>>>(a);
+    const cudaError_t e = evb_launch_pdl(h->early, k_partition, dim3(grid), dim3(EVB_PART_THREADS), 0, h->st, a);
     evb_toc(h, EVB_T_PARTITION);
-    EVB_CUDA(cudaGetLastError());
+    EVB_CUDA(e);
     return EVB_OK;
 }
