@@ -188,8 +188,7 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     h->p = *p;
     h->K = p->K; h->C = 2 * p->K + 1; h->B = p->nbins; h->D = p->max_depth; h->nn = (1 << p->max_depth) - 1;
     h->Ce = (p->loss == EVB_MSE && !getenv("EVB_NO_ELISION")) ? p->K + 1 : h->C;
-    h->nfeats = nfeats; h->RS = nfeats <= 16 ? 16 : (nfeats + 31) / 32 * 32; h->GS = (h->Ce + 3) / 4 * 4; h->n = nobs;
-    { const int nct = (h->Ce + 3) / 4; h->rec_nch = (h->Ce + nct - 1) / nct; }
+    h->nfeats = nfeats; h->RS = nfeats <= 16 ? 16 : (nfeats + 31) / 32 * 32; h->n = nobs;
     h->unit_w = w == nullptr;
     h->ng = h->Ce - 1;                       // gradients (and hessians where they are not 2w)
     h->nq = h->ng + (h->unit_w ? 0 : 1);     // weights are a channel of their own, row counts are not
@@ -210,7 +209,7 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     const int64_t n = nobs;
     const int nids = h->nn + 2, C = h->C, K = h->K, D = h->D;
 
-    EVB_CUDA(dalloc(&h->grad, (size_t)n * h->GS));
+    EVB_CUDA(dalloc(&h->grad, (size_t)n * h->nq));
     if (p->loss == EVB_QUANTILE || p->loss == EVB_MULTIQUANTILE) {
         const size_t e = (size_t)2 * (h->nn + 1);
         EVB_CUDA(dalloc(&h->qs_cnt, e * 256)); EVB_CUDA(dalloc(&h->qs_prefix, e)); EVB_CUDA(dalloc(&h->qs_rank, e));
@@ -850,22 +849,16 @@ extern "C" int32_t evb_get_pred(evb_handle *h, float *pred) {
 extern "C" int32_t evb_get_grads(evb_handle *h, float *grad) {
     EVB_ENTER(h);
     if (!grad) { evb_set_error("null output"); return EVB_ERR_ARG; }
-    // the device keeps padded records of GS floats (channel c at (c / NCH) * 4 + c % NCH); the reference
-    // layout is [C x nobs]
-    std::vector<float> tmp((size_t)h->n * h->GS);
+    // the device keeps records of nq floats: no w when it is 1, no hessians for mse (h = 2w); the reference layout is [C x nobs]
+    std::vector<float> tmp((size_t)h->n * h->nq);
     EVB_CUDA(cudaMemcpyAsync(tmp.data(), h->grad, sizeof(float) * tmp.size(), cudaMemcpyDeviceToHost, h->st));
     EVB_CUDA(cudaStreamSynchronize(h->st));
-    const int NCH = h->rec_nch, C = h->C, GS = h->GS, K = h->K;
-    const bool elided = h->Ce != h->C; // mse: records hold g_1..g_K, w; h_k = 2w
+    const int C = h->C, K = h->K, nq = h->nq;
+    const bool elided = h->Ce != h->C;
     for (int64_t i = 0; i < h->n; ++i) {
-        const float *rec = tmp.data() + (size_t)i * GS;
-        for (int c = 0; c < C; ++c) {
-            float v;
-            if (!elided) v = rec[(c / NCH) * 4 + (c % NCH)];
-            else if (c < K) v = rec[(c / NCH) * 4 + (c % NCH)];
-            else { const float w = rec[(K / NCH) * 4 + (K % NCH)]; v = c < 2 * K ? 2.0f * w : w; }
-            grad[(size_t)i * C + c] = v;
-        }
+        const float *rec = tmp.data() + (size_t)i * nq;
+        const float w = h->unit_w ? 1.0f : rec[nq - 1];
+        for (int c = 0; c < C; ++c) grad[(size_t)i * C + c] = c == C - 1 ? w : elided && c >= K ? 2.0f * w : rec[c];
     }
     return EVB_OK;
 }

@@ -583,7 +583,7 @@ static int32_t evb_hist_geometry(const evb_handle *h, int F, HistGeom *g) {
     g->NFG = (F + 32 * FPL - 1) / (32 * FPL);
     g->U = g->NFG * g->NCT;
     const size_t img = unit_image_bytes(g->BP, g->NCH, FPL);
-    const size_t stage = (size_t)EVB_TILE_ROWS * (h->RS + h->GS * 4);
+    const size_t stage = (size_t)EVB_TILE_ROWS * (h->RS + 16);
     const size_t sm_total = 228 * 1024, blk_max = 227 * 1024, reserve = 1024;
     int UB = g->U < EVB_MAX_UNITS_PER_BLOCK ? g->U : EVB_MAX_UNITS_PER_BLOCK;
     while (UB > 1 && UB * img + 2 * stage + 256 > blk_max) --UB;
@@ -691,7 +691,7 @@ int32_t rows_hist_run(int device, cudaStream_t st, const uint8_t *x_rows, int32_
                       const float *grad, int32_t nch, const uint32_t *rows, int64_t nrows, double *out, float *scratch,
                       size_t scratch_floats, RowsPlan *plan, uint32_t *js, int hist_mode) {
     evb_handle hh{};
-    hh.B = nbins; hh.C = nch; hh.Ce = nch; hh.K = 1; hh.RS = row_stride; hh.GS = 4; hh.nfeats = nfeats; hh.maxslots = 1; hh.n = nrows;
+    hh.B = nbins; hh.C = nch; hh.Ce = nch; hh.K = 1; hh.RS = row_stride; hh.nfeats = nfeats; hh.maxslots = 1; hh.n = nrows;
     int sms = 0;
     EVB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     hh.num_sms = sms;
@@ -738,7 +738,7 @@ extern "C" int32_t evb_hist_rows(int32_t device, void *stream, const uint8_t *x_
     EVB_CUDA(cudaSetDevice(device));
     cudaStream_t st = (cudaStream_t)stream;
     evb_handle hh{};
-    hh.B = nbins; hh.C = nch; hh.Ce = nch; hh.RS = row_stride; hh.GS = 4; hh.nfeats = nfeats; hh.maxslots = 1; hh.n = nrows;
+    hh.B = nbins; hh.C = nch; hh.Ce = nch; hh.RS = row_stride; hh.nfeats = nfeats; hh.maxslots = 1; hh.n = nrows;
     int sms = 0;
     EVB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     hh.num_sms = sms;

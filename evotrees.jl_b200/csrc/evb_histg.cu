@@ -139,7 +139,7 @@ void evb_hg_args(const evb_handle *h, int level, evb_hg::Args *a) {
 
 void evb_hg_quant_args(const evb_handle *h, evb_hg::QuantArgs *a) {
     a->grad = h->grad; a->q = h->use_q2 ? reinterpret_cast<int32_t *>(h->xE) : h->gradq; a->gmax = h->d_gmax; a->qinv = h->d_qinv; a->n = h->n;
-    a->GS = h->GS; a->NCH = h->rec_nch; a->q2 = h->use_q2 ? 1 : 0; a->g = h->hgeo;
+    a->q2 = h->use_q2 ? 1 : 0; a->g = h->hgeo;
 }
 
 int32_t evb_launch_histg(evb_handle *h, int level) {

@@ -283,10 +283,10 @@ struct QuantArgs {
     const unsigned *gmax;   // [nq] bits of max |g|
     double *qinv;           // [nq]
     long long n;
-    int GS, NCH, q2;
+    int q2;
     HGeom g;
 };
-// row i of the grid's rows; every thread of the block calls it
+// row i of the grid's rows (blocks of adjacent rows); every thread of the block calls it
 __device__ __forceinline__ void quantize(const QuantArgs &a, long long i) {
     __shared__ float s_sc[EVB_MAX_Q];
     for (int c = threadIdx.x; c < a.g.nq; c += blockDim.x) {
@@ -304,13 +304,36 @@ __device__ __forceinline__ void quantize(const QuantArgs &a, long long i) {
         if (blockIdx.x == 0) a.qinv[c] = inv;
     }
     __syncthreads();
-    if (i >= a.n) return;
-    const float *rec = a.grad + (size_t)i * a.GS;
-    if (a.q2) { a.q[2 * i] = __float2int_rn(rec[0] * s_sc[0]); return; }
+    const int nq = a.g.nq;
+    if (nq == 1) { // one word per row, in xE beside the row's tail features or alone
+        if (i < a.n) a.q[a.q2 ? 2 * i : i] = __float2int_rn(a.grad[i] * s_sc[0]);
+        return;
+    }
+    // Word by word: the block's 256 rows are contiguous in the records and in every group of q, adjacent threads take adjacent
+    // words (a thread per row would touch nq floats and nqp words at a stride of a row).
+    const long long row0 = i - threadIdx.x;
+    const int nr = (int)min((long long)blockDim.x, a.n - row0);
     for (int z = 0; z < a.g.ngc; ++z) {
-        const int c0 = z * a.g.per, nc = min(a.g.per, a.g.nq - c0), np = nqp(nc);
-        int32_t *d = a.q + evb_hg_qoff(a.g, a.n, z) + (size_t)i * np;
-        for (int c = 0; c < np; ++c) d[c] = c < nc ? __float2int_rn(rec[((c0 + c) / a.NCH) * 4 + (c0 + c) % a.NCH] * s_sc[c0 + c]) : 0;
+        const int c0 = z * a.g.per, nc = min(a.g.per, nq - c0), np = nqp(nc), sh = 31 - __clz(np);
+        int32_t *d = a.q + evb_hg_qoff(a.g, a.n, z) + (size_t)row0 * np;
+        const float *src = a.grad + (size_t)row0 * nq + c0;
+        if (sh >= 2) { // four words at a time
+            for (int e = threadIdx.x; e < nr << (sh - 2); e += blockDim.x) {
+                const int r = e >> (sh - 2), c = 4 * (e & ((np >> 2) - 1));
+                int4 v = make_int4(0, 0, 0, 0);
+                const float *g = src + (size_t)r * nq + c, *sc = s_sc + c0 + c;
+                if (c < nc) v.x = __float2int_rn(g[0] * sc[0]);
+                if (c + 1 < nc) v.y = __float2int_rn(g[1] * sc[1]);
+                if (c + 2 < nc) v.z = __float2int_rn(g[2] * sc[2]);
+                if (c + 3 < nc) v.w = __float2int_rn(g[3] * sc[3]);
+                reinterpret_cast<int4 *>(d)[e] = v;
+            }
+        } else {
+            for (int e = threadIdx.x; e < nr << sh; e += blockDim.x) {
+                const int r = e >> sh, c = e & (np - 1);
+                d[e] = c < nc ? __float2int_rn(src[(size_t)r * nq + c] * s_sc[c0 + c]) : 0;
+            }
+        }
     }
 }
 } // namespace evb_hg

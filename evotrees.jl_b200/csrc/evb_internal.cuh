@@ -72,9 +72,8 @@ struct HGeom {
 struct evb_handle {
     evb_params p;
     int K, C, B, D, nn;        // nn = 2^D-1
-    int Ce;                    // channels actually accumulated: C, or K+1 for mse where h = 2w is rebuilt from w
-    int rec_nch;               // channels per 16-byte group of the float gradient record (see gpos)
-    int nfeats, RS, GS;        // RS: bytes per row of xT (multiple of 32); GS: floats per grad record (multiple of 4)
+    int Ce;                    // channels of a record with its weight: C, or K+1 for mse where h = 2w is rebuilt from w
+    int nfeats, RS;            // RS: bytes per row of xT (16, or a multiple of 32)
     int64_t n;                 // local rows
     int dev, num_sms;
     cudaStream_t st;
@@ -85,7 +84,7 @@ struct evb_handle {
     int edges_dtype, nedges;
     uint8_t *xT;       // [n][RS]  observation-major bins (1..B), zero padded; null when xH / xE hold them
     uint8_t *xC;       // [nfeats][n] feature-major copy (the layout of the caller's x_bin) read by the row partition
-    float *grad;       // [n][GS]  g_1..g_K,h_1..h_K,w,(pad)
+    float *grad;       // [n][nq]  gradient records (grad_row, evb_rows.cu)
     float *pred;       // [n][K]
     void *y;           // float [n][ycols] or uint32 [n]
     int y_dtype, ycols;

@@ -11,29 +11,25 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// Gradient record of one row.  Channel c (reference order g_1..g_K, h_1..h_K, w) lives at float
-// (c / NCH) * 4 + c % NCH: the channels of one histogram unit start on a 16-byte boundary.
-__device__ __forceinline__ int gpos(int c, int NCH) { return (c / NCH) * 4 + (c % NCH); }
-#define REC(c) rec[gpos((c), NCH)]
-// For mse the hessian channels are not stored (h = 2w is rebuilt when the histogram is reduced): the record is
-// g_1..g_K, w, i.e. `elided` shifts w from channel 2K to channel K.
+// Gradient record of one row: the channels whose sums the histograms hold, in the reference's order g_1..g_K, h_1..h_K, w
+// (`cache.∇`, src/init.jl:173).  Left out: w when no weights were given (it is 1) and, for mse, the hessians (h = 2w is
+// rebuilt from the sums of w): `elided`.
 struct AlphaSet { float a[8]; }; // a[0]: alpha of the quantile loss; a[0..K-1]: alphas of the multiquantile loss
-__device__ __forceinline__ void grad_row(int loss, int K, int NCH, bool elided, const float *p, const void *y, int ycols, long long i, float *rec,
+__device__ __forceinline__ void grad_row(int loss, int K, bool elided, const float *p, const void *y, int ycols, long long i, float w, float *rec,
                                          const AlphaSet &al) {
     const float alpha = al.a[0];
-    const float w = REC(elided ? K : 2 * K);
     if (loss == EVB_MSE) {
         const float *yf = (const float *)y + (size_t)i * ycols;
         for (int k = 0; k < K; ++k) {
-            REC(k) = 2.0f * (p[k] - yf[k]) * w;
-            if (!elided) REC(K + k) = 2.0f * w;
+            rec[k] = 2.0f * (p[k] - yf[k]) * w;
+            if (!elided) rec[K + k] = 2.0f * w;
         }
     } else if (loss == EVB_LOGLOSS) {
         const float *yf = (const float *)y + (size_t)i * ycols;
         for (int k = 0; k < K; ++k) {
             const float s = sigmoidf_(p[k]);
-            REC(k) = (s - yf[k]) * w;
-            REC(K + k) = s * (1.0f - s) * w;
+            rec[k] = (s - yf[k]) * w;
+            rec[K + k] = s * (1.0f - s) * w;
         }
     } else if (loss == EVB_MLOGLOSS) {
         const uint32_t yi = ((const uint32_t *)y)[i];
@@ -41,29 +37,29 @@ __device__ __forceinline__ void grad_row(int loss, int K, int NCH, bool elided, 
         for (int k = 0; k < K; ++k) isum += expf(p[k]);
         for (int k = 0; k < K; ++k) {
             const float prob = expf(p[k]) / isum;
-            REC(k) = (((uint32_t)(k + 1) == yi) ? prob - 1.0f : prob) * w;
-            REC(K + k) = prob * (1.0f - prob) * w;
+            rec[k] = (((uint32_t)(k + 1) == yi) ? prob - 1.0f : prob) * w;
+            rec[K + k] = prob * (1.0f - prob) * w;
         }
     } else if (loss == EVB_MULTIQUANTILE) { // one target, one quantile per output row (src/loss.jl:160-172)
         const float yi = ((const float *)y)[i];
         for (int k = 0; k < K; ++k) {
             const float d = yi - p[k];
-            REC(k) = (d > 0.0f ? al.a[k] : al.a[k] - 1.0f) * w;
-            REC(K + k) = d;
+            rec[k] = (d > 0.0f ? al.a[k] : al.a[k] - 1.0f) * w;
+            rec[K + k] = d;
         }
     } else if (loss == EVB_QUANTILE) { // quantile_grad_diff, src/loss.jl:93-98: the second slot keeps the raw residual
         const float *yf = (const float *)y + (size_t)i * ycols;
         for (int k = 0; k < K; ++k) {
             const float d = yf[k] - p[k];
-            REC(k) = (d > 0.0f ? alpha : alpha - 1.0f) * w;
-            REC(K + k) = d;
+            rec[k] = (d > 0.0f ? alpha : alpha - 1.0f) * w;
+            rec[K + k] = d;
         }
     } else if (loss == EVB_MAE || loss == EVB_CRED_VAR || loss == EVB_CRED_STD) { // src/loss.jl:86-91
         const float *yf = (const float *)y + (size_t)i * ycols;
         for (int k = 0; k < K; ++k) {
             const float d = yf[k] - p[k];
-            REC(k) = d * w;
-            REC(K + k) = (loss == EVB_MAE ? 0.0f : d * d) * w;
+            rec[k] = d * w;
+            rec[K + k] = (loss == EVB_MAE ? 0.0f : d * d) * w;
         }
     } else if (loss == EVB_POISSON || loss == EVB_GAMMA || loss == EVB_TWEEDIE) { // src/loss.jl:65-84
         const float *yf = (const float *)y + (size_t)i * ycols;
@@ -77,8 +73,8 @@ __device__ __forceinline__ void grad_row(int loss, int K, int NCH, bool elided, 
                 g = 2.0f * (a - yk * b);
                 h = 2.0f * (0.5f * a + 0.5f * yk * b);
             }
-            REC(k) = g * w;
-            REC(K + k) = h * w;
+            rec[k] = g * w;
+            rec[K + k] = h * w;
         }
     } else if (loss == EVB_LOGISTIC_MLE) { // src/loss.jl:207-217
         const int Y = K / 2;
@@ -87,10 +83,10 @@ __device__ __forceinline__ void grad_row(int loss, int K, int NCH, bool elided, 
             const float loc = p[2 * t], sr = p[2 * t + 1];
             const float scale = softplusf_(sr), ds = sigmoidf_(sr);
             const float z = (yf[t] - loc) / scale, th = tanhf(z / 2.0f);
-            REC(2 * t) = -th / scale * w;
-            REC(2 * t + 1) = (1.0f - z * th) * ds / scale * w;
-            REC(2 * Y + 2 * t) = 1.0f / (3.0f * scale * scale) * w;
-            REC(2 * Y + 2 * t + 1) = (3.14159274f * 3.14159274f + 3.0f) / 9.0f * (ds / scale) * (ds / scale) * w;
+            rec[2 * t] = -th / scale * w;
+            rec[2 * t + 1] = (1.0f - z * th) * ds / scale * w;
+            rec[2 * Y + 2 * t] = 1.0f / (3.0f * scale * scale) * w;
+            rec[2 * Y + 2 * t + 1] = (3.14159274f * 3.14159274f + 3.0f) / 9.0f * (ds / scale) * (ds / scale) * w;
         }
     } else { // EVB_GAUSSIAN_MLE
         const int Y = K / 2;
@@ -100,10 +96,10 @@ __device__ __forceinline__ void grad_row(int loss, int K, int NCH, bool elided, 
             const float scale = softplusf_(sr), ds = sigmoidf_(sr);
             const float resid = loc - yf[t];
             const float s2 = scale * scale;
-            REC(2 * t) = resid / s2 * w;
-            REC(2 * t + 1) = (1.0f - resid * resid / s2) * ds / scale * w;
-            REC(2 * Y + 2 * t) = 1.0f / s2 * w;
-            REC(2 * Y + 2 * t + 1) = 2.0f * (ds / scale) * (ds / scale) * w;
+            rec[2 * t] = resid / s2 * w;
+            rec[2 * t + 1] = (1.0f - resid * resid / s2) * ds / scale * w;
+            rec[2 * Y + 2 * t] = 1.0f / s2 * w;
+            rec[2 * Y + 2 * t + 1] = 2.0f * (ds / scale) * (ds / scale) * w;
         }
     }
 }
@@ -133,41 +129,38 @@ __global__ void k_check_bins(const uint8_t *xC, size_t total, int nbins, int *er
     if (bad) atomicCAS(err, 0, EVB_DERR_BIN_RANGE);
 }
 
-#undef REC
 // wmax: null, or the maximum of the weights goes there (they are a channel of the histograms then)
-__global__ void __launch_bounds__(256) k_init_state(float *grad, float *pred, const float *w, const float *pred0, const float *mu, long long n, int K, int GS, int NCH, int wch, unsigned *wmax) {
+__global__ void __launch_bounds__(256) k_init_state(float *grad, float *pred, const float *w, const float *pred0, const float *mu, long long n, int K, int nq, unsigned *wmax) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (wmax) {
         const unsigned m = __reduce_max_sync(0xffffffffu, i < n ? __float_as_uint(w[i]) : 0u);
         if ((threadIdx.x & 31) == 0 && m > *(volatile unsigned *)wmax) atomicMax(wmax, m);
     }
     if (i >= n) return;
-    float *rec = grad + (size_t)i * GS;
-    for (int c = 0; c < GS; ++c) rec[c] = 0.0f;
-    rec[gpos(wch, NCH)] = w ? w[i] : 1.0f; // ∇[end, :] .= w (src/init.jl:173-174)
+    if (w) grad[(size_t)i * nq + nq - 1] = w[i]; // ∇[end, :] .= w (src/init.jl:173-174)
     for (int k = 0; k < K; ++k) pred[(size_t)i * K + k] = pred0 ? pred0[(size_t)i * K + k] : mu[k];
 }
 
 // ---------------------------------------------------------------------------------- gradients
 // max |g| of every changing channel over the rows of a 256-thread block -> global maxima (bit patterns of non-negative
 // floats, which order like unsigned integers).  rec: the thread's gradient record, or null.  Every thread calls it.
-__device__ __forceinline__ void block_absmax(const float *rec, int NCH, int ng, unsigned *gmax) {
+__device__ __forceinline__ void block_absmax(const float *rec, int ng, unsigned *gmax) {
     __shared__ unsigned s_max[EVB_MAX_Q];
     if (threadIdx.x < ng) s_max[threadIdx.x] = 0u;
     __syncthreads();
     for (int c = 0; c < ng; ++c) {
-        const unsigned m = __reduce_max_sync(FULL, rec ? __float_as_uint(fabsf(rec[gpos(c, NCH)])) : 0u);
+        const unsigned m = __reduce_max_sync(FULL, rec ? __float_as_uint(fabsf(rec[c])) : 0u);
         if ((threadIdx.x & 31) == 0 && m > *(volatile unsigned *)(s_max + c)) atomicMax(s_max + c, m);
     }
     __syncthreads();
     if (threadIdx.x < ng && s_max[threadIdx.x] > *(volatile unsigned *)(gmax + threadIdx.x)) atomicMax(gmax + threadIdx.x, s_max[threadIdx.x]);
 }
-__global__ void __launch_bounds__(256) k_grads(int loss, int K, int GS, int NCH, int elided, int ycols, long long n, const float *pred, const void *y, float *grad, unsigned *gmax, int ng,
-                                               AlphaSet alpha) {
+__global__ void __launch_bounds__(256) k_grads(int loss, int K, int nq, int unit_w, int elided, int ycols, long long n, const float *pred, const void *y, float *grad, unsigned *gmax,
+                                               int ng, AlphaSet alpha) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float *rec = i < n ? grad + (size_t)i * GS : nullptr;
-    if (rec) grad_row(loss, K, NCH, elided != 0, pred + (size_t)i * K, y, ycols, i, rec, alpha);
-    block_absmax(rec, NCH, ng, gmax);
+    float *rec = i < n ? grad + (size_t)i * nq : nullptr;
+    if (rec) grad_row(loss, K, elided != 0, pred + (size_t)i * K, y, ycols, i, unit_w ? 1.0f : rec[nq - 1], rec, alpha);
+    block_absmax(rec, ng, gmax);
 }
 
 // ---------------------------------------------------------------------------------- row sampling
@@ -318,7 +311,7 @@ struct FinArgs {
     unsigned *gmax; // [ng] max |g| of the gradients computed here
     int ng;
     long long n;
-    int RS, K, GS, NCH, elided, loss, nn, ycols, compute_grads, packed_in_smem;
+    int RS, K, nq, unit_w, elided, loss, nn, ycols, compute_grads, packed_in_smem;
     AlphaSet alpha;
     int mode; // 0: traverse, add the leaf, next gradients; 1: traverse only (leaf ids); 2: leaf ids are in nidx, add + gradients
     const uint4 *pub_src; // the finished tree goes to pinned host memory from here (pub_n 16-byte words; 0: a later kernel does it)
@@ -348,24 +341,35 @@ __global__ void __launch_bounds__(256) k_finalize(FinArgs a) {
         float *p = a.pred + (size_t)i * a.K;
         if (a.mode != 1) pred_add(a.loss, a.K, p, a.t_pred + (size_t)(nid - 1) * a.K);
         if (a.compute_grads && a.mode != 1) {
-            rec = a.grad + (size_t)i * a.GS;
-            grad_row(a.loss, a.K, a.NCH, a.elided != 0, p, a.y, a.ycols, i, rec, a.alpha);
+            rec = a.grad + (size_t)i * a.nq;
+            grad_row(a.loss, a.K, a.elided != 0, p, a.y, a.ycols, i, a.unit_w ? 1.0f : rec[a.nq - 1], rec, a.alpha);
         }
     }
-    if (a.compute_grads && a.mode != 1) block_absmax(rec, a.NCH, a.ng, a.gmax);
+    if (a.compute_grads && a.mode != 1) block_absmax(rec, a.ng, a.gmax);
 }
 
-// The same update with the rows of bins staged through shared memory: the CTA copies its 256 rows with fully
-// coalesced 16-byte loads (one memory round trip instead of one per tree level and sector), then every thread walks
-// the tree on its own row out of shared memory.  Rows are padded by one word so that equal byte offsets of different
-// rows fall into different banks.  Used when a row is at most 256 bytes.
+// The same update with everything a CTA's 256 rows hold staged through shared memory: bins, predictions and gradient records are
+// contiguous in memory per CTA but strided per row (K and nq words), so they are copied with coalesced accesses of 16 bytes
+// and every thread works on its own row out of shared memory.  Rows of bins are padded by one word so that equal byte offsets
+// of different rows fall into different banks.  Used when it all fits; KT: outputs known at compile time (0: up to 32), so that a
+// row's predictions and gradients stay in registers.
+// Bound by HBM: per row RS + 8 K + 4 nq + 8 bytes (and y).  Measured before the records went through shared memory: 2M x 28, five
+// outputs 0.140 ms, 5M x 50, two outputs 0.177 ms.
+__device__ __forceinline__ void copy_floats(float *dst, const float *src, int n) { // both 16-byte aligned
+    for (int i = threadIdx.x; i < n >> 2; i += 256) reinterpret_cast<float4 *>(dst)[i] = reinterpret_cast<const float4 *>(src)[i];
+    for (int i = (n & ~3) + threadIdx.x; i < n; i += 256) dst[i] = src[i];
+}
+template <int KT>
 __global__ void __launch_bounds__(256) k_finalize_staged(FinArgs a) {
-    extern __shared__ uint32_t s_fin[]; // [nn] packed tree, then [256][RS / 4 + 1] words of bins
+    extern __shared__ __align__(16) uint32_t s_fin[]; // predictions [256][K], records [256][nq], packed tree [nn], bins [256][RS / 4 + 1]
+    constexpr int KM = KT ? KT : 32;
+    const int K = KT ? KT : a.K, nq = a.nq;
+    float *s_p = reinterpret_cast<float *>(s_fin), *s_g = s_p + 256 * K;
+    uint32_t *s_tree = reinterpret_cast<uint32_t *>(s_g + 256 * nq);
+    uint32_t *s_rows = s_tree + a.nn;
     evb_pdl_next();
     evb_pdl_wait();
     if (blockIdx.x == 0) publish(a.pub_src, a.pub_dst, a.pub_n);
-    uint32_t *s_tree = s_fin;
-    uint32_t *s_rows = s_fin + a.nn;
     const int rw = a.RS >> 2, rwp = rw + 1; // words per row, padded
     for (int i = threadIdx.x; i < a.nn; i += 256) s_tree[i] = a.t_packed[i];
     const long long row0 = (long long)blockIdx.x * 256;
@@ -378,24 +382,39 @@ __global__ void __launch_bounds__(256) k_finalize_staged(FinArgs a) {
         uint32_t *d = s_rows + r * rwp + part * 4;
         d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     }
-    __syncthreads();
+    copy_floats(s_p, a.pred + (size_t)row0 * K, nr * K);
     const long long i = row0 + threadIdx.x;
+    float w = 1.0f;
+    if (a.compute_grads && !a.unit_w && i < a.n) w = a.grad[(size_t)i * nq + nq - 1];
+    __syncthreads();
     float *rec = nullptr;
     if (i < a.n) {
         const int nid = traverse(s_tree, reinterpret_cast<const uint8_t *>(s_rows + threadIdx.x * rwp));
         a.nidx[i] = (uint32_t)nid;
-        float *p = a.pred + (size_t)i * a.K;
-        pred_add(a.loss, a.K, p, a.t_pred + (size_t)(nid - 1) * a.K);
+        float p[KM], leaf[KM], g[2 * KM];
+        float *sp = s_p + threadIdx.x * K;
+#pragma unroll
+        for (int k = 0; k < KM; ++k) if (k < K) { p[k] = sp[k]; leaf[k] = __ldg(a.t_pred + (size_t)(nid - 1) * K + k); }
+        pred_add(a.loss, K, p, leaf);
+#pragma unroll
+        for (int k = 0; k < KM; ++k) if (k < K) sp[k] = p[k];
         if (a.compute_grads) {
-            rec = a.grad + (size_t)i * a.GS;
-            grad_row(a.loss, a.K, a.NCH, a.elided != 0, p, a.y, a.ycols, i, rec, a.alpha);
+            grad_row(a.loss, K, a.elided != 0, p, a.y, a.ycols, i, w, g, a.alpha);
+            rec = s_g + threadIdx.x * nq;
+#pragma unroll
+            for (int c = 0; c < 2 * KM; ++c) if (c < a.ng) rec[c] = g[c];
+            if (!a.unit_w) rec[nq - 1] = w;
         }
     }
-    if (a.compute_grads && a.mode != 1) block_absmax(rec, a.NCH, a.ng, a.gmax);
+    __syncthreads();
+    copy_floats(a.pred + (size_t)row0 * K, s_p, nr * K);
+    if (a.compute_grads) {
+        copy_floats(a.grad + (size_t)row0 * nq, s_g, nr * nq);
+        block_absmax(rec, a.ng, a.gmax);
+    }
 }
 
-// The same update as a pipeline: a few CTAs per SM stay resident and walk over tiles of 256 rows.  The tree (and, for
-// one output, its leaf values) is loaded into shared memory once per CTA; the bins of tile t + 1 are copied into the
+// The same update as a pipeline: a few CTAs per SM stay resident and walk over tiles of 256 rows.  The tree and its leaf values are loaded into shared memory once per CTA; the bins of tile t + 1 are copied into the
 // other of two shared-memory buffers (`cp.async`, 16 bytes per copy; rows sit at an odd number of 16-byte chunks, so
 // the same feature of 8 adjacent rows falls into different banks) while tile t is traversed, and the row's prediction
 // and target are requested before the traversal starts, so that a tile costs one memory round trip, not three.
@@ -408,13 +427,12 @@ struct FinPipeArgs {
     int strideA;          // bytes between rows of rowsA
     int wordsA;           // words copied per row from rowsA
     int S;                // words per row in shared memory: a multiple of 4, an odd number of 16-byte chunks
-    int ntiles, leaf_in_smem;
+    int ntiles;
 };
-// MSE1: mse with one output and the record {g, w} (hessian rebuilt from w): loss, K and the record layout are
-// compile-time constants
+// One output.  MSE1: mse with unit weights (the record is g alone): loss and record layout are compile-time constants
 template <bool MSE1>
 __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
-    // [nnp] packed tree, [nnp] leaf values (one output only), 2 x [256][S] words of bins; nnp = nn rounded up to four
+    // [nnp] packed tree, [nnp] leaf values, 2 x [256][S] words of bins; nnp = nn rounded up to four
     // words, so that the row buffers start on a 16-byte boundary (the copies into them are 16 bytes wide)
     extern __shared__ __align__(16) uint32_t s_fp[];
     const FinArgs &f = a.f;
@@ -424,11 +442,11 @@ __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
     const int nnp = (f.nn + 3) & ~3;
     uint32_t *s_tree = s_fp;
     float *s_leaf = reinterpret_cast<float *>(s_fp + nnp);
-    uint32_t *s_rows = s_fp + nnp + (a.leaf_in_smem ? nnp : 0);
+    uint32_t *s_rows = s_fp + 2 * nnp;
     const int S = a.S, wA = a.wordsA;
     for (int i = threadIdx.x; i < f.nn; i += 256) {
         s_tree[i] = f.t_packed[i];
-        if (a.leaf_in_smem) s_leaf[i] = f.t_pred[i];
+        s_leaf[i] = f.t_pred[i];
     }
     const int cpr = wA >> 2;                     // 16-byte chunks per row
     const uint32_t magic = 65536u / (uint32_t)cpr + 1u; // (c * magic) >> 16 == c / cpr for c < 4096, cpr <= 16
@@ -457,38 +475,35 @@ __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
         stage(tile + gridDim.x, buf ^ 1);
         const long long i = (long long)tile * 256 + threadIdx.x;
         const bool act = i < f.n;
-        float *p = f.pred + (size_t)i * f.K;
-        float p0 = 0.0f;
+        float *p = f.pred + i;
+        float pv = 0.0f;
         if (act) {
-            if (f.K == 1) p0 = *p;
-            else asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-            if (f.compute_grads) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(f.y) + (size_t)i * 4 * (f.ycols > 0 ? f.ycols : 1)));
+            pv = *p;
+            if (f.compute_grads) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(f.y) + (size_t)i * 4));
         }
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads(); // tile `tile` (and, the first time, the tree) is in place
         if (act) {
             const int nid = traverse(s_tree, reinterpret_cast<const uint8_t *>(s_rows + ((size_t)buf * 256 + threadIdx.x) * S));
             f.nidx[i] = (uint32_t)nid;
-            const int loss = MSE1 ? (int)EVB_MSE : f.loss, NCH = MSE1 ? 2 : f.NCH;
-            if (f.K == 1) {
-                float pl[1] = {p0};
-                pred_add(loss, 1, pl, a.leaf_in_smem ? s_leaf + (nid - 1) : f.t_pred + (nid - 1));
-                p[0] = pl[0];
-            } else {
-                pred_add(loss, f.K, p, f.t_pred + (size_t)(nid - 1) * f.K);
-            }
+            const int loss = MSE1 ? (int)EVB_MSE : f.loss;
+            pred_add(loss, 1, &pv, s_leaf + (nid - 1));
+            *p = pv;
             if (f.compute_grads) {
-                grad_row(loss, MSE1 ? 1 : f.K, NCH, MSE1 ? true : f.elided != 0, p, f.y, MSE1 ? 1 : f.ycols, i, f.grad + (size_t)i * f.GS, f.alpha);
-                const float *rec = f.grad + (size_t)i * f.GS;
-                gm = fmaxf(gm, fabsf(rec[0]));
-                if (!MSE1 && f.ng > 1) hm = fmaxf(hm, fabsf(rec[gpos(1, NCH)]));
+                const int nq = MSE1 ? 1 : f.nq;
+                float *rec = f.grad + (size_t)i * nq, g[2]; // one output: g, h and the weight at most
+                const float w = MSE1 || f.unit_w ? 1.0f : rec[nq - 1];
+                grad_row(loss, 1, MSE1 ? true : f.elided != 0, &pv, f.y, 1, i, w, g, f.alpha);
+                rec[0] = g[0];
+                gm = fmaxf(gm, fabsf(g[0]));
+                if (!MSE1 && f.ng > 1) { rec[1] = g[1]; hm = fmaxf(hm, fabsf(g[1])); }
             }
         }
         __syncthreads(); // everybody is done with this buffer: the next iteration refills it
     }
     if (f.compute_grads) {
         const float m2[2] = {gm, hm};
-        block_absmax(m2, 2, f.ng, f.gmax); // K == 1: one or two channels
+        block_absmax(m2, f.ng, f.gmax); // K == 1: one or two channels
     }
 }
 
@@ -756,7 +771,7 @@ int32_t evb_launch_check_bins(evb_handle *h) {
 }
 
 int32_t evb_launch_init_state(evb_handle *h, const float *w_dev, const float *pred0_dev, const float *mu_dev) {
-    k_init_state<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->grad, h->pred, w_dev, pred0_dev, mu_dev, h->n, h->K, h->GS, h->rec_nch, h->Ce - 1,
+    k_init_state<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->grad, h->pred, w_dev, pred0_dev, mu_dev, h->n, h->K, h->nq,
                                                                       h->unit_w ? nullptr : h->d_gmax + h->nq - 1);
     EVB_CUDA(cudaGetLastError());
     return EVB_OK;
@@ -765,7 +780,7 @@ int32_t evb_launch_init_state(evb_handle *h, const float *w_dev, const float *pr
 int32_t evb_launch_grads(evb_handle *h) {
     EVB_CUDA(cudaMemsetAsync(h->d_gmax, 0, sizeof(unsigned) * h->ng, h->st));
     evb_tic(h, EVB_T_GRADS);
-    k_grads<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->p.loss, h->K, h->GS, h->rec_nch, h->Ce != h->C, h->ycols, h->n, h->pred, h->y, h->grad,
+    k_grads<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->p.loss, h->K, h->nq, h->unit_w ? 1 : 0, h->Ce != h->C, h->ycols, h->n, h->pred, h->y, h->grad,
                                                                 h->d_gmax, h->ng, evb_alpha_set(h));
     evb_toc(h, EVB_T_GRADS);
     EVB_CUDA(cudaGetLastError());
@@ -828,14 +843,14 @@ int32_t evb_launch_rows_init(evb_handle *h, int use_mask, uint8_t mask_cond) {
 int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode, void *publish_to) {
     FinArgs a;
     a.xT = h->xT; a.t_packed = h->t_packed; a.t_pred = h->t_pred; a.pred = h->pred; a.grad = h->grad; a.y = h->y;
-    a.nidx = h->nidx; a.n = h->n; a.RS = h->RS; a.K = h->K; a.GS = h->GS; a.NCH = h->rec_nch; a.elided = h->Ce != h->C; a.loss = h->p.loss; a.nn = h->nn;
+    a.nidx = h->nidx; a.n = h->n; a.RS = h->RS; a.K = h->K; a.nq = h->nq; a.unit_w = h->unit_w ? 1 : 0; a.elided = h->Ce != h->C; a.loss = h->p.loss; a.nn = h->nn;
     a.gmax = h->d_gmax; a.ng = h->ng; // cleared by the root's scan
     a.ycols = h->ycols; a.compute_grads = compute_grads ? 1 : 0; a.alpha = evb_alpha_set(h); a.mode = mode;
     a.pub_src = reinterpret_cast<const uint4 *>(h->plan); a.pub_dst = static_cast<uint4 *>(publish_to); a.pub_n = publish_to ? (int)(h->h_tree_bytes / 16) : 0;
     const size_t smem = (size_t)h->nn * 4;
     a.packed_in_smem = smem <= 40 * 1024 ? 1 : 0;
-    const size_t staged = smem + (size_t)256 * (h->RS + 4);
-    static bool attr_set[64] = {}, attr_pipe[64] = {};
+    const size_t staged = smem + (size_t)256 * (h->RS + 4) + (size_t)1024 * (h->K + h->nq);
+    static bool attr_pipe[64] = {};
     static const bool direct = getenv("EVB_FINALIZE_DIRECT") != nullptr;
     static const bool no_pipe = getenv("EVB_FINALIZE_PIPE") != nullptr && atoi(getenv("EVB_FINALIZE_PIPE")) == 0;
     // pipelined kernel: rows from the chunk layout of the fixed-point histogram kernel when it exists, else from xT
@@ -849,8 +864,7 @@ int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode, void *p
     pa.S = pa.wordsA + 4; // one more chunk: room for the tail word, and an odd chunk count (wordsA / 4 is even or RSH-odd)
     if (((pa.S >> 2) & 1) == 0) pa.S += 4;
     pa.ntiles = (int)((h->n + 255) / 256);
-    pa.leaf_in_smem = h->K == 1 ? 1 : 0;
-    const size_t pipe_smem = (size_t)((h->nn + 3) & ~3) * 4 * (pa.leaf_in_smem ? 2 : 1) + (size_t)2 * 256 * pa.S * 4;
+    const size_t pipe_smem = (size_t)((h->nn + 3) & ~3) * 8 + (size_t)2 * 256 * pa.S * 4;
     evb_tic(h, EVB_T_FINALIZE);
     // measured (B200): 0.33 instead of 0.42 ms per 10M rows x 100 features with one output; with several outputs the
     // prediction and gradient streams outweigh the bins and the one-tile-per-CTA kernel below is faster
@@ -865,11 +879,25 @@ int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode, void *p
         if (per_sm < 1) per_sm = 1;
         int grid = h->num_sms * per_sm;
         if (grid > pa.ntiles) grid = pa.ntiles;
-        if (h->p.loss == EVB_MSE && a.elided && h->rec_nch == 2 && h->ycols == 1) EVB_CUDA(evb_launch_pdl(h->early, k_finalize_pipe<true>, dim3(grid), dim3(256), pipe_smem, h->st, pa));
+        if (h->p.loss == EVB_MSE && h->nq == 1) EVB_CUDA(evb_launch_pdl(h->early, k_finalize_pipe<true>, dim3(grid), dim3(256), pipe_smem, h->st, pa));
         else EVB_CUDA(evb_launch_pdl(h->early, k_finalize_pipe<false>, dim3(grid), dim3(256), pipe_smem, h->st, pa));
     } else if (mode == 0 && h->RS <= 256 && staged <= 100 * 1024 && !direct && h->dev < 64) {
-        if (!attr_set[h->dev]) { cudaFuncSetAttribute(k_finalize_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); attr_set[h->dev] = true; }
-        EVB_CUDA(evb_launch_pdl(h->early, k_finalize_staged, dim3((unsigned)((h->n + 255) / 256)), dim3(256), staged, h->st, a));
+        const dim3 tiles((unsigned)((h->n + 255) / 256));
+#define EVB_FIN(KT) do { \
+            if (staged > 48 * 1024) EVB_CUDA(cudaFuncSetAttribute(k_finalize_staged<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024)); \
+            EVB_CUDA(evb_launch_pdl(h->early, k_finalize_staged<KT>, tiles, dim3(256), staged, h->st, a)); } while (0)
+        switch (h->K) {
+        case 1: EVB_FIN(1); break;
+        case 2: EVB_FIN(2); break;
+        case 3: EVB_FIN(3); break;
+        case 4: EVB_FIN(4); break;
+        case 5: EVB_FIN(5); break;
+        case 6: EVB_FIN(6); break;
+        case 7: EVB_FIN(7); break;
+        case 8: EVB_FIN(8); break;
+        default: EVB_FIN(0);
+        }
+#undef EVB_FIN
     } else {
         EVB_CUDA(evb_launch_pdl(h->early, k_finalize, dim3((unsigned)((h->n + 255) / 256)), dim3(256), a.packed_in_smem ? smem : 0, h->st, a));
     }
@@ -902,13 +930,13 @@ int32_t evb_launch_quantile_leaves(evb_handle *h, bool use_mask, uint8_t mask_co
     QselArgs a;
     a.nidx = h->nidx; a.grad = h->grad; a.mask = use_mask ? h->mask_d : nullptr; a.cnt = h->qs_cnt; a.prefix = h->qs_prefix;
     a.rank = h->qs_rank; a.gamma = h->qs_gamma; a.t_split = h->t_split; a.nsum = h->nsum; a.t_pred = h->t_pred; a.n = h->n;
-    a.GS = h->GS; a.nn = h->nn; a.C = h->C; a.cond = mask_cond;
+    a.GS = h->nq; a.nn = h->nn; a.C = h->C; a.cond = mask_cond;
     a.eb = h->p.eta / (double)h->p.bagging_size; a.lambda = h->p.lambda; a.L2 = h->p.L2; a.K = h->K;
     a.clamp = h->p.loss == EVB_QUANTILE ? 1 : 0; // src/predict.jl:270 has the max(eps, .), :279 has not
     evb_tic(h, EVB_T_FINALIZE);
     for (int k = 0; k < h->K; ++k) { // one selection per output row: the residual of row k sits in the slot of h_k
         const int c = h->K + k;
-        a.k = k; a.roff = (c / h->rec_nch) * 4 + (c % h->rec_nch);
+        a.k = k; a.roff = c;
         a.alpha = h->p.loss == EVB_QUANTILE ? h->p.alpha : h->p.alphas[k];
         for (int pass = 0; pass < 4; ++pass) {
             a.pass = pass;
