@@ -184,17 +184,42 @@ __device__ __forceinline__ float leaf_value(const ScanArgs &a, const double *s, 
     return (float)(a.neb * g / fmax(DBL_EPSILON, h + a.lambda * s[C - 1] + a.L2));
 }
 
-// entry (channel c, bin b) of the histogram built for `slot`, feature slot f (feature id `feat`)
-__device__ __forceinline__ double built_entry(const ScanArgs &a, int slot, int f, uint32_t feat, int c, int b, int K, int C) {
-    if (a.qsum) {
-        const size_t cell = (size_t)slot * a.B + b;
-        const bool is_h2w = a.elide_h && c >= K && c < 2 * K; // h = 2w (src/loss.jl:52)
-        if (c < C - 1 && !is_h2w) return (double)(long long)__ldg(a.qsum + (cell * a.nq + c) * a.SC + feat) * __ldg(a.qinv + c);
-        const double w = a.unit_w ? (double)__ldg(a.qcnt + cell * a.SC + feat)
-                                  : (double)(long long)__ldg(a.qsum + (cell * a.nq + a.nq - 1) * a.SC + feat) * __ldg(a.qinv + a.nq - 1);
-        return is_h2w ? 2.0 * w : w;
+// Entries of the histogram built for a slot, channel by channel.  A channel's loads are issued together (`load`, raw bits) and
+// turned into doubles where they are used (`value`): a conversion or a branch between two loads would make each of them
+// wait for the one before it (measured at five classes: 20 us per node and level for a scan, 17 us for a decision).
+struct Chan {
+    bool cnt;          // row counts
+    int idx;           // quantised channel
+    double mul;
+};
+__device__ __forceinline__ Chan chan_of(const ScanArgs &a, int c, int K, int C) {
+    const bool h2w = a.elide_h && c >= K && c < 2 * K; // h = 2w (src/loss.jl:52)
+    const bool w = c == C - 1 || h2w;
+    Chan ch;
+    ch.cnt = w && a.unit_w;
+    ch.idx = w ? a.nq - 1 : c;
+    ch.mul = (h2w ? 2.0 : 1.0) * (ch.cnt || !a.qsum ? 1.0 : __ldg(a.qinv + ch.idx));
+    return ch;
+}
+// bins b0 + j * stride, j < N (past the last one: the last one again), of feature slot f / feature `feat`
+template <int N>
+__device__ __forceinline__ void chan_load(const ScanArgs &a, const Chan &ch, int slot, int f, uint32_t feat, int c, int b0, int stride, int C, long long (&raw)[N]) {
+    if (!a.qsum) {
+        const double *p = a.hcomp + (((size_t)slot * a.F + f) * C + c) * a.B;
+#pragma unroll
+        for (int j = 0; j < N; ++j) raw[j] = __double_as_longlong(p[min(b0 + j * stride, a.B - 1)]);
+    } else if (ch.cnt) {
+        const uint32_t *p = a.qcnt + (size_t)slot * a.B * a.SC + feat;
+#pragma unroll
+        for (int j = 0; j < N; ++j) raw[j] = (long long)__ldg(p + (size_t)min(b0 + j * stride, a.B - 1) * a.SC);
+    } else {
+        const unsigned long long *p = a.qsum + ((size_t)slot * a.B * a.nq + ch.idx) * a.SC + feat;
+#pragma unroll
+        for (int j = 0; j < N; ++j) raw[j] = (long long)__ldg(p + (size_t)min(b0 + j * stride, a.B - 1) * a.nq * a.SC);
     }
-    return a.hcomp[(((size_t)slot * a.F + f) * C + c) * a.B + b];
+}
+__device__ __forceinline__ double chan_value(const ScanArgs &a, const Chan &ch, long long raw) {
+    return a.qsum ? (double)raw * ch.mul : __longlong_as_double(raw);
 }
 
 // Sharded with peer access: sums the ranks' freshly built histograms for the feature slots this rank owns, by
@@ -238,7 +263,6 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     // outputs and the channel tests fold away
     const int C = K1 ? 3 : a.C, K = K1 ? 1 : a.K, B = a.B, F = a.F;
     const uint32_t feat = a.js0[f];
-    auto built = [&](int c, int b) -> double { return built_entry(a, slot, f, feat, c, b, K, C); };
     const int m = 1 << (a.level - 1);
     const size_t FCB = (size_t)F * C * B;
     const double *__restrict__ hp = a.hist + (size_t)(n >> 1) * FCB;
@@ -248,8 +272,12 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
         // root sums = sum over the bins of feature slot 0 (every sampled row has exactly one bin there);
         // the reference sums the gradients of the sampled rows directly (src/fit.jl:66)
         for (int c = 0; c < C; ++c) {
+            const Chan ch = chan_of(a, c, K, C);
+            long long raw[MAXCHK];
+            chan_load<MAXCHK>(a, ch, slot, f, feat, c, lane, 32, C, raw);
             double v = 0.0;
-            for (int b = lane; b < B; b += 32) v += built(c, b);
+#pragma unroll
+            for (int j = 0; j < MAXCHK; ++j) if (lane + 32 * j < B) v += chan_value(a, ch, raw[j]);
             v = warp_sum(v);
             if (lane == 0) { s_sum[c] = v; if (first_owned) a.nsum[(size_t)C + c] = v; }
         }
@@ -276,20 +304,22 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     const bool elide = a.elide_h != 0; // mse: every h entry is exactly twice the w entry (src/loss.jl:52), it is not read
     // entries of channel c in the lane's bins: the loads (`fetch`) run ahead of their use (`take`), which subtracts from the
     // parent's histogram and keeps the result for the children
-    struct Raw { double bv[CH], pv[CH]; };
+    struct Raw { Chan ch; long long b[CH]; double p[CH]; };
     auto fetch = [&](int c, Raw &r) {
+        r.ch = chan_of(a, c, K, C);
+        chan_load<CH>(a, r.ch, slot, f, feat, c, bin0, 1, C, r.b);
+        if (sub) {
 #pragma unroll
-        for (int j = 0; j < CH; ++j) {
-            const int b = bin0 + j;
-            r.bv[j] = b < B ? built(c, b) : 0.0;
-            r.pv[j] = sub && b < B ? __ldg(hp + fo + (size_t)c * B + b) : 0.0;
+            for (int j = 0; j < CH; ++j) r.p[j] = __ldg(hp + fo + (size_t)c * B + min(bin0 + j, B - 1));
         }
     };
     auto take = [&](int c, const Raw &r, double (&v)[CH]) {
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
             const int b = bin0 + j;
-            v[j] = sub ? r.pv[j] - r.bv[j] : r.bv[j];
+            v[j] = chan_value(a, r.ch, r.b[j]);
+            if (sub) v[j] = r.p[j] - v[j];
+            if (b >= B) v[j] = 0.0;
             if (keep && b < B) hn[fo + (size_t)c * B + b] = v[j];
         }
     };
@@ -533,33 +563,46 @@ __device__ __forceinline__ void node_select(const ScanArgs &a, int n, double *s_
         const uint32_t feat = a.js0[bs];
         const bool numeric = a.feattypes[feat] != 0;
         const size_t fo = (size_t)bs * C * B;
-        // entry (channel c, bin b) of the winner's histogram in this node
-        auto entry = [&](int c, int b) -> double {
-            const size_t o = fo + (size_t)c * B + b;
-            if (a.world > 1) return hn[o]; // sharded: the summed histogram of every scanned node is retained locally for the owned features
-            const double built = built_entry(a, slot_n, bs, feat, c, b, K, C);
-            return sub ? hp[o] - built : built;
-        };
-        // eight channels side by side: their loads and their sums over the lanes overlap
-        for (int c0 = 0; c0 < C; c0 += 8) {
-            double v[8];
+        // channels side by side: their loads and their sums over the lanes overlap
+        constexpr int NC = MAXCHK <= 2 ? 6 : 2;
+        for (int c0 = 0; c0 < C; c0 += NC) {
+            long long rb[NC][MAXCHK];
+            double rp[NC][MAXCHK], v[NC];
+            Chan ch[NC];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < NC; ++u) {
+                const int c = min(c0 + u, C - 1);
+                ch[u] = chan_of(a, c, K, C);
+                if (a.world > 1) { // sharded: the summed histogram of every scanned node is retained locally for the owned features
+#pragma unroll
+                    for (int j = 0; j < MAXCHK; ++j) rp[u][j] = hn[fo + (size_t)c * B + min(lane + 32 * j, B - 1)];
+                } else {
+                    chan_load<MAXCHK>(a, ch[u], slot_n, bs, feat, c, lane, 32, C, rb[u]);
+                    if (sub) {
+#pragma unroll
+                        for (int j = 0; j < MAXCHK; ++j) rp[u][j] = hp[fo + (size_t)c * B + min(lane + 32 * j, B - 1)];
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < NC; ++u) {
                 v[u] = 0.0;
 #pragma unroll
                 for (int j = 0; j < MAXCHK; ++j) {
                     const int b = lane + 32 * j;
-                    if (c0 + u < C && b < B && (numeric ? b <= bb : b == bb)) v[u] += entry(c0 + u, b);
+                    double e = rp[u][j];
+                    if (a.world == 1) { e = chan_value(a, ch[u], rb[u][j]); if (sub) e = rp[u][j] - e; }
+                    if (b < B && (numeric ? b <= bb : b == bb)) v[u] += e;
                 }
             }
 #pragma unroll
             for (int d = 16; d >= 1; d >>= 1) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] += __shfl_xor_sync(FULL, v[u], d);
+                for (int u = 0; u < NC; ++u) v[u] += __shfl_xor_sync(FULL, v[u], d);
             }
             if (lane == 0) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u) if (c0 + u < C) s_left[c0 + u] = v[u];
+                for (int u = 0; u < NC; ++u) if (c0 + u < C) s_left[c0 + u] = v[u];
             }
         }
         __syncwarp();
