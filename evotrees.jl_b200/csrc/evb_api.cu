@@ -264,7 +264,7 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     {
         const size_t lv = (size_t)evb_level_nodes(D > 1 ? D - 1 : 1) * nfeats;
         EVB_CUDA(dalloc(&h->fbest_gain, lv)); EVB_CUDA(dalloc(&h->fbest_bin, lv));
-        if (C == 3) EVB_CUDA(dalloc(&h->fbest_left, lv * 3));
+        if (C == 3 || evb_scan_multi(h)) EVB_CUDA(dalloc(&h->fbest_left, lv * C));
         if (p->tree_type == 1) {
             EVB_CUDA(dalloc(&h->obl_gain, ((size_t)evb_level_nodes(D > 1 ? D - 1 : 1) + 1) * nfeats * h->B));
             EVB_CUDA(dalloc(&h->obl_best, (size_t)2));

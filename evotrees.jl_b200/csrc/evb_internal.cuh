@@ -119,7 +119,7 @@ struct evb_handle {
     int32_t *scan_tmp;     // block counts for the mask compaction
     double *fbest_gain;    // [nodes of a level][nfeats] per-feature best split of the scan
     int32_t *fbest_bin;
-    double *fbest_left;    // [nodes of a level][nfeats][3] left sums of that split (one output)
+    double *fbest_left;    // [nodes of a level][nfeats][C] left sums of that split (one output, or evb_scan_multi)
     double *obl_gain;      // oblivious trees: [nodes of a level + 1][nfeats * B] gain of every candidate, last row = level totals
     double *obl_best;      // [2] gain and candidate index (-1: none) of the level's shared split
     int *d_err;            // device error word
@@ -235,6 +235,10 @@ int32_t evb_launch_histg(evb_handle *h, int level);
 int32_t evb_launch_acc_clear(evb_handle *h, int level);
 int32_t evb_launch_acc_to_hcomp(evb_handle *h, int level);
 // The split scan reads the integer accumulators itself unless ranks exchange histograms as doubles.
+// Several outputs scanned side by side (k_scan_multi).  Up to EVB_MULTI_K warps of a CTA, each with its output's sums in registers;
+// more outputs, losses with a gain of their own and oblivious trees (every bin's gain is kept) take one warp per feature.
+#define EVB_MULTI_K 8
+static inline bool evb_scan_multi(const evb_handle *h) { return h->K >= 2 && h->K <= EVB_MULTI_K && h->C == 2 * h->K + 1 && h->p.loss < EVB_MAE && h->p.tree_type != 1; }
 static inline bool evb_acc_direct(const evb_handle *h) { return h->world == 1; }
 // evb_histq2.cu
 bool evb_q2_wanted(const evb_handle *h);

@@ -619,16 +619,18 @@ __device__ __forceinline__ void node_select(const ScanArgs &a, int n, double *s_
         if (has) for (int c = lane; c < C; c += 32) rec[3 + c] = s_left[c];
     }
 }
-// The same for one output on one GPU, by the warp that scanned the node's last feature: the node sums are in s_sum already,
-// everything else is requested at once (gains, bins, left sums of up to 32 features) -- one trip to L2 and one reduction.
-__device__ __forceinline__ void node_decide_k1(const ScanArgs &a, int n, const double *s_sum, double *s_left, double *s_right, int lane) {
-    const int F = a.F, i = n - (1 << (a.level - 1));
+// The same on one GPU where the scans keep their candidates' left sums, by the warp that scanned the node's last feature: the node
+// sums are in s_sum already, gains and bins are requested at once (K1: the left sums of up to 32 features too) -- one trip to L2
+// and one reduction, for several outputs a second trip for the winner's sums.
+template <bool K1>
+__device__ __forceinline__ void node_decide(const ScanArgs &a, int n, const double *s_sum, double *s_left, double *s_right, int lane) {
+    const int F = a.F, C = K1 ? 3 : a.C, i = n - (1 << (a.level - 1));
     const double *gains = a.fbest_gain + (size_t)i * F;
     const int32_t *bins = a.fbest_bin + (size_t)i * F;
-    const double *lefts = a.fbest_left + (size_t)i * F * 3;
+    const double *lefts = a.fbest_left + (size_t)i * F * C;
     const int s0 = a.seg_start[n], c0 = a.seg_cnt[n];
     double l0 = 0.0, l1 = 0.0, l2 = 0.0;
-    if (lane < F) { l0 = __ldcg(lefts + lane * 3); l1 = __ldcg(lefts + lane * 3 + 1); l2 = __ldcg(lefts + lane * 3 + 2); }
+    if (K1 && lane < F) { l0 = __ldcg(lefts + lane * 3); l1 = __ldcg(lefts + lane * 3 + 1); l2 = __ldcg(lefts + lane * 3 + 2); }
     double bg = a.gamma;
     int bs = 0x7fffffff, bb = -1;
 #pragma unroll 4
@@ -645,7 +647,7 @@ __device__ __forceinline__ void node_decide_k1(const ScanArgs &a, int n, const d
     }
     const bool has = bs != 0x7fffffff;
     if (has) {
-        if (bs >= 32) { if (lane < 3) s_left[lane] = __ldcg(lefts + (size_t)bs * 3 + lane); }
+        if (!K1 || bs >= 32) { if (lane < C) s_left[lane] = __ldcg(lefts + (size_t)bs * C + lane); } // C <= 2 * EVB_MULTI_K + 1 < 32
         else if (lane == bs) { s_left[0] = l0; s_left[1] = l1; s_left[2] = l2; }
         if (lane == 0) { a.cur_l[n] = s0; a.cur_r[n] = s0 + c0; }
         __syncwarp();
@@ -691,9 +693,152 @@ __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_fe
         if (lane == 0) { __threadfence(); last = atomicAdd(a.ticket + n, 1u) == (unsigned)(F - 1); }
         if (!__shfl_sync(FULL, last, 0)) return;
         __threadfence();
-        if constexpr (K1) node_decide_k1(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
+        if constexpr (K1) node_decide<true>(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
         else node_select<MAXCHK, false>(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
     }
+}
+
+// Stages 1 and 2 for 2 to EVB_MULTI_K outputs with gradients and hessians on one GPU: one CTA per (node, feature), one warp per
+// output.  The gain is a sum over the outputs, so the warps load, sum and rate their outputs side by side and warp 0 adds the
+// gains up in output order; a warp still holds its running sums when the best bin is known and leaves the left sums for the
+// decision.  One warp for all outputs is a chain of 2 K + 1 channels and pairs of divisions, and the decision had to sum the
+// winner's bins again: a level of the scan took 42 us at 28 features and five classes, 18 now (2 outputs, 50 features: 23 and 14).
+template <int CH>
+__global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_multi(ScanArgs a) {
+    __shared__ double s_gain[EVB_MULTI_K][32 * CH]; // [output][j * 32 + lane] of bin lane * CH + j
+    __shared__ double s_gp[EVB_MULTI_K], s_sum[2 * EVB_MULTI_K + 1], s_left[2 * EVB_MULTI_K + 1], s_right[2 * EVB_MULTI_K + 1];
+    __shared__ int s_bin, s_last;
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int C = a.C, K = a.K, B = a.B, F = a.F;
+    evb_pdl_next();
+    evb_pdl_wait();
+    if (blockIdx.x == 0 && a.level == 1 && threadIdx.x < a.ng) a.gmax[threadIdx.x] = 0u;
+    int gw = blockIdx.x;
+    const int which = a.level > 1 ? gw & 1 : 0;
+    if (a.level > 1) gw >>= 1;
+    const int s = gw / F, f = gw % F;
+    if (s >= a.plan->nbuild) return;
+    const int nb = a.slot_node[s], n = which ? nb ^ 1 : nb, i = n - (1 << (a.level - 1));
+    const uint32_t feat = a.js0[f];
+    const bool numeric = a.feattypes[feat] != 0, sub = which != 0, keep = n < a.hist_nodes, elide = a.elide_h != 0;
+    const int constraint = k == 0 ? a.mono[feat] : 0;
+    const int bin0 = lane * CH, b_max = numeric ? B - 1 : B;
+    const size_t FCB = (size_t)F * C * B, fo = (size_t)f * C * B;
+    const double *__restrict__ hp = a.hist + (size_t)(n >> 1) * FCB + fo;
+    double *__restrict__ hn = a.hist + (size_t)n * FCB + fo;
+    // own gradient and hessian channels and the weights, which every warp needs
+    const Chan cg = chan_of(a, k, K, C), chs = chan_of(a, K + k, K, C), cw = chan_of(a, C - 1, K, C);
+    double gl[CH], hl[CH], wl[CH];
+    double sg, sh, w_p;
+    {
+        long long rg[CH], rh[CH], rw[CH];
+        chan_load<CH>(a, cw, s, f, feat, C - 1, bin0, 1, C, rw);
+        chan_load<CH>(a, cg, s, f, feat, k, bin0, 1, C, rg);
+        if (!elide) chan_load<CH>(a, chs, s, f, feat, K + k, bin0, 1, C, rh);
+        double pg[CH], ph[CH], pw[CH];
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+            const int b = min(bin0 + j, B - 1);
+            pw[j] = sub ? __ldg(hp + (size_t)(C - 1) * B + b) : 0.0;
+            pg[j] = sub ? __ldg(hp + (size_t)k * B + b) : 0.0;
+            ph[j] = sub && !elide ? __ldg(hp + (size_t)(K + k) * B + b) : 0.0;
+        }
+        if (n > 1) { sg = a.nsum[(size_t)n * C + k]; sh = a.nsum[(size_t)n * C + K + k]; w_p = a.nsum[(size_t)n * C + C - 1]; }
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+            const int b = bin0 + j;
+            wl[j] = chan_value(a, cw, rw[j]);
+            gl[j] = chan_value(a, cg, rg[j]);
+            if (sub) { wl[j] = pw[j] - wl[j]; gl[j] = pg[j] - gl[j]; }
+            if (elide) hl[j] = 2.0 * wl[j];
+            else { hl[j] = chan_value(a, chs, rh[j]); if (sub) hl[j] = ph[j] - hl[j]; }
+            if (b >= B) { wl[j] = 0.0; gl[j] = 0.0; hl[j] = 0.0; }
+            else if (keep) {
+                hn[(size_t)k * B + b] = gl[j];
+                hn[(size_t)(K + k) * B + b] = hl[j];
+                if (k == 0) hn[(size_t)(C - 1) * B + b] = wl[j];
+            }
+        }
+    }
+    if (n == 1) { // root sums over the bins of this feature (every sampled row has exactly one); feature slot 0 records them
+        sg = 0.0; sh = 0.0; w_p = 0.0;
+#pragma unroll
+        for (int j = 0; j < CH; ++j) { sg += gl[j]; sh += hl[j]; w_p += wl[j]; }
+        sg = warp_sum(sg); sh = warp_sum(sh); w_p = warp_sum(w_p);
+        if (f == 0 && lane == 0) { a.nsum[C + k] = sg; a.nsum[C + K + k] = sh; if (k == 0) a.nsum[2 * C - 1] = w_p; }
+    }
+    if (lane == 0) {
+        s_sum[k] = sg; s_sum[K + k] = sh;
+        if (k == 0) s_sum[C - 1] = w_p;
+        s_gp[k] = term_gh(sg, sh, w_p, a.lambda, a.L2);
+    }
+    if (numeric) { // running sums over the bins: inside the lane, then over the lanes' totals
+#pragma unroll
+        for (int j = 1; j < CH; ++j) { gl[j] += gl[j - 1]; hl[j] += hl[j - 1]; wl[j] += wl[j - 1]; }
+        double ig = gl[CH - 1], ih = hl[CH - 1], iw = wl[CH - 1];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const double tg = __shfl_up_sync(FULL, ig, d), th = __shfl_up_sync(FULL, ih, d), tw = __shfl_up_sync(FULL, iw, d);
+            if (lane >= d) { ig += tg; ih += th; iw += tw; }
+        }
+        ig = __shfl_up_sync(FULL, ig, 1); ih = __shfl_up_sync(FULL, ih, 1); iw = __shfl_up_sync(FULL, iw, 1);
+        if (lane > 0) {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) { gl[j] += ig; hl[j] += ih; wl[j] += iw; }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < CH; ++j) {
+        const double w_l = wl[j], w_r = w_p - w_l;
+        double g = term_gh(gl[j], hl[j], w_l, a.lambda, a.L2) + term_gh(sg - gl[j], sh - hl[j], w_r, a.lambda, a.L2);
+        bool ok = bin0 + j < b_max && w_l > a.min_weight && w_r > a.min_weight;
+        if (constraint != 0) { // pred_scalar on left / right sums (src/predict.jl:205-208, 235-238)
+            const double pl = a.neb * gl[j] / fmax(DBL_EPSILON, hl[j] + a.lambda * w_l + a.L2);
+            const double pr = a.neb * (sg - gl[j]) / fmax(DBL_EPSILON, (sh - hl[j]) + a.lambda * w_r + a.L2);
+            ok = ok && ((constraint == -1 && pl > pr) || (constraint == 1 && pl < pr));
+        }
+        s_gain[k][j * 32 + lane] = k > 0 || ok ? g : -DBL_MAX; // not a candidate: no sum exceeds gamma (gains are not negative)
+    }
+    __syncthreads();
+    if (k == 0) {
+        double gain_p = s_gp[0], lg = a.gamma; // get_best_split starts at gamma and takes strict improvements (fit-utils.jl:444-450)
+        int lb = 0x7fffffff;
+        for (int q = 1; q < K; ++q) gain_p += s_gp[q];
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+            const double first = s_gain[0][j * 32 + lane];
+            double g = first;
+            for (int q = 1; q < K; ++q) g += s_gain[q][j * 32 + lane];
+            g -= gain_p;
+            if (first != -DBL_MAX && g > lg && a.level < a.D) { lg = g; lb = bin0 + j; }
+        }
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) {
+            const double og = __shfl_xor_sync(FULL, lg, d);
+            const int ob = __shfl_xor_sync(FULL, lb, d);
+            if (og > lg || (og == lg && ob < lb)) { lg = og; lb = ob; }
+        }
+        if (lane == 0) {
+            a.fbest_gain[(size_t)i * F + f] = lg;
+            a.fbest_bin[(size_t)i * F + f] = lb == 0x7fffffff ? -1 : lb;
+            s_bin = lb;
+        }
+    }
+    __syncthreads();
+    const int bin = s_bin;
+    if (bin != 0x7fffffff) {
+        double *l = a.fbest_left + ((size_t)i * F + f) * C;
+#pragma unroll
+        for (int j = 0; j < CH; ++j)
+            if (bin0 + j == bin) { l[k] = gl[j]; l[K + k] = hl[j]; if (k == 0) l[C - 1] = wl[j]; }
+    }
+    __syncthreads();
+    if (k != 0) return;
+    if (lane == 0) { __threadfence(); s_last = atomicAdd(a.ticket + n, 1u) == (unsigned)(F - 1); }
+    __syncwarp();
+    if (!s_last) return;
+    __threadfence();
+    node_decide<false>(a, n, s_sum, s_left, s_right, lane);
 }
 
 // Stage 3 (sharded with peer access only): every rank picks, for every node, the best of the ranks' candidates
@@ -1081,7 +1226,11 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
     }
     const long long warps = (long long)slots * Fown * (level > 1 ? 2 : 1);
     evb_tic(h, EVB_T_SCAN);
-    if (warps > 0) {
+    if (fused && evb_scan_multi(h)) {
+#define EVB_SCAN(M) EVB_CUDA(evb_launch_pdl(h->early, k_scan_multi<M>, dim3((unsigned)warps), dim3(32 * h->K), 0, h->st, a))
+        if (h->B <= 32) EVB_SCAN(1); else if (h->B <= 64) EVB_SCAN(2); else if (h->B <= 128) EVB_SCAN(4); else EVB_SCAN(8);
+#undef EVB_SCAN
+    } else if (warps > 0) {
         const unsigned grid = (unsigned)((warps + 7) / 8);
         const bool own = h->p.loss >= EVB_MAE;
         const bool obl = h->obl_gain != nullptr;
