@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(1024, 1) k_histg(KArgs k) {
     const int P = evb_hg_planes(k.g, blockIdx.z), words = nparts(a.nfull, a.tails) * (a.B + 1) * P * 8;
     for (int i = threadIdx.x; i < words; i += blockDim.x) reinterpret_cast<uint4 *>(s_img)[i] = make_uint4(0u, 0u, 0u, 0u);
     evb_pdl_wait();
-    if ((long long)blockIdx.x * a.min_rows >= max(1ll, (long long)a.plan->R)) return;
+    if ((long long)blockIdx.x * a.min_rows >= max(1ll, (long long)a.plan->R + (long long)a.plan->nbuild * a.pad_rows)) return;
     __syncthreads();
     EVB_HG_DISPATCH(k.g, blockIdx.z, run, a, s_img)
 }
@@ -112,6 +112,9 @@ int32_t evb_hg_configure(evb_handle *h) {
     split_words(W, nf, tl);
     const int parts = nparts(nf, tl), fit = (int)(SMEM_ONE / part);
     g.ngf = (parts + fit - 1) / fit;
+    // fewer rows below the root than the SMs can share (256 each): a CTA takes one part only, its flush is shorter too (60k x 77:
+    // 0.153 -> 0.149 ms per tree; two CTAs of unequal numbers of parts are slower than one)
+    if (h->n / 2 / 256 * g.ngf < h->num_sms) g.ngf = parts;
     const int per_group = (parts + g.ngf - 1) / g.ngf;
     g.wper = g.ngf == 1 ? W : per_group * 8;
     g.ngf = (W + g.wper - 1) / g.wper;
@@ -120,7 +123,8 @@ int32_t evb_hg_configure(evb_handle *h) {
     for (int y = 0; y < g.ngf; ++y) { split_words(std::min(g.wper, W - y * g.wper), nf, tl); most = std::max(most, nparts(nf, tl)); }
     g.smem = most * part;
     g.threads = g.smem <= SMEM_TWO ? 512 : 1024;
-    g.min_rows = 512;
+    // up to four words a row is cheap: 256 rows are too few for a flush (100k x 10 0.099 -> 0.104 ms per tree)
+    g.min_rows = g.wper <= 4 ? 512 : 256;
     EVB_CUDA(cudaFuncSetAttribute(k_histg, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     int occ = 0;
     EVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_histg, g.threads, g.smem));
@@ -134,7 +138,7 @@ size_t evb_hg_q_words(const evb_handle *h) { return evb_hg_qoff(h->hgeo, h->n, h
 void evb_hg_args(const evb_handle *h, int level, evb_hg::Args *a) {
     a->xT = h->xT; a->q = h->gradq; a->rows = h->rows[(level - 1) & 1]; a->plan = h->plan + level; a->cum = h->cum; a->slot_node = h->slot_node;
     a->seg_start = h->seg_start; a->hsum = h->hsum_q; a->hcnt = h->hcnt_q; a->RS = h->RS; a->B = h->B; a->SC = h->SC; a->nq = h->nq; a->F = h->nfeats;
-    a->TE = h->hgeo.TE; a->min_rows = h->hgeo.min_rows; a->n = h->n;
+    a->TE = h->hgeo.TE; a->min_rows = h->hgeo.min_rows; a->pad_rows = evb_pad_rows(h); a->n = h->n;
 }
 
 void evb_hg_quant_args(const evb_handle *h, evb_hg::QuantArgs *a) {

@@ -39,6 +39,7 @@ struct Args {
     int nfull, tails;         // parts of 8 words; bit mask of the tail parts (4, 2, 1)
     int TE;                   // tiles of 32 rows between two flushes
     int min_rows;             // rows per CTA below which fewer CTAs take part
+    int pad_rows;             // what the flush of a slot costs, in rows
     long long n;              // rows of q
 };
 
@@ -193,7 +194,9 @@ template <int NQ, bool CNT, bool PACK>
 __device__ __forceinline__ void accumulate(const Args &a, uint32_t *smem, int b, int G) {
     constexpr int P = planes(NQ, CNT, PACK), NQP = nqp(NQ);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, NW = blockDim.x >> 5;
-    const long long R = a.plan->R;
+    const int nbuild = a.plan->nbuild;
+    // every slot is followed by pad_rows rows that do not exist
+    const long long R = a.plan->R + (long long)nbuild * a.pad_rows;
     {
         const long long want = (R + a.min_rows - 1) / a.min_rows;
         if (want < G) G = want < 1 ? 1 : (int)want;
@@ -201,18 +204,19 @@ __device__ __forceinline__ void accumulate(const Args &a, uint32_t *smem, int b,
     if (b >= G) return;
     const int lo = (int)(R * b / G), hi = (int)(R * (b + 1) / G);
     if (lo >= hi) return;
-    const int nbuild = a.plan->nbuild;
     int s;
     {
-        int l = 0, r = nbuild - 1; // largest s with cum[s] <= lo
-        while (l < r) { const int m = (l + r + 1) >> 1; if (a.cum[m] <= lo) l = m; else r = m - 1; }
+        int l = 0, r = nbuild - 1; // largest s with cum[s] + s * pad_rows <= lo
+        while (l < r) { const int m = (l + r + 1) >> 1; if (a.cum[m] + m * a.pad_rows <= lo) l = m; else r = m - 1; }
         s = l;
     }
     Lane ln;
     ln.init(smem, lane);
     const uint32_t pb = (uint32_t)(a.B + 1) * P * 128;
-    for (int pos = lo; pos < hi; ++s) {
-        const int c0 = a.cum[s], pe = min(hi, a.cum[s + 1]);
+    for (; s < nbuild; ++s) {
+        const int c0 = a.cum[s], off = s * a.pad_rows;
+        if (c0 + off >= hi) break;
+        const int pos = max(lo - off, c0), pe = min(hi - off, a.cum[s + 1]);
         if (pe <= pos) continue;
         const uint32_t *rows = a.rows + ((long long)a.seg_start[a.slot_node[s]] - c0);
         // a piece; every TE tiles the image is emptied
@@ -252,7 +256,6 @@ __device__ __forceinline__ void accumulate(const Args &a, uint32_t *smem, int b,
             flush<NQ, CNT, PACK>(a, smem, s);
             __syncthreads();
         }
-        pos = pe;
     }
 }
 

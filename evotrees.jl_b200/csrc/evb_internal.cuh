@@ -235,6 +235,14 @@ int32_t evb_launch_histg(evb_handle *h, int level);
 int32_t evb_launch_acc_clear(evb_handle *h, int level);
 int32_t evb_launch_acc_to_hcomp(evb_handle *h, int level);
 // The split scan reads the integer accumulators itself unless ranks exchange histograms as doubles.
+// Rows of a level are dealt out to the CTAs of a histogram kernel with this many more for every build node: a flush costs what a
+// few hundred rows do, so a CTA with several small nodes gets fewer rows than one inside a large node.  Per tree, equal ranges
+// and 512 rows at least, then padded ones and 256: 1503 x 7 0.096 -> 0.087 ms, 60k x 77 0.183 -> 0.150, 250k x 33 weighted
+// 0.208 -> 0.190, 2M x 28 five classes 0.98 -> 0.94, 5M x 50 gaussian 1.51 -> 1.49.  Positions stay below 2^31.
+static inline int evb_pad_rows(const evb_handle *h) {
+    const long long room = (0x7fffffffll - h->n) / (h->maxslots > 0 ? h->maxslots : 1);
+    return room < 512 ? (room < 0 ? 0 : (int)room) : 512;
+}
 // Several outputs scanned side by side (k_scan_multi).  Up to EVB_MULTI_K warps of a CTA, each with its output's sums in registers;
 // more outputs, losses with a gain of their own and oblivious trees (every bin's gain is kept) take one warp per feature.
 #define EVB_MULTI_K 8
