@@ -140,6 +140,13 @@ struct ScanArgs {
     double lambda, L2, gamma, min_weight;
 };
 
+// Counts arrivals: what the arriving thread (and threads it has synchronised with) wrote before is visible to whoever sees the count.
+// One release-acquire operation instead of fences on both sides of a relaxed one, each of which waits for L2 (0.5 us).
+__device__ __forceinline__ uint32_t arrive(uint32_t *count) {
+    uint32_t v;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(count) : "memory");
+    return v;
+}
 __device__ __forceinline__ double term_gh(double g, double h, double w, double lambda, double L2) {
     return g * g / fmax(DBL_EPSILON, h + lambda * w + L2) / 2.0; // src/split.jl:1
 }
@@ -403,7 +410,6 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
         if (K1 && mine == lb && lb != 0x7fffffff) { // a bin is one lane's
             double *l = a.fbest_left + ((size_t)(n - m) * F + f) * 3;
             l[0] = best_g; l[1] = best_h; l[2] = best_w;
-            if (a.ticket) __threadfence();
         }
     }
     __syncwarp();
@@ -670,7 +676,8 @@ __global__ void __launch_bounds__(256) k_scan_node(ScanArgs a) {
 // stored as well.  The default instance carries neither code.
 template <int MAXCHK, bool OWN, bool OBL, bool K1>
 __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_feat(ScanArgs a) {
-    __shared__ double s_sum_all[8][72], s_left_all[8][72], s_right_all[8][72];
+    constexpr int NCH = K1 ? 3 : 72;
+    __shared__ double s_sum_all[8][NCH], s_left_all[8][NCH], s_right_all[8][NCH];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     const int F = a.F;
     const int Fown = (F - a.rank + a.world - 1) / a.world;
@@ -690,9 +697,9 @@ __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_fe
     if (!OBL && a.ticket) {
         // the warp that scans the node's last feature decides the node: no launch of its own for that
         unsigned last = 0;
-        if (lane == 0) { __threadfence(); last = atomicAdd(a.ticket + n, 1u) == (unsigned)(F - 1); }
+        if (lane == 0) last = arrive(a.ticket + n) == (unsigned)(F - 1);
         if (!__shfl_sync(FULL, last, 0)) return;
-        __threadfence();
+        __syncwarp();
         if constexpr (K1) node_decide<true>(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
         else node_select<MAXCHK, false>(a, n, s_sum_all[wid], s_left_all[wid], s_right_all[wid], lane);
     }
@@ -834,10 +841,9 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
     }
     __syncthreads();
     if (k != 0) return;
-    if (lane == 0) { __threadfence(); s_last = atomicAdd(a.ticket + n, 1u) == (unsigned)(F - 1); }
+    if (lane == 0) s_last = arrive(a.ticket + n) == (unsigned)(F - 1);
     __syncwarp();
     if (!s_last) return;
-    __threadfence();
     node_decide<false>(a, n, s_sum, s_left, s_right, lane);
 }
 
@@ -952,10 +958,11 @@ __device__ __forceinline__ void plan_level(const PartArgs &a, int *sm) {
         const int i = base + threadIdx.x;
         const int n = lo + i;
         int sp = 0, cnt_build = 0, cnt_all = 0, build_child = 0;
-        if (i < m && a.t_split[n - 1]) {
+        const int nq = min(n, 2 * m - 1); // all loads at once, needed or not
+        const int split = a.t_split[nq - 1], s0 = a.seg_start[nq], c0 = a.seg_cnt[nq], nl = __ldcg(a.cur_l + nq) - s0;
+        if (i < m && split) {
             sp = 1;
             const int L = n << 1, Rn = L + 1;
-            const int s0 = a.seg_start[n], c0 = a.seg_cnt[n], nl = __ldcg(a.cur_l + n) - s0;
             a.seg_start[L] = s0; a.seg_cnt[L] = nl;
             a.seg_start[Rn] = s0 + nl; a.seg_cnt[Rn] = c0 - nl;
             cnt_all = c0;
@@ -1114,13 +1121,9 @@ __global__ void __launch_bounds__(EVB_PART_THREADS) k_partition(PartArgs a) {
     else if (total > EVB_PART_THREADS * (int)gridDim.x) partition_chunks<4>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
     else partition_chunks<1>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_misc[33] = atomicAdd(a.done, 1u) == gridDim.x - 1;
-    }
+    if (threadIdx.x == 0) s_misc[33] = arrive(a.done) == gridDim.x - 1;
     __syncthreads();
     if (!s_misc[33]) return;
-    __threadfence();
     if (threadIdx.x == 0) *a.done = 0u;
     if (a.level > 6) plan_level<false>(a, s_misc);
     else if (threadIdx.x < 32) plan_level<true>(a, s_misc);
