@@ -30,7 +30,7 @@ enum { EVB_DERR_NONE = 0, EVB_DERR_WAIT_FULL = 1, EVB_DERR_WAIT_EMPTY = 2, EVB_D
 
 // ---- geometry constants ---------------------------------------------------------------------------
 constexpr int EVB_TILE_ROWS = 32;    // rows per staged tile (one per producer lane)
-constexpr int EVB_PART_CHUNK = 2048; // rows per partition work item
+constexpr int EVB_PART_CHUNK = 1024; // rows of the largest partition chunk
 constexpr int EVB_PART_THREADS = 256;
 constexpr int EVB_MAX_DEPTH = 15;
 constexpr int EVB_GEN_WORDS = 12;    // 32-bit words of a generator state

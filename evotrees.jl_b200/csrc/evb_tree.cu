@@ -1009,7 +1009,12 @@ __device__ __forceinline__ bool goes_left(uint32_t pk, uint32_t x) { // split_se
     const uint32_t bin = (pk >> 16) & 0xffu;
     return ((pk >> 25) & 1u) ? (x <= bin) : (x == bin);
 }
-constexpr int PART_WARPS = EVB_PART_THREADS / 32;
+// Every CTA takes a range of adjacent chunks: the node of the next one is known without a search unless it ends, and its row ids are
+// on their way while this one's bins arrive and its places are reserved.  What bounds a chunk is that chain of trips to L2, so
+// CTAs matter more than rows per thread: six CTAs of four rows a thread 0.640 ms per tree at 10M x 100, depth 11 (5M x 50 gaussian
+// 0.153), four of eight 0.69 (0.163), eight of four (registers spill) 0.67 (0.167); chunks dealt out in turn and searched for
+// one by one, four of eight, took 0.727 (0.192).
+constexpr int PART_WARPS = EVB_PART_THREADS / 32, PART_CTAS = 6;
 template <int NI>
 __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G, int npl, int total, uint32_t *s_bits, int *s_pref, int *s_misc) {
     constexpr int CHUNK = NI * EVB_PART_THREADS;
@@ -1019,27 +1024,37 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
     auto locate = [&](int p, int &node, int &n0, int &n1, int &off) {
         int l = 0, r = npl - 1; // largest pair with pl_cum <= p
         while (l < r) { const int mid = (l + r + 1) >> 1; if (a.pl_cum[mid] <= p) l = mid; else r = mid - 1; }
-        const int c0 = a.pl_cum[l], first = a.pl_node[l], cl = a.seg_cnt[first];
-        off = a.seg_start[first] - c0; // position -> place in the row list (the pair's segments are adjacent)
-        if (p < c0 + cl) { node = first; n0 = c0; n1 = c0 + cl; }
-        else { node = first + 1; n0 = c0 + cl; n1 = a.pl_cum[l + 1]; }
+        const int c0 = a.pl_cum[l], head = a.pl_node[l], cl = a.seg_cnt[head];
+        off = a.seg_start[head] - c0; // position -> place in the row list (the pair's segments are adjacent)
+        if (p < c0 + cl) { node = head; n0 = c0; n1 = c0 + cl; }
+        else { node = head + 1; n0 = c0 + cl; n1 = a.pl_cum[l + 1]; }
     };
-    for (int chunk = b; chunk < nchunks; chunk += G) {
+    const int first = (int)((long long)nchunks * b / G), last = (int)((long long)nchunks * (b + 1) / G);
+    int node = 0, n0 = 0, n1 = 0, off = 0;
+    bool ahead = false;
+    uint32_t next[NI];
+    for (int chunk = first; chunk < last; ++chunk) {
         const int p0 = chunk * CHUNK, p1 = min(total, p0 + CHUNK);
-        int node, n0, n1, off;
-        locate(p0, node, n0, n1, off);
+        if (p0 >= n1 || p0 < n0) { locate(p0, node, n0, n1, off); ahead = false; }
         uint32_t row[NI], x[NI];
         if (p1 <= n1) { // one node
             const uint32_t pk = a.t_packed[node - 1];
-            if (!((pk >> 24) & 1u)) continue; // not split; uniform
+            if (!((pk >> 24) & 1u)) { ahead = false; continue; } // not split; uniform
             const uint8_t *xf = a.xC + (size_t)(pk & 0xffffu) * a.n;
             const uint32_t *in = a.rows_in + (p0 + off);
             const int cnt = p1 - p0;
             // all row ids first, then all gathers: NI independent loads in flight per thread in each phase
 #pragma unroll
-            for (int i = 0; i < NI; ++i) { const int q = i * EVB_PART_THREADS + threadIdx.x; row[i] = q < cnt ? __ldg(in + q) : 0xffffffffu; }
+            for (int i = 0; i < NI; ++i) { const int q = i * EVB_PART_THREADS + threadIdx.x; row[i] = ahead ? next[i] : q < cnt ? __ldg(in + q) : 0xffffffffu; }
 #pragma unroll
             for (int i = 0; i < NI; ++i) x[i] = row[i] != 0xffffffffu ? (uint32_t)__ldg(xf + row[i]) : 0xffffu;
+            // the next chunk's row ids, if it lies in the same node
+            const int more = min(total, p1 + CHUNK) - p1;
+            ahead = chunk + 1 < last && p1 + more <= n1;
+            if (ahead) {
+#pragma unroll
+                for (int i = 0; i < NI; ++i) { const int q = i * EVB_PART_THREADS + threadIdx.x; next[i] = q < more ? __ldg(in + CHUNK + q) : 0xffffffffu; }
+            }
             unsigned left = 0;
 #pragma unroll
             for (int i = 0; i < NI; ++i) {
@@ -1048,11 +1063,9 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
                 if (lane == 0) s_bits[i * PART_WARPS + wid] = bal;
             }
             __syncthreads();
-            if (wid == 0) { // NI * 8 <= 64 words: two per lane
-                const int c0 = 2 * lane < NI * PART_WARPS ? __popc(s_bits[2 * lane]) : 0, c1 = 2 * lane < NI * PART_WARPS ? __popc(s_bits[2 * lane + 1]) : 0;
-                const int incl = warp_incl_scan_i(c0 + c1, lane);
-                s_pref[2 * lane] = incl - c0 - c1;
-                s_pref[2 * lane + 1] = incl - c1;
+            if (wid == 0) { // NI * 8 <= 32 words: one per lane
+                const int c = lane < NI * PART_WARPS ? __popc(s_bits[lane]) : 0, incl = warp_incl_scan_i(c, lane);
+                s_pref[lane] = incl - c;
                 if (lane == 31) {
                     s_misc[0] = atomicAdd(a.cur_l + node, incl);
                     s_misc[1] = atomicSub(a.cur_r + node, cnt - incl) - (cnt - incl);
@@ -1070,6 +1083,7 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
             }
             __syncthreads();
         } else {
+            ahead = false;
             // 2 * node + side of every row, 0: not a row of a split node
             uint32_t key[NI];
 #pragma unroll
@@ -1104,7 +1118,7 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
         }
     }
 }
-__global__ void __launch_bounds__(EVB_PART_THREADS) k_partition(PartArgs a) {
+__global__ void __launch_bounds__(EVB_PART_THREADS, PART_CTAS) k_partition(PartArgs a) {
     __shared__ uint32_t s_bits[EVB_PART_CHUNK / 32];
     __shared__ int s_pref[EVB_PART_CHUNK / 32], s_misc[34];
     evb_pdl_next();
@@ -1117,8 +1131,9 @@ __global__ void __launch_bounds__(EVB_PART_THREADS) k_partition(PartArgs a) {
         for (size_t i = i0; i < nc; i += st) a.hcnt[i] = 0u;
     }
     // few rows: small chunks, so that they spread over the GPU (their chain of dependent loads is what takes the time)
-    if (total > 4 * EVB_PART_THREADS * (int)gridDim.x) partition_chunks<8>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
-    else if (total > EVB_PART_THREADS * (int)gridDim.x) partition_chunks<4>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
+    const int each = total / (int)gridDim.x;
+    if (each > 2 * EVB_PART_THREADS) partition_chunks<4>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
+    else if (each > EVB_PART_THREADS) partition_chunks<2>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
     else partition_chunks<1>(a, blockIdx.x, gridDim.x, npl, total, s_bits, s_pref, s_misc);
     __syncthreads();
     if (threadIdx.x == 0) s_misc[33] = arrive(a.done) == gridDim.x - 1;
@@ -1148,7 +1163,7 @@ PartArgs make_part_args(evb_handle *h, int level) {
 
 } // namespace
 
-static_assert(EVB_PART_CHUNK == 2048 && EVB_PART_THREADS == 256, "k_partition assumes 64 ballot words per chunk");
+static_assert(EVB_PART_CHUNK == 1024 && EVB_PART_THREADS == 256, "k_partition assumes 32 ballot words per chunk");
 
 int32_t evb_launch_tree_begin(evb_handle *h, bool quantize, bool all_rows, const uint32_t *gen_js_host) {
     BeginArgs a;
@@ -1272,7 +1287,7 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
 int32_t evb_launch_partition(evb_handle *h, int level) {
     PartArgs a = make_part_args(h, level);
     const int64_t chunks = (h->n + EVB_PART_THREADS - 1) / EVB_PART_THREADS; // the smallest ones
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(h->num_sms * 8, chunks));
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(h->num_sms * PART_CTAS, chunks));
     evb_tic(h, EVB_T_PARTITION);
     const cudaError_t e = evb_launch_pdl(h->early, k_partition, dim3(grid), dim3(EVB_PART_THREADS), 0, h->st, a);
     evb_toc(h, EVB_T_PARTITION);
