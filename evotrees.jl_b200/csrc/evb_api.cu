@@ -258,8 +258,8 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     h->early = n <= 1000000;
 
     h->maxslots = evb_level_slots(D > 1 ? D - 1 : 1);
-    EVB_CUDA(dalloc(&h->cum, (size_t)h->maxslots + 1)); EVB_CUDA(dalloc(&h->slot_node, (size_t)h->maxslots));
-    EVB_CUDA(dalloc(&h->pl, ((size_t)h->maxslots + 1) * 4));
+    EVB_CUDA(dalloc(&h->cum, (size_t)h->maxslots + 1)); EVB_CUDA(dalloc(&h->slot_node, (size_t)h->maxslots * 2)); h->rbase = h->slot_node + h->maxslots;
+    EVB_CUDA(dalloc(&h->pl, ((size_t)h->maxslots + 1) * 2));
     EVB_CUDA(dalloc(&h->scan_tmp, (size_t)(n / 2048 + 2)));
     {
         const size_t lv = (size_t)evb_level_nodes(D > 1 ? D - 1 : 1) * nfeats;

@@ -136,8 +136,8 @@ int32_t evb_hg_configure(evb_handle *h) {
 size_t evb_hg_q_words(const evb_handle *h) { return evb_hg_qoff(h->hgeo, h->n, h->hgeo.ngc) + 8; }
 
 void evb_hg_args(const evb_handle *h, int level, evb_hg::Args *a) {
-    a->xT = h->xT; a->q = h->gradq; a->rows = h->rows[(level - 1) & 1]; a->plan = h->plan + level; a->cum = h->cum; a->slot_node = h->slot_node;
-    a->seg_start = h->seg_start; a->hsum = h->hsum_q; a->hcnt = h->hcnt_q; a->RS = h->RS; a->B = h->B; a->SC = h->SC; a->nq = h->nq; a->F = h->nfeats;
+    a->xT = h->xT; a->q = h->gradq; a->rows = h->rows[(level - 1) & 1]; a->plan = h->plan + level; a->cum = h->cum; a->rbase = h->rbase;
+    a->hsum = h->hsum_q; a->hcnt = h->hcnt_q; a->RS = h->RS; a->B = h->B; a->SC = h->SC; a->nq = h->nq; a->F = h->nfeats;
     a->TE = h->hgeo.TE; a->min_rows = h->hgeo.min_rows; a->pad_rows = evb_pad_rows(h); a->n = h->n;
 }
 

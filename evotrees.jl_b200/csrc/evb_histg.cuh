@@ -31,7 +31,7 @@ struct Args {
     const int32_t *q;         // [n][NQP] words of this CTA's channels
     const uint32_t *rows;
     const LevelPlan *plan;
-    const int32_t *cum, *slot_node, *seg_start;
+    const int32_t *cum, *rbase;
     unsigned long long *hsum; // [slot][bin][nq][SC]
     uint32_t *hcnt;           // [slot][bin][SC]
     int RS, B, SC, nq, ch0;   // ch0: first channel of this CTA
@@ -218,7 +218,7 @@ __device__ __forceinline__ void accumulate(const Args &a, uint32_t *smem, int b,
         if (c0 + off >= hi) break;
         const int pos = max(lo - off, c0), pe = min(hi - off, a.cum[s + 1]);
         if (pe <= pos) continue;
-        const uint32_t *rows = a.rows + ((long long)a.seg_start[a.slot_node[s]] - c0);
+        const uint32_t *rows = a.rows + a.rbase[s];
         // a piece; every TE tiles the image is emptied
         for (int p0 = pos; p0 < pe; p0 += a.TE * 32) {
             const int p1 = min(pe, p0 + a.TE * 32);

@@ -42,7 +42,7 @@ struct Q2Args {
     const uint2 *xE;
     const uint32_t *rows;
     const LevelPlan *plan;
-    const int32_t *cum, *slot_node, *seg_start;
+    const int32_t *cum, *rbase;
     unsigned long long *hsum; // [slot][bin][SC] sums of q
     uint32_t *hcnt;           // [slot][bin][SC] row counts
     int RSH, B, SC;
@@ -112,7 +112,7 @@ __device__ __forceinline__ void piece_load(const Q2Args &a, PieceIt &it, int lo,
         const int ps = max(lo - off, c0), pe = min(hi - off, c1);
         if (pe > ps) {
             it.pstart = ps; it.pend = pe; it.nt = (pe - ps + 31) >> 5;
-            it.rows = a.rows + ((long long)a.seg_start[a.slot_node[it.s]] - c0);
+            it.rows = a.rows + a.rbase[it.s];
             return;
         }
         ++it.s;
@@ -421,7 +421,7 @@ int32_t evb_launch_histq2(evb_handle *h, int level) {
     const Q2Geom &g = h->q2;
     Q2Args a;
     a.xH = h->xH; a.xE = h->xE; a.rows = h->rows[(level - 1) & 1];
-    a.plan = h->plan + level; a.cum = h->cum; a.slot_node = h->slot_node; a.seg_start = h->seg_start;
+    a.plan = h->plan + level; a.cum = h->cum; a.rbase = h->rbase;
     a.hsum = h->hsum_q; a.hcnt = h->hcnt_q;
     a.RSH = g.RSH; a.B = h->B; a.SC = h->SC; a.nmain = g.nmain; a.ntail = g.ntail; a.min_rows = g.min_rows; a.pad_rows = evb_pad_rows(h); a.zrow = (uint32_t)h->n;
     evb_tic(h, EVB_T_HIST);

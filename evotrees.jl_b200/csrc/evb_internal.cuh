@@ -103,7 +103,7 @@ struct evb_handle {
     int32_t *seg_start, *seg_cnt; // local row segment of each node
     int32_t *cur_l, *cur_r;       // partition cursors of split nodes
     uint32_t *ticket;             // [nn+2] features of a node whose scan is done; entry 0: CTAs of k_partition that are done
-    int32_t *pl;                  // 2 x {pl_node, pl_cum}[maxslots+1]: sibling pairs of a level and the running sum of their rows
+    int4 *pl;                     // 2 x [maxslots+1] sibling pairs of a level (PartArgs::pl)
     uint8_t *kind;
     int32_t *bslot;
     double *nsum;                 // [nn+1][C]
@@ -115,6 +115,7 @@ struct evb_handle {
     LevelPlan *plan;       // [D+1]
     int32_t *cum;          // [maxslots+1] exclusive prefix of build-node row counts (current level)
     int32_t *slot_node;    // [maxslots]
+    int32_t *rbase;        // [maxslots] place in the row list of a slot's first row, minus cum[slot] (behind slot_node)
     int maxslots;
     int32_t *scan_tmp;     // block counts for the mask compaction
     double *fbest_gain;    // [nodes of a level][nfeats] per-feature best split of the scan

@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(SEL_THREADS) k_sel_pcg(const uint64_t *gen, ui
         bcnt[blockIdx.x] = tot;
     }
 }
-struct RootPlan { int32_t *seg_cnt, *cum, *slot_node, *pl_node, *pl_cum; uint8_t *kind; LevelPlan *plan; };
+struct RootPlan { int32_t *seg_cnt, *cum, *slot_node, *rbase; int4 *pl; uint8_t *kind; LevelPlan *plan; };
 __global__ void __launch_bounds__(1024) k_sel_scan(int32_t *bcnt, int nblocks, RootPlan r) {
     evb_pdl_next();
     evb_pdl_wait();
@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(1024) k_sel_scan(int32_t *bcnt, int nblocks, R
     }
     if (threadIdx.x == 0) { // the root: its rows are the sampled ones
         r.seg_cnt[1] = carry; r.kind[1] = EVB_KIND_BUILD;
-        r.cum[0] = 0; r.cum[1] = carry; r.slot_node[0] = 1;
-        r.pl_node[0] = 1; r.pl_cum[0] = 0; r.pl_cum[1] = carry;
+        r.cum[0] = 0; r.cum[1] = carry; r.slot_node[0] = 1; r.rbase[0] = 0;
+        r.pl[0] = make_int4(1, 0, carry, 0); r.pl[1] = make_int4(0, carry, 0, 0);
         r.plan[1].nbuild = 1; r.plan[1].npl = 1; r.plan[1].R = carry; r.plan[1].n_sel = carry; r.plan[1].total = carry;
     }
 }
@@ -828,7 +828,7 @@ void evb_pcg_advance(uint64_t gen[6], int64_t n) {
 int32_t evb_launch_rows_init(evb_handle *h, int use_mask, uint8_t mask_cond) {
     if (!use_mask) return EVB_OK;
     const int nblocks = (int)((h->n + SEL_CHUNK - 1) / SEL_CHUNK);
-    const RootPlan r{h->seg_cnt, h->cum, h->slot_node, h->pl, h->pl + h->maxslots + 1, h->kind, h->plan};
+    const RootPlan r{h->seg_cnt, h->cum, h->slot_node, h->rbase, h->pl, h->kind, h->plan};
     evb_tic(h, EVB_T_ROWS_INIT);
     if (use_mask == EVB_MASK_PCG) EVB_CUDA(evb_launch_pdl(h->early, k_sel_pcg, dim3(nblocks), dim3(SEL_THREADS), 0, h->st, h->gen_d, mask_cond, h->n, h->mask_d, h->scan_tmp));
     else EVB_CUDA(evb_launch_pdl(h->early, k_sel_count, dim3(nblocks), dim3(SEL_THREADS), 0, h->st, h->mask_d, mask_cond, h->n, h->scan_tmp));

@@ -55,7 +55,8 @@ __device__ __forceinline__ int block_excl_scan(int v, int *sm, int *total) {
 
 // ------------------------------------------------------------------------------------------ begin of a tree
 struct BeginArgs {
-    int32_t *seg_start, *seg_cnt, *bslot, *t_feat, *cum, *slot_node, *pl_node, *pl_cum;
+    int32_t *seg_start, *seg_cnt, *bslot, *t_feat, *cum, *slot_node, *rbase;
+    int4 *pl;
     uint8_t *kind, *t_bin, *t_split;
     float *t_gain, *t_w, *t_pred;
     uint32_t *t_packed;
@@ -82,8 +83,8 @@ __global__ void __launch_bounds__(256) k_tree_begin(BeginArgs a) {
         a.seg_start[i] = 0; a.seg_cnt[i] = root ? (int32_t)a.q.n : 0; a.kind[i] = root ? EVB_KIND_BUILD : EVB_KIND_NONE; a.bslot[i] = 0; a.ticket[i] = 0u;
         for (int c = 0; c < a.C; ++c) a.nsum[(size_t)i * a.C + c] = 0.0;
         if (root) {
-            a.cum[0] = 0; a.cum[1] = (int32_t)a.q.n; a.slot_node[0] = 1;
-            a.pl_node[0] = 1; a.pl_cum[0] = 0; a.pl_cum[1] = (int32_t)a.q.n;
+            a.cum[0] = 0; a.cum[1] = (int32_t)a.q.n; a.slot_node[0] = 1; a.rbase[0] = 0;
+            a.pl[0] = make_int4(1, 0, (int32_t)a.q.n, 0); a.pl[1] = make_int4(0, (int32_t)a.q.n, 0, 0);
             a.plan[1].nbuild = 1; a.plan[1].npl = 1; a.plan[1].R = a.q.n; a.plan[1].n_sel = (int32_t)a.q.n; a.plan[1].total = (int32_t)a.q.n;
         }
     }
@@ -117,6 +118,7 @@ struct ScanArgs {
     double *obl_gain, *obl_best;
     const LevelPlan *plan;
     const int32_t *slot_node;
+    int slots; // build slots the level can have
     // Row-sharded runs with peer access: every rank scans the feature slots f with f % world == rank (`hcomp` then
     // points at the sums made by k_peer_reduce) and publishes one candidate per node to every rank.
     double *peer_cand[EVB_MAX_PEERS];
@@ -145,6 +147,12 @@ struct ScanArgs {
 __device__ __forceinline__ uint32_t arrive(uint32_t *count) {
     uint32_t v;
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(count) : "memory");
+    return v;
+}
+// a load that is issued where it stands, not moved behind the branch its value is used in
+__device__ __forceinline__ int load_now(const int32_t *p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ double term_gh(double g, double h, double w, double lambda, double L2) {
@@ -265,11 +273,10 @@ __global__ void __launch_bounds__(256) k_peer_reduce(PeerReduceArgs a) {
 // staged histogram `sm` of the build node, stores the node's histogram if its children will need it, scans the
 // bins (`_scan_node!`, fit-utils.jl:403-436) and records the best split of this feature.
 template <int MAXCHK, bool OWN, bool OBL, bool K1>
-__device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int f, int slot, double *s_sum, int lane, bool first_owned) {
+__device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int f, uint32_t feat, int slot, double *s_sum, int lane, bool first_owned) {
     // K1: one output with gradient, hessian and weight channels (C = 3), known at compile time: the loops over the
     // outputs and the channel tests fold away
     const int C = K1 ? 3 : a.C, K = K1 ? 1 : a.K, B = a.B, F = a.F;
-    const uint32_t feat = a.js0[f];
     const int m = 1 << (a.level - 1);
     const size_t FCB = (size_t)F * C * B;
     const double *__restrict__ hp = a.hist + (size_t)(n >> 1) * FCB;
@@ -689,11 +696,11 @@ __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_fe
     const int which = a.level > 1 ? (int)(gw & 1) : 0;
     if (a.level > 1) gw >>= 1;
     const int s = (int)(gw / Fown), fi = (int)(gw % Fown);
-    if (s >= a.plan->nbuild) return;
     const int f = fi * a.world + a.rank;
-    const int nb = a.slot_node[s];
+    const int nbuild = load_now(&a.plan->nbuild), nb = load_now(a.slot_node + min(s, a.slots - 1)), feat = load_now(reinterpret_cast<const int32_t *>(a.js0) + f);
+    if (s >= nbuild) return;
     const int n = which ? nb ^ 1 : nb;
-    scan_one<MAXCHK, OWN, OBL, K1>(a, n, which != 0, f, s, s_sum_all[wid], lane, fi == 0);
+    scan_one<MAXCHK, OWN, OBL, K1>(a, n, which != 0, f, (uint32_t)feat, s, s_sum_all[wid], lane, fi == 0);
     if (!OBL && a.ticket) {
         // the warp that scans the node's last feature decides the node: no launch of its own for that
         unsigned last = 0;
@@ -724,9 +731,10 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
     const int which = a.level > 1 ? gw & 1 : 0;
     if (a.level > 1) gw >>= 1;
     const int s = gw / F, f = gw % F;
-    if (s >= a.plan->nbuild) return;
-    const int nb = a.slot_node[s], n = which ? nb ^ 1 : nb, i = n - (1 << (a.level - 1));
-    const uint32_t feat = a.js0[f];
+    const int nbuild = load_now(&a.plan->nbuild), nb = load_now(a.slot_node + min(s, a.slots - 1));
+    const uint32_t feat = (uint32_t)load_now(reinterpret_cast<const int32_t *>(a.js0) + f);
+    if (s >= nbuild) return;
+    const int n = which ? nb ^ 1 : nb, i = n - (1 << (a.level - 1));
     const bool numeric = a.feattypes[feat] != 0, sub = which != 0, keep = n < a.hist_nodes, elide = a.elide_h != 0;
     const int constraint = k == 0 ? a.mono[feat] : 0;
     const int bin0 = lane * CH, b_max = numeric ? B - 1 : B;
@@ -921,10 +929,12 @@ struct PartArgs {
     uint32_t *rows_out;
     const uint8_t *t_split;
     const uint32_t *t_packed;
-    int32_t *seg_start, *seg_cnt, *bslot, *cum, *slot_node;
+    int32_t *seg_start, *seg_cnt, *bslot, *cum, *slot_node, *rbase;
     int32_t *cur_l, *cur_r;     // next free place for left rows (upwards) / past the last free one for right rows (downwards)
-    int32_t *pl_node, *pl_cum;  // sibling pairs of the level (first child's id, the root alone at level 1), running sum of their rows
-    int32_t *pl_node_next, *pl_cum_next;
+    // sibling pairs of the level: {first child's id (the root alone at level 1), rows of the pairs before, rows up to the second
+    // child, position -> place in the row list}; the entry after the last one holds the sum of all rows
+    const int4 *pl;
+    int4 *pl_next;
     uint8_t *kind;
     LevelPlan *plan;
     uint32_t *done;             // CTAs that have finished; the last one plans the next level
@@ -983,14 +993,14 @@ __device__ __forceinline__ void plan_level(const PartArgs &a, int *sm) {
             a.bslot[n << 1] = slot; a.bslot[(n << 1) + 1] = slot;
             a.slot_node[slot] = build_child;
             a.cum[slot] = cpre;
-            a.pl_node_next[slot] = n << 1;
-            a.pl_cum_next[slot] = apre;
+            a.rbase[slot] = s0 - cpre + (build_child & 1 ? nl : 0);
+            a.pl_next[slot] = make_int4(n << 1, apre, apre + nl, s0 - apre);
         }
         carry_slot += tot_s; carry_rows += tot_r; carry_all += tot_a;
     }
     if (threadIdx.x == 0 && scan_children) {
         a.cum[carry_slot] = carry_rows;
-        a.pl_cum_next[carry_slot] = carry_all;
+        a.pl_next[carry_slot] = make_int4(0, carry_all, 0, 0);
         a.plan[a.level + 1].nbuild = carry_slot;
         a.plan[a.level + 1].npl = carry_slot;
         a.plan[a.level + 1].total = carry_all;
@@ -1023,11 +1033,11 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
     // node of position p of the level's row order, its bounds [n0, n1)
     auto locate = [&](int p, int &node, int &n0, int &n1, int &off) {
         int l = 0, r = npl - 1; // largest pair with pl_cum <= p
-        while (l < r) { const int mid = (l + r + 1) >> 1; if (a.pl_cum[mid] <= p) l = mid; else r = mid - 1; }
-        const int c0 = a.pl_cum[l], head = a.pl_node[l], cl = a.seg_cnt[head];
-        off = a.seg_start[head] - c0; // position -> place in the row list (the pair's segments are adjacent)
-        if (p < c0 + cl) { node = head; n0 = c0; n1 = c0 + cl; }
-        else { node = head + 1; n0 = c0 + cl; n1 = a.pl_cum[l + 1]; }
+        while (l < r) { const int mid = (l + r + 1) >> 1; if (a.pl[mid].y <= p) l = mid; else r = mid - 1; }
+        const int4 pr = a.pl[l];
+        off = pr.w; // the pair's segments are adjacent
+        if (p < pr.z) { node = pr.x; n0 = pr.y; n1 = pr.z; }
+        else { node = pr.x + 1; n0 = pr.z; n1 = a.pl[l + 1].y; }
     };
     const int first = (int)((long long)nchunks * b / G), last = (int)((long long)nchunks * (b + 1) / G);
     int node = 0, n0 = 0, n1 = 0, off = 0;
@@ -1149,10 +1159,9 @@ PartArgs make_part_args(evb_handle *h, int level) {
     a.xC = h->xC; a.n = h->n; a.rows_in = h->rows[(level - 1) & 1]; a.rows_out = h->rows[level & 1];
     a.t_split = h->t_split; a.t_packed = h->t_packed;
     a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt;
-    a.bslot = h->bslot; a.cum = h->cum; a.slot_node = h->slot_node; a.kind = h->kind; a.cur_l = h->cur_l; a.cur_r = h->cur_r;
+    a.bslot = h->bslot; a.cum = h->cum; a.slot_node = h->slot_node; a.rbase = h->rbase; a.kind = h->kind; a.cur_l = h->cur_l; a.cur_r = h->cur_r;
     const size_t np = (size_t)h->maxslots + 1;
-    int32_t *p0 = h->pl + ((level - 1) & 1 ? 2 * np : 0), *p1 = h->pl + (level & 1 ? 2 * np : 0);
-    a.pl_node = p0; a.pl_cum = p0 + np; a.pl_node_next = p1; a.pl_cum_next = p1 + np;
+    a.pl = h->pl + ((level - 1) & 1 ? np : 0); a.pl_next = h->pl + (level & 1 ? np : 0);
     a.plan = h->plan; a.done = h->ticket; a.level = level; a.D = h->D; // entry 0 of the tickets belongs to no node
     a.nsum = h->nsum; a.C = h->C; a.by_weight = h->world > 1 ? 1 : 0;
     const bool clear = evb_acc_direct(h); // else the conversion to doubles has cleared them
@@ -1169,8 +1178,8 @@ int32_t evb_launch_tree_begin(evb_handle *h, bool quantize, bool all_rows, const
     BeginArgs a;
     a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt; a.bslot = h->bslot; a.t_feat = h->t_feat; a.kind = h->kind; a.t_bin = h->t_bin;
     a.t_split = h->t_split; a.t_gain = h->t_gain; a.t_w = h->t_w; a.t_pred = h->t_pred; a.t_packed = h->t_packed; a.nsum = h->nsum;
-    a.plan = h->plan; a.ticket = h->ticket; a.rows = h->rows[0]; a.cum = h->cum; a.slot_node = h->slot_node;
-    a.pl_node = h->pl; a.pl_cum = h->pl + h->maxslots + 1;
+    a.plan = h->plan; a.ticket = h->ticket; a.rows = h->rows[0]; a.cum = h->cum; a.slot_node = h->slot_node; a.rbase = h->rbase;
+    a.pl = h->pl;
     a.nids = h->nn + 2; a.nn = h->nn; a.K = h->K; a.C = h->C; a.D = h->D; a.all_rows = all_rows ? 1 : 0;
     a.gen_js_host = gen_js_host; a.gen_js = reinterpret_cast<uint32_t *>(h->gen_d); a.ngen_js = EVB_GEN_WORDS + h->F;
     evb_hg_quant_args(h, &a.q);
@@ -1221,7 +1230,7 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
     a.lambda = h->p.lambda; a.L2 = h->p.L2; a.gamma = h->p.gamma; a.min_weight = h->p.min_weight;
     a.fbest_gain = h->fbest_gain; a.fbest_bin = h->fbest_bin; a.fbest_left = h->fbest_left;
     a.obl_gain = h->obl_gain; a.obl_best = h->obl_best;
-    a.plan = h->plan + level; a.slot_node = h->slot_node;
+    a.plan = h->plan + level; a.slot_node = h->slot_node; a.slots = evb_level_slots(level);
     const bool p2p = h->p2p && h->world > 1;
     a.world = p2p ? h->world : 1; a.rank = p2p ? h->rank : 0;
     for (int q = 0; q < EVB_MAX_PEERS; ++q) a.peer_cand[q] = p2p && q < h->world ? h->peer_cand[q] : nullptr;
