@@ -71,7 +71,11 @@ def get_edges(x: np.ndarray, nbins: int, rng: np.random.Generator):
 def sample_rows(nobs: int, nbins: int, rng: np.random.Generator):
     """The rows `get_edges` takes from `rng`, in no particular order (quantiles do not ask for one); None = all."""
     ns = min(nobs, 1000 * nbins)
-    return rng.choice(nobs, size=ns, replace=False, shuffle=False).astype(np.uint32) if ns < nobs else None
+    if ns >= nobs:
+        return None
+    # an unordered draw is the cheaper one, but between these sizes numpy makes it by another method, with other rows
+    shuffle = nobs > 10_000 and nobs // 50 < ns <= nobs // 20
+    return rng.choice(nobs, size=ns, replace=False, shuffle=shuffle).astype(np.uint32)
 
 
 class RawMatrix:

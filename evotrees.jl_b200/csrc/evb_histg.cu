@@ -107,20 +107,27 @@ int32_t evb_hg_configure(evb_handle *h) {
     }
     const size_t part = part_bytes(h->B, planes(g.per, g.cnt, g.pack));
     if (part > SMEM_ONE) { evb_set_error("histogram image does not fit shared memory (nbins=%d)", h->B); return EVB_ERR_LIMIT; }
-    const int W = (h->nfeats + 3) / 4;
-    int nf, tl;
-    split_words(W, nf, tl);
-    const int parts = nparts(nf, tl), fit = (int)(SMEM_ONE / part);
-    g.ngf = (parts + fit - 1) / fit;
+    const int W = (h->nfeats + 3) / 4, fit = (int)(SMEM_ONE / part);
+    auto most_parts = [&](int wper) { // of a CTA when each takes wper words
+        int most = 0, nf, tl;
+        for (int w = 0; w < W; w += wper) { split_words(std::min(wper, W - w), nf, tl); most = std::max(most, nparts(nf, tl)); }
+        return most;
+    };
+    // all words of a row, else as many whole parts as fit; a tail of 5 or 6 words is two parts, then four words at least
+    g.wper = W;
+    if (most_parts(g.wper) > fit) g.wper = (W - 1) & ~7;
+    while (g.wper > 8 && most_parts(g.wper) > fit) g.wper -= 8;
+    if (g.wper < 8 && W >= 8) g.wper = 8;
+    if (g.wper < 1 || most_parts(g.wper) > fit) g.wper = 4;
+    g.ngf = (W + g.wper - 1) / g.wper;
+    g.wper = std::min(g.wper, g.wper <= 4 ? g.wper : ((W + g.ngf - 1) / g.ngf + 7) & ~7); // the same number of CTAs, evenly filled
     // fewer rows below the root than the SMs can share (256 each): a CTA takes one part only, its flush is shorter too (60k x 77:
     // 0.153 -> 0.149 ms per tree; two CTAs of unequal numbers of parts are slower than one)
-    if (h->n / 2 / 256 * g.ngf < h->num_sms) g.ngf = parts;
-    const int per_group = (parts + g.ngf - 1) / g.ngf;
-    g.wper = g.ngf == 1 ? W : per_group * 8;
+    if (h->n / 2 / 256 * g.ngf < h->num_sms && g.wper > 8) g.wper = 8;
+    g.wper = std::min(g.wper, W);
     g.ngf = (W + g.wper - 1) / g.wper;
     g.W = W;
-    int most = 0;
-    for (int y = 0; y < g.ngf; ++y) { split_words(std::min(g.wper, W - y * g.wper), nf, tl); most = std::max(most, nparts(nf, tl)); }
+    const int most = most_parts(g.wper);
     g.smem = most * part;
     g.threads = g.smem <= SMEM_TWO ? 512 : 1024;
     // up to four words a row is cheap: 256 rows are too few for a flush (100k x 10 0.099 -> 0.104 ms per tree)

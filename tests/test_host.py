@@ -197,3 +197,11 @@ def test_class_codes_equal_unique(pkg, n):
         assert codes.dtype == np.uint32 and np.array_equal(codes, inv + 1) and np.array_equal(counts, np.bincount(inv))
     v = rng.normal(5.0, 2.0, n).astype(np.float32)
     assert abs(_std(v) - np.std(v.astype(np.float64), ddof=1)) < 1e-12
+
+
+@pytest.mark.parametrize("nobs,nbins", [(1_500, 2), (9_000, 2), (39_999, 2), (40_000, 2), (60_013, 2), (99_999, 2), (100_000, 2), (2_000_000, 64), (5_000_000, 32)])
+def test_sample_rows_are_the_rows_of_get_edges(pkg, nobs, nbins):
+    from evotrees_b200.binning import sample_rows
+    rows, ns = sample_rows(nobs, nbins, np.random.default_rng(3)), min(nobs, 1000 * nbins)
+    want = np.random.default_rng(3).choice(nobs, size=ns, replace=False) if ns < nobs else None
+    assert (rows is None and want is None) or np.array_equal(np.sort(rows), np.sort(want))

@@ -13,7 +13,9 @@ CASES = [  # loss, classes, rows, features, bins, depth, weights, columns
     ("logloss", 0, 37, 1, 2, 3, False, 1), ("poisson", 0, 2_049, 7, 33, 4, False, 7), ("gamma", 0, 40_007, 33, 128, 4, True, 20),
     ("mse", 0, 30_001, 13, 255, 5, True, 13), ("mse", 0, 9_000, 21, 64, 4, False, 11), ("gaussian_mle", 0, 30_011, 9, 32, 6, False, 9),
     ("gaussian_mle", 0, 5_000, 130, 16, 4, True, 130), ("mlogloss", 3, 10_240, 15, 65, 5, False, 15), ("mlogloss", 5, 3_001, 28, 64, 5, True, 28),
-    ("mlogloss", 8, 4_097, 4, 255, 5, False, 4), ("mlogloss", 9, 4_099, 5, 40, 4, False, 3), ("logloss", 0, 12_000_000, 2, 8, 3, False, 2)]
+    ("mlogloss", 8, 4_097, 4, 255, 5, False, 4), ("mlogloss", 9, 4_099, 5, 40, 4, False, 3), ("logloss", 0, 12_000_000, 2, 8, 3, False, 2),
+    # one or two parts fit shared memory: rows cut into words of 8 and 4, tails of five words
+    ("mse", 0, 90_001, 50, 255, 4, True, 50), ("logloss", 0, 90_003, 18, 255, 4, False, 18), ("poisson", 0, 90_001, 52, 128, 4, False, 52)]
 
 
 @pytest.mark.parametrize("loss,classes,n,F,B,depth,weighted,ncols", CASES)
