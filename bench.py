@@ -366,12 +366,12 @@ def main():
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
             "higher_is_better": False, "scaling": "strong", "vs_baseline": None,
             "dtype": ("f32 gradients, exact 24-bit fixed-point sums (u32 reductions in shared memory, 64-bit accumulators), f64 split scan"
-                      if w["loss"] == "mse" else "f32 gradients, f32 partial sums in shared memory, f64 histograms and split scan"),
+                      if w["loss"] == "mse" else "f32 gradients, exact 31-bit fixed-point sums (u32 reductions in shared memory, 64-bit accumulators), f64 split scan"),
             "data": "synthetic",
             "config": {"workload": args.workload, "rows": rows, "feats": feats, "max_depth": depth, "nbins": nbins, "loss": w["loss"], "tree_type": args.tree_type,
                        "eta": w["eta"], "rowsample": w["rowsample"], "colsample": w["colsample"], "rows_per_gpu": nloc,
                        "l2_policy": "inputs larger than L2 (bins of the shard: %.0f MB)" % (nloc * (feats + 8) / 1e6)},
-            "roofline": {"bound": "hbm", "kernel": "k_histq2" if w["loss"] == "mse" else "k_hist", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "roofline": {"bound": "hbm", "kernel": "k_histq2" if w["loss"] == "mse" and nloc >= 300000 else "k_histg", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None, "traffic": traffic,
                          "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650",
                          "hist_ms_per_launch": hist_ms / max(1, hist_launches), "hist_launches": hist_launches,
