@@ -68,6 +68,16 @@ def _pack(m: EvoTree, ntree_limit: int):
     return nn, feat, cb, sp, lp
 
 
+_TREE_TYPES = tuple(np.dtype(d) for d in (np.int64, np.uint8, np.uint8, np.float32))
+
+
+def _address(a: np.ndarray) -> int:
+    try:
+        return C.addressof(C.c_char.from_buffer(a))      # a third of the time of the array interface: 0.65 and 1.8 us
+    except (TypeError, ValueError):                      # read-only, or empty
+        return a.__array_interface__["data"][0]
+
+
 def _tree_arrays(t: Tree):
     return t.feat, t.cond_bin, t.split, t.pred
 
@@ -85,8 +95,8 @@ class _Packed:
         self.edges, self.feattypes = m.info["edges"], m.info["feattypes"]
         arrays, self.shared = [], True      # shared: the library reads the model's own arrays, not copies
         for t in self.trees:
-            for a, dt in zip(_tree_arrays(t), (np.int64, np.uint8, np.uint8, np.float32)):
-                if a.dtype != dt and not (dt is np.uint8 and a.dtype == bool) or not a.flags.c_contiguous:
+            for a, dt in zip(_tree_arrays(t), _TREE_TYPES):
+                if a.dtype is not dt and a.dtype != dt and not (dt.itemsize == 1 and a.dtype == bool) or not a.flags.c_contiguous:
                     a, self.shared = np.ascontiguousarray(a, dt), False
                 arrays.append(a)
         e, ft = np.asarray(self.edges), np.asarray(self.feattypes)
@@ -97,7 +107,7 @@ class _Packed:
         self.arrays = arrays
         self.keep = (e, ft)
         n = len(self.trees)
-        src = np.array([a.__array_interface__["data"][0] for a in arrays], np.uint64)
+        src = np.array([_address(a) for a in arrays], np.uint64)
         nodes = np.array([a.size for a in arrays[::4]], np.int32)
         self.handle = C.c_void_p()
         _lib.check(_lib.lib().evb_model_create(
