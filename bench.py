@@ -11,7 +11,7 @@ The other configurations of the benchmark list are selectable with --workload.
 Prints one JSON line (rank 0):
   value      device time of K boosting rounds scaled to 200, the training data already resident in HBM
   e2e        wall time of the public call `fit(params, x_train=, y_train=)` for all 200 rounds from an ordinary
-             (pageable) Float32 host matrix: quantile edges on the host, upload + binarize on the device, boosting loop,
+             (pageable) Float32 host matrix: upload, quantile edges and bins on the device, boosting loop,
              every tree read back -- whatever --steps says
   roofline   the histogram kernel: algorithmic bytes / its summed CUDA-event time, against the measured HBM copy peak
   inference  `m(x)` from raw host features (upload, device binarize, all 201 trees, predictions back), rows sharded
@@ -311,7 +311,7 @@ def main():
         h2d = (nloc * feats * 4 + nloc * 4) / ROUNDS_PER_JOB + feats * 4 + (nloc if w["rowsample"] < 1 else 0)
         d2h = nn * (4 + 4 + 4 + 4 * K + 4 + 1 + 1) + 24 * (depth + 2) + 32
         e2e = {"value": e2e_s, "unit": "s", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h), "rounds": ROUNDS_PER_JOB,
-               "call": "fit(params, x_train=, y_train=): edges on the host, raw Float32 features from pageable memory, binarize on the device, "
+               "call": "fit(params, x_train=, y_train=): edges and bins on the device, raw Float32 features from pageable memory, "
                        "all 200 rounds, every tree read back"}
     if model is not None and not args.no_inference:
         # `m(x)` from raw host features, rows sharded over the ranks (no collective): the training shard, or fresh rows
