@@ -1,6 +1,6 @@
 // Histogram accumulation in integers for any loss: `update_hist!` / `_hist!` (src/fit-utils.jl:345-394; GPU counterpart
-// `hist_kernel!`, ext/EvoTreesKernelAbstractionsExt/fit-utils.jl:57-95).  Device code shared by k_histg and by the kernel that
-// grows a whole tree.
+// `hist_kernel!`, ext/EvoTreesKernelAbstractionsExt/fit-utils.jl:57-95).  Device code of k_histg and of the quantisation in
+// k_tree_begin.
 //
 // Numbers.  Every gradient channel of a row is a fixed-point number q = rint(g 2^s), 2^s the power of two that puts the
 // channel's max |g| just below 2^31 (2^29 for weighted least squares).  An image cell holds two 32-bit words per channel, the
