@@ -148,7 +148,7 @@ static void free_handle(evb_handle *h) {
     evb_dev_free(h->hsum);
     if (exported) { evb_dev_free(h->hcomp, true); h->hcomp = nullptr; }
     free_eval(h);
-    void *ptrs[] = {h->xH, h->xE, h->hsum_q, h->hcnt_q, h->qs_cnt, h->qs_prefix, h->qs_rank, h->qs_gamma, h->gradq, h->d_gmax, h->d_qinv, h->cur_l, h->cur_r, h->ticket, h->pl, h->xT, h->xC, h->grad, h->pred, h->y, h->nidx, h->rows[0], h->rows[1], h->mask_d, h->feattypes_d, h->mono_d,
+    void *ptrs[] = {h->xH, h->xE, h->hsum_q, h->hcnt_q, h->hlow_q, h->low, h->d_signs, h->qs_cnt, h->qs_prefix, h->qs_rank, h->qs_gamma, h->gradq, h->d_gmax, h->d_qinv, h->cur_l, h->cur_r, h->ticket, h->pl, h->xT, h->xC, h->grad, h->pred, h->y, h->nidx, h->rows[0], h->rows[1], h->mask_d, h->feattypes_d, h->mono_d,
                     h->gen_d, h->seg_start, h->seg_cnt, h->kind,
                     h->bslot, h->nsum, h->plan /* base of the tree block */, h->cum, h->slot_node, h->scan_tmp, h->hist, h->hcomp, h->fbest_gain, h->fbest_bin, h->fbest_left, h->obl_gain, h->obl_best, h->edges_d};
     phase("exchange buffers");
@@ -224,6 +224,8 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     }
     EVB_CUDA(dalloc(&h->d_gmax, (size_t)h->nq));
     EVB_CUDA(dalloc(&h->d_qinv, (size_t)h->nq));
+    EVB_CUDA(dalloc(&h->d_signs, (size_t)h->nq));
+    EVB_CUDA(dalloc(&h->low, (size_t)nids));
     EVB_CUDA(dalloc(&h->pred, (size_t)n * K));
     EVB_CUDA(dalloc(&h->nidx, (size_t)n));
     EVB_CUDA(dalloc(&h->rows[0], (size_t)n));
@@ -281,6 +283,10 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
         EVB_CUDA(dalloc(&h->hcnt_q, acc));
         EVB_CUDA(cudaMemsetAsync(h->hsum_q, 0, acc * h->nq * sizeof(unsigned long long), h->st));
         EVB_CUDA(cudaMemsetAsync(h->hcnt_q, 0, acc * sizeof(uint32_t), h->st));
+        if (!h->hgeo.pack) {
+            EVB_CUDA(dalloc(&h->hlow_q, acc * h->nq));
+            EVB_CUDA(cudaMemsetAsync(h->hlow_q, 0, acc * h->nq * sizeof(unsigned long long), h->st));
+        }
     }
 
     // ---- uploads: x_bin is kept feature-major (as given) for the row partition and transposed on the device to
@@ -508,6 +514,7 @@ static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen,
     if (njs != h->F) { // the histogram kernels always accumulate all features; the scan reads the sampled ones
         EVB_CUDA(cudaStreamSynchronize(h->st));
         h->F = njs;
+        h->gradq_valid = false; // how g is rounded may depend on it
         drop_graphs(h);
     }
     if (update_grads) h->bag_idx = 0;

@@ -13,7 +13,7 @@ struct KArgs {
 };
 
 template <int NQ, bool CNT, bool PACK>
-__device__ __forceinline__ void run(const Args &a, uint32_t *smem) { accumulate<NQ, CNT, PACK>(a, smem, blockIdx.x, gridDim.x); }
+__device__ __forceinline__ void run(const Args &a, uint32_t *smem, uint32_t *queue) { accumulate<NQ, CNT, PACK>(a, smem, queue, blockIdx.x, gridDim.x); }
 
 // grid (row ranges, feature groups, channel groups)
 __global__ void __launch_bounds__(1024, 1) k_histg(KArgs k) {
@@ -23,20 +23,24 @@ __global__ void __launch_bounds__(1024, 1) k_histg(KArgs k) {
     evb_hg_select(k.g, a, blockIdx.y, blockIdx.z);
     const int P = evb_hg_planes(k.g, blockIdx.z), words = nparts(a.nfull, a.tails) * (a.B + 1) * P * 8;
     for (int i = threadIdx.x; i < words; i += blockDim.x) reinterpret_cast<uint4 *>(s_img)[i] = make_uint4(0u, 0u, 0u, 0u);
+    uint32_t *queue = s_img + k.g.queue;
+    if (threadIdx.x == 0) queue[QUEUE] = 0u;
     evb_pdl_wait();
     if ((long long)blockIdx.x * a.min_rows >= max(1ll, (long long)a.plan->R + (long long)a.plan->nbuild * a.pad_rows)) return;
     __syncthreads();
-    EVB_HG_DISPATCH(k.g, blockIdx.z, run, a, s_img)
+    EVB_HG_DISPATCH(k.g, blockIdx.z, run, a, s_img, queue)
 }
 
 // clears the accumulators of the level's build slots (all feature columns, sampled or not)
-__global__ void __launch_bounds__(256) k_hg_clear(unsigned long long *hsum, uint32_t *hcnt, const LevelPlan *plan, size_t per_slot, int nq) {
+__global__ void __launch_bounds__(256) k_hg_clear(unsigned long long *hsum, uint32_t *hcnt, unsigned long long *hlow, const uint32_t *low_any, const LevelPlan *plan, size_t per_slot, int nq) {
     evb_pdl_next();
     evb_pdl_wait();
     const size_t n = (size_t)plan->nbuild * per_slot, ns = n * nq;
+    const bool low = hlow && *low_any;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += (size_t)gridDim.x * blockDim.x) {
         hsum[i] = 0ull;
         if (i < n) hcnt[i] = 0u;
+        if (low) hlow[i] = 0ull;
     }
 }
 
@@ -49,6 +53,9 @@ struct ConvArgs {
     const LevelPlan *plan;
     const uint32_t *js0;
     const double *qinv;
+    const unsigned long long *hlow;
+    const uint32_t *low;
+    double low_unit;
     int B, SC, F, C, K, nq, elide, unit_w;
 };
 __global__ void __launch_bounds__(256) k_hg_to_hcomp(ConvArgs a) {
@@ -57,10 +64,12 @@ __global__ void __launch_bounds__(256) k_hg_to_hcomp(ConvArgs a) {
     if (s >= a.plan->nbuild) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, f = f0 + lane;
     const int col = f < a.F ? (int)a.js0[f] : -1;
+    const bool low = a.hlow && a.low[s];
     for (int c = 0; c < a.C; ++c) {
         const bool is_h = a.elide && c >= a.K && c < 2 * a.K; // h = 2w (src/loss.jl:52)
         const bool is_w = c == a.C - 1 || is_h;
         const int ch = is_w ? a.nq - 1 : c;
+        const double unit = is_w && a.unit_w ? 1.0 : a.qinv[ch];
         const double mul = is_h ? 2.0 : 1.0;
         for (int bin0 = 0; bin0 < a.B; bin0 += 64) {
             for (int bl = w; bl < 64; bl += 8) {
@@ -68,8 +77,11 @@ __global__ void __launch_bounds__(256) k_hg_to_hcomp(ConvArgs a) {
                 double v = 0.0;
                 if (bin < a.B && col >= 0) {
                     const size_t cell = (size_t)s * a.B + bin;
-                    v = is_w && a.unit_w ? (double)a.hcnt[cell * a.SC + col]
-                                         : (double)(long long)a.hsum[(cell * a.nq + ch) * a.SC + col] * a.qinv[ch];
+                    if (is_w && a.unit_w) v = (double)a.hcnt[cell * a.SC + col];
+                    else {
+                        v = (double)(long long)a.hsum[(cell * a.nq + ch) * a.SC + col] * unit;
+                        if (low) v += (double)(long long)a.hlow[(cell * a.nq + ch) * a.SC + col] * (unit * a.low_unit);
+                    }
                 }
                 t[bl][lane] = mul * v;
             }
@@ -83,8 +95,8 @@ __global__ void __launch_bounds__(256) k_hg_to_hcomp(ConvArgs a) {
     }
 }
 
-constexpr size_t SMEM_TWO = 113 * 1024;  // two CTAs per SM: 228 KB less 1 KB per CTA
-constexpr size_t SMEM_ONE = 226 * 1024;
+constexpr size_t SMEM_TWO = 113 * 1024 - QUEUE_BYTES;  // image of one of two CTAs per SM: 228 KB less 1 KB per CTA
+constexpr size_t SMEM_ONE = 227 * 1024 - QUEUE_BYTES;
 
 } // namespace
 
@@ -96,8 +108,6 @@ int32_t evb_hg_configure(evb_handle *h) {
     g.nq = h->nq;
     g.pack = h->p.loss == EVB_MSE && h->K == 1 && h->unit_w;
     g.cnt = h->unit_w && !g.pack;
-    g.qbits = g.pack ? 24 : h->p.loss == EVB_MSE ? 29 : 31;
-    g.TE = g.pack ? 255 : 2047;
     if (g.pack) { g.per = 1; g.ngc = 1; }
     else {
         int per = std::min(g.nq, MAX_NQ);
@@ -128,8 +138,9 @@ int32_t evb_hg_configure(evb_handle *h) {
     g.ngf = (W + g.wper - 1) / g.wper;
     g.W = W;
     const int most = most_parts(g.wper);
-    g.smem = most * part;
-    g.threads = g.smem <= SMEM_TWO ? 512 : 1024;
+    g.queue = (int)(most * part / 4);
+    g.smem = most * part + QUEUE_BYTES;
+    g.threads = most * part <= SMEM_TWO ? 512 : 1024;
     // up to four words a row is cheap: 256 rows are too few for a flush (100k x 10 0.099 -> 0.104 ms per tree)
     g.min_rows = g.wper <= 4 ? 512 : 256;
     EVB_CUDA(cudaFuncSetAttribute(k_histg, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
@@ -137,6 +148,16 @@ int32_t evb_hg_configure(evb_handle *h) {
     EVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_histg, g.threads, g.smem));
     if (occ < 1) { evb_set_error("histogram kernel cannot be resident (smem=%zu)", g.smem); return EVB_ERR_CUDA; }
     g.G = std::max(1, occ * h->num_sms / (g.ngf * g.ngc));
+    // More bits leave fewer rows with something left over, but an image then holds fewer rows: as many as the rows of a CTA at the
+    // root allow without an extra flush, 18 at least (8 160 rows).  ms of histograms per tree with 15, 16, 17, 18, 19: 2M x 28 five
+    // classes 0.649, 0.636, 0.633, 0.638, 0.656 (31 bits without the rest 0.617), 5M x 50 gaussian 2.01, 1.19, 1.120, 1.120, 1.187 (1.057).
+    // The sums of all rows have to fit 63 bits.
+    g.hb = 21;
+    while (g.hb > 18 && (1ll << (31 - g.hb)) - 32 < h->n / g.G + 512) --g.hb;
+    int log_n = 0;
+    while ((1ll << log_n) < h->n) ++log_n;
+    g.hb = std::min(g.hb, (61 - log_n) / 2);
+    g.TE = g.pack ? 255 : (1 << (26 - g.hb)) - 1;
     return EVB_OK;
 }
 
@@ -144,13 +165,16 @@ size_t evb_hg_q_words(const evb_handle *h) { return evb_hg_qoff(h->hgeo, h->n, h
 
 void evb_hg_args(const evb_handle *h, int level, evb_hg::Args *a) {
     a->xT = h->xT; a->q = h->gradq; a->rows = h->rows[(level - 1) & 1]; a->plan = h->plan + level; a->cum = h->cum; a->rbase = h->rbase;
-    a->hsum = h->hsum_q; a->hcnt = h->hcnt_q; a->RS = h->RS; a->B = h->B; a->SC = h->SC; a->nq = h->nq; a->F = h->nfeats;
+    a->hsum = h->hsum_q; a->hcnt = h->hcnt_q; a->hlow = h->hlow_q; a->low = h->low + evb_low_slot(level); a->low_any = h->low + evb_low_any(level);
+    a->hb = h->hgeo.hb; a->RS = h->RS; a->B = h->B; a->SC = h->SC; a->nq = h->nq; a->F = h->nfeats;
     a->TE = h->hgeo.TE; a->min_rows = h->hgeo.min_rows; a->pad_rows = evb_pad_rows(h); a->n = h->n;
 }
 
 void evb_hg_quant_args(const evb_handle *h, evb_hg::QuantArgs *a) {
     a->grad = h->grad; a->q = h->use_q2 ? reinterpret_cast<int32_t *>(h->xE) : h->gradq; a->gmax = h->d_gmax; a->qinv = h->d_qinv; a->n = h->n;
-    a->q2 = h->use_q2 ? 1 : 0; a->g = h->hgeo;
+    a->q2 = h->use_q2 ? 1 : 0; a->g = h->hgeo; a->signs = h->d_signs;
+    // the width that weighted least squares has always had where its fixed-point kernel ran
+    a->bits = h->p.loss == EVB_MSE && h->K == 1 && !h->unit_w && h->B <= 128 && h->F == h->nfeats ? 29 : 0;
 }
 
 int32_t evb_launch_histg(evb_handle *h, int level) {
@@ -169,7 +193,8 @@ int32_t evb_launch_acc_clear(evb_handle *h, int level) {
     const size_t per_slot = (size_t)h->B * h->SC;
     const size_t blocks = std::min<size_t>(((size_t)evb_level_slots(level) * per_slot * h->nq + 255) / 256, (size_t)h->num_sms * 8);
     evb_tic(h, EVB_T_HIST_REDUCE);
-    const cudaError_t e = evb_launch_pdl(h->early, k_hg_clear, dim3((unsigned)blocks), dim3(256), 0, h->st, h->hsum_q, h->hcnt_q, h->plan + level, per_slot, h->nq);
+    const cudaError_t e = evb_launch_pdl(h->early, k_hg_clear, dim3((unsigned)blocks), dim3(256), 0, h->st, h->hsum_q, h->hcnt_q, h->hlow_q, h->low + evb_low_any(level),
+                                         h->plan + level, per_slot, h->nq);
     evb_toc(h, EVB_T_HIST_REDUCE);
     EVB_CUDA(e);
     return EVB_OK;
@@ -179,6 +204,7 @@ int32_t evb_launch_acc_clear(evb_handle *h, int level) {
 int32_t evb_launch_acc_to_hcomp(evb_handle *h, int level) {
     ConvArgs a;
     a.hsum = h->hsum_q; a.hcnt = h->hcnt_q; a.hcomp = h->hcomp; a.plan = h->plan + level; a.js0 = h->js_d; a.qinv = h->d_qinv;
+    a.hlow = h->hlow_q; a.low = h->low + evb_low_slot(level); a.low_unit = evb_hg_low_unit(h);
     a.B = h->B; a.SC = h->SC; a.F = h->F; a.C = h->C; a.K = h->K; a.nq = h->nq; a.elide = h->Ce != h->C; a.unit_w = h->unit_w;
     evb_tic(h, EVB_T_HIST_REDUCE);
     k_hg_to_hcomp<<<dim3(evb_level_slots(level), (h->F + 31) / 32), 256, 0, h->st>>>(a);

@@ -65,7 +65,8 @@ struct HGeom {
     int nq, per, ngc;   // channels; channels per CTA; channel groups (grid.z)
     int W, wper, ngf;   // words of a row; words per CTA; feature groups (grid.y)
     int pack, cnt;      // packed words of unit-weight least squares; a plane of row counts in channel group 0
-    int qbits, TE, min_rows, threads, G;
+    int hb, TE, min_rows, threads, G;
+    int queue;          // 32-bit words of shared memory before the row queue
     size_t smem;
 };
 
@@ -142,10 +143,13 @@ struct evb_handle {
     HGeom hgeo;
     int32_t *gradq;       // words of all rows, channel group by channel group
     unsigned *d_gmax;     // [nq] bits of max |g| over the rows, filled by the gradient kernels
-    double *d_qinv;       // [nq] 2^-s of every channel
+    double *d_qinv;       // [nq] unit of every channel's sums
+    unsigned *d_signs;    // [nq] signs of the infinities a channel has had (QuantArgs::signs)
     int SC;               // feature columns per bin of the accumulators
     unsigned long long *hsum_q;   // [maxslots][B][nq][SC] sums of q per build slot
     uint32_t *hcnt_q;             // [maxslots][B][SC] row counts
+    unsigned long long *hlow_q;   // like hsum_q: what the words of a row leave (null: packed words leave nothing)
+    uint32_t *low;                // [nn+2] build slots of a level that have something in hlow_q (evb_low_slot, evb_low_any)
 
     // register-direct variant (mse, one target, unit weights, many rows): rows as 16-byte chunks + {q, tail bins} per row
     bool use_q2;
@@ -249,6 +253,11 @@ static inline int evb_pad_rows(const evb_handle *h) {
 #define EVB_MULTI_K 8
 static inline bool evb_scan_multi(const evb_handle *h) { return h->K >= 2 && h->K <= EVB_MULTI_K && h->C == 2 * h->K + 1 && h->p.loss < EVB_MAE && h->p.tree_type != 1; }
 static inline bool evb_acc_direct(const evb_handle *h) { return h->world == 1; }
+// evb_handle::low, a stretch of 2^(level-1) words per level: its build slots (at most half of them below the root), and in its last
+// word whether any slot has something (the root's only slot says so itself)
+static inline size_t evb_low_slot(int level) { return (size_t)1 << (level - 1); }
+static inline size_t evb_low_any(int level) { return ((size_t)1 << level) - 1; }
+static inline double evb_hg_low_unit(const evb_handle *h) { return 1.0 / (double)(1ull << (2 * h->hgeo.hb + 2)); } // units of hlow_q in those of hsum_q
 // evb_histq2.cu
 bool evb_q2_wanted(const evb_handle *h);
 int32_t evb_q2_configure(evb_handle *h);

@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float gm = 0.0f, hm = 0.0f; // largest |g|, |h| of this thread's rows
+    unsigned gm = 0u, hm = 0u; // bits of the largest |g|, |h| of this thread's rows (a NaN is larger than all numbers)
     int buf = 0;
     stage(blockIdx.x, 0);
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, buf ^= 1) {
@@ -495,14 +495,14 @@ __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
                 const float w = MSE1 || f.unit_w ? 1.0f : rec[nq - 1];
                 grad_row(loss, 1, MSE1 ? true : f.elided != 0, &pv, f.y, 1, i, w, g, f.alpha);
                 rec[0] = g[0];
-                gm = fmaxf(gm, fabsf(g[0]));
-                if (!MSE1 && f.ng > 1) { rec[1] = g[1]; hm = fmaxf(hm, fabsf(g[1])); }
+                gm = max(gm, __float_as_uint(fabsf(g[0])));
+                if (!MSE1 && f.ng > 1) { rec[1] = g[1]; hm = max(hm, __float_as_uint(fabsf(g[1]))); }
             }
         }
         __syncthreads(); // everybody is done with this buffer: the next iteration refills it
     }
     if (f.compute_grads) {
-        const float m2[2] = {gm, hm};
+        const float m2[2] = {__uint_as_float(gm), __uint_as_float(hm)};
         block_absmax(m2, f.ng, f.gmax); // K == 1: one or two channels
     }
 }

@@ -62,7 +62,7 @@ struct BeginArgs {
     uint32_t *t_packed;
     double *nsum;
     LevelPlan *plan;
-    uint32_t *ticket, *rows;
+    uint32_t *ticket, *rows, *low;
     const uint32_t *gen_js_host; // pinned: generator state and column sample of this tree
     uint32_t *gen_js;
     int ngen_js;
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(256) k_tree_begin(BeginArgs a) {
     if (a.all_rows && i < a.q.n) a.rows[i] = (uint32_t)i;
     if (i < a.nids) {
         const bool root = i == 1 && a.all_rows;
-        a.seg_start[i] = 0; a.seg_cnt[i] = root ? (int32_t)a.q.n : 0; a.kind[i] = root ? EVB_KIND_BUILD : EVB_KIND_NONE; a.bslot[i] = 0; a.ticket[i] = 0u;
+        a.seg_start[i] = 0; a.seg_cnt[i] = root ? (int32_t)a.q.n : 0; a.kind[i] = root ? EVB_KIND_BUILD : EVB_KIND_NONE; a.bslot[i] = 0; a.ticket[i] = 0u; a.low[i] = 0u;
         for (int c = 0; c < a.C; ++c) a.nsum[(size_t)i * a.C + c] = 0.0;
         if (root) {
             a.cum[0] = 0; a.cum[1] = (int32_t)a.q.n; a.slot_node[0] = 1; a.rbase[0] = 0;
@@ -131,6 +131,9 @@ struct ScanArgs {
     const unsigned long long *qsum;
     const uint32_t *qcnt;
     const double *qinv;
+    const unsigned long long *qlow; // like qsum, low_unit times as fine: of the build slots in `low`
+    const uint32_t *low;
+    double low_unit;
     int SC, nq, unit_w;
     // non-null: the last feature of a node to be scanned decides the node (one GPU, binary trees)
     uint32_t *ticket;
@@ -236,6 +239,18 @@ __device__ __forceinline__ void chan_load(const ScanArgs &a, const Chan &ch, int
 __device__ __forceinline__ double chan_value(const ScanArgs &a, const Chan &ch, long long raw) {
     return a.qsum ? (double)raw * ch.mul : __longlong_as_double(raw);
 }
+// the build slot has sums below those of qsum; few have, so what they hold is fetched where it is added and not ahead
+__device__ __forceinline__ bool slot_low(const ScanArgs &a, int slot) { return a.qlow && load_now(reinterpret_cast<const int32_t *>(a.low) + slot) != 0; }
+template <int N>
+__device__ __forceinline__ void chan_add_low(const ScanArgs &a, const Chan &ch, int slot, uint32_t feat, int b0, int stride, double (&v)[N]) {
+    if (ch.cnt) return;
+    const unsigned long long *p = a.qlow + ((size_t)slot * a.B * a.nq + ch.idx) * a.SC + feat;
+    long long raw[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) raw[j] = (long long)__ldg(p + (size_t)min(b0 + j * stride, a.B - 1) * a.nq * a.SC);
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] += (double)raw[j] * (ch.mul * a.low_unit);
+}
 
 // Sharded with peer access: sums the ranks' freshly built histograms for the feature slots this rank owns, by
 // loads from the peers' memory past the caches, in rank order (so the result does not depend on timing).  One CTA
@@ -272,8 +287,8 @@ __global__ void __launch_bounds__(256) k_peer_reduce(PeerReduceArgs a) {
 // Scan of one (node, feature): applies the sibling subtraction (`subtract_hist!`, fit-utils.jl:321-332) to the
 // staged histogram `sm` of the build node, stores the node's histogram if its children will need it, scans the
 // bins (`_scan_node!`, fit-utils.jl:403-436) and records the best split of this feature.
-template <int MAXCHK, bool OWN, bool OBL, bool K1>
-__device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int f, uint32_t feat, int slot, double *s_sum, int lane, bool first_owned) {
+template <int MAXCHK, bool OWN, bool OBL, bool K1, bool LOW>
+__device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int f, uint32_t feat, int slot, bool low, double *s_sum, int lane, bool first_owned) {
     // K1: one output with gradient, hessian and weight channels (C = 3), known at compile time: the loops over the
     // outputs and the channel tests fold away
     const int C = K1 ? 3 : a.C, K = K1 ? 1 : a.K, B = a.B, F = a.F;
@@ -289,9 +304,12 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
             const Chan ch = chan_of(a, c, K, C);
             long long raw[MAXCHK];
             chan_load<MAXCHK>(a, ch, slot, f, feat, c, lane, 32, C, raw);
-            double v = 0.0;
+            double b[MAXCHK], v = 0.0;
 #pragma unroll
-            for (int j = 0; j < MAXCHK; ++j) if (lane + 32 * j < B) v += chan_value(a, ch, raw[j]);
+            for (int j = 0; j < MAXCHK; ++j) b[j] = chan_value(a, ch, raw[j]);
+            if (LOW && low) chan_add_low<MAXCHK>(a, ch, slot, feat, lane, 32, b);
+#pragma unroll
+            for (int j = 0; j < MAXCHK; ++j) if (lane + 32 * j < B) v += b[j];
             v = warp_sum(v);
             if (lane == 0) { s_sum[c] = v; if (first_owned) a.nsum[(size_t)C + c] = v; }
         }
@@ -329,9 +347,11 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     };
     auto take = [&](int c, const Raw &r, double (&v)[CH]) {
 #pragma unroll
+        for (int j = 0; j < CH; ++j) v[j] = chan_value(a, r.ch, r.b[j]);
+        if (LOW && low) chan_add_low<CH>(a, r.ch, slot, feat, bin0, 1, v);
+#pragma unroll
         for (int j = 0; j < CH; ++j) {
             const int b = bin0 + j;
-            v[j] = chan_value(a, r.ch, r.b[j]);
             if (sub) v[j] = r.p[j] - v[j];
             if (b >= B) v[j] = 0.0;
             if (keep && b < B) hn[fo + (size_t)c * B + b] = v[j];
@@ -528,6 +548,7 @@ __device__ __forceinline__ void node_select(const ScanArgs &a, int n, double *s_
     const int Fown = (F - a.rank + a.world - 1) / a.world;
     const int slot_n = a.bslot[n];
     const bool sub = a.kind[n] == EVB_KIND_SUB;
+    const bool low = a.world == 1 && slot_low(a, slot_n);
     double fg[4];
     int fb[4];
 #pragma unroll
@@ -600,11 +621,17 @@ __device__ __forceinline__ void node_select(const ScanArgs &a, int n, double *s_
 #pragma unroll
             for (int u = 0; u < NC; ++u) {
                 v[u] = 0.0;
+                double built[MAXCHK];
+                if (a.world == 1) {
+#pragma unroll
+                    for (int j = 0; j < MAXCHK; ++j) built[j] = chan_value(a, ch[u], rb[u][j]);
+                    if (low) chan_add_low<MAXCHK>(a, ch[u], slot_n, feat, lane, 32, built);
+                }
 #pragma unroll
                 for (int j = 0; j < MAXCHK; ++j) {
                     const int b = lane + 32 * j;
                     double e = rp[u][j];
-                    if (a.world == 1) { e = chan_value(a, ch[u], rb[u][j]); if (sub) e = rp[u][j] - e; }
+                    if (a.world == 1) e = sub ? rp[u][j] - built[j] : built[j];
                     if (b < B && (numeric ? b <= bb : b == bb)) v[u] += e;
                 }
             }
@@ -680,8 +707,8 @@ __global__ void __launch_bounds__(256) k_scan_node(ScanArgs a) {
 // build slot: the build node reads the slot's histogram, its sibling subtracts it from the parent's.  Warps are
 // independent, so even the root level (one node) spreads over many SMs.
 // OWN: the loss brings its own split gain (mae, credibility); OBL: oblivious trees, the gain of every candidate is
-// stored as well.  The default instance carries neither code.
-template <int MAXCHK, bool OWN, bool OBL, bool K1>
+// stored as well; LOW: histograms may have a second set of sums (ScanArgs::qlow).  The default instance carries none of that code.
+template <int MAXCHK, bool OWN, bool OBL, bool K1, bool LOW>
 __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_feat(ScanArgs a) {
     constexpr int NCH = K1 ? 3 : 72;
     __shared__ double s_sum_all[8][NCH], s_left_all[8][NCH], s_right_all[8][NCH];
@@ -698,9 +725,10 @@ __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_fe
     const int s = (int)(gw / Fown), fi = (int)(gw % Fown);
     const int f = fi * a.world + a.rank;
     const int nbuild = load_now(&a.plan->nbuild), nb = load_now(a.slot_node + min(s, a.slots - 1)), feat = load_now(reinterpret_cast<const int32_t *>(a.js0) + f);
+    const bool low = LOW && slot_low(a, min(s, a.slots - 1));
     if (s >= nbuild) return;
     const int n = which ? nb ^ 1 : nb;
-    scan_one<MAXCHK, OWN, OBL, K1>(a, n, which != 0, f, (uint32_t)feat, s, s_sum_all[wid], lane, fi == 0);
+    scan_one<MAXCHK, OWN, OBL, K1, LOW>(a, n, which != 0, f, (uint32_t)feat, s, low, s_sum_all[wid], lane, fi == 0);
     if (!OBL && a.ticket) {
         // the warp that scans the node's last feature decides the node: no launch of its own for that
         unsigned last = 0;
@@ -733,6 +761,7 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
     const int s = gw / F, f = gw % F;
     const int nbuild = load_now(&a.plan->nbuild), nb = load_now(a.slot_node + min(s, a.slots - 1));
     const uint32_t feat = (uint32_t)load_now(reinterpret_cast<const int32_t *>(a.js0) + f);
+    const bool low = slot_low(a, min(s, a.slots - 1));
     if (s >= nbuild) return;
     const int n = which ? nb ^ 1 : nb, i = n - (1 << (a.level - 1));
     const bool numeric = a.feattypes[feat] != 0, sub = which != 0, keep = n < a.hist_nodes, elide = a.elide_h != 0;
@@ -761,12 +790,21 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
         if (n > 1) { sg = a.nsum[(size_t)n * C + k]; sh = a.nsum[(size_t)n * C + K + k]; w_p = a.nsum[(size_t)n * C + C - 1]; }
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
-            const int b = bin0 + j;
             wl[j] = chan_value(a, cw, rw[j]);
             gl[j] = chan_value(a, cg, rg[j]);
+            hl[j] = elide ? 0.0 : chan_value(a, chs, rh[j]);
+        }
+        if (low) {
+            chan_add_low<CH>(a, cw, s, feat, bin0, 1, wl);
+            chan_add_low<CH>(a, cg, s, feat, bin0, 1, gl);
+            if (!elide) chan_add_low<CH>(a, chs, s, feat, bin0, 1, hl);
+        }
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+            const int b = bin0 + j;
             if (sub) { wl[j] = pw[j] - wl[j]; gl[j] = pg[j] - gl[j]; }
             if (elide) hl[j] = 2.0 * wl[j];
-            else { hl[j] = chan_value(a, chs, rh[j]); if (sub) hl[j] = ph[j] - hl[j]; }
+            else if (sub) hl[j] = ph[j] - hl[j];
             if (b >= B) { wl[j] = 0.0; gl[j] = 0.0; hl[j] = 0.0; }
             else if (keep) {
                 hn[(size_t)k * B + b] = gl[j];
@@ -940,6 +978,8 @@ struct PartArgs {
     uint32_t *done;             // CTAs that have finished; the last one plans the next level
     const double *nsum; // node sums [id][C]; channel C-1 is the sum of weights
     unsigned long long *hsum;   // accumulators of the level's build slots, cleared here (the scan has read them)
+    unsigned long long *hlow;
+    const uint32_t *low_any;
     uint32_t *hcnt;
     size_t acc_sums, acc_cnts;  // words per build slot
     int C, by_weight;   // by_weight: sharded run, pick the build child by weight sum instead of row count
@@ -1133,11 +1173,12 @@ __global__ void __launch_bounds__(EVB_PART_THREADS, PART_CTAS) k_partition(PartA
     __shared__ int s_pref[EVB_PART_CHUNK / 32], s_misc[34];
     evb_pdl_next();
     evb_pdl_wait();
-    const int npl = a.plan[a.level].npl, total = a.plan[a.level].total;
+    const int npl = a.plan[a.level].npl, total = a.plan[a.level].total, low = a.hlow ? load_now(reinterpret_cast<const int32_t *>(a.low_any)) : 0;
     {
         const size_t nb = (size_t)a.plan[a.level].nbuild, ns = nb * a.acc_sums, nc = nb * a.acc_cnts;
         const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
         for (size_t i = i0; i < ns; i += st) a.hsum[i] = 0ull;
+        if (low) for (size_t i = i0; i < ns; i += st) a.hlow[i] = 0ull;
         for (size_t i = i0; i < nc; i += st) a.hcnt[i] = 0u;
     }
     // few rows: small chunks, so that they spread over the GPU (their chain of dependent loads is what takes the time)
@@ -1165,7 +1206,7 @@ PartArgs make_part_args(evb_handle *h, int level) {
     a.plan = h->plan; a.done = h->ticket; a.level = level; a.D = h->D; // entry 0 of the tickets belongs to no node
     a.nsum = h->nsum; a.C = h->C; a.by_weight = h->world > 1 ? 1 : 0;
     const bool clear = evb_acc_direct(h); // else the conversion to doubles has cleared them
-    a.hsum = h->hsum_q; a.hcnt = h->hcnt_q;
+    a.hsum = h->hsum_q; a.hcnt = h->hcnt_q; a.hlow = h->hlow_q; a.low_any = h->low + evb_low_any(level);
     a.acc_sums = clear ? (size_t)h->B * h->SC * h->nq : 0; a.acc_cnts = clear ? (size_t)h->B * h->SC : 0;
     return a;
 }
@@ -1178,7 +1219,7 @@ int32_t evb_launch_tree_begin(evb_handle *h, bool quantize, bool all_rows, const
     BeginArgs a;
     a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt; a.bslot = h->bslot; a.t_feat = h->t_feat; a.kind = h->kind; a.t_bin = h->t_bin;
     a.t_split = h->t_split; a.t_gain = h->t_gain; a.t_w = h->t_w; a.t_pred = h->t_pred; a.t_packed = h->t_packed; a.nsum = h->nsum;
-    a.plan = h->plan; a.ticket = h->ticket; a.rows = h->rows[0]; a.cum = h->cum; a.slot_node = h->slot_node; a.rbase = h->rbase;
+    a.plan = h->plan; a.ticket = h->ticket; a.low = h->low; a.rows = h->rows[0]; a.cum = h->cum; a.slot_node = h->slot_node; a.rbase = h->rbase;
     a.pl = h->pl;
     a.nids = h->nn + 2; a.nn = h->nn; a.K = h->K; a.C = h->C; a.D = h->D; a.all_rows = all_rows ? 1 : 0;
     a.gen_js_host = gen_js_host; a.gen_js = reinterpret_cast<uint32_t *>(h->gen_d); a.ngen_js = EVB_GEN_WORDS + h->F;
@@ -1223,7 +1264,9 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
     a.loss = h->p.loss; a.neb = -h->p.eta / (double)h->p.bagging_size;
     a.elide_h = h->Ce != h->C ? 1 : 0;
     const bool direct = evb_acc_direct(h);
-    a.qsum = direct ? h->hsum_q : nullptr; a.qcnt = direct ? h->hcnt_q : nullptr; a.qinv = h->d_qinv; a.SC = h->SC; a.nq = h->nq; a.unit_w = h->unit_w ? 1 : 0;
+    a.qsum = direct ? h->hsum_q : nullptr; a.qcnt = direct ? h->hcnt_q : nullptr; a.qinv = h->d_qinv; a.SC = h->SC;
+    a.qlow = direct ? h->hlow_q : nullptr; a.low = h->low + evb_low_slot(level); a.low_unit = evb_hg_low_unit(h);
+    a.nq = h->nq; a.unit_w = h->unit_w ? 1 : 0;
     const bool fused = h->world == 1 && !h->obl_gain;
     a.gmax = h->d_gmax; a.ng = h->ng;
     a.ticket = fused ? h->ticket : nullptr; a.cur_l = h->cur_l; a.cur_r = h->cur_r; a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt;
@@ -1262,11 +1305,12 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
         const bool own = h->p.loss >= EVB_MAE;
         const bool obl = h->obl_gain != nullptr;
 #define EVB_SCAN(M) do { \
-            if (own && obl) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, true, true, false>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else if (own) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, true, false, false>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else if (obl) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, true, false>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else if (h->K == 1 && h->C == 3) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, false>, dim3(grid), dim3(256), 0, h->st, a)); } while (0)
+            if (own && obl) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, true, true, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (own) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, true, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (obl) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, true, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (h->K == 1 && h->C == 3 && !a.qlow) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, true, false>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (h->K == 1 && h->C == 3) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, true, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); } while (0)
         if (h->B <= 32) EVB_SCAN(1); else if (h->B <= 64) EVB_SCAN(2); else if (h->B <= 128) EVB_SCAN(4); else EVB_SCAN(8);
 #undef EVB_SCAN
     }
