@@ -26,6 +26,11 @@ __device__ __forceinline__ double warp_sum(double v) {
     for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
     return v;
 }
+__device__ __forceinline__ long long warp_sum(long long v) {
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
+    return v;
+}
 __device__ __forceinline__ int warp_incl_scan_i(int v, int lane) {
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -252,6 +257,24 @@ __device__ __forceinline__ void chan_add_low(const ScanArgs &a, const Chan &ch, 
     for (int j = 0; j < N; ++j) v[j] += (double)raw[j] * (ch.mul * a.low_unit);
 }
 
+// Root sum of a channel from the whole numbers of the bins of any feature, raw[j]: bin b0 + j * stride (every sampled row has
+// exactly one bin; the reference sums the gradients of the sampled rows directly, src/fit.jl:66).  The total of the whole numbers is
+// the same for every feature and converted once, so that all features' scans and the decision work with the same parent.
+template <int N>
+__device__ __forceinline__ double chan_total(const ScanArgs &a, const Chan &ch, int slot, uint32_t feat, bool low, int b0, int stride, const long long (&raw)[N]) {
+    long long t = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) if (b0 + j * stride < a.B) t += raw[j];
+    double v = (double)warp_sum(t) * ch.mul;
+    if (low && !ch.cnt) {
+        const unsigned long long *p = a.qlow + ((size_t)slot * a.B * a.nq + ch.idx) * a.SC + feat;
+        t = 0;
+        for (int j = 0; j < N; ++j) if (b0 + j * stride < a.B) t += (long long)__ldg(p + (size_t)(b0 + j * stride) * a.nq * a.SC);
+        v += (double)warp_sum(t) * (ch.mul * a.low_unit);
+    }
+    return v;
+}
+
 // Sharded with peer access: sums the ranks' freshly built histograms for the feature slots this rank owns, by
 // loads from the peers' memory past the caches, in rank order (so the result does not depend on timing).  One CTA
 // per (build slot, owned feature); at the root level feature slot 0 is summed on every rank (it gives the root sums).
@@ -298,19 +321,17 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     const bool keep = n < a.hist_nodes;
     double *__restrict__ hn = a.hist + (size_t)n * FCB;
     if (n == 1) {
-        // root sums = sum over the bins of feature slot 0 (every sampled row has exactly one bin there);
-        // the reference sums the gradients of the sampled rows directly (src/fit.jl:66)
         for (int c = 0; c < C; ++c) {
             const Chan ch = chan_of(a, c, K, C);
             long long raw[MAXCHK];
             chan_load<MAXCHK>(a, ch, slot, f, feat, c, lane, 32, C, raw);
-            double b[MAXCHK], v = 0.0;
+            double v = 0.0;
+            if (a.qsum) v = chan_total<MAXCHK>(a, ch, slot, feat, LOW && low, lane, 32, raw);
+            else { // sharded: the bins of feature slot 0, in doubles
 #pragma unroll
-            for (int j = 0; j < MAXCHK; ++j) b[j] = chan_value(a, ch, raw[j]);
-            if (LOW && low) chan_add_low<MAXCHK>(a, ch, slot, feat, lane, 32, b);
-#pragma unroll
-            for (int j = 0; j < MAXCHK; ++j) if (lane + 32 * j < B) v += b[j];
-            v = warp_sum(v);
+                for (int j = 0; j < MAXCHK; ++j) if (lane + 32 * j < B) v += __longlong_as_double(raw[j]);
+                v = warp_sum(v);
+            }
             if (lane == 0) { s_sum[c] = v; if (first_owned) a.nsum[(size_t)C + c] = v; }
         }
     } else {
@@ -788,6 +809,11 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
             ph[j] = sub && !elide ? __ldg(hp + (size_t)(K + k) * B + b) : 0.0;
         }
         if (n > 1) { sg = a.nsum[(size_t)n * C + k]; sh = a.nsum[(size_t)n * C + K + k]; w_p = a.nsum[(size_t)n * C + C - 1]; }
+        else {
+            sg = chan_total<CH>(a, cg, s, feat, low, bin0, 1, rg);
+            w_p = chan_total<CH>(a, cw, s, feat, low, bin0, 1, rw);
+            sh = elide ? 2.0 * w_p : chan_total<CH>(a, chs, s, feat, low, bin0, 1, rh);
+        }
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
             wl[j] = chan_value(a, cw, rw[j]);
@@ -813,13 +839,7 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
             }
         }
     }
-    if (n == 1) { // root sums over the bins of this feature (every sampled row has exactly one); feature slot 0 records them
-        sg = 0.0; sh = 0.0; w_p = 0.0;
-#pragma unroll
-        for (int j = 0; j < CH; ++j) { sg += gl[j]; sh += hl[j]; w_p += wl[j]; }
-        sg = warp_sum(sg); sh = warp_sum(sh); w_p = warp_sum(w_p);
-        if (f == 0 && lane == 0) { a.nsum[C + k] = sg; a.nsum[C + K + k] = sh; if (k == 0) a.nsum[2 * C - 1] = w_p; }
-    }
+    if (n == 1 && f == 0 && lane == 0) { a.nsum[C + k] = sg; a.nsum[C + K + k] = sh; if (k == 0) a.nsum[2 * C - 1] = w_p; }
     if (lane == 0) {
         s_sum[k] = sg; s_sum[K + k] = sh;
         if (k == 0) s_sum[C - 1] = w_p;
