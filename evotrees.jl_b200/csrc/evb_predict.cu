@@ -9,7 +9,9 @@
 #include <atomic>
 #include <mutex>
 #include <new>
+#include <vector>
 #include <string.h>
+#include <sys/mman.h>
 #include <stdlib.h>
 
 namespace {
@@ -319,10 +321,14 @@ struct evb_model {
     // works, so a tree that was changed in place since is noticed.
     std::vector<const void *> src;    // [ntrees][4]: feat, cond_bin, split, leaf_pred
     std::vector<int32_t> nodes;       // nodes of every tree
-    std::vector<size_t> at;           // offset of every tree's copy in `snap`
-    std::vector<unsigned char> snap;
+    std::vector<size_t> at;           // offset of every tree's copy in `snap`, then its size
+    unsigned char *snap = nullptr;
     const void *src_edges = nullptr, *src_ft = nullptr;
     std::vector<unsigned char> snap_edges, snap_ft;
+    evb_model() = default;
+    evb_model(const evb_model &) = delete;
+    evb_model &operator=(const evb_model &) = delete;
+    ~evb_model() { free(snap); }
 };
 
 namespace {
@@ -336,7 +342,7 @@ void verify_range(void *c, size_t b, size_t e) {
         size_t o = j.m->at[t];
         for (int q = 0; q < 4; ++q) {
             const size_t n = tree_bytes(j.m->nodes[t], j.m->K, q);
-            if (memcmp(j.m->src[t * 4 + q], j.m->snap.data() + o, n) != 0) { j.bad.store(1); return; }
+            if (memcmp(j.m->src[t * 4 + q], j.m->snap + o, n) != 0) { j.bad.store(1); return; }
             o += n;
         }
     }
@@ -344,14 +350,75 @@ void verify_range(void *c, size_t b, size_t e) {
 // the sources still hold what was packed
 bool model_current(const evb_model *m) {
     VerifyJob j{m, {0}};
-    const size_t per = m->ntrees > 0 ? m->snap.size() / m->ntrees : 0;
+    const size_t per = m->ntrees > 0 ? m->at[m->ntrees] / m->ntrees : 0;
     const size_t slice = per ? std::max<size_t>(1, ((size_t)256 << 10) / per) : 1;
     evb_parallel(verify_range, &j, (size_t)m->ntrees, slice);
     return j.bad.load() == 0 && (m->snap_edges.empty() || memcmp(m->src_edges, m->snap_edges.data(), m->snap_edges.size()) == 0) &&
            (m->snap_ft.empty() || memcmp(m->src_ft, m->snap_ft.data(), m->snap_ft.size()) == 0);
 }
 
+// Large blocks of host memory that are about to be written by several threads: huge pages where the system has them (a page fault
+// every 4 KB costs more than the copy).  Freed with free().
+unsigned char *big_alloc(size_t bytes) {
+    constexpr size_t HUGE_PAGE = (size_t)2 << 20;
+    if (bytes < 2 * HUGE_PAGE) return static_cast<unsigned char *>(malloc(bytes ? bytes : 1));
+    void *p = nullptr;
+    if (posix_memalign(&p, HUGE_PAGE, bytes) != 0) return nullptr;
+    madvise(p, bytes, MADV_HUGEPAGE);
+    return static_cast<unsigned char *>(p);
+}
+
+// Trees -> packed trees.  With a snapshot a tree is copied there first and packed from the copy, so that the two agree.
+struct PackJob {
+    const evb_model *m;
+    const void *const *src;
+    const int32_t *nodes;
+    const uint8_t *feattypes;
+    unsigned char *snap;
+    std::atomic<long long> bad; // tree and node of a test that cannot be: (tree << 32 | node) + 1
+};
+void pack_trees(void *ctx, char *dst, size_t first, size_t count) {
+    PackJob &j = *static_cast<PackJob *>(ctx);
+    const evb_model &m = *j.m;
+    uint32_t *tr = reinterpret_cast<uint32_t *>(dst);
+    for (size_t t = first; t < first + count; ++t, tr += m.tw) {
+        const void *part[4];
+        const int nn = j.nodes[t];
+        size_t o = j.snap ? m.at[t] : 0;
+        for (int q = 0; q < 4; ++q) {
+            part[q] = j.src[t * 4 + q];
+            if (!j.snap) continue;
+            const size_t n = tree_bytes(nn, m.K, q);
+            memcpy(j.snap + o, part[q], n);
+            part[q] = j.snap + o;
+            o += n;
+        }
+        const unsigned char *feat = static_cast<const unsigned char *>(part[0]); // 8-byte integers, at any address in the snapshot
+        const uint8_t *bin = static_cast<const uint8_t *>(part[1]), *split = static_cast<const uint8_t *>(part[2]);
+        for (int i = 0; i < nn; ++i) {
+            uint32_t w = 0u;
+            if (split[i]) {
+                int64_t f;
+                memcpy(&f, feat + (size_t)i * 8, 8);
+                f -= 1;
+                if (f < 0 || f >= m.nfeats || 2 * i + 2 >= nn) {
+                    long long none = 0;
+                    j.bad.compare_exchange_strong(none, ((long long)t << 32 | i) + 1);
+                } else {
+                    w = (uint32_t)f | ((uint32_t)bin[i] << 16) | (1u << 24) | ((j.feattypes ? (j.feattypes[f] ? 1u : 0u) : 1u) << 25);
+                }
+            }
+            tr[i] = w;
+        }
+        for (int i = nn; i < m.nnp; ++i) tr[i] = 0u;
+        memcpy(tr + m.nnp, part[3], (size_t)nn * m.K * 4);
+        memset(tr + m.nnp + (size_t)nn * m.K, 0, (size_t)(m.nnp - nn) * m.K * 4);
+    }
+}
+
 // src: [ntrees][4] pointers; packs, uploads and keeps the snapshot.  edges may be null (binned input only).
+// All staging threads pack, straight into pinned buffers that are copied meanwhile; one thread into a zeroed image, its upload from
+// pageable memory and a second pass for the snapshot took 2.4 ms at 200 trees of depth 11 and 39 at 500 of depth 13.
 int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32_t *nodes, const void *edges, int e_dtype, int nedges,
                    int nfeats, const uint8_t *feattypes, bool snapshot) {
     const int K = m->K;
@@ -362,50 +429,51 @@ int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32
     m->tw = m->nnp * (1 + K);
     m->levels = 0;
     while ((2 << m->levels) - 1 < nn) ++m->levels;
-    const size_t tbytes = (size_t)ntrees * m->tw * 4, ne = (size_t)m->nedges * nfeats;
-    const size_t o64 = (tbytes + 15) & ~(size_t)15, o32 = o64 + ne * 8;
-    std::vector<unsigned char> host(o32 + ne * 4 + 16, 0);
-    uint32_t *tr = reinterpret_cast<uint32_t *>(host.data());
-    for (int t = 0; t < ntrees; ++t, tr += m->tw) {
-        const int64_t *feat = static_cast<const int64_t *>(src[t * 4]);
-        const uint8_t *bin = static_cast<const uint8_t *>(src[t * 4 + 1]), *split = static_cast<const uint8_t *>(src[t * 4 + 2]);
-        for (int i = 0; i < nodes[t]; ++i) {
-            if (!split[i]) continue;
-            const int64_t f = feat[i] - 1;
-            if (f < 0 || f >= nfeats || 2 * i + 2 >= nodes[t]) {
-                evb_set_error("evb_model: node %d of tree %d tests feature %lld of %d or has no children", i + 1, t + 1, (long long)(f + 1), nfeats);
-                return EVB_ERR_ARG;
-            }
-            tr[i] = (uint32_t)f | ((uint32_t)bin[i] << 16) | (1u << 24) | ((feattypes ? (feattypes[f] ? 1u : 0u) : 1u) << 25);
-        }
-        memcpy(tr + m->nnp, src[t * 4 + 3], (size_t)nodes[t] * K * 4);
+    const size_t unit = (size_t)m->tw * 4, tbytes = (size_t)ntrees * unit, ne = (size_t)m->nedges * nfeats;
+    const size_t o64 = (tbytes + 15) & ~(size_t)15, o32 = o64 + ne * 8, total = o32 + ne * 4 + 16;
+    PackJob job{m, src, nodes, feattypes, nullptr, {0}};
+    if (snapshot) {
+        m->src.assign(src, src + (size_t)ntrees * 4);
+        m->nodes.assign(nodes, nodes + ntrees);
+        m->at.resize((size_t)ntrees + 1);
+        size_t o = 0;
+        for (int t = 0; t < ntrees; ++t) { m->at[t] = o; for (int q = 0; q < 4; ++q) o += tree_bytes(nodes[t], K, q); }
+        m->at[ntrees] = o;
+        m->snap = job.snap = big_alloc(o);
+        if (!m->snap) { evb_set_error("out of host memory"); return EVB_ERR_ARG; }
+        if (edges) { m->src_edges = edges; m->snap_edges.assign((const unsigned char *)edges, (const unsigned char *)edges + ne * (e_dtype == EVB_F64 ? 8 : 4)); }
+        if (feattypes) { m->src_ft = feattypes; m->snap_ft.assign(feattypes, feattypes + nfeats); }
     }
+    // Below a megabyte everything goes up in one copy of an ordinary buffer (so do trees that are larger than a pinned buffer).
+    const bool piped = tbytes > ((size_t)1 << 20) && unit <= evb_stage_bytes();
+    const size_t hosted = piped ? o64 : 0; // bytes of the block that are not in `host`
+    std::vector<unsigned char> host(total - hosted);
     if (edges) {
-        double *e64 = reinterpret_cast<double *>(host.data() + o64);
-        float *e32 = reinterpret_cast<float *>(host.data() + o32);
+        double *e64 = reinterpret_cast<double *>(host.data() + (o64 - hosted));
+        float *e32 = reinterpret_cast<float *>(host.data() + (o32 - hosted));
         for (size_t i = 0; i < ne; ++i) {
             if (e_dtype == EVB_F64) { e64[i] = static_cast<const double *>(edges)[i]; e32[i] = (float)e64[i]; }
             else { e32[i] = static_cast<const float *>(edges)[i]; e64[i] = e32[i]; }
         }
     }
-    EVB_CUDA(evb_dev_alloc(&m->block, host.size()));
-    EVB_CUDA(cudaMemcpy(m->block, host.data(), host.size(), cudaMemcpyHostToDevice));
+    EVB_CUDA(evb_dev_alloc(&m->block, total));
+    cudaStream_t st = nullptr;
+    EVB_CUDA(evb_stream_get(&st));
+    int32_t rc = EVB_OK;
+    if (piped) rc = evb_h2d_made(m->block, unit, (size_t)ntrees, pack_trees, &job, st);
+    else pack_trees(&job, reinterpret_cast<char *>(host.data()), 0, (size_t)ntrees);
+    if (rc == EVB_OK && job.bad.load() != 0) {
+        const long long at = job.bad.load() - 1;
+        evb_set_error("evb_model: node %lld of tree %lld tests a feature that is not one of %d or has no children", (at & 0xffffffffll) + 1, (at >> 32) + 1, nfeats);
+        rc = EVB_ERR_ARG;
+    }
+    if (rc == EVB_OK) rc = evb_h2d_staged(static_cast<char *>(m->block) + hosted, host.data(), host.size(), st);
+    if (cudaStreamSynchronize(st) != cudaSuccess && rc == EVB_OK) { evb_set_error("CUDA error %s while a model was uploaded", cudaGetErrorString(cudaGetLastError())); rc = EVB_ERR_CUDA; }
+    evb_stream_put(st);
+    EVB_CHECK(rc);
     m->d_trees = static_cast<const uint32_t *>(m->block);
     m->d_e64 = reinterpret_cast<const double *>(static_cast<char *>(m->block) + o64);
     m->d_e32 = reinterpret_cast<const float *>(static_cast<char *>(m->block) + o32);
-    if (!snapshot) return EVB_OK;
-    m->src.assign(src, src + (size_t)ntrees * 4);
-    m->nodes.assign(nodes, nodes + ntrees);
-    m->at.resize(ntrees);
-    size_t total = 0;
-    for (int t = 0; t < ntrees; ++t) { m->at[t] = total; for (int q = 0; q < 4; ++q) total += tree_bytes(nodes[t], K, q); }
-    m->snap.resize(total);
-    for (int t = 0; t < ntrees; ++t) {
-        size_t o = m->at[t];
-        for (int q = 0; q < 4; ++q) { const size_t n = tree_bytes(nodes[t], K, q); memcpy(m->snap.data() + o, src[t * 4 + q], n); o += n; }
-    }
-    if (edges) { m->src_edges = edges; m->snap_edges.assign((const unsigned char *)edges, (const unsigned char *)edges + ne * (e_dtype == EVB_F64 ? 8 : 4)); }
-    if (feattypes) { m->src_ft = feattypes; m->snap_ft.assign(feattypes, feattypes + nfeats); }
     return EVB_OK;
 }
 
@@ -420,6 +488,10 @@ extern "C" void evb_model_destroy(evb_model *m) {
     delete m;
 }
 
+static int32_t no_host_memory() {
+    evb_set_error("out of host memory");
+    return EVB_ERR_ARG;
+}
 static int32_t model_args(int32_t loss, int32_t K, int32_t ntrees, int32_t nfeats) {
     if (nfeats < 1 || nfeats > 65535 || ntrees < 0 || K < 1 || K > 64 || loss < 0 || loss > EVB_LOSS_LAST) {
         evb_set_error("evb_predict: invalid argument");
@@ -442,7 +514,9 @@ extern "C" int32_t evb_model_create(evb_model **out, int32_t device, int32_t los
     evb_model *m = new (std::nothrow) evb_model();
     if (!m) { evb_set_error("out of host memory"); return EVB_ERR_ARG; }
     m->device = device; m->loss = loss; m->K = K;
-    const int32_t rc = model_fill(m, ntrees, src, nodes, edges, edges_dtype, nedges, nfeats, feattypes, true);
+    int32_t rc;
+    try { rc = model_fill(m, ntrees, src, nodes, edges, edges_dtype, nedges, nfeats, feattypes, true); }
+    catch (const std::bad_alloc &) { rc = no_host_memory(); }
     if (rc != EVB_OK) { evb_model_destroy(m); return rc; }
     *out = m;
     return EVB_OK;
@@ -682,7 +756,8 @@ extern "C" int32_t evb_model_predict(const evb_model *m, int32_t ntrees, const v
         return EVB_ERR_ARG;
     }
     EVB_CUDA(cudaSetDevice(m->device));
-    return predict_rows(*m, ntrees, x, x_dtype, x_row_major, nobs, apply_link, out, leaf_idx, kernel_ms, true);
+    try { return predict_rows(*m, ntrees, x, x_dtype, x_row_major, nobs, apply_link, out, leaf_idx, kernel_ms, true); }
+    catch (const std::bad_alloc &) { return no_host_memory(); }
 }
 
 // one call with trees that are packed for it: evb_predict (bins) and evb_predict_x (raw features)
@@ -694,16 +769,19 @@ static int32_t predict_once(int32_t device, int32_t loss, int32_t K, int32_t ntr
     EVB_CHECK(model_args(loss, K, ntrees, nfeats));
     EVB_CHECK(evb_check_device(device));
     if (nobs == 0) return EVB_OK;
-    std::vector<const void *> src((size_t)ntrees * 4);
-    std::vector<int32_t> nodes(ntrees, nn);
-    for (int t = 0; t < ntrees; ++t) {
-        const size_t o = (size_t)t * nn;
-        src[4 * t] = feat + o; src[4 * t + 1] = cond_bin + o; src[4 * t + 2] = split + o; src[4 * t + 3] = leaf_pred + o * K;
-    }
     evb_model m;
     m.device = device; m.loss = loss; m.K = K;
-    int32_t rc = model_fill(&m, ntrees, src.data(), nodes.data(), edges, x_type < 0 ? EVB_F32 : x_type, nedges, nfeats, feattypes, false);
-    if (rc == EVB_OK) rc = predict_rows(m, ntrees, x, x_type, x_row_major, nobs, apply_link, out, leaf_idx, ms_out, false);
+    int32_t rc;
+    try {
+        std::vector<const void *> src((size_t)ntrees * 4);
+        std::vector<int32_t> nodes(ntrees, nn);
+        for (int t = 0; t < ntrees; ++t) {
+            const size_t o = (size_t)t * nn;
+            src[4 * t] = feat + o; src[4 * t + 1] = cond_bin + o; src[4 * t + 2] = split + o; src[4 * t + 3] = leaf_pred + o * K;
+        }
+        rc = model_fill(&m, ntrees, src.data(), nodes.data(), edges, x_type < 0 ? EVB_F32 : x_type, nedges, nfeats, feattypes, false);
+        if (rc == EVB_OK) rc = predict_rows(m, ntrees, x, x_type, x_row_major, nobs, apply_link, out, leaf_idx, ms_out, false);
+    } catch (const std::bad_alloc &) { rc = no_host_memory(); }
     evb_dev_free(m.block);
     return rc;
 }

@@ -205,6 +205,37 @@ int32_t evb_h2d_staged_strided(void *dst_dev, const void *src_host, size_t seg_b
     return EVB_OK;
 }
 
+// Memory that is made on the way: fill(ctx, buffer, first, count) writes units [first, first + count) of `unit` bytes each to a pinned
+// buffer (all staging threads, a unit is one thread's), which is copied while the next one is filled.  Returns when everything has arrived.
+// unit <= STAGE_BYTES.
+size_t evb_stage_bytes() { return STAGE_BYTES; }
+int32_t evb_h2d_made(void *dst_dev, size_t unit, size_t count, void (*fill)(void *, char *, size_t, size_t), void *ctx, cudaStream_t st) {
+    int dev = 0;
+    EVB_CUDA(cudaGetDevice(&dev));
+    if (unit == 0 || unit > STAGE_BYTES || dev < 0 || dev >= 64) { evb_set_error("evb_h2d_made: invalid argument"); return EVB_ERR_ARG; }
+    StageRing &r = g_rings[dev];
+    std::lock_guard<std::mutex> lock(r.mu);
+    EVB_CHECK(ring_ready(r));
+    // a few chunks at least, so that the first copy starts early
+    const size_t per = std::max<size_t>(1, std::min(STAGE_BYTES, std::max<size_t>(unit * count / 4, (size_t)1 << 20)) / unit);
+    struct Job { void (*fill)(void *, char *, size_t, size_t); void *ctx; char *buf; size_t first, unit; } j{fill, ctx, nullptr, 0, unit};
+    for (size_t u = 0; u < count; u += per) {
+        const int b = r.next;
+        r.next = (b + 1) % STAGE_NB;
+        const size_t n = std::min(per, count - u);
+        if (r.used[b]) EVB_CUDA(cudaEventSynchronize(r.ev[b]));
+        j.buf = static_cast<char *>(r.buf[b]); j.first = u;
+        evb_parallel([](void *c, size_t b0, size_t e0) { Job &q = *static_cast<Job *>(c); q.fill(q.ctx, q.buf + b0 * q.unit, q.first + b0, e0 - b0); }, &j, n,
+                     std::max<size_t>(1, ((size_t)64 << 10) / unit));
+        EVB_CUDA(cudaMemcpyAsync(static_cast<char *>(dst_dev) + u * unit, r.buf[b], n * unit, cudaMemcpyHostToDevice, st));
+        EVB_CUDA(cudaEventRecord(r.ev[b], st));
+        r.used[b] = true;
+    }
+    for (int q = 0; q < STAGE_NB; ++q)
+        if (r.used[q]) { EVB_CUDA(cudaEventSynchronize(r.ev[q])); r.used[q] = false; }
+    return EVB_OK;
+}
+
 int32_t evb_h2d_staged(void *dst_dev, const void *src_host, size_t bytes, cudaStream_t st, bool drain) {
     return evb_h2d_staged_strided(dst_dev, src_host, bytes, 1, bytes, st, drain);
 }

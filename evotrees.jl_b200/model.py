@@ -68,14 +68,10 @@ def _pack(m: EvoTree, ntree_limit: int):
     return nn, feat, cb, sp, lp
 
 
-_TREE_TYPES = tuple(np.dtype(d) for d in (np.int64, np.uint8, np.uint8, np.float32))
+_TREE_TYPES = [np.dtype(d) for d in (np.int64, np.uint8, np.uint8, np.float32)]
 
 
-def _address(a: np.ndarray) -> int:
-    try:
-        return C.addressof(C.c_char.from_buffer(a))      # a third of the time of the array interface: 0.65 and 1.8 us
-    except (TypeError, ValueError):                      # read-only, or empty
-        return a.__array_interface__["data"][0]
+_addressof, _from_buffer = C.addressof, C.c_char.from_buffer
 
 
 def _tree_arrays(t: Tree):
@@ -93,12 +89,23 @@ class _Packed:
         self.device, self.loss, self.K = device, m.loss, m.K
         self.trees = list(m.trees)
         self.edges, self.feattypes = m.info["edges"], m.info["feattypes"]
-        arrays, self.shared = [], True      # shared: the library reads the model's own arrays, not copies
-        for t in self.trees:
-            for a, dt in zip(_tree_arrays(t), _TREE_TYPES):
-                if a.dtype is not dt and a.dtype != dt and not (dt.itemsize == 1 and a.dtype == bool) or not a.flags.c_contiguous:
-                    a, self.shared = np.ascontiguousarray(a, dt), False
-                arrays.append(a)
+        self.shared = True                  # the library reads the model's own arrays, not copies
+        arrays = [a for t in self.trees for a in (t.feat, t.cond_bin, t.split, t.pred)]
+        n, src = len(self.trees), None
+        size = [a.size for a in arrays]
+        if size[1::4] != size[::4] or size[2::4] != size[::4] or size[3::4] != [s * m.K for s in size[::4]]:
+            raise ValueError("the arrays of a tree must have one entry per node")
+        if [a.dtype for a in arrays] == _TREE_TYPES * n:
+            try:                            # C-contiguous and writable, or it raises; a third of the time of the array interface
+                src = [_addressof(_from_buffer(a)) for a in arrays]
+            except (TypeError, ValueError):
+                pass
+        if src is None:
+            for i, a in enumerate(arrays):
+                dt = _TREE_TYPES[i % 4]
+                if a.dtype != dt and not (dt.itemsize == 1 and a.dtype == bool) or not a.flags.c_contiguous:
+                    arrays[i], self.shared = np.ascontiguousarray(a, dt), False
+            src = [a.__array_interface__["data"][0] for a in arrays]
         e, ft = np.asarray(self.edges), np.asarray(self.feattypes)
         if e.dtype not in (np.float32, np.float64) or not e.flags.c_contiguous:
             e, self.shared = np.ascontiguousarray(e, np.float64), False
@@ -106,9 +113,8 @@ class _Packed:
             ft, self.shared = np.ascontiguousarray(ft, np.uint8), False
         self.arrays = arrays
         self.keep = (e, ft)
-        n = len(self.trees)
-        src = np.array([_address(a) for a in arrays], np.uint64)
-        nodes = np.array([a.size for a in arrays[::4]], np.int32)
+        src = np.array(src, np.uint64)
+        nodes = np.array(size[::4], np.int32)
         self.handle = C.c_void_p()
         _lib.check(_lib.lib().evb_model_create(
             C.byref(self.handle), C.c_int32(device), C.c_int32(_lib.LOSS_CODES[m.loss]), C.c_int32(m.K), C.c_int32(n), _lib.ptr(src), _lib.ptr(nodes),

@@ -80,3 +80,28 @@ def test_packed_model_notices_changes(pkg):
     check()
     m2 = copy.deepcopy(m)
     np.testing.assert_array_equal(pkg.predict(m2, x), pkg.predict(m, x))
+
+
+# Trees of more than a megabyte are packed into pinned buffers by several threads: one chunk and several, a tree per unit that
+# is larger than such a buffer, small trees among large ones.
+@pytest.mark.parametrize("depth,ntrees,K", [(11, 200, 1), (13, 400, 1), (9, 700, 5), (15, 3, 64)])
+def test_large_models(pkg, depth, ntrees, K):
+    m = _model(pkg, 9, depth, ntrees, K, 32, "mse", depth)
+    m.trees[1::3] = _model(pkg, 9, 4, ntrees, K, 32, "mse", 99).trees[1::3]
+    x = np.random.default_rng(1).normal(size=(50, 9))
+    for _ in range(2):
+        np.testing.assert_allclose(pkg.predict(m, x).reshape(50, K), _walk(m, x)[0], rtol=1e-5, atol=1e-5)
+    m.trees[-1].pred[-1] += 1.0             # the last value of the last tree
+    m.trees[-1].split[0], m.trees[-1].feat[0], m.trees[-1].cond_bin[0] = 1, 9, 31
+    np.testing.assert_allclose(pkg.predict(m, x).reshape(50, K), _walk(m, x)[0], rtol=1e-5, atol=1e-5)
+
+
+def test_trees_that_cannot_be_packed(pkg):
+    """Arrays of unequal lengths, a test of a feature that does not exist: errors, not reads past the end."""
+    x = np.random.default_rng(0).normal(size=(3, 6))
+    for change in (lambda t: setattr(t, "cond_bin", t.cond_bin[:-1]), lambda t: setattr(t, "pred", t.pred[:4]), lambda t: t.feat.__setitem__(0, 7)):
+        m = _model(pkg, 6, 5, 8, 1, 16, "mse", 3)
+        m.trees[2].split[0] = 1
+        change(m.trees[2])
+        with pytest.raises(Exception):
+            pkg.predict(m, x)
