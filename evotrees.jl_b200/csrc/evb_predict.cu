@@ -525,8 +525,9 @@ extern "C" int32_t evb_model_create(evb_model **out, int32_t device, int32_t los
 // ================================================================================================= calls
 namespace {
 
-// Work buffers of one call at a time: three sets of {stream, pinned input, device input, pinned output}.  A call takes one
-// from the device's pool and puts it back; the pool keeps at most KEEP of them (evb_trim_cache gives them back).
+// Work buffers of one call at a time: three sets of {stream, pinned input, device input, pinned output}, of the size of a chunk of
+// rows (12 MB of input and output, or one row).  A call takes one from the device's pool and puts it back; the pool keeps at most
+// KEEP of them (evb_trim_cache gives them back).
 constexpr int PRED_SLOTS = 3;
 struct PredWs {
     struct Slot {
@@ -682,7 +683,9 @@ int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, 
     const size_t total = (size_t)nobs * (in_row + out_row);
     size_t cbytes = total / 6;
     cbytes = std::min<size_t>(std::max<size_t>(cbytes, (size_t)1 << 20), (size_t)12 << 20);
-    int64_t chunk = (int64_t)std::max<size_t>(1024, cbytes / (in_row + out_row)) / 1024 * 1024;
+    // Whole CTAs of the kernels where that many rows fit; wide rows: as many as fit, so that no slot pins more than 12 MB (or one row).
+    int64_t chunk = (int64_t)std::max<size_t>(1, cbytes / (in_row + out_row));
+    if (chunk > 32) chunk -= chunk % (chunk >= 1024 ? 1024 : 32);
     chunk = std::min<int64_t>(chunk, nobs);
     // one row or a few: the kernel reads them from pinned memory itself
     const bool zero_copy = (size_t)nobs * in_row <= (size_t)16 * 1024;

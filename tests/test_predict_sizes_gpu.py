@@ -105,3 +105,20 @@ def test_trees_that_cannot_be_packed(pkg):
         change(m.trees[2])
         with pytest.raises(Exception):
             pkg.predict(m, x)
+
+
+def test_work_buffers_are_bounded_in_bytes(pkg):
+    """Rows of 240 KB: the buffers a call keeps are those of a 12 MB chunk (its pinned and its device side are of one size), and
+    the chunks of a few rows add up to the same predictions."""
+    import torch
+    from evotrees_b200 import _lib
+    m = _model(pkg, 60_000, 4, 5, 1, 8, "mse", 1)
+    x = np.random.default_rng(2).normal(size=(1_100, 60_000)).astype(np.float32)
+    want = _walk(m, x[::50])[0][:, 0]
+    pkg.predict(m, x[:1])                    # the model and the context are on the device
+    _lib.check(_lib.lib().evb_trim_cache(0))
+    free = torch.cuda.mem_get_info(0)[0]
+    got = pkg.predict(m, x)
+    kept = free - torch.cuda.mem_get_info(0)[0]
+    np.testing.assert_allclose(got[::50], want, rtol=1e-5, atol=1e-6)
+    assert kept <= 3 * 2 * (12 << 20) + (32 << 20), kept     # three slots, binned rows beside the raw ones, granularity of the allocator
