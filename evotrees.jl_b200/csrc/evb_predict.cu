@@ -537,6 +537,7 @@ struct PredWs {
         void *d_in = nullptr, *d_aux = nullptr;
         size_t cap_pin_in = 0, cap_pin_out = 0, cap_in = 0, cap_aux = 0;
     } s[PRED_SLOTS];
+    cudaEvent_t start = nullptr; // of a timed call
     int dev = 0;
 };
 constexpr size_t KEEP = 4;
@@ -554,6 +555,7 @@ void ws_delete(PredWs *w) {
         evb_dev_free(s.d_in);
         evb_dev_free(s.d_aux);
     }
+    if (w->start) cudaEventDestroy(w->start);
     delete w;
 }
 struct WsGuard { // the device is current
@@ -605,7 +607,7 @@ int32_t allow_smem(K kern, size_t bytes) { // more than the default 48 KB of dyn
     return EVB_OK;
 }
 
-// which kernel takes a chunk of n rows
+// which kernel takes a chunk of n rows (what one launch gets, not what the call has)
 enum { PK_ONE, PK_MID, PK_STAGED, PK_WIDE };
 struct PredPlan { int kind, rows, TB; size_t smem; };
 PredPlan plan_kernel(const evb_model &m, int n, int num_sms) {
@@ -616,7 +618,9 @@ PredPlan plan_kernel(const evb_model &m, int n, int num_sms) {
     const size_t one = (size_t)FW * 4 + (size_t)ONE_THREADS * m.K * 4;
     if (n <= 4 * num_sms && one <= 96 * 1024) return {PK_ONE, 1, 0, one};
     // Staged: the largest CTA that still gives every SM one, as long as two blocks of trees fit beside its rows.  Copying
-    // all trees once per CTA has to be worth it: below `mid_rows` rows the trees are read through L1 instead.
+    // all trees once per CTA has to be worth it: below `mid_rows` rows of a launch the trees are read through L1 instead.  ms of
+    // kernels, staged and mid, chunks one after the other: 1M x 100, depth 11 (30k rows a chunk) 10.1 and 5.3; 1M x 50 gaussian, depth 7
+    // (59k) 4.14 and 3.34; 1M x 28 five classes, depth 8 (79k) 4.53 and 4.93; 4M x 10, depth 6 (285k) 3.13 and 4.27.
     const int mid_rows = 64 * 1024;
     if (n > mid_rows) {
         for (int rows = 1024; rows >= 128; rows >>= 1) {
@@ -695,7 +699,7 @@ int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, 
     a.trees = m.d_trees; a.nnp = m.nnp; a.tw = m.tw; a.levels = m.levels; a.K = m.K; a.loss = m.loss; a.ntrees = ntrees; a.apply_link = apply_link;
     int64_t first[PRED_SLOTS] = {-1, -1, -1};
     int rows_in[PRED_SLOTS] = {};
-    double ms = 0.0;
+    double ms = 0.0, until = 0.0; // ms during which kernels ran, up to `until` ms after the start (chunks overlap)
     auto collect = [&](int q) -> int32_t { // results of the chunk in slot q -> the caller's arrays
         PredWs::Slot &s = w.s[q];
         if (first[q] < 0) return EVB_OK;
@@ -703,7 +707,11 @@ int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, 
         const int64_t r0 = first[q], nr = rows_in[q];
         evb_copy_packed(s.pin_out, out + r0, (size_t)nr * 4, (size_t)nobs * 4, 0, (size_t)nr * 4 * m.K, false);
         if (leaf_idx) evb_copy_packed(s.pin_out + (size_t)nr * 4 * m.K, leaf_idx + r0, (size_t)nr * 4, (size_t)nobs * 4, 0, (size_t)nr * 4 * ntrees, false);
-        if (ms_out) { float v = 0.f; if (cudaEventElapsedTime(&v, s.t0, s.t1) == cudaSuccess) ms += v; }
+        float b = 0.f, e = 0.f;
+        if (ms_out && cudaEventElapsedTime(&b, w.start, s.t0) == cudaSuccess && cudaEventElapsedTime(&e, w.start, s.t1) == cudaSuccess && e > until) {
+            ms += e - std::max<double>(b, until);
+            until = e;
+        }
         first[q] = -1;
         return EVB_OK;
     };
@@ -713,6 +721,10 @@ int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, 
         const int64_t nr = std::min<int64_t>(chunk, nobs - r0);
         EVB_CHECK(collect(q));
         EVB_CHECK(slot_streams(s, ms_out != nullptr));
+        if (ms_out && r0 == 0) {
+            if (!w.start) EVB_CUDA(cudaEventCreate(&w.start));
+            EVB_CUDA(cudaEventRecord(w.start, s.st));
+        }
         EVB_CHECK(pinned_reserve(s.pin_in, s.cap_pin_in, (size_t)chunk * in_row));
         EVB_CHECK(pinned_reserve(s.pin_out, s.cap_pin_out, (size_t)chunk * out_row));
         // rows r0 .. r0 + nr: one piece of a row-major matrix, one segment per feature of a column-major one

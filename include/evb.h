@@ -299,7 +299,7 @@ EVB_API int32_t evb_predict(int32_t device, int32_t loss, int32_t K, int32_t ntr
  *   x            host, EVB_F32 / EVB_F64; column-major [nobs x nfeats] (x_row_major = 0, a Julia Matrix) or
  *                row-major (x_row_major = 1, a C-ordered array)
  *   edges        host [nedges x nfeats] column-major, same dtype as x
- *   kernel_ms    optional: receives the summed device time of the binarize + traversal kernels
+ *   kernel_ms    optional: receives the milliseconds during which kernels of the call ran (those of different chunks overlap)
  */
 EVB_API int32_t evb_predict_x(int32_t device, int32_t loss, int32_t K, int32_t ntrees, int32_t nn, const int64_t *feat,
                               const uint8_t *cond_bin, const uint8_t *split, const float *leaf_pred, const void *x, int32_t x_dtype,

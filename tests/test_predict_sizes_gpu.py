@@ -122,3 +122,16 @@ def test_work_buffers_are_bounded_in_bytes(pkg):
     kept = free - torch.cuda.mem_get_info(0)[0]
     np.testing.assert_allclose(got[::50], want, rtol=1e-5, atol=1e-6)
     assert kept <= 3 * 2 * (12 << 20) + (32 << 20), kept     # three slots, binned rows beside the raw ones, granularity of the allocator
+
+
+def test_kernel_time_counts_overlap_once(pkg):
+    """The chunks of a call run side by side: the time during which kernels ran is no longer than the call."""
+    import time
+    m = _model(pkg, 16, 8, 200, 5, 64, "mlogloss", 1)
+    x = np.random.default_rng(2).normal(size=(500_000, 16)).astype(np.float32)
+    pkg.predict(m, x)
+    for _ in range(3):
+        stats = {}
+        t = time.perf_counter()
+        pkg.predict(m, x, stats=stats)
+        assert 0.0 < stats["kernel_ms"] <= (time.perf_counter() - t) * 1e3
