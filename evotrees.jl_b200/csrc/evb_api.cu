@@ -257,7 +257,6 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     }
     { const char *e = getenv("EVB_GRAPH"); h->use_graphs = e ? atoi(e) != 0 : true; }
     h->graph_mask_cond = -1;
-    h->early = n <= 1000000;
 
     h->maxslots = evb_level_slots(D > 1 ? D - 1 : 1);
     EVB_CUDA(dalloc(&h->cum, (size_t)h->maxslots + 1)); EVB_CUDA(dalloc(&h->slot_node, (size_t)h->maxslots * 2)); h->rbase = h->slot_node + h->maxslots;

@@ -19,22 +19,18 @@ __device__ __forceinline__ void run(const Args &a, uint32_t *smem, uint32_t *que
 __global__ void __launch_bounds__(1024, 1) k_histg(KArgs k) {
     extern __shared__ __align__(128) uint32_t s_img[];
     Args &a = k.a;
-    evb_pdl_next();
+    if ((long long)blockIdx.x * a.min_rows >= max(1ll, (long long)a.plan->R + (long long)a.plan->nbuild * a.pad_rows)) return;
     evb_hg_select(k.g, a, blockIdx.y, blockIdx.z);
     const int P = evb_hg_planes(k.g, blockIdx.z), words = nparts(a.nfull, a.tails) * (a.B + 1) * P * 8;
     for (int i = threadIdx.x; i < words; i += blockDim.x) reinterpret_cast<uint4 *>(s_img)[i] = make_uint4(0u, 0u, 0u, 0u);
     uint32_t *queue = s_img + k.g.queue;
     if (threadIdx.x == 0) queue[QUEUE] = 0u;
-    evb_pdl_wait();
-    if ((long long)blockIdx.x * a.min_rows >= max(1ll, (long long)a.plan->R + (long long)a.plan->nbuild * a.pad_rows)) return;
     __syncthreads();
     EVB_HG_DISPATCH(k.g, blockIdx.z, run, a, s_img, queue)
 }
 
 // clears the accumulators of the level's build slots (all feature columns, sampled or not)
 __global__ void __launch_bounds__(256) k_hg_clear(unsigned long long *hsum, uint32_t *hcnt, unsigned long long *hlow, const uint32_t *low_any, const LevelPlan *plan, size_t per_slot, int nq) {
-    evb_pdl_next();
-    evb_pdl_wait();
     const size_t n = (size_t)plan->nbuild * per_slot, ns = n * nq;
     const bool low = hlow && *low_any;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += (size_t)gridDim.x * blockDim.x) {
@@ -183,7 +179,7 @@ int32_t evb_launch_histg(evb_handle *h, int level) {
     k.g = g;
     evb_hg_args(h, level, &k.a);
     evb_tic(h, EVB_T_HIST);
-    const cudaError_t e = evb_launch_pdl(h->early, k_histg, dim3(g.G, g.ngf, g.ngc), dim3(g.threads), g.smem, h->st, k);
+    const cudaError_t e = evb_launch(k_histg, dim3(g.G, g.ngf, g.ngc), dim3(g.threads), g.smem, h->st, k);
     evb_toc(h, EVB_T_HIST);
     EVB_CUDA(e);
     return EVB_OK;
@@ -193,7 +189,7 @@ int32_t evb_launch_acc_clear(evb_handle *h, int level) {
     const size_t per_slot = (size_t)h->B * h->SC;
     const size_t blocks = std::min<size_t>(((size_t)evb_level_slots(level) * per_slot * h->nq + 255) / 256, (size_t)h->num_sms * 8);
     evb_tic(h, EVB_T_HIST_REDUCE);
-    const cudaError_t e = evb_launch_pdl(h->early, k_hg_clear, dim3((unsigned)blocks), dim3(256), 0, h->st, h->hsum_q, h->hcnt_q, h->hlow_q, h->low + evb_low_any(level),
+    const cudaError_t e = evb_launch(k_hg_clear, dim3((unsigned)blocks), dim3(256), 0, h->st, h->hsum_q, h->hcnt_q, h->hlow_q, h->low + evb_low_any(level),
                                          h->plan + level, per_slot, h->nq);
     evb_toc(h, EVB_T_HIST_REDUCE);
     EVB_CUDA(e);

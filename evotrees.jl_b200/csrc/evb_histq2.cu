@@ -136,10 +136,7 @@ __global__ void __launch_bounds__(Q2_THREADS, 2) k_histq2(Q2Args a) {
     const int tid = threadIdx.x, wid = tid >> 5, l = tid & 31;
     constexpr int NW = Q2_WARPS, NT = Q2_THREADS;
     const int b = blockIdx.x, chunk0 = blockIdx.y * NC;
-    evb_pdl_next();
     uint32_t *img_w = reinterpret_cast<uint32_t *>(smem);
-    for (int i = tid; i < (a.B + 1) * 2 * NCOL; i += NT) img_w[i] = 0u;
-    evb_pdl_wait();
     const int nbuild = a.plan->nbuild;
     const long long R = a.plan->R + (long long)nbuild * a.pad_rows; // pad_rows rows that do not exist after every build node
     // few rows: fewer CTAs take part (every CTA costs one pass over its image)
@@ -151,6 +148,7 @@ __global__ void __launch_bounds__(Q2_THREADS, 2) k_histq2(Q2Args a) {
     if (b >= G) return;
     const int lo = (int)(R * b / G), hi = (int)(R * (b + 1) / G);
     if (lo >= hi) return;
+    for (int i = tid; i < (a.B + 1) * 2 * NCOL; i += NT) img_w[i] = 0u;
     __syncthreads();
 
     int s0;
@@ -311,7 +309,7 @@ __global__ void __launch_bounds__(256) k_q2_tail(const uint8_t *xC, long long n,
 }
 
 template <int NC, bool TAIL>
-int q2_instance(bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st, bool early) {
+int q2_instance(bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st) {
     static size_t attr_set[64] = {}; // dynamic shared memory the kernel has been allowed on each device
     int dev = 0;
     cudaGetDevice(&dev);
@@ -325,25 +323,25 @@ int q2_instance(bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_histq2<NC, TAIL>, Q2_THREADS, smem) != cudaSuccess) nb = 0;
         return nb;
     }
-    return (int)evb_launch_pdl(early, k_histq2<NC, TAIL>, grid, dim3(Q2_THREADS), smem, st, *a);
+    return (int)evb_launch(k_histq2<NC, TAIL>, grid, dim3(Q2_THREADS), smem, st, *a);
 }
 template <bool TAIL>
-int q2_dispatch_nc(int NC, bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st, bool early = false) {
+int q2_dispatch_nc(int NC, bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st) {
     switch (NC) {
-    case 1: return q2_instance<1, TAIL>(launch, a, grid, smem, st, early);
-    case 2: return q2_instance<2, TAIL>(launch, a, grid, smem, st, early);
-    case 3: return q2_instance<3, TAIL>(launch, a, grid, smem, st, early);
-    case 4: return q2_instance<4, TAIL>(launch, a, grid, smem, st, early);
-    case 5: return q2_instance<5, TAIL>(launch, a, grid, smem, st, early);
-    default: return q2_instance<6, TAIL>(launch, a, grid, smem, st, early);
+    case 1: return q2_instance<1, TAIL>(launch, a, grid, smem, st);
+    case 2: return q2_instance<2, TAIL>(launch, a, grid, smem, st);
+    case 3: return q2_instance<3, TAIL>(launch, a, grid, smem, st);
+    case 4: return q2_instance<4, TAIL>(launch, a, grid, smem, st);
+    case 5: return q2_instance<5, TAIL>(launch, a, grid, smem, st);
+    default: return q2_instance<6, TAIL>(launch, a, grid, smem, st);
     }
 }
-int q2_dispatch(int NC, bool tail, bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st, bool early = false) {
-    if (tail) return q2_dispatch_nc<true>(NC, launch, a, grid, smem, st, early);
+int q2_dispatch(int NC, bool tail, bool launch, const Q2Args *a, dim3 grid, size_t smem, cudaStream_t st) {
+    if (tail) return q2_dispatch_nc<true>(NC, launch, a, grid, smem, st);
     switch (NC) {
-    case 7: return q2_instance<7, false>(launch, a, grid, smem, st, early);
-    case 8: return q2_instance<8, false>(launch, a, grid, smem, st, early);
-    default: return q2_dispatch_nc<false>(NC, launch, a, grid, smem, st, early);
+    case 7: return q2_instance<7, false>(launch, a, grid, smem, st);
+    case 8: return q2_instance<8, false>(launch, a, grid, smem, st);
+    default: return q2_dispatch_nc<false>(NC, launch, a, grid, smem, st);
     }
 }
 int q2_ncol(int NC, bool tail) { const int need = 16 * NC + (tail ? 32 : 0); return need <= 32 ? 32 : need <= 64 ? 64 : 128; }
@@ -425,7 +423,7 @@ int32_t evb_launch_histq2(evb_handle *h, int level) {
     a.hsum = h->hsum_q; a.hcnt = h->hcnt_q;
     a.RSH = g.RSH; a.B = h->B; a.SC = h->SC; a.nmain = g.nmain; a.ntail = g.ntail; a.min_rows = g.min_rows; a.pad_rows = evb_pad_rows(h); a.zrow = (uint32_t)h->n;
     evb_tic(h, EVB_T_HIST);
-    const cudaError_t e = (cudaError_t)q2_dispatch(g.NC, g.ntail > 0, true, &a, dim3(g.G, g.ngroups), g.smem, h->st, h->early);
+    const cudaError_t e = (cudaError_t)q2_dispatch(g.NC, g.ntail > 0, true, &a, dim3(g.G, g.ngroups), g.smem, h->st);
     evb_toc(h, EVB_T_HIST);
     EVB_CUDA(e);
     return EVB_OK;

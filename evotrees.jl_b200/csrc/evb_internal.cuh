@@ -172,7 +172,6 @@ struct evb_handle {
     int tree_seq, pending;          // trees started / started but not yet collected
     // one CUDA graph per variant of the per-tree launch sequence (mask, gradients first, gradients fused, slot)
     bool use_graphs;
-    bool early; // launch kernels before their predecessor has ended (evb_launch_pdl)
     cudaGraphExec_t graph[64];
     int graph_calls[64];
     int64_t graph_launches[64][EVB_NTIMERS];
@@ -197,24 +196,15 @@ struct evb_handle {
     evb_timings tm;
 };
 
-// ---- programmatic dependent launch -----------------------------------------------------------------
-// The kernels of a tree follow one another and most are short: each is launched while the one before it still runs
-// (evb_launch_pdl, captured as a programmatic edge of the graph), does what needs no result of it, and waits for its end in
-// evb_pdl_wait.  Every kernel that is launched this way waits before it touches anything another kernel writes or reads.
-// Measured per tree, with / without: 1503 x 7 0.101 / 0.113 ms, 100k x 10 0.108 / 0.112, 1M x 100 (half of the rows) 0.252 / 0.261,
-// but 2M x 28 five classes 1.45 / 1.35 and 5M x 50 gaussian 1.75 / 1.62 (CTAs that wait take the places of others): up to a
-// million rows (evb_handle::early).
+// Plain launches: kernels that were launched before their predecessor's end (programmatic dependent launch) and waited for it cost time
+// at every size but the smallest -- CTAs that wait take the places of others.  ms per tree, with and without it: 1503 x 7 logloss 0.087 and
+// 0.088, 100k x 10 0.096 and 0.094, 60k x 77 poisson 0.150 and 0.129, 250k x 33 weighted 0.151 and 0.144, 200k x 50 gaussian 0.209 and 0.190,
+// 1M x 100 (half of the rows) 0.232 and 0.236, 2M x 20 logloss 0.317 and 0.303.
 #ifdef __CUDACC__
-__device__ __forceinline__ void evb_pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void evb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P, typename... A>
-inline cudaError_t evb_launch_pdl(bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+inline cudaError_t evb_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t c = {};
     c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = at; c.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&c, kern, P(args)...);
 }
 #endif

@@ -166,8 +166,6 @@ __global__ void __launch_bounds__(256) k_grads(int loss, int K, int nq, int unit
 // ---------------------------------------------------------------------------------- row sampling
 constexpr int SEL_CHUNK = 2048, SEL_THREADS = 256;
 __global__ void __launch_bounds__(SEL_THREADS) k_sel_count(const uint8_t *mask, uint8_t cond, long long n, int32_t *bcnt) {
-    evb_pdl_next();
-    evb_pdl_wait();
     __shared__ int s[SEL_THREADS / 32];
     const long long base = (long long)blockIdx.x * SEL_CHUNK;
     int c = 0;
@@ -200,8 +198,6 @@ __device__ __forceinline__ uint64_t pcg_out(u128 s) {
 }
 // gen: {state lo, hi, increment lo, hi, left, left word}: left = 1 when the high half of the last output is still to be used
 __global__ void __launch_bounds__(SEL_THREADS) k_sel_pcg(const uint64_t *gen, uint8_t cond, long long n, uint8_t *mask, int32_t *bcnt) {
-    evb_pdl_next();
-    evb_pdl_wait();
     static_assert(SEL_CHUNK == 8 * SEL_THREADS, "eight rows per thread");
     __shared__ int s[SEL_THREADS / 32];
     const u128 inc = ((u128)gen[3] << 64) | gen[2];
@@ -237,8 +233,6 @@ __global__ void __launch_bounds__(SEL_THREADS) k_sel_pcg(const uint64_t *gen, ui
 }
 struct RootPlan { int32_t *seg_cnt, *cum, *slot_node, *rbase; int4 *pl; uint8_t *kind; LevelPlan *plan; };
 __global__ void __launch_bounds__(1024) k_sel_scan(int32_t *bcnt, int nblocks, RootPlan r) {
-    evb_pdl_next();
-    evb_pdl_wait();
     __shared__ int sm[33];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int carry = 0;
@@ -269,8 +263,6 @@ __global__ void __launch_bounds__(1024) k_sel_scan(int32_t *bcnt, int nblocks, R
     }
 }
 __global__ void __launch_bounds__(SEL_THREADS) k_sel_scatter(const uint8_t *mask, uint8_t cond, long long n, const int32_t *boff, uint32_t *rows) {
-    evb_pdl_next();
-    evb_pdl_wait();
     constexpr int NW = SEL_CHUNK / 32;
     __shared__ uint32_t s_bits[NW];
     __shared__ int s_pref[NW];
@@ -324,8 +316,6 @@ __device__ __forceinline__ void publish(const uint4 *src, uint4 *dst, int n) {
 }
 __global__ void __launch_bounds__(256) k_finalize(FinArgs a) {
     extern __shared__ uint32_t s_packed[];
-    evb_pdl_next();
-    evb_pdl_wait();
     if (blockIdx.x == 0) publish(a.pub_src, a.pub_dst, a.pub_n);
     const uint32_t *packed = a.t_packed;
     if (a.packed_in_smem) {
@@ -367,8 +357,6 @@ __global__ void __launch_bounds__(256) k_finalize_staged(FinArgs a) {
     float *s_p = reinterpret_cast<float *>(s_fin), *s_g = s_p + 256 * K;
     uint32_t *s_tree = reinterpret_cast<uint32_t *>(s_g + 256 * nq);
     uint32_t *s_rows = s_tree + a.nn;
-    evb_pdl_next();
-    evb_pdl_wait();
     if (blockIdx.x == 0) publish(a.pub_src, a.pub_dst, a.pub_n);
     const int rw = a.RS >> 2, rwp = rw + 1; // words per row, padded
     for (int i = threadIdx.x; i < a.nn; i += 256) s_tree[i] = a.t_packed[i];
@@ -436,8 +424,6 @@ __global__ void __launch_bounds__(256) k_finalize_pipe(FinPipeArgs a) {
     // words, so that the row buffers start on a 16-byte boundary (the copies into them are 16 bytes wide)
     extern __shared__ __align__(16) uint32_t s_fp[];
     const FinArgs &f = a.f;
-    evb_pdl_next();
-    evb_pdl_wait();
     if (blockIdx.x == 0) publish(f.pub_src, f.pub_dst, f.pub_n);
     const int nnp = (f.nn + 3) & ~3;
     uint32_t *s_tree = s_fp;
@@ -830,10 +816,10 @@ int32_t evb_launch_rows_init(evb_handle *h, int use_mask, uint8_t mask_cond) {
     const int nblocks = (int)((h->n + SEL_CHUNK - 1) / SEL_CHUNK);
     const RootPlan r{h->seg_cnt, h->cum, h->slot_node, h->rbase, h->pl, h->kind, h->plan};
     evb_tic(h, EVB_T_ROWS_INIT);
-    if (use_mask == EVB_MASK_PCG) EVB_CUDA(evb_launch_pdl(h->early, k_sel_pcg, dim3(nblocks), dim3(SEL_THREADS), 0, h->st, h->gen_d, mask_cond, h->n, h->mask_d, h->scan_tmp));
-    else EVB_CUDA(evb_launch_pdl(h->early, k_sel_count, dim3(nblocks), dim3(SEL_THREADS), 0, h->st, h->mask_d, mask_cond, h->n, h->scan_tmp));
-    EVB_CUDA(evb_launch_pdl(h->early, k_sel_scan, dim3(1), dim3(1024), 0, h->st, h->scan_tmp, nblocks, r));
-    EVB_CUDA(evb_launch_pdl(h->early, k_sel_scatter, dim3(nblocks), dim3(SEL_THREADS), 0, h->st, h->mask_d, mask_cond, h->n, h->scan_tmp, h->rows[0]));
+    if (use_mask == EVB_MASK_PCG) EVB_CUDA(evb_launch(k_sel_pcg, dim3(nblocks), dim3(SEL_THREADS), 0, h->st, h->gen_d, mask_cond, h->n, h->mask_d, h->scan_tmp));
+    else EVB_CUDA(evb_launch(k_sel_count, dim3(nblocks), dim3(SEL_THREADS), 0, h->st, h->mask_d, mask_cond, h->n, h->scan_tmp));
+    EVB_CUDA(evb_launch(k_sel_scan, dim3(1), dim3(1024), 0, h->st, h->scan_tmp, nblocks, r));
+    EVB_CUDA(evb_launch(k_sel_scatter, dim3(nblocks), dim3(SEL_THREADS), 0, h->st, h->mask_d, mask_cond, h->n, h->scan_tmp, h->rows[0]));
     evb_toc(h, EVB_T_ROWS_INIT);
     h->tm.launches[EVB_T_ROWS_INIT] += 2;
     EVB_CUDA(cudaGetLastError());
@@ -879,13 +865,13 @@ int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode, void *p
         if (per_sm < 1) per_sm = 1;
         int grid = h->num_sms * per_sm;
         if (grid > pa.ntiles) grid = pa.ntiles;
-        if (h->p.loss == EVB_MSE && h->nq == 1) EVB_CUDA(evb_launch_pdl(h->early, k_finalize_pipe<true>, dim3(grid), dim3(256), pipe_smem, h->st, pa));
-        else EVB_CUDA(evb_launch_pdl(h->early, k_finalize_pipe<false>, dim3(grid), dim3(256), pipe_smem, h->st, pa));
+        if (h->p.loss == EVB_MSE && h->nq == 1) EVB_CUDA(evb_launch(k_finalize_pipe<true>, dim3(grid), dim3(256), pipe_smem, h->st, pa));
+        else EVB_CUDA(evb_launch(k_finalize_pipe<false>, dim3(grid), dim3(256), pipe_smem, h->st, pa));
     } else if (mode == 0 && h->RS <= 256 && staged <= 100 * 1024 && !direct && h->dev < 64) {
         const dim3 tiles((unsigned)((h->n + 255) / 256));
 #define EVB_FIN(KT) do { \
             if (staged > 48 * 1024) EVB_CUDA(cudaFuncSetAttribute(k_finalize_staged<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024)); \
-            EVB_CUDA(evb_launch_pdl(h->early, k_finalize_staged<KT>, tiles, dim3(256), staged, h->st, a)); } while (0)
+            EVB_CUDA(evb_launch(k_finalize_staged<KT>, tiles, dim3(256), staged, h->st, a)); } while (0)
         switch (h->K) {
         case 1: EVB_FIN(1); break;
         case 2: EVB_FIN(2); break;
@@ -899,7 +885,7 @@ int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode, void *p
         }
 #undef EVB_FIN
     } else {
-        EVB_CUDA(evb_launch_pdl(h->early, k_finalize, dim3((unsigned)((h->n + 255) / 256)), dim3(256), a.packed_in_smem ? smem : 0, h->st, a));
+        EVB_CUDA(evb_launch(k_finalize, dim3((unsigned)((h->n + 255) / 256)), dim3(256), a.packed_in_smem ? smem : 0, h->st, a));
     }
     evb_toc(h, EVB_T_FINALIZE);
     EVB_CUDA(cudaGetLastError());

@@ -78,8 +78,6 @@ struct BeginArgs {
 // gradients into fixed-point numbers.
 __global__ void __launch_bounds__(256) k_tree_begin(BeginArgs a) {
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-    evb_pdl_next();
-    evb_pdl_wait();
     if (i < a.ngen_js) a.gen_js[i] = __ldcv(a.gen_js_host + i);
     if (a.q.grad) evb_hg::quantize(a.q, i);
     if (a.all_rows && i < a.q.n) a.rows[i] = (uint32_t)i;
@@ -736,8 +734,6 @@ __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_fe
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     const int F = a.F;
     const int Fown = (F - a.rank + a.world - 1) / a.world;
-    evb_pdl_next();
-    evb_pdl_wait();
     if (blockIdx.x == 0 && a.level == 1 && threadIdx.x < a.ng) a.gmax[threadIdx.x] = 0u;
     if (Fown <= 0) return;
     long long gw = (long long)blockIdx.x * wpb + wid;
@@ -773,8 +769,6 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
     __shared__ int s_bin, s_last;
     const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int C = a.C, K = a.K, B = a.B, F = a.F;
-    evb_pdl_next();
-    evb_pdl_wait();
     if (blockIdx.x == 0 && a.level == 1 && threadIdx.x < a.ng) a.gmax[threadIdx.x] = 0u;
     int gw = blockIdx.x;
     const int which = a.level > 1 ? gw & 1 : 0;
@@ -1191,8 +1185,6 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
 __global__ void __launch_bounds__(EVB_PART_THREADS, PART_CTAS) k_partition(PartArgs a) {
     __shared__ uint32_t s_bits[EVB_PART_CHUNK / 32];
     __shared__ int s_pref[EVB_PART_CHUNK / 32], s_misc[34];
-    evb_pdl_next();
-    evb_pdl_wait();
     const int npl = a.plan[a.level].npl, total = a.plan[a.level].total, low = a.hlow ? load_now(reinterpret_cast<const int32_t *>(a.low_any)) : 0;
     {
         const size_t nb = (size_t)a.plan[a.level].nbuild, ns = nb * a.acc_sums, nc = nb * a.acc_cnts;
@@ -1247,7 +1239,7 @@ int32_t evb_launch_tree_begin(evb_handle *h, bool quantize, bool all_rows, const
     if (!quantize) a.q.grad = nullptr;
     const int64_t threads = std::max<int64_t>(quantize || all_rows ? h->n : 0, std::max(a.nids, a.ngen_js));
     evb_tic(h, EVB_T_ROWS_INIT);
-    const cudaError_t e = evb_launch_pdl(h->early, k_tree_begin, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, h->st, a);
+    const cudaError_t e = evb_launch(k_tree_begin, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, h->st, a);
     evb_toc(h, EVB_T_ROWS_INIT);
     EVB_CUDA(e);
     return EVB_OK;
@@ -1317,7 +1309,7 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
     const long long warps = (long long)slots * Fown * (level > 1 ? 2 : 1);
     evb_tic(h, EVB_T_SCAN);
     if (fused && evb_scan_multi(h)) {
-#define EVB_SCAN(M) EVB_CUDA(evb_launch_pdl(h->early, k_scan_multi<M>, dim3((unsigned)warps), dim3(32 * h->K), 0, h->st, a))
+#define EVB_SCAN(M) EVB_CUDA(evb_launch(k_scan_multi<M>, dim3((unsigned)warps), dim3(32 * h->K), 0, h->st, a))
         if (h->B <= 32) EVB_SCAN(1); else if (h->B <= 64) EVB_SCAN(2); else if (h->B <= 128) EVB_SCAN(4); else EVB_SCAN(8);
 #undef EVB_SCAN
     } else if (warps > 0) {
@@ -1325,12 +1317,12 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
         const bool own = h->p.loss >= EVB_MAE;
         const bool obl = h->obl_gain != nullptr;
 #define EVB_SCAN(M) do { \
-            if (own && obl) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, true, true, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else if (own) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, true, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else if (obl) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, true, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else if (h->K == 1 && h->C == 3 && !a.qlow) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, true, false>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else if (h->K == 1 && h->C == 3) EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, true, true>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else EVB_CUDA(evb_launch_pdl(h->early, k_scan_feat<M, false, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); } while (0)
+            if (own && obl) EVB_CUDA(evb_launch(k_scan_feat<M, true, true, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (own) EVB_CUDA(evb_launch(k_scan_feat<M, true, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (obl) EVB_CUDA(evb_launch(k_scan_feat<M, false, true, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (h->K == 1 && h->C == 3 && !a.qlow) EVB_CUDA(evb_launch(k_scan_feat<M, false, false, true, false>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (h->K == 1 && h->C == 3) EVB_CUDA(evb_launch(k_scan_feat<M, false, false, true, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else EVB_CUDA(evb_launch(k_scan_feat<M, false, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); } while (0)
         if (h->B <= 32) EVB_SCAN(1); else if (h->B <= 64) EVB_SCAN(2); else if (h->B <= 128) EVB_SCAN(4); else EVB_SCAN(8);
 #undef EVB_SCAN
     }
@@ -1362,7 +1354,7 @@ int32_t evb_launch_partition(evb_handle *h, int level) {
     const int64_t chunks = (h->n + EVB_PART_THREADS - 1) / EVB_PART_THREADS; // the smallest ones
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(h->num_sms * PART_CTAS, chunks));
     evb_tic(h, EVB_T_PARTITION);
-    const cudaError_t e = evb_launch_pdl(h->early, k_partition, dim3(grid), dim3(EVB_PART_THREADS), 0, h->st, a);
+    const cudaError_t e = evb_launch(k_partition, dim3(grid), dim3(EVB_PART_THREADS), 0, h->st, a);
     evb_toc(h, EVB_T_PARTITION);
     EVB_CUDA(e);
     return EVB_OK;
