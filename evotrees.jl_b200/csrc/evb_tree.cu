@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256) k_peer_reduce(PeerReduceArgs a) {
 // staged histogram `sm` of the build node, stores the node's histogram if its children will need it, scans the
 // bins (`_scan_node!`, fit-utils.jl:403-436) and records the best split of this feature.
 template <int MAXCHK, bool OWN, bool OBL, bool K1, bool LOW>
-__device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int f, uint32_t feat, int slot, bool low, double *s_sum, int lane, bool first_owned) {
+__device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int f, uint32_t feat, int slot, double *s_sum, int lane, bool first_owned) {
     // K1: one output with gradient, hessian and weight channels (C = 3), known at compile time: the loops over the
     // outputs and the channel tests fold away
     const int C = K1 ? 3 : a.C, K = K1 ? 1 : a.K, B = a.B, F = a.F;
@@ -319,18 +319,32 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     const bool keep = n < a.hist_nodes;
     double *__restrict__ hn = a.hist + (size_t)n * FCB;
     if (n == 1) {
-        for (int c = 0; c < C; ++c) {
-            const Chan ch = chan_of(a, c, K, C);
-            long long raw[MAXCHK];
-            chan_load<MAXCHK>(a, ch, slot, f, feat, c, lane, 32, C, raw);
-            double v = 0.0;
-            if (a.qsum) v = chan_total<MAXCHK>(a, ch, slot, feat, LOW && low, lane, 32, raw);
-            else { // sharded: the bins of feature slot 0, in doubles
+        constexpr int NB = K1 ? 3 : 1; // channels whose loads are issued together
+        for (int c0 = 0; c0 < C; c0 += NB) {
+            Chan ch[NB];
+            long long raw[NB][MAXCHK];
 #pragma unroll
-                for (int j = 0; j < MAXCHK; ++j) if (lane + 32 * j < B) v += __longlong_as_double(raw[j]);
-                v = warp_sum(v);
+            for (int u = 0; u < NB; ++u) {
+                ch[u] = chan_of(a, c0 + u, K, C);
+                chan_load<MAXCHK>(a, ch[u], slot, f, feat, c0 + u, lane, 32, C, raw[u]);
             }
-            if (lane == 0) { s_sum[c] = v; if (first_owned) a.nsum[(size_t)C + c] = v; }
+            double v[NB];
+            if (a.qsum) {
+#pragma unroll
+                for (int u = 0; u < NB; ++u) v[u] = chan_total<MAXCHK>(a, ch[u], slot, feat, LOW, lane, 32, raw[u]);
+            } else { // sharded: the bins of feature slot 0, in doubles
+#pragma unroll
+                for (int u = 0; u < NB; ++u) {
+                    v[u] = 0.0;
+#pragma unroll
+                    for (int j = 0; j < MAXCHK; ++j) if (lane + 32 * j < B) v[u] += __longlong_as_double(raw[u][j]);
+                    v[u] = warp_sum(v[u]);
+                }
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int u = 0; u < NB; ++u) { s_sum[c0 + u] = v[u]; if (first_owned) a.nsum[(size_t)C + c0 + u] = v[u]; }
+            }
         }
     } else {
         for (int c = lane; c < C; c += 32) s_sum[c] = a.nsum[(size_t)n * C + c];
@@ -367,7 +381,7 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     auto take = [&](int c, const Raw &r, double (&v)[CH]) {
 #pragma unroll
         for (int j = 0; j < CH; ++j) v[j] = chan_value(a, r.ch, r.b[j]);
-        if (LOW && low) chan_add_low<CH>(a, r.ch, slot, feat, bin0, 1, v);
+        if (LOW) chan_add_low<CH>(a, r.ch, slot, feat, bin0, 1, v);
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
             const int b = bin0 + j;
@@ -745,7 +759,9 @@ __global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_fe
     const bool low = LOW && slot_low(a, min(s, a.slots - 1));
     if (s >= nbuild) return;
     const int n = which ? nb ^ 1 : nb;
-    scan_one<MAXCHK, OWN, OBL, K1, LOW>(a, n, which != 0, f, (uint32_t)feat, s, low, s_sum_all[wid], lane, fi == 0);
+    // two bodies: a test between the loads of the channels costs a level 0.5 us
+    if (LOW && low) scan_one<MAXCHK, OWN, OBL, K1, true>(a, n, which != 0, f, (uint32_t)feat, s, s_sum_all[wid], lane, fi == 0);
+    else scan_one<MAXCHK, OWN, OBL, K1, false>(a, n, which != 0, f, (uint32_t)feat, s, s_sum_all[wid], lane, fi == 0);
     if (!OBL && a.ticket) {
         // the warp that scans the node's last feature decides the node: no launch of its own for that
         unsigned last = 0;
@@ -1185,9 +1201,11 @@ __device__ __forceinline__ void partition_chunks(const PartArgs &a, int b, int G
 __global__ void __launch_bounds__(EVB_PART_THREADS, PART_CTAS) k_partition(PartArgs a) {
     __shared__ uint32_t s_bits[EVB_PART_CHUNK / 32];
     __shared__ int s_pref[EVB_PART_CHUNK / 32], s_misc[34];
-    const int npl = a.plan[a.level].npl, total = a.plan[a.level].total, low = a.hlow ? load_now(reinterpret_cast<const int32_t *>(a.low_any)) : 0;
+    const LevelPlan *plan = a.plan + a.level; // all of it at once
+    const int npl = load_now(&plan->npl), total = load_now(&plan->total), nbuild = load_now(&plan->nbuild);
+    const int low = a.hlow ? load_now(reinterpret_cast<const int32_t *>(a.low_any)) : 0;
     {
-        const size_t nb = (size_t)a.plan[a.level].nbuild, ns = nb * a.acc_sums, nc = nb * a.acc_cnts;
+        const size_t nb = (size_t)nbuild, ns = nb * a.acc_sums, nc = nb * a.acc_cnts;
         const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
         for (size_t i = i0; i < ns; i += st) a.hsum[i] = 0ull;
         if (low) for (size_t i = i0; i < ns; i += st) a.hlow[i] = 0ull;
