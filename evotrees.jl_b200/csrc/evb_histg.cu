@@ -127,9 +127,12 @@ int32_t evb_hg_configure(evb_handle *h) {
     if (g.wper < 1 || most_parts(g.wper) > fit) g.wper = 4;
     g.ngf = (W + g.wper - 1) / g.wper;
     g.wper = std::min(g.wper, g.wper <= 4 ? g.wper : ((W + g.ngf - 1) / g.ngf + 7) & ~7); // the same number of CTAs, evenly filled
-    // fewer rows below the root than the SMs can share (256 each): a CTA takes one part only, its flush is shorter too (60k x 77:
-    // 0.153 -> 0.149 ms per tree; two CTAs of unequal numbers of parts are slower than one)
-    if (h->n / 2 / 256 * g.ngf < h->num_sms && g.wper > 8) g.wper = 8;
+    // Fewer rows below the root than the SMs can share (1024 each): a CTA takes one part only, its flush is shorter too.  ms per tree, all
+    // parts and one: 10k x 77 poisson 0.139 and 0.119, 60k x 77 0.146 and 0.130, 200k x 77 0.166 and 0.157, 600k x 77 0.239 and 0.247;
+    // 100k x 40 logloss 0.142 and 0.131, 200k x 40 0.156 and 0.144, 800k x 40 0.232 and 0.239; 200k x 50 gaussian 0.191 and 0.175, 800k x 50
+    // 0.327 and 0.314; 250k x 100 least squares 0.169 and 0.153.  The lines cross between 300k and 600k rows; this one lies at 303k
+    // where all words fit one CTA, at 152k where they take two.
+    if (h->n / 2 / 1024 * g.ngf < h->num_sms && g.wper > 8) g.wper = 8;
     g.wper = std::min(g.wper, W);
     g.ngf = (W + g.wper - 1) / g.wper;
     g.W = W;
@@ -137,7 +140,9 @@ int32_t evb_hg_configure(evb_handle *h) {
     g.queue = (int)(most * part / 4);
     g.smem = most * part + QUEUE_BYTES;
     g.threads = most * part <= SMEM_TWO ? 512 : 1024;
-    // up to four words a row is cheap: 256 rows are too few for a flush (100k x 10 0.099 -> 0.104 ms per tree)
+    // Up to four words a row is cheap and 256 rows are too few for a flush.  ms per tree with 256 and 512: 100k x 10 least squares 0.099 and
+    // 0.096, 100k x 16 logloss 0.124 and 0.118, 30k x 7 poisson 0.112 and 0.112, but 100k x 12 five classes 0.146 and 0.151; with more
+    // words 60k x 28 five classes 0.149 and 0.160, 100k x 100 0.125 and 0.128, 60k x 77 poisson 0.132 and 0.131, 100k x 28 poisson 0.128 and 0.124
     g.min_rows = g.wper <= 4 ? 512 : 256;
     EVB_CUDA(cudaFuncSetAttribute(k_histg, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     int occ = 0;

@@ -334,7 +334,8 @@ __device__ __forceinline__ void accumulate(const Args &a, uint32_t *smem, uint32
             if constexpr (PACK) break;
             else {
                 if (left_rows == 0u) break;
-                // a global reduction costs about 32 of those in shared memory: a row in 32, or the image
+                // One row in 32, by global reductions; more, through the image.  Lines at one in 8 to 128 are within 3 % of each other (300k x 30
+                // gamma, log-normal target of sigma 0.7 to 2; 60k x 77, sigma 3: 0.157 ms per tree at one in 8, 0.153 at 32, 0.154 at 128).
                 const bool few = left_rows <= QUEUE && left_rows * 32 <= (uint32_t)(pe - pos + a.pad_rows);
                 if (!second && few) add_left<NQ>(a, queue, (int)left_rows, s, two_lb);
                 if (second || few) {
