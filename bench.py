@@ -366,7 +366,7 @@ def main():
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
             "higher_is_better": False, "scaling": "strong", "vs_baseline": None,
             "dtype": ("f32 gradients, exact 24-bit fixed-point sums (u32 reductions in shared memory, 64-bit accumulators), f64 split scan"
-                      if w["loss"] == "mse" else "f32 gradients, exact 31-bit fixed-point sums (u32 reductions in shared memory, 64-bit accumulators), f64 split scan"),
+                      if w["loss"] == "mse" else "f32 gradients, exact sums of them in whole numbers (u32 reductions in shared memory, 64-bit accumulators), f64 split scan"),
             "data": "synthetic",
             "config": {"workload": args.workload, "rows": rows, "feats": feats, "max_depth": depth, "nbins": nbins, "loss": w["loss"], "tree_type": args.tree_type,
                        "eta": w["eta"], "rowsample": w["rowsample"], "colsample": w["colsample"], "rows_per_gpu": nloc,

@@ -610,7 +610,6 @@ extern "C" int32_t evb_grow_tree_end(evb_handle *h, int64_t *feat, uint8_t *cond
         evb_set_error("device self-check failed (code %d: %s)", derr,
                       derr == EVB_DERR_WAIT_FULL ? "bounded wait for staged rows expired"
                       : derr == EVB_DERR_WAIT_EMPTY ? "bounded wait for a free stage expired"
-                      : derr == EVB_DERR_PLAN ? "work list overflow"
                       : derr == EVB_DERR_PEER ? "bounded wait for the other ranks expired" : "unknown");
         cudaMemsetAsync(h->d_err, 0, sizeof(int), h->st);
         return EVB_ERR_DEVICE;

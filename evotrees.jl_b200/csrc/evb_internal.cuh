@@ -26,7 +26,7 @@ void evb_set_error(const char *fmt, ...);
     } while (0)
 
 // device-side error codes written to evb_handle::d_err
-enum { EVB_DERR_NONE = 0, EVB_DERR_WAIT_FULL = 1, EVB_DERR_WAIT_EMPTY = 2, EVB_DERR_BIN_RANGE = 3, EVB_DERR_PLAN = 4, EVB_DERR_PEER = 5, EVB_DERR_NAN = 6 };
+enum { EVB_DERR_NONE = 0, EVB_DERR_WAIT_FULL = 1, EVB_DERR_WAIT_EMPTY = 2, EVB_DERR_BIN_RANGE = 3, EVB_DERR_PEER = 5, EVB_DERR_NAN = 6 };
 
 // ---- geometry constants ---------------------------------------------------------------------------
 constexpr int EVB_TILE_ROWS = 32;    // rows per staged tile (one per producer lane)
@@ -229,7 +229,6 @@ size_t evb_hg_q_words(const evb_handle *h);
 int32_t evb_launch_histg(evb_handle *h, int level);
 int32_t evb_launch_acc_clear(evb_handle *h, int level);
 int32_t evb_launch_acc_to_hcomp(evb_handle *h, int level);
-// The split scan reads the integer accumulators itself unless ranks exchange histograms as doubles.
 // Rows of a level are dealt out to the CTAs of a histogram kernel with this many more for every build node: a flush costs what a
 // few hundred rows do, so a CTA with several small nodes gets fewer rows than one inside a large node.  Per tree, equal ranges
 // and 512 rows at least, then padded ones and 256: 1503 x 7 0.096 -> 0.087 ms, 60k x 77 0.183 -> 0.150, 250k x 33 weighted
@@ -242,6 +241,7 @@ static inline int evb_pad_rows(const evb_handle *h) {
 // more outputs, losses with a gain of their own and oblivious trees (every bin's gain is kept) take one warp per feature.
 #define EVB_MULTI_K 8
 static inline bool evb_scan_multi(const evb_handle *h) { return h->K >= 2 && h->K <= EVB_MULTI_K && h->C == 2 * h->K + 1 && h->p.loss < EVB_MAE && h->p.tree_type != 1; }
+// The split scan reads the integer accumulators itself unless ranks exchange histograms as doubles.
 static inline bool evb_acc_direct(const evb_handle *h) { return h->world == 1; }
 // evb_handle::low, a stretch of 2^(level-1) words per level: its build slots (at most half of them below the root), and in its last
 // word whether any slot has something (the root's only slot says so itself)

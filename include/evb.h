@@ -79,7 +79,8 @@ typedef struct {
     double alphas[8];      /* multiquantile loss / metric: the K target quantiles (src/learners.jl:45); else unused */
 } evb_params;
 
-/* Accumulated device time per kernel class since the last evb_reset_timings (EVB_FLAG_TIMING). */
+/* Accumulated device time per kernel class since the last evb_reset_timings (EVB_FLAG_TIMING).  EVB_T_PLAN and EVB_T_D2H stay zero: the
+ * plan of a level is made by the last CTA of the partition, and the finished tree is written to the host by the last kernel. */
 #define EVB_NTIMERS 12
 enum evb_timer {
     EVB_T_GRADS = 0, EVB_T_ROWS_INIT = 1, EVB_T_HIST = 2, EVB_T_HIST_REDUCE = 3, EVB_T_ALLREDUCE = 4,

@@ -57,16 +57,13 @@ def _gain_of(op, hist_node, nsum_node, feat0, bin1, numeric=True):
     return g - gp
 
 
-SUM_SLACK = 1.0   # multiplies the bound of `_sum_err`; see lockstep_check(float_sum_slack=)
-
-
 def _sum_err(op, nsum_node, gmax):
     """Absolute error allowed on a node's gradient sums: 1e-5 x max|g| x (rows of the node), channel by channel -- the same
-    bound the histogram comparison uses.  It covers the float32 partial sums of the float histogram kernel (whose
-    error grows with the sum of |g| of the rows, not with the possibly much smaller |sum of g|); the fixed-point path is
-    exact to 2^-26 of max|g| and stays far inside it."""
+    bound the histogram comparison uses.  The library's sums are exact (least squares: of gradients rounded to 24 or 29
+    bits below max|g|) and stay far inside it; what it leaves room for are the gradients themselves, whose transcendental
+    functions differ in the last places."""
     C = nsum_node.size
-    return SUM_SLACK * RTOL * np.asarray(gmax, np.float64)[:C] * float(nsum_node[C - 1])
+    return RTOL * np.asarray(gmax, np.float64)[:C] * float(nsum_node[C - 1])
 
 
 def _gain_tol(op, gain, nsum_node, gmax):
@@ -153,9 +150,8 @@ def compare_tree(op, tg, to, ohist, onsum, feattypes=None, gmax=None):
 
 
 def compare_hist(hg, ho, gmax, wmin, wroot):
-    """hg, ho [njs, B, C].  The library accumulates float32 partial sums and gets half of the nodes by
-    parent - sibling subtraction, so its absolute error in a bin is set by the bin's population in the
-    ancestor where the chain of subtractions started (at most the root).  Bound used:
+    """hg, ho [njs, B, C].  Half of the nodes come from parent - sibling subtraction, so the absolute error in a bin is set by the bin's
+    population in the ancestor where the chain of subtractions started (at most the root).  Bound used:
     sum|contribution| <= gmax[c] * (root w_bin / wmin)."""
     wbin = wroot[:, :, -1:]
     atol = RTOL * gmax[None, None, :] * (wbin / wmin) + 1e-12
@@ -166,14 +162,9 @@ def compare_hist(hg, ho, gmax, wmin, wroot):
 
 
 def lockstep_check(pkg, orc, params, x, y, rounds, w=None, feattypes=None, x_bin=None, check_hist=True,
-                   max_diverged_frac=0.02, device=0, hist_nodes=None, float_sum_slack=1.0):
+                   max_diverged_frac=0.02, device=0, hist_nodes=None):
     """Grow `rounds` boosting rounds on the GPU; after each tree, rebuild the same tree with the oracle from
-    the library's own pre-round state and compare everything.  Returns summary statistics.
-    `float_sum_slack` widens the allowed error of the node sums (and what follows from them: gains, leaves) for the
-    float histogram kernel on millions of rows, whose float32 partial sums -- inherited through parent - sibling
-    subtractions -- reach a few 1e-5 of max|g| x rows there; the fixed-point path never needs it."""
-    global SUM_SLACK
-    SUM_SLACK = float(float_sum_slack)
+    the library's own pre-round state and compare everything.  Returns summary statistics."""
     from evotrees_b200 import _lib
     from evotrees_b200.fit import init_target
 
@@ -224,7 +215,7 @@ def lockstep_check(pkg, orc, params, x, y, rounds, w=None, feattypes=None, x_bin
                     assert np.array_equal(cache.nidx(from_partition=True), onidx), "row->node ids from the partition differ"
                     leaf = orc.leaf_idx(x_bin, to, feattypes)
                     assert np.array_equal(cache.nidx(from_partition=False), leaf), "leaf ids from the traversal differ"
-                    # float32 partial sums: the absolute error scales with sum|g| <= gmax * (root rows)
+                    # a child's sums are the parent's minus its sibling's: the absolute error scales with sum|g| <= gmax * (root rows)
                     gs, os_ = cache.node_sums()[to.w != 0], onsum[to.w != 0]
                     atol = RTOL * np.abs(grad).max(axis=0).astype(np.float64) * (onsum[0, -1] / wmin)
                     assert (np.abs(gs - os_) <= RTOL * np.abs(os_) + atol[None, :]).all(), "node sums"

@@ -18,9 +18,6 @@ def test_lockstep_at_benchmark_size(pkg, orc, workload, rounds):
     orc.use_all_cores()
     x, y = bench.make_shard(w, w["rows"], 0, 1)
     params = bench.make_params(pkg, w, nrounds=rounds)
-    # mse runs the fixed-point kernel (exact sums); the other losses run the float kernel, whose float32 partial sums
-    # need ten times the bound at these row counts
-    stats = lockstep_check(pkg, orc, params, x, y, rounds=rounds, check_hist=w["rows"] <= 1_000_000, hist_nodes=8,
-                           float_sum_slack=1.0 if w["loss"] == "mse" else 10.0)
+    stats = lockstep_check(pkg, orc, params, x, y, rounds=rounds, check_hist=w["rows"] <= 1_000_000, hist_nodes=8)
     assert stats["trees"] == rounds and stats["splits"] >= rounds * (2 ** (w["depth"] - 2))
     assert stats["diverged"] <= max(1, stats["nodes_compared"] // 500), stats

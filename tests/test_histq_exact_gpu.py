@@ -1,9 +1,8 @@
-"""The fixed-point histogram path (mse, one target, all features): every histogram of the tree must be EXACTLY the sum
+"""Least squares (one target): every histogram of the tree must be EXACTLY the sum
 of the quantised gradients q = rint(g * 2^s) of the node's rows times 2^-s -- for built nodes (integer partial sums),
 for siblings (parent - built child in f64, exact for multiples of 2^-s) and on any number of row pieces.  The check is
-bit-for-bit on float64, for unit weights (row count riding in the low word) and with weights (four words)."""
+bit-for-bit on float64, for unit weights (row count riding in the low word) and, up to 128 bins, with weights."""
 import math
-import os
 
 import numpy as np
 import pytest
@@ -50,9 +49,8 @@ def test_histograms_are_exact_sums_of_quantised_gradients(pkg, nobs, nfeats, nbi
         # first-round gradients as the device computes them (float32): g = 2 (p - y) w
         w32 = np.ones(nobs, np.float32) if w is None else w
         g = (np.float32(2.0) * (np.float32(mu[0]) - yd.astype(np.float32))).astype(np.float32) * w32
-        # unweighted: the registers-direct kernel quantises to 24 bits (26 when asked to, or when the staged kernel runs)
-        qb = 26 if os.environ.get("EVB_HIST_Q2") == "0" or os.environ.get("EVB_Q2_QBITS") == "26" else 24
-        qg, ginv = _quantise(g, 29 if weighted else qb)
+        # 24 bits below max |g| with the row count in the same words, 29 with weights
+        qg, ginv = _quantise(g, 29 if weighted else 24)
         if weighted:
             qw, winv = _quantise(w32, 29)
         else:
@@ -73,9 +71,9 @@ def test_histograms_are_exact_sums_of_quantised_gradients(pkg, nobs, nfeats, nbi
                 sg = np.zeros(nbins, np.int64); np.add.at(sg, b, qg[rows])
                 sw = np.zeros(nbins, np.int64); np.add.at(sw, b, qw[rows])
                 if weighted and nbins > 128:
-                    # four word planes of 257 bin rows do not fit beside the rings: the float kernel runs instead
-                    tol = 1e-5 * float(np.abs(g).max()) * np.maximum(1, np.bincount(b, minlength=nbins))
-                    assert (np.abs(hg[f, :, 0] - sg.astype(np.float64) * ginv) <= tol).all(), (n, f, "g (float kernel)")
+                    # not rounded: half a step of 29 bits per row lies between the two
+                    tol = 2.0 ** -29 * float(np.abs(g).max()) * np.maximum(1, np.bincount(b, minlength=nbins))
+                    assert (np.abs(hg[f, :, 0] - sg.astype(np.float64) * ginv) <= tol).all(), (n, f, "g")
                     continue
                 assert np.array_equal(hg[f, :, 0], sg.astype(np.float64) * ginv), (n, f, "g")
                 assert np.array_equal(hg[f, :, 2], sw.astype(np.float64) * winv), (n, f, "w")
@@ -86,8 +84,8 @@ def test_histograms_are_exact_sums_of_quantised_gradients(pkg, nobs, nfeats, nbi
         cache.close()
 
 
-def test_float_kernel_is_used_with_a_column_sample(pkg):
-    """With colsample < 1 the unit's bins are not adjacent bytes: the float kernel runs and the model still trains."""
+def test_a_model_trains_with_a_column_sample(pkg):
+    """With colsample < 1 the kernel adds all columns and the scan reads the sampled ones: the model still trains."""
     x, y = make_regression(20_000, 20, seed=5)
     m = pkg.fit(pkg.EvoTreeRegressor(loss="mse", nrounds=5, max_depth=4, nbins=32, colsample=0.5, eta=0.3), x_train=x, y_train=y)
     p = np.asarray(m(x)).reshape(x.shape[0], -1)[:, 0]
