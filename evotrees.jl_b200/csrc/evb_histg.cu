@@ -102,7 +102,7 @@ constexpr size_t SMEM_ONE = 227 * 1024 - QUEUE_BYTES;
 int32_t evb_hg_configure(evb_handle *h) {
     HGeom &g = h->hgeo;
     g.nq = h->nq;
-    g.pack = h->p.loss == EVB_MSE && h->K == 1 && h->unit_w;
+    g.pack = h->p.loss == EVB_MSE && h->nq == 1; // one target, unit weights, hessians left out
     g.cnt = h->unit_w && !g.pack;
     if (g.pack) { g.per = 1; g.ngc = 1; }
     else {
@@ -175,7 +175,7 @@ void evb_hg_quant_args(const evb_handle *h, evb_hg::QuantArgs *a) {
     a->grad = h->grad; a->q = h->use_q2 ? reinterpret_cast<int32_t *>(h->xE) : h->gradq; a->gmax = h->d_gmax; a->qinv = h->d_qinv; a->n = h->n;
     a->q2 = h->use_q2 ? 1 : 0; a->g = h->hgeo; a->signs = h->d_signs;
     // the width that weighted least squares has always had where its fixed-point kernel ran
-    a->bits = h->p.loss == EVB_MSE && h->K == 1 && !h->unit_w && h->B <= 128 && h->F == h->nfeats ? 29 : 0;
+    a->bits = h->p.loss == EVB_MSE && h->Ce == 2 && !h->unit_w && h->B <= 128 && h->F == h->nfeats ? 29 : 0;
 }
 
 int32_t evb_launch_histg(evb_handle *h, int level) {

@@ -353,7 +353,7 @@ size_t q2_smem(int B, int NC, bool tail) { return (size_t)(B + 1) * 2 * q2_ncol(
 // does less for features that do not fill a 16-byte chunk and has the smaller image to flush), and the training predict has
 // to be able to read the chunk rows: tree, leaf values and two tiles of rows within 100 KB.
 bool evb_q2_wanted(const evb_handle *h) {
-    if (h->p.loss != EVB_MSE || h->K != 1 || !h->unit_w) return false;
+    if (h->p.loss != EVB_MSE || h->nq != 1) return false; // (hessians left out as well)
     if (const char *e = getenv("EVB_HIST_Q2")) { if (atoi(e) == 0) return false; }
     else if (h->n < 300000) return false;
     const int words = (h->nfeats + 15) / 16 * 4 + 8;

@@ -80,3 +80,16 @@ def test_level_kernels(pkg, loss, classes, n, F, B, depth, weighted, ncols):
                 assert best <= params.gamma + 1e-5 * scale, (node, best)
     finally:
         cache.close()
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("n", [5_000, 320_000])
+def test_hessians_of_least_squares_can_be_accumulated(pkg, orc, monkeypatch, weighted, n):
+    """EVB_NO_ELISION: the hessian channel of mse is summed like any other instead of rebuilt from the weights."""
+    from tests.parity import lockstep_check
+    monkeypatch.setenv("EVB_NO_ELISION", "1")
+    rng = np.random.default_rng(n)
+    x = rng.random((n, 9)).astype(np.float32)
+    y = (x @ rng.normal(size=9) + 0.1 * rng.normal(size=n)).astype(np.float32)
+    w = rng.uniform(0.25, 3.0, n).astype(np.float32) if weighted else None
+    lockstep_check(pkg, orc, pkg.EvoTreeRegressor(loss="mse", nrounds=2, max_depth=5, nbins=32, eta=0.3), x, y, rounds=2, w=w)
