@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) k_hg_to_hcomp(ConvArgs a) {
                     if (is_w && a.unit_w) v = (double)a.hcnt[cell * a.SC + col];
                     else {
                         v = (double)(long long)a.hsum[(cell * a.nq + ch) * a.SC + col] * unit;
-                        if (low) v += (double)(long long)a.hlow[(cell * a.nq + ch) * a.SC + col] * (unit * a.low_unit);
+                        if (low) v += (double)(long long)a.hlow[(((size_t)s * a.SC + col) * a.nq + ch) * a.B + bin] * (unit * a.low_unit);
                     }
                 }
                 t[bl][lane] = mul * v;

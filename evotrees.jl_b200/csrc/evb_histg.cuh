@@ -43,7 +43,7 @@ struct Args {
     const int32_t *cum, *rbase;
     unsigned long long *hsum; // [slot][bin][nq][SC]
     uint32_t *hcnt;           // [slot][bin][SC]
-    unsigned long long *hlow; // like hsum: sums of what hi and lo leave, of the slots in `low`
+    unsigned long long *hlow; // [slot][SC][nq][bin]: sums of what hi and lo leave, of the slots in `low`
     uint32_t *low;            // [slot of the level] nonzero: hlow holds something; low_any: in any slot
     uint32_t *low_any;
     int hb;                   // bits of hi
@@ -189,7 +189,8 @@ __device__ __forceinline__ void flush_part(const Args &a, bool second, uint32_t 
                 const uint32_t cnt = replicas(c);
                 if (out && cnt != 0u && !second) asm volatile("red.global.add.u32 [%0], %1;" ::"l"(a.hcnt + cell * a.SC + f), "r"(cnt) : "memory");
             }
-            unsigned long long *sums = second ? a.hlow : a.hsum;
+            unsigned long long *sums = second ? a.hlow + (((size_t)slot * a.SC + f) * a.nq + a.ch0) * a.B + bin : a.hsum + (cell * a.nq + a.ch0) * a.SC + f;
+            const size_t step = second ? a.B : a.SC;
             uint32_t hi[NQ], lo[NQ];
 #pragma unroll
             for (int c = 0; c < NQ; ++c) { hi[c] = p[64 * c]; lo[c] = p[64 * c + 32]; }
@@ -197,7 +198,7 @@ __device__ __forceinline__ void flush_part(const Args &a, bool second, uint32_t 
             for (int c = 0; c < NQ; ++c) {
                 p[64 * c] = 0u; p[64 * c + 32] = 0u;
                 const long long sum = replicas(((long long)(int32_t)hi[c] << (a.hb + 1)) + (long long)(int32_t)lo[c]);
-                if (out && sum != 0) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(sums + (cell * a.nq + a.ch0 + c) * a.SC + f), "l"(sum) : "memory");
+                if (out && sum != 0) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(sums + c * step), "l"(sum) : "memory");
             }
         }
     }
@@ -230,10 +231,10 @@ __device__ __forceinline__ void add_left(const Args &a, const uint32_t *queue, i
         }
         const uint8_t *x = a.xT + (size_t)rid * a.RS + f0;
         for (int f = lane; f < nf; f += 32) {
-            const size_t cell = (size_t)slot * a.B + (__ldg(x + f) - 1);
+            unsigned long long *d = a.hlow + (((size_t)slot * a.SC + f0 + f) * a.nq + a.ch0) * a.B + (__ldg(x + f) - 1);
 #pragma unroll
             for (int c = 0; c < NQ; ++c)
-                if (v[c] != 0) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(a.hlow + (cell * a.nq + a.ch0 + c) * a.SC + f0 + f), "l"(v[c]) : "memory");
+                if (v[c] != 0) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(d + (size_t)c * a.B), "l"(v[c]) : "memory");
         }
     }
 }

@@ -148,7 +148,7 @@ struct evb_handle {
     int SC;               // feature columns per bin of the accumulators
     unsigned long long *hsum_q;   // [maxslots][B][nq][SC] sums of q per build slot
     uint32_t *hcnt_q;             // [maxslots][B][SC] row counts
-    unsigned long long *hlow_q;   // like hsum_q: what the words of a row leave (null: packed words leave nothing)
+    unsigned long long *hlow_q;   // [maxslots][SC][nq][B] sums of what the words of a row leave (null: packed words leave nothing)
     uint32_t *low;                // [nn+2] build slots of a level that have something in hlow_q (evb_low_slot, evb_low_any)
 
     // register-direct variant (mse, one target, unit weights, many rows): rows as 16-byte chunks + {q, tail bins} per row

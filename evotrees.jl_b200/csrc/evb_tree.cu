@@ -134,7 +134,7 @@ struct ScanArgs {
     const unsigned long long *qsum;
     const uint32_t *qcnt;
     const double *qinv;
-    const unsigned long long *qlow; // like qsum, low_unit times as fine: of the build slots in `low`
+    const unsigned long long *qlow; // [slot][SC][channel][bin], low_unit times as fine as qsum: of the build slots in `low`
     const uint32_t *low;
     double low_unit;
     int SC, nq, unit_w;
@@ -242,17 +242,20 @@ __device__ __forceinline__ void chan_load(const ScanArgs &a, const Chan &ch, int
 __device__ __forceinline__ double chan_value(const ScanArgs &a, const Chan &ch, long long raw) {
     return a.qsum ? (double)raw * ch.mul : __longlong_as_double(raw);
 }
-// the build slot has sums below those of qsum; few have, so what they hold is fetched where it is added and not ahead
+// The build slot has sums below those of qsum, bin after bin so that a scan reads whole sectors (in the layout of qsum, 32 bytes for
+// every 8 used, they cost a scan half of its time again: 1.6M x 69, 255 bins 0.147 -> 0.217 ms per tree).
 __device__ __forceinline__ bool slot_low(const ScanArgs &a, int slot) { return a.qlow && load_now(reinterpret_cast<const int32_t *>(a.low) + slot) != 0; }
 template <int N>
-__device__ __forceinline__ void chan_add_low(const ScanArgs &a, const Chan &ch, int slot, uint32_t feat, int b0, int stride, double (&v)[N]) {
-    if (ch.cnt) return;
-    const unsigned long long *p = a.qlow + ((size_t)slot * a.B * a.nq + ch.idx) * a.SC + feat;
-    long long raw[N];
+__device__ __forceinline__ void chan_load_low(const ScanArgs &a, const Chan &ch, int slot, uint32_t feat, int b0, int stride, long long (&raw)[N]) {
+    const unsigned long long *p = a.qlow + (((size_t)slot * a.SC + feat) * a.nq + (ch.cnt ? 0 : ch.idx)) * a.B;
 #pragma unroll
-    for (int j = 0; j < N; ++j) raw[j] = (long long)__ldg(p + (size_t)min(b0 + j * stride, a.B - 1) * a.nq * a.SC);
+    for (int j = 0; j < N; ++j) raw[j] = (long long)__ldg(p + min(b0 + j * stride, a.B - 1));
+}
+template <int N>
+__device__ __forceinline__ void chan_add_low(const ScanArgs &a, const Chan &ch, const long long (&raw)[N], double (&v)[N]) {
+    const double unit = ch.cnt ? 0.0 : ch.mul * a.low_unit; // (row counts have none: whatever was loaded is finite)
 #pragma unroll
-    for (int j = 0; j < N; ++j) v[j] += (double)raw[j] * (ch.mul * a.low_unit);
+    for (int j = 0; j < N; ++j) v[j] += (double)raw[j] * unit;
 }
 
 // Root sum of a channel from the whole numbers of the bins of any feature, raw[j]: bin b0 + j * stride (every sampled row has
@@ -265,9 +268,9 @@ __device__ __forceinline__ double chan_total(const ScanArgs &a, const Chan &ch, 
     for (int j = 0; j < N; ++j) if (b0 + j * stride < a.B) t += raw[j];
     double v = (double)warp_sum(t) * ch.mul;
     if (low && !ch.cnt) {
-        const unsigned long long *p = a.qlow + ((size_t)slot * a.B * a.nq + ch.idx) * a.SC + feat;
+        const unsigned long long *p = a.qlow + (((size_t)slot * a.SC + feat) * a.nq + ch.idx) * a.B;
         t = 0;
-        for (int j = 0; j < N; ++j) if (b0 + j * stride < a.B) t += (long long)__ldg(p + (size_t)(b0 + j * stride) * a.nq * a.SC);
+        for (int j = 0; j < N; ++j) if (b0 + j * stride < a.B) t += (long long)__ldg(p + b0 + j * stride);
         v += (double)warp_sum(t) * (ch.mul * a.low_unit);
     }
     return v;
@@ -369,10 +372,11 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     const bool elide = a.elide_h != 0; // mse: every h entry is exactly twice the w entry (src/loss.jl:52), it is not read
     // entries of channel c in the lane's bins: the loads (`fetch`) run ahead of their use (`take`), which subtracts from the
     // parent's histogram and keeps the result for the children
-    struct Raw { Chan ch; long long b[CH]; double p[CH]; };
+    struct Raw { Chan ch; long long b[CH], low[LOW ? CH : 1]; double p[CH]; };
     auto fetch = [&](int c, Raw &r) {
         r.ch = chan_of(a, c, K, C);
         chan_load<CH>(a, r.ch, slot, f, feat, c, bin0, 1, C, r.b);
+        if constexpr (LOW) chan_load_low<CH>(a, r.ch, slot, feat, bin0, 1, r.low);
         if (sub) {
 #pragma unroll
             for (int j = 0; j < CH; ++j) r.p[j] = __ldg(hp + fo + (size_t)c * B + min(bin0 + j, B - 1));
@@ -381,7 +385,7 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
     auto take = [&](int c, const Raw &r, double (&v)[CH]) {
 #pragma unroll
         for (int j = 0; j < CH; ++j) v[j] = chan_value(a, r.ch, r.b[j]);
-        if (LOW) chan_add_low<CH>(a, r.ch, slot, feat, bin0, 1, v);
+        if constexpr (LOW) chan_add_low<CH>(a, r.ch, r.low, v);
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
             const int b = bin0 + j;
@@ -658,7 +662,11 @@ __device__ __forceinline__ void node_select(const ScanArgs &a, int n, double *s_
                 if (a.world == 1) {
 #pragma unroll
                     for (int j = 0; j < MAXCHK; ++j) built[j] = chan_value(a, ch[u], rb[u][j]);
-                    if (low) chan_add_low<MAXCHK>(a, ch[u], slot_n, feat, lane, 32, built);
+                    if (low) {
+                        long long raw[MAXCHK];
+                        chan_load_low<MAXCHK>(a, ch[u], slot_n, feat, lane, 32, raw);
+                        chan_add_low<MAXCHK>(a, ch[u], raw, built);
+                    }
                 }
 #pragma unroll
                 for (int j = 0; j < MAXCHK; ++j) {
@@ -831,9 +839,13 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
             hl[j] = elide ? 0.0 : chan_value(a, chs, rh[j]);
         }
         if (low) {
-            chan_add_low<CH>(a, cw, s, feat, bin0, 1, wl);
-            chan_add_low<CH>(a, cg, s, feat, bin0, 1, gl);
-            if (!elide) chan_add_low<CH>(a, chs, s, feat, bin0, 1, hl);
+            long long lw[CH], lg[CH], lh[CH];
+            chan_load_low<CH>(a, cw, s, feat, bin0, 1, lw);
+            chan_load_low<CH>(a, cg, s, feat, bin0, 1, lg);
+            chan_load_low<CH>(a, chs, s, feat, bin0, 1, lh);
+            chan_add_low<CH>(a, cw, lw, wl);
+            chan_add_low<CH>(a, cg, lg, gl);
+            if (!elide) chan_add_low<CH>(a, chs, lh, hl);
         }
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
