@@ -749,8 +749,12 @@ __global__ void __launch_bounds__(256) k_scan_node(ScanArgs a) {
 // independent, so even the root level (one node) spreads over many SMs.
 // OWN: the loss brings its own split gain (mae, credibility); OBL: oblivious trees, the gain of every candidate is
 // stored as well; LOW: histograms may have a second set of sums (ScanArgs::qlow).  The default instance carries none of that code.
+// Registers: with both sets of sums the loads of three channels are in flight twice, and a compiler that is short of registers waits
+// for them one after the other.  ms of scans per tree with 64 and 80 (64 bins): 3M x 20 poisson 0.087 and 0.078, 60k x 77 0.074 and 0.072;
+// with 128 and 170, in CTAs of half the size: 1M x 40 gamma, 128 bins 0.097 and 0.087, 2M x 10 logloss, 255 bins 0.141 and 0.126.
+constexpr int scan_threads(int CH, bool K1, bool LOW) { return K1 && LOW && CH > 2 ? 128 : 256; }
 template <int MAXCHK, bool OWN, bool OBL, bool K1, bool LOW>
-__global__ void __launch_bounds__(256, MAXCHK <= 2 ? (K1 ? 4 : 3) : 2) k_scan_feat(ScanArgs a) {
+__global__ void __launch_bounds__(scan_threads(MAXCHK, K1, LOW), MAXCHK <= 2 ? (K1 && !LOW ? 4 : 3) : K1 && LOW ? 3 : 2) k_scan_feat(ScanArgs a) {
     constexpr int NCH = K1 ? 3 : 72;
     __shared__ double s_sum_all[8][NCH], s_left_all[8][NCH], s_right_all[8][NCH];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
@@ -1343,7 +1347,7 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
         if (h->B <= 32) EVB_SCAN(1); else if (h->B <= 64) EVB_SCAN(2); else if (h->B <= 128) EVB_SCAN(4); else EVB_SCAN(8);
 #undef EVB_SCAN
     } else if (warps > 0) {
-        const unsigned grid = (unsigned)((warps + 7) / 8);
+        const unsigned grid = (unsigned)((warps + 7) / 8), few = (unsigned)((warps + 3) / 4);
         const bool own = h->p.loss >= EVB_MAE;
         const bool obl = h->obl_gain != nullptr;
 #define EVB_SCAN(M) do { \
@@ -1351,7 +1355,7 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
             else if (own) EVB_CUDA(evb_launch(k_scan_feat<M, true, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
             else if (obl) EVB_CUDA(evb_launch(k_scan_feat<M, false, true, false, true>, dim3(grid), dim3(256), 0, h->st, a)); \
             else if (h->K == 1 && h->C == 3 && !a.qlow) EVB_CUDA(evb_launch(k_scan_feat<M, false, false, true, false>, dim3(grid), dim3(256), 0, h->st, a)); \
-            else if (h->K == 1 && h->C == 3) EVB_CUDA(evb_launch(k_scan_feat<M, false, false, true, true>, dim3(grid), dim3(256), 0, h->st, a)); \
+            else if (h->K == 1 && h->C == 3) EVB_CUDA(evb_launch(k_scan_feat<M, false, false, true, true>, dim3(scan_threads(M, true, true) == 128 ? few : grid), dim3(scan_threads(M, true, true)), 0, h->st, a)); \
             else EVB_CUDA(evb_launch(k_scan_feat<M, false, false, false, true>, dim3(grid), dim3(256), 0, h->st, a)); } while (0)
         if (h->B <= 32) EVB_SCAN(1); else if (h->B <= 64) EVB_SCAN(2); else if (h->B <= 128) EVB_SCAN(4); else EVB_SCAN(8);
 #undef EVB_SCAN
