@@ -41,7 +41,8 @@ def test_histograms_keep_small_gradients(pkg, loss, classes, n, F, B, depth, sig
     try:
         C = 2 * K + 1
         js = np.sort(rng.permutation(F)[:ncols]).astype(np.uint32) + 1
-        pkg.grow_tree(cache, params, None, js, update_grads=True)     # leaves the gradients of the next round
+        for _ in range(3):                                            # the fourth tree is a replay of the second one's graph
+            pkg.grow_tree(cache, params, None, js, update_grads=True)
         g = cache.grads().reshape(n, C).astype(np.float64)
         t = pkg.grow_tree(cache, params, None, js, update_grads=True)
         nid = cache.nidx(from_partition=True).astype(np.int64)
