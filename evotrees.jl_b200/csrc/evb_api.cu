@@ -148,7 +148,7 @@ static void free_handle(evb_handle *h) {
     evb_dev_free(h->hsum);
     if (exported) { evb_dev_free(h->hcomp, true); h->hcomp = nullptr; }
     free_eval(h);
-    void *ptrs[] = {h->xH, h->xE, h->hsum_q, h->hcnt_q, h->hlow_q, h->low, h->d_signs, h->qs_cnt, h->qs_prefix, h->qs_rank, h->qs_gamma, h->gradq, h->d_gmax, h->d_qinv, h->cur_l, h->cur_r, h->ticket, h->pl, h->xT, h->xC, h->grad, h->pred, h->y, h->nidx, h->rows[0], h->rows[1], h->mask_d, h->feattypes_d, h->mono_d,
+    void *ptrs[] = {h->xH, h->xE, h->hsum_q, h->hcnt_q, h->hlow_q, h->g_sum, h->g_low, h->g_cnt, h->g_best, h->g_bar, h->low, h->d_signs, h->qs_cnt, h->qs_prefix, h->qs_rank, h->qs_gamma, h->gradq, h->d_gmax, h->d_qinv, h->cur_l, h->cur_r, h->ticket, h->pl, h->xT, h->xC, h->grad, h->pred, h->y, h->nidx, h->rows[0], h->rows[1], h->mask_d, h->feattypes_d, h->mono_d,
                     h->gen_d, h->seg_start, h->seg_cnt, h->kind,
                     h->bslot, h->nsum, h->plan /* base of the tree block */, h->cum, h->slot_node, h->scan_tmp, h->hist, h->hcomp, h->fbest_gain, h->fbest_bin, h->fbest_left, h->obl_gain, h->obl_best, h->edges_d};
     phase("exchange buffers");
@@ -222,7 +222,7 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
         EVB_CUDA(dalloc(&h->xT, (size_t)n * h->RS));
         EVB_CUDA(dalloc(&h->gradq, evb_hg_q_words(h)));
     }
-    EVB_CUDA(dalloc(&h->d_gmax, (size_t)h->nq));
+    EVB_CUDA(dalloc(&h->d_gmax, (size_t)h->nq * 2));
     EVB_CUDA(dalloc(&h->d_qinv, (size_t)h->nq));
     EVB_CUDA(dalloc(&h->d_signs, (size_t)h->nq));
     EVB_CUDA(dalloc(&h->low, (size_t)nids));
@@ -287,11 +287,22 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
             EVB_CUDA(cudaMemsetAsync(h->hlow_q, 0, acc * h->nq * sizeof(unsigned long long), h->st));
         }
     }
+    evb_grow_configure(h);
+    if (h->grow.on) {
+        EVB_CUDA(dalloc(&h->g_sum, 2 * evb_grow_sums(h))); EVB_CUDA(dalloc(&h->g_cnt, 2 * evb_grow_cnts(h))); EVB_CUDA(dalloc(&h->g_best, 2 * evb_grow_best(h)));
+        EVB_CUDA(dalloc(&h->g_bar, (size_t)2));
+        EVB_CUDA(cudaMemsetAsync(h->g_sum, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st));
+        EVB_CUDA(cudaMemsetAsync(h->g_cnt, 0, 2 * evb_grow_cnts(h) * sizeof(uint32_t), h->st));
+        if (!h->hgeo.pack) {
+            EVB_CUDA(dalloc(&h->g_low, 2 * evb_grow_sums(h)));
+            EVB_CUDA(cudaMemsetAsync(h->g_low, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st));
+        }
+    }
 
     // ---- uploads: x_bin is kept feature-major (as given) for the row partition and transposed on the device to
     // observation-major rows for the histogram gathers and the tree traversal
     phase("allocations");
-    EVB_CUDA(dalloc(&h->xC, (size_t)n * nfeats));
+    EVB_CUDA(dalloc(&h->xC, (size_t)n * nfeats + 8)); // k_grow reads whole words
     if (h->use_q2) {
         EVB_CUDA(dalloc(&h->xH, (size_t)(n + 1) * h->q2.RSH));
         EVB_CUDA(dalloc(&h->xE, (size_t)n + 1));
@@ -457,11 +468,15 @@ extern "C" int32_t evb_comm_init(evb_handle *h, const uint8_t id[128], int32_t r
 static int32_t enqueue_tree(evb_handle *h, int use_mask, uint8_t mask_cond, bool run_grads, bool quantize, bool fuse, int slot) {
     const int D = h->D;
     if (run_grads) EVB_CHECK(evb_launch_grads(h));
-    EVB_CHECK(evb_launch_tree_begin(h, quantize, use_mask == EVB_MASK_NONE, h->h_js[slot]));
+    const bool whole = evb_grows_whole(h);
+    if (evb_one_launch(h, use_mask != EVB_MASK_NONE)) return evb_launch_grow(h, false, mask_cond, slot, fuse);
+    EVB_CHECK(evb_launch_tree_begin(h, quantize && !whole, use_mask == EVB_MASK_NONE, h->h_js[slot]));
+    if (whole && !use_mask) return evb_launch_grow(h, false, mask_cond, slot, fuse);
     EVB_CHECK(evb_launch_rows_init(h, use_mask, mask_cond));
+    if (whole) EVB_CHECK(evb_launch_grow(h, true, mask_cond, slot, fuse));
     const int last = D > 1 ? D - 1 : 1;
     const bool full_part = (h->p.flags & EVB_FLAG_FULL_PARTITION) != 0;
-    for (int level = 1; level <= last; ++level) {
+    for (int level = 1; !whole && level <= last; ++level) {
         EVB_CHECK(h->use_q2 ? evb_launch_histq2(h, level) : evb_launch_histg(h, level));
         if (!evb_acc_direct(h)) EVB_CHECK(evb_launch_acc_to_hcomp(h, level));
         if (h->world > 1 && !h->p2p) { // with peer access the ranks' histograms are summed inside the split scan instead
@@ -514,6 +529,7 @@ static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen,
         EVB_CUDA(cudaStreamSynchronize(h->st));
         h->F = njs;
         h->gradq_valid = false; // how g is rounded may depend on it
+        if (h->g_sum) evb_grow_configure(h);
         drop_graphs(h);
     }
     if (update_grads) h->bag_idx = 0;
@@ -539,7 +555,7 @@ static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen,
     if (update_grads) h->gradq_valid = false;
     const bool quantize = !h->gradq_valid;
     if (quantize) h->gradq_valid = true;
-    const int key = (use_mask ? 1 : 0) | (use_mask == EVB_MASK_PCG ? 32 : 0) | (run_grads ? 2 : 0) | (fuse ? 4 : 0) | (slot ? 8 : 0) | (quantize ? 16 : 0);
+    const int key = (use_mask ? 1 : 0) | (use_mask == EVB_MASK_PCG ? 32 : 0) | (run_grads ? 2 : 0) | (fuse ? 4 : 0) | (slot ? 8 : 0) | (quantize ? 16 : 0) | (h->gmax_sel ? 64 : 0);
     if (h->graph_mask_cond != (int)mask_cond) { drop_graphs(h); h->graph_mask_cond = mask_cond; }
     bool launched = false;
     // Sharded runs over NCCL stay on direct launches: a run that captured the NCCL collectives into the graph did not
@@ -547,7 +563,7 @@ static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen,
     // library's own kernels (the barrier counts on the device), which replay like any other.
     // (The quantile losses add their leaves' digit counts with NCCL on every sharded path.)
     const bool quantile_leaves = h->p.loss == EVB_QUANTILE || h->p.loss == EVB_MULTIQUANTILE;
-    if (h->use_graphs && !h->timing && (h->world == 1 || (h->p2p && !quantile_leaves))) {
+    if (h->use_graphs && !h->timing && !evb_one_launch(h, use_mask != EVB_MASK_NONE) && (h->world == 1 || (h->p2p && !quantile_leaves))) {
         if (!h->graph[key] && h->tree_seq >= 1) { // the very first tree of a handle always runs directly
             int64_t before[EVB_NTIMERS];
             memcpy(before, h->tm.launches, sizeof(before));
@@ -575,6 +591,7 @@ static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen,
     h->graph_calls[key] += 1;
     if (h->timing) cudaEventRecord(h->ev_tot[1], h->st);
     EVB_CUDA(cudaEventRecord(h->ev_done[slot], h->st));
+    if (evb_grows_whole(h) && fuse) h->gmax_sel ^= 1;
     h->grads_fresh = fuse;
     h->bag_idx += 1;
     h->tree_seq += 1;
@@ -610,8 +627,16 @@ extern "C" int32_t evb_grow_tree_end(evb_handle *h, int64_t *feat, uint8_t *cond
         evb_set_error("device self-check failed (code %d: %s)", derr,
                       derr == EVB_DERR_WAIT_FULL ? "bounded wait for staged rows expired"
                       : derr == EVB_DERR_WAIT_EMPTY ? "bounded wait for a free stage expired"
+                      : derr == EVB_DERR_GRID ? "bounded wait for the other CTAs of a tree expired"
                       : derr == EVB_DERR_PEER ? "bounded wait for the other ranks expired" : "unknown");
         cudaMemsetAsync(h->d_err, 0, sizeof(int), h->st);
+        if (h->g_sum) { // a tree that was given up leaves its sums
+            cudaMemsetAsync(h->g_bar, 0, 2 * sizeof(uint32_t), h->st);
+            cudaMemsetAsync(h->low, 0, sizeof(uint32_t) * (h->nn + 2), h->st);
+            cudaMemsetAsync(h->g_sum, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st);
+            cudaMemsetAsync(h->g_cnt, 0, 2 * evb_grow_cnts(h) * sizeof(uint32_t), h->st);
+            if (h->g_low) cudaMemsetAsync(h->g_low, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st);
+        }
         return EVB_ERR_DEVICE;
     }
     memcpy(h->last_eval, hb + L.evsum, sizeof(h->last_eval));
@@ -650,7 +675,7 @@ static int32_t eval_attach_impl(evb_handle *h, int64_t nobs, const uint8_t *x_bi
     h->ev_blocks = (int)std::min<int64_t>((nobs + 255) / 256, (int64_t)h->num_sms * 8);
     EVB_CUDA(dalloc(&h->ev_xT, (size_t)nobs * h->RS));
     EVB_CUDA(dalloc(&h->ev_pred, (size_t)nobs * K));
-    EVB_CUDA(dalloc(&h->ev_part, (size_t)h->ev_blocks * 2));
+    EVB_CUDA(dalloc(&h->ev_part, (size_t)std::max(h->ev_blocks, h->num_sms) * 2));
     const size_t ybytes = (size_t)nobs * (h->y_dtype == EVB_U32 ? 4 : 4 * (size_t)h->ycols);
     EVB_CUDA(evb_dev_alloc(&h->ev_y, ybytes));
     EVB_CHECK(evb_h2d_staged(h->ev_y, y, ybytes, h->st, false));

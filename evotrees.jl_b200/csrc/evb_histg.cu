@@ -171,11 +171,13 @@ void evb_hg_args(const evb_handle *h, int level, evb_hg::Args *a) {
     a->TE = h->hgeo.TE; a->min_rows = h->hgeo.min_rows; a->pad_rows = evb_pad_rows(h); a->n = h->n;
 }
 
+// the width that weighted least squares has always had where its fixed-point kernel ran
+int evb_hg_round_bits(const evb_handle *h) { return h->p.loss == EVB_MSE && h->Ce == 2 && !h->unit_w && h->B <= 128 && h->F == h->nfeats ? 29 : 0; }
+
 void evb_hg_quant_args(const evb_handle *h, evb_hg::QuantArgs *a) {
-    a->grad = h->grad; a->q = h->use_q2 ? reinterpret_cast<int32_t *>(h->xE) : h->gradq; a->gmax = h->d_gmax; a->qinv = h->d_qinv; a->n = h->n;
+    a->grad = h->grad; a->q = h->use_q2 ? reinterpret_cast<int32_t *>(h->xE) : h->gradq; a->gmax = evb_gmax(h, false); a->qinv = h->d_qinv; a->n = h->n;
     a->q2 = h->use_q2 ? 1 : 0; a->g = h->hgeo; a->signs = h->d_signs;
-    // the width that weighted least squares has always had where its fixed-point kernel ran
-    a->bits = h->p.loss == EVB_MSE && h->Ce == 2 && !h->unit_w && h->B <= 128 && h->F == h->nfeats ? 29 : 0;
+    a->bits = evb_hg_round_bits(h);
 }
 
 int32_t evb_launch_histg(evb_handle *h, int level) {

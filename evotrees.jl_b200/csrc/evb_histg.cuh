@@ -402,32 +402,37 @@ __device__ __forceinline__ int32_t quant(const Quant &k, float g, unsigned *sign
     const float v = g > 0.0f ? 2.0f : -2.0f;
     return k.back == 0.0f ? (int32_t)v : __float_as_int(v * k.back);
 }
+// how a channel's values become words, and the unit of its sums; bits: of its largest magnitude
+__device__ __forceinline__ Quant quant_of(unsigned bits, bool pack, int hb, int round_bits, double *unit) {
+    auto pow2 = [](int e) { return __int_as_float((e + 127) << 23); };
+    const int ub = pack ? 24 : 2 * hb + 1; // bits of a sum's unit below max |g|
+    Quant k = {1.0f, 0.0f, QK_FLOAT};      // (a channel of zeros: any scale)
+    *unit = 1.0;
+    if (bits - 1u < 0x7f7fffffu) {
+        // max |g| = f 2^e, f in [0.5, 1); a channel of denormals keeps its scale inside the range of a float
+        const int e = max((int)(bits >> 23), 1) - 126, top = pack ? 24 : hb, s = min(top - e, 127);
+        k.sc = pow2(s);
+        if (pack) k.kind = QK_INT;
+        else if (round_bits) {
+            const int sr = min(round_bits - e, 127);
+            k = {pow2(sr), pow2(s - sr), QK_ROUND};
+        }
+        *unit = __longlong_as_double((long long)(1023 - (s + ub - top)) << 52);
+    } else if (bits != 0u) {
+        k.kind = QK_INF;
+        k.back = pack ? 0.0f : pow2(-(hb + 1)); // in units of lo
+        *unit = bits == 0x7f800000u ? DBL_MAX : __longlong_as_double(0x7ff8000000000000ll);
+    }
+    return k;
+}
 // row i of the grid's rows (blocks of adjacent rows); every thread of the block calls it
 __device__ __forceinline__ void quantize(const QuantArgs &a, long long i) {
     __shared__ Quant s_k[EVB_MAX_Q];
     __shared__ float s_sc[EVB_MAX_Q];
-    auto pow2 = [](int e) { return __int_as_float((e + 127) << 23); };
     bool ok = true;
     for (int c = threadIdx.x; c < a.g.nq; c += blockDim.x) {
-        const unsigned bits = a.gmax[c];
-        const int unit = a.g.pack ? 24 : 2 * a.g.hb + 1; // bits of a sum's unit below max |g|
-        Quant k = {1.0f, 0.0f, QK_FLOAT};                // (a channel of zeros: any scale)
-        double inv = 1.0;
-        if (bits - 1u < 0x7f7fffffu) {
-            // max |g| = f 2^e, f in [0.5, 1); a channel of denormals keeps its scale inside the range of a float
-            const int e = max((int)(bits >> 23), 1) - 126, top = a.g.pack ? 24 : a.g.hb, s = min(top - e, 127);
-            k.sc = pow2(s);
-            if (a.g.pack) k.kind = QK_INT;
-            else if (a.bits) {
-                const int sr = min(a.bits - e, 127);
-                k = {pow2(sr), pow2(s - sr), QK_ROUND};
-            }
-            inv = __longlong_as_double((long long)(1023 - (s + unit - top)) << 52);
-        } else if (bits != 0u) {
-            k.kind = QK_INF;
-            k.back = a.g.pack ? 0.0f : pow2(-(a.g.hb + 1)); // in units of lo
-            inv = bits == 0x7f800000u ? DBL_MAX : __longlong_as_double(0x7ff8000000000000ll);
-        }
+        double inv;
+        const Quant k = quant_of(a.gmax[c], a.g.pack != 0, a.g.hb, a.bits, &inv);
         s_k[c] = k;
         s_sc[c] = k.sc;
         ok = k.kind == QK_FLOAT;

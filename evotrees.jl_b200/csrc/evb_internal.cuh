@@ -26,7 +26,7 @@ void evb_set_error(const char *fmt, ...);
     } while (0)
 
 // device-side error codes written to evb_handle::d_err
-enum { EVB_DERR_NONE = 0, EVB_DERR_WAIT_FULL = 1, EVB_DERR_WAIT_EMPTY = 2, EVB_DERR_BIN_RANGE = 3, EVB_DERR_PEER = 5, EVB_DERR_NAN = 6 };
+enum { EVB_DERR_NONE = 0, EVB_DERR_WAIT_FULL = 1, EVB_DERR_WAIT_EMPTY = 2, EVB_DERR_BIN_RANGE = 3, EVB_DERR_PEER = 5, EVB_DERR_NAN = 6, EVB_DERR_GRID = 7 };
 
 // ---- geometry constants ---------------------------------------------------------------------------
 constexpr int EVB_TILE_ROWS = 32;    // rows per staged tile (one per producer lane)
@@ -67,6 +67,14 @@ struct HGeom {
     int pack, cnt;      // packed words of unit-weight least squares; a plane of row counts in channel group 0
     int hb, TE, min_rows, threads, G;
     int queue;          // 32-bit words of shared memory before the row queue
+    size_t smem;
+};
+
+// geometry of the kernel that grows a whole tree (evb_grow.cu)
+struct GrowGeom {
+    bool on;
+    int lw, NG, NR, rpc; // log2 of the words of four features a CTA takes; CTAs side by side: feature groups x row ranges; rows of a range
+    int fit, hb;         // images in shared memory; bits of the high words
     size_t smem;
 };
 
@@ -142,7 +150,8 @@ struct evb_handle {
     int nq, ng;           // quantised channels; those of them that change from round to round (all but the weight)
     HGeom hgeo;
     int32_t *gradq;       // words of all rows, channel group by channel group
-    unsigned *d_gmax;     // [nq] bits of max |g| over the rows, filled by the gradient kernels
+    unsigned *d_gmax;     // [2][nq] bits of max |g| over the rows, filled by the gradient kernels
+    int gmax_sel;         // which of the two belongs to the gradients in place (evb_gmax)
     double *d_qinv;       // [nq] unit of every channel's sums
     unsigned *d_signs;    // [nq] signs of the infinities a channel has had (QuantArgs::signs)
     int SC;               // feature columns per bin of the accumulators
@@ -160,6 +169,13 @@ struct evb_handle {
     // quantile loss: work memory of the per-leaf order-statistic selection
     uint32_t *qs_cnt, *qs_prefix, *qs_rank; float *qs_gamma;
 
+    // whole trees in one launch
+    GrowGeom grow;
+    unsigned long long *g_sum, *g_low; // [2][maxslots][nfeats][nq][B]
+    uint32_t *g_cnt;                   // [2][maxslots][nfeats][B]
+    double2 *g_best;
+    uint32_t *g_bar;
+
     // histograms
     double *hist;     // [2^(D-2) nodes][F][C][B] retained for the subtraction trick
     int hist_nodes;   // nodes with id < hist_nodes are retained
@@ -172,9 +188,9 @@ struct evb_handle {
     int tree_seq, pending;          // trees started / started but not yet collected
     // one CUDA graph per variant of the per-tree launch sequence (mask, gradients first, gradients fused, slot)
     bool use_graphs;
-    cudaGraphExec_t graph[64];
-    int graph_calls[64];
-    int64_t graph_launches[64][EVB_NTIMERS];
+    cudaGraphExec_t graph[128];
+    int graph_calls[128];
+    int64_t graph_launches[128][EVB_NTIMERS];
     int graph_mask_cond;
 
     // multi-GPU
@@ -225,6 +241,7 @@ int32_t evb_upload_binarize(evb_handle *h, const void *x, int32_t dtype, const v
 int evb_hist_mode_env();
 // evb_histg.cu
 int32_t evb_hg_configure(evb_handle *h);
+int evb_hg_round_bits(const evb_handle *h);
 size_t evb_hg_q_words(const evb_handle *h);
 int32_t evb_launch_histg(evb_handle *h, int level);
 int32_t evb_launch_acc_clear(evb_handle *h, int level);
@@ -245,8 +262,8 @@ static inline bool evb_scan_multi(const evb_handle *h) { return h->K >= 2 && h->
 static inline bool evb_acc_direct(const evb_handle *h) { return h->world == 1; }
 // evb_handle::low, a stretch of 2^(level-1) words per level: its build slots (at most half of them below the root), and in its last
 // word whether any slot has something (the root's only slot says so itself)
-static inline size_t evb_low_slot(int level) { return (size_t)1 << (level - 1); }
-static inline size_t evb_low_any(int level) { return ((size_t)1 << level) - 1; }
+__host__ __device__ static inline size_t evb_low_slot(int level) { return (size_t)1 << (level - 1); }
+__host__ __device__ static inline size_t evb_low_any(int level) { return ((size_t)1 << level) - 1; }
 static inline double evb_hg_low_unit(const evb_handle *h) { return 1.0 / (double)(1ull << (2 * h->hgeo.hb + 2)); } // units of hlow_q in those of hsum_q
 // evb_histq2.cu
 bool evb_q2_wanted(const evb_handle *h);
@@ -254,6 +271,17 @@ int32_t evb_q2_configure(evb_handle *h);
 int32_t evb_q2_build_layout(evb_handle *h);
 int32_t evb_q2_clear_layout(evb_handle *h);
 int32_t evb_launch_histq2(evb_handle *h, int level);
+// evb_grow.cu
+void evb_grow_configure(evb_handle *h);
+size_t evb_grow_sums(const evb_handle *h);
+size_t evb_grow_cnts(const evb_handle *h);
+size_t evb_grow_best(const evb_handle *h);
+int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot, bool next_grads);
+constexpr int EVB_GROW_JS = 512;   // sampled columns that travel with a launch
+static inline bool evb_grows_whole(const evb_handle *h) { return h->grow.on && h->world == 1; }
+static inline bool evb_one_launch(const evb_handle *h, bool masked) { return evb_grows_whole(h) && !masked && (h->F == h->nfeats || h->F <= EVB_GROW_JS); }
+// Maxima of |g| of the gradients in place and, when the tree kernel reads them while it makes the next ones, of those
+static inline unsigned *evb_gmax(const evb_handle *h, bool next) { return h->d_gmax + (size_t)h->nq * (evb_grows_whole(h) && next ? h->gmax_sel ^ 1 : h->gmax_sel); }
 // evb_tree.cu
 int32_t evb_launch_tree_begin(evb_handle *h, bool quantize, bool all_rows, const uint32_t *gen_js_host);
 int32_t evb_launch_scan(evb_handle *h, int level);

@@ -11,99 +11,6 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// Gradient record of one row: the channels whose sums the histograms hold, in the reference's order g_1..g_K, h_1..h_K, w
-// (`cache.∇`, src/init.jl:173).  Left out: w when no weights were given (it is 1) and, for mse, the hessians (h = 2w is
-// rebuilt from the sums of w): `elided`.
-struct AlphaSet { float a[8]; }; // a[0]: alpha of the quantile loss; a[0..K-1]: alphas of the multiquantile loss
-__device__ __forceinline__ void grad_row(int loss, int K, bool elided, const float *p, const void *y, int ycols, long long i, float w, float *rec,
-                                         const AlphaSet &al) {
-    const float alpha = al.a[0];
-    if (loss == EVB_MSE) {
-        const float *yf = (const float *)y + (size_t)i * ycols;
-        for (int k = 0; k < K; ++k) {
-            rec[k] = 2.0f * (p[k] - yf[k]) * w;
-            if (!elided) rec[K + k] = 2.0f * w;
-        }
-    } else if (loss == EVB_LOGLOSS) {
-        const float *yf = (const float *)y + (size_t)i * ycols;
-        for (int k = 0; k < K; ++k) {
-            const float s = sigmoidf_(p[k]);
-            rec[k] = (s - yf[k]) * w;
-            rec[K + k] = s * (1.0f - s) * w;
-        }
-    } else if (loss == EVB_MLOGLOSS) {
-        const uint32_t yi = ((const uint32_t *)y)[i];
-        float isum = 0.0f;
-        for (int k = 0; k < K; ++k) isum += expf(p[k]);
-        for (int k = 0; k < K; ++k) {
-            const float prob = expf(p[k]) / isum;
-            rec[k] = (((uint32_t)(k + 1) == yi) ? prob - 1.0f : prob) * w;
-            rec[K + k] = prob * (1.0f - prob) * w;
-        }
-    } else if (loss == EVB_MULTIQUANTILE) { // one target, one quantile per output row (src/loss.jl:160-172)
-        const float yi = ((const float *)y)[i];
-        for (int k = 0; k < K; ++k) {
-            const float d = yi - p[k];
-            rec[k] = (d > 0.0f ? al.a[k] : al.a[k] - 1.0f) * w;
-            rec[K + k] = d;
-        }
-    } else if (loss == EVB_QUANTILE) { // quantile_grad_diff, src/loss.jl:93-98: the second slot keeps the raw residual
-        const float *yf = (const float *)y + (size_t)i * ycols;
-        for (int k = 0; k < K; ++k) {
-            const float d = yf[k] - p[k];
-            rec[k] = (d > 0.0f ? alpha : alpha - 1.0f) * w;
-            rec[K + k] = d;
-        }
-    } else if (loss == EVB_MAE || loss == EVB_CRED_VAR || loss == EVB_CRED_STD) { // src/loss.jl:86-91
-        const float *yf = (const float *)y + (size_t)i * ycols;
-        for (int k = 0; k < K; ++k) {
-            const float d = yf[k] - p[k];
-            rec[k] = d * w;
-            rec[K + k] = (loss == EVB_MAE ? 0.0f : d * d) * w;
-        }
-    } else if (loss == EVB_POISSON || loss == EVB_GAMMA || loss == EVB_TWEEDIE) { // src/loss.jl:65-84
-        const float *yf = (const float *)y + (size_t)i * ycols;
-        for (int k = 0; k < K; ++k) {
-            const float pr = expf(p[k]), yk = yf[k];
-            float g, h;
-            if (loss == EVB_POISSON) { g = pr - yk; h = pr; }
-            else if (loss == EVB_GAMMA) { g = 2.0f * (1.0f - yk / pr); h = 2.0f * yk / pr; }
-            else { // rho = 1.5: pred^(2-rho) = sqrt(pred), pred^(1-rho) = 1 / sqrt(pred)
-                const float a = sqrtf(pr), b = 1.0f / a;
-                g = 2.0f * (a - yk * b);
-                h = 2.0f * (0.5f * a + 0.5f * yk * b);
-            }
-            rec[k] = g * w;
-            rec[K + k] = h * w;
-        }
-    } else if (loss == EVB_LOGISTIC_MLE) { // src/loss.jl:207-217
-        const int Y = K / 2;
-        const float *yf = (const float *)y + (size_t)i * ycols;
-        for (int t = 0; t < Y; ++t) {
-            const float loc = p[2 * t], sr = p[2 * t + 1];
-            const float scale = softplusf_(sr), ds = sigmoidf_(sr);
-            const float z = (yf[t] - loc) / scale, th = tanhf(z / 2.0f);
-            rec[2 * t] = -th / scale * w;
-            rec[2 * t + 1] = (1.0f - z * th) * ds / scale * w;
-            rec[2 * Y + 2 * t] = 1.0f / (3.0f * scale * scale) * w;
-            rec[2 * Y + 2 * t + 1] = (3.14159274f * 3.14159274f + 3.0f) / 9.0f * (ds / scale) * (ds / scale) * w;
-        }
-    } else { // EVB_GAUSSIAN_MLE
-        const int Y = K / 2;
-        const float *yf = (const float *)y + (size_t)i * ycols;
-        for (int t = 0; t < Y; ++t) {
-            const float loc = p[2 * t], sr = p[2 * t + 1];
-            const float scale = softplusf_(sr), ds = sigmoidf_(sr);
-            const float resid = loc - yf[t];
-            const float s2 = scale * scale;
-            rec[2 * t] = resid / s2 * w;
-            rec[2 * t + 1] = (1.0f - resid * resid / s2) * ds / scale * w;
-            rec[2 * Y + 2 * t] = 1.0f / s2 * w;
-            rec[2 * Y + 2 * t + 1] = 2.0f * (ds / scale) * (ds / scale) * w;
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------------- layout
 // xT[row][j] = xcol[j][row] for a block of columns; one thread = one row x 4 consecutive features
 __global__ void k_transpose(const uint8_t *xcol, long long ld, long long nrows, int j0, int nj, uint8_t *xT, int RS) {
@@ -310,10 +217,6 @@ struct FinArgs {
     uint4 *pub_dst;
     int pub_n;
 };
-// A copy node of the graph would cost 5 to 10 us between the kernels of two trees; these stores cost nothing.
-__device__ __forceinline__ void publish(const uint4 *src, uint4 *dst, int n) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
-}
 __global__ void __launch_bounds__(256) k_finalize(FinArgs a) {
     extern __shared__ uint32_t s_packed[];
     if (blockIdx.x == 0) publish(a.pub_src, a.pub_dst, a.pub_n);
@@ -628,51 +531,6 @@ __global__ void __launch_bounds__(256) k_binarize(const T *x, long long ld, long
 }
 
 // ---------------------------------------------------------------------------------- evaluation data
-// Per-row metric value in float, as `_metric_value` / `_mle2p_metric_value` / `mlogloss` compute it
-// (src/metrics.jl:1-110): the caller multiplies by w and accumulates in double.
-__device__ __forceinline__ float metric_row(int metric, int K, const float *p, const void *y, int ycols, long long i, float w, const AlphaSet &al) {
-    const float alpha = al.a[0];
-    if (metric == EVB_METRIC_MLOGLOSS) {
-        const uint32_t yi = ((const uint32_t *)y)[i];
-        float isum = 0.0f;
-        for (int k = 0; k < K; ++k) isum += expf(p[k]);
-        return w * (logf(isum) - p[yi - 1]);
-    }
-    const float *yf = (const float *)y + (size_t)i * ycols;
-    if (metric == EVB_METRIC_MULTIQUANTILE) { // src/metrics.jl:120-141
-        float acc = 0.0f;
-        for (int k = 0; k < K; ++k) acc += al.a[k] * fmaxf(yf[0] - p[k], 0.0f) + (1.0f - al.a[k]) * fmaxf(p[k] - yf[0], 0.0f);
-        return w * acc / (float)K;
-    }
-    if (metric == EVB_METRIC_GAUSSIAN_MLE || metric == EVB_METRIC_LOGISTIC_MLE) {
-        const int Y = K / 2;
-        float acc = 0.0f;
-        for (int t = 0; t < Y; ++t) {
-            const float scale = softplusf_(p[2 * t + 1]), d = yf[t] - p[2 * t];
-            if (metric == EVB_METRIC_GAUSSIAN_MLE) acc += -(logf(scale) + d * d / (2.0f * scale * scale));
-            else { const float az = fabsf(d / scale); acc += -logf(scale) - az - 2.0f * log1pf(expf(-az)); } // src/metrics.jl:84-89
-        }
-        return w * acc / (float)Y;
-    }
-    float acc = 0.0f;
-    for (int k = 0; k < K; ++k) {
-        const float pk = p[k], yk = yf[k];
-        if (metric == EVB_METRIC_MSE) acc += (pk - yk) * (pk - yk);
-        else if (metric == EVB_METRIC_MAE) acc += fabsf(pk - yk);
-        else if (metric == EVB_METRIC_QUANTILE) acc += alpha * fmaxf(yk - pk, 0.0f) + (1.0f - alpha) * fmaxf(pk - yk, 0.0f); // src/metrics.jl:4-6
-        else if (metric == EVB_METRIC_LOGLOSS) { const float s = sigmoidf_(pk); acc += -yk * logf(s) + (yk - 1.0f) * logf(1.0f - s); }
-        else if (metric == EVB_METRIC_POISSON) { // src/metrics.jl:13-17; eps(1f-7)
-            const float pr = expf(pk);
-            acc += 2.0f * (yk * logf(yk / pr + 7.1054274e-15f) + pr - yk);
-        } else if (metric == EVB_METRIC_GAMMA) { const float pr = expf(pk); acc += 2.0f * (logf(pr / yk) + yk / pr - 1.0f); }
-        else { // tweedie, rho = 1.5 (src/metrics.jl:24-28)
-            const float pr = expf(pk), a = sqrtf(pr);
-            acc += 2.0f * (sqrtf(yk) / -0.5f / 0.5f - yk * (1.0f / a) / -0.5f + a / 0.5f);
-        }
-    }
-    return w * acc / (float)K;
-}
-
 struct EvalArgs {
     const uint8_t *xT;
     const uint32_t *t_packed;
@@ -734,13 +592,6 @@ __global__ void __launch_bounds__(256) k_eval_sum(const double *part, int nblock
 } // namespace
 
 // =====================================================================================================
-static AlphaSet evb_alpha_set(const evb_handle *h) {
-    AlphaSet s;
-    for (int k = 0; k < 8; ++k) s.a[k] = (float)h->p.alphas[k];
-    if (h->p.loss != EVB_MULTIQUANTILE) s.a[0] = (float)h->p.alpha;
-    return s;
-}
-
 int32_t evb_launch_transpose(evb_handle *, const uint8_t *xcol_dev, int64_t ld, int64_t nrows, int j0, int nj, uint8_t *xT,
                              int RS, cudaStream_t st) {
     dim3 grid((unsigned)((nrows + 255) / 256), (unsigned)((nj + 3) / 4));
@@ -764,10 +615,10 @@ int32_t evb_launch_init_state(evb_handle *h, const float *w_dev, const float *pr
 }
 
 int32_t evb_launch_grads(evb_handle *h) {
-    EVB_CUDA(cudaMemsetAsync(h->d_gmax, 0, sizeof(unsigned) * h->ng, h->st));
+    EVB_CUDA(cudaMemsetAsync(evb_gmax(h, false), 0, sizeof(unsigned) * h->ng, h->st));
     evb_tic(h, EVB_T_GRADS);
     k_grads<<<(unsigned)((h->n + 255) / 256), 256, 0, h->st>>>(h->p.loss, h->K, h->nq, h->unit_w ? 1 : 0, h->Ce != h->C, h->ycols, h->n, h->pred, h->y, h->grad,
-                                                                h->d_gmax, h->ng, evb_alpha_set(h));
+                                                                evb_gmax(h, false), h->ng, evb_alpha_set(h));
     evb_toc(h, EVB_T_GRADS);
     EVB_CUDA(cudaGetLastError());
     return EVB_OK;
@@ -830,7 +681,7 @@ int32_t evb_launch_finalize(evb_handle *h, bool compute_grads, int mode, void *p
     FinArgs a;
     a.xT = h->xT; a.t_packed = h->t_packed; a.t_pred = h->t_pred; a.pred = h->pred; a.grad = h->grad; a.y = h->y;
     a.nidx = h->nidx; a.n = h->n; a.RS = h->RS; a.K = h->K; a.nq = h->nq; a.unit_w = h->unit_w ? 1 : 0; a.elided = h->Ce != h->C; a.loss = h->p.loss; a.nn = h->nn;
-    a.gmax = h->d_gmax; a.ng = h->ng; // cleared by the root's scan
+    a.gmax = evb_gmax(h, true); a.ng = h->ng; // cleared by the root's scan or the tree kernel
     a.ycols = h->ycols; a.compute_grads = compute_grads ? 1 : 0; a.alpha = evb_alpha_set(h); a.mode = mode;
     a.pub_src = reinterpret_cast<const uint4 *>(h->plan); a.pub_dst = static_cast<uint4 *>(publish_to); a.pub_n = publish_to ? (int)(h->h_tree_bytes / 16) : 0;
     const size_t smem = (size_t)h->nn * 4;

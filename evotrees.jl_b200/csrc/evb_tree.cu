@@ -6,6 +6,7 @@
 // bounds, build/subtract choice, work lists) lives in device memory, so the host enqueues a fixed sequence of
 // launches per level and never reads anything back until the tree is complete.
 #include "evb_histg.cuh"
+#include "evb_device.cuh"
 #include <float.h>
 #include <algorithm>
 
@@ -13,32 +14,6 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-__device__ __forceinline__ double warp_incl_scan(double v, int lane) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        double t = __shfl_up_sync(FULL, v, d);
-        if (lane >= d) v += t;
-    }
-    return v;
-}
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
-    return v;
-}
-__device__ __forceinline__ long long warp_sum(long long v) {
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
-    return v;
-}
-__device__ __forceinline__ int warp_incl_scan_i(int v, int lane) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        int t = __shfl_up_sync(FULL, v, d);
-        if (lane >= d) v += t;
-    }
-    return v;
-}
 // exclusive scan over the threads of a block (blockDim.x <= 1024, multiple of 32); returns the exclusive
 // prefix of v and writes the block total to *total.  `sm` is 33 ints of shared memory.
 __device__ __forceinline__ int block_excl_scan(int v, int *sm, int *total) {
@@ -148,21 +123,11 @@ struct ScanArgs {
     double lambda, L2, gamma, min_weight;
 };
 
-// Counts arrivals: what the arriving thread (and threads it has synchronised with) wrote before is visible to whoever sees the count.
-// One release-acquire operation instead of fences on both sides of a relaxed one, each of which waits for L2 (0.5 us).
-__device__ __forceinline__ uint32_t arrive(uint32_t *count) {
-    uint32_t v;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(count) : "memory");
-    return v;
-}
 // a load that is issued where it stands, not moved behind the branch its value is used in
 __device__ __forceinline__ int load_now(const int32_t *p) {
     int v;
     asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
-}
-__device__ __forceinline__ double term_gh(double g, double h, double w, double lambda, double L2) {
-    return g * g / fmax(DBL_EPSILON, h + lambda * w + L2) / 2.0; // src/split.jl:1
 }
 // mae: |mean of the side - mean of the parent| * weight / (1 + lambda + L2 / w)   (src/split.jl:2, 119-130)
 __device__ __forceinline__ double term_shift(double g, double w, double mu_p, double d) { return fabs(g / w - mu_p) * w / d; }
@@ -1101,10 +1066,6 @@ __device__ __forceinline__ void plan_level(const PartArgs &a, int *sm) {
 // launches and the prefix sums between them less per level.
 // A chunk is NI rows per thread.  A chunk inside one node (nearly all of them while nodes are large) takes the block-wide
 // path, else every warp looks its rows' nodes up and the lanes of the same node and side share an atomic.
-__device__ __forceinline__ bool goes_left(uint32_t pk, uint32_t x) { // split_set! predicate (fit-utils.jl:173, 291)
-    const uint32_t bin = (pk >> 16) & 0xffu;
-    return ((pk >> 25) & 1u) ? (x <= bin) : (x == bin);
-}
 // Every CTA takes a range of adjacent chunks: the node of the next one is known without a search unless it ends, and its row ids are
 // on their way while this one's bins arrive and its places are reserved.  What bounds a chunk is that chain of trips to L2, so
 // CTAs matter more than rows per thread: six CTAs of four rows a thread 0.640 ms per tree at 10M x 100, depth 11 (5M x 50 gaussian
@@ -1314,7 +1275,7 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
     a.qlow = direct ? h->hlow_q : nullptr; a.low = h->low + evb_low_slot(level); a.low_unit = evb_hg_low_unit(h);
     a.nq = h->nq; a.unit_w = h->unit_w ? 1 : 0;
     const bool fused = h->world == 1 && !h->obl_gain;
-    a.gmax = h->d_gmax; a.ng = h->ng;
+    a.gmax = evb_gmax(h, false); a.ng = h->ng;
     a.ticket = fused ? h->ticket : nullptr; a.cur_l = h->cur_l; a.cur_r = h->cur_r; a.seg_start = h->seg_start; a.seg_cnt = h->seg_cnt;
     a.lambda = h->p.lambda; a.L2 = h->p.L2; a.gamma = h->p.gamma; a.min_weight = h->p.min_weight;
     a.fbest_gain = h->fbest_gain; a.fbest_bin = h->fbest_bin; a.fbest_left = h->fbest_left;
