@@ -12,6 +12,8 @@
 //   decisions    every CTA takes all of them, so that nothing has to be handed around; the children's weights say which one is built
 //   rows         every CTA moves its own rows, looking up the split feature's bin (other groups' CTAs do the same for theirs)
 // With one range of rows a CTA scans its own features' sums and the first barrier falls away.
+// Where at most 16 CTAs hold the rows they are one cluster: sums, histograms and best splits lie in their shared memory, added to and handed
+// out by remote accesses, and its barriers are the hardware's (0.4 us with the wait for the slowest CTA, 1.3 through L2).
 // ms per tree before (level kernels) and here: 1503 x 7 logloss, depth 5 0.085 and 0.052; 100k x 10, 32 bins, depth 6 0.098 and 0.061; 60k x 77
 // poisson, depth 6 0.128 and 0.099.  At 100k x 10 a level takes 8 us: histograms 1.4, barriers 1.4 and 1.3, scan 1.5, decisions 1.3, rows 1.3.
 #include "evb_histg.cuh"
@@ -54,8 +56,9 @@ struct GrowArgs {
     int *err;
     long long n;
     int cond, F, B, D, hist_nodes, loss, elide, hb, ng, round_bits, nn;
-    int NG, NR, rpc, lw, fit, M;
+    int NG, NR, rpc, lw, lc, fit, M; // lc: log2 of the columns of an image
     int o_x, o_q, o_idx, o_node;
+    int o_sum, o_cnt, o_best, o_hist, fo; // one cluster only: sums of the features a CTA scans, fo at most; o_hist == 0: their histograms are in `hist`
     unsigned max_polls;
     double low_unit, neb, lambda, L2, gamma, min_weight;
     // no row sample: the kernel also clears the tree before and brings it to every row afterwards
@@ -100,13 +103,36 @@ extern __shared__ __align__(128) unsigned char s_raw[];
 #define S_CR (reinterpret_cast<int *>(s_raw + a.o_node + (2 * PAIR_BYTES + 4) * a.M))
 #define S_MISC (reinterpret_cast<int *>(s_raw + a.o_node + NODE_BYTES * a.M))
 #define S_UNIT (reinterpret_cast<double *>(s_raw + a.o_node + NODE_BYTES * a.M + 64))                              /* units of the channels' sums */
+#define S_ROOT (reinterpret_cast<double *>(s_raw + a.o_node + NODE_BYTES * a.M + 96))                               /* sums of the root (one cluster) */
 #define S_RED (reinterpret_cast<double *>(s_raw + a.o_node + NODE_BYTES * a.M + 128))                              /* [2 NW] */
 #define S_QUANT (reinterpret_cast<Quant *>(s_raw + a.o_node + NODE_BYTES * a.M + 128))                             /* [NQ], while the rows are loaded */
 #define S_TREE (reinterpret_cast<uint32_t *>(s_raw + a.o_node + NODE_BYTES * a.M + MISC_BYTES))                    /* [nn] packed nodes */
 #define S_VALUE (reinterpret_cast<float *>(S_TREE + a.nn))                                                         /* [nn] leaf values */
 #define S_FEAT (S_TREE + 2 * a.nn)                                                                                 /* [F] feature | numeric << 16 | (constraint + 1) << 17 */
 #define S_LEAF (reinterpret_cast<uint16_t *>(S_FEAT + a.F))                                                        /* leaf of every row this CTA updates */
+// one cluster only
+#define S_SUM (reinterpret_cast<unsigned long long *>(s_raw + a.o_sum))  /* [slot][fo][NQ][B] */
+#define S_CNTS (reinterpret_cast<uint32_t *>(s_raw + a.o_cnt))           /* [slot][fo][B], then [slot] nonzero: the slot has something in `low` */
+#define S_LOW (S_CNTS + (a.M / 2) * a.fo * a.B)
+#define S_BEST (reinterpret_cast<double2 *>(s_raw + a.o_best))           /* [node][F][3], of all features */
 enum { M_LEFT = 0, M_OK = 1, M_CNT = 2, M_INF = 3, M_MAX = 4 }; // M_MAX: two words
+
+// shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t remote(const void *p, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void remote_add(uint32_t at, unsigned long long v) { asm volatile("red.relaxed.cluster.shared::cluster.add.u64 [%0], %1;" ::"r"(at), "l"(v) : "memory"); }
+__device__ __forceinline__ void remote_add(uint32_t at, uint32_t v) { asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+__device__ __forceinline__ void remote_put(uint32_t at, double x, double y) {
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(at), "d"(x), "d"(y) : "memory");
+}
+__device__ __forceinline__ void remote_put(uint32_t at, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // All CTAs have arrived `k` times.  The launch is cooperative, so all of them run; the wait is bounded all the same: a CTA whose
 // wait runs out (or that sees another's has) leaves an error word and the kernel ends.
@@ -146,15 +172,26 @@ __device__ __forceinline__ void warp_first_max(double &v, int &id) {
 
 // ---------------------------------------------------------------------------------------------- histograms of a level
 // Rows of the build nodes of slots [s0, s1), a tile of 32 rows of one node per warp; lanes and banks as in evb_histg.cuh
-template <int NQ, bool CNT, bool PACK, int LW>
+// (LC == 5: 32 columns, 8 / W replicas of W words; fewer columns, fewer replicas: lanes meet in a bank, the image is emptied faster)
+template <int NQ, bool CNT, bool PACK, int PB, int C = 0>
+__device__ __forceinline__ void add_cell(uint32_t addr, const uint32_t (&hi)[NQ], const uint32_t (&lo)[NQ]) {
+    if constexpr (C < NQ) {
+        red_at<2 * PB * C>(addr, hi[C]);
+        red_at<2 * PB * C + PB>(addr, lo[C]);
+        add_cell<NQ, CNT, PACK, PB, C + 1>(addr, hi, lo);
+    } else if constexpr (CNT && !PACK) {
+        red_at<2 * PB * NQ>(addr, 1u);
+    }
+}
+template <int NQ, bool CNT, bool PACK, int LW, int LC>
 __device__ __forceinline__ void add_rows(const GrowArgs &a, const Pairs &pr, const uint16_t *idx, int s0, int s1, bool second) {
-    constexpr int P = planes(NQ, CNT, PACK), W = 1 << LW;
-    constexpr uint32_t STRIDE = P * 128;
+    constexpr int P = planes(NQ, CNT, PACK), W = 1 << LW, PB = 4 << LC, R = 1 << (LC - 2 - LW);
+    constexpr uint32_t STRIDE = P * PB;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float two_lb = __int_as_float((128 + a.hb) << 23); // 2^(hb + 1)
     Lane ln;
     ln.init(S_IMG, lane);
-    const uint32_t rep = 16u * (uint32_t)(lane & 7 & ~(W - 1)), slot_bytes = (uint32_t)(a.B + 1) * STRIDE;
+    const uint32_t rep = 16u * (uint32_t)(lane & (R * W - 1) & ~(W - 1)), slot_bytes = (uint32_t)(a.B + 1) * STRIDE;
     int base = 0;
     for (int s = s0; s < s1; ++s) {
         const int b = pr.build()[s], r0 = b ? pr.mid()[s] : pr.st()[s], cnt = (b ? pr.en()[s] : pr.mid()[s]) - r0, nt = (cnt + 31) >> 5;
@@ -186,7 +223,7 @@ __device__ __forceinline__ void add_rows(const GrowArgs &a, const Pairs &pr, con
                     const int word = (lane + w) & (W - 1);
                     const uint32_t v = S_X[word * a.rpc + r], at = img + 16u * (uint32_t)word;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) red_cell<NQ, CNT, PACK>(__byte_perm(v, 0u, ln.sel[k]) * STRIDE + (ln.col[k] + at), qh, ql);
+                    for (int k = 0; k < 4; ++k) add_cell<NQ, CNT, PACK, PB>(__byte_perm(v, 0u, ln.sel[k]) * STRIDE + (ln.col[k] + at), qh, ql);
                 }
             }
         }
@@ -197,77 +234,92 @@ __device__ __forceinline__ void add_rows(const GrowArgs &a, const Pairs &pr, con
 // The images of slots [s0, s1) -> sums of the level; clears them.  A warp takes BO adjacent bins of FB features at a time, so that the
 // lanes of a reduction fill whole sectors of [feature][channel][bin]; replicas are read in an order that differs from bin to bin
 // (they sit 4 W columns apart: one bank for all bins).
-template <int NQ, bool CNT, bool PACK, int LW>
-__device__ __forceinline__ void flush(const GrowArgs &a, const Pairs &pr, int set, int s0, int s1, int f0, bool second) {
-    constexpr int P = planes(NQ, CNT, PACK), W = 1 << LW, R = 8 / W, FB = LW == 0 ? 4 : 8, BO = 32 / FB, NC = 4 * W / FB;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, bo = lane % BO;
-    const int nbb = (a.B + BO - 1) / BO, per = NC * nbb, slot_words = (a.B + 1) * P * 32;
+template <int NQ, bool CNT, bool PACK, int LW, int LC, bool CL>
+__device__ __forceinline__ void flush(const GrowArgs &a, const Pairs &pr, int set, int s0, int s1, int g, bool second) {
+    constexpr int P = planes(NQ, CNT, PACK), W = 1 << LW, COLS = 1 << LC, R = 1 << (LC - 2 - LW), FB = LW == 0 ? 4 : 8, BO = 32 / FB, NC = 4 * W / FB;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, bo = lane % BO, f0 = g * 4 * W;
+    const int nbb = (a.B + BO - 1) / BO, per = NC * nbb, slot_words = (a.B + 1) * P * COLS;
     const bool own = a.NR == 1; // no other CTA adds to these cells
-    unsigned long long *sums = (second ? a.low : a.sum) + (size_t)set * a.sum_set;
-    uint32_t *cnts = a.cnt + (size_t)set * a.cnt_set;
     for (int u = wid; u < (s1 - s0) * per; u += NW) {
         const int s = u / per, e = u - s * per, ch = e / nbb, bin = (e - ch * nbb) * BO + bo, f = ch * FB + lane / BO, slot = s0 + s;
         if (!pr.dec()[slot] || (!own && pr.st()[slot] == pr.en()[slot])) continue;
         if (bin >= a.B) continue;
-        uint32_t *p = S_IMG + (size_t)s * slot_words + (size_t)(bin + 1) * (P * 32) + f;
+        uint32_t *p = S_IMG + (size_t)s * slot_words + (size_t)(bin + 1) * (P * COLS) + f;
         const bool out = f0 + f < a.F;
-        const size_t cell = (size_t)slot * a.F + (f0 + f);
+        // where the sums go: this CTA's share of the features (CL), CTA f % NR of the group's, or global memory
+        const int lf = CL ? f / a.NR : 0, rank = CL ? (f - lf * a.NR) * a.NG + g : 0;
+        const size_t cell = CL && !second ? (size_t)slot * a.fo + lf : (size_t)slot * a.F + (f0 + f);
+        auto put = [&](int c, unsigned long long v) {
+            const size_t at = (cell * NQ + c) * a.B + bin;
+            if (CL && !second) {
+                if (own) S_SUM[at] = v;
+                else if (v != 0ull) remote_add(remote(S_SUM + at, rank), v);
+            } else {
+                unsigned long long *d = (second ? a.low : a.sum) + (size_t)set * a.sum_set + at;
+                if (own) *d = v;
+                else if (v != 0ull) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(d), "l"(v) : "memory");
+            }
+        };
+        auto put_count = [&](uint32_t v) {
+            const size_t at = cell * a.B + bin;
+            if (CL) {
+                if (own) S_CNTS[at] = v;
+                else if (v != 0u) remote_add(remote(S_CNTS + at, rank), v);
+            } else {
+                uint32_t *d = a.cnt + (size_t)set * a.cnt_set + at;
+                if (own) *d = v;
+                else if (v != 0u) asm volatile("red.global.add.u32 [%0], %1;" ::"l"(d), "r"(v) : "memory");
+            }
+        };
         if constexpr (PACK) {
             long long v = 0;
             uint32_t c = 0;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 uint32_t *w = p + ((i + bo) & (R - 1)) * (4 * W);
-                const uint32_t hi = w[0], lo = w[32];
-                w[0] = 0u; w[32] = 0u;
+                const uint32_t hi = w[0], lo = w[COLS];
+                w[0] = 0u; w[COLS] = 0u;
                 v += ((long long)(int32_t)hi << 6) + (long long)(lo & 0x7ffffu);
                 c += lo >> 19;
             }
-            if (!out) continue;
-            if (own) { sums[cell * a.B + bin] = (unsigned long long)v; cnts[cell * a.B + bin] = c; }
-            else if (c != 0u) {
-                asm volatile("red.global.add.u64 [%0], %1;" ::"l"(sums + cell * a.B + bin), "l"(v) : "memory");
-                asm volatile("red.global.add.u32 [%0], %1;" ::"l"(cnts + cell * a.B + bin), "r"(c) : "memory");
-            }
+            if (out && (own || c != 0u)) { put(0, (unsigned long long)v); put_count(c); }
         } else {
             if constexpr (CNT) {
                 uint32_t c = 0;
 #pragma unroll
-                for (int i = 0; i < R; ++i) { uint32_t *w = p + ((i + bo) & (R - 1)) * (4 * W) + 64 * NQ; c += *w; *w = 0u; }
+                for (int i = 0; i < R; ++i) { uint32_t *w = p + ((i + bo) & (R - 1)) * (4 * W) + 2 * COLS * NQ; c += *w; *w = 0u; }
                 if (!own && c == 0u) continue; // no row: all words are zero
-                if (out && !second) {
-                    if (own) cnts[cell * a.B + bin] = c;
-                    else asm volatile("red.global.add.u32 [%0], %1;" ::"l"(cnts + cell * a.B + bin), "r"(c) : "memory");
-                }
+                if (out && !second) put_count(c);
             }
 #pragma unroll
             for (int c = 0; c < NQ; ++c) {
-                long long v = 0;
+                long long hi = 0, lo = 0;
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
-                    uint32_t *w = p + ((i + bo) & (R - 1)) * (4 * W) + 64 * c;
-                    v += ((long long)(int32_t)w[0] << (a.hb + 1)) + (long long)(int32_t)w[32];
-                    w[0] = 0u; w[32] = 0u;
+                    uint32_t *w = p + ((i + bo) & (R - 1)) * (4 * W) + 2 * COLS * c;
+                    hi += (long long)(int32_t)w[0]; lo += (long long)(int32_t)w[COLS];
+                    w[0] = 0u; w[COLS] = 0u;
                 }
-                if (!out) continue;
-                unsigned long long *d = sums + (cell * NQ + c) * a.B + bin;
-                if (own) *d = (unsigned long long)v;
-                else if (v != 0) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(d), "l"(v) : "memory");
+                if (out) put(c, (unsigned long long)((hi << (a.hb + 1)) + lo));
             }
         }
     }
 }
 
-template <int NQ, bool CNT, bool PACK, int LW>
-__device__ __forceinline__ void hist_level(const GrowArgs &a, const Pairs &pr, const uint16_t *idx, int np, int set, int f0, int level) {
+template <int NQ, bool CNT, bool PACK, int LW, int LC, bool CL>
+__device__ __forceinline__ void hist_level(const GrowArgs &a, const Pairs &pr, const uint16_t *idx, int np, int set, int g, int level) {
     for (int s0 = 0; s0 < np; s0 += a.fit) {
         const int s1 = min(np, s0 + a.fit);
         for (bool second = false;; second = true) {
-            add_rows<NQ, CNT, PACK, LW>(a, pr, idx, s0, s1, second);
+            add_rows<NQ, CNT, PACK, LW, LC>(a, pr, idx, s0, s1, second);
             __syncthreads();
             const bool again = !PACK && !second && S_MISC[M_LEFT] != 0;
-            flush<NQ, CNT, PACK, LW>(a, pr, set, s0, s1, f0, second);
-            if (second) for (int s = s0 + (int)threadIdx.x; s < s1; s += T) a.lowflag[evb_low_slot(level) + s] = 1u;
+            flush<NQ, CNT, PACK, LW, LC, CL>(a, pr, set, s0, s1, g, second);
+            if (second) {
+                if constexpr (CL) {
+                    for (int e = threadIdx.x; e < (s1 - s0) * (int)gridDim.x; e += T) remote_put(remote(S_LOW + s0 + e / gridDim.x, e % gridDim.x), 1u);
+                } else for (int s = s0 + (int)threadIdx.x; s < s1; s += T) a.lowflag[evb_low_slot(level) + s] = 1u;
+            }
             __syncthreads();
             if (!again) break;
             if (threadIdx.x == 0) S_MISC[M_LEFT] = 0; // (read again behind the next barrier)
@@ -277,29 +329,41 @@ __device__ __forceinline__ void hist_level(const GrowArgs &a, const Pairs &pr, c
 
 // ---------------------------------------------------------------------------------------------- split scan
 // One warp: node n (of pair `slot`, number j of the level) and feature slot f.  The same sums, in the same order, as k_scan_feat.
-template <int NQ, bool CNT, bool PACK, int CH>
-__device__ __forceinline__ void scan(const GrowArgs &a, int level, int set, int slot, int f, int n, int j, bool sub, const double *node_sum) {
+template <int NQ, bool CNT, bool PACK, int CH, bool CL>
+__device__ __forceinline__ void scan(const GrowArgs &a, int level, int set, int slot, int f, int lf, int n, int j, bool sub, const double *node_sum) {
     const int lane = threadIdx.x & 31, B = a.B, F = a.F, bin0 = lane * CH;
     const bool counted = CNT || PACK, keep = n < a.hist_nodes, elide = a.elide != 0;
-    const size_t cell = (size_t)slot * F + f;
-    const unsigned long long *ps = a.sum + (size_t)set * a.sum_set + cell * NQ * B;
-    const uint32_t *pc = a.cnt + (size_t)set * a.cnt_set + cell * B;
+    const size_t cell = (size_t)slot * F + f, own = (size_t)slot * a.fo + lf;
+    const unsigned long long *ps = CL ? S_SUM + own * NQ * B : a.sum + (size_t)set * a.sum_set + cell * NQ * B;
+    const uint32_t *pc = CL ? S_CNTS + own * B : a.cnt + (size_t)set * a.cnt_set + cell * B;
     const double *hp = a.hist + ((size_t)(n >> 1) * F + f) * 3 * B;
     double *hn = a.hist + ((size_t)n * F + f) * 3 * B;
+    // one cluster: histograms of this level and the one before also in shared memory, the larger half for the levels that are an even
+    // number of levels above the last one kept
+    const bool near = CL && a.o_hist != 0;
+    const int hs = elide ? 2 : 3, up = a.D - 2 - level;
+    auto near_at = [&](int node, int above) {
+        return reinterpret_cast<double *>(s_raw + a.o_hist) + ((size_t)((above & 1) ? max(1, a.M >> 1) : 0) + node) * a.fo * hs * B + (size_t)lf * hs * B;
+    };
+    double *kn = near ? near_at(j, up) : nullptr;
+    if (near) hp = near_at(j >> 1, up + 1);
+    const int wo = near ? hs - 1 : 2;
+    auto ldu = [](const unsigned long long *p) { if constexpr (CL) return *p; else return __ldcg(p); };
+    auto ldc = [](const uint32_t *p) { if constexpr (CL) return *p; else return __ldcg(p); };
     long long rg[CH], rh[CH], rw[CH];
     double pg[CH], ph[CH], pw[CH];
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
         const int b = min(bin0 + i, B - 1);
-        rg[i] = (long long)__ldcg(ps + b);
-        rh[i] = elide ? 0ll : (long long)__ldcg(ps + B + b);
-        rw[i] = counted ? (long long)__ldcg(pc + b) : (long long)__ldcg(ps + (NQ - 1) * B + b);
+        rg[i] = (long long)ldu(ps + b);
+        rh[i] = elide ? 0ll : (long long)ldu(ps + B + b);
+        rw[i] = counted ? (long long)ldc(pc + b) : (long long)ldu(ps + (NQ - 1) * B + b);
         pg[i] = ph[i] = pw[i] = 0.0;
-        if (sub) { pg[i] = __ldcg(hp + b); if (!elide) ph[i] = __ldcg(hp + B + b); pw[i] = __ldcg(hp + 2 * B + b); }
+        if (sub) { pg[i] = CL ? hp[b] : __ldcg(hp + b); if (!elide) ph[i] = CL ? hp[B + b] : __ldcg(hp + B + b); pw[i] = CL ? hp[wo * B + b] : __ldcg(hp + wo * B + b); }
     }
     const uint32_t feat = S_FEAT[f];
     const double ig = S_UNIT[0], ih = elide ? 0.0 : S_UNIT[NQ > 1 ? 1 : 0], iw = counted ? 1.0 : S_UNIT[NQ - 1];
-    const bool numeric = (feat >> 16) & 1u, low = !PACK && __ldcg(a.lowflag + evb_low_slot(level) + slot) != 0u;
+    const bool numeric = (feat >> 16) & 1u, low = !PACK && (CL ? S_LOW[slot] : __ldcg(a.lowflag + evb_low_slot(level) + slot)) != 0u;
     const int constraint = (int)((feat >> 17) & 3u) - 1;
     double g[CH], h[CH], w[CH];
 #pragma unroll
@@ -329,6 +393,7 @@ __device__ __forceinline__ void scan(const GrowArgs &a, int level, int set, int 
     if (n == 1) {
         if (elide) sh = 2.0 * sw; // h = 2w (src/loss.jl:52)
         if (f == 0 && lane == 0) { a.nsum[3] = sg; a.nsum[4] = sh; a.nsum[5] = sw; }
+        if (CL && f == 0 && lane < (int)gridDim.x) { remote_put(remote(S_ROOT, lane), sg, sh); remote_put(remote(S_ROOT + 2, lane), sw, 0.0); }
     }
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
@@ -336,7 +401,10 @@ __device__ __forceinline__ void scan(const GrowArgs &a, int level, int set, int 
         if (sub) { g[i] = pg[i] - g[i]; h[i] = ph[i] - h[i]; w[i] = pw[i] - w[i]; }
         if (elide) h[i] = 2.0 * w[i];
         if (b >= B) g[i] = h[i] = w[i] = 0.0;
-        else if (keep) { hn[b] = g[i]; hn[B + b] = h[i]; hn[2 * B + b] = w[i]; }
+        else if (keep) {
+            hn[b] = g[i]; hn[B + b] = h[i]; hn[2 * B + b] = w[i];
+            if (near && up >= 0) { kn[b] = g[i]; kn[wo * B + b] = w[i]; if (!elide) kn[B + b] = h[i]; }
+        }
     }
     if (numeric) { // running sums over the bins: inside the lane, then over the lanes' totals
 #pragma unroll
@@ -376,22 +444,36 @@ __device__ __forceinline__ void scan(const GrowArgs &a, int level, int set, int 
     }
     const int mine = lb;
     warp_first_max(lg, lb);
-    double2 *rec = a.best + (((size_t)set * a.M + j) * F + f) * 3;
-    if (lane == 0) rec[0] = make_double2(lg, lb == 0x7fffffff ? -1.0 : (double)lb);
-    if (mine == lb && lb != 0x7fffffff) { rec[1] = make_double2(bg, bh); rec[2] = make_double2(bw, 0.0); }
+    if constexpr (CL) { // to every CTA
+        const int src = min(lb / CH, 31);
+        bg = __shfl_sync(FULL, bg, src); bh = __shfl_sync(FULL, bh, src); bw = __shfl_sync(FULL, bw, src);
+        if (lane < (int)gridDim.x) {
+            const uint32_t rec = remote(S_BEST + ((size_t)j * F + f) * 3, lane);
+            remote_put(rec, lg, lb == 0x7fffffff ? -1.0 : (double)lb);
+            remote_put(rec + 16, bg, bh);
+            remote_put(rec + 32, bw, 0.0);
+        }
+    } else {
+        double2 *rec = a.best + (((size_t)set * a.M + j) * F + f) * 3;
+        if (lane == 0) rec[0] = make_double2(lg, lb == 0x7fffffff ? -1.0 : (double)lb);
+        if (mine == lb && lb != 0x7fffffff) { rec[1] = make_double2(bg, bh); rec[2] = make_double2(bw, 0.0); }
+    }
 }
 
-template <int NQ, bool CNT, bool PACK, int CH>
+template <int NQ, bool CNT, bool PACK, int CH, bool CL>
 __device__ __forceinline__ void scan_level(const GrowArgs &a, const Pairs &pr, int level, int set, int np, int g) {
     const int both = level > 1 ? 1 : 0, wid = threadIdx.x >> 5;
-    const bool own = a.NR == 1; // the CTA's own features; else all (pair, feature, child) over all CTAs
-    const int f0 = own ? g * (4 << a.lw) : 0, nf = own ? min(4 << a.lw, a.F - f0) : a.F;
+    const bool own = CL || a.NR == 1; // the CTA's own features; else all (pair, feature, child) over all CTAs
+    // one cluster: features r, r + NR, r + 2 NR .. of the group
+    const int r = CL ? (int)blockIdx.x / a.NG : 0, stride = CL ? a.NR : 1, in_group = min(4 << a.lw, a.F - g * (4 << a.lw));
+    const int f0 = own ? g * (4 << a.lw) + r : 0, nf = CL ? (in_group - r + stride - 1) / stride : own ? in_group : a.F;
+    if (nf <= 0) return;
     const int total = (np * nf) << both, step = own ? NW : NW * (int)gridDim.x;
     for (int t = own ? wid : wid * (int)gridDim.x + (int)blockIdx.x; t < total; t += step) {
-        const int which = t & both, e = t >> both, s = e / nf, f = f0 + (e - s * nf);
+        const int which = t & both, e = t >> both, s = e / nf, lf = e - s * nf, f = f0 + lf * stride;
         if (!pr.dec()[s]) continue;
         const int c = pr.build()[s] ^ which, j = 2 * s + c;
-        scan<NQ, CNT, PACK, CH>(a, level, set, s, f, (1 << (level - 1)) + j, j, which != 0, pr.sum() + 3 * j);
+        scan<NQ, CNT, PACK, CH, CL>(a, level, set, s, f, lf, (1 << (level - 1)) + j, j, which != 0, pr.sum() + 3 * j);
     }
 }
 
@@ -401,6 +483,7 @@ __device__ __forceinline__ float leaf_of(const GrowArgs &a, double g, double h, 
 // Every CTA decides every node, a warp per node, and so knows the slots of the next level; CTA j of the grid writes what belongs to
 // node j.  The child with the smaller weight is built, the left one when they are equal (with unit weights the reference's rule on
 // row counts, src/fit.jl:123-129).  Returns whether the thread's warp has split a node.
+template <bool CL>
 __device__ __forceinline__ bool decide(const GrowArgs &a, const Pairs &pr, const Pairs &nx, int level, int set) {
     const int lane = threadIdx.x & 31, F = a.F, nodes = 1 << (level - 1);
     bool any = false;
@@ -410,16 +493,17 @@ __device__ __forceinline__ bool decide(const GrowArgs &a, const Pairs &pr, const
             if (lane == 0) { nx.dec()[j] = 0u; nx.st()[j] = nx.mid()[j] = nx.en()[j] = pr.en()[s]; }
             continue;
         }
-        const double2 *rec = a.best + ((size_t)set * a.M + j) * F * 3;
+        const double2 *rec = CL ? S_BEST + (size_t)j * F * 3 : a.best + ((size_t)set * a.M + j) * F * 3;
+        auto ld = [](const double2 *p) { if constexpr (CL) return *p; else return __ldcg(p); };
         double2 l1 = make_double2(0.0, 0.0), l2 = l1; // left sums of the lane's best feature
         double s0, s1, s2;
-        if (level == 1) { s0 = __ldcg(a.nsum + 3); s1 = __ldcg(a.nsum + 4); s2 = __ldcg(a.nsum + 5); }
+        if (level == 1) { s0 = CL ? S_ROOT[0] : __ldcg(a.nsum + 3); s1 = CL ? S_ROOT[1] : __ldcg(a.nsum + 4); s2 = CL ? S_ROOT[2] : __ldcg(a.nsum + 5); }
         else { s0 = pr.sum()[3 * j]; s1 = pr.sum()[3 * j + 1]; s2 = pr.sum()[3 * j + 2]; }
         double bg = a.gamma;
         int bs = 0x7fffffff, bb = -1;
 #pragma unroll 2
         for (int f = lane; f < F; f += 32) {
-            const double2 r = __ldcg(rec + 3 * f), r1 = __ldcg(rec + 3 * f + 1), r2 = __ldcg(rec + 3 * f + 2);
+            const double2 r = ld(rec + 3 * f), r1 = ld(rec + 3 * f + 1), r2 = ld(rec + 3 * f + 2);
             if (r.y >= 0.0 && r.x > bg) { bg = r.x; bs = f; bb = (int)r.y; l1 = r1; l2 = r2; }
         }
         warp_first_max(bg, bs);
@@ -636,10 +720,25 @@ __device__ __forceinline__ void clear_sums(const GrowArgs &a, int NQ, int set, i
             for (size_t i = i0; i < per * NQ; i += st) l[k * per * NQ + i] = 0ull;
 }
 
-template <int NQ, bool CNT, bool PACK, int CH>
+// one cluster, several ranges of rows: the sums that have been scanned
+template <int NQ, bool PACK>
+__device__ __forceinline__ void clear_own(const GrowArgs &a, int set, int np, int g) {
+    for (int i = threadIdx.x; i < np * a.fo * NQ * a.B; i += T) S_SUM[i] = 0ull;
+    for (int i = threadIdx.x; i < np * a.fo * a.B; i += T) S_CNTS[i] = 0u;
+    if constexpr (!PACK) {
+        const int r = (int)blockIdx.x / a.NG, end = min((g + 1) * (4 << a.lw), a.F);
+        for (int s = 0; s < np; ++s) {
+            if (!S_LOW[s]) continue;
+            for (int f = g * (4 << a.lw) + r; f < end; f += a.NR)
+                for (int i = threadIdx.x; i < NQ * a.B; i += T) a.low[(size_t)set * a.sum_set + ((size_t)s * a.F + f) * NQ * a.B + i] = 0ull;
+        }
+    }
+}
+
+// CL: the grid is one cluster; sums, histograms and best splits are exchanged through the CTAs' shared memory and the barriers are the cluster's
+template <int NQ, bool CNT, bool PACK, int CH, bool CL>
 __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
-    constexpr int P = planes(NQ, CNT, PACK);
-    const size_t img_bytes = (size_t)(a.B + 1) * P * 128;
+    const size_t img_bytes = (size_t)(a.B + 1) * planes(NQ, CNT, PACK) * 4 << a.lc;
     const int g = blockIdx.x % a.NG, f0 = g * (4 << a.lw);
     const long long row0 = (long long)(blockIdx.x / a.NG) * a.rpc;
     const int nr = (int)min((long long)a.rpc, a.n - row0), lane = threadIdx.x & 31;
@@ -675,6 +774,11 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
     {
         uint4 *z = reinterpret_cast<uint4 *>(S_IMG);
         for (int i = threadIdx.x; i < (int)(a.fit * img_bytes / 16); i += T) z[i] = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (CL) {
+            const int slots = a.M / 2;
+            for (int i = threadIdx.x; i < slots * a.fo * NQ * a.B; i += T) S_SUM[i] = 0ull;
+            for (int i = threadIdx.x; i < slots * a.fo * a.B + slots; i += T) S_CNTS[i] = 0u;
+        }
     }
     __syncthreads();
     {
@@ -703,7 +807,8 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         }
     __syncthreads();
     if (threadIdx.x == 0) { const int c = a.mask ? S_MISC[M_CNT] : nr; const Pairs root = S_PAIRS(0); root.mid()[0] = c; root.en()[0] = c; }
-    __syncthreads();
+    if constexpr (CL) cluster_barrier(); // the sums of all CTAs are empty
+    else __syncthreads();
 
     const int cnt = S_PAIRS(0).en()[0];
     int np = 1, done_np = 0; // slots of the level and of the one before
@@ -712,25 +817,40 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         const int cur = (level - 1) & 1, set = level & 1;
         const Pairs pr = S_PAIRS(cur), nx = S_PAIRS(cur ^ 1);
         const uint16_t *idx = S_IDX(cur);
-        if (a.lw == 0) hist_level<NQ, CNT, PACK, 0>(a, pr, idx, np, set, f0, level);
-        else if (a.lw == 1) hist_level<NQ, CNT, PACK, 1>(a, pr, idx, np, set, f0, level);
-        else hist_level<NQ, CNT, PACK, 2>(a, pr, idx, np, set, f0, level);
-        if (a.NR > 1) {
-            if (!grid_barrier(a, S_MISC + M_OK, ++arrivals)) return;
-            if (level > 1) clear_sums(a, NQ, set ^ 1, done_np, level - 1);
+        if constexpr (CL) {
+            if (a.lw == 0 && a.lc == 3) hist_level<NQ, CNT, PACK, 0, 3, true>(a, pr, idx, np, set, g, level);
+            else if (a.lw == 0) hist_level<NQ, CNT, PACK, 0, 4, true>(a, pr, idx, np, set, g, level);
+            else if (a.lw == 1) hist_level<NQ, CNT, PACK, 1, 4, true>(a, pr, idx, np, set, g, level);
+            else hist_level<NQ, CNT, PACK, 2, 5, true>(a, pr, idx, np, set, g, level);
+            cluster_barrier();
+        } else {
+            if (a.lw == 0) hist_level<NQ, CNT, PACK, 0, 5, false>(a, pr, idx, np, set, g, level);
+            else if (a.lw == 1) hist_level<NQ, CNT, PACK, 1, 5, false>(a, pr, idx, np, set, g, level);
+            else hist_level<NQ, CNT, PACK, 2, 5, false>(a, pr, idx, np, set, g, level);
+            if (a.NR > 1) {
+                if (!grid_barrier(a, S_MISC + M_OK, ++arrivals)) return;
+                if (level > 1) clear_sums(a, NQ, set ^ 1, done_np, level - 1);
+            }
         }
         if (level == 1 && S_MISC[M_INF]) { // infinities of both signs: no sum means anything
             if (threadIdx.x < NQ && *(volatile unsigned *)(a.signs + threadIdx.x) == 3u && a.gmax[threadIdx.x] >= 0x7f800000u) S_UNIT[threadIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
             __syncthreads();
         }
-        scan_level<NQ, CNT, PACK, CH>(a, pr, level, set, np, g);
-        if (gridDim.x > 1) { if (!grid_barrier(a, S_MISC + M_OK, ++arrivals)) return; }
+        scan_level<NQ, CNT, PACK, CH, CL>(a, pr, level, set, np, g);
+        if constexpr (CL) {
+            if (a.NR > 1) {
+                __syncthreads();
+                clear_own<NQ, PACK>(a, set, np, g);
+            }
+            if constexpr (!PACK) { __syncthreads(); for (int s = threadIdx.x; s < np; s += T) S_LOW[s] = 0u; }
+            cluster_barrier();
+        } else if (gridDim.x > 1) { if (!grid_barrier(a, S_MISC + M_OK, ++arrivals)) return; }
         else __syncthreads();
-        const bool split = __syncthreads_or(decide(a, pr, nx, level, set)) != 0;
+        const bool split = __syncthreads_or(decide<CL>(a, pr, nx, level, set)) != 0;
         const bool last = level + 1 == a.D || !split;
         if (!last || a.whole) place(a, pr, nx, idx, S_IDX(cur ^ 1), level, cnt, a.xC + row0, last, u0, u1);
         if (last) { // these were the last sums
-            if (a.NR > 1) clear_sums(a, NQ, set, np, level);
+            if (!CL && a.NR > 1) clear_sums(a, NQ, set, np, level);
             break;
         }
         done_np = np;
@@ -751,13 +871,17 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         update_rows<NQ>(a, row0, u0, u1, CNT || PACK);
         if (a.ev_n > 0) evaluate(a);
     }
-    // the CTA that is done last hands the tree over
-    __syncthreads();
-    if (threadIdx.x == 0) S_MISC[M_OK] = arrive(a.bar + 1) == gridDim.x - 1;
-    __syncthreads();
-    if (!S_MISC[M_OK]) return;
-    if (threadIdx.x < 2) a.bar[threadIdx.x] = 0u;
-    if (a.low) for (int i = threadIdx.x; i < a.nn + 2; i += T) a.lowflag[i] = 0u;
+    if constexpr (CL) {
+        cluster_barrier();
+        if (blockIdx.x != 0) return;
+    } else { // the CTA that is done last hands the tree over
+        __syncthreads();
+        if (threadIdx.x == 0) S_MISC[M_OK] = arrive(a.bar + 1) == gridDim.x - 1;
+        __syncthreads();
+        if (!S_MISC[M_OK]) return;
+        if (threadIdx.x < 2) a.bar[threadIdx.x] = 0u;
+        if (a.low) for (int i = threadIdx.x; i < a.nn + 2; i += T) a.lowflag[i] = 0u;
+    }
     if (a.ev_n > 0 && threadIdx.x < 32) {
         double v = 0.0, w = 0.0;
         for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) { v += __ldcg(a.ev_part + 2 * b); w += __ldcg(a.ev_part + 2 * b + 1); }
@@ -768,22 +892,79 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
     publish(a.pub_src, a.pub_dst, a.pub_n);
 }
 
-template <int NQ, bool CNT, bool PACK, int CH>
-cudaError_t launch(const GrowArgs &a, int grid, size_t smem, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(k_grow<NQ, CNT, PACK, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+constexpr int SMEM_MAX = 227 * 1024, MAX_CLUSTER = 16;
+template <int NQ, bool CNT, bool PACK, int CH, bool CL>
+cudaError_t launch(const GrowArgs *a, int grid, size_t smem, cudaStream_t st, int *clusters) {
+    cudaError_t e = cudaFuncSetAttribute(k_grow<NQ, CNT, PACK, CH, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+    if (e == cudaSuccess && CL) e = cudaFuncSetAttribute(k_grow<NQ, CNT, PACK, CH, CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3((unsigned)grid); c.blockDim = dim3(T); c.dynamicSmemBytes = smem; c.stream = st;
     cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
+    if (CL) { at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = (unsigned)grid; at.val.clusterDim.y = at.val.clusterDim.z = 1; }
+    else { at.id = cudaLaunchAttributeCooperative; at.val.cooperative = 1; }
     c.attrs = &at; c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, k_grow<NQ, CNT, PACK, CH>, a);
+    if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_grow<NQ, CNT, PACK, CH, CL>, &c);
+    return cudaLaunchKernelEx(&c, k_grow<NQ, CNT, PACK, CH, CL>, *a);
+}
+template <int NQ, bool CNT, bool PACK, int CH>
+cudaError_t launch(const evb_handle *h, const GrowGeom &g, const GrowArgs *a, int *clusters) {
+    return g.cluster ? launch<NQ, CNT, PACK, CH, true>(a, g.NG * g.NR, g.smem, h->st, clusters) : launch<NQ, CNT, PACK, CH, false>(a, g.NG * g.NR, g.smem, h->st, clusters);
 }
 template <int NQ, bool CNT, bool PACK>
-cudaError_t launch(const GrowArgs &a, int grid, size_t smem, cudaStream_t st) {
-    return a.B <= 32 ? launch<NQ, CNT, PACK, 1>(a, grid, smem, st) : a.B <= 64 ? launch<NQ, CNT, PACK, 2>(a, grid, smem, st)
-         : a.B <= 128 ? launch<NQ, CNT, PACK, 4>(a, grid, smem, st) : launch<NQ, CNT, PACK, 8>(a, grid, smem, st);
+cudaError_t launch(const evb_handle *h, const GrowGeom &g, const GrowArgs *a, int *clusters) {
+    return h->B <= 32 ? launch<NQ, CNT, PACK, 1>(h, g, a, clusters) : h->B <= 64 ? launch<NQ, CNT, PACK, 2>(h, g, a, clusters)
+         : h->B <= 128 ? launch<NQ, CNT, PACK, 4>(h, g, a, clusters) : launch<NQ, CNT, PACK, 8>(h, g, a, clusters);
+}
+// launches the kernel for the handle, or (a == null) finds out how many clusters of its size the GPU holds
+cudaError_t launch(const evb_handle *h, const GrowGeom &g, const GrowArgs *a, int *clusters) {
+    if (h->hgeo.pack) return launch<1, true, true>(h, g, a, clusters);
+    if (h->hgeo.cnt) return launch<2, true, false>(h, g, a, clusters);
+    return h->nq == 2 ? launch<2, false, false>(h, g, a, clusters) : launch<3, false, false>(h, g, a, clusters);
+}
+
+int grow_bits(const evb_handle *h, long long rows_of_cell) { // of the high words
+    int hb = 21, log_n = 0;
+    while (hb > 18 && (1ll << (31 - hb)) - 64 < rows_of_cell) --hb;
+    while ((1ll << log_n) < h->n) ++log_n;
+    return std::min(hb, (61 - log_n) / 2);
+}
+
+// One cluster of CTAs
+bool cluster_geom(const evb_handle *h, GrowGeom &best) {
+    const int B = h->B, D = h->D, NQ = h->nq, P = planes(NQ, h->hgeo.cnt, h->hgeo.pack), M = 1 << std::max(1, D - 2), hs = h->Ce != h->C ? 2 : 3;
+    const size_t small = (size_t)NODE_BYTES * M + MISC_BYTES + (size_t)h->nn * 8 + (size_t)h->F * 4, room = 226 * 1024;
+    double least = 10000.0; // clocks that the rows of the root may take
+    bool found = false;
+    for (int lw = 0; lw <= 2; ++lw) {
+        const int W = 1 << lw, NG = (h->F + 4 * W - 1) / (4 * W);
+        if (NG > MAX_CLUSTER) continue;
+        int NR = (int)std::min<long long>(MAX_CLUSTER / NG, (h->n + 127) / 128);
+        const long long rpc = ((h->n + NR - 1) / NR + 31) & ~31ll;
+        if (rpc > 16000) continue;
+        NR = (int)((h->n + rpc - 1) / rpc);
+        const int lc = lw == 0 ? (rpc > 1024 ? 4 : 3) : lw + 3, R = 1 << (lc - 2 - lw);
+        const double add = (double)rpc / 32 * 4 * W * P * (R == 4 ? 2.0 : 2.9) / 0.87;
+        if (add >= least) continue;
+        GrowGeom g = {};
+        g.on = g.cluster = true; g.lw = lw; g.lc = lc; g.NG = NG; g.NR = NR; g.rpc = (int)rpc; g.fo = (std::min(4 * W, h->F) + NR - 1) / NR;
+        const size_t img = (size_t)(B + 1) * P * 4 << lc, slots = (size_t)M / 2, kept = (size_t)std::max(1, M / 2) + std::max(1, M / 4);
+        size_t o = (size_t)rpc * (4 + 4 * W + 4 * NQ) + small + (((rpc >> 5) + NG - 1) / NG * 64);
+        auto take = [&](size_t bytes) { const size_t at = (o + 15) & ~(size_t)15; o = at + bytes; return at; };
+        const size_t sum = take(slots * g.fo * NQ * B * 8), cnt = take((slots * g.fo * B + slots) * 4), bst = take((size_t)M * h->F * 48);
+        size_t before = o, hist = take(kept * g.fo * hs * B * 8);
+        if (o + img > room) { o = before; hist = 0; }
+        if (o + img + 128 > room) continue;
+        g.fit = (int)std::min<size_t>((room - 128 - o) / img, slots);
+        const size_t base = (size_t)g.fit * img; // the images come first
+        g.o_sum = (int)(base + sum); g.o_cnt = (int)(base + cnt); g.o_best = (int)(base + bst); g.o_hist = hist ? (int)(base + hist) : 0;
+        g.smem = base + o;
+        g.hb = grow_bits(h, rpc / R + 32);
+        int clusters = 0;
+        if (launch(h, g, nullptr, &clusters) != cudaSuccess || clusters < 1) { cudaGetLastError(); continue; }
+        best = g; least = add; found = true;
+    }
+    return found;
 }
 
 } // namespace
@@ -791,7 +972,7 @@ cudaError_t launch(const GrowArgs &a, int grid, size_t smem, cudaStream_t st) {
 // Words of features and rows of a CTA.  Called again when the number of sampled columns changes.
 void evb_grow_configure(evb_handle *h) {
     GrowGeom &g = h->grow;
-    g.on = false;
+    g = GrowGeom{};
     const int loss = h->p.loss, D = h->D, B = h->B;
     const bool gh = loss == EVB_MSE || loss == EVB_LOGLOSS || loss == EVB_POISSON || loss == EVB_GAMMA || loss == EVB_TWEEDIE;
     // Every CTA empties an image per slot and feature group into sums that all row ranges share, whatever few rows the slot has there: that is
@@ -802,6 +983,10 @@ void evb_grow_configure(evb_handle *h) {
     if (!gh || h->K != 1 || h->use_q2 || h->p.tree_type == 1 || D < 2 || D > MAX_D || (h->p.flags & EVB_FLAG_FULL_PARTITION) || h->nfeats > 65535) return;
     const int NQ = h->nq, P = planes(NQ, h->hgeo.cnt, h->hgeo.pack), M = 1 << std::max(1, D - 2);
     const size_t img = (size_t)(B + 1) * P * 128, small = (size_t)NODE_BYTES * M + MISC_BYTES + (size_t)h->nn * 8 + (size_t)h->F * 4, room = 226 * 1024;
+    if (cluster_geom(h, g)) {
+        if (!h->hgeo.pack) { h->hgeo.hb = g.hb; h->hgeo.TE = (1 << (26 - g.hb)) - 1; }
+        return;
+    }
     if (((size_t)img << (D - 2)) > (size_t)(D - 1) * 300 * 1024) return;
     double best = 0.0;
     for (int lw = 0; lw <= 2; ++lw) {
@@ -821,15 +1006,11 @@ void evb_grow_configure(evb_handle *h) {
         const double add = (double)rpc * 4 * W * P / 25.0 * D / 2.0, fl = (double)NR * h->F * B * P * (1 << (D - 2)) / 400.0;
         if (g.on && add + fl >= best) continue;
         best = add + fl;
-        g.on = true; g.lw = lw; g.NG = NG; g.NR = NR; g.rpc = (int)rpc;
+        g.on = true; g.lw = lw; g.lc = 5; g.NG = NG; g.NR = NR; g.rpc = (int)rpc;
         const size_t rows = (size_t)(rpc * pr) + (size_t)(((rpc >> 5) + NG - 1) / NG * 64); // and the leaves of those it updates
         g.fit = (int)std::min<size_t>((room - small - rows) / img, (size_t)std::max(1, M / 2));
         g.smem = (size_t)g.fit * img + small + rows;
-        int hb = 21;
-        while (hb > 18 && (1ll << (31 - hb)) - 64 < rpc * W / 8 + 32) --hb;
-        int log_n = 0;
-        while ((1ll << log_n) < h->n) ++log_n;
-        g.hb = std::min(hb, (61 - log_n) / 2);
+        g.hb = grow_bits(h, rpc * W / 8 + 32);
     }
     if (g.on && !h->hgeo.pack) { h->hgeo.hb = g.hb; h->hgeo.TE = (1 << (26 - g.hb)) - 1; } // how k_tree_begin scales g
 }
@@ -855,7 +1036,8 @@ int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot,
     a.F = h->F; a.B = h->B; a.D = h->D; a.hist_nodes = h->hist_nodes; a.loss = h->p.loss; a.elide = h->Ce != h->C; a.hb = h->hgeo.hb; a.ng = h->ng; a.nn = h->nn;
     a.round_bits = evb_hg_round_bits(h);
     a.NG = g.NG; a.NR = g.NR; a.rpc = g.rpc; a.lw = g.lw; a.fit = g.fit; a.M = 1 << std::max(1, h->D - 2);
-    const size_t img = (size_t)(h->B + 1) * planes(h->nq, h->hgeo.cnt, h->hgeo.pack) * 128;
+    const size_t img = (size_t)(h->B + 1) * planes(h->nq, h->hgeo.cnt, h->hgeo.pack) * 4 << g.lc;
+    a.lc = g.lc; a.o_sum = g.o_sum; a.o_cnt = g.o_cnt; a.o_best = g.o_best; a.o_hist = g.o_hist; a.fo = g.fo;
     a.o_x = (int)(g.fit * img); a.o_q = a.o_x + (g.rpc * 4 << g.lw); a.o_idx = a.o_q + g.rpc * 4 * h->nq; a.o_node = a.o_idx + g.rpc * 4;
     a.max_polls = 8000000u; // seconds
     a.low_unit = evb_hg_low_unit(h); a.neb = -h->p.eta / (double)h->p.bagging_size;
@@ -870,13 +1052,8 @@ int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot,
             a.ev_RS = h->RS; a.ev_metric = h->ev_metric;
         }
     }
-    const int grid = g.NG * g.NR;
-    cudaError_t e;
     evb_tic(h, EVB_T_HIST);
-    if (h->hgeo.pack) e = launch<1, true, true>(a, grid, g.smem, h->st);
-    else if (h->hgeo.cnt) e = launch<2, true, false>(a, grid, g.smem, h->st);
-    else if (h->nq == 2) e = launch<2, false, false>(a, grid, g.smem, h->st);
-    else e = launch<3, false, false>(a, grid, g.smem, h->st);
+    const cudaError_t e = launch(h, g, &a, nullptr);
     evb_toc(h, EVB_T_HIST);
     EVB_CUDA(e);
     return EVB_OK;
