@@ -91,7 +91,7 @@ struct Pairs { // state of a level: slot = parent's number in its level (at leve
     __device__ __forceinline__ int *en() const { return reinterpret_cast<int *>(b + 36 * M); }
     __device__ __forceinline__ uint32_t *dec() const { return reinterpret_cast<uint32_t *>(b + 40 * M); } // the parents' splits (packed as in t_packed); 0: none
 };
-constexpr int PAIR_BYTES = 48, NODE_BYTES = 2 * PAIR_BYTES + 8, MISC_BYTES = 512;
+constexpr int PAIR_BYTES = 48, NODE_BYTES = 2 * PAIR_BYTES + 8 + 32, MISC_BYTES = 512;
 extern __shared__ __align__(128) unsigned char s_raw[];
 // image(s), bins [word][row], words of gradients [channel][row], row lists, then per node of a level
 #define S_IMG (reinterpret_cast<uint32_t *>(s_raw))
@@ -101,6 +101,7 @@ extern __shared__ __align__(128) unsigned char s_raw[];
 #define S_PAIRS(cur) (Pairs{s_raw + a.o_node + (cur) * PAIR_BYTES * a.M, a.M})
 #define S_CL (reinterpret_cast<int *>(s_raw + a.o_node + 2 * PAIR_BYTES * a.M))                                    /* cursors of the partition */
 #define S_CR (reinterpret_cast<int *>(s_raw + a.o_node + (2 * PAIR_BYTES + 4) * a.M))
+#define S_OUT (reinterpret_cast<double4 *>(s_raw + a.o_node + (2 * PAIR_BYTES + 8) * a.M))                          /* [node] left sums, gain */
 #define S_MISC (reinterpret_cast<int *>(s_raw + a.o_node + NODE_BYTES * a.M))
 #define S_UNIT (reinterpret_cast<double *>(s_raw + a.o_node + NODE_BYTES * a.M + 64))                              /* units of the channels' sums */
 #define S_ROOT (reinterpret_cast<double *>(s_raw + a.o_node + NODE_BYTES * a.M + 96))                               /* sums of the root (one cluster) */
@@ -129,16 +130,21 @@ __device__ __forceinline__ void remote_put(uint32_t at, double x, double y) {
     asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(at), "d"(x), "d"(y) : "memory");
 }
 __device__ __forceinline__ void remote_put(uint32_t at, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
-__device__ __forceinline__ void cluster_barrier() {
+template <typename F>
+__device__ __forceinline__ void cluster_barrier(F meanwhile) {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    meanwhile();
+    __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_barrier() { cluster_barrier([] {}); }
 
 // All CTAs have arrived `k` times.  The launch is cooperative, so all of them run; the wait is bounded all the same: a CTA whose
 // wait runs out (or that sees another's has) leaves an error word and the kernel ends.
-__device__ __forceinline__ bool grid_barrier(const GrowArgs &a, int *ok, unsigned k) {
+template <typename F>
+__device__ __forceinline__ bool grid_barrier(const GrowArgs &a, int *ok, unsigned k, F meanwhile) {
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == T - 1) {
         const uint32_t target = k * gridDim.x;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
         bool good = false;
@@ -153,7 +159,7 @@ __device__ __forceinline__ bool grid_barrier(const GrowArgs &a, int *ok, unsigne
             if (a.pub_dst) reinterpret_cast<volatile int *>(a.pub_dst)[a.pub_err] = EVB_DERR_GRID;
         }
         *ok = good;
-    }
+    } else meanwhile();
     __syncthreads();
     return *ok != 0;
 }
@@ -238,16 +244,20 @@ template <int NQ, bool CNT, bool PACK, int LW, int LC, bool CL>
 __device__ __forceinline__ void flush(const GrowArgs &a, const Pairs &pr, int set, int s0, int s1, int g, bool second) {
     constexpr int P = planes(NQ, CNT, PACK), W = 1 << LW, COLS = 1 << LC, R = 1 << (LC - 2 - LW), FB = LW == 0 ? 4 : 8, BO = 32 / FB, NC = 4 * W / FB;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, bo = lane % BO, f0 = g * 4 * W;
-    const int nbb = (a.B + BO - 1) / BO, per = NC * nbb, slot_words = (a.B + 1) * P * COLS;
+    const int nbb = (a.B + BO - 1) / BO, slot_words = (a.B + 1) * P * COLS;
     const bool own = a.NR == 1; // no other CTA adds to these cells
-    for (int u = wid; u < (s1 - s0) * per; u += NW) {
-        const int s = u / per, e = u - s * per, ch = e / nbb, bin = (e - ch * nbb) * BO + bo, f = ch * FB + lane / BO, slot = s0 + s;
+    int base = 0;
+    for (int slot = s0; slot < s1; ++slot) {
         if (!pr.dec()[slot] || (!own && pr.st()[slot] == pr.en()[slot])) continue;
+#pragma unroll
+    for (int ch = 0; ch < NC; ++ch, base += nbb)
+    for (int bb = (wid - base) & (NW - 1); bb < nbb; bb += NW) {
+        const int bin = bb * BO + bo, f = ch * FB + lane / BO;
         if (bin >= a.B) continue;
-        uint32_t *p = S_IMG + (size_t)s * slot_words + (size_t)(bin + 1) * (P * COLS) + f;
+        uint32_t *p = S_IMG + (slot - s0) * slot_words + (bin + 1) * (P * COLS) + f;
         const bool out = f0 + f < a.F;
         // where the sums go: this CTA's share of the features (CL), CTA f % NR of the group's, or global memory
-        const int lf = CL ? f / a.NR : 0, rank = CL ? (f - lf * a.NR) * a.NG + g : 0;
+        const int lf = CL ? own ? f : f / a.NR : 0, rank = CL ? (f - lf * a.NR) * a.NG + g : 0;
         const size_t cell = CL && !second ? (size_t)slot * a.fo + lf : (size_t)slot * a.F + (f0 + f);
         auto put = [&](int c, unsigned long long v) {
             const size_t at = (cell * NQ + c) * a.B + bin;
@@ -303,6 +313,7 @@ __device__ __forceinline__ void flush(const GrowArgs &a, const Pairs &pr, int se
                 if (out) put(c, (unsigned long long)((hi << (a.hb + 1)) + lo));
             }
         }
+    }
     }
 }
 
@@ -432,7 +443,7 @@ __device__ __forceinline__ void scan(const GrowArgs &a, int level, int set, int 
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
         const double w_l = w[i], w_r = sw - w_l;
-        double v = term_gh(g[i], h[i], w_l, a.lambda, a.L2) + term_gh(sg - g[i], sh - h[i], w_r, a.lambda, a.L2);
+        double v = terms_gh(g[i], h[i], w_l, sg - g[i], sh - h[i], w_r, a.lambda, a.L2);
         bool ok = bin0 + i < b_max && w_l > a.min_weight && w_r > a.min_weight;
         if (constraint != 0) { // pred_scalar on left / right sums (src/predict.jl:205-208, 235-238)
             const double pl = a.neb * g[i] / fmax(DBL_EPSILON, h[i] + a.lambda * w_l + a.L2);
@@ -469,8 +480,9 @@ __device__ __forceinline__ void scan_level(const GrowArgs &a, const Pairs &pr, i
     const int f0 = own ? g * (4 << a.lw) + r : 0, nf = CL ? (in_group - r + stride - 1) / stride : own ? in_group : a.F;
     if (nf <= 0) return;
     const int total = (np * nf) << both, step = own ? NW : NW * (int)gridDim.x;
+    const float per_nf = 1.0f / (float)nf;
     for (int t = own ? wid : wid * (int)gridDim.x + (int)blockIdx.x; t < total; t += step) {
-        const int which = t & both, e = t >> both, s = e / nf, lf = e - s * nf, f = f0 + lf * stride;
+        const int which = t & both, e = t >> both, s = (int)(((float)e + 0.5f) * per_nf), lf = e - s * nf, f = f0 + lf * stride; // (e / nf: fewer than 2^20 of them)
         if (!pr.dec()[s]) continue;
         const int c = pr.build()[s] ^ which, j = 2 * s + c;
         scan<NQ, CNT, PACK, CH, CL>(a, level, set, s, f, lf, (1 << (level - 1)) + j, j, which != 0, pr.sum() + 3 * j);
@@ -480,8 +492,7 @@ __device__ __forceinline__ void scan_level(const GrowArgs &a, const Pairs &pr, i
 // ---------------------------------------------------------------------------------------------- decisions
 __device__ __forceinline__ float leaf_of(const GrowArgs &a, double g, double h, double w) { return (float)(a.neb * g / fmax(DBL_EPSILON, h + a.lambda * w + a.L2)); }
 
-// Every CTA decides every node, a warp per node, and so knows the slots of the next level; CTA j of the grid writes what belongs to
-// node j.  The child with the smaller weight is built, the left one when they are equal (with unit weights the reference's rule on
+// Every CTA decides every node, a warp per node, and so knows the slots of the next level.  The child with the smaller weight is built, the left one when they are equal (with unit weights the reference's rule on
 // row counts, src/fit.jl:123-129).  Returns whether the thread's warp has split a node.
 template <bool CL>
 __device__ __forceinline__ bool decide(const GrowArgs &a, const Pairs &pr, const Pairs &nx, int level, int set) {
@@ -529,18 +540,28 @@ __device__ __forceinline__ bool decide(const GrowArgs &a, const Pairs &pr, const
             nx.st()[j] = has ? st : en; nx.mid()[j] = en; nx.en()[j] = en;
             S_CL[j] = st; S_CR[j] = en;
         }
-        if (j % gridDim.x != blockIdx.x) continue;
-        a.t_w[n - 1] = (float)s2;
-        if (!has) { a.t_pred[n - 1] = S_VALUE[n - 1]; continue; }
-        double *c = a.nsum + (size_t)6 * n;
-        c[0] = l1.x; c[1] = l1.y; c[2] = l2.x; c[3] = r0; c[4] = r1; c[5] = r2;
-        a.t_gain[n - 1] = (float)bg; a.t_bin[n - 1] = (uint8_t)(bb + 1); a.t_feat[n - 1] = (int32_t)(packed & 0xffffu) + 1; a.t_split[n - 1] = 1; a.t_packed[n - 1] = packed;
-        if (level + 1 == a.D) {
-            a.t_pred[2 * n - 1] = S_VALUE[2 * n - 1]; a.t_pred[2 * n] = S_VALUE[2 * n];
-            a.t_w[2 * n - 1] = (float)l2.x; a.t_w[2 * n] = (float)r2;
-        } else atomicAdd(&a.plan[level + 1].nbuild, 1);
+        if (level == 1) { pr.sum()[0] = s0; pr.sum()[1] = s1; pr.sum()[2] = s2; }
+        S_OUT[j] = make_double4(l1.x, l1.y, l2.x, bg);
     }
     return any;
+}
+// What a level has decided goes to the tree in global memory while the CTA waits for others
+__device__ __forceinline__ void record(const GrowArgs &a, const Pairs &pr, int level) {
+    const int nodes = 1 << (level - 1), j = (int)(blockIdx.x + gridDim.x * threadIdx.x);
+    if (j >= nodes || !pr.dec()[j >> 1]) return; // CTA j % gridDim.x writes what belongs to node j (the grid has no fewer than 2^9 threads)
+    const int n = nodes + j;
+    const uint32_t packed = S_TREE[n - 1];
+    const double s0 = pr.sum()[3 * j], s1 = pr.sum()[3 * j + 1], s2 = pr.sum()[3 * j + 2];
+    a.t_w[n - 1] = (float)s2;
+    if (!packed) { a.t_pred[n - 1] = S_VALUE[n - 1]; return; }
+    const double4 l = S_OUT[j];
+    double *c = a.nsum + (size_t)6 * n;
+    c[0] = l.x; c[1] = l.y; c[2] = l.z; c[3] = s0 - l.x; c[4] = s1 - l.y; c[5] = s2 - l.z;
+    a.t_gain[n - 1] = (float)l.w; a.t_bin[n - 1] = (uint8_t)((packed >> 16) & 0xffu); a.t_feat[n - 1] = (int32_t)(packed & 0xffffu) + 1; a.t_split[n - 1] = 1; a.t_packed[n - 1] = packed;
+    if (level + 1 == a.D) {
+        a.t_pred[2 * n - 1] = S_VALUE[2 * n - 1]; a.t_pred[2 * n] = S_VALUE[2 * n];
+        a.t_w[2 * n - 1] = (float)l.z; a.t_w[2 * n] = (float)(s2 - l.z);
+    } else atomicAdd(&a.plan[level + 1].nbuild, 1);
 }
 
 // The CTA's rows to the children of the nodes that split: left rows from the start of the node's places, right rows from its end.  Every
@@ -560,50 +581,87 @@ __device__ __forceinline__ void place(const GrowArgs &a, const Pairs &pr, const 
         const unsigned m = __ballot_sync(FULL, i < nodes && ((i & 1) ? pr.en()[s] : pr.mid()[s]) > p);
         if (m) { j += __ffs(m) - 1; break; }
     }
-    for (; j < nodes; ++j) {
-        const int s = j >> 1, st = (j & 1) ? pr.mid()[s] : pr.st()[s], en = (j & 1) ? pr.en()[s] : pr.mid()[s];
-        p = max(p, st);
+    auto end_of = [&](int i) { return (i & 1) ? pr.en()[i >> 1] : pr.mid()[i >> 1]; };
+    auto start_of = [&](int i) { return (i & 1) ? pr.mid()[i >> 1] : pr.st()[i >> 1]; };
+    const uint32_t n_up = (uint32_t)(u1 - u0);
+    while (p < pend) {
+        while (j < nodes && end_of(j) <= p) ++j;
+        if (j >= nodes) break;
+        p = max(p, start_of(j));
         if (p >= pend) break;
-        const uint32_t dec = nx.dec()[j], bin = (dec >> 16) & 0xffu, lo = (dec >> 25) & 1u ? 0u : bin, span = bin - lo; // left: lo <= x <= bin
-        const uint8_t *xf = xrows + (size_t)(dec & 0xffffu) * a.n;
-        const int lim = min(pend, en);
-        if (dec && !last) {
-            for (; p < lim; p += 32 * U) {
-                uint32_t row[U], x[U];
-                unsigned l[U];
+        const int lim = min(pend, end_of(j));
+        if (p >= lim) continue; // nothing of the node is left, and what lies before it belongs to nodes that have ended
+        if (lim - p >= 64 || lim == pend) { // one node
+            const uint32_t dec = nx.dec()[j], bin = (dec >> 16) & 0xffu, lo = (dec >> 25) & 1u ? 0u : bin, span = bin - lo; // left: lo <= x <= bin
+            const uint8_t *xf = xrows + (size_t)(dec & 0xffffu) * a.n;
+            if (dec && !last) {
+                for (; p < lim; p += 32 * U) {
+                    uint32_t row[U], x[U];
+                    unsigned l[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) { const int q = p + 32 * u + lane; row[u] = q < lim ? in[q] : 0xffffu; }
+                    for (int u = 0; u < U; ++u) { const int q = p + 32 * u + lane; row[u] = q < lim ? in[q] : 0xffffu; }
 #pragma unroll
-                for (int u = 0; u < U; ++u) x[u] = row[u] != 0xffffu ? (uint32_t)__ldg(xf + row[u]) : 0u;
-                int nl = 0;
+                    for (int u = 0; u < U; ++u) x[u] = row[u] != 0xffffu ? (uint32_t)__ldg(xf + row[u]) : 0u;
+                    int nl = 0;
 #pragma unroll
-                for (int u = 0; u < U; ++u) { l[u] = __ballot_sync(FULL, row[u] != 0xffffu && x[u] - lo <= span); nl += __popc(l[u]); }
-                const int nr = min(lim - p, 32 * U) - nl;
-                int at = 0;
-                if (lane == 0) at = atomicAdd(S_CL + j, nl);
-                if (lane == 1) at = atomicSub(S_CR + j, nr) - nr;
-                int dl = __shfl_sync(FULL, at, 0), dr = __shfl_sync(FULL, at, 1);
+                    for (int u = 0; u < U; ++u) { l[u] = __ballot_sync(FULL, row[u] != 0xffffu && x[u] - lo <= span); nl += __popc(l[u]); }
+                    const int nr = min(lim - p, 32 * U) - nl;
+                    int at = 0;
+                    if (lane == 0) at = atomicAdd(S_CL + j, nl);
+                    if (lane == 1) at = atomicSub(S_CR + j, nr) - nr;
+                    int dl = __shfl_sync(FULL, at, 0), dr = __shfl_sync(FULL, at, 1);
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int b = __popc(l[u] & below);
-                    if (row[u] != 0xffffu) out[(l[u] >> lane) & 1u ? dl + b : dr + lane - b] = (uint16_t)row[u];
-                    dl += __popc(l[u]); dr += 32 - __popc(l[u]);
+                    for (int u = 0; u < U; ++u) {
+                        const int b = __popc(l[u] & below);
+                        if (row[u] != 0xffffu) out[(l[u] >> lane) & 1u ? dl + b : dr + lane - b] = (uint16_t)row[u];
+                        dl += __popc(l[u]); dr += 32 - __popc(l[u]);
+                    }
+                }
+            } else if (a.whole) {
+                const uint32_t id = dec ? 2u * (uint32_t)(nodes + j) : (uint32_t)(nodes + j);
+                for (; p < lim; p += 32 * U) {
+                    uint32_t row[U], x[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) { const int q = p + 32 * u + lane; row[u] = q < lim ? (uint32_t)in[q] - (uint32_t)u0 : 0xffffffffu; }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) x[u] = dec && row[u] < n_up ? (uint32_t)__ldg(xf + u0 + row[u]) : 0u;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) if (row[u] < n_up) S_LEAF[row[u]] = (uint16_t)(id + (dec && x[u] - lo > span ? 1u : 0u));
                 }
             }
-        } else if (a.whole) {
-            const uint32_t id = dec ? 2u * (uint32_t)(nodes + j) : (uint32_t)(nodes + j), n_up = (uint32_t)(u1 - u0);
-            for (; p < lim; p += 32 * U) {
-                uint32_t row[U], x[U];
+            p = lim;
+        } else { // several small ones: every lane finds its row's node, lanes of one child share a reservation
+            uint32_t key[2], row[2], dec[2], x[2];
 #pragma unroll
-                for (int u = 0; u < U; ++u) { const int q = p + 32 * u + lane; row[u] = q < lim ? (uint32_t)in[q] - (uint32_t)u0 : 0xffffffffu; }
-#pragma unroll
-                for (int u = 0; u < U; ++u) x[u] = dec && row[u] < n_up ? (uint32_t)__ldg(xf + u0 + row[u]) : 0u;
-#pragma unroll
-                for (int u = 0; u < U; ++u) if (row[u] < n_up) S_LEAF[row[u]] = (uint16_t)(id + (dec && x[u] - lo > span ? 1u : 0u));
+            for (int u = 0; u < 2; ++u) {
+                const int q = p + 32 * u + lane;
+                int l = j, r = nodes - 1; // first node that ends behind q
+                while (l < r) { const int m = (l + r) >> 1; if (end_of(m) > q) r = m; else l = m + 1; }
+                const bool act = q < pend && q < end_of(l) && q >= start_of(l);
+                row[u] = act ? (uint32_t)in[q] : 0xffffu;
+                dec[u] = act ? nx.dec()[l] : 0u;
+                key[u] = act ? (uint32_t)l + 1u : 0u;
+                const bool look = dec[u] && (!last || row[u] - (uint32_t)u0 < n_up);
+                x[u] = look ? (uint32_t)__ldg(xrows + (size_t)(dec[u] & 0xffffu) * a.n + row[u]) : 0u;
             }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t bin = (dec[u] >> 16) & 0xffu, lo = (dec[u] >> 25) & 1u ? 0u : bin, child = x[u] - lo <= bin - lo ? 0u : 1u;
+                const bool moves = dec[u] && !last;
+                if (key[u] && !moves && a.whole && row[u] - (uint32_t)u0 < n_up) {
+                    const uint32_t n = (uint32_t)nodes + key[u] - 1u;
+                    S_LEAF[row[u] - u0] = (uint16_t)(dec[u] ? 2u * n + child : n);
+                }
+                if (last) continue;
+                const unsigned peers = __match_any_sync(FULL, moves ? 2u * key[u] + child : 0u);
+                const int c = __popc(peers);
+                int at = 0;
+                if (moves && (peers & below) == 0u) at = child ? atomicSub(S_CR + (key[u] - 1u), c) - c : atomicAdd(S_CL + (key[u] - 1u), c);
+                at = __shfl_sync(FULL, at, __ffs(peers) - 1);
+                if (moves) out[at + __popc(peers & below)] = (uint16_t)row[u];
+            }
+            p += 64;
         }
-        p = lim;
-        if (en > pend) break;
     }
 }
 
@@ -682,12 +740,13 @@ __device__ __forceinline__ void evaluate(const GrowArgs &a) {
 }
 
 // bins of the CTA's features, a 32-bit word for four of them: [word][row]
+__device__ __forceinline__ uint32_t column(const GrowArgs &a, int f) { return a.js_inline ? a.js[f] : a.js0 ? a.js0[f] : (uint32_t)f; }
 __device__ __forceinline__ void load_bins(const GrowArgs &a, uint32_t *x, int f0, long long row0, int nr) {
     const int quads = (nr + 3) >> 2;
     for (int w = 0; w < 1 << a.lw; ++w) {
         const uint8_t *col[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) { const int f = f0 + 4 * w + k; col[k] = f < a.F ? a.xC + (size_t)(S_FEAT[f] & 0xffffu) * a.n + row0 : nullptr; }
+        for (int k = 0; k < 4; ++k) { const int f = f0 + 4 * w + k; col[k] = f < a.F ? a.xC + (size_t)column(a, f) * a.n + row0 : nullptr; }
 #pragma unroll 2
         for (int e = threadIdx.x; e < quads; e += T) {
             uint32_t v[4];
@@ -750,7 +809,7 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         root.dec()[0] = 1u; root.build()[0] = 0; root.st()[0] = 0;
     }
     for (int f = threadIdx.x; f < a.F; f += T) {
-        const uint32_t feat = a.js_inline ? a.js[f] : a.js0 ? a.js0[f] : (uint32_t)f;
+        const uint32_t feat = column(a, f);
         const int mono = a.mono[feat];
         S_FEAT[f] = feat | (a.feattypes[feat] != 0 ? 1u << 16 : 0u) | (mono >= -1 && mono <= 1 ? (uint32_t)(mono + 1) : 3u) << 17;
     }
@@ -764,6 +823,14 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
             }
         }
     }
+    // rows on their way to shared memory before anything waits: gradients as they are, scaled in place when the scale is known
+    const float *rec = a.grad + (size_t)row0 * NQ;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nr; i += T) {
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) S_Q[c * a.rpc + i] = __float_as_int(__ldcg(rec + (size_t)i * NQ + c));
+    }
+    load_bins(a, S_X, f0, row0, nr);
     if (threadIdx.x < NQ) {
         double unit;
         const Quant k = quant_of(a.gmax[threadIdx.x], PACK, a.hb, a.round_bits, &unit);
@@ -785,15 +852,11 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         Quant k[NQ];
 #pragma unroll
         for (int c = 0; c < NQ; ++c) k[c] = S_QUANT[c];
-#pragma unroll 4
         for (int i = threadIdx.x; i < nr; i += T) {
-            const float *rec = a.grad + (size_t)(row0 + i) * NQ;
 #pragma unroll
-            for (int c = 0; c < NQ; ++c) S_Q[c * a.rpc + i] = quant(k[c], __ldcg(rec + c), a.signs + c, a.qinv + c);
+            for (int c = 0; c < NQ; ++c) S_Q[c * a.rpc + i] = quant(k[c], __int_as_float(S_Q[c * a.rpc + i]), a.signs + c, a.qinv + c);
         }
     }
-    load_bins(a, S_X, f0, row0, nr);
-    __syncthreads();
     if (!a.mask) for (int i = threadIdx.x; i < nr; i += T) S_IDX(0)[i] = (uint16_t)i;
     else
         for (int i0 = (int)threadIdx.x - lane; i0 < nr; i0 += T) {
@@ -817,6 +880,7 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         const int cur = (level - 1) & 1, set = level & 1;
         const Pairs pr = S_PAIRS(cur), nx = S_PAIRS(cur ^ 1);
         const uint16_t *idx = S_IDX(cur);
+        auto write_out = [&] { if (level > 1) record(a, nx, level - 1); }; // (nx: still the level before)
         if constexpr (CL) {
             if (a.lw == 0 && a.lc == 3) hist_level<NQ, CNT, PACK, 0, 3, true>(a, pr, idx, np, set, g, level);
             else if (a.lw == 0) hist_level<NQ, CNT, PACK, 0, 4, true>(a, pr, idx, np, set, g, level);
@@ -828,7 +892,7 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
             else if (a.lw == 1) hist_level<NQ, CNT, PACK, 1, 5, false>(a, pr, idx, np, set, g, level);
             else hist_level<NQ, CNT, PACK, 2, 5, false>(a, pr, idx, np, set, g, level);
             if (a.NR > 1) {
-                if (!grid_barrier(a, S_MISC + M_OK, ++arrivals)) return;
+                if (!grid_barrier(a, S_MISC + M_OK, ++arrivals, [] {})) return;
                 if (level > 1) clear_sums(a, NQ, set ^ 1, done_np, level - 1);
             }
         }
@@ -843,13 +907,14 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
                 clear_own<NQ, PACK>(a, set, np, g);
             }
             if constexpr (!PACK) { __syncthreads(); for (int s = threadIdx.x; s < np; s += T) S_LOW[s] = 0u; }
-            cluster_barrier();
-        } else if (gridDim.x > 1) { if (!grid_barrier(a, S_MISC + M_OK, ++arrivals)) return; }
-        else __syncthreads();
+            cluster_barrier(write_out);
+        } else if (gridDim.x > 1) { if (!grid_barrier(a, S_MISC + M_OK, ++arrivals, write_out)) return; }
+        else { write_out(); __syncthreads(); }
         const bool split = __syncthreads_or(decide<CL>(a, pr, nx, level, set)) != 0;
         const bool last = level + 1 == a.D || !split;
         if (!last || a.whole) place(a, pr, nx, idx, S_IDX(cur ^ 1), level, cnt, a.xC + row0, last, u0, u1);
         if (last) { // these were the last sums
+            record(a, pr, level);
             if (!CL && a.NR > 1) clear_sums(a, NQ, set, np, level);
             break;
         }
