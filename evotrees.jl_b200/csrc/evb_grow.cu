@@ -91,7 +91,7 @@ struct Pairs { // state of a level: slot = parent's number in its level (at leve
     __device__ __forceinline__ int *en() const { return reinterpret_cast<int *>(b + 36 * M); }
     __device__ __forceinline__ uint32_t *dec() const { return reinterpret_cast<uint32_t *>(b + 40 * M); } // the parents' splits (packed as in t_packed); 0: none
 };
-constexpr int PAIR_BYTES = 48, NODE_BYTES = 2 * PAIR_BYTES + 8 + 32, MISC_BYTES = 512;
+constexpr int PAIR_BYTES = 48, NODE_BYTES = 2 * PAIR_BYTES + 8 + 32, MISC_BYTES = 512; // (8: the cursors of right rows, and room)
 extern __shared__ __align__(128) unsigned char s_raw[];
 // image(s), bins [word][row], words of gradients [channel][row], row lists, then per node of a level
 #define S_IMG (reinterpret_cast<uint32_t *>(s_raw))
@@ -99,12 +99,12 @@ extern __shared__ __align__(128) unsigned char s_raw[];
 #define S_Q (reinterpret_cast<int32_t *>(s_raw + a.o_q))
 #define S_IDX(cur) (reinterpret_cast<uint16_t *>(s_raw + a.o_idx + (cur) * 2 * a.rpc))
 #define S_PAIRS(cur) (Pairs{s_raw + a.o_node + (cur) * PAIR_BYTES * a.M, a.M})
-#define S_CL (reinterpret_cast<int *>(s_raw + a.o_node + 2 * PAIR_BYTES * a.M))                                    /* cursors of the partition */
-#define S_CR (reinterpret_cast<int *>(s_raw + a.o_node + (2 * PAIR_BYTES + 4) * a.M))
+#define S_CR (reinterpret_cast<int *>(s_raw + a.o_node + 2 * PAIR_BYTES * a.M))                                    /* where a node's right rows begin so far */
 #define S_OUT (reinterpret_cast<double4 *>(s_raw + a.o_node + (2 * PAIR_BYTES + 8) * a.M))                          /* [node] left sums, gain */
 #define S_MISC (reinterpret_cast<int *>(s_raw + a.o_node + NODE_BYTES * a.M))
 #define S_UNIT (reinterpret_cast<double *>(s_raw + a.o_node + NODE_BYTES * a.M + 64))                              /* units of the channels' sums */
 #define S_ROOT (reinterpret_cast<double *>(s_raw + a.o_node + NODE_BYTES * a.M + 96))                               /* sums of the root (one cluster) */
+#define S_INF (S_MISC + 8)                                                                                          /* [NQ] the channel has an infinity */
 #define S_RED (reinterpret_cast<double *>(s_raw + a.o_node + NODE_BYTES * a.M + 128))                              /* [2 NW] */
 #define S_QUANT (reinterpret_cast<Quant *>(s_raw + a.o_node + NODE_BYTES * a.M + 128))                             /* [NQ], while the rows are loaded */
 #define S_TREE (reinterpret_cast<uint32_t *>(s_raw + a.o_node + NODE_BYTES * a.M + MISC_BYTES))                    /* [nn] packed nodes */
@@ -116,7 +116,7 @@ extern __shared__ __align__(128) unsigned char s_raw[];
 #define S_CNTS (reinterpret_cast<uint32_t *>(s_raw + a.o_cnt))           /* [slot][fo][B], then [slot] nonzero: the slot has something in `low` */
 #define S_LOW (S_CNTS + (a.M / 2) * a.fo * a.B)
 #define S_BEST (reinterpret_cast<double2 *>(s_raw + a.o_best))           /* [node][F][3], of all features */
-enum { M_LEFT = 0, M_OK = 1, M_CNT = 2, M_INF = 3, M_MAX = 4 }; // M_MAX: two words
+enum { M_LEFT = 0, M_OK = 1, M_CNT = 2, M_MAX = 4 }; // M_MAX: two words
 
 // shared memory of CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t remote(const void *p, int rank) {
@@ -537,8 +537,8 @@ __device__ __forceinline__ bool decide(const GrowArgs &a, const Pairs &pr, const
             double *ns = nx.sum() + 6 * j;
             ns[0] = l1.x; ns[1] = l1.y; ns[2] = l2.x; ns[3] = r0; ns[4] = r1; ns[5] = r2;
             nx.build()[j] = r2 >= l2.x ? 0 : 1;
-            nx.st()[j] = has ? st : en; nx.mid()[j] = en; nx.en()[j] = en;
-            S_CL[j] = st; S_CR[j] = en;
+            nx.st()[j] = has ? st : en; nx.mid()[j] = has ? st : en; nx.en()[j] = en; // mid: grows while the rows are placed
+            S_CR[j] = en;
         }
         if (level == 1) { pr.sum()[0] = s0; pr.sum()[1] = s1; pr.sum()[2] = s2; }
         S_OUT[j] = make_double4(l1.x, l1.y, l2.x, bg);
@@ -607,7 +607,7 @@ __device__ __forceinline__ void place(const GrowArgs &a, const Pairs &pr, const 
                     for (int u = 0; u < U; ++u) { l[u] = __ballot_sync(FULL, row[u] != 0xffffu && x[u] - lo <= span); nl += __popc(l[u]); }
                     const int nr = min(lim - p, 32 * U) - nl;
                     int at = 0;
-                    if (lane == 0) at = atomicAdd(S_CL + j, nl);
+                    if (lane == 0) at = atomicAdd(nx.mid() + j, nl);
                     if (lane == 1) at = atomicSub(S_CR + j, nr) - nr;
                     int dl = __shfl_sync(FULL, at, 0), dr = __shfl_sync(FULL, at, 1);
 #pragma unroll
@@ -656,7 +656,7 @@ __device__ __forceinline__ void place(const GrowArgs &a, const Pairs &pr, const 
                 const unsigned peers = __match_any_sync(FULL, moves ? 2u * key[u] + child : 0u);
                 const int c = __popc(peers);
                 int at = 0;
-                if (moves && (peers & below) == 0u) at = child ? atomicSub(S_CR + (key[u] - 1u), c) - c : atomicAdd(S_CL + (key[u] - 1u), c);
+                if (moves && (peers & below) == 0u) at = child ? atomicSub(S_CR + (key[u] - 1u), c) - c : atomicAdd(nx.mid() + (key[u] - 1u), c);
                 at = __shfl_sync(FULL, at, __ffs(peers) - 1);
                 if (moves) out[at + __popc(peers & below)] = (uint16_t)row[u];
             }
@@ -804,11 +804,12 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
     const int per_up = ((a.rpc >> 5) + a.NG - 1) / a.NG * 32, u0 = min(g * per_up, nr), u1 = min(u0 + per_up, nr); // rows this CTA updates
     if (blockIdx.x == 0 && threadIdx.x < NQ) a.gmax_next[threadIdx.x] = (int)threadIdx.x < a.ng ? 0u : a.gmax[threadIdx.x]; // (weights keep theirs)
     if (threadIdx.x == 0) {
-        S_MISC[M_LEFT] = 0; S_MISC[M_CNT] = 0; S_MISC[M_INF] = 0; S_MISC[M_MAX] = 0; S_MISC[M_MAX + 1] = 0;
+        S_MISC[M_LEFT] = 0; S_MISC[M_CNT] = 0; S_MISC[M_MAX] = 0; S_MISC[M_MAX + 1] = 0;
         const Pairs root = S_PAIRS(0);
         root.dec()[0] = 1u; root.build()[0] = 0; root.st()[0] = 0;
     }
-    for (int f = threadIdx.x; f < a.F; f += T) {
+    // (each warp has one trip to memory of these beside its rows: the last warps the features, warp 1 the scales)
+    for (int f = T - 1 - (int)threadIdx.x; f < a.F; f += T) {
         const uint32_t feat = column(a, f);
         const int mono = a.mono[feat];
         S_FEAT[f] = feat | (a.feattypes[feat] != 0 ? 1u << 16 : 0u) | (mono >= -1 && mono <= 1 ? (uint32_t)(mono + 1) : 3u) << 17;
@@ -823,6 +824,14 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
             }
         }
     }
+    if (threadIdx.x >= 32 && threadIdx.x < 32 + NQ) {
+        const int c = threadIdx.x - 32;
+        double unit;
+        const Quant k = quant_of(a.gmax[c], PACK, a.hb, a.round_bits, &unit);
+        S_QUANT[c] = k;
+        S_UNIT[c] = unit;
+        S_INF[c] = k.kind == QK_INF;
+    }
     // rows on their way to shared memory before anything waits: gradients as they are, scaled in place when the scale is known
     const float *rec = a.grad + (size_t)row0 * NQ;
 #pragma unroll 4
@@ -831,13 +840,6 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         for (int c = 0; c < NQ; ++c) S_Q[c * a.rpc + i] = __float_as_int(__ldcg(rec + (size_t)i * NQ + c));
     }
     load_bins(a, S_X, f0, row0, nr);
-    if (threadIdx.x < NQ) {
-        double unit;
-        const Quant k = quant_of(a.gmax[threadIdx.x], PACK, a.hb, a.round_bits, &unit);
-        S_QUANT[threadIdx.x] = k;
-        S_UNIT[threadIdx.x] = unit;
-        if (k.kind == QK_INF) S_MISC[M_INF] = 1;
-    }
     {
         uint4 *z = reinterpret_cast<uint4 *>(S_IMG);
         for (int i = threadIdx.x; i < (int)(a.fit * img_bytes / 16); i += T) z[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -880,7 +882,14 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         const int cur = (level - 1) & 1, set = level & 1;
         const Pairs pr = S_PAIRS(cur), nx = S_PAIRS(cur ^ 1);
         const uint16_t *idx = S_IDX(cur);
-        auto write_out = [&] { if (level > 1) record(a, nx, level - 1); }; // (nx: still the level before)
+        auto write_out = [&] {
+            if (level == 1) return;
+            record(a, nx, level - 1); // (nx: still the level before)
+            if (g != 0) return;
+            int rows = 0; // of this CTA's range that were added up, for the host's statistics
+            for (int k = threadIdx.x; k < np; k += T) if (pr.dec()[k]) rows += pr.build()[k] ? pr.en()[k] - pr.mid()[k] : pr.mid()[k] - pr.st()[k];
+            if (rows > 0) atomicAdd(reinterpret_cast<unsigned long long *>(&a.plan[level].R), (unsigned long long)rows);
+        };
         if constexpr (CL) {
             if (a.lw == 0 && a.lc == 3) hist_level<NQ, CNT, PACK, 0, 3, true>(a, pr, idx, np, set, g, level);
             else if (a.lw == 0) hist_level<NQ, CNT, PACK, 0, 4, true>(a, pr, idx, np, set, g, level);
@@ -896,7 +905,7 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
                 if (level > 1) clear_sums(a, NQ, set ^ 1, done_np, level - 1);
             }
         }
-        if (level == 1 && S_MISC[M_INF]) { // infinities of both signs: no sum means anything
+        if (level == 1 && (S_INF[0] | S_INF[NQ > 1 ? 1 : 0] | S_INF[NQ - 1])) { // infinities of both signs: no sum means anything
             if (threadIdx.x < NQ && *(volatile unsigned *)(a.signs + threadIdx.x) == 3u && a.gmax[threadIdx.x] >= 0x7f800000u) S_UNIT[threadIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
             __syncthreads();
         }
@@ -920,15 +929,6 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         }
         done_np = np;
         np = 1 << (level - 1);
-        __syncthreads();
-        int rows = 0;
-        for (int s = threadIdx.x; s < np; s += T) {
-            if (!nx.dec()[s]) continue;
-            const int mid = S_CL[s];
-            nx.mid()[s] = mid;
-            rows += nx.build()[s] ? nx.en()[s] - mid : mid - nx.st()[s];
-        }
-        if (g == 0 && rows > 0) atomicAdd(reinterpret_cast<unsigned long long *>(&a.plan[level + 1].R), (unsigned long long)rows);
         __syncthreads();
     }
     if (a.whole) {
