@@ -18,7 +18,7 @@
 // poisson, depth 6 0.128 and 0.099.  At 100k x 10 a level takes 8 us: histograms 1.4, barriers 1.4 and 1.3, scan 1.5, decisions 1.3, rows 1.3.
 #include "evb_histg.cuh"
 #include "evb_device.cuh"
-#include <stdlib.h>
+#include <string.h>
 #include <algorithm>
 
 namespace {
@@ -56,7 +56,8 @@ struct GrowArgs {
     int *err;
     long long n;
     int cond, F, B, D, hist_nodes, loss, elide, hb, ng, round_bits, nn;
-    int NG, NR, rpc, lw, lc, fit, M; // lc: log2 of the columns of an image
+    int NG, NR, rpc, lw, M;
+    uint8_t lc[MAX_D];          // [level] log2 of the columns of an image
     int o_x, o_q, o_idx, o_node;
     int o_sum, o_cnt, o_best, o_hist, fo; // one cluster only: sums of the features a CTA scans, fo at most; o_hist == 0: their histograms are in `hist`
     unsigned max_polls;
@@ -178,7 +179,8 @@ __device__ __forceinline__ void warp_first_max(double &v, int &id) {
 
 // ---------------------------------------------------------------------------------------------- histograms of a level
 // Rows of the build nodes of slots [s0, s1), a tile of 32 rows of one node per warp; lanes and banks as in evb_histg.cuh
-// (LC == 5: 32 columns, 8 / W replicas of W words; fewer columns, fewer replicas: lanes meet in a bank, the image is emptied faster)
+// LC == 5: 32 columns, 8 / W replicas of W words, a bank for every lane.  With fewer columns 32 / columns lanes share one (their bins decide
+// whether they meet), but an image is emptied faster and more of them fit: what small nodes want (level_columns).
 template <int NQ, bool CNT, bool PACK, int PB, int C = 0>
 __device__ __forceinline__ void add_cell(uint32_t addr, const uint32_t (&hi)[NQ], const uint32_t (&lo)[NQ]) {
     if constexpr (C < NQ) {
@@ -247,6 +249,7 @@ __device__ __forceinline__ void flush(const GrowArgs &a, const Pairs &pr, int se
     const int nbb = (a.B + BO - 1) / BO, slot_words = (a.B + 1) * P * COLS;
     const bool own = a.NR == 1; // no other CTA adds to these cells
     int base = 0;
+    for (int i = threadIdx.x; i < (s1 - s0) * (P * COLS); i += T) S_IMG[(i / (P * COLS)) * slot_words + i % (P * COLS)] = 0u; // the guard rows: other levels cut images elsewhere
     for (int slot = s0; slot < s1; ++slot) {
         if (!pr.dec()[slot] || (!own && pr.st()[slot] == pr.en()[slot])) continue;
 #pragma unroll
@@ -317,10 +320,78 @@ __device__ __forceinline__ void flush(const GrowArgs &a, const Pairs &pr, int se
     }
 }
 
+// Nodes of so few rows in this range that most cells of an image would stay empty or hold one row: every row straight to the sums, one
+// reduction per feature and channel (and one for the count), no image, no barrier.
+template <int NQ, bool CNT, bool PACK, bool CL>
+__device__ __forceinline__ void add_direct(const GrowArgs &a, const Pairs &pr, const uint16_t *idx, int np, int set, int g, int level, bool second) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, f0 = g * (4 << a.lw), nf = min(4 << a.lw, a.F - f0);
+    const float two_lb = __int_as_float((128 + a.hb) << 23);
+    int base = 0;
+    for (int s = 0; s < np; ++s) {
+        const int b = pr.build()[s], r0 = b ? pr.mid()[s] : pr.st()[s], cnt = (b ? pr.en()[s] : pr.mid()[s]) - r0, nt = (cnt + 31) >> 5;
+        bool left_any = false;
+        for (int t = (wid - base) & (NW - 1); t < nt; t += NW) {
+            const bool act = t * 32 + lane < cnt;
+            const int r = idx[r0 + (act ? t * 32 + lane : 0)];
+            unsigned long long v[NQ];
+            uint32_t some = 0u;
+#pragma unroll
+            for (int c = 0; c < NQ; ++c) {
+                if constexpr (PACK) v[c] = (unsigned long long)(long long)S_Q[r];
+                else {
+                    uint32_t hi, lo;
+                    const float left = take_apart(__int_as_float(S_Q[c * a.rpc + r]), two_lb, hi, lo);
+                    some |= __float_as_uint(left);
+                    if (second) take_apart(left * two_lb, two_lb, hi, lo);
+                    v[c] = (unsigned long long)(((long long)(int32_t)hi << (a.hb + 1)) + (long long)(int32_t)lo);
+                }
+            }
+            if (!act) some = 0u;
+            left_any = left_any || some != 0u;
+            if (!act || (second && some == 0u)) continue;
+            for (int f = 0; f < nf; ++f) {
+                const uint32_t bin = (S_X[(f >> 2) * a.rpc + r] >> (8 * (f & 3)) & 0xffu) - 1u;
+                if (CL && !second) {
+                    const int lf = f / a.NR, rank = (f - lf * a.NR) * a.NG + g, cell = s * a.fo + lf;
+                    const uint32_t at = remote(S_SUM + cell * NQ * a.B, rank) + 8u * bin;
+#pragma unroll
+                    for (int c = 0; c < NQ; ++c) if (v[c] != 0ull) remote_add(at + 8u * (uint32_t)(c * a.B), v[c]);
+                    if (CNT || PACK) remote_add(remote(S_CNTS + cell * a.B, rank) + 4u * bin, 1u);
+                } else {
+                    const size_t cell = (size_t)s * a.F + f0 + f;
+                    unsigned long long *d = (second ? a.low : a.sum) + (size_t)set * a.sum_set + cell * NQ * a.B + bin;
+#pragma unroll
+                    for (int c = 0; c < NQ; ++c) if (v[c] != 0ull) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(d + c * a.B), "l"(v[c]) : "memory");
+                    if ((CNT || PACK) && !second) asm volatile("red.global.add.u32 [%0], 1;" ::"l"(a.cnt + (size_t)set * a.cnt_set + cell * a.B + bin) : "memory");
+                }
+            }
+        }
+        base += nt;
+        if constexpr (!PACK) {
+            if (!second && __any_sync(FULL, left_any)) { // all slots are looked through again (rows that leave nothing are skipped)
+                if (lane == 0) S_MISC[M_LEFT] = 1;
+                if constexpr (CL) { if (lane < (int)gridDim.x) remote_put(remote(S_LOW + s, lane), 1u); }
+                else if (lane == 0) a.lowflag[evb_low_slot(level) + s] = 1u;
+            }
+        }
+    }
+}
+template <int NQ, bool CNT, bool PACK, bool CL>
+__device__ __forceinline__ void direct_level(const GrowArgs &a, const Pairs &pr, const uint16_t *idx, int np, int set, int g, int level) {
+    add_direct<NQ, CNT, PACK, CL>(a, pr, idx, np, set, g, level, false);
+    if constexpr (!PACK) {
+        __syncthreads();
+        if (S_MISC[M_LEFT] == 0) return;
+        add_direct<NQ, CNT, PACK, CL>(a, pr, idx, np, set, g, level, true);
+        __syncthreads();
+        if (threadIdx.x == 0) S_MISC[M_LEFT] = 0;
+    }
+}
 template <int NQ, bool CNT, bool PACK, int LW, int LC, bool CL>
 __device__ __forceinline__ void hist_level(const GrowArgs &a, const Pairs &pr, const uint16_t *idx, int np, int set, int g, int level) {
-    for (int s0 = 0; s0 < np; s0 += a.fit) {
-        const int s1 = min(np, s0 + a.fit);
+    const int fit = a.o_x / ((a.B + 1) * planes(NQ, CNT, PACK) * (4 << LC)); // images come first in shared memory
+    for (int s0 = 0; s0 < np; s0 += fit) {
+        const int s1 = min(np, s0 + fit);
         for (bool second = false;; second = true) {
             add_rows<NQ, CNT, PACK, LW, LC>(a, pr, idx, s0, s1, second);
             __syncthreads();
@@ -498,22 +569,32 @@ template <bool CL>
 __device__ __forceinline__ bool decide(const GrowArgs &a, const Pairs &pr, const Pairs &nx, int level, int set) {
     const int lane = threadIdx.x & 31, F = a.F, nodes = 1 << (level - 1);
     bool any = false;
+    auto records = [&](int j) { return CL ? S_BEST + (size_t)j * F * 3 : a.best + ((size_t)set * a.M + j) * F * 3; };
+    auto ld = [](const double2 *p) { if constexpr (CL) return *p; else return __ldcg(p); };
+    double2 q0, q1, q2; // the first 32 features' records of the warp's next node are on their way while it decides one
+    auto ahead = [&](int j) {
+        q0 = make_double2(0.0, -1.0);
+        if (j < nodes && lane < F && pr.dec()[j >> 1]) { const double2 *r = records(j) + 3 * lane; q0 = ld(r); q1 = ld(r + 1); q2 = ld(r + 2); }
+    };
+    ahead(threadIdx.x >> 5);
     for (int j = threadIdx.x >> 5; j < nodes; j += NW) {
         const int n = nodes + j, s = j >> 1;
         if (!pr.dec()[s]) {
             if (lane == 0) { nx.dec()[j] = 0u; nx.st()[j] = nx.mid()[j] = nx.en()[j] = pr.en()[s]; }
+            ahead(j + NW);
             continue;
         }
-        const double2 *rec = CL ? S_BEST + (size_t)j * F * 3 : a.best + ((size_t)set * a.M + j) * F * 3;
-        auto ld = [](const double2 *p) { if constexpr (CL) return *p; else return __ldcg(p); };
+        const double2 *rec = records(j);
         double2 l1 = make_double2(0.0, 0.0), l2 = l1; // left sums of the lane's best feature
         double s0, s1, s2;
         if (level == 1) { s0 = CL ? S_ROOT[0] : __ldcg(a.nsum + 3); s1 = CL ? S_ROOT[1] : __ldcg(a.nsum + 4); s2 = CL ? S_ROOT[2] : __ldcg(a.nsum + 5); }
         else { s0 = pr.sum()[3 * j]; s1 = pr.sum()[3 * j + 1]; s2 = pr.sum()[3 * j + 2]; }
         double bg = a.gamma;
         int bs = 0x7fffffff, bb = -1;
+        if (q0.y >= 0.0 && q0.x > bg) { bg = q0.x; bs = lane; bb = (int)q0.y; l1 = q1; l2 = q2; }
+        ahead(j + NW);
 #pragma unroll 2
-        for (int f = lane; f < F; f += 32) {
+        for (int f = lane + 32; f < F; f += 32) {
             const double2 r = ld(rec + 3 * f), r1 = ld(rec + 3 * f + 1), r2 = ld(rec + 3 * f + 2);
             if (r.y >= 0.0 && r.x > bg) { bg = r.x; bs = f; bb = (int)r.y; l1 = r1; l2 = r2; }
         }
@@ -747,7 +828,7 @@ __device__ __forceinline__ void load_bins(const GrowArgs &a, uint32_t *x, int f0
         const uint8_t *col[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) { const int f = f0 + 4 * w + k; col[k] = f < a.F ? a.xC + (size_t)column(a, f) * a.n + row0 : nullptr; }
-#pragma unroll 2
+#pragma unroll 4
         for (int e = threadIdx.x; e < quads; e += T) {
             uint32_t v[4];
 #pragma unroll
@@ -797,7 +878,6 @@ __device__ __forceinline__ void clear_own(const GrowArgs &a, int set, int np, in
 // CL: the grid is one cluster; sums, histograms and best splits are exchanged through the CTAs' shared memory and the barriers are the cluster's
 template <int NQ, bool CNT, bool PACK, int CH, bool CL>
 __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
-    const size_t img_bytes = (size_t)(a.B + 1) * planes(NQ, CNT, PACK) * 4 << a.lc;
     const int g = blockIdx.x % a.NG, f0 = g * (4 << a.lw);
     const long long row0 = (long long)(blockIdx.x / a.NG) * a.rpc;
     const int nr = (int)min((long long)a.rpc, a.n - row0), lane = threadIdx.x & 31;
@@ -835,14 +915,24 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
     // rows on their way to shared memory before anything waits: gradients as they are, scaled in place when the scale is known
     const float *rec = a.grad + (size_t)row0 * NQ;
 #pragma unroll 4
-    for (int i = threadIdx.x; i < nr; i += T) {
+    for (int i = threadIdx.x; i < nr >> 2; i += T) { // four records at a time
+        float v[4 * NQ];
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) {
+            const float4 t = __ldcg(reinterpret_cast<const float4 *>(rec) + (size_t)i * NQ + c);
+            v[4 * c] = t.x; v[4 * c + 1] = t.y; v[4 * c + 2] = t.z; v[4 * c + 3] = t.w;
+        }
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) *reinterpret_cast<float4 *>(S_Q + c * a.rpc + 4 * i) = make_float4(v[c], v[NQ + c], v[2 * NQ + c], v[3 * NQ + c]);
+    }
+    for (int i = (nr & ~3) + threadIdx.x; i < nr; i += T) {
 #pragma unroll
         for (int c = 0; c < NQ; ++c) S_Q[c * a.rpc + i] = __float_as_int(__ldcg(rec + (size_t)i * NQ + c));
     }
     load_bins(a, S_X, f0, row0, nr);
     {
         uint4 *z = reinterpret_cast<uint4 *>(S_IMG);
-        for (int i = threadIdx.x; i < (int)(a.fit * img_bytes / 16); i += T) z[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = threadIdx.x; i < a.o_x / 16; i += T) z[i] = make_uint4(0u, 0u, 0u, 0u);
         if constexpr (CL) {
             const int slots = a.M / 2;
             for (int i = threadIdx.x; i < slots * a.fo * NQ * a.B; i += T) S_SUM[i] = 0ull;
@@ -854,6 +944,7 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         Quant k[NQ];
 #pragma unroll
         for (int c = 0; c < NQ; ++c) k[c] = S_QUANT[c];
+#pragma unroll 2
         for (int i = threadIdx.x; i < nr; i += T) {
 #pragma unroll
             for (int c = 0; c < NQ; ++c) S_Q[c * a.rpc + i] = quant(k[c], __int_as_float(S_Q[c * a.rpc + i]), a.signs + c, a.qinv + c);
@@ -890,16 +981,27 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
             for (int k = threadIdx.x; k < np; k += T) if (pr.dec()[k]) rows += pr.build()[k] ? pr.en()[k] - pr.mid()[k] : pr.mid()[k] - pr.st()[k];
             if (rows > 0) atomicAdd(reinterpret_cast<unsigned long long *>(&a.plan[level].R), (unsigned long long)rows);
         };
+        auto hist = [&] {
+            const int lc = a.lc[level];
+            if (lc == 0) direct_level<NQ, CNT, PACK, CL>(a, pr, idx, np, set, g, level);
+            else if (CL || a.lw == 0) {
+                if (lc == 5) hist_level<NQ, CNT, PACK, 0, 5, CL>(a, pr, idx, np, set, g, level);
+                else if (lc == 4) hist_level<NQ, CNT, PACK, 0, 4, CL>(a, pr, idx, np, set, g, level);
+                else hist_level<NQ, CNT, PACK, 0, 3, CL>(a, pr, idx, np, set, g, level);
+            } else if (a.lw == 1) {
+                if (lc == 5) hist_level<NQ, CNT, PACK, 1, 5, CL>(a, pr, idx, np, set, g, level);
+                else if (lc == 4) hist_level<NQ, CNT, PACK, 1, 4, CL>(a, pr, idx, np, set, g, level);
+                else hist_level<NQ, CNT, PACK, 1, 3, CL>(a, pr, idx, np, set, g, level);
+            } else {
+                if (lc == 5) hist_level<NQ, CNT, PACK, 2, 5, CL>(a, pr, idx, np, set, g, level);
+                else hist_level<NQ, CNT, PACK, 2, 4, CL>(a, pr, idx, np, set, g, level);
+            }
+        };
         if constexpr (CL) {
-            if (a.lw == 0 && a.lc == 3) hist_level<NQ, CNT, PACK, 0, 3, true>(a, pr, idx, np, set, g, level);
-            else if (a.lw == 0) hist_level<NQ, CNT, PACK, 0, 4, true>(a, pr, idx, np, set, g, level);
-            else if (a.lw == 1) hist_level<NQ, CNT, PACK, 1, 4, true>(a, pr, idx, np, set, g, level);
-            else hist_level<NQ, CNT, PACK, 2, 5, true>(a, pr, idx, np, set, g, level);
+            hist();
             cluster_barrier();
         } else {
-            if (a.lw == 0) hist_level<NQ, CNT, PACK, 0, 5, false>(a, pr, idx, np, set, g, level);
-            else if (a.lw == 1) hist_level<NQ, CNT, PACK, 1, 5, false>(a, pr, idx, np, set, g, level);
-            else hist_level<NQ, CNT, PACK, 2, 5, false>(a, pr, idx, np, set, g, level);
+            hist();
             if (a.NR > 1) {
                 if (!grid_barrier(a, S_MISC + M_OK, ++arrivals, [] {})) return;
                 if (level > 1) clear_sums(a, NQ, set ^ 1, done_np, level - 1);
@@ -988,48 +1090,108 @@ cudaError_t launch(const evb_handle *h, const GrowGeom &g, const GrowArgs *a, in
     return h->nq == 2 ? launch<2, false, false>(h, g, a, clusters) : launch<3, false, false>(h, g, a, clusters);
 }
 
-int grow_bits(const evb_handle *h, long long rows_of_cell) { // of the high words
+// Columns of the images of every level, from what a level's rows and images cost in clocks: a reduction of a warp a clock, as often as
+// the most lanes meet in a bank; an image read and cleared; 1300 for every pass over as many slots as fit `room`.  Returns the bytes used.
+size_t level_columns(const evb_handle *h, GrowGeom &g, size_t room, double *clocks) {
+    static const double meet[6] = {0, 0, 0, 3.8, 2.0, 1.0}; // (of 4 and 2 lanes: features of few bins meet nearly always)
+    static const int choice[3][3] = {{5, 4, 3}, {5, 4, 3}, {5, 4, 0}};
+    const int P = planes(h->nq, h->hgeo.cnt, h->hgeo.pack);
+    size_t used = 0;
+    *clocks = 0.0;
+    for (int level = 1; level < h->D; ++level) {
+        const int slots = evb_level_slots(level);
+        const double tiles = (double)g.rpc / (level == 1 ? 32.0 : 64.0) + 0.5 * slots;
+        double least = 0.0;
+        size_t bytes = 0;
+        if (g.NR > 1 && level > 2 && g.rpc / 2 < slots * h->B / 2) { // few rows a cell: without images
+            g.lc[level] = 0;
+            *clocks += tiles * (4 << g.lw) * (h->nq + 1) * 4.0;
+            continue;
+        }
+        for (int lc : choice[g.lw]) {
+            const size_t img = (size_t)(h->B + 1) * P * 4 << lc;
+            const long long share = 4ll << g.lw; // columns of one replica: rows of a cell = rows x share / columns
+            if (!lc || img > room || (long long)g.rpc * share >> lc > (h->hgeo.pack ? 8100 : 8050)) continue; // (more than a cell can hold)
+            const int fit = (int)std::min<size_t>(room / img, slots), passes = (slots + fit - 1) / fit;
+            const double c = tiles * (4 << g.lw) * P * meet[lc] / 0.87 + slots * (double)img / 64.0 + passes * 1300.0;
+            if (bytes && c >= least) continue;
+            least = c; bytes = fit * img; g.lc[level] = (uint8_t)lc;
+        }
+        if (!bytes) return 0;
+        used = std::max(used, bytes);
+        *clocks += least;
+    }
+    return (used + 127) & ~(size_t)127;
+}
+// bits of the high words
+int grow_bits(const evb_handle *h, const GrowGeom &g) {
+    long long rows = 0;
+    for (int level = 1; level < h->D; ++level) if (g.lc[level]) rows = std::max(rows, ((long long)g.rpc * (4ll << g.lw) >> g.lc[level]) + 32);
     int hb = 21, log_n = 0;
-    while (hb > 18 && (1ll << (31 - hb)) - 64 < rows_of_cell) --hb;
+    while (hb > 18 && (1ll << (31 - hb)) - 64 < rows) --hb;
     while ((1ll << log_n) < h->n) ++log_n;
     return std::min(hb, (61 - log_n) / 2);
 }
 
-// One cluster of CTAs
-bool cluster_geom(const evb_handle *h, GrowGeom &best) {
-    const int B = h->B, D = h->D, NQ = h->nq, P = planes(NQ, h->hgeo.cnt, h->hgeo.pack), M = 1 << std::max(1, D - 2), hs = h->Ce != h->C ? 2 : 3;
-    const size_t small = (size_t)NODE_BYTES * M + MISC_BYTES + (size_t)h->nn * 8 + (size_t)h->F * 4, room = 226 * 1024;
-    double least = 10000.0; // clocks that the rows of the root may take
-    bool found = false;
-    for (int lw = 0; lw <= 2; ++lw) {
-        const int W = 1 << lw, NG = (h->F + 4 * W - 1) / (4 * W);
-        if (NG > MAX_CLUSTER) continue;
-        int NR = (int)std::min<long long>(MAX_CLUSTER / NG, (h->n + 127) / 128);
-        const long long rpc = ((h->n + NR - 1) / NR + 31) & ~31ll;
-        if (rpc > 16000) continue;
-        NR = (int)((h->n + rpc - 1) / rpc);
-        const int lc = lw == 0 ? (rpc > 1024 ? 4 : 3) : lw + 3, R = 1 << (lc - 2 - lw);
-        const double add = (double)rpc / 32 * 4 * W * P * (R == 4 ? 2.0 : 2.9) / 0.87;
-        if (add >= least) continue;
-        GrowGeom g = {};
-        g.on = g.cluster = true; g.lw = lw; g.lc = lc; g.NG = NG; g.NR = NR; g.rpc = (int)rpc; g.fo = (std::min(4 * W, h->F) + NR - 1) / NR;
-        const size_t img = (size_t)(B + 1) * P * 4 << lc, slots = (size_t)M / 2, kept = (size_t)std::max(1, M / 2) + std::max(1, M / 4);
-        size_t o = (size_t)rpc * (4 + 4 * W + 4 * NQ) + small + (((rpc >> 5) + NG - 1) / NG * 64);
-        auto take = [&](size_t bytes) { const size_t at = (o + 15) & ~(size_t)15; o = at + bytes; return at; };
-        const size_t sum = take(slots * g.fo * NQ * B * 8), cnt = take((slots * g.fo * B + slots) * 4), bst = take((size_t)M * h->F * 48);
-        size_t before = o, hist = take(kept * g.fo * hs * B * 8);
-        if (o + img > room) { o = before; hist = 0; }
-        if (o + img + 128 > room) continue;
-        g.fit = (int)std::min<size_t>((room - 128 - o) / img, slots);
-        const size_t base = (size_t)g.fit * img; // the images come first
-        g.o_sum = (int)(base + sum); g.o_cnt = (int)(base + cnt); g.o_best = (int)(base + bst); g.o_hist = hist ? (int)(base + hist) : 0;
-        g.smem = base + o;
-        g.hb = grow_bits(h, rpc / R + 32);
-        int clusters = 0;
-        if (launch(h, g, nullptr, &clusters) != cudaSuccess || clusters < 1) { cudaGetLastError(); continue; }
-        best = g; least = add; found = true;
+// Clocks of a tree: histograms, the steps whose length is a chain of trips (12000 a level over the grid, 9000 in a cluster), rounds of
+// scans and decisions beyond the first, the rows of a CTA through a step, and over the grid what meets in L2: sums of all row ranges, a
+// sector per row and feature group for the way to the children.  And of the level kernels.  Both from the sweeps that gave the other
+// figures here (100 shapes of 1k to 600k rows, 4 to 128 features, depths 4 to 9).
+double tree_clocks(const evb_handle *h, const GrowGeom &g, double hist) {
+    const int ch = h->B <= 32 ? 0 : h->B <= 64 ? 1 : h->B <= 128 ? 2 : 3;
+    static const double scan[4] = {2400, 3900, 7000, 13000};
+    const int scanners = g.cluster ? std::min(g.NG * std::min(g.NR, 4 << g.lw), h->F) : g.NG * g.NR;
+    double c = hist + 10000.0;
+    for (int level = 1; level < h->D; ++level) {
+        const double slots = evb_level_slots(level), cells = std::min(slots * h->B, g.rpc / (level > 1 ? 2.0 : 1.0));
+        const int nodes = evb_level_nodes(level), scans = (nodes * h->F + scanners * NW - 1) / (scanners * NW);
+        c += (g.cluster ? 9000.0 : 12000.0) + 0.5 * g.rpc + scans * scan[ch] - 3900.0 + (nodes + NW - 1) / NW * 1200.0 - 1200.0;
+        if (!g.cluster) c += g.NR * cells * h->F * (h->nq + 1) / 300.0 + (double)g.NG * h->n * std::min(32, nodes) / 2500.0;
     }
-    return found;
+    return c;
+}
+// The estimate runs at 0.6 of what is measured, this one at 0.9; the line between them (`worth`) lies where the measured ones cross.
+// Measured, level kernels / this one, at estimates of: 0.34 (1503 x 7, depth 5) 1.92, 0.42 (100k x 10, depth 6) 1.6, 0.59 (60k x 77, depth 6) 1.33,
+// 0.73 (353k x 11, depth 7) 1.15, 0.80 (250k x 33 weighted, depth 7) 1.13, 0.82 (407k x 14 weighted, depth 7) 0.90; from depth 8 on 0.44 (16k x 23) 1.34,
+// 0.54 (290k x 4, depth 9) 1.29, 0.57 (28k x 59) 1.13, 0.70 (200k x 20) 0.84, 0.84 (140k x 21, depth 9) 0.85.
+double level_kernel_clocks(const evb_handle *h) {
+    return (h->D - 1) * (38000.0 + 0.0015 * (double)h->n * h->nfeats) * (h->B <= 64 ? 1.0 : h->B <= 128 ? 1.3 : 1.7);
+}
+double worth(const evb_handle *h) { return (h->D <= 7 ? 0.81 : 0.62) * level_kernel_clocks(h); }
+
+// One cluster of CTAs
+bool cluster_geom(const evb_handle *h, GrowGeom &best, double least) {
+    const int B = h->B, D = h->D, NQ = h->nq, M = 1 << std::max(1, D - 2), hs = h->Ce != h->C ? 2 : 3, NG = (h->F + 3) / 4;
+    const size_t small = (size_t)NODE_BYTES * M + MISC_BYTES + (size_t)h->nn * 8 + (size_t)h->F * 4, room = 226 * 1024;
+    if (NG > MAX_CLUSTER) return false;
+    int NR = (int)std::min<long long>(MAX_CLUSTER / NG, (h->n + 127) / 128);
+    const long long rpc = ((h->n + NR - 1) / NR + 31) & ~31ll;
+    // More rows a CTA: the whole grid is faster (us per tree: 22k x 7, 2.8k rows a CTA 44 and 44; 26k x 5, 3.3k 40 and 38; 13k x 13, 3.3k, 128 bins 90 and 72; 100k x 10 81 and 60)
+    if (rpc > 2816) return false;
+    NR = (int)((h->n + rpc - 1) / rpc);
+    GrowGeom g = {};
+    g.on = g.cluster = true; g.NG = NG; g.NR = NR; g.rpc = (int)rpc; g.fo = (std::min(4, h->F) + NR - 1) / NR;
+    const size_t slots = (size_t)M / 2, kept = (size_t)std::max(1, M / 2) + std::max(1, M / 4);
+    size_t o = (size_t)rpc * (8 + 4 * NQ) + small + (((rpc >> 5) + NG - 1) / NG * 64);
+    auto take = [&](size_t bytes) { const size_t at = (o + 15) & ~(size_t)15; o = at + bytes; return at; };
+    const size_t sum = take(slots * g.fo * NQ * B * 8), cnt = take((slots * g.fo * B + slots) * 4), bst = take((size_t)M * h->F * 48);
+    const size_t without = o;
+    size_t hist = take(kept * g.fo * hs * B * 8), base = 0;
+    double clocks = 0.0;
+    if (o + 128 < room) base = level_columns(h, g, room - 128 - o, &clocks);
+    if (!base) { // histograms of parents from L2
+        o = without; hist = 0;
+        if (o + 128 < room) base = level_columns(h, g, room - 128 - o, &clocks);
+    }
+    if (!base || tree_clocks(h, g, clocks) > least) return false;
+    g.o_x = (int)base; // the images come first
+    g.o_sum = (int)(base + sum); g.o_cnt = (int)(base + cnt); g.o_best = (int)(base + bst); g.o_hist = hist ? (int)(base + hist) : 0;
+    g.smem = base + o;
+    g.hb = grow_bits(h, g);
+    int clusters = 0;
+    if (launch(h, g, nullptr, &clusters) != cudaSuccess || clusters < 1) { cudaGetLastError(); return false; }
+    best = g;
+    return true;
 }
 
 } // namespace
@@ -1040,43 +1202,33 @@ void evb_grow_configure(evb_handle *h) {
     g = GrowGeom{};
     const int loss = h->p.loss, D = h->D, B = h->B;
     const bool gh = loss == EVB_MSE || loss == EVB_LOGLOSS || loss == EVB_POISSON || loss == EVB_GAMMA || loss == EVB_TWEEDIE;
-    // Every CTA empties an image per slot and feature group into sums that all row ranges share, whatever few rows the slot has there: that is
-    // what deep trees cost, while the level kernels move the rows of a node together first.  Trees as fast as theirs from about 2^(D-2)
-    // images of 300 KB a level on.  ms per tree, level kernels and this one: 22k x 13 poisson, depth 4 0.073 and 0.044; 1.8k x 54 poisson,
-    // 32 bins, depth 5 0.096 and 0.051; 60k x 77 poisson, depth 6 0.128 and 0.099; 250k x 33 weighted, depth 7 0.183 and 0.169; 16k x 23
-    // logloss, depth 8 0.173 and 0.170; but 99k x 6 poisson, 255 bins, depth 8 0.236 and 0.308.
     if (!gh || h->K != 1 || h->use_q2 || h->p.tree_type == 1 || D < 2 || D > MAX_D || (h->p.flags & EVB_FLAG_FULL_PARTITION) || h->nfeats > 65535) return;
     const int NQ = h->nq, P = planes(NQ, h->hgeo.cnt, h->hgeo.pack), M = 1 << std::max(1, D - 2);
-    const size_t img = (size_t)(B + 1) * P * 128, small = (size_t)NODE_BYTES * M + MISC_BYTES + (size_t)h->nn * 8 + (size_t)h->F * 4, room = 226 * 1024;
-    if (cluster_geom(h, g)) {
-        if (!h->hgeo.pack) { h->hgeo.hb = g.hb; h->hgeo.TE = (1 << (26 - g.hb)) - 1; }
-        return;
-    }
-    if (((size_t)img << (D - 2)) > (size_t)(D - 1) * 300 * 1024) return;
-    double best = 0.0;
+    const size_t small = (size_t)NODE_BYTES * M + MISC_BYTES + (size_t)h->nn * 8 + (size_t)h->F * 4, room = 226 * 1024;
+    double least = worth(h);
     for (int lw = 0; lw <= 2; ++lw) {
         const int W = 1 << lw, NG = (h->F + 4 * W - 1) / (4 * W);
-        if (NG > h->num_sms || img + small > room) continue;
+        if (NG > h->num_sms) continue;
         const long long pr = 4 + 4 * W + 4 * NQ; // bytes of a row: its two places, bins and words
-        // rows whose sums a cell holds: 4 W of 32 rows of a tile meet in a replica
-        const long long cell = (h->hgeo.pack ? 8160ll : 8100ll) * 8 / W;
-        const long long most = std::min<long long>({(long long)(room - img - small - 64) / (pr + 2) * 1ll, cell, 65504ll}) & ~31ll;
-        if (most < 32) continue;
         int NR = h->num_sms / NG;
         NR = (int)std::min<long long>(NR, std::max<long long>(1, h->n / 512));
-        if (h->n <= 4096 && h->n <= most) NR = 1;
         const long long rpc = ((h->n + NR - 1) / NR + 31) & ~31ll;
-        if (rpc > most) continue;
         NR = (int)((h->n + rpc - 1) / rpc);
-        const double add = (double)rpc * 4 * W * P / 25.0 * D / 2.0, fl = (double)NR * h->F * B * P * (1 << (D - 2)) / 400.0;
-        if (g.on && add + fl >= best) continue;
-        best = add + fl;
-        g.on = true; g.lw = lw; g.lc = 5; g.NG = NG; g.NR = NR; g.rpc = (int)rpc;
-        const size_t rows = (size_t)(rpc * pr) + (size_t)(((rpc >> 5) + NG - 1) / NG * 64); // and the leaves of those it updates
-        g.fit = (int)std::min<size_t>((room - small - rows) / img, (size_t)std::max(1, M / 2));
-        g.smem = (size_t)g.fit * img + small + rows;
-        g.hb = grow_bits(h, rpc * W / 8 + 32);
+        GrowGeom t = {};
+        t.on = true; t.lw = lw; t.NG = NG; t.NR = NR; t.rpc = (int)rpc;
+        const size_t rest = small + (size_t)(rpc * pr) + (size_t)(((rpc >> 5) + NG - 1) / NG * 64); // and the leaves of the rows it updates
+        double clocks = 0.0;
+        if (rpc > 65504 || rest >= room) continue;
+        const size_t base = level_columns(h, t, room - rest, &clocks);
+        if (!base) continue;
+        clocks = tree_clocks(h, t, clocks);
+        if (clocks > least) continue;
+        least = clocks;
+        t.o_x = (int)base; t.smem = base + rest; t.hb = grow_bits(h, t);
+        g = t;
+        break; // few features a CTA: fewer row ranges share a sum
     }
+    cluster_geom(h, g, least);
     if (g.on && !h->hgeo.pack) { h->hgeo.hb = g.hb; h->hgeo.TE = (1 << (26 - g.hb)) - 1; } // how k_tree_begin scales g
 }
 
@@ -1100,10 +1252,11 @@ int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot,
     a.plan = h->plan; a.bar = h->g_bar; a.err = h->d_err; a.n = h->n;
     a.F = h->F; a.B = h->B; a.D = h->D; a.hist_nodes = h->hist_nodes; a.loss = h->p.loss; a.elide = h->Ce != h->C; a.hb = h->hgeo.hb; a.ng = h->ng; a.nn = h->nn;
     a.round_bits = evb_hg_round_bits(h);
-    a.NG = g.NG; a.NR = g.NR; a.rpc = g.rpc; a.lw = g.lw; a.fit = g.fit; a.M = 1 << std::max(1, h->D - 2);
-    const size_t img = (size_t)(h->B + 1) * planes(h->nq, h->hgeo.cnt, h->hgeo.pack) * 4 << g.lc;
-    a.lc = g.lc; a.o_sum = g.o_sum; a.o_cnt = g.o_cnt; a.o_best = g.o_best; a.o_hist = g.o_hist; a.fo = g.fo;
-    a.o_x = (int)(g.fit * img); a.o_q = a.o_x + (g.rpc * 4 << g.lw); a.o_idx = a.o_q + g.rpc * 4 * h->nq; a.o_node = a.o_idx + g.rpc * 4;
+    a.NG = g.NG; a.NR = g.NR; a.rpc = g.rpc; a.lw = g.lw; a.M = 1 << std::max(1, h->D - 2);
+    static_assert(sizeof(a.lc) == sizeof(g.lc), "levels");
+    memcpy(a.lc, g.lc, sizeof(a.lc));
+    a.o_sum = g.o_sum; a.o_cnt = g.o_cnt; a.o_best = g.o_best; a.o_hist = g.o_hist; a.fo = g.fo;
+    a.o_x = g.o_x; a.o_q = a.o_x + (g.rpc * 4 << g.lw); a.o_idx = a.o_q + g.rpc * 4 * h->nq; a.o_node = a.o_idx + g.rpc * 4;
     a.max_polls = 8000000u; // seconds
     a.low_unit = evb_hg_low_unit(h); a.neb = -h->p.eta / (double)h->p.bagging_size;
     a.lambda = h->p.lambda; a.L2 = h->p.L2; a.gamma = h->p.gamma; a.min_weight = h->p.min_weight;

@@ -74,9 +74,10 @@ struct HGeom {
 struct GrowGeom {
     bool on;
     int lw, NG, NR, rpc; // log2 of the words of four features a CTA takes; CTAs side by side: feature groups x row ranges; rows of a range
-    int lc, fit, hb;     // log2 of the columns of an image; images in shared memory; bits of the high words
+    int hb;              // bits of the high words
+    uint8_t lc[10];      // [level] log2 of the columns of an image
     bool cluster;        // the grid is one cluster; offsets of what its CTAs keep in shared memory for it (GrowArgs)
-    int o_sum, o_cnt, o_best, o_hist, fo;
+    int o_x, o_sum, o_cnt, o_best, o_hist, fo;
     size_t smem;
 };
 

@@ -51,7 +51,10 @@ CASES = [  # loss, rows, features, bins, depth, weights
     ("mse", 1, 1, 2, 2, False), ("logloss", 31, 3, 16, 3, False), ("mse", 33, 4, 32, 3, True), ("poisson", 4_096, 5, 33, 4, False),
     ("poisson", 4_097, 7, 64, 5, True), ("gamma", 9_999, 8, 65, 5, False), ("tweedie", 20_011, 33, 128, 6, False), ("mse", 12_345, 13, 129, 5, False),
     ("logloss", 3_001, 6, 255, 4, True), ("mse", 100_003, 10, 32, 6, False), ("mse", 50_021, 100, 64, 5, False), ("logloss", 299_999, 28, 64, 5, False),
-    ("mse", 70_001, 61, 64, 6, True), ("poisson", 2_000, 130, 64, 4, False), ("mse", 290_000, 3, 33, 9, False), ("logloss", 40_000, 4, 16, 9, False), ("mse", 40_000, 4, 16, 10, False)]
+    ("mse", 70_001, 61, 64, 6, True), ("poisson", 2_000, 130, 64, 4, False), ("mse", 290_000, 3, 33, 9, False), ("logloss", 40_000, 4, 16, 9, False), ("mse", 40_000, 4, 16, 10, False),
+    # small nodes: rows straight to the sums, images of fewer columns
+    ("poisson", 5_031, 5, 64, 7, False), ("logloss", 6_443, 79, 128, 7, True), ("mse", 11_639, 30, 255, 8, False), ("gamma", 16_577, 22, 64, 8, True),
+    ("mse", 2_245, 9, 128, 6, False), ("tweedie", 63_211, 11, 255, 6, False), ("mse", 190_000, 33, 64, 7, True), ("poisson", 353_000, 11, 64, 7, False)]
 
 
 @pytest.mark.parametrize("loss,n,F,B,depth,weighted", CASES)
@@ -79,12 +82,12 @@ def test_categories_and_constraints(pkg):
     assert (t.split != 0).sum() > 5
 
 
-@pytest.mark.parametrize("n", [3_000, 60_000])
+@pytest.mark.parametrize("n,depth", [(3_000, 5), (3_000, 7), (60_000, 5), (30_000, 8)])
 @pytest.mark.parametrize("loss", ["gamma", "mse"])
-def test_wide_ranges(pkg, loss, n):
+def test_wide_ranges(pkg, loss, n, depth):
     """Gradients over many orders of magnitude: the second set of sums; infinities of one sign and of both"""
     x, y, w = _data(n, 6, 64, loss, 4, loss == "mse")
-    params = pkg.EvoTreeRegressor(loss=loss, nrounds=1, max_depth=5, nbins=64, eta=0.3)
+    params = pkg.EvoTreeRegressor(loss=loss, nrounds=1, max_depth=depth, nbins=64, eta=0.3)
     rng = np.random.default_rng(n)
     wide = np.exp(5.0 * rng.normal(size=n)).astype(np.float32)
     _same(pkg, params, x, wide, w, rounds=2)
