@@ -14,8 +14,9 @@
 // With one range of rows a CTA scans its own features' sums and the first barrier falls away.
 // Where at most 16 CTAs hold the rows they are one cluster: sums, histograms and best splits lie in their shared memory, added to and handed
 // out by remote accesses, and its barriers are the hardware's (0.4 us with the wait for the slowest CTA, 1.3 through L2).
-// ms per tree before (level kernels) and here: 1503 x 7 logloss, depth 5 0.085 and 0.052; 100k x 10, 32 bins, depth 6 0.098 and 0.061; 60k x 77
-// poisson, depth 6 0.128 and 0.099.  At 100k x 10 a level takes 8 us: histograms 1.4, barriers 1.4 and 1.3, scan 1.5, decisions 1.3, rows 1.3.
+// ms per tree of level kernels and this one: 1503 x 7 logloss, depth 5 0.085 and 0.041; 100k x 10, 32 bins, depth 6 0.095 and 0.060; 60k x 77
+// poisson (54 columns), depth 6 0.124 and 0.095; 6.4k x 80, 128 bins, depth 7 0.169 and 0.119. At 100k x 10 a level takes 8 us: histograms 1.4,
+// barriers 1.7 and 1.3, scan 1.2, decisions 1.1, rows 1.5 to 2.8.
 #include "evb_histg.cuh"
 #include "evb_device.cuh"
 #include <string.h>
@@ -1150,14 +1151,14 @@ double tree_clocks(const evb_handle *h, const GrowGeom &g, double hist) {
     }
     return c;
 }
-// The estimate runs at 0.6 of what is measured, this one at 0.9; the line between them (`worth`) lies where the measured ones cross.
-// Measured, level kernels / this one, at estimates of: 0.34 (1503 x 7, depth 5) 1.92, 0.42 (100k x 10, depth 6) 1.6, 0.59 (60k x 77, depth 6) 1.33,
-// 0.73 (353k x 11, depth 7) 1.15, 0.80 (250k x 33 weighted, depth 7) 1.13, 0.82 (407k x 14 weighted, depth 7) 0.90; from depth 8 on 0.44 (16k x 23) 1.34,
-// 0.54 (290k x 4, depth 9) 1.29, 0.57 (28k x 59) 1.13, 0.70 (200k x 20) 0.84, 0.84 (140k x 21, depth 9) 0.85.
+// The estimate runs at 0.65 of what is measured, this one at 0.95; the line between them (`worth`) lies where the measured ones cross.
+// Measured, level kernels / this kernel, at estimates of: 0.47 (50k x 50, depth 6) 1.49, 0.59 (60k x 54 poisson, depth 6) 1.30, 0.67 (130k x 108,
+// 32 bins, depth 7) 0.99, 0.74 (353k x 11, depth 7) 1.16, 0.80 (250k x 33 weighted, depth 7) 1.01, 0.83 (407k x 14 weighted, depth 7) 0.92; from depth
+// 8 on 0.48 (16.6k x 23) 1.33, 0.54 (290k x 4, depth 9) 1.28, 0.57 (28k x 30) 1.12, 0.64 (41k x 63) 0.94, 0.70 (200k x 20) 0.90, 0.86 (140k x 17, depth 9) 0.83.
 double level_kernel_clocks(const evb_handle *h) {
     return (h->D - 1) * (38000.0 + 0.0015 * (double)h->n * h->nfeats) * (h->B <= 64 ? 1.0 : h->B <= 128 ? 1.3 : 1.7);
 }
-double worth(const evb_handle *h) { return (h->D <= 7 ? 0.81 : 0.62) * level_kernel_clocks(h); }
+double worth(const evb_handle *h) { return (h->D <= 7 ? 0.81 : 0.6) * level_kernel_clocks(h); }
 
 // One cluster of CTAs
 bool cluster_geom(const evb_handle *h, GrowGeom &best, double least) {
