@@ -18,8 +18,13 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// Trees in device memory: tree t at word t * tw, [nnp] packed nodes, then [nnp * K] leaf values (zero padded); nnp = nodes
-// rounded up to a multiple of four, so that every tree starts on a 16-byte boundary.
+// Trees in device memory: tree t at word t * tw.  Every tree of a model is a complete one of `levels` tests: [ni] nodes in heap order, then the
+// values of the 2^levels leaves, [leaf][K].  A node is feature | b << 16 | a << 24: a row whose bin is x goes left where (x ^ a) <= b -- numeric
+// tests have a = 0 and b the bin, categories a the bin and b = 0.  A leaf above the last level is a node that sends every row left (STOP), and so
+// on to the last level, where its value is.  A walk is the same number of steps for all lanes, about half the instructions of one
+// that looks for the end of its path (25 a level), and the trees take half the room.  ni: 2^levels, at least four, so that every part starts on a
+// 16-byte boundary.
+constexpr uint32_t STOP = 0x00ff0000u;
 struct PredArgs {
     const void *x;          // raw features (T = float / double) or bins (T = uint8_t)
     long long ld;           // row-major: elements between rows; column-major: between features
@@ -28,7 +33,7 @@ struct PredArgs {
     const void *edges;      // [nfeats][nedges] ascending, same type as x
     int nedges, nfeats, FW; // FW: words of four bins per row
     const uint32_t *trees;
-    int nnp, tw, levels;    // levels: tests on the longest path of a tree
+    int ni, tw, levels;     // levels: tests on the longest path of a tree
     float *out;             // column k of row i at k * out_ld + i
     long long out_ld;
     uint32_t *leaf_idx;     // null, or tree t of row i at t * out_ld + i
@@ -75,22 +80,114 @@ __device__ __forceinline__ uint32_t bin_word(const PredArgs &a, long long i, int
     }
 }
 
-__device__ __forceinline__ void link_row(int loss, int K, float *p) { // apply_prediction_link! (src/predict.jl:105-116)
-    if (loss == EVB_LOGLOSS) { for (int k = 0; k < K; ++k) p[k] = sigmoidf_(p[k]); }
-    else if (loss == EVB_GAUSSIAN_MLE || loss == EVB_LOGISTIC_MLE) { for (int k = 1; k < K; k += 2) p[k] = softplusf_(p[k]); }
-    else if (loss == EVB_POISSON || loss == EVB_GAMMA || loss == EVB_TWEEDIE) { for (int k = 0; k < K; ++k) p[k] = expf(p[k]); }
-    else if (loss == EVB_MLOGLOSS) {
+template <int KMAX>
+__device__ __forceinline__ void link_row(int loss, int K, float (&p)[KMAX]) { // apply_prediction_link! (src/predict.jl:105-116)
+    constexpr int U = KMAX > 8 ? 1 : KMAX;
+    if (loss == EVB_LOGLOSS) {
+#pragma unroll U
+        for (int k = 0; k < KMAX; ++k) if (k < K) p[k] = sigmoidf_(p[k]);
+    } else if (loss == EVB_GAUSSIAN_MLE || loss == EVB_LOGISTIC_MLE) {
+#pragma unroll U
+        for (int k = 1; k < KMAX; k += 2) if (k < K) p[k] = softplusf_(p[k]);
+    } else if (loss == EVB_POISSON || loss == EVB_GAMMA || loss == EVB_TWEEDIE) {
+#pragma unroll U
+        for (int k = 0; k < KMAX; ++k) if (k < K) p[k] = expf(p[k]);
+    } else if (loss == EVB_MLOGLOSS) {
         float s = 0.0f;
-        for (int k = 0; k < K; ++k) { p[k] = expf(p[k]); s += p[k]; }
-        for (int k = 0; k < K; ++k) p[k] /= s;
+#pragma unroll U
+        for (int k = 0; k < KMAX; ++k) if (k < K) { p[k] = expf(p[k]); s += p[k]; }
+#pragma unroll U
+        for (int k = 0; k < KMAX; ++k) if (k < K) p[k] /= s;
     }
 }
 
-// one test of a node: the child of node `nid` for a row whose word of bins `word` holds the node's feature
-__device__ __forceinline__ int child(uint32_t pk, uint32_t word, int nid) {
-    const uint32_t x = (word >> (8u * (pk & 3u))) & 0xffu, bin = (pk >> 16) & 0xffu;
-    const bool cond = ((pk >> 25) & 1u) ? (x <= bin) : (x == bin);
-    return (nid << 1) + (cond ? 0 : 1); // nid = nid << 1 + !cond (src/predict.jl:7)
+// pred_add (evb_device.cuh) for up to KMAX outputs in registers.  Loops over a K that only the launch knows index p, so it lived in local
+// memory: adding a tree took 900 clocks at seven classes, most of the time of a call of some thousand rows.
+template <int KMAX>
+__device__ __forceinline__ void add_leaf(int loss, int K, float (&p)[KMAX], const float *leaf, int stride) {
+    if constexpr (KMAX > 8) {
+        float v[KMAX];
+        for (int k = 0; k < K; ++k) v[k] = leaf[k * stride];
+        pred_add(loss, K, p, v);
+    } else {
+#pragma unroll
+        for (int k = 0; k < KMAX; ++k) if (k < K) p[k] += leaf[k * stride];
+        if (loss == EVB_LOGLOSS) {
+#pragma unroll
+            for (int k = 0; k < KMAX; ++k) p[k] = fminf(fmaxf(p[k], -15.0f), 15.0f);
+        } else if (loss == EVB_GAUSSIAN_MLE || loss == EVB_LOGISTIC_MLE) {
+#pragma unroll
+            for (int k = 1; k < KMAX; k += 2) p[k] = fmaxf(-15.0f, p[k]);
+        } else if (loss == EVB_MLOGLOSS) {
+            float q[KMAX];
+#pragma unroll
+            for (int k = 0; k < KMAX; ++k) q[k] = k < K ? p[k] : -INFINITY;
+#pragma unroll
+            for (int d = 1; d < KMAX; d <<= 1)
+#pragma unroll
+                for (int k = 0; k + d < KMAX; k += 2 * d) q[k] = fmaxf(q[k], q[k + d]);
+#pragma unroll
+            for (int k = 0; k < KMAX; ++k) p[k] = fmaxf(-15.0f, p[k] - q[0]);
+        }
+    }
+}
+
+// Leaf values of n trees, [tree][K] at `stride`, in order: the next tree's are on their way while one is added, the loss is told apart once
+template <int KMAX, int LOSS>
+__device__ __forceinline__ void add_trees_of(int K, float (&p)[KMAX], const float *leaf, int n, int stride) {
+    float v[KMAX];
+    auto fetch = [&](int t) {
+#pragma unroll
+        for (int k = 0; k < KMAX; ++k) v[k] = k < K ? leaf[(t * K + k) * stride] : 0.0f;
+    };
+    fetch(0);
+    for (int t = 1; t <= n; ++t) {
+        float w[KMAX];
+#pragma unroll
+        for (int k = 0; k < KMAX; ++k) w[k] = v[k];
+        if (t < n) fetch(t);
+        add_leaf<KMAX>(LOSS, K, p, w, 1);
+    }
+}
+template <int KMAX>
+__device__ __forceinline__ void add_trees(int loss, int K, float (&p)[KMAX], const float *leaf, int n, int stride) {
+    if (n <= 0) return;
+    if constexpr (KMAX > 8) { for (int t = 0; t < n; ++t) add_leaf<KMAX>(loss, K, p, leaf + t * K * stride, stride); }
+    else if (loss == EVB_MLOGLOSS) add_trees_of<KMAX, EVB_MLOGLOSS>(K, p, leaf, n, stride);
+    else if (loss == EVB_LOGLOSS) add_trees_of<KMAX, EVB_LOGLOSS>(K, p, leaf, n, stride);
+    else if (loss == EVB_GAUSSIAN_MLE || loss == EVB_LOGISTIC_MLE) add_trees_of<KMAX, EVB_GAUSSIAN_MLE>(K, p, leaf, n, stride);
+    else add_trees_of<KMAX, EVB_MSE>(K, p, leaf, n, stride);
+}
+template <int KMAX>
+__device__ __forceinline__ void put_row(const PredArgs &a, long long i, const float (&p)[KMAX]) {
+    constexpr int U = KMAX > 8 ? 1 : KMAX;
+#pragma unroll U
+    for (int k = 0; k < KMAX; ++k) if (k < a.K) a.out[(size_t)k * a.out_ld + i] = p[k];
+}
+
+// Leaf (0 .. 2^levels - 1) of a row in one tree; word(w): the row's bins 4 w .. 4 w + 3, node(i): the tree's node i
+template <typename N, typename X>
+__device__ __forceinline__ int walk(int levels, N node, X word) {
+    int i = 0;
+    for (int l = 0; l < levels; ++l) {
+        const uint32_t pk = node(i);
+        const uint32_t x = __byte_perm(word((pk & 0xffffu) >> 2), 0u, 0x4440u | (pk & 3u));
+        i = 2 * i + ((x ^ (pk >> 24)) <= ((pk >> 16) & 0xffu) ? 1 : 2);
+    }
+    return i + 1 - (1 << levels);
+}
+// the same for the id of the node where the row's path ends (`predict_leaf_idx`): the first that stops, else the leaf itself
+template <typename N, typename X>
+__device__ __forceinline__ int walk_id(int levels, N node, X word, int &leaf) {
+    int i = 0, id = 0;
+    for (int l = 0; l < levels; ++l) {
+        const uint32_t pk = node(i);
+        if (id == 0 && pk == STOP) id = i + 1;
+        const uint32_t x = __byte_perm(word((pk & 0xffffu) >> 2), 0u, 0x4440u | (pk & 3u));
+        i = 2 * i + ((x ^ (pk >> 24)) <= ((pk >> 16) & 0xffu) ? 1 : 2);
+    }
+    leaf = i + 1 - (1 << levels);
+    return id ? id : i + 1;
 }
 
 // ---------------------------------------------------------------------------------- few rows
@@ -126,25 +223,22 @@ __global__ void __launch_bounds__(ONE_THREADS) k_predict_one(PredArgs a) {
         const int t = t0 + tid;
         if (t < a.ntrees) {
             const uint32_t *tr = a.trees + (size_t)t * a.tw;
-            int nid = 1;
-            uint32_t pk = __ldg(tr);
-            while ((pk >> 24) & 1u) {
-                nid = child(pk, s_one[(pk & 0xffffu) >> 2], nid);
-                pk = __ldg(tr + nid - 1);
-            }
-            if (a.leaf_idx) a.leaf_idx[(size_t)t * a.out_ld + i] = (uint32_t)nid;
-            for (int k = 0; k < K; ++k) s_leaf[tid * K + k] = __uint_as_float(__ldg(tr + a.nnp + (nid - 1) * K + k));
+            auto node = [&](int n) { return __ldg(tr + n); };
+            auto word = [&](uint32_t w) { return s_one[w]; };
+            int leaf;
+            if (a.leaf_idx) a.leaf_idx[(size_t)t * a.out_ld + i] = (uint32_t)walk_id(a.levels, node, word, leaf);
+            else leaf = walk(a.levels, node, word);
+            for (int k = 0; k < K; ++k) s_leaf[tid * K + k] = __uint_as_float(__ldg(tr + a.ni + leaf * K + k));
         }
         __syncthreads();
         if (tid == 0) {
             const int nt = min(ONE_THREADS, a.ntrees - t0);
-#pragma unroll 4
-            for (int q = 0; q < nt; ++q) pred_add(a.loss, K, p, s_leaf + q * K);
+            add_trees<KMAX>(a.loss, K, p, s_leaf, nt, 1);
         }
     }
     if (tid == 0) {
-        if (a.apply_link) link_row(a.loss, K, p);
-        for (int k = 0; k < K; ++k) a.out[(size_t)k * a.out_ld + i] = p[k];
+        if (a.apply_link) link_row<KMAX>(a.loss, K, p);
+        put_row<KMAX>(a, i, p);
     }
 }
 
@@ -153,8 +247,8 @@ __global__ void __launch_bounds__(ONE_THREADS) k_predict_one(PredArgs a) {
 // memory, four trees at a time per lane so that four chains of loads overlap; the eighth warp adds the previous block's
 // values in order meanwhile.  Nodes come through L1: 32 rows do not pay for copying a tree into shared memory.  Bins are
 // word-major ([word of the row][row]): a lane only ever reads its own bank.
-// Measured (call of 20 011 rows x 28, 201 trees of depth 8, five classes): 1.26 ms with 20 CTAs of 1024 rows (378 us of it
-// their kernel), 0.235 ms like this.
+// Measured (call of 20 011 rows x 28, 201 trees of depth 8, five classes): 0.206 ms, with k_predict_tiles 0.175.  Used where two trees and
+// 32 rows do not fit shared memory.
 constexpr int MID_WARPS = 8, MID_ILP = 4;
 template <int KMAX, typename T>
 __global__ void __launch_bounds__(MID_WARPS * 32) k_predict_mid(PredArgs a, int TB) {
@@ -174,51 +268,116 @@ __global__ void __launch_bounds__(MID_WARPS * 32) k_predict_mid(PredArgs a, int 
         if (wid > 0) {
             for (int tb = wid - 1; tb < nt; tb += (MID_WARPS - 1) * MID_ILP) {
                 const uint32_t *tr[MID_ILP];
-                int nid[MID_ILP];
-                uint32_t pk[MID_ILP];
+                int at[MID_ILP], id[MID_ILP];
 #pragma unroll
                 for (int u = 0; u < MID_ILP; ++u) {
                     const int t = tb + u * (MID_WARPS - 1);
                     tr[u] = a.trees + (size_t)(t0 + (t < nt ? t : tb)) * a.tw;
-                    nid[u] = 1;
-                    pk[u] = __ldg(tr[u]);
+                    at[u] = 0; id[u] = 0;
                 }
                 for (int l = 0; l < a.levels; ++l) {
+                    uint32_t pk[MID_ILP];
+#pragma unroll
+                    for (int u = 0; u < MID_ILP; ++u) pk[u] = __ldg(tr[u] + at[u]);
 #pragma unroll
                     for (int u = 0; u < MID_ILP; ++u) {
-                        if ((pk[u] >> 24) & 1u) {
-                            nid[u] = child(pk[u], s_mid[((pk[u] & 0xffffu) >> 2) * 32 + lane], nid[u]);
-                            pk[u] = __ldg(tr[u] + nid[u] - 1);
-                        }
+                        if (id[u] == 0 && pk[u] == STOP) id[u] = at[u] + 1;
+                        const uint32_t x = __byte_perm(s_mid[((pk[u] & 0xffffu) >> 2) * 32 + lane], 0u, 0x4440u | (pk[u] & 3u));
+                        at[u] = 2 * at[u] + ((x ^ (pk[u] >> 24)) <= ((pk[u] >> 16) & 0xffu) ? 1 : 2);
                     }
                 }
 #pragma unroll
                 for (int u = 0; u < MID_ILP; ++u) {
                     const int t = tb + u * (MID_WARPS - 1);
                     if (t < nt) {
-                        const uint32_t *lf = tr[u] + a.nnp + (nid[u] - 1) * K;
+                        const uint32_t *lf = tr[u] + a.ni + (at[u] + 1 - (1 << a.levels)) * K;
                         float *d = s_leaf + ((size_t)(buf * TB + t) * K) * 32 + lane;
                         for (int k = 0; k < K; ++k) d[k * 32] = __uint_as_float(__ldg(lf + k));
-                        if (a.leaf_idx && act) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = (uint32_t)nid[u];
+                        if (a.leaf_idx && act) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = (uint32_t)(id[u] ? id[u] : at[u] + 1);
                     }
                 }
             }
         } else if (t0 > 0) {
             const int np = min(TB, a.ntrees - (t0 - TB));
             const float *s = s_leaf + ((size_t)(buf ^ 1) * TB * K) * 32 + lane;
-            for (int t = 0; t < np; ++t) {
-                float lf[KMAX];
-#pragma unroll
-                for (int k = 0; k < KMAX; ++k) if (k < K) lf[k] = s[(t * K + k) * 32];
-                pred_add(a.loss, K, p, lf);
-            }
+            add_trees<KMAX>(a.loss, K, p, s, np, 32);
         }
         if (nt <= 0) break;
         __syncthreads();
     }
     if (wid == 0 && act) {
-        if (a.apply_link) link_row(a.loss, K, p);
-        for (int k = 0; k < K; ++k) a.out[(size_t)k * a.out_ld + i] = p[k];
+        if (a.apply_link) link_row<KMAX>(a.loss, K, p);
+        put_row<KMAX>(a, i, p);
+    }
+}
+
+// The same division of work with the trees in shared memory: a CTA of 32 warps takes RG groups of 32 rows, WARPS / RG warps each, one
+// of which adds; blocks of TB trees arrive by cp.async while the block before is walked.  A node then is one bank conflict away
+// instead of a line of L1 per lane, and so is a leaf: its K values cost k_predict_mid K loads of up to 32 lines each.  What bounds it is
+// instructions, 13 a level, and with several outputs the chain of additions.  us of a call, before (k_predict_mid, nodes that say where a path
+// ends, sums in local memory) and here: 20k x 28, 200 trees of depth 8, five classes 241 and 175; 900 x 12, 200 of depth 6, seven classes 128
+// and 59; 90k x 12, the same model 616 and 346; 1.5k x 60, 100 of depth 9, two outputs 84 and 63; 6k x 30 doubles, 150 of depth 10 141 and 115.
+constexpr int TILE_WARPS = 32;
+template <int KMAX, typename T>
+__global__ void __launch_bounds__(TILE_WARPS * 32, 1) k_predict_tiles(PredArgs a, int RG, int TB) {
+    extern __shared__ __align__(16) uint32_t s_tl[]; // [2][TB][tw] trees, [2][TB][K][R] leaf values, [FW][R] bins; R = 32 RG rows
+    const int K = KMAX > 8 ? a.K : KMAX, tw = a.tw, R = 32 * RG, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, grp = wid % RG, role = wid / RG, walkers = (TILE_WARPS - grp + RG - 1) / RG - 1;
+    float *s_leaf = reinterpret_cast<float *>(s_tl + (size_t)2 * TB * tw);
+    uint32_t *s_bins = reinterpret_cast<uint32_t *>(s_leaf + (size_t)2 * TB * K * R);
+    auto load_block = [&](int t0, int buf) {
+        const int nt = min(TB, a.ntrees - t0);
+        if (nt > 0) {
+            const uint4 *src = reinterpret_cast<const uint4 *>(a.trees + (size_t)t0 * tw);
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_tl + (size_t)buf * TB * tw);
+            for (int c = threadIdx.x; c < nt * (tw >> 2); c += TILE_WARPS * 32)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)c * 16u), "l"(src + c) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_block(0, 0);
+    const long long row0 = (long long)blockIdx.x * R, i = row0 + grp * 32 + lane;
+    const bool act = i < a.n;
+    for (int e = wid; e < a.FW * RG; e += TILE_WARPS) {
+        const int w = e / RG, g = e - w * RG;
+        const long long r = row0 + g * 32 + lane;
+        s_bins[w * R + g * 32 + lane] = r < a.n ? bin_word<T>(a, r, w) : 0u;
+    }
+    const uint32_t *xcol = s_bins + grp * 32 + lane;
+    float p[KMAX];
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) p[k] = 0.0f;
+    int buf = 0;
+    for (int t0 = 0;; t0 += TB, buf ^= 1) {
+        const int nt = min(TB, a.ntrees - t0); // <= 0: only the last block's sum is left
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads(); // this block's trees and the last one's leaf values are in place, the other buffers free
+        load_block(t0 + TB, buf ^ 1);
+        if (role > 0) {
+            for (int t = role - 1; t < nt; t += walkers) {
+                const uint32_t *tr = s_tl + ((size_t)buf * TB + t) * tw;
+                auto node = [&](int n) { return tr[n]; };
+                auto word = [&](uint32_t w) { return xcol[w * R]; };
+                int leaf;
+                if (a.leaf_idx) {
+                    const uint32_t id = (uint32_t)walk_id(a.levels, node, word, leaf);
+                    if (act) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = id;
+                } else leaf = walk(a.levels, node, word);
+                const float *lf = reinterpret_cast<const float *>(tr + a.ni) + leaf * K;
+                float *d = s_leaf + ((size_t)(buf * TB + t) * K) * R + grp * 32 + lane;
+                constexpr int U = KMAX > 8 ? 1 : KMAX;
+#pragma unroll U
+                for (int k = 0; k < KMAX; ++k) if (k < K) d[k * R] = lf[k];
+            }
+        } else if (t0 > 0) {
+            const int np = min(TB, a.ntrees - (t0 - TB));
+            const float *d = s_leaf + ((size_t)(buf ^ 1) * TB * K) * R + grp * 32 + lane;
+            add_trees<KMAX>(a.loss, K, p, d, np, R);
+        }
+        if (nt <= 0) break;
+    }
+    if (role == 0 && act) {
+        if (a.apply_link) link_row<KMAX>(a.loss, K, p);
+        put_row<KMAX>(a, i, p);
     }
 }
 
@@ -260,21 +419,19 @@ __global__ void __launch_bounds__(1024) k_predict_staged(PredArgs a, int TB) {
         if (act) {
             for (int t = 0; t < nt; ++t) {
                 const uint32_t *tr = s_trees + ((size_t)buf * TB + t) * tw;
-                int nid = 1;
-                uint32_t pk = tr[0];
-                while ((pk >> 24) & 1u) {
-                    nid = child(pk, xcol[((pk & 0xffffu) >> 2) * rows], nid);
-                    pk = tr[nid - 1];
-                }
-                if (a.leaf_idx) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = (uint32_t)nid;
-                pred_add(a.loss, K, p, reinterpret_cast<const float *>(tr + a.nnp) + (size_t)(nid - 1) * K);
+                auto node = [&](int n) { return tr[n]; };
+                auto word = [&](uint32_t w) { return xcol[w * rows]; };
+                int leaf;
+                if (a.leaf_idx) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = (uint32_t)walk_id(a.levels, node, word, leaf);
+                else leaf = walk(a.levels, node, word);
+                add_leaf<KMAX>(a.loss, K, p, reinterpret_cast<const float *>(tr + a.ni) + leaf * K, 1);
             }
         }
         __syncthreads(); // everybody is done with this buffer: the next iteration refills it
     }
     if (!act) return;
-    if (a.apply_link) link_row(a.loss, K, p);
-    for (int k = 0; k < K; ++k) a.out[(size_t)k * a.out_ld + i] = p[k];
+    if (a.apply_link) link_row<KMAX>(a.loss, K, p);
+    put_row<KMAX>(a, i, p);
 }
 
 // rows of more bins than shared memory holds: bins in global memory ([row][FW] words), one thread per row
@@ -295,24 +452,22 @@ __global__ void __launch_bounds__(256) k_predict_wide(PredArgs a, const uint32_t
     const int K = a.K;
     for (int t = 0; t < a.ntrees; ++t) {
         const uint32_t *tr = a.trees + (size_t)t * a.tw;
-        int nid = 1;
-        uint32_t pk = __ldg(tr);
-        while ((pk >> 24) & 1u) {
-            nid = child(pk, xr[(pk & 0xffffu) >> 2], nid);
-            pk = __ldg(tr + nid - 1);
-        }
-        if (a.leaf_idx) a.leaf_idx[(size_t)t * a.out_ld + i] = (uint32_t)nid;
-        pred_add(a.loss, K, p, reinterpret_cast<const float *>(tr + a.nnp) + (size_t)(nid - 1) * K);
+        auto node = [&](int n) { return __ldg(tr + n); };
+        auto word = [&](uint32_t w) { return xr[w]; };
+        int leaf;
+        if (a.leaf_idx) a.leaf_idx[(size_t)t * a.out_ld + i] = (uint32_t)walk_id(a.levels, node, word, leaf);
+        else leaf = walk(a.levels, node, word);
+        add_leaf<KMAX>(a.loss, K, p, reinterpret_cast<const float *>(tr + a.ni) + leaf * K, 1);
     }
-    if (a.apply_link) link_row(a.loss, K, p);
-    for (int k = 0; k < K; ++k) a.out[(size_t)k * a.out_ld + i] = p[k];
+    if (a.apply_link) link_row<KMAX>(a.loss, K, p);
+    put_row<KMAX>(a, i, p);
 }
 
 } // namespace
 
 // ================================================================================================= models
 struct evb_model {
-    int device = 0, loss = 0, K = 1, ntrees = 0, nnp = 4, tw = 8, levels = 0, nfeats = 0, nedges = 0;
+    int device = 0, loss = 0, K = 1, ntrees = 0, ni = 4, tw = 8, levels = 0, nfeats = 0, nedges = 0;
     void *block = nullptr;            // trees, then the edges as double and as float
     const uint32_t *d_trees = nullptr;
     const double *d_e64 = nullptr;
@@ -377,10 +532,17 @@ struct PackJob {
     unsigned char *snap;
     std::atomic<long long> bad; // tree and node of a test that cannot be: (tree << 32 | node) + 1
 };
+template <int K>
+void pack_leaves(float *leaf, const int *at, int n, const char *pred, int KR) { // K 0: KR outputs
+    static const float none[64] = {};
+    const size_t bytes = (size_t)(K ? K : KR) * 4;
+    for (int l = 0; l < n; ++l) memcpy(leaf + (size_t)l * (K ? K : KR), at[l] >= 0 ? pred + (size_t)at[l] * bytes : reinterpret_cast<const char *>(none), bytes);
+}
 void pack_trees(void *ctx, char *dst, size_t first, size_t count) {
     PackJob &j = *static_cast<PackJob *>(ctx);
     const evb_model &m = *j.m;
     uint32_t *tr = reinterpret_cast<uint32_t *>(dst);
+    std::vector<int> at;
     for (size_t t = first; t < first + count; ++t, tr += m.tw) {
         const void *part[4];
         const int nn = j.nodes[t];
@@ -395,24 +557,55 @@ void pack_trees(void *ctx, char *dst, size_t first, size_t count) {
         }
         const unsigned char *feat = static_cast<const unsigned char *>(part[0]); // 8-byte integers, at any address in the snapshot
         const uint8_t *bin = static_cast<const uint8_t *>(part[1]), *split = static_cast<const uint8_t *>(part[2]);
+        const char *pred = static_cast<const char *>(part[3]); // floats, at any address as well
+        float *leaf = reinterpret_cast<float *>(tr + m.ni);
+        const int last = (1 << m.levels) - 1; // first node of the last level
+        at.resize((size_t)2 * last + 1);      // node of the tree that a node of the complete one stands for; -1: no row comes there
+        // (No branch on what a node holds: mispredicted ones and a memcpy call a leaf were two thirds of the time.)
+        bool bad = false;
         for (int i = 0; i < nn; ++i) {
-            uint32_t w = 0u;
-            if (split[i]) {
+            int64_t f;
+            memcpy(&f, feat + (size_t)i * 8, 8);
+            bad |= (split[i] != 0) & ((uint64_t)(f - 1) >= (uint64_t)m.nfeats || 2 * i + 2 >= nn);
+        }
+        if (bad) {
+            for (int i = 0; i < nn; ++i) {
                 int64_t f;
                 memcpy(&f, feat + (size_t)i * 8, 8);
-                f -= 1;
-                if (f < 0 || f >= m.nfeats || 2 * i + 2 >= nn) {
-                    long long none = 0;
-                    j.bad.compare_exchange_strong(none, ((long long)t << 32 | i) + 1);
-                } else {
-                    w = (uint32_t)f | ((uint32_t)bin[i] << 16) | (1u << 24) | ((j.feattypes ? (j.feattypes[f] ? 1u : 0u) : 1u) << 25);
-                }
+                if (!split[i] || (f >= 1 && f <= m.nfeats && 2 * i + 2 < nn)) continue;
+                long long none = 0;
+                j.bad.compare_exchange_strong(none, ((long long)t << 32 | i) + 1);
+                break;
             }
-            tr[i] = w;
+            continue;
         }
-        for (int i = nn; i < m.nnp; ++i) tr[i] = 0u;
-        memcpy(tr + m.nnp, part[3], (size_t)nn * m.K * 4);
-        memset(tr + m.nnp + (size_t)nn * m.K, 0, (size_t)(m.nnp - nn) * m.K * 4);
+        at[0] = 0;
+        for (int i = 0; i < last; ++i) {
+            const int o = at[i], from = o < 0 ? 0 : o;
+            const bool s = (o >= 0) & (split[from] != 0);
+            int64_t f;
+            memcpy(&f, feat + (size_t)from * 8, 8);
+            f = s ? f - 1 : 0;
+            const int shift = !j.feattypes || j.feattypes[f] ? 16 : 24;
+            uint32_t w = (uint32_t)f | (uint32_t)bin[from] << shift;
+            w |= (uint32_t)(w == STOP) << 24; // bin 255 of feature 0: all rows go left as well, but the path does not end
+            tr[i] = s ? w : STOP;
+            at[2 * i + 1] = s ? 2 * o + 1 : o;
+            at[2 * i + 2] = s ? 2 * o + 2 : -1;
+        }
+        for (int i = last; i < m.ni; ++i) tr[i] = 0u;
+        switch (m.K) {
+            case 1: pack_leaves<1>(leaf, at.data() + last, last + 1, pred, 1); break;
+            case 2: pack_leaves<2>(leaf, at.data() + last, last + 1, pred, 2); break;
+            case 3: pack_leaves<3>(leaf, at.data() + last, last + 1, pred, 3); break;
+            case 4: pack_leaves<4>(leaf, at.data() + last, last + 1, pred, 4); break;
+            case 5: pack_leaves<5>(leaf, at.data() + last, last + 1, pred, 5); break;
+            case 6: pack_leaves<6>(leaf, at.data() + last, last + 1, pred, 6); break;
+            case 7: pack_leaves<7>(leaf, at.data() + last, last + 1, pred, 7); break;
+            case 8: pack_leaves<8>(leaf, at.data() + last, last + 1, pred, 8); break;
+            default: pack_leaves<0>(leaf, at.data() + last, last + 1, pred, m.K);
+        }
+        for (int e = (last + 1) * m.K; e < m.tw - m.ni; ++e) leaf[e] = 0.0f;
     }
 }
 
@@ -425,10 +618,10 @@ int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32
     int nn = 1;
     for (int t = 0; t < ntrees; ++t) nn = std::max(nn, (int)nodes[t]);
     m->ntrees = ntrees; m->nfeats = nfeats; m->nedges = edges ? nedges : 0;
-    m->nnp = (nn + 3) & ~3;
-    m->tw = m->nnp * (1 + K);
     m->levels = 0;
     while ((2 << m->levels) - 1 < nn) ++m->levels;
+    m->ni = std::max(4, 1 << m->levels);
+    m->tw = m->ni + (((K << m->levels) + 3) & ~3);
     const size_t unit = (size_t)m->tw * 4, tbytes = (size_t)ntrees * unit, ne = (size_t)m->nedges * nfeats;
     const size_t o64 = (tbytes + 15) & ~(size_t)15, o32 = o64 + ne * 8, total = o32 + ne * 4 + 16;
     PackJob job{m, src, nodes, feattypes, nullptr, {0}};
@@ -444,8 +637,8 @@ int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32
         if (edges) { m->src_edges = edges; m->snap_edges.assign((const unsigned char *)edges, (const unsigned char *)edges + ne * (e_dtype == EVB_F64 ? 8 : 4)); }
         if (feattypes) { m->src_ft = feattypes; m->snap_ft.assign(feattypes, feattypes + nfeats); }
     }
-    // Below a megabyte everything goes up in one copy of an ordinary buffer (so do trees that are larger than a pinned buffer).
-    const bool piped = tbytes > ((size_t)1 << 20) && unit <= evb_stage_bytes();
+    // Below half a megabyte everything goes up in one copy of an ordinary buffer (so do trees that are larger than a pinned buffer).
+    const bool piped = tbytes > ((size_t)512 << 10) && unit <= evb_stage_bytes();
     const size_t hosted = piped ? o64 : 0; // bytes of the block that are not in `host`
     std::vector<unsigned char> host(total - hosted);
     if (edges) {
@@ -608,19 +801,18 @@ int32_t allow_smem(K kern, size_t bytes) { // more than the default 48 KB of dyn
 }
 
 // which kernel takes a chunk of n rows (what one launch gets, not what the call has)
-enum { PK_ONE, PK_MID, PK_STAGED, PK_WIDE };
+enum { PK_ONE, PK_MID, PK_TILES, PK_STAGED, PK_WIDE };
 struct PredPlan { int kind, rows, TB; size_t smem; };
-PredPlan plan_kernel(const evb_model &m, int n, int num_sms) {
+PredPlan plan_kernel(const evb_model &m, int n, bool more, int num_sms) { // more: another chunk's kernel will run beside this one
     PredPlan p{PK_WIDE, 256, 0, 0};
     const int FW = (m.nfeats + 3) / 4;
     const size_t tree = (size_t)m.tw * 4;
     // a CTA per row while the rows alone do not give every SM several of the 32-row CTAs of the next kernel
     const size_t one = (size_t)FW * 4 + (size_t)ONE_THREADS * m.K * 4;
     if (n <= 4 * num_sms && one <= 96 * 1024) return {PK_ONE, 1, 0, one};
-    // Staged: the largest CTA that still gives every SM one, as long as two blocks of trees fit beside its rows.  Copying
-    // all trees once per CTA has to be worth it: below `mid_rows` rows of a launch the trees are read through L1 instead.  ms of
-    // kernels, staged and mid, chunks one after the other: 1M x 100, depth 11 (30k rows a chunk) 10.1 and 5.3; 1M x 50 gaussian, depth 7
-    // (59k) 4.14 and 3.34; 1M x 28 five classes, depth 8 (79k) 4.53 and 4.93; 4M x 10, depth 6 (285k) 3.13 and 4.27.
+    // Staged: the largest CTA that still gives every SM one, as long as two blocks of trees fit beside its rows.  One thread a row needs rows:
+    // below `mid_rows` of a launch the next kernel is faster.  ms of kernels of a call, staged and tiles: 4M x 10, depth 6 (285k rows a
+    // chunk) 3.10 and 3.65; 1M x 28 five classes, depth 8 (79k) 2.95 and 2.68; 300k x 6, depth 9 (50k) 0.52 and 0.43.
     const int mid_rows = 64 * 1024;
     if (n > mid_rows) {
         for (int rows = 1024; rows >= 128; rows >>= 1) {
@@ -631,6 +823,19 @@ PredPlan plan_kernel(const evb_model &m, int n, int num_sms) {
             return {PK_STAGED, rows, TB, rb + 2 * (size_t)TB * tree};
         }
     }
+    {
+        // The fewest groups of rows a CTA with which all CTAs have an SM at once (chunks overlap: twice their rows, but the last one's time shows): every CTA copies all trees.  us of a
+        // call, 1, 2 and 4 groups: 900 x 12 seven classes 59, 63, 71; 9k x 12 seven classes 112, 99, 107; 20k x 28 five classes, in chunks (every one with two times its rows) 203, 180, 190;
+        // 6k x 30, depth 10 115, 122, 132; 90k x 12 seven classes, in chunks 529, 383, 342.  k_predict_mid: 77, 122, 206, 127, 489.
+        const int RG = std::max(1, std::min(4, (n * (more ? 2 : 1) + 32 * num_sms - 1) / (32 * num_sms)));
+        const size_t R = 32 * RG, room = (size_t)216 * 1024, bins = FW * R * 4, per = 2 * (tree + m.K * R * 4);
+        if (bins + per <= room) {
+            const int most = (int)((room - bins) / per), walk = TILE_WARPS / RG - 1;
+            int TB = std::min(most, 64);
+            if (TB > walk) TB = TB / walk * walk;
+            return {PK_TILES, RG, TB, bins + (size_t)TB * per};
+        }
+    }
     const size_t rb = (size_t)FW * 128;
     int TB = std::max(1, 96 / m.K); // 2 x TB x K x 128 bytes <= 24 KB
     if (TB > (MID_WARPS - 1) * MID_ILP) TB = TB / ((MID_WARPS - 1) * MID_ILP) * ((MID_WARPS - 1) * MID_ILP);
@@ -639,6 +844,12 @@ PredPlan plan_kernel(const evb_model &m, int n, int num_sms) {
     return p;
 }
 
+template <int K, typename T>
+int32_t launch_tiles(const PredPlan &p, const PredArgs &a, cudaStream_t st) {
+    EVB_CHECK(allow_smem(k_predict_tiles<K, T>, p.smem));
+    k_predict_tiles<K, T><<<(a.n + 32 * p.rows - 1) / (32 * p.rows), TILE_WARPS * 32, p.smem, st>>>(a, p.rows, p.TB);
+    return EVB_OK;
+}
 template <int KMAX, typename T>
 int32_t launch_t(const PredPlan &p, PredArgs &a, uint32_t *xw, cudaStream_t st) {
     if (p.kind == PK_ONE) {
@@ -647,6 +858,18 @@ int32_t launch_t(const PredPlan &p, PredArgs &a, uint32_t *xw, cudaStream_t st) 
     } else if (p.kind == PK_MID) {
         EVB_CHECK(allow_smem(k_predict_mid<KMAX, T>, p.smem));
         k_predict_mid<KMAX, T><<<(a.n + 31) / 32, MID_WARPS * 32, p.smem, st>>>(a, p.TB);
+    } else if (p.kind == PK_TILES) {
+        if constexpr (KMAX > 8) EVB_CHECK((launch_tiles<64, T>(p, a, st)));
+        else switch (a.K) { // outputs known at compile time: adding a tree is a third shorter
+            case 1: EVB_CHECK((launch_tiles<1, T>(p, a, st))); break;
+            case 2: EVB_CHECK((launch_tiles<2, T>(p, a, st))); break;
+            case 3: EVB_CHECK((launch_tiles<3, T>(p, a, st))); break;
+            case 4: EVB_CHECK((launch_tiles<4, T>(p, a, st))); break;
+            case 5: EVB_CHECK((launch_tiles<5, T>(p, a, st))); break;
+            case 6: EVB_CHECK((launch_tiles<6, T>(p, a, st))); break;
+            case 7: EVB_CHECK((launch_tiles<7, T>(p, a, st))); break;
+            default: EVB_CHECK((launch_tiles<8, T>(p, a, st)));
+        }
     } else if (p.kind == PK_STAGED) {
         EVB_CHECK(allow_smem(k_predict_staged<KMAX, T>, p.smem));
         k_predict_staged<KMAX, T><<<(a.n + p.rows - 1) / p.rows, p.rows, p.smem, st>>>(a, p.TB);
@@ -696,7 +919,7 @@ int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, 
     PredArgs a;
     a.row_major = row_major; a.nedges = m.nedges; a.nfeats = m.nfeats; a.FW = (m.nfeats + 3) / 4;
     a.edges = x_type == EVB_F64 ? (const void *)m.d_e64 : (const void *)m.d_e32;
-    a.trees = m.d_trees; a.nnp = m.nnp; a.tw = m.tw; a.levels = m.levels; a.K = m.K; a.loss = m.loss; a.ntrees = ntrees; a.apply_link = apply_link;
+    a.trees = m.d_trees; a.ni = m.ni; a.tw = m.tw; a.levels = m.levels; a.K = m.K; a.loss = m.loss; a.ntrees = ntrees; a.apply_link = apply_link;
     int64_t first[PRED_SLOTS] = {-1, -1, -1};
     int rows_in[PRED_SLOTS] = {};
     double ms = 0.0, until = 0.0; // ms during which kernels ran, up to `until` ms after the start (chunks overlap)
@@ -741,7 +964,7 @@ int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, 
         }
         a.out = reinterpret_cast<float *>(s.pin_out); a.out_ld = nr;
         a.leaf_idx = leaf_idx ? reinterpret_cast<uint32_t *>(s.pin_out + (size_t)nr * 4 * m.K) : nullptr;
-        const PredPlan p = plan_kernel(m, (int)nr, sms);
+        const PredPlan p = plan_kernel(m, (int)nr, r0 + nr < nobs, sms);
         if (p.kind == PK_WIDE) EVB_CHECK(device_reserve(s.d_aux, s.cap_aux, (size_t)chunk * a.FW * 4));
         if (ms_out) EVB_CUDA(cudaEventRecord(s.t0, s.st));
         uint32_t *xw = static_cast<uint32_t *>(s.d_aux);

@@ -135,3 +135,49 @@ def test_kernel_time_counts_overlap_once(pkg):
         t = time.perf_counter()
         pkg.predict(m, x, stats=stats)
         assert 0.0 < stats["kernel_ms"] <= (time.perf_counter() - t) * 1e3
+
+
+@pytest.mark.parametrize("K,loss", [(1, "mse"), (1, "logloss"), (2, "gaussian_mle"), (3, "mlogloss"), (5, "mlogloss"), (7, "mlogloss"), (8, "mlogloss"), (9, "mlogloss")])
+@pytest.mark.parametrize("n,depth,ntrees", [(593, 5, 1), (4_737, 9, 70), (20_011, 7, 33)])
+def test_incomplete_trees_row_groups_and_outputs(pkg, K, loss, n, depth, ntrees):
+    """Trees whose paths end anywhere, categories, a test that every bin passes; every number of outputs that has a kernel of its own"""
+    rng = np.random.default_rng(n + K)
+    F, B, nn = 6, 255, 2 ** depth - 1
+    edges = np.sort(rng.normal(size=(F, B - 1)).astype(np.float32), axis=1)
+    ft = rng.random(F) < 0.6
+    trees = []
+    for _ in range(ntrees):
+        split = (rng.random(nn) < 0.85) & (np.arange(nn) < nn // 2)
+        for i in range(1, nn):
+            split[i] &= split[(i - 1) // 2]
+        feat, cond = rng.integers(0, F, nn), rng.integers(1, 256, nn)
+        cond[rng.random(nn) < 0.05] = 255
+        trees.append(pkg.Tree(np.where(split, feat + 1, 0).astype(np.int64), np.where(split, cond, 0).astype(np.uint8), np.zeros(nn, np.float32), np.zeros(nn, np.float32),
+                              rng.normal(size=(nn, K)).astype(np.float32), split.astype(np.uint8)))
+    m = pkg.EvoTree(loss, K, trees, {"edges": edges, "feattypes": ft, "feature_names": [f"f{i}" for i in range(F)], "target_levels": None, "featbins": np.full(F, B, np.uint8)})
+    x = rng.normal(size=(n, F)).astype(np.float32)
+    xb = np.stack([1 + np.searchsorted(edges[j], x[:, j], side="left") for j in range(F)], 1)
+    p, ids = np.zeros((n, K), np.float32), np.empty((n, ntrees), np.int64)
+    for t, tr in enumerate(trees):
+        nid = np.ones(n, np.int64)
+        for _ in range(depth - 1):
+            s = tr.split[nid - 1] != 0
+            f, c = np.maximum(tr.feat[nid - 1] - 1, 0), tr.cond_bin[nid - 1]
+            v = xb[np.arange(n), f]
+            left = np.where(ft[f], v <= c, v == c)
+            nid = np.where(s, 2 * nid + ~left, nid)
+        ids[:, t] = nid
+        p += tr.pred[nid - 1]
+        if loss == "logloss":
+            p = np.clip(p, np.float32(-15), np.float32(15))
+        elif loss == "gaussian_mle":
+            p[:, 1] = np.maximum(np.float32(-15), p[:, 1])
+        elif loss == "mlogloss":
+            p = np.maximum(np.float32(-15), p - p.max(1, keepdims=True))
+    assert np.array_equal(pkg.predict_leaf_idx(m, x), ids)
+    got = pkg.predict(m, x).reshape(n, -1)
+    p = p.astype(np.float64)
+    want = {"mse": lambda: p, "logloss": lambda: 1 / (1 + np.exp(-p)), "gaussian_mle": lambda: np.stack([p[:, 0], np.log1p(np.exp(-abs(p[:, 1]))) + np.maximum(p[:, 1], 0)], 1),
+            "mlogloss": lambda: np.exp(p) / np.exp(p).sum(1, keepdims=True)}[loss]()
+    # the sums are the same float32 additions in the same order; the link's functions are within a few units in the last place
+    np.testing.assert_allclose(got, want, rtol=2e-6, atol=1e-7)
