@@ -59,7 +59,7 @@ enum evb_dtype { EVB_F32 = 0, EVB_U32 = 1, EVB_F64 = 2 };
 
 /* flags of evb_params.flags */
 #define EVB_FLAG_TIMING 1u         /* record a CUDA-event pair (and an NVTX range) around every kernel class (see evb_get_timings) */
-#define EVB_FLAG_FULL_PARTITION 2u /* also partition the rows of the last split level (only evb_get_nidx(.., 1) reads that) */
+#define EVB_FLAG_FULL_PARTITION 2u /* also partition the rows of the last split level (only evb_get_nidx(.., 1) reads that); trees are grown level by level, whatever the size */
 #define EVB_FLAG_KEEP_ALL_HIST 4u  /* retain the histograms of the last split level too (for evb_get_hist)               */
 
 /* Learner hyper-parameters needed on the device; filled by the glue from the reference's learner
@@ -80,7 +80,8 @@ typedef struct {
 } evb_params;
 
 /* Accumulated device time per kernel class since the last evb_reset_timings (EVB_FLAG_TIMING).  EVB_T_PLAN and EVB_T_D2H stay zero: the
- * plan of a level is made by the last CTA of the partition, and the finished tree is written to the host by the last kernel. */
+ * plan of a level is made by the last CTA of the partition, and the finished tree is written to the host by the last kernel.  A tree that is
+ * grown in one launch counts under EVB_T_HIST. */
 #define EVB_NTIMERS 12
 enum evb_timer {
     EVB_T_GRADS = 0, EVB_T_ROWS_INIT = 1, EVB_T_HIST = 2, EVB_T_HIST_REDUCE = 3, EVB_T_ALLREDUCE = 4,
