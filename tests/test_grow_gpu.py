@@ -139,3 +139,29 @@ def test_bags_and_replays(pkg):
         out.append((np.concatenate([t.pred for t in m.trees]), c.pred()))
         c.close()
     assert len(m.trees) == 21 and all(np.array_equal(p, q) for p, q in zip(*out))
+
+
+def test_handles_side_by_side(pkg):
+    """Handles of several threads on streams of their own: whole-GPU launches, clusters, level kernels and inference at the same time"""
+    from concurrent.futures import ThreadPoolExecutor
+    shapes = [("mse", 100_003, 10, 32, 6), ("logloss", 1_503, 7, 64, 5), ("poisson", 60_013, 40, 64, 6), ("mse", 300_007, 40, 64, 6), ("gamma", 3_001, 9, 64, 7), ("mse", 100_003, 10, 32, 6)]
+
+    def run(s):
+        loss, n, F, B, depth = s
+        x, y, w = _data(n, F, B, loss, n + F, False)
+        params = pkg.EvoTreeRegressor(loss=loss, nrounds=1, max_depth=depth, nbins=B, eta=0.2)
+        c = _cache(pkg, params, x, y, w, 0)
+        try:
+            m = pkg.EvoTree(loss, 1, [], {"edges": np.sort(np.random.default_rng(F).random((F, B - 1)).astype(np.float32), axis=1), "feattypes": np.ones(F, bool), "nrounds": 0})
+            out = []
+            for _ in range(4):
+                pkg.grow_rounds(m, c, params, 10)
+                out.append(pkg.predict(m, (x[:5_000] / B).astype(np.float32)))
+            return np.concatenate([t.pred for t in m.trees]), c.pred(), np.stack(out)
+        finally:
+            c.close()
+
+    alone = [run(s) for s in shapes]
+    with ThreadPoolExecutor(len(shapes)) as pool:
+        for a, b in zip(alone, pool.map(run, shapes)):
+            assert all(np.array_equal(p, q) for p, q in zip(a, b))
