@@ -170,6 +170,14 @@ static void free_handle(evb_handle *h) {
 
 extern "C" void evb_destroy(evb_handle *h) { free_handle(h); }
 
+// sums of whole trees in one launch (evb_grow.cu)
+static cudaError_t clear_grow_sums(evb_handle *h) {
+    cudaError_t e = cudaMemsetAsync(h->g_sum, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->g_cnt, 0, 2 * evb_grow_cnts(h) * sizeof(uint32_t), h->st);
+    if (e == cudaSuccess && h->g_low) e = cudaMemsetAsync(h->g_low, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st);
+    return e;
+}
+
 // x_bin: the binned matrix; mx: the raw matrix on the device; else the raw matrix x on the host (x_dtype), with its edges
 static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int32_t nfeats, const uint8_t *x_bin, const evb_matrix *mx,
                            const void *x, int32_t x_dtype, const void *edges, int32_t nedges, const void *y,
@@ -291,12 +299,8 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
     if (h->grow.on) {
         EVB_CUDA(dalloc(&h->g_sum, 2 * evb_grow_sums(h))); EVB_CUDA(dalloc(&h->g_cnt, 2 * evb_grow_cnts(h))); EVB_CUDA(dalloc(&h->g_best, 2 * evb_grow_best(h)));
         EVB_CUDA(dalloc(&h->g_bar, (size_t)2));
-        EVB_CUDA(cudaMemsetAsync(h->g_sum, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st));
-        EVB_CUDA(cudaMemsetAsync(h->g_cnt, 0, 2 * evb_grow_cnts(h) * sizeof(uint32_t), h->st));
-        if (!h->hgeo.pack) {
-            EVB_CUDA(dalloc(&h->g_low, 2 * evb_grow_sums(h)));
-            EVB_CUDA(cudaMemsetAsync(h->g_low, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st));
-        }
+        if (!h->hgeo.pack) EVB_CUDA(dalloc(&h->g_low, 2 * evb_grow_sums(h)));
+        EVB_CUDA(clear_grow_sums(h));
     }
 
     // ---- uploads: x_bin is kept feature-major (as given) for the row partition and transposed on the device to
@@ -529,7 +533,12 @@ static int32_t tree_begin(evb_handle *h, const uint8_t *row_mask, uint64_t *gen,
         EVB_CUDA(cudaStreamSynchronize(h->st));
         h->F = njs;
         h->gradq_valid = false; // how g is rounded may depend on it
-        if (h->g_sum) evb_grow_configure(h);
+        if (h->g_sum) {
+            // one range of rows stores its sums and leaves them; several, which add theirs up, start from zeros
+            const bool stored = h->grow.on && h->grow.NR == 1;
+            evb_grow_configure(h);
+            if (stored) EVB_CUDA(clear_grow_sums(h));
+        }
         drop_graphs(h);
     }
     if (update_grads) h->bag_idx = 0;
@@ -633,9 +642,7 @@ extern "C" int32_t evb_grow_tree_end(evb_handle *h, int64_t *feat, uint8_t *cond
         if (h->g_sum) { // a tree that was given up leaves its sums
             cudaMemsetAsync(h->g_bar, 0, 2 * sizeof(uint32_t), h->st);
             cudaMemsetAsync(h->low, 0, sizeof(uint32_t) * (h->nn + 2), h->st);
-            cudaMemsetAsync(h->g_sum, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st);
-            cudaMemsetAsync(h->g_cnt, 0, 2 * evb_grow_cnts(h) * sizeof(uint32_t), h->st);
-            if (h->g_low) cudaMemsetAsync(h->g_low, 0, 2 * evb_grow_sums(h) * sizeof(unsigned long long), h->st);
+            clear_grow_sums(h);
         }
         return EVB_ERR_DEVICE;
     }

@@ -74,6 +74,28 @@ def test_samples_of_rows_and_columns(pkg, loss, weighted):
     _same(pkg, params, x, y, w, rounds=8, samples=[(m, j) for j in js for m in (mask, None)])
 
 
+# rows, columns, loss, weights, numbers of sampled columns of the trees one after the other; row ranges of the kernel (148 SMs)
+COLUMN_COUNTS = [(2_000, 400, "mse", False, (400, 200, 400, 100)),       # 1, 2, 1, 3 over the grid
+                 (5_000, 300, "gamma", True, (300, 100, 300, 150)),      # 1, 5, 1, 2 or more
+                 (2_500, 64, "gamma", True, (64, 32, 64, 16)),           # one cluster: 1, 2, 1, 4
+                 (900, 100, "logloss", True, (100, 30, 100, 7))]         # the grid's one range, then a cluster
+
+
+@pytest.mark.parametrize("n,F,loss,weighted,counts", COLUMN_COUNTS)
+def test_another_number_of_columns_in_every_tree(pkg, n, F, loss, weighted, counts):
+    """One range of rows stores its sums, several add theirs up: what a tree leaves behind must not be found by the next.  Gradients over many
+    orders of magnitude, so that the second set of sums is used too."""
+    x, y, w = _data(n, F, 64, loss, 11, weighted)
+    rng = np.random.default_rng(n)
+    if loss == "gamma":
+        y = np.exp(4.0 * rng.normal(size=n)).astype(np.float32)
+    if w is not None:
+        w = np.exp(4.0 * rng.normal(size=n)).astype(np.float32)
+    js = [(np.sort(rng.permutation(F)[:k]) + 1).astype(np.uint32) for k in counts]
+    params = pkg.EvoTreeRegressor(loss=loss, nrounds=1, max_depth=5, nbins=64, eta=0.3)
+    _same(pkg, params, x, y, w, rounds=2 * len(js), samples=[(None, j) for j in js])
+
+
 def test_categories_and_constraints(pkg):
     n, F = 30_011, 9
     x, y, w = _data(n, F, 40, "logloss", 8, False)
