@@ -79,6 +79,7 @@ struct BusyGuard {
     if (!(h)) { evb_set_error("null handle"); return EVB_ERR_ARG; }                    \
     BusyGuard _guard(h);                                                               \
     if (!_guard.ok) { evb_set_error("handle is in use by another thread"); return EVB_ERR_BUSY; } \
+    if ((h)->failed) { evb_set_error("a tree of this handle was given up: it can only be destroyed"); return EVB_ERR_DEVICE; } \
     EVB_CUDA(cudaSetDevice((h)->dev));                                                 \
     g_alloc_stream = (h)->st
 
@@ -301,6 +302,7 @@ static int32_t create_impl(evb_handle *h, const evb_params *p, int64_t nobs, int
         EVB_CUDA(dalloc(&h->g_bar, (size_t)2));
         if (!h->hgeo.pack) EVB_CUDA(dalloc(&h->g_low, 2 * evb_grow_sums(h)));
         EVB_CUDA(clear_grow_sums(h));
+        h->grow_polls = 8000000u; // seconds
     }
 
     // ---- uploads: x_bin is kept feature-major (as given) for the row partition and transposed on the device to
@@ -638,12 +640,10 @@ extern "C" int32_t evb_grow_tree_end(evb_handle *h, int64_t *feat, uint8_t *cond
                       : derr == EVB_DERR_WAIT_EMPTY ? "bounded wait for a free stage expired"
                       : derr == EVB_DERR_GRID ? "bounded wait for the other CTAs of a tree expired"
                       : derr == EVB_DERR_PEER ? "bounded wait for the other ranks expired" : "unknown");
-        cudaMemsetAsync(h->d_err, 0, sizeof(int), h->st);
-        if (h->g_sum) { // a tree that was given up leaves its sums
-            cudaMemsetAsync(h->g_bar, 0, 2 * sizeof(uint32_t), h->st);
-            cudaMemsetAsync(h->low, 0, sizeof(uint32_t) * (h->nn + 2), h->st);
-            clear_grow_sums(h);
-        }
+        // Another tree may be in flight behind this one.  The tree kernel sees the error word and ends before it adds to what is left of
+        // this one; what has been done to the predictions by then is not known.
+        if (derr == EVB_DERR_GRID) h->failed = true;
+        else cudaMemsetAsync(h->d_err, 0, sizeof(int), h->st);
         return EVB_ERR_DEVICE;
     }
     memcpy(h->last_eval, hb + L.evsum, sizeof(h->last_eval));
@@ -868,6 +868,17 @@ extern "C" int32_t evb_test_peer_timeout(evb_handle *h, int32_t max_polls) {
     if (derr == EVB_DERR_PEER) { evb_set_error("device self-check failed (code %d: bounded wait for the other ranks expired)", derr); return EVB_ERR_DEVICE; }
     evb_set_error("evb_test_peer_timeout: the wait did not run out (error word %d)", derr);
     return EVB_ERR_ARG;
+}
+
+extern "C" int32_t evb_test_grid_timeout(evb_handle *h, int32_t max_polls) {
+    EVB_ENTER(h);
+    if (max_polls < 1 || max_polls > 8000000) { evb_set_error("evb_test_grid_timeout: max_polls outside 1..8000000"); return EVB_ERR_ARG; }
+    if (h->pending > 0) { evb_set_error("evb_test_grid_timeout: a tree is in flight"); return EVB_ERR_BUSY; }
+    if (!evb_grows_whole(h) || h->grow.cluster || h->grow.NG * h->grow.NR < 2) { evb_set_error("evb_test_grid_timeout: this handle's trees have no barrier of the grid"); return EVB_ERR_ARG; }
+    EVB_CUDA(cudaMemsetAsync(h->g_bar, 0xff, sizeof(uint32_t), h->st)); // one arrival less than none
+    h->grow_polls = (unsigned)max_polls;
+    drop_graphs(h); // the limit is an argument of the launch
+    return EVB_OK;
 }
 
 extern "C" int32_t evb_set_timing(evb_handle *h, int32_t on) {

@@ -885,6 +885,7 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
     const int per_up = ((a.rpc >> 5) + a.NG - 1) / a.NG * 32, u0 = min(g * per_up, nr), u1 = min(u0 + per_up, nr); // rows this CTA updates
     if (blockIdx.x == 0 && threadIdx.x < NQ) a.gmax_next[threadIdx.x] = (int)threadIdx.x < a.ng ? 0u : a.gmax[threadIdx.x]; // (weights keep theirs)
     if (threadIdx.x == 0) {
+        S_MISC[M_OK] = *(volatile int *)a.err == 0;
         S_MISC[M_LEFT] = 0; S_MISC[M_CNT] = 0; S_MISC[M_MAX] = 0; S_MISC[M_MAX + 1] = 0;
         const Pairs root = S_PAIRS(0);
         root.dec()[0] = 1u; root.build()[0] = 0; root.st()[0] = 0;
@@ -941,6 +942,10 @@ __global__ void __launch_bounds__(T, 1) k_grow(GrowArgs a) {
         }
     }
     __syncthreads();
+    if (!S_MISC[M_OK]) { // the tree before this one was given up: its barriers have counts and its sums rows left
+        if (a.pub_dst && threadIdx.x == 0) reinterpret_cast<volatile int *>(a.pub_dst)[a.pub_err] = *(volatile int *)a.err;
+        return;
+    }
     {
         Quant k[NQ];
 #pragma unroll
@@ -1258,7 +1263,7 @@ int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot,
     memcpy(a.lc, g.lc, sizeof(a.lc));
     a.o_sum = g.o_sum; a.o_cnt = g.o_cnt; a.o_best = g.o_best; a.o_hist = g.o_hist; a.fo = g.fo;
     a.o_x = g.o_x; a.o_q = a.o_x + (g.rpc * 4 << g.lw); a.o_idx = a.o_q + g.rpc * 4 * h->nq; a.o_node = a.o_idx + g.rpc * 4;
-    a.max_polls = 8000000u; // seconds
+    a.max_polls = h->grow_polls;
     a.low_unit = evb_hg_low_unit(h); a.neb = -h->p.eta / (double)h->p.bagging_size;
     a.lambda = h->p.lambda; a.L2 = h->p.L2; a.gamma = h->p.gamma; a.min_weight = h->p.min_weight;
     a.alpha = evb_alpha_set(h);

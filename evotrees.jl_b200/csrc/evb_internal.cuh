@@ -178,6 +178,8 @@ struct evb_handle {
     uint32_t *g_cnt;                   // [2][maxslots][nfeats][B]
     double2 *g_best;
     uint32_t *g_bar;
+    unsigned grow_polls;               // of a wait at the grid's barrier before the tree is given up
+    bool failed;                       // a tree was given up: predictions, gradients and sums are in no defined state, calls are refused
 
     // histograms
     double *hist;     // [2^(D-2) nodes][F][C][B] retained for the subtraction trick

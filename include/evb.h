@@ -258,6 +258,13 @@ EVB_API int32_t evb_eval_detach(evb_handle *h);
  */
 EVB_API int32_t evb_test_peer_timeout(evb_handle *h, int32_t max_polls);
 
+/*
+ * The same for the barrier of the kernel that grows a whole tree: the barriers of the handle's next tree wait for one arrival more than there
+ * are blocks, for max_polls polls (under a microsecond each).  evb_grow_tree* then returns EVB_ERR_DEVICE, and so does every later call on the
+ * handle, which can only be destroyed: other trees may have been in flight.  EVB_ERR_ARG: trees of this handle have no such barrier.
+ */
+EVB_API int32_t evb_test_grid_timeout(evb_handle *h, int32_t max_polls);
+
 /* Switches the per-kernel CUDA-event timing of EVB_FLAG_TIMING on or off (timed trees run without graphs); with it
  * on, every kernel class is also an NVTX range ("evb:hist", "evb:scan", ...). */
 EVB_API int32_t evb_set_timing(evb_handle *h, int32_t on);

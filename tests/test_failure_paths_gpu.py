@@ -73,6 +73,41 @@ def test_bounded_wait_for_a_silent_peer_runs_out(pkg):
     cache.close()
 
 
+@pytest.mark.parametrize("masked,in_flight", [(False, 1), (False, 2), (True, 1), (True, 2)])
+def test_bounded_wait_for_other_blocks_runs_out(pkg, masked, in_flight):
+    """A barrier of the tree kernel that one arrival never reaches: trees in flight end with an error, the handle is refused from then on,
+    others work."""
+    from evotrees_b200 import _lib
+    lib = _lib.lib()
+    cache, params = _cache(pkg, n=30_000, depth=6)
+    js = np.arange(1, cache.nfeats + 1, dtype=np.uint32)
+    mask = (np.arange(cache.nobs) % 3).astype(np.uint8) if masked else None
+    args = (cache.handle, _lib.ptr(mask), C.c_uint8(1), _lib.ptr(js), C.c_int32(js.size), C.c_int32(1))
+    first = pkg.grow_tree(cache, params, mask, js, True)
+    assert first.split[0] and cache.timings()["launches"]["scan"] == 0            # the tree kernel
+    assert lib.evb_test_grid_timeout(cache.handle, C.c_int32(0)) == -1
+    assert lib.evb_test_grid_timeout(cache.handle, C.c_int32(5_000)) == 0         # milliseconds
+    t = pkg.Tree.empty(params.max_depth, 1)
+    out = [_lib.ptr(getattr(t, k)) for k in ("feat", "cond_bin", "w", "gain", "pred", "split")]
+    for _ in range(in_flight):
+        assert lib.evb_grow_tree_begin(*args) == 0
+    assert lib.evb_grow_tree_end(cache.handle, *out) == -5                        # EVB_ERR_DEVICE
+    assert "other CTAs of a tree expired" in lib.evb_last_error().decode()
+    for call in (lambda: lib.evb_grow_tree_end(cache.handle, *out), lambda: lib.evb_grow_tree_begin(*args), lambda: lib.evb_test_grid_timeout(cache.handle, C.c_int32(9))):
+        assert call() == -5 and "only be destroyed" in lib.evb_last_error().decode()
+    with pytest.raises(_lib.EvbError):
+        cache.pred()
+    cache.close()
+    for depth in (6, 11):                                                         # the same blocks of memory again; level kernels have no such barrier
+        cache, params = _cache(pkg, n=30_000, depth=depth)
+        again = pkg.grow_tree(cache, params, mask, js, True)
+        if depth == 6:
+            assert all(np.array_equal(getattr(first, k), getattr(again, k)) for k in ("feat", "cond_bin", "split", "w", "gain", "pred"))
+        else:
+            assert lib.evb_test_grid_timeout(cache.handle, C.c_int32(9)) == -1
+        cache.close()
+
+
 def test_peer_access_setup_out_of_order(pkg):
     from evotrees_b200 import _lib
     lib = _lib.lib()
