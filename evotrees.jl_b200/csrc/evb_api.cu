@@ -465,6 +465,7 @@ extern "C" int32_t evb_comm_init(evb_handle *h, const uint8_t id[128], int32_t r
     if (world == 1) return EVB_OK;
     if (!h->hcomp) EVB_CUDA(dalloc(&h->hcomp, (size_t)h->maxslots * h->nfeats * h->C * h->B));
     drop_graphs(h);
+    h->gradq_valid = false; // the level kernels' words: trees grown in one launch have not made them
     EVB_CHECK(evb_nccl_init(h, id, rank, world));
     return EVB_OK;
 }

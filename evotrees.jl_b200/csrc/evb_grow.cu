@@ -1235,7 +1235,6 @@ void evb_grow_configure(evb_handle *h) {
         break; // few features a CTA: fewer row ranges share a sum
     }
     cluster_geom(h, g, least);
-    if (g.on && !h->hgeo.pack) { h->hgeo.hb = g.hb; h->hgeo.TE = (1 << (26 - g.hb)) - 1; } // how k_tree_begin scales g
 }
 
 // words of the sums and of the counts of one level; records of one level
@@ -1256,7 +1255,7 @@ int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot,
     a.gmax = evb_gmax(h, false); a.gmax_next = evb_gmax(h, true);
     a.t_feat = h->t_feat; a.t_bin = h->t_bin; a.t_split = h->t_split; a.t_gain = h->t_gain; a.t_w = h->t_w; a.t_pred = h->t_pred; a.t_packed = h->t_packed;
     a.plan = h->plan; a.bar = h->g_bar; a.err = h->d_err; a.n = h->n;
-    a.F = h->F; a.B = h->B; a.D = h->D; a.hist_nodes = h->hist_nodes; a.loss = h->p.loss; a.elide = h->Ce != h->C; a.hb = h->hgeo.hb; a.ng = h->ng; a.nn = h->nn;
+    a.F = h->F; a.B = h->B; a.D = h->D; a.hist_nodes = h->hist_nodes; a.loss = h->p.loss; a.elide = h->Ce != h->C; a.hb = g.hb; a.ng = h->ng; a.nn = h->nn;
     a.round_bits = evb_hg_round_bits(h);
     a.NG = g.NG; a.NR = g.NR; a.rpc = g.rpc; a.lw = g.lw; a.M = 1 << std::max(1, h->D - 2);
     static_assert(sizeof(a.lc) == sizeof(g.lc), "levels");
@@ -1264,7 +1263,7 @@ int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot,
     a.o_sum = g.o_sum; a.o_cnt = g.o_cnt; a.o_best = g.o_best; a.o_hist = g.o_hist; a.fo = g.fo;
     a.o_x = g.o_x; a.o_q = a.o_x + (g.rpc * 4 << g.lw); a.o_idx = a.o_q + g.rpc * 4 * h->nq; a.o_node = a.o_idx + g.rpc * 4;
     a.max_polls = h->grow_polls;
-    a.low_unit = evb_hg_low_unit(h); a.neb = -h->p.eta / (double)h->p.bagging_size;
+    a.low_unit = evb_hg_low_unit(g.hb); a.neb = -h->p.eta / (double)h->p.bagging_size;
     a.lambda = h->p.lambda; a.L2 = h->p.L2; a.gamma = h->p.gamma; a.min_weight = h->p.min_weight;
     a.alpha = evb_alpha_set(h);
     if (!masked) {

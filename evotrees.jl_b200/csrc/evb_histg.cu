@@ -207,7 +207,7 @@ int32_t evb_launch_acc_clear(evb_handle *h, int level) {
 int32_t evb_launch_acc_to_hcomp(evb_handle *h, int level) {
     ConvArgs a;
     a.hsum = h->hsum_q; a.hcnt = h->hcnt_q; a.hcomp = h->hcomp; a.plan = h->plan + level; a.js0 = h->js_d; a.qinv = h->d_qinv;
-    a.hlow = h->hlow_q; a.low = h->low + evb_low_slot(level); a.low_unit = evb_hg_low_unit(h);
+    a.hlow = h->hlow_q; a.low = h->low + evb_low_slot(level); a.low_unit = evb_hg_low_unit(h->hgeo.hb);
     a.B = h->B; a.SC = h->SC; a.F = h->F; a.C = h->C; a.K = h->K; a.nq = h->nq; a.elide = h->Ce != h->C; a.unit_w = h->unit_w;
     evb_tic(h, EVB_T_HIST_REDUCE);
     k_hg_to_hcomp<<<dim3(evb_level_slots(level), (h->F + 31) / 32), 256, 0, h->st>>>(a);

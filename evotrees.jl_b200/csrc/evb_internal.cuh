@@ -74,7 +74,7 @@ struct HGeom {
 struct GrowGeom {
     bool on;
     int lw, NG, NR, rpc; // log2 of the words of four features a CTA takes; CTAs side by side: feature groups x row ranges; rows of a range
-    int hb;              // bits of the high words
+    int hb;              // bits of the high words (the level kernels have their own: HGeom)
     uint8_t lc[10];      // [level] log2 of the columns of an image
     bool cluster;        // the grid is one cluster; offsets of what its CTAs keep in shared memory for it (GrowArgs)
     int o_x, o_sum, o_cnt, o_best, o_hist, fo;
@@ -269,7 +269,7 @@ static inline bool evb_acc_direct(const evb_handle *h) { return h->world == 1; }
 // word whether any slot has something (the root's only slot says so itself)
 __host__ __device__ static inline size_t evb_low_slot(int level) { return (size_t)1 << (level - 1); }
 __host__ __device__ static inline size_t evb_low_any(int level) { return ((size_t)1 << level) - 1; }
-static inline double evb_hg_low_unit(const evb_handle *h) { return 1.0 / (double)(1ull << (2 * h->hgeo.hb + 2)); } // units of hlow_q in those of hsum_q
+static inline double evb_hg_low_unit(int hb) { return 1.0 / (double)(1ull << (2 * hb + 2)); } // units of hlow_q (g_low) in those of hsum_q (g_sum)
 // evb_histq2.cu
 bool evb_q2_wanted(const evb_handle *h);
 int32_t evb_q2_configure(evb_handle *h);

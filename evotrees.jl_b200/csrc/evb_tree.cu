@@ -1272,7 +1272,7 @@ int32_t evb_launch_scan(evb_handle *h, int level) {
     a.elide_h = h->Ce != h->C ? 1 : 0;
     const bool direct = evb_acc_direct(h);
     a.qsum = direct ? h->hsum_q : nullptr; a.qcnt = direct ? h->hcnt_q : nullptr; a.qinv = h->d_qinv; a.SC = h->SC;
-    a.qlow = direct ? h->hlow_q : nullptr; a.low = h->low + evb_low_slot(level); a.low_unit = evb_hg_low_unit(h);
+    a.qlow = direct ? h->hlow_q : nullptr; a.low = h->low + evb_low_slot(level); a.low_unit = evb_hg_low_unit(h->hgeo.hb);
     a.nq = h->nq; a.unit_w = h->unit_w ? 1 : 0;
     const bool fused = h->world == 1 && !h->obl_gain;
     a.gmax = evb_gmax(h, false); a.ng = h->ng;
