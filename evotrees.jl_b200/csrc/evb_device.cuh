@@ -72,11 +72,12 @@ __device__ __forceinline__ uint32_t arrive(uint32_t *count) {
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(count) : "memory");
     return v;
 }
-// a / b for a >= 0 and b >= DBL_EPSILON, rounded to nearest: the quotient by a reciprocal from Newton's iteration, corrected by its exact
-// remainder (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).
-// Equal to the division in 6.4 G random pairs; a below 1e-270, whose remainder underflows, may be off by the last bit of a quotient
-// below 1e-254.  The division of the language checks its range with a branch of its own, so that quotients are worked out one after the
-// other (four: 521 clocks, 130 each); these overlap.
+// a / b for operands that quot_ok lets through: the quotient by a reciprocal from Newton's iteration, corrected by its exact remainder
+// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  The reciprocal is
+// within 0.5 + 2^-20 units in its last place, so the quotient is within 0.5 + 2^-50 of its own: it can differ from the division, in the last bit,
+// only where a / b lies that close to the middle of two numbers.  In tests/test_quotients_gpu.py it never does, neither in random pairs nor in
+// those that lie closest.  The division of the language checks its range with a branch of its own, so that quotients are worked out one
+// after the other (four: 521 clocks, 130 each); these overlap.
 __device__ __forceinline__ double quot(double a, double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
@@ -85,7 +86,11 @@ __device__ __forceinline__ double quot(double a, double b) {
     const double q = a * r;
     return fma(fma(-b, q, a), r, q);
 }
-__device__ __forceinline__ bool quot_ok(double a, double b) { return a < 1e290 && b < 1e290; } // neither infinite nor a NaN
+// a zero or 2^-600 <= a < 2^600, DBL_EPSILON <= b < 2^300: quotient, reciprocal and the last bit of the remainder (2^-104 a) are normal numbers
+__device__ __forceinline__ bool quot_ok(double a, double b) {
+    constexpr uint32_t lo = (1023u - 600u) << 20, hi = (1023u + 600u) << 20, b_hi = (1023u + 300u) << 20;
+    return (a == 0.0 || (uint32_t)__double2hiint(a) - lo < hi - lo) && (uint32_t)__double2hiint(b) < b_hi;
+}
 // both sides of a candidate split (src/split.jl:1)
 __device__ __forceinline__ double terms_gh(double gl, double hl, double wl, double gr, double hr, double wr, double lambda, double L2) {
     const double a = gl * gl, b = fmax(DBL_EPSILON, hl + lambda * wl + L2), c = gr * gr, d = fmax(DBL_EPSILON, hr + lambda * wr + L2);

@@ -858,6 +858,28 @@ struct DevBuf {
     template <typename T> T *as() { return reinterpret_cast<T *>(p); }
 };
 
+// Diagnostic: the quotients of a split scan
+static __global__ void __launch_bounds__(256) k_quotients(const double *a, const double *b, double *q, uint8_t *ok, long long n) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const double x = a[i], y = b[i];
+    ok[i] = quot_ok(x, y) ? 1 : 0;
+    q[i] = quot_ok(x, y) ? quot(x, y) : x / y;
+}
+extern "C" int32_t evb_test_quotients(int32_t device, int64_t n, const double *a, const double *b, double *q, uint8_t *ok) {
+    if (n < 1 || n > (int64_t)1 << 26 || !a || !b || !q || !ok) { evb_set_error("evb_test_quotients: invalid argument"); return EVB_ERR_ARG; }
+    EVB_CHECK(evb_check_device(device));
+    DevBuf d_a, d_b, d_q, d_ok;
+    EVB_CUDA(d_a.alloc((size_t)n * 8)); EVB_CUDA(d_b.alloc((size_t)n * 8)); EVB_CUDA(d_q.alloc((size_t)n * 8)); EVB_CUDA(d_ok.alloc((size_t)n));
+    EVB_CUDA(cudaMemcpy(d_a.p, a, (size_t)n * 8, cudaMemcpyHostToDevice));
+    EVB_CUDA(cudaMemcpy(d_b.p, b, (size_t)n * 8, cudaMemcpyHostToDevice));
+    k_quotients<<<(unsigned)((n + 255) / 256), 256>>>(d_a.as<double>(), d_b.as<double>(), d_q.as<double>(), d_ok.as<uint8_t>(), n);
+    EVB_CUDA(cudaGetLastError());
+    EVB_CUDA(cudaMemcpy(q, d_q.p, (size_t)n * 8, cudaMemcpyDeviceToHost));
+    EVB_CUDA(cudaMemcpy(ok, d_ok.p, (size_t)n, cudaMemcpyDeviceToHost));
+    return EVB_OK;
+}
+
 extern "C" int32_t evb_binarize(int32_t device, const void *x, int32_t dtype, int64_t nobs, int32_t nfeats, const void *edges,
                                 int32_t nedges, uint8_t *x_bin) {
     if (!x || !edges || !x_bin || nobs < 0 || nfeats < 1 || nedges < 1 || nedges > 254 || (dtype != EVB_F32 && dtype != EVB_F64)) {

@@ -265,6 +265,12 @@ EVB_API int32_t evb_test_peer_timeout(evb_handle *h, int32_t max_polls);
  */
 EVB_API int32_t evb_test_grid_timeout(evb_handle *h, int32_t max_polls);
 
+/*
+ * Diagnostic: q[i] = the quotient a[i] / b[i] as a split scan works it out (host arrays); ok[i]: 1 where its own division was used, 0 where
+ * the operands are outside its range and the language's was.
+ */
+EVB_API int32_t evb_test_quotients(int32_t device, int64_t n, const double *a, const double *b, double *q, uint8_t *ok);
+
 /* Switches the per-kernel CUDA-event timing of EVB_FLAG_TIMING on or off (timed trees run without graphs); with it
  * on, every kernel class is also an NVTX range ("evb:hist", "evb:scan", ...). */
 EVB_API int32_t evb_set_timing(evb_handle *h, int32_t on);
