@@ -888,6 +888,20 @@ int32_t launch_k(const PredPlan &p, PredArgs &a, uint32_t *xw, cudaStream_t st) 
     return launch_t<64, T>(p, a, xw, st);
 }
 
+// Rows of a chunk, of in_row bytes going up and out_row coming back each.
+// Big enough that a chunk's fixed costs (about 15 us of launches) vanish in its transfer, small enough that the
+// first transfer and the last kernel, which nothing overlaps with, do not show; three of them stay in the host's L3.  10M x 50
+// floats, on a slow box: 4 MB 73 ms, 8 MB 56, 12 and 16 MB 47, 24 MB 46; 500k x 100: 6.5, 4.4, 4.05, 4.1, 4.8.
+int64_t chunk_rows(int64_t nobs, size_t in_row, size_t out_row) {
+    const size_t total = (size_t)nobs * (in_row + out_row);
+    size_t cbytes = total / 6;
+    cbytes = std::min<size_t>(std::max<size_t>(cbytes, (size_t)1 << 20), (size_t)12 << 20);
+    // Whole CTAs of the kernels where that many rows fit; wide rows: as many as fit, so that no slot pins more than 12 MB (or one row).
+    int64_t chunk = (int64_t)std::max<size_t>(1, cbytes / (in_row + out_row));
+    if (chunk > 32) chunk -= chunk % (chunk >= 1024 ? 1024 : 32);
+    return std::min<int64_t>(chunk, nobs);
+}
+
 // x: host rows (x_type 0 float, 2 double, -1 bins); out / leaf_idx: host.  `check`: compare the model's sources while the
 // GPU works and return EVB_ERR_STALE when they changed.
 int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, int row_major, int64_t nobs, int apply_link, float *out,
@@ -904,16 +918,7 @@ int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, 
     }
     const size_t es = x_type < 0 ? 1 : x_type == EVB_F64 ? 8 : 4;
     const size_t in_row = es * m.nfeats, out_row = 4 * ((size_t)m.K + (leaf_idx ? ntrees : 0));
-    // Chunks: big enough that a chunk's fixed costs (about 15 us of launches) vanish in its transfer, small enough that the
-    // first transfer and the last kernel, which nothing overlaps with, do not show; three of them stay in the host's L3.  10M x 50
-    // floats, on a slow box: 4 MB 73 ms, 8 MB 56, 12 and 16 MB 47, 24 MB 46; 500k x 100: 6.5, 4.4, 4.05, 4.1, 4.8.
-    const size_t total = (size_t)nobs * (in_row + out_row);
-    size_t cbytes = total / 6;
-    cbytes = std::min<size_t>(std::max<size_t>(cbytes, (size_t)1 << 20), (size_t)12 << 20);
-    // Whole CTAs of the kernels where that many rows fit; wide rows: as many as fit, so that no slot pins more than 12 MB (or one row).
-    int64_t chunk = (int64_t)std::max<size_t>(1, cbytes / (in_row + out_row));
-    if (chunk > 32) chunk -= chunk % (chunk >= 1024 ? 1024 : 32);
-    chunk = std::min<int64_t>(chunk, nobs);
+    const int64_t chunk = chunk_rows(nobs, in_row, out_row);
     // one row or a few: the kernel reads them from pinned memory itself
     const bool zero_copy = (size_t)nobs * in_row <= (size_t)16 * 1024;
     PredArgs a;
@@ -996,6 +1001,19 @@ extern "C" int32_t evb_model_predict(const evb_model *m, int32_t ntrees, const v
     EVB_CUDA(cudaSetDevice(m->device));
     try { return predict_rows(*m, ntrees, x, x_dtype, x_row_major, nobs, apply_link, out, leaf_idx, kernel_ms, true); }
     catch (const std::bad_alloc &) { return no_host_memory(); }
+}
+
+extern "C" int32_t evb_test_predict_plan(const evb_model *m, int32_t x_dtype, int64_t nobs, int32_t leaf_trees, int64_t launches[5]) {
+    if (!m || nobs < 1 || leaf_trees < 0 || leaf_trees > m->ntrees || !launches || (x_dtype != -1 && x_dtype != EVB_F32 && x_dtype != EVB_F64)) {
+        evb_set_error("evb_test_predict_plan: invalid argument");
+        return EVB_ERR_ARG;
+    }
+    int sms = 0;
+    EVB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));
+    for (int k = 0; k < 5; ++k) launches[k] = 0;
+    const int64_t chunk = chunk_rows(nobs, (size_t)(x_dtype < 0 ? 1 : x_dtype == EVB_F64 ? 8 : 4) * m->nfeats, 4 * ((size_t)m->K + leaf_trees));
+    for (int64_t r0 = 0; r0 < nobs; r0 += chunk) launches[plan_kernel(*m, (int)std::min(chunk, nobs - r0), r0 + chunk < nobs, sms).kind] += 1;
+    return EVB_OK;
 }
 
 // one call with trees that are packed for it: evb_predict (bins) and evb_predict_x (raw features)

@@ -338,6 +338,12 @@ EVB_API int32_t evb_model_create(evb_model **out, int32_t device, int32_t loss, 
                                  const uint8_t *feattypes);
 EVB_API int32_t evb_model_predict(const evb_model *m, int32_t ntrees, const void *x, int32_t x_dtype, int32_t x_row_major, int64_t nobs,
                                   int32_t apply_link, float *out, uint32_t *leaf_idx, double *kernel_ms);
+/*
+ * Diagnostic: how often evb_model_predict launches each of its kernels for nobs rows (leaf_trees: trees whose leaf numbers are asked for;
+ * x_dtype -1: evb_predict with bins):
+ * launches[0] a CTA per row, [1] 32 rows, trees through L1, [2] row groups, trees in shared memory, [3] a thread per row, [4] wide rows.
+ */
+EVB_API int32_t evb_test_predict_plan(const evb_model *m, int32_t x_dtype, int64_t nobs, int32_t leaf_trees, int64_t launches[5]);
 EVB_API void evb_model_destroy(evb_model *m);
 
 /*

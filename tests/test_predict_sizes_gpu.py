@@ -1,6 +1,6 @@
-"""`m(x)` at the sizes where the choice of the inference kernel changes (one CTA per row, 32 rows per CTA, staged trees, rows
-wider than shared memory) and where chunks of rows end, against a walk over the trees in numpy; and a packed model after its
-trees have changed."""
+"""`m(x)` at the sizes where the choice of the inference kernel changes (one CTA per row, row groups beside staged trees, 32 rows per CTA, a
+thread per row, rows wider than shared memory; `test_every_kernel` asks which one a call runs) and where chunks of rows end, against a
+walk over the trees in numpy; and a packed model after its trees have changed."""
 import numpy as np
 import pytest
 
@@ -56,6 +56,52 @@ def test_predict_at_the_edges_of_the_kernel_choice(pkg, rows, nfeats, depth, ntr
     want, leaves = _walk(m, x)
     np.testing.assert_allclose(pkg.predict(m, x).reshape(want.shape), want, rtol=1e-5, atol=1e-6)
     assert np.array_equal(pkg.predict_leaf_idx(m, x), leaves)
+
+
+ONE, MID, TILES, STAGED, WIDE = range(5)
+
+
+# Trees: full ones, paths that end anywhere, one bias tree.  Rows: what a kernel takes least, a remainder of its CTAs, several chunks.
+@pytest.mark.parametrize("kernel,rows,nfeats,depth,ntrees,K,nbins", [
+    (ONE, 592, 9, 6, 30, 1, 64), (TILES, 593, 9, 6, 30, 1, 64), (TILES, 20_011, 28, 8, 9, 5, 64),
+    (MID, 593, 5, 15, 4, 1, 64), (MID, 700, 30, 11, 3, 64, 33), (MID, 5_003, 7, 14, 6, 3, 255), (MID, 1_000, 12, 13, 5, 8, 64), (MID, 9_001, 100, 15, 3, 1, 64),
+    (STAGED, 400_003, 4, 7, 12, 1, 64), (STAGED, 420_011, 3, 6, 9, 5, 255), (STAGED, 500_009, 3, 5, 5, 9, 16), (STAGED, 500_017, 2, 9, 30, 2, 33),
+    (WIDE, 100, 65_000, 3, 4, 33, 8), (WIDE, 70, 40_001, 4, 5, 64, 16)])
+@pytest.mark.parametrize("order,dtype", [("C", np.float32), ("F", np.float32), ("F", np.float64)])
+def test_every_kernel(pkg, kernel, rows, nfeats, depth, ntrees, K, nbins, order, dtype):
+    import ctypes as C
+    from evotrees_b200 import _lib
+    m = _model(pkg, nfeats, depth, ntrees, K, nbins, "mlogloss" if K > 2 else "mse", rows)
+    for t in m.trees[1:]:                                                     # all paths of every other tree are full ones
+        if depth > 2 and (t.split[0] == 0 or t is m.trees[-1]):
+            nn = t.feat.size
+            t.split[: nn // 2] = 1
+            t.feat[: nn // 2] = np.maximum(t.feat[: nn // 2], 1)
+            t.cond_bin[: nn // 2] = np.maximum(t.cond_bin[: nn // 2], 1)
+    x = np.asarray(np.random.default_rng(rows).normal(size=(rows, nfeats)), dtype=dtype, order=order)
+    got, ids = pkg.predict(m, x), pkg.predict_leaf_idx(m, x)
+    n = (C.c_int64 * 5)()
+    _lib.check(_lib.lib().evb_test_predict_plan(m._dev.handle, C.c_int32(0 if dtype == np.float32 else 2), C.c_int64(rows), C.c_int32(0), n))
+    assert n[kernel] > 0, list(n)
+    want, leaves = _walk(m, x)
+    # float32 sums of up to 40 values of size 0.1 in the same order, a power and a division of the link behind them
+    np.testing.assert_allclose(got.reshape(want.shape), want, rtol=1e-5, atol=1e-6)
+    assert np.array_equal(ids, leaves)
+
+
+@pytest.mark.parametrize("K", [1, 3])
+def test_wide_rows_of_bins(pkg, K):
+    """Rows of 7 000 bins: too wide for the kernels that keep a row in shared memory"""
+    import ctypes as C
+    from evotrees_b200 import _lib
+    m = _model(pkg, 7_000, 6, 8, K, 16, "mlogloss" if K > 2 else "mse", K)
+    x = np.random.default_rng(K).normal(size=(4_000, 7_000)).astype(np.float32)
+    pkg.predict(m, x[:1])                    # the model is on the device
+    n = (C.c_int64 * 5)()
+    _lib.check(_lib.lib().evb_test_predict_plan(m._dev.handle, C.c_int32(-1), C.c_int64(4_000), C.c_int32(0), n))
+    assert n[WIDE] > 0, list(n)
+    xb = np.asfortranarray(np.stack([1 + np.searchsorted(m.info["edges"][j].astype(np.float32), x[:, j], side="left") for j in range(7_000)], axis=1).astype(np.uint8))
+    np.testing.assert_allclose(pkg.predict_binned(m, xb).reshape(4_000, K), _walk(m, x)[0], rtol=1e-5, atol=1e-6)
 
 
 def test_packed_model_notices_changes(pkg):
