@@ -529,20 +529,48 @@ struct PackJob {
     const void *const *src;
     const int32_t *nodes;
     const uint8_t *feattypes;
+    bool categories;            // some feature is not numeric
     unsigned char *snap;
     std::atomic<long long> bad; // tree and node of a test that cannot be: (tree << 32 | node) + 1
 };
-template <int K>
-void pack_leaves(float *leaf, const int *at, int n, const char *pred, int KR) { // K 0: KR outputs
-    static const float none[64] = {};
-    const size_t bytes = (size_t)(K ? K : KR) * 4;
-    for (int l = 0; l < n; ++l) memcpy(leaf + (size_t)l * (K ? K : KR), at[l] >= 0 ? pred + (size_t)at[l] * bytes : reinterpret_cast<const char *>(none), bytes);
+// last of the nodes [b, e) that has a test; -1: none
+int deepest_split(const uint8_t *split, int b, int e) {
+    while (e - b >= 8) {
+        uint64_t v;
+        memcpy(&v, split + e - 8, 8);
+        if (v) break;
+        e -= 8;
+    }
+    while (e > b && split[e - 1] == 0) --e;
+    return e > b ? e - 1 : -1;
+}
+// A node of the complete tree is the tree's own node of the same number where a path comes there: `live` says whether one does.  Nothing branches on
+// what a node holds (mispredicted ones cost more than the rest).  NUM: no categories.  Returns whether a test is of a feature that is none.
+template <bool NUM>
+bool pack_nodes(uint32_t *tr, int n, const unsigned char *feat, const uint8_t *bin, const uint8_t *split, const uint8_t *numeric, uint64_t nfeats, uint32_t *live) {
+    uint32_t bad = 0u;
+    for (int i = 0; i < n; ++i) {
+        int64_t f;
+        memcpy(&f, feat + (size_t)i * 8, 8); // (at any address)
+        const uint64_t g = (uint64_t)(f - 1);
+        const uint32_t s = split[i] != 0 ? 1u : 0u, known = g < nfeats ? 1u : 0u, q = known ? (uint32_t)g : 0u;
+        bad |= s & ~known;
+        uint32_t w = q | (uint32_t)bin[i] << (NUM || numeric[q] ? 16 : 24);
+        w |= (uint32_t)(w == STOP) << 24; // bin 255 of feature 0: all rows go left as well, but the path does not end
+        const uint32_t l = live[i] & s;
+        tr[i] = l ? w : STOP;
+        live[2 * i + 1] = live[2 * i + 2] = l;
+    }
+    return bad != 0u;
 }
 void pack_trees(void *ctx, char *dst, size_t first, size_t count) {
     PackJob &j = *static_cast<PackJob *>(ctx);
     const evb_model &m = *j.m;
     uint32_t *tr = reinterpret_cast<uint32_t *>(dst);
-    std::vector<int> at;
+    const int last = (1 << m.levels) - 1; // first node of the last level
+    const size_t row = (size_t)m.K * 4;
+    std::vector<uint32_t> live((size_t)2 * last + 1);
+    std::vector<int> ends((size_t)last + 1);
     for (size_t t = first; t < first + count; ++t, tr += m.tw) {
         const void *part[4];
         const int nn = j.nodes[t];
@@ -555,57 +583,42 @@ void pack_trees(void *ctx, char *dst, size_t first, size_t count) {
             part[q] = j.snap + o;
             o += n;
         }
-        const unsigned char *feat = static_cast<const unsigned char *>(part[0]); // 8-byte integers, at any address in the snapshot
+        const unsigned char *feat = static_cast<const unsigned char *>(part[0]);
         const uint8_t *bin = static_cast<const uint8_t *>(part[1]), *split = static_cast<const uint8_t *>(part[2]);
         const char *pred = static_cast<const char *>(part[3]); // floats, at any address as well
-        float *leaf = reinterpret_cast<float *>(tr + m.ni);
-        const int last = (1 << m.levels) - 1; // first node of the last level
-        at.resize((size_t)2 * last + 1);      // node of the tree that a node of the complete one stands for; -1: no row comes there
-        // (No branch on what a node holds: mispredicted ones and a memcpy call a leaf were two thirds of the time.)
-        bool bad = false;
-        for (int i = 0; i < nn; ++i) {
-            int64_t f;
-            memcpy(&f, feat + (size_t)i * 8, 8);
-            bad |= (split[i] != 0) & ((uint64_t)(f - 1) >= (uint64_t)m.nfeats || 2 * i + 2 >= nn);
-        }
+        const int inner = std::min(last, std::max(0, (nn - 1) / 2));        // nodes that may test something: their children are nodes of the tree
+        live[0] = nn > 0 ? 1u : 0u;
+        bool bad = deepest_split(split, inner, nn) >= 0;
+        bad |= j.categories ? pack_nodes<false>(tr, inner, feat, bin, split, j.feattypes, (uint64_t)m.nfeats, live.data())
+                            : pack_nodes<true>(tr, inner, feat, bin, split, nullptr, (uint64_t)m.nfeats, live.data());
         if (bad) {
-            for (int i = 0; i < nn; ++i) {
+            int i = 0;
+            for (; i < nn; ++i) {
                 int64_t f;
                 memcpy(&f, feat + (size_t)i * 8, 8);
-                if (!split[i] || (f >= 1 && f <= m.nfeats && 2 * i + 2 < nn)) continue;
-                long long none = 0;
-                j.bad.compare_exchange_strong(none, ((long long)t << 32 | i) + 1);
-                break;
+                if (split[i] && (f < 1 || f > m.nfeats || i >= inner)) break;
             }
+            long long none = 0;
+            j.bad.compare_exchange_strong(none, ((long long)t << 32 | i) + 1);
             continue;
         }
-        at[0] = 0;
-        for (int i = 0; i < last; ++i) {
-            const int o = at[i], from = o < 0 ? 0 : o;
-            const bool s = (o >= 0) & (split[from] != 0);
-            int64_t f;
-            memcpy(&f, feat + (size_t)from * 8, 8);
-            f = s ? f - 1 : 0;
-            const int shift = !j.feattypes || j.feattypes[f] ? 16 : 24;
-            uint32_t w = (uint32_t)f | (uint32_t)bin[from] << shift;
-            w |= (uint32_t)(w == STOP) << 24; // bin 255 of feature 0: all rows go left as well, but the path does not end
-            tr[i] = s ? w : STOP;
-            at[2 * i + 1] = s ? 2 * o + 1 : o;
-            at[2 * i + 2] = s ? 2 * o + 2 : -1;
-        }
+        for (int i = inner; i < last; ++i) { tr[i] = STOP; live[2 * i + 1] = live[2 * i + 2] = 0u; } // (a tree of fewer levels)
         for (int i = last; i < m.ni; ++i) tr[i] = 0u;
-        switch (m.K) {
-            case 1: pack_leaves<1>(leaf, at.data() + last, last + 1, pred, 1); break;
-            case 2: pack_leaves<2>(leaf, at.data() + last, last + 1, pred, 2); break;
-            case 3: pack_leaves<3>(leaf, at.data() + last, last + 1, pred, 3); break;
-            case 4: pack_leaves<4>(leaf, at.data() + last, last + 1, pred, 4); break;
-            case 5: pack_leaves<5>(leaf, at.data() + last, last + 1, pred, 5); break;
-            case 6: pack_leaves<6>(leaf, at.data() + last, last + 1, pred, 6); break;
-            case 7: pack_leaves<7>(leaf, at.data() + last, last + 1, pred, 7); break;
-            case 8: pack_leaves<8>(leaf, at.data() + last, last + 1, pred, 8); break;
-            default: pack_leaves<0>(leaf, at.data() + last, last + 1, pred, m.K);
+        // Values of the last level lie together in the tree too; those of paths that end above it go to the leftmost leaf below.  (Leaves
+        // that no path comes to hold anything.)
+        char *leaf = reinterpret_cast<char *>(tr + m.ni);
+        const size_t have = (size_t)std::max(0, std::min(nn - last, last + 1)) * row;
+        memcpy(leaf, pred + (have ? (size_t)last * row : 0), have);
+        memset(leaf + have, 0, (size_t)(m.tw - m.ni) * 4 - have);
+        int full = 0;
+        for (int i = last; i <= 2 * last; ++i) full += (int)live[i];
+        if (full == last + 1) continue;
+        int n = 0;
+        for (int i = 0; i < last; ++i) { ends[n] = i; n += (int)(live[i] & (tr[i] == STOP ? 1u : 0u)); }
+        for (int e = 0; e < n; ++e) {
+            const int i = ends[e], at = ((i + 1) << (m.levels - (31 - __builtin_clz((unsigned)i + 1u)))) - (last + 1);
+            memcpy(leaf + (size_t)at * row, pred + (size_t)i * row, row);
         }
-        for (int e = (last + 1) * m.K; e < m.tw - m.ni; ++e) leaf[e] = 0.0f;
     }
 }
 
@@ -624,7 +637,8 @@ int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32
     m->tw = m->ni + (((K << m->levels) + 3) & ~3);
     const size_t unit = (size_t)m->tw * 4, tbytes = (size_t)ntrees * unit, ne = (size_t)m->nedges * nfeats;
     const size_t o64 = (tbytes + 15) & ~(size_t)15, o32 = o64 + ne * 8, total = o32 + ne * 4 + 16;
-    PackJob job{m, src, nodes, feattypes, nullptr, {0}};
+    const bool categories = feattypes && memchr(feattypes, 0, (size_t)nfeats) != nullptr;
+    PackJob job{m, src, nodes, feattypes, categories, nullptr, {0}};
     if (snapshot) {
         m->src.assign(src, src + (size_t)ntrees * 4);
         m->nodes.assign(nodes, nodes + ntrees);

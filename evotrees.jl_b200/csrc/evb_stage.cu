@@ -226,7 +226,7 @@ int32_t evb_h2d_made(void *dst_dev, size_t unit, size_t count, void (*fill)(void
         if (r.used[b]) EVB_CUDA(cudaEventSynchronize(r.ev[b]));
         j.buf = static_cast<char *>(r.buf[b]); j.first = u;
         evb_parallel([](void *c, size_t b0, size_t e0) { Job &q = *static_cast<Job *>(c); q.fill(q.ctx, q.buf + b0 * q.unit, q.first + b0, e0 - b0); }, &j, n,
-                     std::max<size_t>(1, ((size_t)64 << 10) / unit));
+                     std::max<size_t>(1, ((size_t)32 << 10) / unit));
         EVB_CUDA(cudaMemcpyAsync(static_cast<char *>(dst_dev) + u * unit, r.buf[b], n * unit, cudaMemcpyHostToDevice, st));
         EVB_CUDA(cudaEventRecord(r.ev[b], st));
         r.used[b] = true;
