@@ -628,11 +628,16 @@ void pack_trees(void *ctx, char *dst, size_t first, size_t count) {
 int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32_t *nodes, const void *edges, int e_dtype, int nedges,
                    int nfeats, const uint8_t *feattypes, bool snapshot) {
     const int K = m->K;
-    int nn = 1;
-    for (int t = 0; t < ntrees; ++t) nn = std::max(nn, (int)nodes[t]);
+    // Levels: down to the last test of any tree, whatever room its arrays have.  200 trees of depth 11 whose paths end at depth 4 take 4 steps
+    // a row, not 10.
+    int deepest = -1;
+    for (int t = 0; t < ntrees; ++t) {
+        const int i = deepest_split(static_cast<const uint8_t *>(src[t * 4 + 2]), std::min((int)nodes[t], deepest + 1), std::max(0, (nodes[t] - 1) / 2));
+        deepest = std::max(deepest, i);
+    }
     m->ntrees = ntrees; m->nfeats = nfeats; m->nedges = edges ? nedges : 0;
     m->levels = 0;
-    while ((2 << m->levels) - 1 < nn) ++m->levels;
+    while ((1 << m->levels) <= deepest + 1) ++m->levels;
     m->ni = std::max(4, 1 << m->levels);
     m->tw = m->ni + (((K << m->levels) + 3) & ~3);
     const size_t unit = (size_t)m->tw * 4, tbytes = (size_t)ntrees * unit, ne = (size_t)m->nedges * nfeats;

@@ -89,6 +89,30 @@ def test_every_kernel(pkg, kernel, rows, nfeats, depth, ntrees, K, nbins, order,
     assert np.array_equal(ids, leaves)
 
 
+def test_walks_end_at_the_deepest_test(pkg):
+    """Arrays of depth 15 whose tests end at level 4: such a model is packed, and walked, as one of five levels; a test further down is seen
+    by the next call."""
+    import ctypes as C
+    from evotrees_b200 import _lib
+    m = _model(pkg, 9, 15, 6, 1, 64, "mse", 4)
+    for t in m.trees[1:]:
+        t.split[15:] = 0
+        t.split[:15] = 1
+        t.feat[:15], t.cond_bin[:15] = np.maximum(t.feat[:15], 1), np.maximum(t.cond_bin[:15], 1)
+    x = np.random.default_rng(3).normal(size=(2_000, 9))
+    n = (C.c_int64 * 5)()
+    for kernel, node in ((TILES, None), (TILES, 20), (MID, 16_000)):
+        if node is not None:
+            while node > 0:                                                   # a path down to it
+                m.trees[3].split[node], m.trees[3].feat[node], m.trees[3].cond_bin[node] = 1, 2, 30
+                node = (node - 1) // 2
+        want, leaves = _walk(m, x)
+        np.testing.assert_allclose(pkg.predict(m, x), want[:, 0], rtol=1e-5, atol=1e-6)
+        assert np.array_equal(pkg.predict_leaf_idx(m, x), leaves)
+        _lib.check(_lib.lib().evb_test_predict_plan(m._dev.handle, C.c_int32(2), C.c_int64(2_000), C.c_int32(0), n))
+        assert n[kernel] == 1, list(n)
+
+
 @pytest.mark.parametrize("K", [1, 3])
 def test_wide_rows_of_bins(pkg, K):
     """Rows of 7 000 bins: too wide for the kernels that keep a row in shared memory"""
