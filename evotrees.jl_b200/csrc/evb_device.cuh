@@ -73,11 +73,11 @@ __device__ __forceinline__ uint32_t arrive(uint32_t *count) {
     return v;
 }
 // a / b for operands that quot_ok lets through: the quotient by a reciprocal from Newton's iteration, corrected by its exact remainder
-// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  The reciprocal is
-// within 0.5 + 2^-20 units in its last place, so the quotient is within 0.5 + 2^-50 of its own: it can differ from the division, in the last bit,
-// only where a / b lies that close to the middle of two numbers.  In tests/test_quotients_gpu.py it never does, neither in random pairs nor in
-// those that lie closest.  The division of the language checks its range with a branch of its own, so that quotients are worked out one
-// after the other (four: 521 clocks, 130 each); these overlap.
+// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  It is the division's
+// unless b's bits are all ones, the method's known exception: a power of two by such a number is one unit in the last place too small.
+// tests/test_quotients_gpu.py: random pairs, those whose quotients lie closest to the middle of two numbers, the ends of the range.  The division
+// of the language checks its range with a branch of its own, so that quotients are worked out one after the other (four: 521 clocks, 130
+// each); these overlap.
 __device__ __forceinline__ double quot(double a, double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
