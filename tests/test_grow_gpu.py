@@ -74,26 +74,39 @@ def test_samples_of_rows_and_columns(pkg, loss, weighted):
     _same(pkg, params, x, y, w, rounds=8, samples=[(m, j) for j in js for m in (mask, None)])
 
 
-# rows, columns, loss, weights, numbers of sampled columns of the trees one after the other; row ranges of the kernel (148 SMs)
-COLUMN_COUNTS = [(2_000, 400, "mse", False, (400, 200, 400, 100)),       # 1, 2, 1, 3 over the grid
-                 (5_000, 300, "gamma", True, (300, 100, 300, 150)),      # 1, 5, 1, 2 or more
-                 (2_500, 64, "gamma", True, (64, 32, 64, 16)),           # one cluster: 1, 2, 1, 4
-                 (900, 100, "logloss", True, (100, 30, 100, 7))]         # the grid's one range, then a cluster
+# rows, columns, depth, loss, weights, numbers of sampled columns of the trees one after the other
+COLUMN_COUNTS = [(2_000, 400, 5, "mse", False, (400, 200, 400, 100)), (5_000, 300, 5, "gamma", True, (300, 100, 300, 150)), (2_500, 64, 5, "gamma", True, (64, 32, 64, 16)),
+                 (900, 100, 5, "logloss", True, (100, 30, 100, 7)), (1_100, 60, 4, "poisson", True, (60, 20, 60, 5, 33)), (900, 33, 6, "gamma", False, (33, 4, 30, 9))]
 
 
-@pytest.mark.parametrize("n,F,loss,weighted,counts", COLUMN_COUNTS)
-def test_another_number_of_columns_in_every_tree(pkg, n, F, loss, weighted, counts):
-    """One range of rows stores its sums, several add theirs up: what a tree leaves behind must not be found by the next.  Gradients over many
-    orders of magnitude, so that the second set of sums is used too."""
+@pytest.mark.parametrize("n,F,depth,loss,weighted,counts", COLUMN_COUNTS)
+def test_another_number_of_columns_in_every_tree(pkg, n, F, depth, loss, weighted, counts):
+    """One range of rows stores its sums, several add theirs up: what a tree leaves behind must not be found by the next, whose geometry is another.
+    Every tree is that of a handle which starts from the same predictions.  Gradients over many orders of magnitude, so that the second set of sums
+    is used too (the level kernels round such sums elsewhere: they are compared where all fit a double)."""
+    from evotrees_b200 import _lib
     x, y, w = _data(n, F, 64, loss, 11, weighted)
     rng = np.random.default_rng(n)
+    js = [(np.sort(rng.permutation(F)[:k]) + 1).astype(np.uint32) for k in counts]
+    params = pkg.EvoTreeRegressor(loss=loss, nrounds=1, max_depth=depth, nbins=64, eta=0.3)
+    _same(pkg, params, x, y, None, rounds=2 * len(js), samples=[(None, j) for j in js])
     if loss == "gamma":
         y = np.exp(4.0 * rng.normal(size=n)).astype(np.float32)
     if w is not None:
         w = np.exp(4.0 * rng.normal(size=n)).astype(np.float32)
-    js = [(np.sort(rng.permutation(F)[:k]) + 1).astype(np.uint32) for k in counts]
-    params = pkg.EvoTreeRegressor(loss=loss, nrounds=1, max_depth=5, nbins=64, eta=0.3)
-    _same(pkg, params, x, y, w, rounds=2 * len(js), samples=[(None, j) for j in js])
+    a = _cache(pkg, params, x, y, w, _lib.FLAG_KEEP_ALL_HIST)
+    try:
+        for r in range(2 * len(js)):
+            j = js[r % len(js)]
+            b = _cache(pkg, params, x, y, w, _lib.FLAG_KEEP_ALL_HIST, pred0=a.pred())
+            s, t = (pkg.grow_tree(c, params, None, j, update_grads=True) for c in (a, b))
+            same = [np.array_equal(getattr(s, k), getattr(t, k)) for k in ("feat", "cond_bin", "split", "w", "gain", "pred")] + [np.array_equal(a.node_sums(), b.node_sums())]
+            same += [np.array_equal(a.hist(node, j.size, 64), b.hist(node, j.size, 64)) for node in range(1, 2 ** (depth - 1)) if node == 1 or s.split[node // 2 - 1]]
+            b.close()
+            assert all(same), (r, same)
+        assert a.timings()["launches"]["scan"] == 0
+    finally:
+        a.close()
 
 
 def test_categories_and_constraints(pkg):
