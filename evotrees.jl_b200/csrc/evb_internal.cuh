@@ -328,7 +328,7 @@ void evb_copy_packed(void *packed, const void *strided, size_t seg, size_t strid
 int32_t evb_d2h_staged(void *dst_host, const void *src_dev, size_t bytes, cudaStream_t st);
 int32_t evb_h2d_staged(void *dst_dev, const void *src_host, size_t bytes, cudaStream_t st, bool drain = true);
 size_t evb_stage_bytes();
-int32_t evb_h2d_made(void *dst_dev, size_t unit, size_t count, void (*fill)(void *, char *, size_t, size_t), void *ctx, cudaStream_t st);
+int32_t evb_h2d_made(void *dst_dev, size_t unit, size_t count, size_t piece, void (*fill)(void *, char *, size_t, size_t), void *ctx, cudaStream_t st);
 int32_t evb_h2d_staged_strided(void *dst_dev, const void *src_host, size_t seg_bytes, size_t nseg, size_t stride, cudaStream_t st, bool drain = true);
 
 // timing helpers (evb_api.cu)

@@ -466,6 +466,10 @@ __global__ void __launch_bounds__(256) k_predict_wide(PredArgs a, const uint32_t
 } // namespace
 
 // ================================================================================================= models
+static int32_t no_host_memory() {
+    evb_set_error("out of host memory");
+    return EVB_ERR_ARG;
+}
 struct evb_model {
     int device = 0, loss = 0, K = 1, ntrees = 0, ni = 4, tw = 8, levels = 0, nfeats = 0, nedges = 0;
     void *block = nullptr;            // trees, then the edges as double and as float
@@ -531,7 +535,7 @@ struct PackJob {
     const uint8_t *feattypes;
     bool categories;            // some feature is not numeric
     unsigned char *snap;
-    std::atomic<long long> bad; // tree and node of a test that cannot be: (tree << 32 | node) + 1
+    std::atomic<long long> bad; // tree and node of a test that cannot be: (tree << 32 | node) + 1; -1: out of memory
 };
 // last of the nodes [b, e) that has a test; -1: none
 int deepest_split(const uint8_t *split, int b, int e) {
@@ -563,8 +567,7 @@ bool pack_nodes(uint32_t *tr, int n, const unsigned char *feat, const uint8_t *b
     }
     return bad != 0u;
 }
-void pack_trees(void *ctx, char *dst, size_t first, size_t count) {
-    PackJob &j = *static_cast<PackJob *>(ctx);
+void pack_trees_of(PackJob &j, char *dst, size_t first, size_t count) {
     const evb_model &m = *j.m;
     uint32_t *tr = reinterpret_cast<uint32_t *>(dst);
     const int last = (1 << m.levels) - 1; // first node of the last level
@@ -622,6 +625,12 @@ void pack_trees(void *ctx, char *dst, size_t first, size_t count) {
     }
 }
 
+void pack_trees(void *ctx, char *dst, size_t first, size_t count) { // (on any thread)
+    PackJob &j = *static_cast<PackJob *>(ctx);
+    try { pack_trees_of(j, dst, first, count); }
+    catch (const std::bad_alloc &) { j.bad.store(-1); }
+}
+
 // src: [ntrees][4] pointers; packs, uploads and keeps the snapshot.  edges may be null (binned input only).
 // All staging threads pack, straight into pinned buffers that are copied meanwhile; one thread into a zeroed image, its upload from
 // pageable memory and a second pass for the snapshot took 2.4 ms at 200 trees of depth 11 and 39 at 500 of depth 13.
@@ -672,9 +681,17 @@ int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32
     cudaStream_t st = nullptr;
     EVB_CUDA(evb_stream_get(&st));
     int32_t rc = EVB_OK;
-    if (piped) rc = evb_h2d_made(m->block, unit, (size_t)ntrees, pack_trees, &job, st);
-    else pack_trees(&job, reinterpret_cast<char *>(host.data()), 0, (size_t)ntrees);
-    if (rc == EVB_OK && job.bad.load() != 0) {
+    // a thread's piece: trees of 128 KB in the caller's arrays, whatever is left of them when they are packed
+    size_t nodes_all = 0;
+    for (int t = 0; t < ntrees; ++t) nodes_all += (size_t)std::max(nodes[t], 1);
+    const size_t piece = std::max<size_t>(1, ((size_t)128 << 10) * ntrees / std::max<size_t>(1, nodes_all * (10 + (size_t)K * 4)));
+    if (piped) rc = evb_h2d_made(m->block, unit, (size_t)ntrees, piece, pack_trees, &job, st);
+    else {
+        struct Hosted { PackJob *job; char *to; size_t unit; } hj{&job, reinterpret_cast<char *>(host.data()), unit};
+        evb_parallel([](void *c, size_t b, size_t e) { Hosted &q = *static_cast<Hosted *>(c); pack_trees(q.job, q.to + b * q.unit, b, e - b); }, &hj, (size_t)ntrees, piece);
+    }
+    if (rc == EVB_OK && job.bad.load() == -1) rc = no_host_memory();
+    if (rc == EVB_OK && job.bad.load() > 0) {
         const long long at = job.bad.load() - 1;
         evb_set_error("evb_model: node %lld of tree %lld tests a feature that is not one of %d or has no children", (at & 0xffffffffll) + 1, (at >> 32) + 1, nfeats);
         rc = EVB_ERR_ARG;
@@ -700,10 +717,6 @@ extern "C" void evb_model_destroy(evb_model *m) {
     delete m;
 }
 
-static int32_t no_host_memory() {
-    evb_set_error("out of host memory");
-    return EVB_ERR_ARG;
-}
 static int32_t model_args(int32_t loss, int32_t K, int32_t ntrees, int32_t nfeats) {
     if (nfeats < 1 || nfeats > 65535 || ntrees < 0 || K < 1 || K > 64 || loss < 0 || loss > EVB_LOSS_LAST) {
         evb_set_error("evb_predict: invalid argument");

@@ -206,10 +206,10 @@ int32_t evb_h2d_staged_strided(void *dst_dev, const void *src_host, size_t seg_b
 }
 
 // Memory that is made on the way: fill(ctx, buffer, first, count) writes units [first, first + count) of `unit` bytes each to a pinned
-// buffer (all staging threads, a unit is one thread's), which is copied while the next one is filled.  Returns when everything has arrived.
+// buffer (all staging threads, `piece` units at a time), which is copied while the next one is filled.  Returns when everything has arrived.
 // unit <= STAGE_BYTES.
 size_t evb_stage_bytes() { return STAGE_BYTES; }
-int32_t evb_h2d_made(void *dst_dev, size_t unit, size_t count, void (*fill)(void *, char *, size_t, size_t), void *ctx, cudaStream_t st) {
+int32_t evb_h2d_made(void *dst_dev, size_t unit, size_t count, size_t piece, void (*fill)(void *, char *, size_t, size_t), void *ctx, cudaStream_t st) {
     int dev = 0;
     EVB_CUDA(cudaGetDevice(&dev));
     if (unit == 0 || unit > STAGE_BYTES || dev < 0 || dev >= 64) { evb_set_error("evb_h2d_made: invalid argument"); return EVB_ERR_ARG; }
@@ -225,8 +225,7 @@ int32_t evb_h2d_made(void *dst_dev, size_t unit, size_t count, void (*fill)(void
         const size_t n = std::min(per, count - u);
         if (r.used[b]) EVB_CUDA(cudaEventSynchronize(r.ev[b]));
         j.buf = static_cast<char *>(r.buf[b]); j.first = u;
-        evb_parallel([](void *c, size_t b0, size_t e0) { Job &q = *static_cast<Job *>(c); q.fill(q.ctx, q.buf + b0 * q.unit, q.first + b0, e0 - b0); }, &j, n,
-                     std::max<size_t>(1, ((size_t)32 << 10) / unit));
+        evb_parallel([](void *c, size_t b0, size_t e0) { Job &q = *static_cast<Job *>(c); q.fill(q.ctx, q.buf + b0 * q.unit, q.first + b0, e0 - b0); }, &j, n, piece);
         EVB_CUDA(cudaMemcpyAsync(static_cast<char *>(dst_dev) + u * unit, r.buf[b], n * unit, cudaMemcpyHostToDevice, st));
         EVB_CUDA(cudaEventRecord(r.ev[b], st));
         r.used[b] = true;
