@@ -1242,8 +1242,13 @@ size_t evb_grow_sums(const evb_handle *h) { return (size_t)h->maxslots * h->nfea
 size_t evb_grow_cnts(const evb_handle *h) { return (size_t)h->maxslots * h->nfeats * h->B; }
 size_t evb_grow_best(const evb_handle *h) { return (size_t)(1 << std::max(1, h->D - 2)) * h->nfeats * 3; }
 
+// Evaluation rows inside the launch: up to this many a CTA.  Kernels of their own cost 10 us a tree, and have many times the threads of one
+// cluster.  us per tree, inside and in launches of its own: 1503 x 7 (16 CTAs) with 5k rows 45.4 and 52.6, 20k 49.1 and 53.2, 60k 55.4 and 55.2, 300k 98.1 and 57.7;
+// 5000 x 20 (15 CTAs) 10k 57.2 and 63.7, 40k 62.4 and 64.3, 300k 93.4 and 85.7; 100k x 10 (147 CTAs) 100k 63.5 and 73.5, 500k 71.8 and 80.8.
+constexpr int EVAL_ROWS = 3072;
 int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot, bool next_grads) {
     const GrowGeom &g = h->grow;
+    const bool eval_inside = h->ev_n <= (int64_t)EVAL_ROWS * g.NG * g.NR;
     GrowArgs a = {};
     a.xC = h->xC; a.grad = h->grad; a.mask = masked ? h->mask_d : nullptr; a.cond = mask_cond; a.feattypes = h->feattypes_d; a.mono = h->mono_d;
     if (h->F < h->nfeats) {
@@ -1268,9 +1273,11 @@ int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot,
     a.alpha = evb_alpha_set(h);
     if (!masked) {
         a.whole = 1; a.next_grads = next_grads ? 1 : 0; a.pred = h->pred; a.y = h->y; a.nidx = h->nidx;
-        a.pub_src = reinterpret_cast<const uint4 *>(h->plan); a.pub_dst = static_cast<uint4 *>(h->h_tree[slot]); a.pub_n = (int)(h->h_tree_bytes / 16);
-        a.pub_err = (int)(h->d_err - reinterpret_cast<int *>(h->plan));
-        if (h->ev_n > 0) {
+        if (h->ev_n == 0 || eval_inside) { // else the evaluation's own kernels hand the tree over
+            a.pub_src = reinterpret_cast<const uint4 *>(h->plan); a.pub_dst = static_cast<uint4 *>(h->h_tree[slot]); a.pub_n = (int)(h->h_tree_bytes / 16);
+            a.pub_err = (int)(h->d_err - reinterpret_cast<int *>(h->plan));
+        }
+        if (h->ev_n > 0 && eval_inside) {
             a.ev_xT = h->ev_xT; a.ev_y = h->ev_y; a.ev_w = h->ev_w; a.ev_pred = h->ev_pred; a.ev_part = h->ev_part; a.ev_sum = h->d_evsum; a.ev_n = h->ev_n;
             a.ev_RS = h->RS; a.ev_metric = h->ev_metric;
         }
@@ -1279,5 +1286,5 @@ int32_t evb_launch_grow(evb_handle *h, bool masked, uint8_t mask_cond, int slot,
     const cudaError_t e = launch(h, g, &a, nullptr);
     evb_toc(h, EVB_T_HIST);
     EVB_CUDA(e);
-    return EVB_OK;
+    return masked || eval_inside || h->ev_n == 0 ? EVB_OK : evb_launch_eval(h, nullptr, h->h_tree[slot]);
 }

@@ -142,9 +142,10 @@ def test_deeper_than_the_rows_carry(pkg):
         _same(pkg, pkg.EvoTreeRegressor(loss="mse", nrounds=1, max_depth=8, nbins=32, eta=0.3, gamma=gamma, min_weight=mw), x, y, None)
 
 
-@pytest.mark.parametrize("n,ev,F", [(1_503, 501, 7), (30_000, 40_003, 40), (5_000, 1, 3)])
-def test_metric_of_every_tree(pkg, orc, n, ev, F):
-    """Evaluation rows inside the launch: the metric of each tree is that of the model's own predictions"""
+# 16 CTAs to 49 152 rows, 148 to 454 656: inside the tree's launch; more of them in launches of their own
+@pytest.mark.parametrize("n,ev,F,own", [(1_503, 501, 7, False), (30_000, 40_003, 40, False), (5_000, 1, 3, False), (1_503, 49_153, 7, True), (1_503, 300_007, 7, True), (20_000, 460_001, 6, True)])
+def test_metric_of_every_tree(pkg, orc, n, ev, F, own):
+    """Evaluation rows in the tree's launch or behind it: the metric of each tree is that of the model's own predictions"""
     rng = np.random.default_rng(n)
     x, xe = rng.random((n, F)).astype(np.float32), rng.random((ev, F)).astype(np.float32)
     beta = rng.normal(size=F)
@@ -152,7 +153,8 @@ def test_metric_of_every_tree(pkg, orc, n, ev, F):
     we = rng.uniform(0.5, 2.0, ev).astype(np.float32)
     m, cache = pkg.fit(pkg.EvoTreeRegressor(loss="mse", nrounds=12, max_depth=5, nbins=32, eta=0.3, bagging_size=1, early_stopping_rounds=100), x_train=x, y_train=y, x_eval=xe,
                        y_eval=ye, w_eval=we, return_cache=True)
-    assert cache.timings()["launches"]["scan"] == 0
+    launches = cache.timings()["launches"]
+    assert launches["scan"] == 0 and (launches["finalize"] >= 12) == own
     np.testing.assert_allclose(cache.pred(), m(x).reshape(n, 1), rtol=1e-5, atol=1e-6)
     cache.close()
     for i in (0, 1, 5, 12):
