@@ -34,6 +34,7 @@ struct PredArgs {
     int nedges, nfeats, FW; // FW: words of four bins per row
     const uint32_t *trees;
     int ni, tw, levels;     // levels: tests on the longest path of a tree
+    bool early;             // most paths end above the last level (evb_model::early)
     float *out;             // column k of row i at k * out_ld + i
     long long out_ld;
     uint32_t *leaf_idx;     // null, or tree t of row i at t * out_ld + i
@@ -165,11 +166,21 @@ __device__ __forceinline__ void put_row(const PredArgs &a, long long i, const fl
     for (int k = 0; k < KMAX; ++k) if (k < a.K) a.out[(size_t)k * a.out_ld + i] = p[k];
 }
 
-// Leaf (0 .. 2^levels - 1) of a row in one tree; word(w): the row's bins 4 w .. 4 w + 3, node(i): the tree's node i
+// Leaf (0 .. 2^levels - 1) of a row in one tree; word(w): the row's bins 4 w .. 4 w + 3, node(i): the tree's node i.  early: a lane leaves the loop
+// where its path ends (PredArgs::early)
 template <typename N, typename X>
-__device__ __forceinline__ int walk(int levels, N node, X word) {
-    int i = 0;
-    for (int l = 0; l < levels; ++l) {
+__device__ __forceinline__ int walk(int levels, bool early, N node, X word) {
+    int i = 0, l = 0;
+    if (early) {
+        for (; l < levels; ++l) {
+            const uint32_t pk = node(i);
+            if (pk == STOP) break;
+            const uint32_t x = __byte_perm(word((pk & 0xffffu) >> 2), 0u, 0x4440u | (pk & 3u));
+            i = 2 * i + ((x ^ (pk >> 24)) <= ((pk >> 16) & 0xffu) ? 1 : 2);
+        }
+        return ((i + 1) << (levels - l)) - (1 << levels); // the leftmost leaf below
+    }
+    for (; l < levels; ++l) {
         const uint32_t pk = node(i);
         const uint32_t x = __byte_perm(word((pk & 0xffffu) >> 2), 0u, 0x4440u | (pk & 3u));
         i = 2 * i + ((x ^ (pk >> 24)) <= ((pk >> 16) & 0xffu) ? 1 : 2);
@@ -179,15 +190,15 @@ __device__ __forceinline__ int walk(int levels, N node, X word) {
 // the same for the id of the node where the row's path ends (`predict_leaf_idx`): the first that stops, else the leaf itself
 template <typename N, typename X>
 __device__ __forceinline__ int walk_id(int levels, N node, X word, int &leaf) {
-    int i = 0, id = 0;
-    for (int l = 0; l < levels; ++l) {
+    int i = 0, l = 0;
+    for (; l < levels; ++l) {
         const uint32_t pk = node(i);
-        if (id == 0 && pk == STOP) id = i + 1;
+        if (pk == STOP) break;
         const uint32_t x = __byte_perm(word((pk & 0xffffu) >> 2), 0u, 0x4440u | (pk & 3u));
         i = 2 * i + ((x ^ (pk >> 24)) <= ((pk >> 16) & 0xffu) ? 1 : 2);
     }
-    leaf = i + 1 - (1 << levels);
-    return id ? id : i + 1;
+    leaf = ((i + 1) << (levels - l)) - (1 << levels);
+    return i + 1;
 }
 
 // ---------------------------------------------------------------------------------- few rows
@@ -227,7 +238,7 @@ __global__ void __launch_bounds__(ONE_THREADS) k_predict_one(PredArgs a) {
             auto word = [&](uint32_t w) { return s_one[w]; };
             int leaf;
             if (a.leaf_idx) a.leaf_idx[(size_t)t * a.out_ld + i] = (uint32_t)walk_id(a.levels, node, word, leaf);
-            else leaf = walk(a.levels, node, word);
+            else leaf = walk(a.levels, a.early, node, word);
             for (int k = 0; k < K; ++k) s_leaf[tid * K + k] = __uint_as_float(__ldg(tr + a.ni + leaf * K + k));
         }
         __syncthreads();
@@ -278,7 +289,7 @@ __global__ void __launch_bounds__(MID_WARPS * 32) k_predict_mid(PredArgs a, int 
                 for (int l = 0; l < a.levels; ++l) {
                     uint32_t pk[MID_ILP];
 #pragma unroll
-                    for (int u = 0; u < MID_ILP; ++u) pk[u] = __ldg(tr[u] + at[u]);
+                    for (int u = 0; u < MID_ILP; ++u) pk[u] = id[u] == 0 ? __ldg(tr[u] + at[u]) : STOP;
 #pragma unroll
                     for (int u = 0; u < MID_ILP; ++u) {
                         if (id[u] == 0 && pk[u] == STOP) id[u] = at[u] + 1;
@@ -361,7 +372,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, 1) k_predict_tiles(PredArgs a
                 if (a.leaf_idx) {
                     const uint32_t id = (uint32_t)walk_id(a.levels, node, word, leaf);
                     if (act) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = id;
-                } else leaf = walk(a.levels, node, word);
+                } else leaf = walk(a.levels, a.early, node, word);
                 const float *lf = reinterpret_cast<const float *>(tr + a.ni) + leaf * K;
                 float *d = s_leaf + ((size_t)(buf * TB + t) * K) * R + grp * 32 + lane;
                 constexpr int U = KMAX > 8 ? 1 : KMAX;
@@ -423,7 +434,7 @@ __global__ void __launch_bounds__(1024) k_predict_staged(PredArgs a, int TB) {
                 auto word = [&](uint32_t w) { return xcol[w * rows]; };
                 int leaf;
                 if (a.leaf_idx) a.leaf_idx[(size_t)(t0 + t) * a.out_ld + i] = (uint32_t)walk_id(a.levels, node, word, leaf);
-                else leaf = walk(a.levels, node, word);
+                else leaf = walk(a.levels, a.early, node, word);
                 add_leaf<KMAX>(a.loss, K, p, reinterpret_cast<const float *>(tr + a.ni) + leaf * K, 1);
             }
         }
@@ -456,7 +467,7 @@ __global__ void __launch_bounds__(256) k_predict_wide(PredArgs a, const uint32_t
         auto word = [&](uint32_t w) { return xr[w]; };
         int leaf;
         if (a.leaf_idx) a.leaf_idx[(size_t)t * a.out_ld + i] = (uint32_t)walk_id(a.levels, node, word, leaf);
-        else leaf = walk(a.levels, node, word);
+        else leaf = walk(a.levels, a.early, node, word);
         add_leaf<KMAX>(a.loss, K, p, reinterpret_cast<const float *>(tr + a.ni) + leaf * K, 1);
     }
     if (a.apply_link) link_row<KMAX>(a.loss, K, p);
@@ -472,6 +483,7 @@ static int32_t no_host_memory() {
 }
 struct evb_model {
     int device = 0, loss = 0, K = 1, ntrees = 0, ni = 4, tw = 8, levels = 0, nfeats = 0, nedges = 0;
+    bool early = false;               // fewer than an eighth of the complete trees' inner nodes test anything
     void *block = nullptr;            // trees, then the edges as double and as float
     const uint32_t *d_trees = nullptr;
     const double *d_e64 = nullptr;
@@ -536,6 +548,7 @@ struct PackJob {
     bool categories;            // some feature is not numeric
     unsigned char *snap;
     std::atomic<long long> bad; // tree and node of a test that cannot be: (tree << 32 | node) + 1; -1: out of memory
+    std::atomic<long long> tests; // nodes of all trees that paths come to and that test something
 };
 // last of the nodes [b, e) that has a test; -1: none
 int deepest_split(const uint8_t *split, int b, int e) {
@@ -551,8 +564,8 @@ int deepest_split(const uint8_t *split, int b, int e) {
 // A node of the complete tree is the tree's own node of the same number where a path comes there: `live` says whether one does.  Nothing branches on
 // what a node holds (mispredicted ones cost more than the rest).  NUM: no categories.  Returns whether a test is of a feature that is none.
 template <bool NUM>
-bool pack_nodes(uint32_t *tr, int n, const unsigned char *feat, const uint8_t *bin, const uint8_t *split, const uint8_t *numeric, uint64_t nfeats, uint32_t *live) {
-    uint32_t bad = 0u;
+bool pack_nodes(uint32_t *tr, int n, const unsigned char *feat, const uint8_t *bin, const uint8_t *split, const uint8_t *numeric, uint64_t nfeats, uint32_t *live, long long &tests) {
+    uint32_t bad = 0u, n_tests = 0u;
     for (int i = 0; i < n; ++i) {
         int64_t f;
         memcpy(&f, feat + (size_t)i * 8, 8); // (at any address)
@@ -564,7 +577,9 @@ bool pack_nodes(uint32_t *tr, int n, const unsigned char *feat, const uint8_t *b
         const uint32_t l = live[i] & s;
         tr[i] = l ? w : STOP;
         live[2 * i + 1] = live[2 * i + 2] = l;
+        n_tests += l;
     }
+    tests += n_tests;
     return bad != 0u;
 }
 void pack_trees_of(PackJob &j, char *dst, size_t first, size_t count) {
@@ -574,6 +589,7 @@ void pack_trees_of(PackJob &j, char *dst, size_t first, size_t count) {
     const size_t row = (size_t)m.K * 4;
     std::vector<uint32_t> live((size_t)2 * last + 1);
     std::vector<int> ends((size_t)last + 1);
+    long long tests = 0;
     for (size_t t = first; t < first + count; ++t, tr += m.tw) {
         const void *part[4];
         const int nn = j.nodes[t];
@@ -592,8 +608,8 @@ void pack_trees_of(PackJob &j, char *dst, size_t first, size_t count) {
         const int inner = std::min(last, std::max(0, (nn - 1) / 2));        // nodes that may test something: their children are nodes of the tree
         live[0] = nn > 0 ? 1u : 0u;
         bool bad = deepest_split(split, inner, nn) >= 0;
-        bad |= j.categories ? pack_nodes<false>(tr, inner, feat, bin, split, j.feattypes, (uint64_t)m.nfeats, live.data())
-                            : pack_nodes<true>(tr, inner, feat, bin, split, nullptr, (uint64_t)m.nfeats, live.data());
+        bad |= j.categories ? pack_nodes<false>(tr, inner, feat, bin, split, j.feattypes, (uint64_t)m.nfeats, live.data(), tests)
+                            : pack_nodes<true>(tr, inner, feat, bin, split, nullptr, (uint64_t)m.nfeats, live.data(), tests);
         if (bad) {
             int i = 0;
             for (; i < nn; ++i) {
@@ -623,6 +639,7 @@ void pack_trees_of(PackJob &j, char *dst, size_t first, size_t count) {
             memcpy(leaf + (size_t)at * row, pred + (size_t)i * row, row);
         }
     }
+    j.tests.fetch_add(tests);
 }
 
 void pack_trees(void *ctx, char *dst, size_t first, size_t count) { // (on any thread)
@@ -652,7 +669,7 @@ int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32
     const size_t unit = (size_t)m->tw * 4, tbytes = (size_t)ntrees * unit, ne = (size_t)m->nedges * nfeats;
     const size_t o64 = (tbytes + 15) & ~(size_t)15, o32 = o64 + ne * 8, total = o32 + ne * 4 + 16;
     const bool categories = feattypes && memchr(feattypes, 0, (size_t)nfeats) != nullptr;
-    PackJob job{m, src, nodes, feattypes, categories, nullptr, {0}};
+    PackJob job{m, src, nodes, feattypes, categories, nullptr, {0}, {0}};
     if (snapshot) {
         m->src.assign(src, src + (size_t)ntrees * 4);
         m->nodes.assign(nodes, nodes + ntrees);
@@ -700,6 +717,7 @@ int32_t model_fill(evb_model *m, int ntrees, const void *const *src, const int32
     if (cudaStreamSynchronize(st) != cudaSuccess && rc == EVB_OK) { evb_set_error("CUDA error %s while a model was uploaded", cudaGetErrorString(cudaGetLastError())); rc = EVB_ERR_CUDA; }
     evb_stream_put(st);
     EVB_CHECK(rc);
+    m->early = 8 * job.tests.load() < (long long)ntrees * ((1 << m->levels) - 1);
     m->d_trees = static_cast<const uint32_t *>(m->block);
     m->d_e64 = reinterpret_cast<const double *>(static_cast<char *>(m->block) + o64);
     m->d_e32 = reinterpret_cast<const float *>(static_cast<char *>(m->block) + o32);
@@ -920,6 +938,12 @@ int32_t launch_k(const PredPlan &p, PredArgs &a, uint32_t *xw, cudaStream_t st) 
     return launch_t<64, T>(p, a, xw, st);
 }
 
+// Models most of whose paths end early: a lane leaves the loop there.  That is two instructions more a level and lanes that wait for each other, so it pays
+// where little is left of the complete trees, and not where a few warps an SM wait for their loads.  us of a call, to the last level and leaving, 200 trees of
+// depth 11, one output, at shares of the inner nodes that test something: 500k rows 1.0 1938 and 2050, 0.37 1920 and 1931, 0.14 1908 and 1793, 0.11 1922 and 1471; 20k rows
+// 0.14 174 and 177, 0.11 175 and 167; 2k rows 0.11 76 and 84; depth 8, 500k rows 0.26 1377 and 1298, 0.10 1369 and 1239.
+constexpr int EARLY_ROWS = 8 * 1024;
+
 // Rows of a chunk, of in_row bytes going up and out_row coming back each.
 // Big enough that a chunk's fixed costs (about 15 us of launches) vanish in its transfer, small enough that the
 // first transfer and the last kernel, which nothing overlaps with, do not show; three of them stay in the host's L3.  10M x 50
@@ -992,6 +1016,7 @@ int32_t predict_rows(const evb_model &m, int ntrees, const void *x, int x_type, 
         if (row_major) evb_copy_packed(s.pin_in, xs + (size_t)r0 * in_row, (size_t)nr * in_row, 0, 0, (size_t)nr * in_row, true);
         else evb_copy_packed(s.pin_in, xs + (size_t)r0 * es, (size_t)nr * es, (size_t)nobs * es, 0, (size_t)nr * in_row, true);
         a.n = (int)nr; a.ld = row_major ? m.nfeats : nr;
+        a.early = m.early && nr > EARLY_ROWS;
         a.vec = row_major && es == 4 && (m.nfeats & 3) == 0;
         a.x = s.pin_in;
         if (!zero_copy) {

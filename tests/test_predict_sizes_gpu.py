@@ -113,6 +113,25 @@ def test_walks_end_at_the_deepest_test(pkg):
         assert n[kernel] == 1, list(n)
 
 
+@pytest.mark.parametrize("K", [1, 2, 5, 9])
+@pytest.mark.parametrize("rows", [8_192, 8_193, 400_003])
+def test_models_whose_paths_end_early(pkg, K, rows):
+    """One deep path a tree, all others end at a few levels: lanes of launches of more than 8192 rows leave the walk where their path ends"""
+    m = _model(pkg, 4, 11, 9, K, 64, "mlogloss" if K > 2 else "mse", rows + K)
+    rng = np.random.default_rng(K)
+    for i, t in enumerate(m.trees[1:]):
+        t.split[2 ** (i % 4) - 1:] = 0
+        n = 0
+        while 2 * n + 2 < t.feat.size:                                        # the path of a random row, all the way down
+            t.split[n], t.feat[n], t.cond_bin[n] = 1, rng.integers(1, 5), rng.integers(20, 40)
+            n = 2 * n + 1 + rng.integers(2)
+    x = np.random.default_rng(rows).normal(size=(rows, 4)).astype(np.float32)
+    want, leaves = _walk(m, x)
+    assert leaves.max() >= 2 ** 10 - 1                                        # some rows get there
+    np.testing.assert_allclose(pkg.predict(m, x).reshape(want.shape), want, rtol=1e-5, atol=1e-6)
+    assert np.array_equal(pkg.predict_leaf_idx(m, x), leaves)
+
+
 @pytest.mark.parametrize("K", [1, 3])
 def test_wide_rows_of_bins(pkg, K):
     """Rows of 7 000 bins: too wide for the kernels that keep a row in shared memory"""
